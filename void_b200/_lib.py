@@ -4,6 +4,7 @@ The library is the only compute path of this package: there is no CPU or PyTorch
 Loading fails loudly when the shared object is missing and cannot be built.
 """
 import ctypes
+import importlib.util
 import os
 import threading
 
@@ -105,7 +106,7 @@ def load():
         if _LIB is not None:
             return _LIB
         path = _build.LIB_PATH
-        if not os.path.exists(path) or (_build.needs_build() and _build.have_nvcc()):
+        if not (os.path.exists(path) and os.path.exists(_build.NATIVE_PATH)) or (_build.needs_build() and _build.have_nvcc()):
             path = _build.build()
         if not os.path.exists(path):
             raise VoidB200Error(
@@ -120,6 +121,27 @@ def load():
             raise VoidB200Error("void_b200: ABI version mismatch, rebuild with python -m void_b200.build --force")
         _LIB = lib
     return _LIB
+
+
+_NATIVE = None
+
+
+def native():
+    """The native host path (csrc/host.cpp), loaded on first use."""
+    global _NATIVE
+    if _NATIVE is None:
+        load()
+        with _LOCK:
+            if _NATIVE is None:
+                if not os.path.exists(_build.NATIVE_PATH):
+                    raise VoidB200Error("void_b200: the native host library %s is missing and could not be built"
+                                        % _build.NATIVE_PATH)
+                spec = importlib.util.spec_from_file_location("void_b200._native", _build.NATIVE_PATH)
+                mod = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(mod)
+                mod.set_error(VoidB200Error)
+                _NATIVE = mod
+    return _NATIVE
 
 
 def check(status, what=""):

@@ -3,9 +3,9 @@
 Every function here ends in a call of the C ABI (include/void_b200.h).  Nothing computes on the
 CPU; tensors that are not on a CUDA device are rejected.
 """
-import ctypes
+import functools
 import weakref
-from dataclasses import dataclass
+from dataclasses import dataclass, field
 from typing import Optional
 
 import torch
@@ -15,7 +15,7 @@ from . import _lib
 TILE = 32
 PANEL = 128
 FLAG_DIRECT_STORES, FLAG_A_STABLE, FLAG_STORE_PER_TILE = 2, 4, 16   # bits of void_spmm_args.flags
-FLAG_NO_EARLY_A = 1 << 30   # Python side only: never set FLAG_A_STABLE (measurements)
+FLAG_NO_EARLY_A = 1 << 30   # host side only: never set FLAG_A_STABLE (measurements)
 
 
 def _aligned_empty(nbytes: int, device, align: int = 1024) -> torch.Tensor:
@@ -41,14 +41,30 @@ class PackedTiles:
     shape: tuple
     kind: int                  # _lib.KIND_*
     terms: int = 1             # packed tiles per stored tile (2 / 3: FP8 tiles stored as sums of E4M3 terms)
-    key: tuple = ()
     stable: bool = False       # the kernels that wrote the arrays above are known to have finished
     row_order: Optional[torch.Tensor] = None   # int32 [nbr]: tile rows by falling tile count (launches without a plan)
+    native: object = field(default=None, init=False, repr=False, compare=False)   # the native host path's view of this store (handle())
 
     def is_stable(self) -> bool:
         """True when no kernel still in flight can be writing this store.  A launch may then read
         the store before it waits for the previous kernel of its stream (flag bit 2 of void_spmm_args)."""
         return self.stable
+
+    @functools.cached_property
+    def sms(self) -> int:
+        return sm_count(self.tiles.device)
+
+    def new_handle(self):
+        """What the native host path launches products of this store from, as its fields are now."""
+        return _lib.native().packed_handle(
+            self.shape[0], self.shape[1], self.kind, self.terms, self.nnz, self.stable, _lib.status_word(self.tiles.device),
+            self.tiles, self.tile_cols, self.tile_scales, self.row_ptr, self.row_scale, self.row_order)
+
+    def handle(self):
+        """The handle the operators use, made once."""
+        if self.native is None:
+            self.native = self.new_handle()
+        return self.native
 
 
 def pack(values: torch.Tensor, scales: Optional[torch.Tensor], block_rows: torch.Tensor, block_cols: torch.Tensor,
@@ -138,12 +154,10 @@ def _mark_ready(p: PackedTiles) -> PackedTiles:
 
 def cached_pack(owner, values, scales, block_rows, block_cols, shape, kind) -> PackedTiles:
     """Packed store cached on the tensor object, rebuilt when its storage or contents change."""
-    key = (kind, values.data_ptr(), values._version, None if scales is None else (scales.data_ptr(), scales._version),
-           block_rows.data_ptr(), block_cols.data_ptr(), str(values.device), tuple(shape))
-    p = getattr(owner, "_packed_cache", None)
-    if p is None or p.key != key:
+    p = owner.__dict__.get("_packed_cache")
+    if p is None or not _lib.native().packed_is_current(p.native, values, scales, block_rows, block_cols, shape):
         p = _mark_ready(pack(values, scales, block_rows, block_cols, shape, kind))
-        p.key = key
+        _lib.native().packed_made_from(p.handle(), values, scales, block_rows, block_cols)
         owner._packed_cache = p
         owner._plan_cache = {}
     return p
@@ -179,6 +193,13 @@ class Plan:
     counters: torch.Tensor
     mode: int
     chunk_tiles: int
+
+    def native_args(self) -> tuple:
+        return self.segs, self.cta_seg_ptr, self.n_cta, self.partials, self.counters, self.np
+
+    def options(self, acc_out=None, worker_partials=None) -> tuple:
+        """The native product call's options for a launch with this plan."""
+        return self.native_args(), acc_out, worker_partials, 0, 0, 0, 0, 0, None, 0, 0, None, True
 
 
 def default_panels(nbr: int, N: int, sms: int) -> int:
@@ -273,80 +294,10 @@ def spmm(packed: PackedTiles, b: torch.Tensor, out: torch.Tensor, *, scale_mode:
          grid: int = 0, tiles_per_stage: int = 0, cta_shape: int = 0, trace=None, flags: int = 0,
          row_bias=None, transposed: bool = False, test_hooks: int = 0, sorted_rows: Optional[bool] = None) -> torch.Tensor:
     """One launch of void_spmm_i8 / void_spmm_f8 / void_spmm_fp on the current stream of b's device.
-    With ``transposed`` b is [N, K] and out is [N, M]: the product is out = b @ A^T, both used as they lie."""
-    lib = _lib.load()
-    _lib.require_cuda(b, out, packed.tiles)
-    dev = b.device
-    M, K = packed.shape
-    N = b.shape[0] if transposed else b.shape[1]
-    if (b.shape[1] if transposed else b.shape[0]) != K:
-        raise _lib.VoidB200Error("shape mismatch: A is %s, B is %s" % (packed.shape, tuple(b.shape)))
-    want = (N, M) if transposed else (M, N)
-    if tuple(out.shape) != want or out.stride(1) != 1:
-        raise _lib.VoidB200Error("out must be a row-major [%d, %d] tensor" % want)
-    if out.dtype not in _lib.OUT_DTYPE_CODE:
-        raise _lib.VoidB200Error("unsupported output dtype %s" % out.dtype)
-    es = _lib.KIND_ELEM_BYTES[packed.kind]
-    b = prepare_b(b, es)
-    a = _lib.SpmmArgs()
-    a.tiles = packed.tiles.data_ptr()
-    a.tile_cols = packed.tile_cols.data_ptr()
-    a.tile_scales = packed.tile_scales.data_ptr()
-    a.row_ptr = packed.row_ptr.data_ptr()
-    a.row_scale = packed.row_scale.data_ptr() if (use_row_scale and scale_mode == _lib.SCALE_ROW_MEAN and es == 1) else None
-    a.nbr, a.nbc, a.nnz = packed.nbr, packed.nbc, packed.nnz
-    a.b, a.ldb, a.K, a.N = b.data_ptr(), b.stride(0) * es, K, N
-    keep = [b]
-    if col_scale is not None:
-        col_scale = col_scale.to(device=dev, dtype=torch.float32).contiguous()
-        keep.append(col_scale)
-        a.col_scale = col_scale.data_ptr()
-    a.b_scale = float(b_scale)
-    if bias is not None:
-        bias = bias.to(device=dev, dtype=torch.float32).contiguous()
-        keep.append(bias)
-        a.bias = bias.data_ptr()
-    if row_bias is not None:
-        row_bias = row_bias.to(device=dev, dtype=torch.float32).contiguous()
-        if row_bias.numel() != M:
-            raise _lib.VoidB200Error("row bias must have %d elements, got %d" % (M, row_bias.numel()))
-        keep.append(row_bias)
-        a.row_bias = row_bias.data_ptr()
-    a.out, a.ldc, a.M = out.data_ptr(), out.stride(0), M
-    a.out_dtype = _lib.OUT_DTYPE_CODE[out.dtype]
-    a.act = act
-    a.scale_mode = scale_mode
-    a.acc_out = None if acc_out is None else acc_out.data_ptr()
-    if plan is not None:
-        a.segs, a.cta_seg_ptr, a.n_cta = plan.segs.data_ptr(), plan.cta_seg_ptr.data_ptr(), plan.n_cta
-        if plan.partials is not None:
-            a.partials, a.partials_bytes = plan.partials.data_ptr(), plan.partials.numel() * 4
-        a.counters = plan.counters.data_ptr()
-        panels_per_item = plan.np
-    # tile rows taken by falling tile count: measured on B200 at the 4096^2 sweep and at 16384^2, INT8 gains 3 - 5 %
-    # (6.80 -> 6.58 us at 90 %, 10.33 -> 10.02 at 70 %, 72.7 -> 68.7 at 16384^2); FP8 tiles stored as two terms gain at
-    # 90 % (7.88 -> 7.57) and lose at 70 % (13.55 -> 13.76), 16- and 32-bit tiles lose (TF32 70 %: 31.7 -> 33.1): the
-    # balance it buys weighs less, and the scattered order of A more, the more bytes a tile row holds.  By default:
-    # INT8 always, FP8 while a tile row averages at most 16 tiles, the floating kinds never
-    if sorted_rows is None:
-        sorted_rows = packed.kind == _lib.KIND_I8 or (packed.kind == _lib.KIND_F8E4M3 and packed.nnz <= 16 * packed.nbr)
-    if plan is None and sorted_rows and packed.row_order is not None:
-        a.row_order = packed.row_order.data_ptr()
-    a.worker_partials = None if worker_partials is None else worker_partials.data_ptr()
-    a.status = _lib.status_word(dev).data_ptr()
-    a.panels_per_item, a.stages, a.grid, a.tiles_per_stage = panels_per_item, stages, grid, tiles_per_stage
-    a.trace = None if trace is None else trace.data_ptr()
-    a.cta_shape = cta_shape
-    a.transposed = 1 if transposed else 0
-    # bit 2: the packed store (and the plan, whose builder synchronises) is complete, so the kernel may
-    # read it before it waits for the previous kernel of the stream
-    a.flags = (flags & 0xffff) | (FLAG_A_STABLE if (packed.is_stable() and not (flags & FLAG_NO_EARLY_A)) else 0)
-    a.test_hooks = test_hooks
-    a.tile_terms = packed.terms
-    with torch.cuda.device(dev):
-        if es > 1:
-            _lib.check(lib.void_spmm_fp(ctypes.byref(a), packed.kind, _lib.stream_ptr(dev)), "void_spmm_fp")
-        else:
-            fn = lib.void_spmm_i8 if packed.kind == _lib.KIND_I8 else lib.void_spmm_f8
-            _lib.check(fn(ctypes.byref(a), _lib.stream_ptr(dev)), "void_spmm")
-    return out
+    With ``transposed`` b is [N, K] and out is [N, M]: the product is out = b @ A^T, both used as they lie.
+    The operators call the native host path directly; this form names every option of a launch and takes the
+    fields of ``packed`` as they are at the call."""
+    opts = (None if plan is None else plan.native_args(), acc_out, worker_partials, panels_per_item, stages, grid,
+            tiles_per_stage, cta_shape, trace, flags, test_hooks, sorted_rows, use_row_scale)
+    return _lib.native().spmm(packed.new_handle(), b, out, None, scale_mode == _lib.SCALE_PER_TILE, col_scale, b_scale, bias,
+                              row_bias, act, transposed, opts)

@@ -1,23 +1,27 @@
-"""Builds the C-ABI shared library of the SpMM path for sm_100a with nvcc.
+"""Builds the libraries of the SpMM path in-tree (void_b200/lib): the C-ABI library for sm_100a with nvcc, and the
+native host path of the Python operators (a CPython extension on top of it) with the C++ compiler.
 
-The library is built in-tree (void_b200/lib/libvoid_b200.so).  nvcc cross-compiles for
-sm_100a without a GPU.  Run as ``python -m void_b200.build``.
+nvcc cross-compiles for sm_100a without a GPU.  Run as ``python -m void_b200.build``.
 """
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
+import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libvoid_b200.so")
+NATIVE_PATH = os.path.join(LIB_DIR, "_native.so")
 SOURCES = ["spmm.cu", "prep.cu", "plan.cu", "format.cu", "tile_grad.cu"]
+HOST_SOURCE = os.path.join(CSRC, "host.cpp")
 HEADERS = [os.path.join(CSRC, "ptx.cuh"), os.path.join(HERE, "..", "include", "void_b200.h")]
 
 NVCC_FLAGS = [
     "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
-    "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "-shared",
+    "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
 ]
 
 
@@ -33,25 +37,56 @@ def have_nvcc():
 
 
 def needs_build():
-    if not os.path.exists(LIB_PATH):
+    if not (os.path.exists(LIB_PATH) and os.path.exists(NATIVE_PATH)):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, s) for s in SOURCES if os.path.exists(os.path.join(CSRC, s))] + HEADERS
+    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(NATIVE_PATH))
+    deps = [os.path.join(CSRC, s) for s in SOURCES if os.path.exists(os.path.join(CSRC, s))] + HEADERS + [HOST_SOURCE]
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _host_compile(obj):
+    """Command that compiles host.cpp against the headers of this Python and of the installed torch."""
+    import torch
+    from torch.utils import cpp_extension
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    inc = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden",
+            "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)] \
+        + [f for d in inc for f in ("-isystem", d)] + ["-c", HOST_SOURCE, "-o", obj]
+
+
+def _host_link(obj):
+    from torch.utils import cpp_extension
+    dirs = cpp_extension.library_paths()
+    return ["g++", "-shared", "-o", NATIVE_PATH, obj, LIB_PATH] + [f for d in dirs for f in ("-L" + d, "-Wl,-rpath," + d)] \
+        + ["-Wl,-rpath,$ORIGIN", "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+
+
+def _run_all(cmds, verbose):
+    """Runs the commands side by side; raises with the output of the first that failed."""
+    procs = [(c, subprocess.Popen(c, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)) for c in cmds]
+    outs = [(c, p.communicate()[0], p.returncode) for c, p in procs]
+    for c, out, rc in outs:
+        if rc != 0:
+            raise RuntimeError("%s failed:\n%s" % (" ".join(c[:1]), out))
+        if verbose:
+            print(out)
+
+
 def build(force=False, verbose=False):
-    """Compile every .cu source into one shared library; returns its path."""
+    """Compile every source (in parallel) and link both libraries; returns the C-ABI library's path."""
     if not force and not needs_build():
         return LIB_PATH
     os.makedirs(LIB_DIR, exist_ok=True)
-    srcs = [os.path.join(CSRC, s) for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
-    cmd = [_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", LIB_PATH] + srcs
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
-    if verbose:
-        print(res.stdout + res.stderr)
+    srcs = [s for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
+    with tempfile.TemporaryDirectory() as tmp:
+        objs = [os.path.join(tmp, s + ".o") for s in srcs]
+        extra = ["-Xptxas", "-v"] if verbose else []
+        host_obj = os.path.join(tmp, "host.o")
+        _run_all([[_nvcc()] + NVCC_FLAGS + extra + ["-c", os.path.join(CSRC, s), "-o", o] for s, o in zip(srcs, objs)]
+                 + [_host_compile(host_obj)], verbose)
+        _run_all([[_nvcc()] + NVCC_FLAGS + ["-shared", "-o", LIB_PATH] + objs], verbose)
+        _run_all([_host_link(host_obj)], verbose)
     return LIB_PATH
 
 

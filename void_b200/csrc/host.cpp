@@ -1,0 +1,336 @@
+// Host path of the operators: argument checks, output allocation and the call of the C ABI, natively.
+//
+// One product of a served layer takes 3 - 15 us on the GPU; the same call written in Python (ctypes structure filled
+// field by field, device guards, property reads) took 17 - 20 us of host time, so the stream ran dry between calls.
+// Everything here ends in the entry points of include/void_b200.h; nothing computes on the CPU.  Functions take their
+// arguments by position (METH_FASTCALL) from the Python operators, which keep the public signatures.
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <string>
+
+#include "../../include/void_b200.h"
+
+namespace {
+
+PyObject* g_error = nullptr;  // void_b200._lib.VoidB200Error
+
+// Raised as VoidB200Error; caught at the boundary of every function of the module.
+struct Failure {
+  std::string text;
+};
+[[noreturn]] void fail(const std::string& text) { throw Failure{text}; }
+void check(int status, const char* what) {
+  if (status != VOID_OK)
+    fail(std::string("void_b200 ") + what + " failed: " + void_strerror(status) + " (status " + std::to_string(status) + ")");
+}
+
+bool none(PyObject* o) { return o == Py_None || o == nullptr; }
+const at::Tensor& tensor(PyObject* o, const char* what) {
+  if (!THPVariable_Check(o)) throw torch::TypeError(std::string(what) + " must be a tensor");
+  return THPVariable_Unpack(o);
+}
+const at::Tensor& cuda_tensor(PyObject* o, const char* what) {
+  const at::Tensor& t = tensor(o, what);
+  if (!t.is_cuda())
+    fail("void_b200 runs on a B200 GPU only: got a tensor on " + t.device().str() + " (there is no CPU path)");
+  return t;
+}
+int64_t integer(PyObject* o) {
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) throw python_error();
+  return v;
+}
+double real(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw python_error();
+  return v;
+}
+int out_code(at::ScalarType t) {
+  switch (t) {
+    case at::kFloat: return VOID_OUT_F32;
+    case at::kHalf: return VOID_OUT_F16;
+    case at::kBFloat16: return VOID_OUT_BF16;
+    default: fail(std::string("unsupported output dtype ") + c10::toString(t));
+  }
+}
+int elem_bytes(int kind) { return kind == VOID_KIND_TF32 ? 4 : ((kind == VOID_KIND_F16 || kind == VOID_KIND_BF16) ? 2 : 1); }
+at::Tensor new_cuda(at::IntArrayRef size, at::ScalarType type, c10::Device dev) {
+  return at::Tensor(at::detail::empty_cuda(size, type, dev, std::nullopt));
+}
+void_stream_t stream_of(c10::DeviceIndex dev) { return c10::cuda::getCurrentCUDAStream(dev).stream(); }
+
+#define NATIVE_BEGIN                                    \
+  HANDLE_TH_ERRORS                                      \
+  try {
+#define NATIVE_END                                      \
+  }                                                     \
+  catch (const Failure& f) {                            \
+    PyErr_SetString(g_error, f.text.c_str());           \
+    return nullptr;                                     \
+  }                                                     \
+  END_HANDLE_TH_ERRORS
+
+// ------------------------------------------------------------------------------------------ packed A
+// The C ABI's view of a packed tensor and the identity (address and version) of the tensors it was made from.
+struct Identity {
+  const void* ptr = nullptr;
+  int64_t version = 0;
+  bool operator==(const Identity& o) const { return ptr == o.ptr && version == o.version; }
+};
+Identity identity(PyObject* o) {
+  Identity id;
+  if (none(o)) return id;
+  const at::Tensor& t = tensor(o, "operand");
+  id.ptr = t.const_data_ptr();
+  id.version = t.is_inference() ? 0 : (int64_t)t._version();
+  return id;
+}
+struct PackedObject {
+  PyObject_HEAD
+  void_spmm_args args;   // the fields of A; everything of a launch is filled into a copy
+  const int32_t* row_order;
+  const float* row_scale;
+  Identity made_from[4]; // values, scales, block rows, block columns
+  int64_t M, K;
+  int32_t kind;
+  int32_t stable;
+  c10::DeviceIndex device;
+};
+PyTypeObject* g_packed_type = nullptr;
+
+PackedObject* packed_of(PyObject* o) {
+  if (Py_TYPE(o) != g_packed_type) throw torch::TypeError("expected a packed tensor handle");
+  return reinterpret_cast<PackedObject*>(o);
+}
+template <typename T>
+T* data_or_null(PyObject* o) {
+  return none(o) ? nullptr : static_cast<T*>(tensor(o, "operand").data_ptr());
+}
+
+// packed_handle(M, K, kind, terms, nnz, stable, status, tiles, tile_cols, tile_scales, row_ptr, row_scale, row_order)
+PyObject* packed_handle(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 13) throw torch::TypeError("packed_handle takes 13 arguments");
+  PyObject* self = PyType_GenericAlloc(g_packed_type, 0);
+  if (self == nullptr) return nullptr;
+  PackedObject* p = reinterpret_cast<PackedObject*>(self);
+  p->args = void_spmm_args();
+  p->M = integer(a[0]);
+  p->K = integer(a[1]);
+  p->kind = (int32_t)integer(a[2]);
+  p->args.tile_terms = (int32_t)integer(a[3]);
+  p->args.nnz = integer(a[4]);
+  p->stable = (int32_t)integer(a[5]);
+  p->args.status = data_or_null<int32_t>(a[6]);
+  p->args.tiles = data_or_null<void>(a[7]);
+  p->args.tile_cols = data_or_null<int32_t>(a[8]);
+  p->args.tile_scales = data_or_null<float>(a[9]);
+  p->args.row_ptr = data_or_null<int32_t>(a[10]);
+  p->row_scale = data_or_null<float>(a[11]);
+  p->row_order = data_or_null<int32_t>(a[12]);
+  p->args.nbr = (int32_t)((p->M + 31) / 32);
+  p->args.nbc = (int32_t)((p->K + 31) / 32);
+  p->args.M = (int32_t)p->M;
+  p->args.K = (int32_t)p->K;
+  p->device = tensor(a[7], "tiles").device().index();
+  return self;
+  NATIVE_END
+}
+
+// packed_made_from(handle, values, scales, block_rows, block_cols): note what the store was packed from
+PyObject* packed_made_from(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 5) throw torch::TypeError("packed_made_from takes 5 arguments");
+  PackedObject* p = packed_of(a[0]);
+  for (int i = 0; i < 4; ++i) p->made_from[i] = identity(a[1 + i]);
+  Py_RETURN_NONE;
+  NATIVE_END
+}
+// packed_is_current(handle, values, scales, block_rows, block_cols, shape): the store still belongs to these tensors
+PyObject* packed_is_current(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 6) throw torch::TypeError("packed_is_current takes 6 arguments");
+  const PackedObject* p = packed_of(a[0]);
+  for (int i = 0; i < 4; ++i)
+    if (!(p->made_from[i] == identity(a[1 + i]))) Py_RETURN_FALSE;
+  PyObject* shape = a[5];
+  if (!PyTuple_Check(shape) || PyTuple_GET_SIZE(shape) != 2 || integer(PyTuple_GET_ITEM(shape, 0)) != p->M ||
+      integer(PyTuple_GET_ITEM(shape, 1)) != p->K)
+    Py_RETURN_FALSE;
+  Py_RETURN_TRUE;
+  NATIVE_END
+}
+
+// ------------------------------------------------------------------------------------------ products
+// B with unit column stride and rows on 16-byte boundaries, as the copy engine needs them; others are copied.
+at::Tensor kernel_operand(const at::Tensor& b, int es) {
+  if (b.element_size() != es)
+    fail("B must have " + std::to_string(es) + "-byte elements to match A, got " + c10::toString(b.scalar_type()));
+  const int64_t per16 = 16 / es;
+  if (b.stride(1) == 1 && b.stride(0) % per16 == 0 && (reinterpret_cast<uintptr_t>(b.const_data_ptr()) & 15u) == 0 &&
+      b.stride(0) >= b.size(1))
+    return b;
+  const int64_t ld = (b.size(1) + per16 - 1) / per16 * per16;
+  at::Tensor padded = at::zeros({b.size(0), ld}, b.options());
+  at::Tensor view = padded.narrow(1, 0, b.size(1));
+  view.copy_(b);
+  return view;
+}
+at::Tensor fp32_vector(PyObject* o, c10::Device dev, const char* what) {
+  const at::Tensor& t = tensor(o, what);
+  if (t.scalar_type() == at::kFloat && t.device() == dev && t.is_contiguous()) return t;
+  return t.to(dev, at::kFloat).contiguous();
+}
+
+// spmm(handle, b, out | None, out_dtype | None, per_tile, col_scale | None, b_scale, bias | None, row_bias | None, act,
+//      transposed, options | None) -> out
+// options: (plan | None, acc_out, worker_partials, panels, stages, grid, tiles_per_stage, cta_shape, trace, flags,
+//           test_hooks, sorted_rows | None, use_row_scale); plan: (segs, cta_seg_ptr, n_cta, partials | None, counters, panels)
+PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 12) throw torch::TypeError("spmm takes 12 arguments");
+  const PackedObject* pk = packed_of(a[0]);
+  const at::Tensor& b_in = cuda_tensor(a[1], "B");
+  const c10::Device dev = b_in.device();
+  const bool tr = PyObject_IsTrue(a[10]) == 1;
+  if (b_in.dim() != 2) fail("B must be a matrix");
+  if (b_in.size(tr ? 1 : 0) != pk->K)
+    fail("shape mismatch: A is (" + std::to_string(pk->M) + ", " + std::to_string(pk->K) + "), B is (" +
+         std::to_string(b_in.size(0)) + ", " + std::to_string(b_in.size(1)) + ")");
+  if (dev.index() != pk->device) fail("A and B are on different devices");
+  const int64_t N = b_in.size(tr ? 0 : 1);
+  const int64_t rows = tr ? N : pk->M, cols = tr ? pk->M : N;
+  const int es = elem_bytes(pk->kind);
+  c10::cuda::OptionalCUDAGuard guard;
+  if (c10::cuda::current_device() != dev.index()) guard.set_device(dev);
+
+  at::Tensor out;
+  if (none(a[2])) {
+    const at::ScalarType type = none(a[3]) ? at::kFloat : reinterpret_cast<THPDtype*>(a[3])->scalar_type;
+    out_code(type);
+    out = new_cuda({rows, cols}, type, dev);
+  } else {
+    out = cuda_tensor(a[2], "out");
+    if (out.dim() != 2 || out.size(0) != rows || out.size(1) != cols || out.stride(1) != 1)
+      fail("out must be a row-major [" + std::to_string(rows) + ", " + std::to_string(cols) + "] tensor");
+  }
+  const at::Tensor b = kernel_operand(b_in, es);
+
+  void_spmm_args s = pk->args;
+  const bool per_tile = PyObject_IsTrue(a[4]) == 1;
+  s.scale_mode = per_tile ? VOID_SCALE_PER_TILE : VOID_SCALE_ROW_MEAN;
+  bool use_row_scale = true;
+  s.b = b.const_data_ptr();
+  s.ldb = b.stride(0) * es;
+  s.N = (int32_t)N;
+  at::Tensor col_scale, bias, row_bias;   // keep converted copies alive until the launch is queued
+  if (!none(a[5])) {
+    col_scale = fp32_vector(a[5], dev, "col_scale");
+    s.col_scale = col_scale.const_data_ptr<float>();
+  }
+  s.b_scale = (float)real(a[6]);
+  if (!none(a[7])) {
+    bias = fp32_vector(a[7], dev, "bias");
+    s.bias = bias.const_data_ptr<float>();
+  }
+  if (!none(a[8])) {
+    row_bias = fp32_vector(a[8], dev, "row bias");
+    if (row_bias.numel() != pk->M)
+      fail("row bias must have " + std::to_string(pk->M) + " elements, got " + std::to_string(row_bias.numel()));
+    s.row_bias = row_bias.const_data_ptr<float>();
+  }
+  s.out = out.data_ptr();
+  s.ldc = out.stride(0);
+  s.out_dtype = out_code(out.scalar_type());
+  s.act = (int32_t)integer(a[9]);
+  s.transposed = tr ? 1 : 0;
+  // Tile rows taken by falling tile count: measured at the 4096^2 sweep and at 16384^2, INT8 gains 3 - 5 %
+  // (6.80 -> 6.58 us at 90 %, 10.33 -> 10.02 at 70 %, 72.7 -> 68.7 at 16384^2); FP8 tiles stored as two terms gain at
+  // 90 % (7.88 -> 7.57) and lose at 70 % (13.55 -> 13.76), 16- and 32-bit tiles lose (TF32 70 %: 31.7 -> 33.1): the
+  // balance it buys weighs less, and the scattered order of A more, the more bytes a tile row holds.
+  bool sorted_rows = pk->kind == VOID_KIND_I8 || (pk->kind == VOID_KIND_F8E4M3 && s.nnz <= 16ll * s.nbr);
+  int64_t flags = 0;
+  if (!none(a[11])) {
+    PyObject* o = a[11];
+    if (!PyTuple_Check(o) || PyTuple_GET_SIZE(o) != 13) throw torch::TypeError("spmm: options is a tuple of 13");
+    PyObject* plan = PyTuple_GET_ITEM(o, 0);
+    s.panels_per_item = (int32_t)integer(PyTuple_GET_ITEM(o, 3));
+    if (!none(plan)) {
+      if (!PyTuple_Check(plan) || PyTuple_GET_SIZE(plan) != 6) throw torch::TypeError("spmm: a plan is a tuple of 6");
+      s.segs = data_or_null<int32_t>(PyTuple_GET_ITEM(plan, 0));
+      s.cta_seg_ptr = data_or_null<int32_t>(PyTuple_GET_ITEM(plan, 1));
+      s.n_cta = (int32_t)integer(PyTuple_GET_ITEM(plan, 2));
+      if (!none(PyTuple_GET_ITEM(plan, 3))) {
+        const at::Tensor& parts = tensor(PyTuple_GET_ITEM(plan, 3), "partials");
+        s.partials = parts.data_ptr();
+        s.partials_bytes = parts.numel() * 4;
+      }
+      s.counters = data_or_null<int32_t>(PyTuple_GET_ITEM(plan, 4));
+      s.panels_per_item = (int32_t)integer(PyTuple_GET_ITEM(plan, 5));
+    }
+    s.acc_out = data_or_null<void>(PyTuple_GET_ITEM(o, 1));
+    s.worker_partials = data_or_null<void>(PyTuple_GET_ITEM(o, 2));
+    s.stages = (int32_t)integer(PyTuple_GET_ITEM(o, 4));
+    s.grid = (int32_t)integer(PyTuple_GET_ITEM(o, 5));
+    s.tiles_per_stage = (int32_t)integer(PyTuple_GET_ITEM(o, 6));
+    s.cta_shape = (int32_t)integer(PyTuple_GET_ITEM(o, 7));
+    s.trace = data_or_null<void>(PyTuple_GET_ITEM(o, 8));
+    flags = integer(PyTuple_GET_ITEM(o, 9));
+    s.test_hooks = (int32_t)integer(PyTuple_GET_ITEM(o, 10));
+    if (!none(PyTuple_GET_ITEM(o, 11))) sorted_rows = PyObject_IsTrue(PyTuple_GET_ITEM(o, 11)) == 1;
+    use_row_scale = PyObject_IsTrue(PyTuple_GET_ITEM(o, 12)) == 1;
+  }
+  if (use_row_scale && !per_tile && es == 1) s.row_scale = pk->row_scale;
+  if (s.segs == nullptr && sorted_rows) s.row_order = pk->row_order;
+  // bit 2: the packed store (and the plan, whose builder synchronises) is complete, so the kernel may read it
+  // before it waits for the previous kernel; bit 30 (measurements) keeps it from doing so
+  s.flags = (int32_t)(flags & 0xffff) | ((pk->stable && !(flags & (1ll << 30))) ? 4 : 0);
+  const void_stream_t st = stream_of(dev.index());
+  if (es > 1) check(void_spmm_fp(&s, pk->kind, st), "void_spmm_fp");
+  else check(pk->kind == VOID_KIND_I8 ? void_spmm_i8(&s, st) : void_spmm_f8(&s, st), "void_spmm");
+  if (!none(a[2])) {
+    Py_INCREF(a[2]);
+    return a[2];
+  }
+  return THPVariable_Wrap(out);
+  NATIVE_END
+}
+
+PyObject* set_error(PyObject*, PyObject* cls) {
+  Py_INCREF(cls);
+  g_error = cls;
+  Py_RETURN_NONE;
+}
+
+#define FAST(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
+PyMethodDef kMethods[] = {
+    {"set_error", set_error, METH_O, nullptr},
+    FAST(packed_handle),
+    FAST(packed_made_from),
+    FAST(packed_is_current),
+    FAST(spmm),
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+void packed_dealloc(PyObject* self) {
+  PyTypeObject* type = Py_TYPE(self);
+  type->tp_free(self);
+  Py_DECREF(type);
+}
+PyType_Slot kPackedSlots[] = {{Py_tp_dealloc, (void*)packed_dealloc}, {0, nullptr}};
+PyType_Spec kPackedSpec = {"_native.Packed", (int)sizeof(PackedObject), 0, Py_TPFLAGS_DEFAULT, kPackedSlots};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) {
+  g_packed_type = reinterpret_cast<PyTypeObject*>(PyType_FromSpec(&kPackedSpec));
+  if (g_packed_type == nullptr) return nullptr;
+  return PyModule_Create(&kModule);
+}

@@ -245,14 +245,13 @@ class FP8VOIDTensor:
     def packed_split(self, terms: int) -> _spmm.PackedTiles:
         """Packed copy with the tile scales folded in: every tile as a sum of ``terms`` E4M3 tiles relative to
         the largest scale of its tile row (built once per ``terms``, cached)."""
-        v, sc = self.values_fp8.view(torch.uint8), self.scaling_info.scale
-        key = (terms, v.data_ptr(), v._version, sc.data_ptr(), sc._version, self.block_rows.data_ptr(),
-               self.block_cols.data_ptr(), str(v.device), tuple(self.shape))
+        v, sc = self.values_fp8, self.scaling_info.scale
         cache = self.__dict__.setdefault("_packed_split_cache", {})
         p = cache.get(terms)
-        if p is None or p.key != key:
-            p = _spmm._mark_ready(_spmm.pack_f8_split(v, sc, self.block_rows, self.block_cols, self.shape, terms))
-            p.key = key
+        if p is None or not _lib.native().packed_is_current(p.native, v, sc, self.block_rows, self.block_cols, self.shape):
+            p = _spmm._mark_ready(_spmm.pack_f8_split(v.view(torch.uint8), sc, self.block_rows, self.block_cols, self.shape,
+                                                      terms))
+            _lib.native().packed_made_from(p.handle(), v, sc, self.block_rows, self.block_cols)
             cache[terms] = p
         return p
 
@@ -290,9 +289,7 @@ def void_spmm_fp8(a: FP8VOIDTensor, b: torch.Tensor, output_dtype: torch.dtype =
     _lib.require_cuda(a.values_fp8, b)
     if a.scaling_info.config.format != FP8Format.E4M3:
         raise NotImplementedError("void_b200 implements E4M3 only")
-    M, K = a.shape
-    N = b.shape[1]
-    if b.dtype != torch.float8_e4m3fn:
+    if b.dtype is not torch.float8_e4m3fn:
         # B in floating point stays in floating point, as in the reference kernel (void/fp8.py:648-659: the tile
         # is dequantised, B is loaded as it is, tl.dot multiplies them as TF32): the tiles are dequantised once
         # (cached on the tensor) and the floating-point kernel runs - TF32 for an fp32 B, exact 16-bit products
@@ -307,20 +304,16 @@ def void_spmm_fp8(a: FP8VOIDTensor, b: torch.Tensor, output_dtype: torch.dtype =
         if hit is None or hit[0] != key:
             hit = cache[dt] = (key, a.to_void_tensor(dt))
         if out is None:
-            out = torch.empty(M, N, dtype=output_dtype, device=b.device)
+            out = torch.empty(a.shape[0], b.shape[1], dtype=output_dtype, device=b.device)
         return void_spmm(hit[1], b if b.dtype == dt else b.to(dt), out, activation=activation, bias=bias)
-    b8, col_scale = b, (None if b_scale is None else b_scale.reshape(-1))
-    if out is None:
-        out = torch.empty(M, N, dtype=output_dtype, device=b.device)
+    col_scale = b_scale if b_scale is None or b_scale.dim() == 1 else b_scale.reshape(-1)
     if scale_terms is None:
-        scale_terms = DEFAULT_SCALE_TERMS[out.dtype]
+        scale_terms = DEFAULT_SCALE_TERMS[output_dtype if out is None else out.dtype]
     if scale_terms not in (0, 2, 3):
         raise ValueError("scale_terms must be 0, 2, 3 or None")
-    if scale_terms == 0:
-        return _spmm.spmm(a.packed(), b8.view(torch.uint8), out, scale_mode=_lib.SCALE_PER_TILE, col_scale=col_scale,
-                          bias=bias, act=activation)
-    return _spmm.spmm(a.packed_split(scale_terms), b8.view(torch.uint8), out, scale_mode=_lib.SCALE_ROW_MEAN,
-                      col_scale=col_scale, bias=bias, act=activation)
+    packed = a.packed() if scale_terms == 0 else a.packed_split(scale_terms)
+    return _lib.native().spmm(packed.native, b, out, output_dtype, scale_terms == 0, col_scale, 1.0, bias, None, activation,
+                              False, None)
 
 
 def void_tensor_to_fp8(void_tensor, format: str = "e4m3", scale_mode: str = "per_block") -> FP8VOIDTensor:

@@ -261,18 +261,14 @@ def void_spmm_int8(a: Int8VOIDTensor, b: torch.Tensor, b_scale: Union[None, floa
     Returns fp32 [M, N] unless ``out`` / ``out_dtype`` ask for fp16 / bf16.  ``acc_out`` (int32
     [n_block_rows*32, N]) receives the raw int32 accumulators.
     """
-    M, K = a.shape
-    N = b.shape[1]
     _lib.require_cuda(a.values, b, out)
     b_q, scalar, col_scale = _resolve_b(b, b_scale)
-    if out is None:
-        out = torch.empty(M, N, dtype=out_dtype or torch.float32, device=b.device)
     packed = a.packed()
-    mode = _lib.SCALE_PER_TILE if exact_scales else _lib.SCALE_ROW_MEAN
     # every element of out is written by the kernel (zeros for empty tile rows), so the
     # reference's torch.zeros / out.zero_() (:580-583) has no counterpart here
-    return _spmm.spmm(packed, b_q, out, scale_mode=mode, col_scale=col_scale, b_scale=scalar, bias=bias,
-                      act=activation, acc_out=acc_out, row_bias=row_bias)
+    opts = None if acc_out is None else (None, acc_out, None, 0, 0, 0, 0, 0, None, 0, 0, None, True)
+    return _lib.native().spmm(packed.native, b_q, out, out_dtype or torch.float32, exact_scales, col_scale, scalar, bias,
+                              row_bias, activation, False, opts)
 
 
 def get_quantization_error(original: torch.Tensor, config: IntQuantConfig) -> dict:

@@ -34,15 +34,13 @@ def packed_fp(a: VOIDTensor, kind: int) -> _spmm.PackedTiles:
     cache = getattr(a, "_packed_fp_cache", None)
     if cache is None:
         cache = a._packed_fp_cache = {}
-    key = (a.values.data_ptr(), a.values._version, a.block_rows.data_ptr(), a.block_cols.data_ptr(),
-           str(a.values.device), tuple(a.shape))
     hit = cache.get(kind)
-    if hit is not None and hit.key == key:
+    if hit is not None and _lib.native().packed_is_current(hit.native, a.values, None, a.block_rows, a.block_cols, a.shape):
         return hit
     vals = a.values if a.values.dtype == _KIND_DTYPE[kind] else a.values.to(_KIND_DTYPE[kind])
     row_ptr, block_indices = a.get_row_block_info()
     p = _spmm._mark_ready(_spmm.pack(vals, None, a.block_rows, a.block_cols, a.shape, kind, row_ptr, block_indices))
-    p.key = key
+    _lib.native().packed_made_from(p.handle(), a.values, None, a.block_rows, a.block_cols)
     cache[kind] = p
     a._plan_cache = {}
     return p
@@ -60,21 +58,23 @@ def void_spmm(a: VOIDTensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
     assert b.dim() == 2
     assert a.shape[1] == b.shape[0], f"Dimension mismatch: A is {a.shape}, B is {tuple(b.shape)}"
     _lib.require_cuda(a.values, b)
-    M, _ = a.shape
-    N = b.shape[1]
-    if b.dtype not in _lib.OUT_DTYPE_CODE:
-        raise _lib.VoidB200Error("void_spmm: B must be float32, float16 or bfloat16, got %s" % b.dtype)
-    if out is None:
-        out = torch.empty(M, N, dtype=b.dtype, device=b.device)
+    dtype = b.dtype
+    if dtype not in _lib.OUT_DTYPE_CODE:
+        raise _lib.VoidB200Error("void_spmm: B must be float32, float16 or bfloat16, got %s" % dtype)
     if a.n_blocks == 0 and activation == 0 and bias is None and row_bias is None and plan is None \
             and acc_out is None and worker_partials is None:
-        return out.zero_()      # nothing stored: zeros, whatever the tile size (void/ops.py:169-173)
+        # nothing stored: zeros, whatever the tile size (void/ops.py:169-173)
+        return torch.zeros(a.shape[0], b.shape[1], dtype=dtype, device=b.device) if out is None else out.zero_()
     kind = product_kind(a, b)
     packed = packed_fp(a, kind)
-    if b.dtype != _KIND_DTYPE[kind]:
+    if dtype is not _KIND_DTYPE[kind]:
         b = b.to(_KIND_DTYPE[kind])
-    return _spmm.spmm(packed, b, out, scale_mode=_lib.SCALE_ROW_MEAN, use_row_scale=False, bias=bias, act=activation,
-                      row_bias=row_bias, plan=plan, acc_out=acc_out, worker_partials=worker_partials)
+    opts = None
+    if plan is not None:
+        opts = plan.options(acc_out, worker_partials)
+    elif acc_out is not None or worker_partials is not None:
+        opts = (None, acc_out, worker_partials, 0, 0, 0, 0, 0, None, 0, 0, None, True)
+    return _lib.native().spmm(packed.native, b, out, dtype, False, None, 1.0, bias, row_bias, activation, False, opts)
 
 
 def void_linear(a, x: torch.Tensor, bias: Optional[torch.Tensor] = None, activation: int = 0,
@@ -95,20 +95,16 @@ def void_linear(a, x: torch.Tensor, bias: Optional[torch.Tensor] = None, activat
         if x.dtype != torch.int8:
             raise _lib.VoidB200Error("void_linear with an Int8VOIDTensor takes int8 activations, got %s" % x.dtype)
         scalar, col_scale = (1.0, x_scale) if isinstance(x_scale, torch.Tensor) else (1.0 if x_scale is None else float(x_scale), None)
-        if out is None:
-            out = torch.empty(x.shape[0], M, dtype=out_dtype or torch.float32, device=x.device)
-        return _spmm.spmm(a.packed(), x, out, scale_mode=_lib.SCALE_ROW_MEAN, col_scale=col_scale, b_scale=scalar,
-                          act=activation, row_bias=bias, transposed=True)
+        return _lib.native().spmm(a.packed().native, x, out, out_dtype or torch.float32, False, col_scale, scalar, None,
+                                  bias, activation, True, None)
     if x.dtype not in _lib.OUT_DTYPE_CODE:
         raise _lib.VoidB200Error("void_linear: x must be float32, float16 or bfloat16, got %s" % x.dtype)
-    if out is None:
-        out = torch.empty(x.shape[0], M, dtype=x.dtype, device=x.device)
+    dtype = x.dtype
     kind = product_kind(a, x)
     packed = packed_fp(a, kind)
-    if x.dtype != _KIND_DTYPE[kind]:
+    if dtype is not _KIND_DTYPE[kind]:
         x = x.to(_KIND_DTYPE[kind])
-    return _spmm.spmm(packed, x, out, scale_mode=_lib.SCALE_ROW_MEAN, use_row_scale=False, act=activation, row_bias=bias,
-                      transposed=True)
+    return _lib.native().spmm(packed.native, x, out, dtype, False, None, 1.0, None, bias, activation, True, None)
 
 
 def void_spmv(a: VOIDTensor, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -51,7 +51,7 @@ def compute_stream_k_workload(void_tensor, n_workers: Optional[int] = None,
 
 
 def _plan_for(a, packed, N: int, workload: StreamKWorkload, per_worker: bool, n_cta: Optional[int]):
-    sms = _spmm.sm_count(packed.tiles.device)
+    sms = packed.sms
     np_ = _spmm.default_panels(packed.nbr, N, sms) if _lib.KIND_ELEM_BYTES[packed.kind] == 1 else 1
     if n_cta is None:
         n_cta = sms * 4          # four slim CTAs per SM
@@ -86,20 +86,15 @@ def void_spmm_stream_k(a: Int8VOIDTensor, b: torch.Tensor, workload: Optional[St
         return _stream_k_fp(a, b, workload, out, activation, bias, worker_partials, acc_out, n_cta)
     if not isinstance(a, Int8VOIDTensor):
         raise TypeError("void_spmm_stream_k takes a VOIDTensor or an Int8VOIDTensor, got %s" % type(a).__name__)
-    M, K = a.shape
-    N = b.shape[1]
     b_q, scalar, col_scale = _resolve_b(b, b_scale)
-    if out is None:
-        out = torch.empty(M, N, dtype=out_dtype or torch.float32, device=b.device)
     packed = a.packed()
-    if a.n_blocks == 0:
-        return _spmm.spmm(packed, b_q, out, scale_mode=_lib.SCALE_ROW_MEAN, col_scale=col_scale, b_scale=scalar,
-                          bias=bias, act=activation)
-    if workload is None:
-        workload = _cached_workload(a)
-    plan = _plan_for(a, packed, N, workload, worker_partials is not None, n_cta)
-    return _spmm.spmm(packed, b_q, out, scale_mode=_lib.SCALE_ROW_MEAN, col_scale=col_scale, b_scale=scalar, bias=bias,
-                      act=activation, plan=plan, worker_partials=worker_partials, acc_out=acc_out)
+    opts = None
+    if a.n_blocks != 0:
+        if workload is None:
+            workload = _cached_workload(a)
+        opts = _plan_for(a, packed, b.shape[1], workload, worker_partials is not None, n_cta).options(acc_out, worker_partials)
+    return _lib.native().spmm(packed.native, b_q, out, out_dtype or torch.float32, False, col_scale, scalar, bias, None,
+                              activation, False, opts)
 
 
 def _cached_workload(a) -> StreamKWorkload:
