@@ -302,6 +302,43 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_END
 }
 
+// ------------------------------------------------------------------------------------------ quantisers
+// quant_cols(b, kind) -> (q [K, N], scale [N], scale_inv [N] | None): per-column INT8 or E4M3 of a matrix
+PyObject* quant_cols(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 2) throw torch::TypeError("quant_cols takes 2 arguments");
+  const at::Tensor& in = cuda_tensor(a[0], "b");
+  const int kind = (int)integer(a[1]);
+  if (in.dim() != 2) fail("quantising columns needs a matrix");
+  const c10::Device dev = in.device();
+  c10::cuda::OptionalCUDAGuard guard;
+  if (c10::cuda::current_device() != dev.index()) guard.set_device(dev);
+  at::Tensor b = in.scalar_type() == at::kFloat ? in : in.to(at::kFloat);
+  if (!b.is_contiguous()) b = b.contiguous();
+  const int64_t K = b.size(0), N = b.size(1), ld = (N + 15) / 16 * 16;
+  const bool i8 = kind == VOID_KIND_I8;
+  at::Tensor q = new_cuda({K, ld}, i8 ? at::kChar : at::kFloat8_e4m3fn, dev);
+  at::Tensor scale = new_cuda({N}, at::kFloat, dev);
+  at::Tensor inv;
+  if (!i8) inv = new_cuda({N}, at::kFloat, dev);
+  check(void_quant_cols(b.const_data_ptr<float>(), b.stride(0), (int32_t)K, (int32_t)N, kind, q.data_ptr(), ld,
+                        scale.data_ptr<float>(), i8 ? nullptr : inv.data_ptr<float>(), stream_of(dev.index())),
+        "void_quant_cols");
+  if (ld != N) q = q.narrow(1, 0, N);
+  PyObject* res = PyTuple_New(3);
+  if (res == nullptr) return nullptr;
+  PyTuple_SET_ITEM(res, 0, THPVariable_Wrap(q));
+  PyTuple_SET_ITEM(res, 1, THPVariable_Wrap(scale));
+  if (i8) {
+    Py_INCREF(Py_None);
+    PyTuple_SET_ITEM(res, 2, Py_None);
+  } else {
+    PyTuple_SET_ITEM(res, 2, THPVariable_Wrap(inv));
+  }
+  return res;
+  NATIVE_END
+}
+
 PyObject* set_error(PyObject*, PyObject* cls) {
   Py_INCREF(cls);
   g_error = cls;
@@ -315,6 +352,7 @@ PyMethodDef kMethods[] = {
     FAST(packed_made_from),
     FAST(packed_is_current),
     FAST(spmm),
+    FAST(quant_cols),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

@@ -111,19 +111,7 @@ def _fresh_info(config, scale, scale_inv, amax) -> FP8ScalingInfo:
 def quantize_cols_fp8(b: torch.Tensor):
     """Per-column E4M3 of a [K, N] matrix -> (float8_e4m3fn [K, N], scale [N], scale_inv [N]).
     Same numbers as quantize_to_fp8(b.T, scale_mode='per_row') transposed back."""
-    _lib.require_cuda(b)
-    lib = _lib.load()
-    K, N = b.shape
-    bf = b.to(torch.float32).contiguous()
-    ld = (N + 15) // 16 * 16
-    q = torch.empty(K, ld, dtype=torch.uint8, device=b.device)
-    scale = torch.empty(N, dtype=torch.float32, device=b.device)
-    scale_inv = torch.empty(N, dtype=torch.float32, device=b.device)
-    with torch.cuda.device(b.device):
-        _lib.check(lib.void_quant_cols(_lib.ptr(bf), bf.stride(0), K, N, _lib.KIND_F8E4M3, _lib.ptr(q), ld,
-                                       _lib.ptr(scale), _lib.ptr(scale_inv), _lib.stream_ptr(b.device)),
-                   "void_quant_cols")
-    return q.view(torch.float8_e4m3fn)[:, :N], scale, scale_inv
+    return _lib.native().quant_cols(b, _lib.KIND_F8E4M3)
 
 
 def quantize_to_fp8(tensor: torch.Tensor, config: Optional[FP8Config] = None,

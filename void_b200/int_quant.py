@@ -136,17 +136,8 @@ class Int8VOIDTensor:
 def quantize_cols_int8(b: torch.Tensor):
     """Per-column symmetric INT8 of a [K, N] matrix -> (int8 [K, N], float32 scales [N]).
     Same numbers as quantize_tensor(b.T, PER_CHANNEL) transposed back."""
-    _lib.require_cuda(b)
-    lib = _lib.load()
-    K, N = b.shape
-    bf = b.to(torch.float32).contiguous()
-    ld = (N + 15) // 16 * 16
-    q = torch.empty(K, ld, dtype=torch.int8, device=b.device)
-    scale = torch.empty(N, dtype=torch.float32, device=b.device)
-    with torch.cuda.device(b.device):
-        _lib.check(lib.void_quant_cols(_lib.ptr(bf), bf.stride(0), K, N, _lib.KIND_I8, _lib.ptr(q), ld, _lib.ptr(scale),
-                                       None, _lib.stream_ptr(b.device)), "void_quant_cols")
-    return q[:, :N], scale
+    q, scale, _ = _lib.native().quant_cols(b, _lib.KIND_I8)
+    return q, scale
 
 
 def _quantize_matrix_per_tensor(b: torch.Tensor):
