@@ -160,6 +160,17 @@ VOID_API int void_pack_tiles_fp(const void* values, int32_t elem_bytes, const in
                                 const int32_t* block_indices, int64_t nnz, void* packed,
                                 int32_t* tile_cols, void_stream_t stream);
 
+/* The packed tiles alone, for a structure whose tile_cols are known already and whose values change (a training step):
+ * as void_pack_tiles_fp, or with transposed = 1 the packed form of every tile's transpose, in the order of the
+ * transposed matrix's block_indices - what the product with A^T reads (void/autograd.py:178-191), with no transposed
+ * copy of the tiles in between. */
+VOID_API int void_repack_tiles_fp(const void* values, int32_t elem_bytes, const int32_t* block_indices,
+                                  int64_t nnz, int32_t transposed, void* packed, void_stream_t stream);
+/* Column sums of a row-major [rows, cols] matrix of type elem (VOID_ELEM_*), ld elements between rows, accumulated in
+ * fp32 in a fixed order, written in the same type: the gradient of a linear layer's bias. */
+VOID_API int void_column_sum(const void* in, int32_t elem, int64_t ld, int32_t rows, int32_t cols, void* out,
+                             void_stream_t stream);
+
 /* ---------------------------------------------------------------------------------------
  * Quantisers.
  * void_quant_i8_tiles: per-tile symmetric INT8, scale = max(absmax/128, 1e-8),
@@ -394,6 +405,15 @@ VOID_API int void_spmm_tile_grad(const void* grad_out, int64_t ldg, const void* 
                                  const int32_t* items, int32_t n_items, const int32_t* tile_cols,
                                  const int32_t* block_indices, void* grad_tiles,
                                  int32_t out_dtype, int32_t* status, void_stream_t stream);
+
+/* The same gradient for a linear layer y = x A^T: grad_out is dL/dy [N, M] and x is [N, K], both as the layer holds
+ * them (row-major, N the batch), so that the reduction index is the slow one and neither is transposed first
+ * (void/autograd.py:336 transposes both).  Other arguments as above; ldg / ldx in BYTES. */
+VOID_API int void_linear_tile_grad(const void* grad_out, int64_t ldg, const void* x, int64_t ldx,
+                                   int32_t M, int32_t K, int32_t N, int32_t kind,
+                                   const int32_t* items, int32_t n_items, const int32_t* tile_cols,
+                                   const int32_t* block_indices, void* grad_tiles,
+                                   int32_t out_dtype, int32_t* status, void_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------
  * void_spmm_i8 for callers that have no way to hand over scratch memory.  (This entry point has

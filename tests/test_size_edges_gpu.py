@@ -32,3 +32,31 @@ def test_quantised_columns_match_the_oracle_bits(k, n):
     off = torch.zeros(k, n + 3).cuda()[:, 1:n + 1]                        # rows that start off 16-byte boundaries
     off.copy_(b)
     assert torch.equal(void.quantize_cols_int8(off)[0], q)
+
+
+# ------------------------------------------------------------------------------------------ training
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,k,n", [(32, 32, 1), (64, 96, 31), (96, 160, 64), (200, 168, 65), (320, 264, 130), (40, 72, 515)])
+def test_linear_gradients_exact_on_small_integers(dtype, m, k, n):
+    gen = torch.Generator().manual_seed(m + k + n)
+    nbr, nbc = (m + 31) // 32, (k + 31) // 32
+    mask = torch.rand(nbr, nbc, generator=gen) < 0.6
+    mask[0, 0] = True
+    dense = torch.randint(-2, 3, (m, k), generator=gen).float() * mask.repeat_interleave(32, 0).repeat_interleave(32, 1)[:m, :k]
+    a = void.dense_to_void(dense.cuda()).to_dtype(dtype)
+    lin = void.SparseLinear(k, m, a, bias=True)
+    x = torch.randint(-2, 3, (n, k), generator=gen).cuda().to(dtype).requires_grad_(True)
+    gy = torch.randint(-1, 2, (n, m), generator=gen).cuda().to(dtype)
+    y = lin(x)
+    y.backward(gy)
+    void.check_device_status()
+    ref = a.to_dense().float().requires_grad_(True)
+    xr = x.detach().float().requires_grad_(True)
+    yr = xr @ ref.t()
+    yr.backward(gy.float())
+    assert torch.equal(y.float(), yr.to(dtype).float()) and torch.equal(x.grad.float(), xr.grad.to(dtype).float())
+    assert torch.equal(lin.bias.grad.float(), gy.float().sum(0).to(dtype).float())
+    grid = torch.zeros(nbr * 32, nbc * 32, device="cuda")
+    grid[:m, :k] = ref.grad
+    tiles = grid.reshape(nbr, 32, nbc, 32).permute(0, 2, 1, 3)[a.block_rows.long(), a.block_cols.long()]
+    assert torch.equal(lin.sparse_weight.values.grad.float(), tiles.to(dtype).float())

@@ -12,31 +12,45 @@ from typing import Any, Optional, Tuple
 import torch
 from torch.autograd import Function
 
-from . import _lib, _spmm, ops
+from . import _lib
 from .format import VOIDTensor
 
 
-# Tile index, backward work items and packed column list per sparsity structure.  The autograd function
-# only sees bare tensors, and a layer's structure stays fixed while its values train, so the derived
+# Index arrays per sparsity structure: tile index and column list of A and of A^T, work items of the tile gradient.  The
+# autograd functions only see bare tensors, and a layer's structure stays fixed while its values train, so the derived
 # arrays are kept here, keyed by the identity of the index tensors (a handful of layers; oldest dropped).
 _STRUCTURE = {}
 _STRUCTURE_MAX = 64
 
 
 def _structure(block_rows, block_cols, shape, n_blocks):
-    key = (block_rows.data_ptr(), block_cols.data_ptr(), block_rows._version, block_cols._version, tuple(shape),
-           n_blocks, str(block_rows.device))
+    """The native path's structure handle (csrc/host.cpp)."""
+    key = (block_rows.data_ptr(), block_cols.data_ptr(), block_rows._version, block_cols._version, shape[0], shape[1], n_blocks)
     hit = _STRUCTURE.get(key)
     if hit is None:
         from .format import build_tile_index
+        _lib.require_cuda(block_rows, block_cols)
         nbr, nbc = (shape[0] + 31) // 32, (shape[1] + 31) // 32
         row_ptr, block_indices = build_tile_index(block_rows, block_cols, nbr, nbc)
+        row_ptr_t, block_indices_t = build_tile_index(block_cols, block_rows, nbc, nbr)
         tile_cols = block_cols.to(torch.int32)[block_indices.long()].contiguous()
-        hit = (row_ptr, block_indices, tile_grad_items(row_ptr), tile_cols, block_rows, block_cols)  # keeps the keys alive
+        tile_cols_t = block_rows.to(torch.int32)[block_indices_t.long()].contiguous()
+        st = _lib.native().structure(row_ptr, block_indices, tile_cols, row_ptr_t, block_indices_t, tile_cols_t,
+                                     tile_grad_items(row_ptr), _lib.status_word(block_rows.device), shape[0], shape[1], n_blocks)
+        hit = (st, row_ptr, block_indices, block_rows, block_cols)     # keeps the keys alive
         if len(_STRUCTURE) >= _STRUCTURE_MAX:
-            _STRUCTURE.pop(next(iter(_STRUCTURE)))
+            _STRUCTURE.pop(next(iter(_STRUCTURE)), None)
         _STRUCTURE[key] = hit
     return hit
+
+
+def _require_operands(values, tile_size, dense):
+    _lib.require_cuda(values, dense)
+    if tuple(tile_size) != (32, 32):
+        raise NotImplementedError("void_b200 kernels are built for 32x32 tiles, got tile_size=%s" % (tile_size,))
+    if dense.dtype not in _lib.OUT_DTYPE_CODE or not values.dtype.is_floating_point:
+        raise _lib.VoidB200Error("the sparse product takes floating-point tiles and a float32, float16 or bfloat16 operand, "
+                                 "got %s and %s" % (values.dtype, dense.dtype))
 
 
 def _bare_void(values, block_rows, block_cols, shape, tile_size, n_blocks) -> VOIDTensor:
@@ -46,7 +60,7 @@ def _bare_void(values, block_rows, block_cols, shape, tile_size, n_blocks) -> VO
                    tile_size=tuple(tile_size), nnz_original=0, n_blocks=n_blocks, density=0.0, dtype=values.dtype)
     if values.is_cuda and tuple(tile_size) == (32, 32):
         st = _structure(block_rows, block_cols, shape, n_blocks)
-        v._row_ptr_cache, v._block_indices_cache = st[0], st[1]
+        v._row_ptr_cache, v._block_indices_cache = st[1], st[2]
     return v
 
 
@@ -77,89 +91,37 @@ def spmm_tile_grad(a: VOIDTensor, grad_output: torch.Tensor, b: torch.Tensor,
     M, K = a.shape
     N = b.shape[1]
     assert grad_output.shape == (M, N) and b.shape[0] == K
-    out_dtype = out_dtype or a.values.dtype
-    dev = b.device
-    grad = torch.zeros(a.n_blocks, 32, 32, dtype=out_dtype, device=dev)     # torch.zeros_like(a_values), :198
-    if a.n_blocks == 0 or N == 0:
-        return grad
-    dt = grad_output.dtype if (grad_output.dtype == b.dtype and b.dtype in (torch.float16, torch.bfloat16)) \
-        else torch.float32
-    kind = _lib.FP_KIND[dt]
-    g = _spmm.prepare_b(grad_output.to(dt), dt.itemsize)
-    bb = _spmm.prepare_b(b.to(dt), dt.itemsize)
-    _, block_indices, items, tile_cols = _structure(a.block_rows, a.block_cols, a.shape, a.n_blocks)[:4]
-    lib = _lib.load()
-    with torch.cuda.device(dev):
-        _lib.check(lib.void_spmm_tile_grad(_lib.ptr(g), g.stride(0) * dt.itemsize, _lib.ptr(bb), bb.stride(0) * dt.itemsize,
-                                           M, K, N, kind, _lib.ptr(items), items.shape[0], _lib.ptr(tile_cols),
-                                           _lib.ptr(block_indices), _lib.ptr(grad), _lib.OUT_DTYPE_CODE[out_dtype],
-                                           _lib.ptr(_lib.status_word(dev)), _lib.stream_ptr(dev)), "void_spmm_tile_grad")
-    return grad
+    st = _structure(a.block_rows, a.block_cols, a.shape, a.n_blocks)[0]
+    return _lib.native().tile_gradient(st, grad_output, b, False, out_dtype or a.values.dtype)
 
 
 class VOIDSpMMFunction(Function):
-    """C = A @ B with gradients for A's stored tiles and for B (void/autograd.py:99-221)."""
+    """C = A @ B with gradients for A's stored tiles and for B (void/autograd.py:99-221), both for one backward pass."""
 
     @staticmethod
-    def forward(ctx: Any, a_values, a_block_rows, a_block_cols, a_shape: Tuple[int, int], a_tile_size: Tuple[int, int],
-                a_n_blocks: int, b: torch.Tensor) -> torch.Tensor:
-        a = _bare_void(a_values.detach(), a_block_rows, a_block_cols, a_shape, a_tile_size, a_n_blocks)
-        c = ops.void_spmm(a, b.detach())
-        ctx.save_for_backward(a_values, a_block_rows, a_block_cols, b)
-        ctx.a_shape, ctx.a_tile_size, ctx.a_n_blocks = tuple(a_shape), tuple(a_tile_size), a_n_blocks
-        return c
-
-    @staticmethod
-    def backward(ctx: Any, grad_output: torch.Tensor):
-        a_values, a_block_rows, a_block_cols, b = ctx.saved_tensors
-        M, K = ctx.a_shape
-        grad_a_values = grad_b = None
-        grad_output = grad_output.contiguous()
-        if ctx.needs_input_grad[6]:
-            a_t = _bare_void(a_values.detach().permute(0, 2, 1).contiguous(), a_block_cols, a_block_rows, (K, M),
-                             ctx.a_tile_size[::-1], ctx.a_n_blocks)
-            grad_b = ops.void_spmm(a_t, grad_output.to(b.dtype)) if ctx.a_n_blocks else torch.zeros_like(b)
-        if ctx.needs_input_grad[0]:
-            a = _bare_void(a_values.detach(), a_block_rows, a_block_cols, ctx.a_shape, ctx.a_tile_size, ctx.a_n_blocks)
-            grad_a_values = spmm_tile_grad(a, grad_output, b.detach())
-        return grad_a_values, None, None, None, None, None, grad_b
+    def apply(a_values, a_block_rows, a_block_cols, a_shape: Tuple[int, int], a_tile_size: Tuple[int, int], a_n_blocks: int,
+              b: torch.Tensor) -> torch.Tensor:
+        _require_operands(a_values, a_tile_size, b)
+        assert b.dim() == 2 and a_shape[1] == b.shape[0], f"Dimension mismatch: A is {a_shape}, B is {tuple(b.shape)}"
+        st = _structure(a_block_rows, a_block_cols, a_shape, a_n_blocks)[0]
+        return _lib.native().values_product(st, a_values, b, False, None)
 
 
 class VOIDLinearFunction(Function):
     """y = x @ A^T (+ bias) for x [batch, in]: the linear layer on activations as they lie in memory
     (ops.void_linear), differentiable in A's stored tiles, x and the bias.
         dL/dx        = dL/dy @ A          - void_linear with the transposed tensor
-        dL/dA_values = (dL/dy)^T @ x      - for the stored tiles only (void_spmm_tile_grad; its operands need
-                                            the batch index contiguous, so dL/dy and x are transposed here)
+        dL/dA_values = (dL/dy)^T @ x      - for the stored tiles only (void_linear_tile_grad reads both as they lie)
         dL/dbias     = column sums of dL/dy
     The reference's SparseLinear computes (A @ x^T)^T through VOIDSpMMFunction and adds the bias as a
     separate op (void/autograd.py:320-344)."""
 
     @staticmethod
-    def forward(ctx: Any, a_values, a_block_rows, a_block_cols, a_shape, a_tile_size, a_n_blocks: int, x, bias):
-        a = _bare_void(a_values.detach(), a_block_rows, a_block_cols, a_shape, a_tile_size, a_n_blocks)
-        y = ops.void_linear(a, x.detach(), None if bias is None else bias.detach())
-        ctx.save_for_backward(a_values, a_block_rows, a_block_cols, x)
-        ctx.a_shape, ctx.a_tile_size, ctx.a_n_blocks = tuple(a_shape), tuple(a_tile_size), a_n_blocks
-        ctx.has_bias = bias is not None
-        return y
-
-    @staticmethod
-    def backward(ctx: Any, grad_output: torch.Tensor):
-        a_values, a_block_rows, a_block_cols, x = ctx.saved_tensors
-        M, K = ctx.a_shape
-        grad_output = grad_output.contiguous()
-        grad_a_values = grad_x = grad_bias = None
-        if ctx.needs_input_grad[6]:
-            a_t = _bare_void(a_values.detach().permute(0, 2, 1).contiguous(), a_block_cols, a_block_rows, (K, M),
-                             ctx.a_tile_size[::-1], ctx.a_n_blocks)
-            grad_x = ops.void_linear(a_t, grad_output.to(x.dtype)) if ctx.a_n_blocks else torch.zeros_like(x)
-        if ctx.needs_input_grad[0]:
-            a = _bare_void(a_values.detach(), a_block_rows, a_block_cols, ctx.a_shape, ctx.a_tile_size, ctx.a_n_blocks)
-            grad_a_values = spmm_tile_grad(a, grad_output.T.contiguous(), x.detach().T.contiguous())
-        if ctx.has_bias and ctx.needs_input_grad[7]:
-            grad_bias = grad_output.sum(0)
-        return grad_a_values, None, None, None, None, None, grad_x, grad_bias
+    def apply(a_values, a_block_rows, a_block_cols, a_shape, a_tile_size, a_n_blocks: int, x, bias):
+        _require_operands(a_values, a_tile_size, x)
+        assert x.dim() == 2 and x.shape[1] == a_shape[1], f"Dimension mismatch: A is {a_shape}, x is {tuple(x.shape)}"
+        st = _structure(a_block_rows, a_block_cols, a_shape, a_n_blocks)[0]
+        return _lib.native().values_product(st, a_values, x, True, bias)
 
 
 class VOIDSpMM(torch.nn.Module):
@@ -203,12 +165,11 @@ class SparseLinear(torch.nn.Module):
             self.register_parameter("bias", None)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        input_shape = x.shape
-        x_flat = x.reshape(-1, self.in_features)
         w = self.sparse_weight
-        y = VOIDLinearFunction.apply(w.values, w.block_rows, w.block_cols, w.shape, w.tile_size, w.n_blocks, x_flat,
-                                     self.bias)
-        return y.reshape(input_shape[:-1] + (self.out_features,))
+        flat = x.dim() == 2 and x.shape[1] == self.in_features      # no views (and none in the backward pass) needed
+        y = VOIDLinearFunction.apply(w.values, w.block_rows, w.block_cols, w.shape, w.tile_size, w.n_blocks,
+                                     x if flat else x.reshape(-1, self.in_features), self.bias)
+        return y if flat else y.reshape(x.shape[:-1] + (self.out_features,))
 
     def extra_repr(self) -> str:
         return f"in_features={self.in_features}, out_features={self.out_features}, bias={self.bias is not None}"

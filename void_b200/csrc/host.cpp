@@ -10,8 +10,13 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
 
+#include <memory>
+#include <mutex>
 #include <string>
 
 #include "../../include/void_b200.h"
@@ -339,6 +344,201 @@ PyObject* quant_cols(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_END
 }
 
+// ------------------------------------------------------------------------------------------ training
+// The index arrays of one sparsity structure, both ways round; they outlive the values that train over them.
+struct Structure {
+  at::Tensor row_ptr[2], block_indices[2], tile_cols[2];   // of A, of A^T
+  at::Tensor items, status;
+  int64_t M = 0, K = 0, nnz = 0;
+};
+struct StructureObject {
+  PyObject_HEAD
+  std::shared_ptr<const Structure> st;
+};
+PyTypeObject* g_structure_type = nullptr;
+
+// structure(row_ptr, block_indices, tile_cols, row_ptr_t, block_indices_t, tile_cols_t, items, status, M, K, n_blocks)
+PyObject* structure(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 11) throw torch::TypeError("structure takes 11 arguments");
+  auto st = std::make_shared<Structure>();
+  for (int i = 0; i < 2; ++i) {
+    st->row_ptr[i] = cuda_tensor(a[3 * i], "row_ptr");
+    st->block_indices[i] = cuda_tensor(a[3 * i + 1], "block_indices");
+    st->tile_cols[i] = cuda_tensor(a[3 * i + 2], "tile_cols");
+  }
+  st->items = cuda_tensor(a[6], "items");
+  st->status = cuda_tensor(a[7], "status");
+  st->M = integer(a[8]);
+  st->K = integer(a[9]);
+  st->nnz = integer(a[10]);
+  PyObject* self = PyType_GenericAlloc(g_structure_type, 0);
+  if (self == nullptr) return nullptr;
+  new (&reinterpret_cast<StructureObject*>(self)->st) std::shared_ptr<const Structure>(std::move(st));
+  return self;
+  NATIVE_END
+}
+std::shared_ptr<const Structure> structure_of(PyObject* o) {
+  if (Py_TYPE(o) != g_structure_type) throw torch::TypeError("expected a structure handle");
+  return reinterpret_cast<StructureObject*>(o)->st;
+}
+int common_kind(at::ScalarType a, at::ScalarType b) {   // their common 16-bit type, else fp32 operands (TF32)
+  if (a == b && a == at::kHalf) return VOID_KIND_F16;
+  if (a == b && a == at::kBFloat16) return VOID_KIND_BF16;
+  return VOID_KIND_TF32;
+}
+at::ScalarType kind_type(int kind) { return kind == VOID_KIND_F16 ? at::kHalf : (kind == VOID_KIND_BF16 ? at::kBFloat16 : at::kFloat); }
+at::Tensor as_type(const at::Tensor& t, at::ScalarType type) { return t.scalar_type() == type ? t : t.to(type); }
+
+// Product with tiles that change from call to call: they are packed (their transposes for A^T) and multiplied at once.
+// linear: b is x [N, K] and the result x A^T [N, M]; otherwise b is [K, N] and the result A b [M, N].
+at::Tensor product_of_values(const Structure& st, bool a_transposed, const at::Tensor& values_in, const at::Tensor& b_in,
+                             bool linear, const at::Tensor* row_bias) {
+  const c10::Device dev = b_in.device();
+  const int kind = common_kind(values_in.scalar_type(), b_in.scalar_type());
+  const int es = elem_bytes(kind);
+  const at::Tensor values = as_type(values_in, kind_type(kind)).contiguous();
+  const at::Tensor b = kernel_operand(as_type(b_in, kind_type(kind)), es);
+  const int64_t M = a_transposed ? st.K : st.M, K = a_transposed ? st.M : st.K;
+  const int64_t N = b.size(linear ? 0 : 1);
+  if (b.size(linear ? 1 : 0) != K) fail("shape mismatch between the sparse matrix and the dense operand");
+  at::Tensor out = new_cuda({linear ? N : M, linear ? M : N}, b_in.scalar_type(), dev);
+  at::Tensor store = new_cuda({std::max<int64_t>(st.nnz, 1) * 1024 * es + 1024}, at::kByte, dev);
+  uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(store.data_ptr()) + 1023) & ~uintptr_t(1023));
+  const void_stream_t stream = stream_of(dev.index());
+  const int way = a_transposed ? 1 : 0;
+  check(void_repack_tiles_fp(values.const_data_ptr(), es, st.block_indices[way].const_data_ptr<int32_t>(), st.nnz, way, tiles, stream),
+        "void_repack_tiles_fp");
+  void_spmm_args s = void_spmm_args();
+  s.tiles = tiles;
+  s.tile_cols = st.tile_cols[way].const_data_ptr<int32_t>();
+  s.row_ptr = st.row_ptr[way].const_data_ptr<int32_t>();
+  s.nbr = (int32_t)((M + 31) / 32);
+  s.nbc = (int32_t)((K + 31) / 32);
+  s.nnz = st.nnz;
+  s.b = b.const_data_ptr();
+  s.ldb = b.stride(0) * es;
+  s.K = (int32_t)K;
+  s.N = (int32_t)N;
+  s.b_scale = 1.0f;
+  at::Tensor bias;
+  if (row_bias != nullptr) {
+    bias = row_bias->to(dev, at::kFloat).contiguous();
+    if (bias.numel() != M) fail("row bias must have " + std::to_string(M) + " elements, got " + std::to_string(bias.numel()));
+    s.row_bias = bias.const_data_ptr<float>();
+  }
+  s.out = out.data_ptr();
+  s.ldc = out.stride(0);
+  s.M = (int32_t)M;
+  s.out_dtype = out_code(out.scalar_type());
+  s.scale_mode = VOID_SCALE_ROW_MEAN;
+  s.status = st.status.data_ptr<int32_t>();
+  s.transposed = linear ? 1 : 0;
+  check(void_spmm_fp(&s, kind, stream), "void_spmm_fp");
+  return out;
+}
+
+// dL/dA for the stored tiles; linear: g [N, M], x [N, K], otherwise g [M, N], x [K, N]
+at::Tensor gradient_of_values(const Structure& st, const at::Tensor& g_in, const at::Tensor& x_in, at::ScalarType type, bool linear) {
+  const c10::Device dev = x_in.device();
+  const int64_t N = x_in.size(linear ? 0 : 1);
+  if (st.nnz == 0 || N == 0) return at::zeros({st.nnz, 32, 32}, x_in.options().dtype(type));
+  const int kind = common_kind(g_in.scalar_type(), x_in.scalar_type());
+  const int es = elem_bytes(kind);
+  const at::Tensor g = kernel_operand(as_type(g_in, kind_type(kind)), es);
+  const at::Tensor x = kernel_operand(as_type(x_in, kind_type(kind)), es);
+  at::Tensor grad = new_cuda({st.nnz, 32, 32}, type, dev);   // every stored tile is written
+  check((linear ? void_linear_tile_grad : void_spmm_tile_grad)(
+            g.const_data_ptr(), g.stride(0) * es, x.const_data_ptr(), x.stride(0) * es, (int32_t)st.M, (int32_t)st.K, (int32_t)N,
+            kind, st.items.const_data_ptr<int32_t>(), (int32_t)st.items.size(0), st.tile_cols[0].const_data_ptr<int32_t>(),
+            st.block_indices[0].const_data_ptr<int32_t>(), grad.data_ptr(), out_code(type), st.status.data_ptr<int32_t>(),
+            stream_of(dev.index())),
+        "void_spmm_tile_grad");
+  return grad;
+}
+
+at::Tensor column_sums(const at::Tensor& m) {
+  at::Tensor out = new_cuda({m.size(1)}, m.scalar_type(), m.device());
+  check(void_column_sum(m.const_data_ptr(), out_code(m.scalar_type()), std::max<int64_t>(m.stride(0), m.size(1)), (int32_t)m.size(0),
+                        (int32_t)m.size(1), out.data_ptr(), stream_of(m.device().index())),
+        "void_column_sum");
+  return out;
+}
+
+// The gradients of A b (or of x A^T + bias): an autograd node of its own, so that a backward pass runs in the engine's
+// thread without taking the interpreter's lock.
+struct ProductBackward : torch::autograd::Node {
+  torch::autograd::SavedVariable values, dense;
+  std::shared_ptr<const Structure> st;
+  bool linear = false;
+
+  std::string name() const override { return "VOIDProductBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    values.reset_data();
+    dense.reset_data();
+  }
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    at::AutoDispatchBelowADInplaceOrView below;
+    torch::autograd::variable_list out(3);
+    if (!grads[0].defined()) return out;
+    const at::Tensor v = values.unpack(), b = dense.unpack(), g = grads[0].contiguous();
+    c10::cuda::OptionalCUDAGuard guard(b.device());
+    try {
+      if (task_should_compute_output(1))
+        out[1] = st->nnz ? product_of_values(*st, true, v, as_type(g, b.scalar_type()), linear, nullptr) : at::zeros_like(b);
+      if (task_should_compute_output(0)) out[0] = gradient_of_values(*st, g, b, v.scalar_type(), linear);
+      if (task_should_compute_output(2)) out[2] = column_sums(g);
+    } catch (const Failure& f) {
+      TORCH_CHECK(false, f.text);
+    }
+    return out;
+  }
+};
+
+// values_product(structure, values, b, linear, bias | None) -> A b, or x A^T + bias; differentiable in all three
+PyObject* values_product(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 5) throw torch::TypeError("values_product takes 5 arguments");
+  std::shared_ptr<const Structure> st = structure_of(a[0]);
+  const at::Tensor& values = cuda_tensor(a[1], "values");
+  const at::Tensor& b = cuda_tensor(a[2], "the dense operand");
+  c10::cuda::OptionalCUDAGuard guard(b.device());
+  const bool linear = PyObject_IsTrue(a[3]) == 1;
+  const at::Tensor none_given;
+  const at::Tensor& bias = none(a[4]) ? none_given : tensor(a[4], "bias");
+  at::Tensor out;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    out = product_of_values(*st, false, values, b, linear, bias.defined() ? &bias : nullptr);
+  }
+  if (torch::autograd::compute_requires_grad(values, b, bias)) {
+    auto node = std::shared_ptr<ProductBackward>(new ProductBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(values, b, bias));
+    node->values = torch::autograd::SavedVariable(values, false);
+    node->dense = torch::autograd::SavedVariable(b, false);
+    node->st = std::move(st);
+    node->linear = linear;
+    torch::autograd::set_history(out, node);
+  }
+  return THPVariable_Wrap(out);
+  NATIVE_END
+}
+
+// tile_gradient(structure, grad, b, linear, dtype) -> dL/dA_values
+PyObject* tile_gradient(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 5) throw torch::TypeError("tile_gradient takes 5 arguments");
+  const std::shared_ptr<const Structure> st = structure_of(a[0]);
+  const at::Tensor& b = cuda_tensor(a[2], "the dense operand");
+  c10::cuda::OptionalCUDAGuard guard(b.device());
+  at::AutoDispatchBelowADInplaceOrView below;
+  return THPVariable_Wrap(gradient_of_values(*st, cuda_tensor(a[1], "the gradient"), b, reinterpret_cast<THPDtype*>(a[4])->scalar_type,
+                                             PyObject_IsTrue(a[3]) == 1));
+  NATIVE_END
+}
+
 PyObject* set_error(PyObject*, PyObject* cls) {
   Py_INCREF(cls);
   g_error = cls;
@@ -353,6 +553,9 @@ PyMethodDef kMethods[] = {
     FAST(packed_is_current),
     FAST(spmm),
     FAST(quant_cols),
+    FAST(structure),
+    FAST(values_product),
+    FAST(tile_gradient),
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
@@ -362,6 +565,14 @@ void packed_dealloc(PyObject* self) {
   type->tp_free(self);
   Py_DECREF(type);
 }
+void structure_dealloc(PyObject* self) {
+  PyTypeObject* type = Py_TYPE(self);
+  reinterpret_cast<StructureObject*>(self)->st.~shared_ptr();
+  type->tp_free(self);
+  Py_DECREF(type);
+}
+PyType_Slot kStructureSlots[] = {{Py_tp_dealloc, (void*)structure_dealloc}, {0, nullptr}};
+PyType_Spec kStructureSpec = {"_native.Structure", (int)sizeof(StructureObject), 0, Py_TPFLAGS_DEFAULT, kStructureSlots};
 PyType_Slot kPackedSlots[] = {{Py_tp_dealloc, (void*)packed_dealloc}, {0, nullptr}};
 PyType_Spec kPackedSpec = {"_native.Packed", (int)sizeof(PackedObject), 0, Py_TPFLAGS_DEFAULT, kPackedSlots};
 
@@ -369,6 +580,7 @@ PyType_Spec kPackedSpec = {"_native.Packed", (int)sizeof(PackedObject), 0, Py_TP
 
 PyMODINIT_FUNC PyInit__native(void) {
   g_packed_type = reinterpret_cast<PyTypeObject*>(PyType_FromSpec(&kPackedSpec));
-  if (g_packed_type == nullptr) return nullptr;
+  g_structure_type = reinterpret_cast<PyTypeObject*>(PyType_FromSpec(&kStructureSpec));
+  if (g_packed_type == nullptr || g_structure_type == nullptr) return nullptr;
   return PyModule_Create(&kModule);
 }

@@ -17,6 +17,12 @@
 // memory) is read back by four warps, warp j holding tile j: lane k, column m = dA_tile_j[m][k], so
 // every store instruction writes 32 consecutive elements of one tile row.
 //
+// The linear-layer form (MN = true, void_linear_tile_grad) takes dL/dy [N, M] and x [N, K] as the layer holds them: n is
+// now the slow index, so both operands are MN-major.  A row block is 32 columns of one matrix and 128 / ES rows of n
+// (4 KB, the swizzle span is the 32 columns: 128 bytes with 32-byte atoms for fp32, 64 bytes for 16-bit types); the four
+// tiles' blocks stand side by side along M, and an MMA takes 1024 bytes further along n each time.  It replaces two
+// transposed copies of 8 MB at 4096^2, N = 512 fp32 (20 us).
+//
 // Work items (tile row, first tile, tile count <= 4) come from the caller (they depend on A's
 // structure only).  Every wait is bounded like in the SpMM kernels.
 #include <cuda_bf16.h>
@@ -46,8 +52,8 @@ struct GradParams {
   void* grad;                    // [nnz][32][32] in the caller's order
   int32_t* status;
   int n_items;
-  int n_slices;                  // ceil(N * element bytes / 128)
-  int slice_elems;               // elements per 128 bytes
+  int n_slices;                  // slices of n: 128 bytes of it (K-major), 128 / element bytes rows of it (MN-major)
+  int slice_elems;               // n per slice
   int out_dtype;
   unsigned long long desc_hi;
   unsigned int idesc;
@@ -66,7 +72,7 @@ __device__ __forceinline__ void issue(uint32_t d, uint64_t a, uint64_t b, uint32
   else mma_f16(d, a, b, idesc, acc);
 }
 
-template <int KIND>
+template <int KIND, bool MN>
 __global__ void __launch_bounds__(kThreads, 2) tile_grad_kernel(const __grid_constant__ CUtensorMap tmap_b,
                                                                 const __grid_constant__ CUtensorMap tmap_g,
                                                                 const __grid_constant__ GradParams p) {
@@ -128,7 +134,9 @@ __global__ void __launch_bounds__(kThreads, 2) tile_grad_kernel(const __grid_con
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) { alive = false; break; }
-        if (mine) tma_load_2d(base + (uint32_t)lane * kBlockBytes, lane == 4 ? &tmap_g : &tmap_b, s * p.slice_elems, y, full);
+        if (mine)
+          tma_load_2d(base + (uint32_t)lane * kBlockBytes, lane == 4 ? &tmap_g : &tmap_b, MN ? y : s * p.slice_elems,
+                      MN ? s * p.slice_elems : y, full);
       }
     }
   } else if (warp == 1) {
@@ -156,8 +164,9 @@ __global__ void __launch_bounds__(kThreads, 2) tile_grad_kernel(const __grid_con
           const uint32_t base = ring + (uint32_t)stage * kStageBytes;
           const uint64_t ad = smem_desc(hi, base), bd = smem_desc(hi, base + 4u * kBlockBytes);
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {  // 32 bytes of n per MMA: the start address moves inside the swizzle atom
-            if (leader) issue<KIND>(d, ad + 2u * kk, bd + 2u * kk, idesc, acc);
+          for (int kk = 0; kk < 4; ++kk) {  // 32 bytes of n per MMA (inside the swizzle atom), or 1024 bytes of its rows
+            constexpr uint64_t kStep = MN ? (1024u >> 4) : 2u;
+            if (leader) issue<KIND>(d, ad + kStep * kk, bd + kStep * kk, idesc, acc);
             acc = 1u;
           }
           if (leader) tc_commit(smem_u32(&bars.empty[stage]));
@@ -242,27 +251,36 @@ static PFN_cuTensorMapEncodeTiled_v12000 encoder() {
   return fn;
 }
 
-// [rows, N] row-major matrix as a tensor of 128-byte-wide, 32-row boxes with the 128-byte swizzle.
-static bool row_block_map(CUtensorMap* m, const void* base, int64_t ld_bytes, int rows, int N, int es) {
+// A row-major matrix [rows, cols] as a tensor of 4 KB boxes: 32 rows of 128 bytes (K-major form), or 128 / es rows of 32
+// columns (MN-major form).
+static bool row_block_map(CUtensorMap* m, const void* base, int64_t ld_bytes, int rows, int cols, int es, bool mn) {
   PFN_cuTensorMapEncodeTiled_v12000 enc = encoder();
   if (enc == nullptr) return false;
   const CUtensorMapDataType dt = (es == 2) ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT32;
-  const cuuint64_t gdim[2] = {(cuuint64_t)N, (cuuint64_t)rows};
+  const cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   const cuuint64_t gstride[1] = {(cuuint64_t)ld_bytes};
-  const cuuint32_t box[2] = {(cuuint32_t)(128 / es), (cuuint32_t)kTile};
+  const cuuint32_t box[2] = {(cuuint32_t)(mn ? kTile : 128 / es), (cuuint32_t)(mn ? 128 / es : kTile)};
   const cuuint32_t estride[2] = {1, 1};
-  return enc(m, dt, 2, const_cast<void*>(base), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  const CUtensorMapSwizzle swz = !mn ? CU_TENSOR_MAP_SWIZZLE_128B
+                                     : (es == 4 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_64B);
+  return enc(m, dt, 2, const_cast<void*>(base), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-}  // namespace vbg
+template <int KIND, bool MN>
+static int launch(const GradParams& p, const CUtensorMap& map_b, const CUtensorMap& map_g, int sms, cudaStream_t st) {
+  auto kernel = tile_grad_kernel<KIND, MN>;
+  const int smem = kStages * kStageBytes + 1024;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return VOID_ERR_CUDA;
+  int grid = 2 * sms;
+  if (grid > p.n_items) grid = p.n_items;
+  kernel<<<grid, kThreads, smem, st>>>(map_b, map_g, p);
+  return cudaGetLastError() == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
+}
 
-extern "C" int void_spmm_tile_grad(const void* grad_out, int64_t ldg, const void* b, int64_t ldb, int32_t M, int32_t K,
-                                   int32_t N, int32_t kind, const int32_t* items, int32_t n_items,
-                                   const int32_t* tile_cols, const int32_t* block_indices, void* grad_tiles,
-                                   int32_t out_dtype, int32_t* status, void_stream_t stream) {
-  using namespace vbg;
+static int tile_grad(const void* grad_out, int64_t ldg, const void* b, int64_t ldb, int M, int K, int N, int kind,
+                     const int32_t* items, int n_items, const int32_t* tile_cols, const int32_t* block_indices,
+                     void* grad_tiles, int out_dtype, int32_t* status, cudaStream_t st, bool mn) {
   if (M < 0 || K < 0 || N < 0 || n_items < 0) return VOID_ERR_BAD_ARG;
   if (kind != VOID_KIND_TF32 && kind != VOID_KIND_F16 && kind != VOID_KIND_BF16) return VOID_ERR_BAD_ARG;
   if (out_dtype < VOID_OUT_F32 || out_dtype > VOID_OUT_BF16) return VOID_ERR_BAD_ARG;
@@ -272,7 +290,7 @@ extern "C" int void_spmm_tile_grad(const void* grad_out, int64_t ldg, const void
   if (N > 0) {
     if (grad_out == nullptr || b == nullptr) return VOID_ERR_BAD_ARG;
     if ((reinterpret_cast<uintptr_t>(grad_out) & 15u) || (reinterpret_cast<uintptr_t>(b) & 15u) || (ldg & 15) || (ldb & 15) ||
-        ldg < (int64_t)N * es || ldb < (int64_t)N * es)
+        ldg < (int64_t)(mn ? M : N) * es || ldb < (int64_t)(mn ? K : N) * es)
       return VOID_ERR_ALIGN;
   }
   int dev = 0, cc = 0, sms = 0;
@@ -291,34 +309,41 @@ extern "C" int void_spmm_tile_grad(const void* grad_out, int64_t ldg, const void
   p.slice_elems = 128 / es;
   p.n_slices = (N + p.slice_elems - 1) / p.slice_elems;
   p.out_dtype = out_dtype;
-  // K-major operands with the 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart
-  p.desc_hi = smem_desc_hi(16, 1024, kLayoutSw128);
+  // K-major: rows of 128 bytes, groups of 8 rows 1024 bytes apart.  MN-major: the tiles' blocks 4096 bytes apart along M,
+  // groups of 4 (fp32, 128-byte rows) or 8 (16-bit, 64-byte rows) rows of n 512 bytes apart.
+  p.desc_hi = mn ? smem_desc_hi(kBlockBytes, 512, es == 4 ? kLayoutSw128Base32 : kLayoutSw64) : smem_desc_hi(16, 1024, kLayoutSw128);
   const uint32_t fmt = (kind == VOID_KIND_TF32) ? 2u : (kind == VOID_KIND_BF16 ? 1u : 0u);
-  p.idesc = instr_desc(/*c f32*/ 1, fmt, fmt, /*a K-major*/ 0, /*b K-major*/ 0, 128, 32);
+  p.idesc = instr_desc(/*c f32*/ 1, fmt, fmt, mn ? 1 : 0, mn ? 1 : 0, 128, 32);
 
   CUtensorMap map_b, map_g;
   memset(&map_b, 0, sizeof(map_b));
   memset(&map_g, 0, sizeof(map_g));
   if (N > 0) {
-    if (!row_block_map(&map_b, b, ldb, K, N, es) || !row_block_map(&map_g, grad_out, ldg, M, N, es))
+    if (!row_block_map(&map_b, b, ldb, mn ? N : K, mn ? K : N, es, mn) || !row_block_map(&map_g, grad_out, ldg, mn ? N : M, mn ? M : N, es, mn))
       return VOID_ERR_TENSOR_MAP;
   }
-  const int smem = kStages * kStageBytes + 1024;
-  int grid = 2 * sms;
-  if (grid > n_items) grid = n_items;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  static std::mutex mu;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (kind == VOID_KIND_TF32) {
-      if (cudaFuncSetAttribute(tile_grad_kernel<VOID_KIND_TF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return VOID_ERR_CUDA;
-    } else {
-      if (cudaFuncSetAttribute(tile_grad_kernel<VOID_KIND_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return VOID_ERR_CUDA;
-    }
-  }
-  if (kind == VOID_KIND_TF32) tile_grad_kernel<VOID_KIND_TF32><<<grid, kThreads, smem, st>>>(map_b, map_g, p);
-  else tile_grad_kernel<VOID_KIND_F16><<<grid, kThreads, smem, st>>>(map_b, map_g, p);
-  return cudaGetLastError() == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
+  if (kind == VOID_KIND_TF32) return mn ? launch<VOID_KIND_TF32, true>(p, map_b, map_g, sms, st) : launch<VOID_KIND_TF32, false>(p, map_b, map_g, sms, st);
+  return mn ? launch<VOID_KIND_F16, true>(p, map_b, map_g, sms, st) : launch<VOID_KIND_F16, false>(p, map_b, map_g, sms, st);
 }
+
+}  // namespace vbg
+
+extern "C" {
+
+int void_spmm_tile_grad(const void* grad_out, int64_t ldg, const void* b, int64_t ldb, int32_t M, int32_t K, int32_t N,
+                        int32_t kind, const int32_t* items, int32_t n_items, const int32_t* tile_cols,
+                        const int32_t* block_indices, void* grad_tiles, int32_t out_dtype, int32_t* status,
+                        void_stream_t stream) {
+  return vbg::tile_grad(grad_out, ldg, b, ldb, M, K, N, kind, items, n_items, tile_cols, block_indices, grad_tiles, out_dtype,
+                        status, reinterpret_cast<cudaStream_t>(stream), false);
+}
+
+int void_linear_tile_grad(const void* grad_out, int64_t ldg, const void* x, int64_t ldx, int32_t M, int32_t K, int32_t N,
+                          int32_t kind, const int32_t* items, int32_t n_items, const int32_t* tile_cols,
+                          const int32_t* block_indices, void* grad_tiles, int32_t out_dtype, int32_t* status,
+                          void_stream_t stream) {
+  return vbg::tile_grad(grad_out, ldg, x, ldx, M, K, N, kind, items, n_items, tile_cols, block_indices, grad_tiles, out_dtype,
+                        status, reinterpret_cast<cudaStream_t>(stream), true);
+}
+
+}  // extern "C"

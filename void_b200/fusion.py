@@ -113,11 +113,9 @@ def fused_sparse_mlp(x: torch.Tensor, w1: VOIDTensor, w2: VOIDTensor, activation
     code = get_activation_code(activation)
     if code > _lib.ACT_SILU:
         raise NotImplementedError("activation %r is not fused on B200 (none, relu, gelu, silu are)" % activation)
-    input_shape = x.shape
-    x_2d = x.reshape(-1, x.shape[-1])
-    hidden = void_linear(w1, x_2d, bias1, code)
+    hidden = void_linear(w1, x if x.dim() == 2 else x.reshape(-1, x.shape[-1]), bias1, code)
     out = void_linear(w2, hidden, bias2, 0)
-    return out.reshape(input_shape[:-1] + (out.shape[-1],))
+    return out if x.dim() == 2 else out.reshape(x.shape[:-1] + (out.shape[-1],))
 
 
 @dataclass
