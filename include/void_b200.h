@@ -95,7 +95,7 @@ VOID_API int void_build_tile_index(const int32_t* block_rows, const int32_t* blo
  *        16384 tiles along a side), shared by the calls of one conversion.
  *   1. void_dense_mark: a tile is kept when the sum of |x| over it exceeds threshold (:391-394);
  *      elem = VOID_ELEM_*; or void_csr_mark: a tile is kept when the CSR matrix stores an entry
- *      in it, zero or not (:287-296).  counts[2] (device, int64) receives the number of kept
+ *      in it, zero or not (:287-296).  counts[2] (int64; device memory or pinned host memory) receives the number of kept
  *      tiles and, for the dense form, the number of nonzero elements (nnz_original, :429).
  *   2. the caller reads counts[0], allocates, and calls void_morton_emit: block_rows,
  *      block_cols, morton_codes [n_blocks] in ascending Morton order.
@@ -129,7 +129,10 @@ VOID_API int void_csr_scatter(const int32_t* crow, const int32_t* col, const flo
  * reference's avg_scale for b_scale = 1, void/int_quant.py:516-526.  scales may hold one
  * value for all tiles (n_scales == 1, per-tensor mode).
  * packed must be 1024-byte aligned and hold nnz*1024 bytes.
+ * void_row_order: the tile rows by falling tile count (ties in their own order), for void_spmm_args.row_order.
+ * Its work grows with nbr * nbr / 32 per warp: meant for up to a few thousand tile rows.
  * ------------------------------------------------------------------------------------- */
+VOID_API int void_row_order(const int32_t* row_ptr, int32_t nbr, int32_t* order, void_stream_t stream);
 VOID_API int void_pack_tiles(const void* values, const float* scales, int64_t n_scales,
                     const int32_t* block_cols, const int32_t* block_indices,
                     const int32_t* row_ptr, int64_t nnz, int32_t nbr, void* packed,
@@ -184,6 +187,12 @@ VOID_API int void_column_sum(const void* in, int32_t elem, int64_t ld, int32_t r
  *   quantize_tensor(B.T, PER_CHANNEL), void/int_quant.py:273-274, and
  *   quantize_to_fp8(B.T, per_row), void/fp8.py:177-180.  q is [K, ldq] bytes.
  * ------------------------------------------------------------------------------------- */
+/* void_quant_tiles: both of the above for tiles of type elem (VOID_ELEM_*; read in that type), kind = VOID_KIND_I8 or
+ * VOID_KIND_F8E4M3.  scale_inv, amax, zero_points (zeros) and the copies rows_out / cols_out of the tile coordinates are
+ * written where not NULL, so that a quantised tensor is one launch. */
+VOID_API int void_quant_tiles(const void* values, int32_t elem, int64_t nnz, int32_t kind, void* q, float* scale,
+                              float* scale_inv, float* amax, int8_t* zero_points, const int32_t* block_rows,
+                              const int32_t* block_cols, int32_t* rows_out, int32_t* cols_out, void_stream_t stream);
 VOID_API int void_quant_i8_tiles(const float* values, int64_t nnz, int8_t* q, float* scales,
                         void_stream_t stream);
 VOID_API int void_quant_fp8_tiles(const float* values, int64_t nnz, uint8_t* q, float* scale,

@@ -60,3 +60,55 @@ def test_linear_gradients_exact_on_small_integers(dtype, m, k, n):
     grid[:m, :k] = ref.grad
     tiles = grid.reshape(nbr, 32, nbc, 32).permute(0, 2, 1, 3)[a.block_rows.long(), a.block_cols.long()]
     assert torch.equal(lin.sparse_weight.values.grad.float(), tiles.to(dtype).float())
+
+
+# ------------------------------------------------------------------------------------------ format and set-up
+@pytest.mark.parametrize("m,n,off,dtype,threshold", [
+    (1, 1, 0, torch.float32, 0.0), (31, 33, 0, torch.float32, 0.0), (64, 126, 1, torch.float32, 0.0),
+    (100, 130, 0, torch.float16, 2.0), (65, 257, 0, torch.bfloat16, 0.0), (33, 264, 1, torch.bfloat16, 1.5),
+    (64, 256, 0, torch.float32, -1.0), (32, 32800, 0, torch.float16, 0.0)])
+def test_dense_to_void_widths_and_alignments(m, n, off, dtype, threshold):
+    gen = torch.Generator().manual_seed(m * 7 + n)
+    full = (torch.randn(m, n, generator=gen) * (torch.rand(m, n, generator=gen) < 0.01)).to(dtype)
+    wide = torch.zeros(m, n + off, dtype=dtype, device="cuda")
+    wide[:, off:] = full.cuda()
+    v = void.dense_to_void(wide[:, off:], threshold=threshold)
+    f = vo.dense_to_void_fields(full.float().numpy(), threshold=threshold)
+    assert v.n_blocks == f["n_blocks"] and v.nnz_original == f["nnz_original"]
+    for name in ("block_rows", "block_cols", "morton_codes"):
+        assert np.array_equal(getattr(v, name).cpu().numpy(), f[name])
+    assert np.array_equal(v.values.float().cpu().numpy(), f["values"])
+
+
+@pytest.mark.parametrize("nbr,nbc", [(1, 1), (1, 70), (1023, 33), (1025, 2), (4096, 3), (4097, 3), (600, 2100)])
+def test_packed_store_of_grids_of_every_size(nbr, nbc):
+    gen = torch.Generator().manual_seed(nbr + nbc)
+    mask = (torch.rand(nbr, nbc, generator=gen) < min(0.4, 3000 / (nbr * nbc))).numpy()
+    mask[0, nbc - 1] = True
+    rows, cols = np.nonzero(mask)
+    perm = np.random.default_rng(0).permutation(len(rows))
+    rows, cols = rows[perm].astype(np.int32), cols[perm].astype(np.int32)
+    a = void.VOIDTensor(torch.randn(len(rows), 32, 32).cuda().half(), torch.from_numpy(rows).cuda(), torch.from_numpy(cols).cuda(),
+                        torch.zeros(len(rows), dtype=torch.int64, device="cuda"), (nbr * 32, nbc * 32), (32, 32), 0, len(rows), 0.0)
+    q = void.quantize_void_tensor(a)                                     # 16-bit tiles are quantised as they are
+    ref_q, ref_s = vo.quantize_int8_tiles(a.values.float().cpu().numpy())
+    assert np.array_equal(q.values.cpu().numpy(), ref_q) and np.array_equal(q.scales.cpu().numpy(), ref_s)
+    assert torch.equal(q.block_rows, a.block_rows) and q.block_rows.data_ptr() != a.block_rows.data_ptr()
+    p = q.packed()
+    ref_rp, ref_bi = vo.row_block_info(rows, cols, nbr, nbc)
+    assert np.array_equal(p.row_ptr.cpu().numpy(), ref_rp) and np.array_equal(p.block_indices.cpu().numpy(), ref_bi)
+    assert np.array_equal(p.tile_cols.cpu().numpy(), cols[ref_bi]) and np.array_equal(p.tile_scales.cpu().numpy(), ref_s[ref_bi])
+    order = np.argsort(-np.diff(ref_rp), kind="stable")
+    assert np.array_equal(p.row_order.cpu().numpy(), order)
+
+
+def test_tile_lists_that_are_not_valid_are_refused():
+    for rows, cols in (([0, 5], [0, 0]), ([0, 0], [1, 1]), ([-1, 0], [0, 0])):
+        br, bc = torch.tensor(rows, dtype=torch.int32, device="cuda"), torch.tensor(cols, dtype=torch.int32, device="cuda")
+        a = void.VOIDTensor(torch.randn(2, 32, 32, device="cuda"), br, bc, torch.zeros(2, dtype=torch.int64, device="cuda"),
+                            (64, 64), (32, 32), 0, 2, 0.5)
+        b = torch.randn(64, 8, device="cuda")
+        for call in (a.get_row_block_info, lambda: void.void_spmm(a, b), lambda: void.quantize_void_tensor(a).packed(),
+                     lambda: void.void_tensor_to_fp8(a).packed_split(2)):
+            with pytest.raises(ValueError, match="invalid VOID tile list"):
+                call()

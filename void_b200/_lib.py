@@ -62,6 +62,8 @@ _PROTOTYPES = {
     "void_morton_emit": (ctypes.c_int, [c_vp, c_i32, c_i32, c_i64, c_vp, c_vp, c_vp, c_vp]),
     "void_dense_gather": (ctypes.c_int, [c_vp, c_i32, c_i64, c_i32, c_i32, c_vp, c_vp, c_i64, c_vp, c_vp]),
     "void_csr_scatter": (ctypes.c_int, [c_vp, c_vp, c_vp, c_i32, c_i32, c_vp, c_i64, c_vp, c_vp]),
+    "void_row_order": (ctypes.c_int, [c_vp, c_i32, c_vp, c_vp]),
+    "void_quant_tiles": (ctypes.c_int, [c_vp, c_i32, c_i64, c_i32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "void_pack_tiles": (ctypes.c_int, [c_vp, c_vp, c_i64, c_vp, c_vp, c_vp, c_i64, c_i32, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "void_pack_tiles_f8_split": (ctypes.c_int, [c_vp, c_vp, c_i64, c_vp, c_vp, c_vp, c_vp, c_i64, c_i32, c_i32, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "void_reduce_slots": (ctypes.c_int, [c_vp, c_vp, c_i32, c_i32, c_i32, c_i32, c_i32, c_vp, c_vp, c_f32, c_vp, c_i32, c_vp, c_i64,

@@ -18,13 +18,6 @@ FLAG_DIRECT_STORES, FLAG_A_STABLE, FLAG_STORE_PER_TILE = 2, 4, 16   # bits of vo
 FLAG_NO_EARLY_A = 1 << 30   # host side only: never set FLAG_A_STABLE (measurements)
 
 
-def _aligned_empty(nbytes: int, device, align: int = 1024) -> torch.Tensor:
-    """uint8 buffer whose data pointer is ``align``-byte aligned."""
-    raw = torch.empty(nbytes + align, dtype=torch.uint8, device=device)
-    off = (-raw.data_ptr()) % align
-    return raw[off:off + nbytes]
-
-
 @dataclass
 class PackedTiles:
     """A in the layout the kernels stream: tiles in tile-row-major order, 1024 elements each, already
@@ -68,73 +61,27 @@ class PackedTiles:
 
 
 def pack(values: torch.Tensor, scales: Optional[torch.Tensor], block_rows: torch.Tensor, block_cols: torch.Tensor,
-         shape, kind: int, row_ptr=None, block_indices=None) -> PackedTiles:
-    """Build the packed store of a VOID tensor on its device: void_pack_tiles for the 8-bit kinds,
-    void_pack_tiles_fp for fp16 / bf16 / fp32 tiles (no scales)."""
-    from .format import build_tile_index
+         shape, kind: int, row_ptr=None, block_indices=None, terms: int = 1) -> PackedTiles:
+    """Build the packed store of a VOID tensor on its device: void_pack_tiles for the 8-bit kinds, with ``terms`` > 1
+    void_pack_tiles_f8_split (FP8 tiles with their scales folded in: every tile as a sum of that many E4M3 tiles relative
+    to the largest tile scale of its tile row, which lands in row_scale), void_pack_tiles_fp for fp16 / bf16 / fp32 tiles
+    (no scales).  The tile index is built on the way unless it is given; _mark_ready waits for all of it and checks it."""
     _lib.require_cuda(values, block_rows, block_cols)
-    lib = _lib.load()
-    dev = values.device
     M, K = shape
-    nbr, nbc = (M + TILE - 1) // TILE, (K + TILE - 1) // TILE
-    nnz = values.shape[0]
     es = _lib.KIND_ELEM_BYTES[kind]
     if values.dim() != 3 or values.shape[1] != TILE or values.shape[2] != TILE or values.element_size() != es:
         raise _lib.VoidB200Error("void_b200 kernels need 32x32 tiles of %d-byte elements here, got %s %s"
                                  % (es, tuple(values.shape), values.dtype))
-    with torch.cuda.device(dev):
-        if row_ptr is None or block_indices is None:
-            row_ptr, block_indices = build_tile_index(block_rows, block_cols, nbr, nbc)
-        vals = values.contiguous()
-        tiles = _aligned_empty(max(nnz, 1) * 1024 * es, dev)
-        tile_cols = torch.empty(max(nnz, 1), dtype=torch.int32, device=dev)
-        tile_scales = torch.empty(max(nnz, 1), dtype=torch.float32, device=dev)
-        row_scale = torch.empty(max(nbr, 1), dtype=torch.float32, device=dev)
-        sc = None if scales is None else scales.contiguous().to(torch.float32).reshape(-1)
-        bc = block_cols.contiguous().to(torch.int32)
-        if es > 1:
-            _lib.check(lib.void_pack_tiles_fp(_lib.ptr(vals), es, _lib.ptr(bc), _lib.ptr(block_indices), nnz,
-                                              _lib.ptr(tiles), _lib.ptr(tile_cols), _lib.stream_ptr(dev)),
-                       "void_pack_tiles_fp")
-            return PackedTiles(tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale, nbr, nbc, nnz,
-                               (M, K), kind)
-        _lib.check(lib.void_pack_tiles(_lib.ptr(vals), _lib.ptr(sc), 0 if sc is None else sc.numel(), _lib.ptr(bc),
-                                       _lib.ptr(block_indices), _lib.ptr(row_ptr), nnz, nbr, _lib.ptr(tiles),
-                                       _lib.ptr(tile_cols), _lib.ptr(tile_scales), _lib.ptr(row_scale),
-                                       _lib.stream_ptr(dev)), "void_pack_tiles")
-    return PackedTiles(tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale, nbr, nbc, nnz,
-                       (M, K), kind)
+    tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale = _lib.native().pack_store(
+        values, scales, block_rows, block_cols, M, K, kind, terms, row_ptr, block_indices)
+    return PackedTiles(tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale, (M + TILE - 1) // TILE,
+                       (K + TILE - 1) // TILE, values.shape[0], (M, K), kind, terms)
 
 
 def pack_f8_split(values: torch.Tensor, scales: Optional[torch.Tensor], block_rows: torch.Tensor,
                   block_cols: torch.Tensor, shape, terms: int) -> PackedTiles:
-    """Packed store of FP8 tiles with their scales folded in (void_pack_tiles_f8_split): every tile as a sum
-    of ``terms`` E4M3 tiles relative to the largest tile scale of its tile row, which lands in row_scale."""
-    from .format import build_tile_index
-    _lib.require_cuda(values, block_rows, block_cols)
-    lib = _lib.load()
-    dev = values.device
-    M, K = shape
-    nbr, nbc = (M + TILE - 1) // TILE, (K + TILE - 1) // TILE
-    nnz = values.shape[0]
-    if values.dim() != 3 or tuple(values.shape[1:]) != (TILE, TILE) or values.element_size() != 1:
-        raise _lib.VoidB200Error("void_b200 kernels need 32x32 FP8 tiles here, got %s %s" % (tuple(values.shape), values.dtype))
-    with torch.cuda.device(dev):
-        row_ptr, block_indices = build_tile_index(block_rows, block_cols, nbr, nbc)
-        vals = values.contiguous()
-        tiles = _aligned_empty(max(nnz, 1) * 1024 * terms, dev)
-        tile_cols = torch.empty(max(nnz, 1), dtype=torch.int32, device=dev)
-        tile_scales = torch.empty(max(nnz, 1), dtype=torch.float32, device=dev)
-        row_scale = torch.empty(max(nbr, 1), dtype=torch.float32, device=dev)
-        sc = None if scales is None else scales.contiguous().to(torch.float32).reshape(-1)
-        br = block_rows.contiguous().to(torch.int32)
-        bc = block_cols.contiguous().to(torch.int32)
-        _lib.check(lib.void_pack_tiles_f8_split(_lib.ptr(vals), _lib.ptr(sc), 0 if sc is None else sc.numel(), _lib.ptr(br),
-                                                _lib.ptr(bc), _lib.ptr(block_indices), _lib.ptr(row_ptr), nnz, nbr, terms,
-                                                _lib.ptr(tiles), _lib.ptr(tile_cols), _lib.ptr(tile_scales),
-                                                _lib.ptr(row_scale), _lib.stream_ptr(dev)), "void_pack_tiles_f8_split")
-    return PackedTiles(tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale, nbr, nbc, nnz, (M, K),
-                       _lib.KIND_F8E4M3, terms)
+    """Packed store of FP8 tiles with their scales folded in."""
+    return pack(values, scales, block_rows, block_cols, shape, _lib.KIND_F8E4M3, terms=terms)
 
 
 def _mark_ready(p: PackedTiles) -> PackedTiles:
@@ -143,11 +90,10 @@ def _mark_ready(p: PackedTiles) -> PackedTiles:
     # capture nothing can be waited for; a store built there is simply never read early.
     # The CTAs that start first take the first work items: with the tile rows sorted by falling tile count the
     # longest rows start earliest and the shortest are left for the CTAs that share an SM with the most others.
-    if p.nbr > 0:
-        counts = p.row_ptr[1:] - p.row_ptr[:-1]
-        p.row_order = torch.argsort(counts, descending=True, stable=True).to(torch.int32)
-    if not torch.cuda.is_current_stream_capturing():
-        torch.cuda.current_stream(p.tiles.device).synchronize()
+    from .format import check_indexed
+    p.row_order, indexed = _lib.native().finish_store(p.row_ptr, p.nbr)
+    if indexed is not None:
+        check_indexed(indexed, p.nnz)
         p.stable = True
     return p
 

@@ -68,6 +68,7 @@ int elem_bytes(int kind) { return kind == VOID_KIND_TF32 ? 4 : ((kind == VOID_KI
 at::Tensor new_cuda(at::IntArrayRef size, at::ScalarType type, c10::Device dev) {
   return at::Tensor(at::detail::empty_cuda(size, type, dev, std::nullopt));
 }
+at::Tensor as_type(const at::Tensor& t, at::ScalarType type) { return t.scalar_type() == type ? t : t.to(type); }
 void_stream_t stream_of(c10::DeviceIndex dev) { return c10::cuda::getCurrentCUDAStream(dev).stream(); }
 
 #define NATIVE_BEGIN                                    \
@@ -344,6 +345,220 @@ PyObject* quant_cols(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_END
 }
 
+// ------------------------------------------------------------------------------------------ set-up of a tensor
+// Waits for the stream with the interpreter free to run other threads.
+void wait_for(void_stream_t st) {
+  cudaError_t rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = cudaStreamSynchronize(reinterpret_cast<cudaStream_t>(st));
+  Py_END_ALLOW_THREADS
+  if (rc != cudaSuccess) throw std::runtime_error(std::string("CUDA error: ") + cudaGetErrorString(rc));
+}
+bool capturing(void_stream_t st) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(reinterpret_cast<cudaStream_t>(st), &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
+}
+// Host memory the GPU writes a few integers to (the caching host allocator hands the same block out again).
+at::Tensor host_words(int64_t n) {
+  return at::empty({n}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
+}
+at::Tensor as_index(PyObject* o, const char* what) {
+  const at::Tensor& t = cuda_tensor(o, what);
+  return as_type(t, at::kInt).contiguous();
+}
+PyObject* pack_tuple(std::initializer_list<at::Tensor> ts) {
+  PyObject* res = PyTuple_New((Py_ssize_t)ts.size());
+  if (res == nullptr) throw python_error();
+  Py_ssize_t i = 0;
+  for (const at::Tensor& t : ts) {
+    if (t.defined()) {
+      PyTuple_SET_ITEM(res, i++, THPVariable_Wrap(t));
+    } else {
+      Py_INCREF(Py_None);
+      PyTuple_SET_ITEM(res, i++, Py_None);
+    }
+  }
+  return res;
+}
+
+// dense_build(matrix, threshold) -> (values, block_rows, block_cols, morton_codes, n_blocks, nonzeros)
+PyObject* dense_build(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 2) throw torch::TypeError("dense_build takes 2 arguments");
+  const at::Tensor& in = cuda_tensor(a[0], "matrix");
+  const float threshold = (float)real(a[1]);
+  const c10::Device dev = in.device();
+  c10::cuda::OptionalCUDAGuard guard(dev);
+  const int64_t M = in.size(0), N = in.size(1);
+  const at::Tensor m = (N == 0 || (in.stride(1) == 1 && in.stride(0) >= N)) ? in : in.contiguous();
+  const int elem = out_code(m.scalar_type());
+  const int64_t ld = M > 1 ? m.stride(0) : std::max<int64_t>(N, 1);
+  const int32_t nbr = (int32_t)((M + 31) / 32), nbc = (int32_t)((N + 31) / 32);
+  const size_t ws_bytes = void_format_ws_bytes(nbr, nbc);
+  if (ws_bytes == 0)
+    fail("block grid " + std::to_string(nbr) + " x " + std::to_string(nbc) + " is too large for the device format builder");
+  const void_stream_t st = stream_of(dev.index());
+  const at::Tensor ws = new_cuda({(int64_t)ws_bytes}, at::kByte, dev);
+  const at::Tensor counts = host_words(2);
+  check(void_dense_mark(m.const_data_ptr(), elem, ld, (int32_t)M, (int32_t)N, threshold, ws.data_ptr(), ws_bytes,
+                        counts.data_ptr<int64_t>(), st),
+        "void_dense_mark");
+  wait_for(st);   // the one synchronisation, like .nonzero(): the outputs' sizes
+  const int64_t kept = counts.data_ptr<int64_t>()[0], nonzeros = counts.data_ptr<int64_t>()[1];
+  at::Tensor values = new_cuda({kept, 32, 32}, m.scalar_type(), dev);
+  at::Tensor rows = new_cuda({kept}, at::kInt, dev), cols = new_cuda({kept}, at::kInt, dev);
+  at::Tensor codes = new_cuda({kept}, at::kLong, dev);
+  check(void_morton_emit(ws.const_data_ptr(), nbr, nbc, kept, rows.data_ptr<int32_t>(), cols.data_ptr<int32_t>(),
+                         codes.data_ptr<int64_t>(), st),
+        "void_morton_emit");
+  check(void_dense_gather(m.const_data_ptr(), elem, ld, (int32_t)M, (int32_t)N, rows.const_data_ptr<int32_t>(),
+                          cols.const_data_ptr<int32_t>(), kept, values.data_ptr(), st),
+        "void_dense_gather");
+  return Py_BuildValue("NNNNLL", THPVariable_Wrap(values), THPVariable_Wrap(rows), THPVariable_Wrap(cols), THPVariable_Wrap(codes),
+                       (long long)kept, (long long)nonzeros);
+  NATIVE_END
+}
+
+// quant_tiles_i8(values [n, 32, 32], block_rows, block_cols) -> (q, scales, zero_points, block_rows copy, block_cols copy)
+PyObject* quant_tiles_i8(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 3) throw torch::TypeError("quant_tiles_i8 takes 3 arguments");
+  const at::Tensor& in = cuda_tensor(a[0], "values");
+  const c10::Device dev = in.device();
+  c10::cuda::OptionalCUDAGuard guard(dev);
+  const at::ScalarType t = in.scalar_type();
+  const at::Tensor v = (t == at::kFloat || t == at::kHalf || t == at::kBFloat16 ? in : in.to(at::kFloat)).contiguous();
+  const int64_t count = v.size(0);
+  at::Tensor q = new_cuda(v.sizes(), at::kChar, dev), scales = new_cuda({count}, at::kFloat, dev);
+  at::Tensor zeros = new_cuda({count}, at::kChar, dev);
+  at::Tensor copy[2];
+  const int32_t* from[2] = {nullptr, nullptr};
+  int32_t* to[2] = {nullptr, nullptr};
+  for (int i = 0; i < 2; ++i) {
+    const at::Tensor& c = tensor(a[1 + i], "block coordinates");
+    if (c.scalar_type() == at::kInt && c.is_contiguous() && c.device() == dev && c.numel() == count) {
+      copy[i] = new_cuda(c.sizes(), at::kInt, dev);
+      from[i] = c.const_data_ptr<int32_t>();
+      to[i] = copy[i].data_ptr<int32_t>();
+    } else {
+      copy[i] = c.clone();
+    }
+  }
+  check(void_quant_tiles(v.const_data_ptr(), out_code(v.scalar_type()), count, VOID_KIND_I8, q.data_ptr(), scales.data_ptr<float>(),
+                         nullptr, nullptr, zeros.data_ptr<int8_t>(), from[0], from[1], to[0], to[1], stream_of(dev.index())),
+        "void_quant_tiles");
+  return pack_tuple({q, scales, zeros, copy[0], copy[1]});
+  NATIVE_END
+}
+
+void build_index(const at::Tensor& rows, const at::Tensor& cols, int32_t nbr, int32_t nbc, at::Tensor& row_ptr, at::Tensor& block_indices,
+                 void_stream_t st) {
+  const c10::Device dev = rows.device();
+  const int64_t count = rows.numel();
+  row_ptr = new_cuda({nbr + 1}, at::kInt, dev);
+  block_indices = new_cuda({count}, at::kInt, dev);
+  const size_t ws_bytes = void_tile_index_ws_bytes(nbr, nbc);
+  const at::Tensor ws = new_cuda({(int64_t)ws_bytes}, at::kByte, dev);
+  check(void_build_tile_index(rows.const_data_ptr<int32_t>(), cols.const_data_ptr<int32_t>(), count, nbr, nbc, row_ptr.data_ptr<int32_t>(),
+                              block_indices.data_ptr<int32_t>(), ws.data_ptr(), ws_bytes, st),
+        "void_build_tile_index");
+}
+// Waits for the index and reads how many tiles it holds: one read of one integer per built index.
+long long indexed_tiles(const at::Tensor& row_ptr, int32_t nbr, void_stream_t st) {
+  const at::Tensor last = host_words(1);
+  if (cudaMemcpyAsync(last.data_ptr(), row_ptr.const_data_ptr<int32_t>() + nbr, 4, cudaMemcpyDeviceToHost,
+                      reinterpret_cast<cudaStream_t>(st)) != cudaSuccess)
+    throw std::runtime_error("CUDA error: reading the tile index failed");
+  wait_for(st);
+  return *static_cast<const int32_t*>(last.data_ptr());
+}
+
+// tile_index(block_rows, block_cols, nbr, nbc) -> (row_ptr, block_indices, indexed tiles)
+PyObject* tile_index(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 4) throw torch::TypeError("tile_index takes 4 arguments");
+  const at::Tensor rows = as_index(a[0], "block_rows"), cols = as_index(a[1], "block_cols");
+  c10::cuda::OptionalCUDAGuard guard(rows.device());
+  const void_stream_t st = stream_of(rows.device().index());
+  const int32_t nbr = (int32_t)integer(a[2]), nbc = (int32_t)integer(a[3]);
+  at::Tensor row_ptr, block_indices;
+  build_index(rows, cols, nbr, nbc, row_ptr, block_indices, st);
+  const long long indexed = indexed_tiles(row_ptr, nbr, st);
+  return Py_BuildValue("NNL", THPVariable_Wrap(row_ptr), THPVariable_Wrap(block_indices), indexed);
+  NATIVE_END
+}
+
+// pack_store(values, scales | None, block_rows, block_cols, M, K, kind, terms, row_ptr | None, block_indices | None)
+//   -> (tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale)
+// The packed store of a tensor, its tile index built on the way when it is not given.  The caller waits for it
+// and checks the index (finish_store); until then a list that is not valid is packed without leaving its arrays.
+PyObject* pack_store(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 10) throw torch::TypeError("pack_store takes 10 arguments");
+  const at::Tensor values = cuda_tensor(a[0], "values").contiguous();
+  const at::Tensor rows = as_index(a[2], "block_rows"), cols = as_index(a[3], "block_cols");
+  const c10::Device dev = values.device();
+  c10::cuda::OptionalCUDAGuard guard(dev);
+  const void_stream_t st = stream_of(dev.index());
+  const int64_t M = integer(a[4]), K = integer(a[5]), count = values.size(0);
+  const int kind = (int)integer(a[6]), terms = (int)integer(a[7]), es = elem_bytes(kind);
+  const int32_t nbr = (int32_t)((M + 31) / 32), nbc = (int32_t)((K + 31) / 32);
+  at::Tensor row_ptr, block_indices, scales;
+  if (none(a[8]) || none(a[9])) {
+    build_index(rows, cols, nbr, nbc, row_ptr, block_indices, st);
+  } else {
+    row_ptr = tensor(a[8], "row_ptr");
+    block_indices = tensor(a[9], "block_indices");
+  }
+  if (!none(a[1])) scales = as_type(tensor(a[1], "scales"), at::kFloat).contiguous();
+  const float* sc = scales.defined() ? scales.const_data_ptr<float>() : nullptr;
+  const int64_t n_sc = scales.defined() ? scales.numel() : 0;
+  const int64_t room = std::max<int64_t>(count, 1);
+  const at::Tensor raw = new_cuda({room * 1024 * es * terms + 1024}, at::kByte, dev);
+  const int64_t off = -reinterpret_cast<intptr_t>(raw.data_ptr()) & 1023;   // tiles start on a 1024-byte boundary
+  const at::Tensor tiles = raw.narrow(0, off, room * 1024 * es * terms);
+  const at::Tensor tile_cols = new_cuda({room}, at::kInt, dev), tile_scales = new_cuda({room}, at::kFloat, dev);
+  const at::Tensor row_scale = new_cuda({std::max<int64_t>(nbr, 1)}, at::kFloat, dev);
+  const int32_t *rp = row_ptr.const_data_ptr<int32_t>(), *bi = block_indices.const_data_ptr<int32_t>();
+  const int32_t *br = rows.const_data_ptr<int32_t>(), *bc = cols.const_data_ptr<int32_t>();
+  int32_t* tc = tile_cols.data_ptr<int32_t>();
+  float *ts = tile_scales.data_ptr<float>(), *rs = row_scale.data_ptr<float>();
+  if (es > 1)
+    check(void_pack_tiles_fp(values.const_data_ptr(), es, bc, bi, count, tiles.data_ptr(), tc, st), "void_pack_tiles_fp");
+  else if (terms > 1)
+    check(void_pack_tiles_f8_split(values.const_data_ptr(), sc, n_sc, br, bc, bi, rp, count, nbr, terms, tiles.data_ptr(), tc, ts, rs, st),
+          "void_pack_tiles_f8_split");
+  else
+    check(void_pack_tiles(values.const_data_ptr(), sc, n_sc, bc, bi, rp, count, nbr, tiles.data_ptr(), tc, ts, rs, st), "void_pack_tiles");
+  return pack_tuple({tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale});
+  NATIVE_END
+}
+
+// finish_store(row_ptr, nbr) -> (row_order, indexed tiles | None): the order of the tile rows, then - outside a stream
+// capture, where nothing can be waited for - the wait until the store is complete and the size of its index
+PyObject* finish_store(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 2) throw torch::TypeError("finish_store takes 2 arguments");
+  const at::Tensor& row_ptr = cuda_tensor(a[0], "row_ptr");
+  const int32_t nbr = (int32_t)integer(a[1]);
+  const c10::Device dev = row_ptr.device();
+  c10::cuda::OptionalCUDAGuard guard(dev);
+  const void_stream_t st = stream_of(dev.index());
+  at::Tensor order;
+  if (nbr > 0 && nbr <= 4096) {
+    order = new_cuda({nbr}, at::kInt, dev);
+    check(void_row_order(row_ptr.const_data_ptr<int32_t>(), nbr, order.data_ptr<int32_t>(), st), "void_row_order");
+  } else if (nbr > 0) {   // beyond a few thousand rows a sort does less work than comparing all pairs
+    order = at::argsort(row_ptr.narrow(0, 1, nbr) - row_ptr.narrow(0, 0, nbr), /*stable=*/true, 0, /*descending=*/true).to(at::kInt);
+  }
+  PyObject* o = Py_None;
+  if (order.defined()) o = THPVariable_Wrap(order);
+  else Py_INCREF(o);
+  if (capturing(st)) return Py_BuildValue("NO", o, Py_None);
+  return Py_BuildValue("NL", o, indexed_tiles(row_ptr, nbr, st));
+  NATIVE_END
+}
+
 // ------------------------------------------------------------------------------------------ training
 // The index arrays of one sparsity structure, both ways round; they outlive the values that train over them.
 struct Structure {
@@ -388,7 +603,6 @@ int common_kind(at::ScalarType a, at::ScalarType b) {   // their common 16-bit t
   return VOID_KIND_TF32;
 }
 at::ScalarType kind_type(int kind) { return kind == VOID_KIND_F16 ? at::kHalf : (kind == VOID_KIND_BF16 ? at::kBFloat16 : at::kFloat); }
-at::Tensor as_type(const at::Tensor& t, at::ScalarType type) { return t.scalar_type() == type ? t : t.to(type); }
 
 // Product with tiles that change from call to call: they are packed (their transposes for A^T) and multiplied at once.
 // linear: b is x [N, K] and the result x A^T [N, M]; otherwise b is [K, N] and the result A b [M, N].
@@ -553,6 +767,11 @@ PyMethodDef kMethods[] = {
     FAST(packed_is_current),
     FAST(spmm),
     FAST(quant_cols),
+    FAST(dense_build),
+    FAST(quant_tiles_i8),
+    FAST(tile_index),
+    FAST(pack_store),
+    FAST(finish_store),
     FAST(structure),
     FAST(values_product),
     FAST(tile_gradient),

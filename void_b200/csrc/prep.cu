@@ -49,9 +49,11 @@ __device__ void block_exclusive_scan(const int32_t* in, int32_t* out, int n) {
 // Coordinates outside the block grid are skipped here and in rank_tiles_kernel: the caller sees them (and
 // repeated coordinates, which set one bit twice) as row_ptr[nbr] < nnz.
 __global__ void mark_tiles_kernel(const int32_t* __restrict__ brow, const int32_t* __restrict__ bcol, int64_t nnz,
-                                  int nbr, int nbc, int wpr, uint32_t* __restrict__ bitmap) {
+                                  int nbr, int nbc, int wpr, uint32_t* __restrict__ bitmap,
+                                  int32_t* __restrict__ block_indices) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nnz) return;
+  block_indices[i] = 0;   // every entry is a valid position even when the list is rejected afterwards
   const int r = brow[i], c = bcol[i];
   if ((unsigned)r >= (unsigned)nbr || (unsigned)c >= (unsigned)nbc) return;
   atomicOr(bitmap + (size_t)r * wpr + (c >> 5), 1u << (c & 31));
@@ -68,6 +70,20 @@ __global__ void count_rows_kernel(const uint32_t* __restrict__ bitmap, int nbr, 
 }
 
 __global__ void __launch_bounds__(1024) scan_rows_kernel(const int32_t* counts, int32_t* row_ptr, int nbr) {
+  block_exclusive_scan(counts, row_ptr, nbr);
+}
+
+// both in one launch, for bitmaps one block reads in a couple of microseconds
+constexpr int kOneBlockBitmap = 32768;   // words
+__global__ void __launch_bounds__(1024) count_scan_rows_kernel(const uint32_t* __restrict__ bitmap, int nbr, int wpr,
+                                                               int32_t* __restrict__ counts, int32_t* __restrict__ row_ptr) {
+  const int per = (nbr + 1023) / 1024;
+  for (int r = threadIdx.x * per; r < (int)(threadIdx.x + 1) * per && r < nbr; ++r) {
+    int c = 0;
+    for (int w = 0; w < wpr; ++w) c += __popc(bitmap[(size_t)r * wpr + w]);
+    counts[r] = c;
+  }
+  __syncthreads();
   block_exclusive_scan(counts, row_ptr, nbr);
 }
 
@@ -89,8 +105,20 @@ __global__ void rank_tiles_kernel(const int32_t* __restrict__ brow, const int32_
 // One thread per 16-byte chunk of the packed tile.  Packed chunk q of a tile holds bytes
 // [c16*16, c16*16+16) of tile row r with  q = (r/8)*16 + c16*8 + (r%8): four groups of eight
 // rows, each group stored as two 8x16-byte core matrices (k bytes 0..15, then 16..31).
+// The first thread of a tile also gathers its block column and scale.
+struct TileMeta {
+  const int32_t* block_cols;
+  const float* scales;     // null: 1
+  int64_t n_scales;        // 1 (one scale for all tiles) or one per tile
+  int32_t* tile_cols;      // null: not wanted
+  float* tile_scales;      // null: not wanted
+};
+__device__ __forceinline__ void put_meta(const TileMeta& m, int64_t packed, int64_t src) {
+  if (m.tile_cols != nullptr) m.tile_cols[packed] = m.block_cols[src];
+  if (m.tile_scales != nullptr) m.tile_scales[packed] = m.scales == nullptr ? 1.0f : (m.n_scales == 1 ? m.scales[0] : m.scales[src]);
+}
 __global__ void pack_tiles_kernel(const uint4* __restrict__ values, const int32_t* __restrict__ block_indices,
-                                  int64_t nnz, uint4* __restrict__ packed) {
+                                  int64_t nnz, uint4* __restrict__ packed, TileMeta meta) {
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= nnz * 64) return;
   const int64_t j = g >> 6;
@@ -99,13 +127,14 @@ __global__ void pack_tiles_kernel(const uint4* __restrict__ values, const int32_
   const int c16 = (q >> 3) & 1;
   const int64_t src_tile = block_indices[j];
   packed[g] = values[src_tile * 64 + r * 2 + c16];
+  if (q == 0) put_meta(meta, j, src_tile);
 }
 
 // The same for elements of ES bytes: a tile row holds KC = 2*ES 16-byte chunks, a packed tile
 // 64*ES of them in the order [row / 8][chunk][row % 8].
 template <int ES>
 __global__ void pack_tiles_fp_kernel(const uint4* __restrict__ values, const int32_t* __restrict__ block_indices,
-                                     int64_t nnz, uint4* __restrict__ packed) {
+                                     int64_t nnz, uint4* __restrict__ packed, TileMeta meta) {
   constexpr int KC = 2 * ES, PER_TILE = 64 * ES;
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= nnz * PER_TILE) return;
@@ -124,6 +153,7 @@ __global__ void pack_tiles_fp_kernel(const uint4* __restrict__ values, const int
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(v.w) : "f"(__uint_as_float(v.w)));
   }
   packed[g] = v;
+  if (q == 0) put_meta(meta, j, src_tile);
 }
 
 // The packed form of the TRANSPOSED tiles (A^T for the gradient of the dense operand): chunk kc of row r' holds
@@ -167,7 +197,7 @@ template <int TERMS>
 __global__ void pack_tiles_f8_split_kernel(const uint4* __restrict__ values, const float* __restrict__ scales,
                                            int64_t n_scales, const int32_t* __restrict__ block_rows,
                                            const int32_t* __restrict__ block_indices,
-                                           const float* __restrict__ row_scale, int64_t nnz,
+                                           const float* __restrict__ row_scale, int64_t nnz, int nbr,
                                            uint4* __restrict__ packed) {
   const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= nnz * 64) return;
@@ -178,7 +208,8 @@ __global__ void pack_tiles_f8_split_kernel(const uint4* __restrict__ values, con
   const int64_t src = block_indices[j];
   const uint4 v = values[src * 64 + r * 2 + c16];
   const float s = (scales == nullptr) ? 1.0f : (n_scales == 1 ? scales[0] : scales[src]);
-  const float R = row_scale[block_rows[src]];
+  const int row = block_rows[src];
+  const float R = (unsigned)row < (unsigned)nbr ? row_scale[row] : 0.0f;   // (the list is checked after it is packed)
   const float ratio = (R > 0.0f) ? __fdiv_rn(s, R) : 0.0f;
   const uint32_t in[4] = {v.x, v.y, v.z, v.w};
   uint32_t out[TERMS][4];
@@ -284,6 +315,22 @@ __global__ void row_scale_kernel(const int32_t* __restrict__ row_ptr, const floa
   row_scale[r] = (t1 > t0) ? __fdiv_rn(s, (float)(t1 - t0)) : 0.0f;
 }
 
+// Tile rows by falling tile count, ties in their own order: a row's place is the number of rows that come before it.  One
+// warp per row counts them, which for the few thousand rows of a matrix takes less than a sort's launches.
+__global__ void row_order_kernel(const int32_t* __restrict__ row_ptr, int nbr, int32_t* __restrict__ order) {
+  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (r >= nbr) return;
+  const int mine = row_ptr[r + 1] - row_ptr[r];
+  int before = 0;
+#pragma unroll 4
+  for (int i = lane; i < nbr; i += 32) {
+    const int c = row_ptr[i + 1] - row_ptr[i];
+    before += (c > mine || (c == mine && i < r)) ? 1 : 0;
+  }
+  before = __reduce_add_sync(0xffffffffu, before);
+  if (lane == 0) order[before] = r;
+}
+
 // ------------------------------------------------------------------------------ quantisers
 __device__ __forceinline__ float warp_max(float v) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -330,55 +377,62 @@ __device__ __forceinline__ uint32_t quant_e4m3x4(const float4 x, const float4 in
          (uint32_t)__nv_cvt_float2_to_fp8x2(b, __NV_SATFINITE, __NV_E4M3) << 16;
 }
 
-// one warp per tile: 1024 fp32 values, 32 per lane
-__global__ void quant_i8_tiles_kernel(const float4* __restrict__ values, int64_t nnz, int8_t* __restrict__ q,
-                                      float* __restrict__ scales) {
-  const int64_t tile = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (tile >= nnz) return;
-  const float4* src = values + tile * 256;
-  float4 v[8];
-  float amax = 0.0f;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    v[i] = src[i * 32 + lane];
-    amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
-  }
-  amax = warp_max(amax);
-  const float scale = fmaxf(__fdiv_rn(amax, 128.0f), 1e-8f), inv = __fdiv_rn(1.0f, scale);
-  if (lane == 0) scales[tile] = scale;
-  uint32_t* dst = reinterpret_cast<uint32_t*>(q) + tile * 256;
-  const float4 sc = make_float4(scale, scale, scale, scale), si = make_float4(inv, inv, inv, inv);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) dst[i * 32 + lane] = quant_i8x4(v[i], sc, si);
+// What a quantised tensor carries beside its tiles: zero points (all zero) and its own copy of the tile coordinates.
+// Written by the quantiser's warps, so that the tensor costs one launch.
+struct StoreExtras {
+  int8_t* zero_points;
+  const int32_t* rows_in;
+  const int32_t* cols_in;
+  int32_t* rows_out;
+  int32_t* cols_out;
+};
+template <typename T>
+__device__ __forceinline__ float4 load4(const T* p);
+template <>
+__device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <>
+__device__ __forceinline__ float4 load4<__half>(const __half* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+  return make_float4(a.x, a.y, b.x, b.y);
 }
-
-__global__ void quant_fp8_tiles_kernel(const float4* __restrict__ values, int64_t nnz, uint8_t* __restrict__ q,
-                                       float* __restrict__ scale_out, float* __restrict__ scale_inv_out,
-                                       float* __restrict__ amax_out) {
+template <>
+__device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+                     __uint_as_float(u.y & 0xffff0000u));
+}
+// One warp per tile: 1024 values, 32 per lane, read once and in their own type.
+template <int KIND, typename T>
+__global__ void __launch_bounds__(256) quant_tiles_kernel(const T* __restrict__ values, int64_t nnz, uint8_t* __restrict__ q,
+                                                          float* __restrict__ scale_out, float* __restrict__ scale_inv_out,
+                                                          float* __restrict__ amax_out, StoreExtras x) {
   const int64_t tile = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (tile >= nnz) return;
-  const float4* src = values + tile * 256;
+  const T* src = values + tile * 1024;
   float4 v[8];
   float amax = 0.0f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    v[i] = src[i * 32 + lane];
+  for (int i = 0; i < 8; ++i) v[i] = load4<T>(src + (i * 32 + lane) * 4);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
     amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
-  }
   amax = warp_max(amax);
-  const float scale = fmaxf(__fdiv_rn(amax, 448.0f), 1e-12f);
+  const float scale = KIND == VOID_KIND_I8 ? fmaxf(__fdiv_rn(amax, 128.0f), 1e-8f) : fmaxf(__fdiv_rn(amax, 448.0f), 1e-12f);
   const float inv = __fdiv_rn(1.0f, scale);
   if (lane == 0) {
     scale_out[tile] = scale;
     if (scale_inv_out != nullptr) scale_inv_out[tile] = inv;
     if (amax_out != nullptr) amax_out[tile] = amax;
+    if (x.zero_points != nullptr) x.zero_points[tile] = 0;
+    if (x.rows_out != nullptr) x.rows_out[tile] = x.rows_in[tile];
+    if (x.cols_out != nullptr) x.cols_out[tile] = x.cols_in[tile];
   }
   uint32_t* dst = reinterpret_cast<uint32_t*>(q) + tile * 256;
-  const float4 si = make_float4(inv, inv, inv, inv);
+  const float4 sc = make_float4(scale, scale, scale, scale), si = make_float4(inv, inv, inv, inv);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) dst[i * 32 + lane] = quant_e4m3x4(v[i], si);
+  for (int i = 0; i < 8; ++i) dst[i * 32 + lane] = KIND == VOID_KIND_I8 ? quant_i8x4(v[i], sc, si) : quant_e4m3x4(v[i], si);
 }
 
 // column absmax of a row-major [K, N] matrix: block = 128 columns x a slab of k rows
@@ -763,15 +817,26 @@ int void_build_tile_index(const int32_t* block_rows, const int32_t* block_cols, 
   int32_t* counts = reinterpret_cast<int32_t*>(bitmap + (size_t)nbr * wpr);
   if (cudaMemsetAsync(bitmap, 0, (size_t)nbr * wpr * 4, st) != cudaSuccess) return VOID_ERR_CUDA;
   const int tb = 256;
-  // every entry of block_indices is a valid position even when the list is rejected afterwards
-  if (nnz > 0 && cudaMemsetAsync(block_indices, 0, (size_t)nnz * 4, st) != cudaSuccess) return VOID_ERR_CUDA;
   if (nnz > 0)
-    mark_tiles_kernel<<<(unsigned)((nnz + tb - 1) / tb), tb, 0, st>>>(block_rows, block_cols, nnz, nbr, nbc, wpr, bitmap);
-  count_rows_kernel<<<(unsigned)(((int64_t)nbr * 32 + tb - 1) / tb), tb, 0, st>>>(bitmap, nbr, wpr, counts);
-  scan_rows_kernel<<<1, 1024, 0, st>>>(counts, row_ptr, nbr);
+    mark_tiles_kernel<<<(unsigned)((nnz + tb - 1) / tb), tb, 0, st>>>(block_rows, block_cols, nnz, nbr, nbc, wpr, bitmap,
+                                                                     block_indices);
+  if ((int64_t)nbr * wpr <= kOneBlockBitmap) {
+    count_scan_rows_kernel<<<1, 1024, 0, st>>>(bitmap, nbr, wpr, counts, row_ptr);
+  } else {
+    count_rows_kernel<<<(unsigned)(((int64_t)nbr * 32 + tb - 1) / tb), tb, 0, st>>>(bitmap, nbr, wpr, counts);
+    scan_rows_kernel<<<1, 1024, 0, st>>>(counts, row_ptr, nbr);
+  }
   if (nnz > 0)
     rank_tiles_kernel<<<(unsigned)((nnz + tb - 1) / tb), tb, 0, st>>>(block_rows, block_cols, nnz, nbr, nbc, wpr, bitmap,
                                                                      row_ptr, block_indices);
+  return last_status();
+}
+
+int void_row_order(const int32_t* row_ptr, int32_t nbr, int32_t* order, void_stream_t stream) {
+  if (nbr < 0) return VOID_ERR_BAD_ARG;
+  if (nbr == 0) return VOID_OK;
+  if (row_ptr == nullptr || order == nullptr) return VOID_ERR_BAD_ARG;
+  row_order_kernel<<<(unsigned)(((int64_t)nbr * 32 + 255) / 256), 256, 0, as_stream(stream)>>>(row_ptr, nbr, order);
   return last_status();
 }
 
@@ -789,9 +854,8 @@ int void_pack_tiles(const void* values, const float* scales, int64_t n_scales, c
       return VOID_ERR_ALIGN;
     if (scales != nullptr && n_scales != 1 && n_scales != nnz) return VOID_ERR_BAD_ARG;
     pack_tiles_kernel<<<(unsigned)((nnz * 64 + tb - 1) / tb), tb, 0, st>>>(
-        reinterpret_cast<const uint4*>(values), block_indices, nnz, reinterpret_cast<uint4*>(packed));
-    gather_tile_meta_kernel<<<(unsigned)((nnz + tb - 1) / tb), tb, 0, st>>>(block_cols, scales, n_scales, block_indices,
-                                                                           nnz, tile_cols, tile_scales);
+        reinterpret_cast<const uint4*>(values), block_indices, nnz, reinterpret_cast<uint4*>(packed),
+        TileMeta{block_cols, scales, n_scales, tile_cols, tile_scales});
   }
   if (row_scale != nullptr && nbr > 0) {
     if (row_ptr == nullptr || (nnz > 0 && tile_scales == nullptr)) return VOID_ERR_BAD_ARG;
@@ -823,11 +887,11 @@ int void_pack_tiles_f8_split(const void* values, const float* scales, int64_t n_
     const unsigned blocks = (unsigned)((nnz * 64 + tb - 1) / tb);
     if (terms == 2)
       pack_tiles_f8_split_kernel<2><<<blocks, tb, 0, st>>>(reinterpret_cast<const uint4*>(values), scales, n_scales,
-                                                           block_rows, block_indices, row_scale, nnz,
+                                                           block_rows, block_indices, row_scale, nnz, nbr,
                                                            reinterpret_cast<uint4*>(packed));
     else
       pack_tiles_f8_split_kernel<3><<<blocks, tb, 0, st>>>(reinterpret_cast<const uint4*>(values), scales, n_scales,
-                                                           block_rows, block_indices, row_scale, nnz,
+                                                           block_rows, block_indices, row_scale, nnz, nbr,
                                                            reinterpret_cast<uint4*>(packed));
   }
   return last_status();
@@ -859,14 +923,13 @@ int void_pack_tiles_fp(const void* values, int32_t elem_bytes, const int32_t* bl
   cudaStream_t st = as_stream(stream);
   const int tb = 256;
   const unsigned blocks = (unsigned)((nnz * 64 * elem_bytes + tb - 1) / tb);
+  const TileMeta meta{block_cols, nullptr, 0, tile_cols, nullptr};
   if (elem_bytes == 2)
     pack_tiles_fp_kernel<2><<<blocks, tb, 0, st>>>(reinterpret_cast<const uint4*>(values), block_indices, nnz,
-                                                   reinterpret_cast<uint4*>(packed));
+                                                   reinterpret_cast<uint4*>(packed), meta);
   else
     pack_tiles_fp_kernel<4><<<blocks, tb, 0, st>>>(reinterpret_cast<const uint4*>(values), block_indices, nnz,
-                                                   reinterpret_cast<uint4*>(packed));
-  gather_tile_meta_kernel<<<(unsigned)((nnz + tb - 1) / tb), tb, 0, st>>>(block_cols, nullptr, 0, block_indices, nnz,
-                                                                         tile_cols, nullptr);
+                                                   reinterpret_cast<uint4*>(packed), meta);
   return last_status();
 }
 
@@ -886,8 +949,8 @@ int void_repack_tiles_fp(const void* values, int32_t elem_bytes, const int32_t* 
     if (elem_bytes == 2) pack_tiles_fp_t_kernel<2><<<blocks, tb, 0, st>>>(values, block_indices, nnz, o);
     else pack_tiles_fp_t_kernel<4><<<blocks, tb, 0, st>>>(values, block_indices, nnz, o);
   } else {
-    if (elem_bytes == 2) pack_tiles_fp_kernel<2><<<blocks, tb, 0, st>>>(v, block_indices, nnz, o);
-    else pack_tiles_fp_kernel<4><<<blocks, tb, 0, st>>>(v, block_indices, nnz, o);
+    if (elem_bytes == 2) pack_tiles_fp_kernel<2><<<blocks, tb, 0, st>>>(v, block_indices, nnz, o, TileMeta{});
+    else pack_tiles_fp_kernel<4><<<blocks, tb, 0, st>>>(v, block_indices, nnz, o, TileMeta{});
   }
   return last_status();
 }
@@ -903,27 +966,41 @@ int void_column_sum(const void* in, int32_t elem, int64_t ld, int32_t rows, int3
   return ok ? last_status() : VOID_ERR_CUDA;
 }
 
-int void_quant_i8_tiles(const float* values, int64_t nnz, int8_t* q, float* scales, void_stream_t stream) {
-  if (nnz < 0) return VOID_ERR_BAD_ARG;
+int void_quant_tiles(const void* values, int32_t elem, int64_t nnz, int32_t kind, void* q, float* scale, float* scale_inv,
+                     float* amax, int8_t* zero_points, const int32_t* block_rows, const int32_t* block_cols,
+                     int32_t* rows_out, int32_t* cols_out, void_stream_t stream) {
+  if (nnz < 0 || elem < VOID_ELEM_F32 || elem > VOID_ELEM_BF16 || (kind != VOID_KIND_I8 && kind != VOID_KIND_F8E4M3))
+    return VOID_ERR_BAD_ARG;
   if (nnz == 0) return VOID_OK;
-  if (values == nullptr || q == nullptr || scales == nullptr) return VOID_ERR_BAD_ARG;
+  if (values == nullptr || q == nullptr || scale == nullptr) return VOID_ERR_BAD_ARG;
+  if ((rows_out != nullptr && block_rows == nullptr) || (cols_out != nullptr && block_cols == nullptr)) return VOID_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(values) & 15u) != 0 || (reinterpret_cast<uintptr_t>(q) & 3u) != 0) return VOID_ERR_ALIGN;
-  const int tb = 256;
-  quant_i8_tiles_kernel<<<(unsigned)((nnz * 32 + tb - 1) / tb), tb, 0, as_stream(stream)>>>(
-      reinterpret_cast<const float4*>(values), nnz, q, scales);
+  const StoreExtras x{zero_points, block_rows, block_cols, rows_out, cols_out};
+  const unsigned blocks = (unsigned)((nnz * 32 + 255) / 256);
+  uint8_t* dst = reinterpret_cast<uint8_t*>(q);
+  cudaStream_t st = as_stream(stream);
+#define VB_QUANT(T)                                                                                                             \
+  do {                                                                                                                          \
+    const T* v = reinterpret_cast<const T*>(values);                                                                            \
+    if (kind == VOID_KIND_I8) quant_tiles_kernel<VOID_KIND_I8, T><<<blocks, 256, 0, st>>>(v, nnz, dst, scale, scale_inv, amax, x); \
+    else quant_tiles_kernel<VOID_KIND_F8E4M3, T><<<blocks, 256, 0, st>>>(v, nnz, dst, scale, scale_inv, amax, x);               \
+  } while (0)
+  if (elem == VOID_ELEM_F32) VB_QUANT(float);
+  else if (elem == VOID_ELEM_F16) VB_QUANT(__half);
+  else VB_QUANT(__nv_bfloat16);
+#undef VB_QUANT
   return last_status();
+}
+
+int void_quant_i8_tiles(const float* values, int64_t nnz, int8_t* q, float* scales, void_stream_t stream) {
+  return void_quant_tiles(values, VOID_ELEM_F32, nnz, VOID_KIND_I8, q, scales, nullptr, nullptr, nullptr, nullptr, nullptr,
+                          nullptr, nullptr, stream);
 }
 
 int void_quant_fp8_tiles(const float* values, int64_t nnz, uint8_t* q, float* scale, float* scale_inv, float* amax,
                          void_stream_t stream) {
-  if (nnz < 0) return VOID_ERR_BAD_ARG;
-  if (nnz == 0) return VOID_OK;
-  if (values == nullptr || q == nullptr || scale == nullptr) return VOID_ERR_BAD_ARG;
-  if ((reinterpret_cast<uintptr_t>(values) & 15u) != 0 || (reinterpret_cast<uintptr_t>(q) & 3u) != 0) return VOID_ERR_ALIGN;
-  const int tb = 256;
-  quant_fp8_tiles_kernel<<<(unsigned)((nnz * 32 + tb - 1) / tb), tb, 0, as_stream(stream)>>>(
-      reinterpret_cast<const float4*>(values), nnz, q, scale, scale_inv, amax);
-  return last_status();
+  return void_quant_tiles(values, VOID_ELEM_F32, nnz, VOID_KIND_F8E4M3, q, scale, scale_inv, amax, nullptr, nullptr, nullptr,
+                          nullptr, nullptr, stream);
 }
 
 static void quant_pass(const float* b, int64_t ldb, int K, int N, int kind, void* q, int64_t ldq, const float* scale,

@@ -55,31 +55,22 @@ def morton_encode_batch(rows: np.ndarray, cols: np.ndarray) -> np.ndarray:
 def build_tile_index(block_rows: torch.Tensor, block_cols: torch.Tensor, nbr: int, nbc: int):
     """row_ptr[nbr+1] and block_indices[nnz] of a tile list on the GPU (void_build_tile_index)."""
     _lib.require_cuda(block_rows, block_cols)
-    lib = _lib.load()
-    dev = block_rows.device
-    nnz = block_rows.numel()
-    with torch.cuda.device(dev):
-        row_ptr = torch.empty(nbr + 1, dtype=torch.int32, device=dev)
-        block_indices = torch.empty(nnz, dtype=torch.int32, device=dev)
-        ws_bytes = lib.void_tile_index_ws_bytes(nbr, nbc)
-        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-        br = block_rows.contiguous().to(torch.int32)
-        bc = block_cols.contiguous().to(torch.int32)
-        _lib.check(lib.void_build_tile_index(_lib.ptr(br), _lib.ptr(bc), nnz, nbr, nbc, _lib.ptr(row_ptr),
-                                             _lib.ptr(block_indices), _lib.ptr(ws), ws_bytes, _lib.stream_ptr(dev)),
-                   "void_build_tile_index")
-        check_tile_index(row_ptr, nnz)
+    row_ptr, block_indices, indexed = _lib.native().tile_index(block_rows, block_cols, nbr, nbc)
+    check_indexed(indexed, block_rows.numel())
     return row_ptr, block_indices
 
 
-def check_tile_index(row_ptr: torch.Tensor, nnz: int) -> None:
+def check_indexed(indexed: int, nnz: int) -> None:
     """The index builder skips block coordinates outside the grid and counts a repeated (row, column) pair
-    once; either shows as fewer indexed tiles than listed ones.  (One read of one integer per built index;
-    the index is cached on its tensor.)"""
-    indexed = int(row_ptr[-1].item())
+    once; either shows as fewer indexed tiles than listed ones."""
     if indexed != nnz:
         raise ValueError("invalid VOID tile list: %d of %d tiles have block coordinates outside the block grid or "
                          "repeat an earlier (block_row, block_col) pair" % (nnz - indexed, nnz))
+
+
+def check_tile_index(row_ptr: torch.Tensor, nnz: int) -> None:
+    """check_indexed for an index that is at hand."""
+    check_indexed(int(row_ptr[-1].item()), nnz)
 
 
 @dataclass
@@ -178,7 +169,7 @@ class VOIDTensor:
 
 
 def _build_on_device(mark, fill, M: int, N: int, dev, value_dtype: torch.dtype):
-    """Shared tail of the device builders: mark kept tiles, read their count, emit the Morton-ordered
+    """Tail of the device builder for CSR arrays: mark kept tiles, read their count, emit the Morton-ordered
     index and fill the tile values.  Returns (values, block_rows, block_cols, morton_codes, n_blocks, nnz)."""
     lib = _lib.load()
     nbr, nbc = (M + 31) // 32, (N + 31) // 32
@@ -210,22 +201,11 @@ def dense_to_void(matrix: torch.Tensor, tile_size: int = 32, threshold: float = 
     if matrix.dtype not in _lib.ELEM_CODE:
         raise _lib.VoidB200Error("dense_to_void takes float32, float16 or bfloat16, got %s" % matrix.dtype)
     M, N = matrix.shape
-    dev = matrix.device
-    a = matrix if matrix.stride(1) == 1 and matrix.stride(0) >= max(N, 1) else matrix.contiguous()
-    elem, ld = _lib.ELEM_CODE[a.dtype], a.stride(0) if M > 1 else max(N, 1)
-
-    def mark(lib, ws, ws_bytes, counts):
-        _lib.check(lib.void_dense_mark(_lib.ptr(a), elem, ld, M, N, float(threshold), _lib.ptr(ws), ws_bytes,
-                                       _lib.ptr(counts), _lib.stream_ptr(dev)), "void_dense_mark")
-
-    def fill(lib, ws, n_blocks, block_rows, block_cols, values):
-        _lib.check(lib.void_dense_gather(_lib.ptr(a), elem, ld, M, N, _lib.ptr(block_rows), _lib.ptr(block_cols),
-                                         n_blocks, _lib.ptr(values), _lib.stream_ptr(dev)), "void_dense_gather")
-
-    values, block_rows, block_cols, codes, n_blocks, nnz, grid = _build_on_device(mark, fill, M, N, dev, a.dtype)
+    values, block_rows, block_cols, codes, n_blocks, nnz = _lib.native().dense_build(matrix, threshold)
+    grid = ((M + 31) // 32) * ((N + 31) // 32)
     return VOIDTensor(values=values, block_rows=block_rows, block_cols=block_cols, morton_codes=codes, shape=(M, N),
                       tile_size=(32, 32), nnz_original=nnz, n_blocks=n_blocks,
-                      density=(n_blocks / grid) if n_blocks else 0.0, dtype=a.dtype)
+                      density=(n_blocks / grid) if n_blocks else 0.0, dtype=values.dtype)
 
 
 def _csr_to_void_device(matrix, dtype: torch.dtype, device) -> VOIDTensor:

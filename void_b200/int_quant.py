@@ -186,26 +186,19 @@ def quantize_void_tensor(void_tensor, config: Optional[IntQuantConfig] = None) -
     _require_supported(config)
     values = void_tensor.values
     _lib.require_cuda(values)
-    lib = _lib.load()
     n_blocks = void_tensor.n_blocks
-    tile_m, tile_k = void_tensor.tile_size
-    dev = values.device
     if config.scale_mode == ScaleMode.PER_BLOCK:
-        if (tile_m, tile_k) != (32, 32):
+        if tuple(void_tensor.tile_size) != (32, 32):
             raise NotImplementedError("void_b200 kernels are built for 32x32 tiles")
-        vf = values.to(torch.float32).contiguous()
-        q = torch.empty(n_blocks, tile_m, tile_k, dtype=torch.int8, device=dev)
-        scales = torch.empty(n_blocks, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
-            _lib.check(lib.void_quant_i8_tiles(_lib.ptr(vf), n_blocks, _lib.ptr(q), _lib.ptr(scales),
-                                               _lib.stream_ptr(dev)), "void_quant_i8_tiles")
+        q, scales, zero_points, block_rows, block_cols = _lib.native().quant_tiles_i8(values, void_tensor.block_rows,
+                                                                                      void_tensor.block_cols)
     else:
         q_flat, params = quantize_tensor(values.reshape(1, -1), IntQuantConfig(scale_mode=ScaleMode.PER_TENSOR))
-        q = q_flat.reshape(n_blocks, tile_m, tile_k)
+        q = q_flat.reshape((n_blocks,) + tuple(void_tensor.tile_size))
         scales = params.scale.reshape(1).expand(n_blocks).contiguous()
-    return Int8VOIDTensor(values=q, scales=scales,
-                          zero_points=torch.zeros(n_blocks, dtype=torch.int8, device=dev),
-                          block_rows=void_tensor.block_rows.clone(), block_cols=void_tensor.block_cols.clone(),
+        zero_points = torch.zeros(n_blocks, dtype=torch.int8, device=values.device)
+        block_rows, block_cols = void_tensor.block_rows.clone(), void_tensor.block_cols.clone()
+    return Int8VOIDTensor(values=q, scales=scales, zero_points=zero_points, block_rows=block_rows, block_cols=block_cols,
                           shape=void_tensor.shape, tile_size=void_tensor.tile_size, n_blocks=n_blocks, config=config)
 
 
