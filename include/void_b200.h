@@ -169,6 +169,10 @@ VOID_API int void_pack_tiles_fp(const void* values, int32_t elem_bytes, const in
  * copy of the tiles in between. */
 VOID_API int void_repack_tiles_fp(const void* values, int32_t elem_bytes, const int32_t* block_indices,
                                   int64_t nnz, int32_t transposed, void* packed, void_stream_t stream);
+/* Copy of a row-major [rows, cols] matrix of elem_bytes-wide elements to rows that start on 16-byte boundaries, what the
+ * products need of B (ld_in / ld_out in BYTES, ld_out a multiple of 16); the padding is zeroed. */
+VOID_API int void_copy_rows(const void* in, int64_t ld_in, void* out, int64_t ld_out, int32_t elem_bytes, int64_t rows,
+                            int32_t cols, void_stream_t stream);
 /* Column sums of a row-major [rows, cols] matrix of type elem (VOID_ELEM_*), ld elements between rows, accumulated in
  * fp32 in a fixed order, written in the same type: the gradient of a linear layer's bias. */
 VOID_API int void_column_sum(const void* in, int32_t elem, int64_t ld, int32_t rows, int32_t cols, void* out,

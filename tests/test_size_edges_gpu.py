@@ -112,3 +112,61 @@ def test_tile_lists_that_are_not_valid_are_refused():
                      lambda: void.void_tensor_to_fp8(a).packed_split(2)):
             with pytest.raises(ValueError, match="invalid VOID tile list"):
                 call()
+
+
+# ------------------------------------------------------------------------------------------ few columns
+def _integer_matrix(m, k, density, seed):
+    gen = torch.Generator().manual_seed(seed)
+    nbr, nbc = (m + 31) // 32, (k + 31) // 32
+    mask = torch.rand(nbr, nbc, generator=gen) < density
+    mask[nbr // 2] = False                                                # an empty tile row
+    mask[0, nbc - 1] = True
+    dense = torch.randint(-3, 4, (m, k), generator=gen).float()
+    return dense * mask.repeat_interleave(32, 0).repeat_interleave(32, 1)[:m, :k], gen
+
+
+@pytest.mark.parametrize("dtype", [torch.int8, torch.float8_e4m3fn, torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,k,density", [(32, 32, 1.0), (95, 200, 0.7), (330, 1100, 0.9), (64, 2500, 0.8)])
+def test_products_with_few_columns_are_exact_on_small_integers(dtype, m, k, density):
+    dense, gen = _integer_matrix(m, k, density, m + k)
+    a = void.dense_to_void(dense.cuda())
+    scale = 1.0
+    if dtype == torch.int8:
+        q = void.quantize_void_tensor(a)
+        q.values, q.scales = a.values.to(torch.int8), torch.ones_like(q.scales)
+    elif dtype == torch.float8_e4m3fn:
+        q = void.void_tensor_to_fp8(a)
+        q.values_fp8 = a.values.to(dtype)
+        q.scaling_info.scale = torch.ones_like(q.scaling_info.scale)
+    else:
+        q = a.to_dtype(dtype)
+    for n in (1, 2, 7, 8, 9, 16, 17, 31, 32, 33, 63, 64, 100, 128, 129):
+        b = torch.randint(-3, 4, (k, n), generator=gen).float()
+        ref = dense.double() @ b.double()
+        bias = torch.randint(-4, 5, (n,), generator=gen).float()
+        if dtype == torch.int8:
+            cs = torch.tensor([1.0, 2.0, 0.5]).repeat(n)[:n]
+            got = void.void_spmm_int8(q, b.to(torch.int8).cuda(), cs.cuda() if n > 1 else scale, bias=bias.cuda())
+            assert torch.equal(got.double().cpu(), ref * (cs.double() if n > 1 else 1.0) + bias.double()), n
+            y = void.void_linear(q, b.t().contiguous().to(torch.int8).cuda(), None, 1)
+            assert torch.equal(y.double().cpu(), ref.t().clamp(min=0)), n
+        elif dtype == torch.float8_e4m3fn:
+            b8 = torch.zeros(k, (n + 15) // 16 * 16, dtype=torch.float8_e4m3fn, device="cuda")[:, :n]
+            b8.view(torch.uint8).copy_(b.to(dtype).view(torch.uint8).cuda())
+            got = void.void_spmm_fp8(q, b8, torch.float32, bias=bias.cuda())
+            assert torch.equal(got.double().cpu(), ref + bias.double()), n
+        else:
+            bd = b.cuda().to(dtype)
+            got = void.void_spmm(q, bd, bias=bias.cuda())
+            assert torch.equal(got.double().cpu(), (ref + bias.double()).to(dtype).double()), n
+            rb = torch.randint(-4, 5, (m,), generator=gen).float().cuda()
+            y = void.void_linear(q, bd.t().contiguous(), rb)
+            assert torch.equal(y.double().cpu(), (ref.t() + rb.double().cpu()).to(dtype).double()), n
+    if dtype not in (torch.int8, torch.float8_e4m3fn):
+        x = torch.randint(-3, 4, (k,), generator=gen).float()
+        y = void.void_spmv(q, x.cuda().to(dtype))
+        assert torch.equal(y.double().cpu(), (dense.double() @ x.double()).to(dtype).double())
+        wide = torch.zeros(m, 3, dtype=dtype, device="cuda")
+        void.void_spmv(q, x.cuda().to(dtype), wide[:, 1])                # a result with a stride
+        assert torch.equal(wide[:, 1], y)
+    void.check_device_status()

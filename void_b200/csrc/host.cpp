@@ -174,19 +174,30 @@ PyObject* packed_is_current(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // ------------------------------------------------------------------------------------------ products
-// B with unit column stride and rows on 16-byte boundaries, as the copy engine needs them; others are copied.
+// B with unit column stride and rows on 16-byte boundaries, as the copy engine needs them; others are copied (one pass).
+// A single row has no pitch, so only its start matters.
 at::Tensor kernel_operand(const at::Tensor& b, int es) {
   if (b.element_size() != es)
     fail("B must have " + std::to_string(es) + "-byte elements to match A, got " + c10::toString(b.scalar_type()));
-  const int64_t per16 = 16 / es;
-  if (b.stride(1) == 1 && b.stride(0) % per16 == 0 && (reinterpret_cast<uintptr_t>(b.const_data_ptr()) & 15u) == 0 &&
-      b.stride(0) >= b.size(1))
+  const int64_t rows = b.size(0), cols = b.size(1), per16 = 16 / es;
+  const bool unit = b.stride(1) == 1 || cols <= 1;
+  if (unit && (reinterpret_cast<uintptr_t>(b.const_data_ptr()) & 15u) == 0 &&
+      (rows == 1 || (b.stride(0) % per16 == 0 && b.stride(0) >= cols)))
     return b;
-  const int64_t ld = (b.size(1) + per16 - 1) / per16 * per16;
-  at::Tensor padded = at::zeros({b.size(0), ld}, b.options());
-  at::Tensor view = padded.narrow(1, 0, b.size(1));
-  view.copy_(b);
+  const int64_t ld = (cols + per16 - 1) / per16 * per16;
+  at::Tensor padded = new_cuda({rows, ld}, b.scalar_type(), b.device());
+  at::Tensor view = padded.narrow(1, 0, cols);
+  if (unit && b.stride(0) >= cols)
+    check(void_copy_rows(b.const_data_ptr(), b.stride(0) * es, padded.data_ptr(), ld * es, es, rows, (int32_t)cols,
+                         stream_of(b.device().index())),
+          "void_copy_rows");
+  else
+    view.copy_(b);
   return view;
+}
+// Bytes between the rows of a kernel operand.
+int64_t row_pitch(const at::Tensor& b, int es) {
+  return b.size(0) == 1 ? (b.size(1) * es + 15) / 16 * 16 : b.stride(0) * es;
 }
 at::Tensor fp32_vector(PyObject* o, c10::Device dev, const char* what) {
   const at::Tensor& t = tensor(o, what);
@@ -233,7 +244,7 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   s.scale_mode = per_tile ? VOID_SCALE_PER_TILE : VOID_SCALE_ROW_MEAN;
   bool use_row_scale = true;
   s.b = b.const_data_ptr();
-  s.ldb = b.stride(0) * es;
+  s.ldb = row_pitch(b, es);
   s.N = (int32_t)N;
   at::Tensor col_scale, bias, row_bias;   // keep converted copies alive until the launch is queued
   if (!none(a[5])) {
@@ -300,6 +311,41 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const void_stream_t st = stream_of(dev.index());
   if (es > 1) check(void_spmm_fp(&s, pk->kind, st), "void_spmm_fp");
   else check(pk->kind == VOID_KIND_I8 ? void_spmm_i8(&s, st) : void_spmm_f8(&s, st), "void_spmm");
+  if (!none(a[2])) {
+    Py_INCREF(a[2]);
+    return a[2];
+  }
+  return THPVariable_Wrap(out);
+  NATIVE_END
+}
+
+// spmv(handle, x [K], out [M] | None, out_dtype) -> y = A x
+PyObject* spmv(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 4) throw torch::TypeError("spmv takes 4 arguments");
+  const PackedObject* pk = packed_of(a[0]);
+  at::Tensor x = cuda_tensor(a[1], "x");
+  const c10::Device dev = x.device();
+  const int es = elem_bytes(pk->kind);
+  if (dev.index() != pk->device) fail("A and x are on different devices");
+  if (x.dim() != 1 || x.size(0) != pk->K || x.element_size() != es) fail("x must be a vector of K elements of A's type");
+  c10::cuda::OptionalCUDAGuard guard;
+  if (c10::cuda::current_device() != dev.index()) guard.set_device(dev);
+  if (x.stride(0) != 1 || (reinterpret_cast<uintptr_t>(x.const_data_ptr()) & 15u) != 0) x = x.clone(at::MemoryFormat::Contiguous);
+  at::Tensor out = none(a[2]) ? new_cuda({pk->M}, reinterpret_cast<THPDtype*>(a[3])->scalar_type, dev) : cuda_tensor(a[2], "out");
+  if (out.dim() != 1 || out.size(0) != pk->M || out.stride(0) != 1) fail("out must be a contiguous vector of M elements");
+  void_spmm_args s = pk->args;
+  s.scale_mode = VOID_SCALE_ROW_MEAN;
+  s.b = x.const_data_ptr();
+  s.ldb = (pk->K * es + 15) / 16 * 16;
+  s.N = 1;
+  s.b_scale = 1.0f;
+  s.out = out.data_ptr();
+  s.ldc = pk->M;
+  s.out_dtype = out_code(out.scalar_type());
+  s.transposed = 1;
+  s.flags = pk->stable ? 4 : 0;
+  check(void_spmm_fp(&s, pk->kind, stream_of(dev.index())), "void_spmm_fp");
   if (!none(a[2])) {
     Py_INCREF(a[2]);
     return a[2];
@@ -631,7 +677,7 @@ at::Tensor product_of_values(const Structure& st, bool a_transposed, const at::T
   s.nbc = (int32_t)((K + 31) / 32);
   s.nnz = st.nnz;
   s.b = b.const_data_ptr();
-  s.ldb = b.stride(0) * es;
+  s.ldb = row_pitch(b, es);
   s.K = (int32_t)K;
   s.N = (int32_t)N;
   s.b_scale = 1.0f;
@@ -663,7 +709,7 @@ at::Tensor gradient_of_values(const Structure& st, const at::Tensor& g_in, const
   const at::Tensor x = kernel_operand(as_type(x_in, kind_type(kind)), es);
   at::Tensor grad = new_cuda({st.nnz, 32, 32}, type, dev);   // every stored tile is written
   check((linear ? void_linear_tile_grad : void_spmm_tile_grad)(
-            g.const_data_ptr(), g.stride(0) * es, x.const_data_ptr(), x.stride(0) * es, (int32_t)st.M, (int32_t)st.K, (int32_t)N,
+            g.const_data_ptr(), row_pitch(g, es), x.const_data_ptr(), row_pitch(x, es), (int32_t)st.M, (int32_t)st.K, (int32_t)N,
             kind, st.items.const_data_ptr<int32_t>(), (int32_t)st.items.size(0), st.tile_cols[0].const_data_ptr<int32_t>(),
             st.block_indices[0].const_data_ptr<int32_t>(), grad.data_ptr(), out_code(type), st.status.data_ptr<int32_t>(),
             stream_of(dev.index())),
@@ -766,6 +812,7 @@ PyMethodDef kMethods[] = {
     FAST(packed_made_from),
     FAST(packed_is_current),
     FAST(spmm),
+    FAST(spmv),
     FAST(quant_cols),
     FAST(dense_build),
     FAST(quant_tiles_i8),

@@ -703,6 +703,25 @@ static bool launch_column_sum(const void* in, int64_t ld, int rows, int cols, vo
               : cudaLaunchKernelEx(&cfg, column_sum_kernel<T, false>, src, ld, rows, cols, dst)) == cudaSuccess;
 }
 
+// Rows copied to a pitch of whole 16-byte pieces (what the copy engine reads); one thread per piece of the result.  The
+// padding is written as zeros.
+template <typename T>
+__global__ void __launch_bounds__(256) copy_rows_kernel(const T* __restrict__ in, int64_t ld_in, uint4* __restrict__ out,
+                                                        int64_t pieces, int64_t rows, int cols) {
+  constexpr int E = 16 / (int)sizeof(T);
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (i >= rows * pieces) return;
+  const int64_t r = i / pieces;
+  const int c0 = (int)(i - r * pieces) * E;
+  const T* src = in + r * ld_in + c0;
+  union { uint4 v; T e[E]; } o;
+#pragma unroll
+  for (int k = 0; k < E; ++k) o.e[k] = c0 + k < cols ? src[k] : T(0);
+  out[i] = o.v;
+}
+
 // ------------------------------------------------------------------------------ Stream-K table
 __global__ void __launch_bounds__(1024) streamk_offsets_kernel(const int32_t* __restrict__ row_ptr, int nbr,
                                                                int target, int32_t* __restrict__ woff,
@@ -953,6 +972,34 @@ int void_repack_tiles_fp(const void* values, int32_t elem_bytes, const int32_t* 
     else pack_tiles_fp_kernel<4><<<blocks, tb, 0, st>>>(v, block_indices, nnz, o, TileMeta{});
   }
   return last_status();
+}
+
+int void_copy_rows(const void* in, int64_t ld_in, void* out, int64_t ld_out, int32_t elem_bytes, int64_t rows, int32_t cols,
+                   void_stream_t stream) {
+  if (rows < 0 || cols < 0 || (elem_bytes != 1 && elem_bytes != 2 && elem_bytes != 4)) return VOID_ERR_BAD_ARG;
+  if (rows == 0 || cols == 0) return VOID_OK;
+  if (in == nullptr || out == nullptr) return VOID_ERR_BAD_ARG;
+  if (ld_in % elem_bytes != 0 || ld_out % 16 != 0 || (reinterpret_cast<uintptr_t>(out) & 15u) != 0 ||
+      (reinterpret_cast<uintptr_t>(in) & (uintptr_t)(elem_bytes - 1)) != 0)
+    return VOID_ERR_ALIGN;
+  if (ld_out < (int64_t)cols * elem_bytes) return VOID_ERR_SHAPE;
+  const int64_t pieces = ld_out / 16, blocks = (rows * pieces + 255) / 256;
+  if (blocks > 0x7fffffffLL) return VOID_ERR_TOO_LARGE;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3(256);
+  cfg.stream = as_stream(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  uint4* dst = reinterpret_cast<uint4*>(out);
+  cudaError_t rc;
+  if (elem_bytes == 1) rc = cudaLaunchKernelEx(&cfg, copy_rows_kernel<uint8_t>, reinterpret_cast<const uint8_t*>(in), ld_in, dst, pieces, rows, cols);
+  else if (elem_bytes == 2) rc = cudaLaunchKernelEx(&cfg, copy_rows_kernel<uint16_t>, reinterpret_cast<const uint16_t*>(in), ld_in / 2, dst, pieces, rows, cols);
+  else rc = cudaLaunchKernelEx(&cfg, copy_rows_kernel<uint32_t>, reinterpret_cast<const uint32_t*>(in), ld_in / 4, dst, pieces, rows, cols);
+  return rc == cudaSuccess ? last_status() : VOID_ERR_CUDA;
 }
 
 int void_column_sum(const void* in, int32_t elem, int64_t ld, int32_t rows, int32_t cols, void* out, void_stream_t stream) {

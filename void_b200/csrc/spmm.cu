@@ -52,6 +52,7 @@
 
 #include "../../include/void_b200.h"
 #include "ptx.cuh"
+#include "skinny.cuh"
 
 namespace vb {
 
@@ -1321,6 +1322,23 @@ static void launch_pdl(Kernel kernel, int grid, int threads, int smem_bytes, cud
   cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// Products the kernel for few columns (skinny.cu) takes: plain launches that ask for nothing else, with N at most 16, or
+// with little enough work.  That kernel's time grows with the (tile, 32 columns) pairs, about 0.7 / 0.9 / 1.4 ns each for 8- /
+// 16- / 32-bit tiles; the tensor-memory kernel's with the length of a tile row, which one CTA streams through its ring, about
+// 0.13 / 0.22 / 0.42 us per tile.  The lines were swept at 16 ... 512 tile rows of 2 ... 64 tiles, N = 1 ... 128; at 4096^2,
+// 90 % (13 tiles per row) fp16: N = 8 5.2 us against 9.6, N = 64 6.3 against 7.5, N = 128 10.7 against 7.6; at 16384^2, 90 %
+// (51 tiles) INT8: N = 16 12.9 against 23.8, N = 32 21.6 against 13.9.
+static bool few_columns(const void_spmm_args* a, int kind, int es, bool drain) {
+  if (drain || a->N > kPanelN || a->segs != nullptr || a->acc_out != nullptr || a->worker_partials != nullptr ||
+      a->trace != nullptr || a->n_peers != 0 || a->test_hooks != 0 || a->panels_per_item != 0 || a->stages != 0 || a->grid != 0 ||
+      a->tiles_per_stage != 0 || a->cta_shape != 0 || (a->flags & ~4) != 0)
+    return false;
+  if (a->N <= 16) return true;
+  const long long pairs = a->nnz * ((a->N + 31) / 32), rows = a->nbr > 0 ? a->nbr : 1;
+  if (kind == VOID_KIND_F8E4M3 && a->tile_terms > 1) return pairs * rows < 150 * (a->nnz - 10 * rows);
+  return pairs * rows < (es == 1 ? 180 : 270) * (a->nnz + rows);
+}
+
 static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   if (a == nullptr) return VOID_ERR_BAD_ARG;
   if (a->M < 0 || a->N < 0 || a->K < 0 || a->nbr < 0 || a->nnz < 0) return VOID_ERR_BAD_ARG;
@@ -1355,6 +1373,28 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   if (dev.cc_major != 10) return VOID_ERR_ARCH;
 
   const bool drain = (a->scale_mode == VOID_SCALE_PER_TILE);
+  if (few_columns(a, kind, es, drain)) {
+    SkinnyParams s;
+    s.tiles = reinterpret_cast<const uint8_t*>(a->tiles);
+    s.tile_cols = a->tile_cols;
+    s.row_ptr = a->row_ptr;
+    s.row_scale = a->row_scale;
+    s.b = reinterpret_cast<const uint8_t*>(a->b);
+    s.ldb = a->ldb;
+    s.K = a->K; s.N = a->N; s.M = a->M;
+    s.col_scale = a->col_scale;
+    s.b_scale = a->b_scale;
+    s.bias = a->bias;
+    s.row_bias = a->row_bias;
+    s.out = a->out;
+    s.ldc = a->ldc;
+    s.out_dtype = a->out_dtype;
+    s.act = a->act;
+    s.terms = a->tile_terms == 0 ? 1 : a->tile_terms;
+    s.a_stable = (a->flags & 4) ? 1 : 0;
+    if (s.terms < 1 || s.terms > 3 || (s.terms > 1 && kind != VOID_KIND_F8E4M3)) return VOID_ERR_BAD_ARG;
+    return skinny_launch(s, kind, tr, a->nbr, a->nnz, stream) == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
+  }
   const int total_panels = (a->N + kPanelN - 1) / kPanelN;
   int np = a->panels_per_item;
   if (np != 0 && np != 1 && np != 2 && np != 4) return VOID_ERR_BAD_ARG;

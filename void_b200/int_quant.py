@@ -127,9 +127,11 @@ class Int8VOIDTensor:
 
     def packed(self) -> _spmm.PackedTiles:
         """The tile-row-major packed copy the kernels stream (built once, cached)."""
-        p = _spmm.cached_pack(self, self.values, self.scales, self.block_rows, self.block_cols, self.shape,
-                              _lib.KIND_I8)
-        self._row_ptr, self._block_indices = p.row_ptr, p.block_indices
+        p = self.__dict__.get("_packed_cache")
+        if p is None or not _lib.native().packed_is_current(p.native, self.values, self.scales, self.block_rows,
+                                                            self.block_cols, self.shape):
+            p = _spmm.cached_pack(self, self.values, self.scales, self.block_rows, self.block_cols, self.shape, _lib.KIND_I8)
+            self._row_ptr, self._block_indices = p.row_ptr, p.block_indices
         return p
 
 
@@ -219,18 +221,20 @@ def dequantize_void_tensor(int8_tensor: Int8VOIDTensor):
 
 def _resolve_b(b: torch.Tensor, b_scale):
     """(int8 B, scalar scale, per-column scale tensor or None) from the caller's B and b_scale."""
-    if b.dtype != torch.int8:
+    if b.dtype is not torch.int8:
+        _lib.require_cuda(b)
         # a floating-point B is quantised with one scale for the whole tensor, void/int_quant.py:565-573
         q, scale = _quantize_matrix_per_tensor(b)
         return q, 1.0, scale.expand(b.shape[1])
     if b_scale is None:
         return b, 1.0, None
     if isinstance(b_scale, torch.Tensor):
-        if b_scale.numel() == 1:
+        n = b_scale.numel()
+        if n == 1:
             return b, float(b_scale.item()), None
-        if b_scale.numel() != b.shape[1]:
+        if n != b.shape[1]:
             raise ValueError("b_scale must be a scalar or hold one scale per column of B")
-        return b, 1.0, b_scale.reshape(-1)
+        return b, 1.0, (b_scale if b_scale.dim() == 1 else b_scale.reshape(-1))
     return b, float(b_scale), None
 
 
@@ -245,9 +249,8 @@ def void_spmm_int8(a: Int8VOIDTensor, b: torch.Tensor, b_scale: Union[None, floa
     Returns fp32 [M, N] unless ``out`` / ``out_dtype`` ask for fp16 / bf16.  ``acc_out`` (int32
     [n_block_rows*32, N]) receives the raw int32 accumulators.
     """
-    _lib.require_cuda(a.values, b, out)
-    b_q, scalar, col_scale = _resolve_b(b, b_scale)
     packed = a.packed()
+    b_q, scalar, col_scale = _resolve_b(b, b_scale)
     # every element of out is written by the kernel (zeros for empty tile rows), so the
     # reference's torch.zeros / out.zero_() (:580-583) has no counterpart here
     opts = None if acc_out is None else (None, acc_out, None, 0, 0, 0, 0, 0, None, 0, 0, None, True)

@@ -13,14 +13,16 @@ import torch
 
 from . import _lib, _spmm
 from .format import VOIDTensor
+from .int_quant import Int8VOIDTensor
 
 _KIND_DTYPE = {_lib.KIND_F16: torch.float16, _lib.KIND_BF16: torch.bfloat16, _lib.KIND_TF32: torch.float32}
 
 
 def product_kind(a: VOIDTensor, b: torch.Tensor) -> int:
     """Tensor-core kind for A's tiles and B: their common 16-bit type, else fp32 operands (TF32)."""
-    if a.values.dtype == b.dtype and b.dtype in (torch.float16, torch.bfloat16):
-        return _lib.FP_KIND[b.dtype]
+    dtype = b.dtype
+    if a.values.dtype is dtype and dtype in _lib.FP_KIND:
+        return _lib.FP_KIND[dtype]
     if not (a.values.dtype.is_floating_point and b.dtype.is_floating_point):
         raise _lib.VoidB200Error("void_spmm takes floating-point tiles and a floating-point B, got %s and %s"
                                  % (a.values.dtype, b.dtype))
@@ -29,14 +31,14 @@ def product_kind(a: VOIDTensor, b: torch.Tensor) -> int:
 
 def packed_fp(a: VOIDTensor, kind: int) -> _spmm.PackedTiles:
     """Packed copy of a floating VOIDTensor for ``kind`` (built once per kind, cached on the tensor)."""
-    if tuple(a.tile_size) != (_spmm.TILE, _spmm.TILE):
-        raise NotImplementedError("void_b200 kernels are built for 32x32 tiles, got tile_size=%s" % (a.tile_size,))
-    cache = getattr(a, "_packed_fp_cache", None)
+    cache = a.__dict__.get("_packed_fp_cache")
     if cache is None:
         cache = a._packed_fp_cache = {}
     hit = cache.get(kind)
     if hit is not None and _lib.native().packed_is_current(hit.native, a.values, None, a.block_rows, a.block_cols, a.shape):
         return hit
+    if tuple(a.tile_size) != (_spmm.TILE, _spmm.TILE):
+        raise NotImplementedError("void_b200 kernels are built for 32x32 tiles, got tile_size=%s" % (a.tile_size,))
     vals = a.values if a.values.dtype == _KIND_DTYPE[kind] else a.values.to(_KIND_DTYPE[kind])
     row_ptr, block_indices = getattr(a, "_row_ptr_cache", None), getattr(a, "_block_indices_cache", None)
     if row_ptr is not None and row_ptr.device != a.block_rows.device:
@@ -88,7 +90,6 @@ def void_linear(a, x: torch.Tensor, bias: Optional[torch.Tensor] = None, activat
     they lie in memory.  ``a`` is a floating VOIDTensor (y in x's dtype) or an Int8VOIDTensor (x int8 with
     per-row scales ``x_scale`` [batch], or a float scalar; y fp32 unless ``out_dtype`` / ``out`` say otherwise).
     ``bias`` has one value per output feature."""
-    from .int_quant import Int8VOIDTensor
     assert x.dim() == 2 and x.shape[1] == a.shape[1], f"Dimension mismatch: A is {a.shape}, x is {tuple(x.shape)}"
     _lib.require_cuda(a.values, x)
     M = a.shape[0]
@@ -111,18 +112,23 @@ def void_linear(a, x: torch.Tensor, bias: Optional[torch.Tensor] = None, activat
 
 
 def void_spmv(a: VOIDTensor, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """y = A @ x (void/ops.py:286-349): the one-column case of void_spmm."""
+    """y = A @ x (void/ops.py:286-349): the one-column case of void_spmm, launched as one row of the transposed form,
+    which needs no row pitch and so no copy of x."""
     squeeze_output = False
     if x.dim() == 2 and x.shape[1] == 1:
         x = x.squeeze(1)
         squeeze_output = True
     assert x.dim() == 1, "x must be 1D vector"
     assert a.shape[1] == x.shape[0], f"Dimension mismatch: A is {a.shape}, x is {tuple(x.shape)}"
-    M = a.shape[0]
     if out is not None:
-        assert out.shape == (M,)
-    y = void_spmm(a, x.unsqueeze(1), None if out is None else out.unsqueeze(1))
-    y = y.squeeze(1) if out is None else out
+        assert out.shape == (a.shape[0],)
+    if a.n_blocks == 0 or x.dtype not in _lib.OUT_DTYPE_CODE or (out is not None and out.stride(0) != 1):
+        y = void_spmm(a, x.unsqueeze(1), None if out is None else out.unsqueeze(1)).squeeze(1)
+        y = y if out is None else out
+    else:
+        kind = product_kind(a, x)
+        packed = packed_fp(a, kind)
+        y = _lib.native().spmv(packed.native, x if x.dtype is _KIND_DTYPE[kind] else x.to(_KIND_DTYPE[kind]), out, x.dtype)
     return y.unsqueeze(1) if squeeze_output else y
 
 
