@@ -17,7 +17,8 @@ LIB_PATH = os.path.join(LIB_DIR, "libvoid_b200.so")
 NATIVE_PATH = os.path.join(LIB_DIR, "_native.so")
 SOURCES = ["spmm.cu", "skinny.cu", "prep.cu", "plan.cu", "format.cu", "tile_grad.cu"]
 HOST_SOURCE = os.path.join(CSRC, "host.cpp")
-HEADERS = [os.path.join(CSRC, "ptx.cuh"), os.path.join(CSRC, "skinny.cuh"), os.path.join(HERE, "..", "include", "void_b200.h")]
+HEADERS = [os.path.join(CSRC, h) for h in ("ptx.cuh", "kinds.cuh", "epilogue.cuh", "launch.cuh", "skinny.cuh")] + [
+    os.path.join(HERE, "..", "include", "void_b200.h")]
 
 NVCC_FLAGS = [
     "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",

@@ -51,22 +51,14 @@
 #include <mutex>
 
 #include "../../include/void_b200.h"
+#include "epilogue.cuh"
+#include "kinds.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "skinny.cuh"
 
 namespace vb {
 
-constexpr int kTile = 32;
-constexpr int kTileBytes = 1024;
-constexpr int kPanelN = 128;
-constexpr int kPanelBytes = kTile * kPanelN;  // 4096
-// Bytes per element of the operands of a kind: the 8-bit kinds, fp16 / bf16, fp32 read as TF32.  A tile
-// takes kTileBytes * ES bytes, a 128-column panel kPanelBytes * ES (stored as ES blocks of 32 k-rows x
-// 128 bytes, one swizzle atom wide each), and one (tile, panel) product takes ES MMAs of 32 bytes of k.
-template <int KIND>
-struct Elem {
-  static constexpr int ES = (KIND == VOID_KIND_TF32) ? 4 : ((KIND == VOID_KIND_F16 || KIND == VOID_KIND_BF16) ? 2 : 1);
-};
 constexpr int kMaxStages = 16;
 constexpr int kMaxSlots = 16;
 // Warp roles of a CTA: PW producer warps (0..PW-1) stream tiles and panels, warp PW issues the MMAs
@@ -207,234 +199,10 @@ __device__ __forceinline__ int panels_in_chunk(const SpmmParams& p, int chunk) {
   return left < p.np ? left : p.np;
 }
 
-// GELU in the tanh form written with a sigmoid, void/fusion.py:38-43.  exp and the reciprocal use
-// the hardware approximations (a few ulp; far inside the path's 1e-3 bar): with the full-precision
-// versions this epilogue, run by two warps per scheduler, cost more than the product itself.
-__device__ __forceinline__ float fast_sigmoid(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
-__device__ __forceinline__ float gelu_tanh_sigmoid(float x) {
-  // x * 0.5 * (1 + (2 sigmoid(2u) - 1)) = x * sigmoid(2u),  2u = 1.5957691216 (x + 0.044715 x^3)
-  const float two_u = 1.5957691216f * x * fmaf(0.044715f * x, x, 1.0f);
-  return x * fast_sigmoid(two_u);
-}
-// What an epilogue thread needs to know about C, read from the kernel parameters once.
-struct OutDesc {
-  void* out;
-  long long ldc;
-  void* acc_out;
-  const float* row_bias;  // [M] added per output row before the activation (linear-layer bias), or null
-  int M, N, dtype, act;
-};
 __device__ __forceinline__ OutDesc out_desc(const SpmmParams& p) {
   OutDesc o;
   o.out = p.out; o.ldc = p.ldc; o.acc_out = p.acc_out; o.row_bias = p.row_bias; o.M = p.M; o.N = p.N; o.dtype = p.out_dtype; o.act = p.act;
   return o;
-}
-
-// Store eight finished values of output column n: matrix rows row*32 + m0 .. + 7.
-__device__ __forceinline__ void store8(const OutDesc& o, int row, int n, int m0, float (&v)[8]) {
-  const int r0 = row * kTile + m0;
-  const int rows = o.M - r0;  // rows left below r0
-  if (o.row_bias != nullptr) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (k < rows) v[k] += __ldg(o.row_bias + r0 + k);
-  }
-  switch (o.act) {
-    case VOID_ACT_RELU:
-#pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = fmaxf(v[k], 0.0f);
-      break;
-    case VOID_ACT_GELU:
-#pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = gelu_tanh_sigmoid(v[k]);
-      break;
-    case VOID_ACT_SILU:
-#pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = v[k] * fast_sigmoid(v[k]);
-      break;
-    default:
-      break;
-  }
-  if (o.dtype == VOID_OUT_F16) {
-    __half* dst = reinterpret_cast<__half*>(o.out) + (size_t)r0 * o.ldc + n;
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (k < rows) dst[(size_t)k * o.ldc] = __float2half_rn(v[k]);
-  } else if (o.dtype == VOID_OUT_BF16) {
-    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(o.out) + (size_t)r0 * o.ldc + n;
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (k < rows) dst[(size_t)k * o.ldc] = __float2bfloat16_rn(v[k]);
-  } else {
-    float* dst = reinterpret_cast<float*>(o.out) + (size_t)r0 * o.ldc + n;
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (k < rows) dst[(size_t)k * o.ldc] = v[k];
-  }
-}
-
-// Epilogue of eight raw accumulators of one output column: dequantise, bias, activation, store.
-template <int KIND>
-__device__ __forceinline__ void finish8(const OutDesc& o, int row, int n, int m0, const uint32_t (&r)[8],
-                                        float row_scale, float cs, float bias) {
-  if (n >= o.N) return;
-  if (o.acc_out != nullptr) {
-    uint32_t* a = reinterpret_cast<uint32_t*>(o.acc_out) + ((size_t)row * kTile + m0) * o.N + n;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) a[(size_t)k * o.N] = r[k];
-  }
-  float v[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const float x = (KIND == VOID_KIND_I8) ? __int2float_rn((int)r[k]) : __uint_as_float(r[k]);
-    v[k] = (x * row_scale) * cs + bias;
-  }
-  store8(o, row, n, m0, v);
-}
-
-// Fast epilogue of sixteen raw accumulators of output column n (tile rows m0 .. m0 + 15) straight to C
-// (no raw-accumulator dump, no split row), stores specialised per output type.
-template <int KIND>
-__device__ __forceinline__ void finish16(const OutDesc& o, int row, int n, int m0, const uint32_t* r,
-                                         float row_scale, float cs, float bias) {
-  if (n >= o.N) return;
-  float v[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    const float x = (KIND == VOID_KIND_I8) ? __int2float_rn((int)r[k]) : __uint_as_float(r[k]);
-    v[k] = (x * row_scale) * cs + bias;
-  }
-  const int r0 = row * kTile + m0;
-  const int rows = o.M - r0;
-  if (o.row_bias != nullptr) {
-#pragma unroll
-    for (int k = 0; k < 16; ++k)
-      if (k < rows) v[k] += __ldg(o.row_bias + r0 + k);
-  }
-  if (o.act != VOID_ACT_NONE) {
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      if (o.act == VOID_ACT_GELU) v[k] = gelu_tanh_sigmoid(v[k]);
-      else if (o.act == VOID_ACT_RELU) v[k] = fmaxf(v[k], 0.0f);
-      else v[k] = v[k] * fast_sigmoid(v[k]);
-    }
-  }
-  const size_t first = (size_t)r0 * o.ldc + n;
-  if (o.dtype == VOID_OUT_F16) {
-    __half* dst = reinterpret_cast<__half*>(o.out) + first;
-#pragma unroll
-    for (int k = 0; k < 16; ++k, dst += o.ldc)
-      if (k < rows) *dst = __float2half_rn(v[k]);
-  } else if (o.dtype == VOID_OUT_BF16) {
-    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(o.out) + first;
-#pragma unroll
-    for (int k = 0; k < 16; ++k, dst += o.ldc)
-      if (k < rows) *dst = __float2bfloat16_rn(v[k]);
-  } else {
-    float* dst = reinterpret_cast<float*>(o.out) + first;
-#pragma unroll
-    for (int k = 0; k < 16; ++k, dst += o.ldc)
-      if (k < rows) *dst = v[k];
-  }
-}
-
-// Sixteen finished 16-bit values of output column n into a staging tile [32 m][PITCH n] in shared memory
-// (stage_col points at element [0][n - n0]); same arithmetic as finish16.
-template <int KIND, int PITCH>
-__device__ __forceinline__ void finish16_stage(const OutDesc& o, int row, int n, int m0, const uint32_t* r,
-                                               float row_scale, float cs, float bias, uint16_t* stage_col) {
-  float v[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    const float x = (KIND == VOID_KIND_I8) ? __int2float_rn((int)r[k]) : __uint_as_float(r[k]);
-    v[k] = (x * row_scale) * cs + bias;
-  }
-  const int r0 = row * kTile + m0;
-  const int rows = o.M - r0;
-  if (o.row_bias != nullptr) {
-#pragma unroll
-    for (int k = 0; k < 16; ++k)
-      if (k < rows) v[k] += __ldg(o.row_bias + r0 + k);
-  }
-  if (o.act != VOID_ACT_NONE) {
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      if (o.act == VOID_ACT_GELU) v[k] = gelu_tanh_sigmoid(v[k]);
-      else if (o.act == VOID_ACT_RELU) v[k] = fmaxf(v[k], 0.0f);
-      else v[k] = v[k] * fast_sigmoid(v[k]);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    uint16_t h;
-    if (o.dtype == VOID_OUT_F16) h = __half_as_ushort(__float2half_rn(v[k]));
-    else h = __bfloat16_as_ushort(__float2bfloat16_rn(v[k]));
-    stage_col[(m0 + k) * PITCH] = h;
-  }
-}
-
-// Transposed output (C stored as [N, M], m contiguous): the thread owns output row n and sixteen consecutive
-// columns m0 .. m0 + 15 of it, so the values leave in 16-byte stores.  bias_n is the bias of this n, the
-// per-m bias (o.row_bias) is the same for every thread of the warp.
-template <int KIND>
-__device__ __forceinline__ void finish16_tr(const OutDesc& o, int row, int n, int m0, const uint32_t* r,
-                                            float row_scale, float cs, float bias_n) {
-  if (n >= o.N) return;
-  const int c0 = row * kTile + m0;   // first output column (a row index of A)
-  const int cols = o.M - c0;         // columns left
-  if (cols <= 0) return;
-  float v[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    const float x = (KIND == VOID_KIND_I8) ? __int2float_rn((int)r[k]) : __uint_as_float(r[k]);
-    v[k] = (x * row_scale) * cs + bias_n;
-  }
-  if (o.row_bias != nullptr) {
-#pragma unroll
-    for (int k = 0; k < 16; ++k)
-      if (k < cols) v[k] += __ldg(o.row_bias + c0 + k);
-  }
-  if (o.act != VOID_ACT_NONE) {
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      if (o.act == VOID_ACT_GELU) v[k] = gelu_tanh_sigmoid(v[k]);
-      else if (o.act == VOID_ACT_RELU) v[k] = fmaxf(v[k], 0.0f);
-      else v[k] = v[k] * fast_sigmoid(v[k]);
-    }
-  }
-  const size_t first = (size_t)n * o.ldc + c0;
-  if (o.dtype == VOID_OUT_F32) {
-    float* dst = reinterpret_cast<float*>(o.out) + first;
-    if (cols >= 16 && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
-#pragma unroll
-      for (int k = 0; k < 16; k += 4) *reinterpret_cast<float4*>(dst + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 16; ++k)
-        if (k < cols) dst[k] = v[k];
-    }
-  } else {
-    uint32_t h[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      if (o.dtype == VOID_OUT_F16) {
-        const __half2 t = __floats2half2_rn(v[2 * k], v[2 * k + 1]);
-        h[k] = *reinterpret_cast<const uint32_t*>(&t);
-      } else {
-        const __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-        h[k] = *reinterpret_cast<const uint32_t*>(&t);
-      }
-    }
-    uint16_t* dst = reinterpret_cast<uint16_t*>(o.out) + first;
-    if (cols >= 16 && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
-      *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
-      *reinterpret_cast<uint4*>(dst + 8) = make_uint4(h[4], h[5], h[6], h[7]);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 16; ++k)
-        if (k < cols) dst[k] = (uint16_t)(h[k >> 1] >> ((k & 1) * 16));
-    }
-  }
 }
 
 struct __align__(8) PipeBars {
@@ -565,14 +333,6 @@ __device__ __forceinline__ void producer_loop(const SpmmParams& p, const CUtenso
     }
   }
   if (!waited) grid_dependency_wait();
-}
-
-template <int KIND>
-__device__ __forceinline__ void issue_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  if (KIND == VOID_KIND_I8) mma_i8(d, a, b, idesc, acc);
-  else if (KIND == VOID_KIND_F8E4M3) mma_f8(d, a, b, idesc, acc);
-  else if (KIND == VOID_KIND_TF32) mma_tf32(d, a, b, idesc, acc);
-  else mma_f16(d, a, b, idesc, acc);
 }
 
 // Barriers, tensor memory and the launch of the next kernel's set-up.  Nothing here touches global memory,
@@ -1246,82 +1006,6 @@ __global__ void __launch_bounds__(C::THREADS, (NP == 4) ? 1 : C::CTAS_PER_SM) sp
 // ------------------------------------------------------------------------------------------
 // Host side: tensor map, launch shape, argument checks.
 // ------------------------------------------------------------------------------------------
-static PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
-static std::once_flag g_encode_once;
-
-static PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
-  std::call_once(g_encode_once, [] {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      g_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-  });
-  return g_encode;
-}
-
-struct DeviceInfo {
-  int sms = 0, cc_major = 0, cc_minor = 0, max_smem = 0, smem_per_sm = 0;
-  bool ok = false;
-};
-static DeviceInfo device_info() {
-  static DeviceInfo cache[64];
-  static std::mutex mu;
-  int dev = 0;
-  DeviceInfo none;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return none;
-  std::lock_guard<std::mutex> lock(mu);   // a record is filled and read under the lock: no half-written fields
-  if (!cache[dev].ok) {
-    DeviceInfo d;
-    if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return none;
-    cudaDeviceGetAttribute(&d.cc_major, cudaDevAttrComputeCapabilityMajor, dev);
-    cudaDeviceGetAttribute(&d.cc_minor, cudaDevAttrComputeCapabilityMinor, dev);
-    cudaDeviceGetAttribute(&d.max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaDeviceGetAttribute(&d.smem_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-    d.ok = true;
-    cache[dev] = d;
-  }
-  return cache[dev];
-}
-
-// cudaFuncSetAttribute per (kernel, device), repeated only when a larger ring is asked for.
-// All kernels share one C++ function-pointer type, so the record is keyed by the pointer value.  The table
-// holds every instantiation of this file on up to 16 devices; beyond that the attribute is simply set again
-// on every launch of the pairs that found no room (correct, a little slower).
-static int ensure_smem(const void* kernel, int bytes) {
-  struct Rec { const void* fn; int dev; int bytes; };
-  constexpr int kRecs = 48 * 16;
-  static Rec recs[kRecs];
-  static int n_recs = 0;
-  static std::mutex mu;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return -1;
-  std::lock_guard<std::mutex> lock(mu);
-  Rec* r = nullptr;
-  for (int i = 0; i < n_recs; ++i)
-    if (recs[i].fn == kernel && recs[i].dev == dev) r = &recs[i];
-  if (r != nullptr && r->bytes >= bytes) return 0;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return -1;
-  if (r == nullptr && n_recs < kRecs) r = &recs[n_recs++];
-  if (r != nullptr) { r->fn = kernel; r->dev = dev; r->bytes = bytes; }
-  return 0;
-}
-
-template <typename Kernel, typename... Args>
-static void launch_pdl(Kernel kernel, int grid, int threads, int smem_bytes, cudaStream_t stream, const Args&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = (size_t)smem_bytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // Products the kernel for few columns (skinny.cu) takes: plain launches that ask for nothing else, with N at most 16, or
 // with little enough work.  That kernel's time grows with the (tile, 32 columns) pairs, about 0.7 / 0.9 / 1.4 ns each for 8- /
 // 16- / 32-bit tiles; the tensor-memory kernel's with the length of a tile row, which one CTA streams through its ring, about
@@ -1408,28 +1092,41 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
     }
   }
   const int n_chunks = (total_panels + np - 1) / np;
-  // CTA shape: the slim one (four CTAs per SM) for the row-accumulate kernel with at most two panels
-  // per item; the wide one for the per-tile kernel and for four-panel items (TMEM: 2 x np x 32
-  // columns per row-accumulate CTA, 512 per SM)
+  // CTA shape: the slim one (four CTAs per SM) for the 8-bit row-accumulate kernel with at most two panels per item and for
+  // work plans; the wide one for floating operands without a plan (two CTAs share a ring twice as deep: what a CTA takes
+  // for its row is the row's tiles times the ring's round trip, and a slim ring holds two 32-bit tiles or four 16-bit
+  // ones; 4096^2, 90 %, N = 512: fp32 15.7 -> 13.1 us, fp16 9.1 -> 8.8; 2048^2, 80 %, N = 256 fp32 12.1 -> 8.1), for the
+  // per-tile kernel and for four-panel items (TMEM: 2 x np x 32 columns per row-accumulate CTA, 512 per SM)
   int shape = a->cta_shape;
   if (shape < 0 || shape > 5) return VOID_ERR_BAD_ARG;
   if (tr && np > 2) return VOID_ERR_BAD_ARG;
-  if (tr && shape == 1) return VOID_ERR_BAD_ARG;  // built for the slim shape only
-  if (shape == 0) shape = (!drain && np <= 2) ? 2 : ((drain && np == 1) ? kDefaultDrainShape : 1);
+  if (tr && shape == 1 && kind == VOID_KIND_I8) return VOID_ERR_BAD_ARG;  // (8-bit transposed: the slim shape only)
+  if (shape == 0) shape = (!drain && np <= 2) ? ((floating && np == 1 && a->segs == nullptr) ? 1 : 2) : ((drain && np == 1) ? kDefaultDrainShape : 1);
   if (shape == 2 && (np > 2 || (drain && np > 1))) return VOID_ERR_BAD_ARG;
   if (shape >= 3 && (!drain || np != 1 || tr)) return VOID_ERR_BAD_ARG;  // shapes of the per-tile kernel
   const bool slim = (shape == 2);
   const int producer_warps = (shape == 1) ? Wide::PW : ((shape >= 4) ? 1 : Slim::PW);
   const int ctas_per_sm = (slim || shape == 5) ? 4 : (shape >= 3 ? 3 : ((np == 4) ? 1 : Wide::CTAS_PER_SM));
+  // CTAs that will share an SM: fewer than fit it when there are not enough work items, and each then has more of its
+  // shared memory for the ring
+  int share = ctas_per_sm;
+  if (!drain && a->segs == nullptr && a->grid == 0) {
+    const long long per_sm = ((long long)a->nbr * n_chunks + dev.sms - 1) / dev.sms;
+    if (per_sm < share) share = per_sm < 1 ? 1 : (int)per_sm;
+  }
   int group = a->tiles_per_stage;  // 0 = default
   // What a CTA streams is bounded by the bytes its ring keeps in flight over a stage's round trip, so the defaults fill
-  // the shared memory four CTAs per SM leave each other: nine (tile + panel) units as 3 stages x 3 for one 8-bit panel per
-  // item (swept on B200, headline / 70 % / 16384^2: 2 x 4 units 7.02 / 11.06 / 69.9 us, 3 x 3: 6.76 / 10.21 / 65.1,
-  // 4 x 2: 6.96 / 10.87 / 69.4, 9 x 1: 8.64 / 16.2 / 111); stages of one or two tiles pay the fixed cost of a stage too often
-  if (group == 0) group = (np == 1) ? 3 : 2;
-  if (a->tiles_per_stage == 0 && floating) group = (es == 2 && np == 1) ? 2 : 1;
-  // wider tiles (an FP8 tile stored as two or three terms): 3 stages x 2 (headline 7.66 us, 2 x 3: 7.93)
-  if (a->tiles_per_stage == 0 && a->tile_terms > 1) group = (np == 1) ? 2 : 1;
+  // the shared memory the CTAs of an SM leave each other: nine (tile + panel) units as 3 stages x 3 for one 8-bit panel per
+  // item and four CTAs (swept on B200, headline / 70 % / 16384^2: 2 x 4 units 7.02 / 11.06 / 69.9 us, 3 x 3: 6.76 / 10.21 /
+  // 65.1, 4 x 2: 6.96 / 10.87 / 69.4, 9 x 1: 8.64 / 16.2 / 111); stages of one or two tiles pay the fixed cost of a stage
+  // too often.  With fewer CTAs on the SM longer stages pay (1024 x 8192, 70 %, N = 256, one CTA per SM: INT8 3 x 3 12.4
+  // us, 7 x 6 10.4; FP8 of two terms 17.4 -> 13.3; fp16 21.5 -> 13.4 with 6 x 3; fp32 41.2 -> 25.3 with 8 x 1).
+  if (group == 0) {
+    if (floating) group = (es == 2 && np == 1) ? ((tr && share > 1) || shape == 2 ? 2 : 3) : 1;
+    // (a tile stored as several terms is that much longer: 3 stages x 2 at four CTAs, headline 7.66 us, 2 x 3: 7.93)
+    else if (a->tile_terms > 1) group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 3 : 2)) : 1;
+    else group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 4 : 3)) : 2;
+  }
   if (group < 1 || group > 8) return VOID_ERR_BAD_ARG;
   if (drain && np == 1 && shape != 1 && a->tiles_per_stage == 0) group = 2;
   int drain_tmem = 32;   // the largest power of two that lets ctas_per_sm CTAs share the SM's 512 columns
@@ -1449,10 +1146,10 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   const int staging_bytes = tma_store ? kTile * kPanelN * 2 : 0;
   int stages = a->stages;
   if (stages == 0) {
-    // dynamic shared memory a CTA may use so that ctas_per_sm of them fit an SM: the SM's bytes less the kilobyte
+    // dynamic shared memory a CTA may use so that its share of them fits an SM: the SM's bytes less the kilobyte
     // the system keeps per CTA and the kernel's static variables, less this kernel's 1 KB of slack for alignment
     // and the staging tile
-    const int budget = dev.smem_per_sm / ctas_per_sm - 1024 - 640 - 1024 - staging_bytes;
+    const int budget = dev.smem_per_sm / share - 1024 - 640 - 1024 - staging_bytes;
     stages = budget / stage_bytes;
     if (stages > 8) stages = 8;
   }
@@ -1462,7 +1159,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   // 3 x 2 FP8 tiles of two terms costs more in stage turns than it brings (7.49 against 7.44 us, 13.54 against 13.25)
   int last_group = group;
   if (a->stages == 0 && !drain) {
-    const int budget = dev.smem_per_sm / ctas_per_sm - 1024 - 640 - 1024 - staging_bytes;
+    const int budget = dev.smem_per_sm / share - 1024 - 640 - 1024 - staging_bytes;
     const int left = (budget - stages * stage_bytes) / (stage_bytes / group);
     if (left >= 1 && 5 * left >= stages * group && stages < kMaxStages) {
       last_group = left < group ? left : group;
@@ -1582,64 +1279,19 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
     if (grid < 1) grid = 1;
   }
 
-  // B as a tensor for the copy engine, 128-byte swizzle, zero fill outside [K, N]:
-  //   3-D (N a multiple of 128): dim0 = 128 columns of a panel, dim1 = k, dim2 = panel; box 128 x 32 x np
-  //   2-D (ragged N):            dim0 = n, dim1 = k;                                      box 128 x 32
   CUtensorMap tmap;
   memset(&tmap, 0, sizeof(tmap));
   if (a->nnz > 0) {
-    PFN_cuTensorMapEncodeTiled_v12000 enc = get_encode();
-    if (enc == nullptr) return VOID_ERR_CUDA;
-    CUresult r = CUDA_ERROR_INVALID_VALUE;
-    // elements of es bytes: every box is 128 bytes (kPanelN / es columns) wide, a panel takes es of them
-    const CUtensorMapDataType dt = (es == 1) ? CU_TENSOR_MAP_DATA_TYPE_UINT8
-                                   : (es == 2) ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT32;
-    const int box_n = kPanelN / es;
-    const CUtensorMapSwizzle swz = (es == 4) ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B;
-    if (tr) {
-      //   transposed: dim0 = k, dim1 = n; box 32 k x 128 n, swizzle span = the 32 * es bytes of a row
-      const cuuint64_t gdim[2] = {(cuuint64_t)a->K, (cuuint64_t)a->N};
-      const cuuint64_t gstride[1] = {(cuuint64_t)a->ldb};
-      const cuuint32_t box[2] = {(cuuint32_t)kTile, (cuuint32_t)kPanelN};
-      const cuuint32_t estride[2] = {1, 1};
-      const CUtensorMapSwizzle sw = (es == 4) ? CU_TENSOR_MAP_SWIZZLE_128B
-                                    : (es == 2) ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
-      r = enc(&tmap, dt, 2, const_cast<void*>(a->b), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    } else if (p.use3d) {
-      const cuuint64_t gdim[3] = {(cuuint64_t)box_n, (cuuint64_t)a->K, (cuuint64_t)(a->N / box_n)};
-      const cuuint64_t gstride[2] = {(cuuint64_t)a->ldb, (cuuint64_t)kPanelN};
-      const cuuint32_t box[3] = {(cuuint32_t)box_n, (cuuint32_t)kTile, (cuuint32_t)(np * es)};
-      const cuuint32_t estride[3] = {1, 1, 1};
-      r = enc(&tmap, dt, 3, const_cast<void*>(a->b), gdim, gstride, box, estride,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (r != CUDA_SUCCESS) p.use3d = 0;  // fall back to one 2-D copy per panel
-    }
-    if (!p.use3d && !tr) {
-      const cuuint64_t gdim[2] = {(cuuint64_t)a->N, (cuuint64_t)a->K};
-      const cuuint64_t gstride[1] = {(cuuint64_t)a->ldb};
-      const cuuint32_t box[2] = {(cuuint32_t)box_n, (cuuint32_t)kTile};
-      const cuuint32_t estride[2] = {1, 1};
-      r = enc(&tmap, dt, 2, const_cast<void*>(a->b), gdim, gstride, box, estride,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    }
-    if (r != CUDA_SUCCESS) return VOID_ERR_TENSOR_MAP;
+    bool whole = p.use3d != 0;
+    const bool ok = tr ? panel_map_transposed(&tmap, a->b, a->ldb, a->K, a->N, es) : panel_map(&tmap, a->b, a->ldb, a->K, a->N, es, np, &whole);
+    if (!ok) return VOID_ERR_TENSOR_MAP;
+    p.use3d = whole ? 1 : 0;
   }
 
   CUtensorMap tmap_c;
   memset(&tmap_c, 0, sizeof(tmap_c));
   if (tma_store) {
-    PFN_cuTensorMapEncodeTiled_v12000 enc = get_encode();
-    if (enc == nullptr) return VOID_ERR_CUDA;
-    const cuuint64_t gdim[2] = {(cuuint64_t)a->N, (cuuint64_t)a->M};
-    const cuuint64_t gstride[1] = {(cuuint64_t)a->ldc * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)((a->flags & 16) ? kPanelN : 32), (cuuint32_t)kTile};
-    const cuuint32_t estride[2] = {1, 1};
-    if (enc(&tmap_c, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, a->out, gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return VOID_ERR_TENSOR_MAP;
+    if (!store_map(&tmap_c, a->out, a->ldc, a->M, a->N, (a->flags & 16) ? kPanelN : 32)) return VOID_ERR_TENSOR_MAP;
   }
 
 #define VB_LAUNCH(KERNEL, SHAPE)                                                               \
@@ -1654,7 +1306,9 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   } while (0)
   const bool traced = a->trace != nullptr;
   if (tr) {
-    if (kind == VOID_KIND_TF32) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_TF32, Slim, true>), Slim);
+    if (kind == VOID_KIND_TF32 && !slim) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_TF32, Wide, true>), Wide);
+    else if (kind == VOID_KIND_TF32) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_TF32, Slim, true>), Slim);
+    else if (kind != VOID_KIND_I8 && !slim) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_F16, Wide, true>), Wide);
     else if (kind == VOID_KIND_I8) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_I8, Slim, true>), Slim);
     else VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_F16, Slim, true>), Slim);
   } else if (floating) {
