@@ -170,3 +170,21 @@ def test_products_with_few_columns_are_exact_on_small_integers(dtype, m, k, dens
         void.void_spmv(q, x.cuda().to(dtype), wide[:, 1])                # a result with a stride
         assert torch.equal(wide[:, 1], y)
     void.check_device_status()
+
+
+# ------------------------------------------------------------------------------------------ many tile rows
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,k,n,density", [(3169, 1000, 300, 0.2), (9473, 330, 1100, 0.3), (4800, 1250, 260, 0.5), (2401, 640, 1030, 0.9)])
+def test_products_with_many_tile_rows_are_exact_on_small_integers(dtype, m, k, n, density):
+    dense, gen = _integer_matrix(m, k, density, m + k)
+    a = void.dense_to_void(dense.cuda()).to_dtype(dtype)
+    b = torch.randint(-3, 4, (k, n), generator=gen).float().cuda()
+    ref = dense.cuda().double() @ b.double()
+    bias = torch.randint(-4, 5, (n,), generator=gen).float().cuda()
+    rb = torch.randint(-4, 5, (m,), generator=gen).float().cuda()
+    for _ in range(3):
+        got = void.void_spmm(a, b.to(dtype), bias=bias)
+        assert torch.equal(got.double(), (ref + bias.double()).to(dtype).double())
+        y = void.void_linear(a, b.to(dtype).t().contiguous(), rb, 1)
+        assert torch.equal(y.double(), (ref.t() + rb.double()).clamp(min=0).to(dtype).double())
+    void.check_device_status()

@@ -65,7 +65,8 @@ constexpr int kMaxSlots = 16;
 // and owns the TMEM allocation, EW epilogue warps follow (EW/4 per TMEM lane quadrant, each taking
 // 32/(EW/4) accumulator columns).  Two shapes are built: a wide one (4 + 1 + 8 warps, two CTAs per
 // SM) and a slim one (2 + 1 + 4 warps, four CTAs per SM).  A CTA's stream is bound by the round trip of
-// its ring, so four slim CTAs per SM move more tiles than two wide ones.
+// its ring, so 8-bit tiles move faster through four slim CTAs per SM than through two wide ones, and 16- and 32-bit tiles
+// through two wide CTAs, whose rings are twice as deep.
 template <int PW_, int EW_, int CTAS_>
 struct Shape {
   static constexpr int PW = PW_;
@@ -1096,12 +1097,17 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   // work plans; the wide one for floating operands without a plan (two CTAs share a ring twice as deep: what a CTA takes
   // for its row is the row's tiles times the ring's round trip, and a slim ring holds two 32-bit tiles or four 16-bit
   // ones; 4096^2, 90 %, N = 512: fp32 15.7 -> 13.1 us, fp16 9.1 -> 8.8; 2048^2, 80 %, N = 256 fp32 12.1 -> 8.1), for the
-  // per-tile kernel and for four-panel items (TMEM: 2 x np x 32 columns per row-accumulate CTA, 512 per SM)
+  // per-tile kernel and for four-panel items (TMEM: 2 x np x 32 columns per row-accumulate CTA, 512 per SM).  Short tile
+  // rows of 16-bit tiles are bound by what an item costs besides its stream, which four CTAs hide better where the SM has
+  // more than two items: 16384 x 4096, N = 2048 at 4 / 8 / 13 tiles per row: slim 41 / 53 / 74 us, wide 60 / 67 / 82; N = 512:
+  // 12 / 16.5 / 22.5 against 16 / 18 / 21.9.  Transposed, N = 2048, 4 tiles: 55 against 61, and even from 6 tiles on.
   int shape = a->cta_shape;
   if (shape < 0 || shape > 5) return VOID_ERR_BAD_ARG;
   if (tr && np > 2) return VOID_ERR_BAD_ARG;
   if (tr && shape == 1 && kind == VOID_KIND_I8) return VOID_ERR_BAD_ARG;  // (8-bit transposed: the slim shape only)
-  if (shape == 0) shape = (!drain && np <= 2) ? ((floating && np == 1 && a->segs == nullptr) ? 1 : 2) : ((drain && np == 1) ? kDefaultDrainShape : 1);
+  const long long n_items = (long long)a->nbr * n_chunks;
+  const bool short_rows = es == 2 && n_items > 2ll * dev.sms && a->nnz <= (tr ? 6ll : (n_items > 20ll * dev.sms ? 14ll : 10ll)) * a->nbr;
+  if (shape == 0) shape = (!drain && np <= 2) ? ((floating && np == 1 && a->segs == nullptr && !short_rows) ? 1 : 2) : ((drain && np == 1) ? kDefaultDrainShape : 1);
   if (shape == 2 && (np > 2 || (drain && np > 1))) return VOID_ERR_BAD_ARG;
   if (shape >= 3 && (!drain || np != 1 || tr)) return VOID_ERR_BAD_ARG;  // shapes of the per-tile kernel
   const bool slim = (shape == 2);
