@@ -173,6 +173,10 @@ VOID_API int void_repack_tiles_fp(const void* values, int32_t elem_bytes, const 
  * products need of B (ld_in / ld_out in BYTES, ld_out a multiple of 16); the padding is zeroed. */
 VOID_API int void_copy_rows(const void* in, int64_t ld_in, void* out, int64_t ld_out, int32_t elem_bytes, int64_t rows,
                             int32_t cols, void_stream_t stream);
+/* Transposed copy: out [cols, rows] of in [rows, cols], both row-major with elem_bytes-wide elements (ld_in / ld_out in
+ * BYTES; out on a 16-byte boundary, ld_out a multiple of 16, the padding of its rows zeroed). */
+VOID_API int void_transpose(const void* in, int64_t ld_in, void* out, int64_t ld_out, int32_t elem_bytes, int32_t rows,
+                            int32_t cols, void_stream_t stream);
 /* Column sums of a row-major [rows, cols] matrix of type elem (VOID_ELEM_*), ld elements between rows, accumulated in
  * fp32 in a fixed order, written in the same type: the gradient of a linear layer's bias. */
 VOID_API int void_column_sum(const void* in, int32_t elem, int64_t ld, int32_t rows, int32_t cols, void* out,
@@ -337,7 +341,8 @@ typedef struct void_spmm_args {
    * memory, no transposed copies (the reference transposes both, void/fusion.py:586-598,
    * void/autograd.py:336).  Index meanings are unchanged: col_scale / bias are per n, row_bias per m.
    * Row-accumulate kernel only: not with VOID_SCALE_PER_TILE, FP8, a plan, acc_out or
-   * worker_partials; at most two panels per work item.  0: as described above.               */
+   * worker_partials; at most two panels per work item.  2: C alone is transposed (out [N, M], b [K, N]), with
+   * the same limits.  0: as described above.                                                       */
   int32_t transposed;
   /* 0 for every ordinary launch.  Test hooks: bits 0..15 = limit of every device-side wait in
    * milliseconds (0: the default of 2000); bit 16 = the first group of tiles of each CTA is never

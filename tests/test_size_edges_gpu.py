@@ -188,3 +188,62 @@ def test_products_with_many_tile_rows_are_exact_on_small_integers(dtype, m, k, n
         y = void.void_linear(a, b.to(dtype).t().contiguous(), rb, 1)
         assert torch.equal(y.double(), (ref.t() + rb.double()).clamp(min=0).to(dtype).double())
     void.check_device_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.int8, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,cols,off", [(1, 1, 0), (3, 130, 1), (64, 64, 0), (129, 31, 0), (33, 257, 0), (200, 96, 2)])
+def test_transposed_copies(dtype, rows, cols, off):
+    from void_b200 import _lib
+    es = torch.empty(0, dtype=dtype).element_size()
+    x = torch.randint(-100, 100, (rows, cols + 3), device="cuda").to(dtype)[:, off:off + cols]
+    ld = (rows * es + 15) // 16 * 16 // es
+    out = torch.full((cols + 1, ld), 7, dtype=dtype, device="cuda")
+    _lib.check(_lib.load().void_transpose(x.data_ptr(), x.stride(0) * es, out.data_ptr(), ld * es, es, rows, cols, _lib.stream_ptr(x.device)),
+               "void_transpose")
+    assert torch.equal(out[:cols, :rows], x.t()) and (out[:cols, rows:] == 0).all() and (out[cols] == 7).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.int8, torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,k,n,density", [(4099, 2090, 1100, 0.85), (9000, 4100, 515, 0.5), (1030, 8200, 2050, 0.4)])
+def test_large_linear_layers_are_exact_on_small_integers(dtype, m, k, n, density):
+    dense, gen = _integer_matrix(m, k, density, m + k)
+    a = void.dense_to_void(dense.cuda())
+    x = torch.randint(-3, 4, (n, k), generator=gen).float().cuda()
+    rb = torch.randint(-4, 5, (m,), generator=gen).float().cuda()
+    ref = x.double() @ dense.cuda().double().t()
+    if dtype == torch.int8:
+        q = void.quantize_void_tensor(a)
+        q.values, q.scales = a.values.to(torch.int8), torch.ones_like(q.scales)
+        scale = torch.tensor([1.0, 2.0, 0.5]).repeat(n)[:n].cuda()
+        for _ in range(2):
+            y = void.void_linear(q, x.to(dtype), rb, x_scale=scale)
+            assert torch.equal(y.double(), ref * scale.double()[:, None] + rb.double())
+    else:
+        a = a.to_dtype(dtype)
+        wide = torch.zeros(n, k + 5, dtype=dtype, device="cuda")[:, 1:k + 1]      # rows off 16-byte boundaries
+        wide.copy_(x)
+        for b in (x.to(dtype), wide, wide):
+            y = void.void_linear(a, b, rb, 1)
+            assert torch.equal(y.double(), (ref + rb.double()).clamp(min=0).to(dtype).double())
+        g = torch.randint(-2, 3, (n, m), generator=gen).float().cuda()
+        layer = void.SparseLinear(k, m, a, bias=False)
+        xg = x.to(dtype).requires_grad_(True)
+        layer(xg).backward(g.to(dtype))
+        assert torch.equal(xg.grad.double(), (g.double() @ dense.cuda().double()).to(dtype).double())
+    void.check_device_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,k,n", [(64, 96, 1), (520, 330, 17), (4099, 1290, 129), (9001, 1100, 1500)])
+def test_two_layers_are_exact_on_small_integers(dtype, m, k, n, density=0.3):
+    d1, gen = _integer_matrix(m, k, density, m + k)
+    d2, _ = _integer_matrix(k, m, density, m + n)
+    w1, w2 = (void.dense_to_void(d.cuda()).to_dtype(dtype) for d in (d1, d2))
+    x = torch.randint(-2, 3, (n, k), generator=gen).float().cuda()
+    b1, b2 = (torch.randint(-4, 5, (s,), generator=gen).float().cuda() for s in (m, k))
+    hidden = (x.double() @ d1.cuda().double().t() + b1.double()).clamp(min=0).to(dtype).double()
+    ref = hidden @ d2.cuda().double().t() + b2.double()
+    for _ in range(2):
+        y = void.fused_sparse_mlp(x.to(dtype), w1, w2, "relu", b1, b2)
+        assert y.dtype == dtype and torch.equal(y.double(), ref.to(dtype).double())
+    void.check_device_status()

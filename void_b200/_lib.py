@@ -88,6 +88,7 @@ _PROTOTYPES = {
     "void_linear_tile_grad": (ctypes.c_int, [c_vp, c_i64, c_vp, c_i64, c_i32, c_i32, c_i32, c_i32, c_vp, c_i32, c_vp, c_vp,
                                              c_vp, c_i32, c_vp, c_vp]),
     "void_repack_tiles_fp": (ctypes.c_int, [c_vp, c_i32, c_vp, c_i64, c_i32, c_vp, c_vp]),
+    "void_transpose": (ctypes.c_int, [c_vp, c_i64, c_vp, c_i64, c_i32, c_i32, c_i32, c_vp]),
     "void_copy_rows": (ctypes.c_int, [c_vp, c_i64, c_vp, c_i64, c_i32, c_i64, c_i32, c_vp]),
     "void_column_sum": (ctypes.c_int, [c_vp, c_i32, c_i64, c_i32, c_i32, c_vp, c_vp]),
     "void_spmm_i8_static_scratch": (ctypes.c_int, [ctypes.POINTER(SpmmArgs), c_i32, c_vp]),

@@ -199,6 +199,35 @@ at::Tensor kernel_operand(const at::Tensor& b, int es) {
 int64_t row_pitch(const at::Tensor& b, int es) {
   return b.size(0) == 1 ? (b.size(1) * es + 15) / 16 * 16 : b.stride(0) * es;
 }
+// A linear layer on x [N, K] either reads x as it lies (its 32-element pieces of rows load at a fraction of the rate of
+// whole panels) or has it transposed to [K, N] first and its result written transposed.  The copy costs two passes over x
+// and a launch that nothing overlaps; what it saves grows with the (tile, 128 columns) products: INT8 0.36 ns each (8192^2,
+// N = 1024, 80 %: 73.4 -> 40.6 us), 16 bits 0.1 (70 %: 98.0 -> 92.9; 4096^2, N = 4096, 60 %: 134 -> 127), fp32 no more than
+// the copy takes (8192^2, N = 1024, 50 %: 298.5 against 298.8).
+double copy_saves_ns(int kind, int64_t nnz, int64_t N) {
+  const double per = kind == VOID_KIND_I8 ? 0.36 : (kind == VOID_KIND_TF32 ? 0.0 : 0.1);
+  return per * (double)nnz * (double)((N + 127) / 128);
+}
+double copy_costs_ns(int64_t N, int64_t K, int es) { return 5000.0 + 2.0 * (double)N * (double)K * es / 4500.0; }
+bool copy_pays(int kind, int64_t nnz, int64_t N, int64_t K) {
+  return N > 128 && copy_saves_ns(kind, nnz, N) > copy_costs_ns(N, K, elem_bytes(kind));
+}
+// A matrix with rows on 16-byte boundaries whose contents are to be written.
+at::Tensor pitched(int64_t rows, int64_t cols, at::ScalarType type, int es, c10::Device dev) {
+  const int64_t per16 = 16 / es, ld = (cols + per16 - 1) / per16 * per16;
+  const at::Tensor t = new_cuda({rows, ld}, type, dev);
+  return ld == cols ? t : t.narrow(1, 0, cols);
+}
+at::Tensor transposed_copy(const at::Tensor& x_in, int es) {
+  if (x_in.element_size() != es)
+    fail("B must have " + std::to_string(es) + "-byte elements to match A, got " + c10::toString(x_in.scalar_type()));
+  const at::Tensor x = x_in.stride(1) == 1 && x_in.stride(0) >= x_in.size(1) ? x_in : x_in.contiguous();
+  const at::Tensor out = pitched(x.size(1), x.size(0), x.scalar_type(), es, x.device());
+  check(void_transpose(x.const_data_ptr(), x.stride(0) * es, out.data_ptr(), out.stride(0) * es, es, (int32_t)x.size(0),
+                       (int32_t)x.size(1), stream_of(x.device().index())),
+        "void_transpose");
+  return out;
+}
 at::Tensor fp32_vector(PyObject* o, c10::Device dev, const char* what) {
   const at::Tensor& t = tensor(o, what);
   if (t.scalar_type() == at::kFloat && t.device() == dev && t.is_contiguous()) return t;
@@ -237,7 +266,8 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (out.dim() != 2 || out.size(0) != rows || out.size(1) != cols || out.stride(1) != 1)
       fail("out must be a row-major [" + std::to_string(rows) + ", " + std::to_string(cols) + "] tensor");
   }
-  const at::Tensor b = kernel_operand(b_in, es);
+  const bool copied = tr && none(a[11]) && copy_pays(pk->kind, pk->args.nnz, N, pk->K);
+  const at::Tensor b = copied ? transposed_copy(b_in, es) : kernel_operand(b_in, es);
 
   void_spmm_args s = pk->args;
   const bool per_tile = PyObject_IsTrue(a[4]) == 1;
@@ -266,7 +296,7 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   s.ldc = out.stride(0);
   s.out_dtype = out_code(out.scalar_type());
   s.act = (int32_t)integer(a[9]);
-  s.transposed = tr ? 1 : 0;
+  s.transposed = copied ? 2 : (tr ? 1 : 0);
   // Tile rows taken by falling tile count: measured at the 4096^2 sweep and at 16384^2, INT8 gains 3 - 5 %
   // (6.80 -> 6.58 us at 90 %, 10.33 -> 10.02 at 70 %, 72.7 -> 68.7 at 16384^2); FP8 tiles stored as two terms gain at
   // 90 % (7.88 -> 7.57) and lose at 70 % (13.55 -> 13.76): the balance it buys weighs less, and the scattered order of A
@@ -315,6 +345,54 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!none(a[2])) {
     Py_INCREF(a[2]);
     return a[2];
+  }
+  return THPVariable_Wrap(out);
+  NATIVE_END
+}
+
+// mlp(handle1, handle2, x [N, K], bias1 | None, act, bias2 | None) -> act(x A1^T + b1) A2^T + b2 [N, M2], in x's type
+// The activations in between have the layout that suits the products: [N, M1] where the layers read them as they lie, or
+// [M1, N] where copying x pays, which then serves both layers.
+PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 6) throw torch::TypeError("mlp takes 6 arguments");
+  const PackedObject* pk[2] = {packed_of(a[0]), packed_of(a[1])};
+  const at::Tensor& x = cuda_tensor(a[2], "x");
+  const c10::Device dev = x.device();
+  if (x.dim() != 2 || x.size(1) != pk[0]->K || pk[1]->K != pk[0]->M) fail("shape mismatch between the layers and their input");
+  if (dev.index() != pk[0]->device || dev.index() != pk[1]->device) fail("A and B are on different devices");
+  if (pk[0]->kind != pk[1]->kind || elem_bytes(pk[0]->kind) == 1) fail("mlp takes two floating layers of one type");
+  c10::cuda::OptionalCUDAGuard guard;
+  if (c10::cuda::current_device() != dev.index()) guard.set_device(dev);
+  const int kind = pk[0]->kind, es = elem_bytes(kind);
+  const int64_t N = x.size(0);
+  const bool columns = N > 128 && copy_saves_ns(kind, pk[0]->args.nnz + pk[1]->args.nnz, N) > copy_costs_ns(N, pk[0]->K, es);
+  const void_stream_t st = stream_of(dev.index());
+  at::Tensor in = columns ? transposed_copy(x, es) : kernel_operand(x, es), bias[2], out;
+  for (int layer = 0; layer < 2; ++layer) {
+    const PackedObject* p = pk[layer];
+    void_spmm_args s = p->args;
+    s.scale_mode = VOID_SCALE_ROW_MEAN;
+    s.row_order = p->row_order;
+    s.b = in.const_data_ptr();
+    s.ldb = row_pitch(in, es);
+    s.N = (int32_t)N;
+    s.b_scale = 1.0f;
+    if (!none(a[layer == 0 ? 3 : 5])) {
+      bias[layer] = fp32_vector(a[layer == 0 ? 3 : 5], dev, "bias");
+      if (bias[layer].numel() != p->M) fail("bias must have " + std::to_string(p->M) + " elements, got " + std::to_string(bias[layer].numel()));
+      s.row_bias = bias[layer].const_data_ptr<float>();
+    }
+    if (layer == 1) out = new_cuda({N, p->M}, x.scalar_type(), dev);
+    else out = columns ? pitched(p->M, N, x.scalar_type(), es, dev) : pitched(N, p->M, x.scalar_type(), es, dev);
+    s.out = out.data_ptr();
+    s.ldc = out.stride(0);
+    s.out_dtype = out_code(out.scalar_type());
+    s.act = layer == 0 ? (int32_t)integer(a[4]) : VOID_ACT_NONE;
+    s.transposed = columns ? (layer == 0 ? 0 : 2) : 1;
+    s.flags = p->stable ? 4 : 0;
+    check(void_spmm_fp(&s, kind, st), "void_spmm_fp");
+    in = out;
   }
   return THPVariable_Wrap(out);
   NATIVE_END
@@ -659,10 +737,12 @@ at::Tensor product_of_values(const Structure& st, bool a_transposed, const at::T
   const int kind = common_kind(values_in.scalar_type(), b_in.scalar_type());
   const int es = elem_bytes(kind);
   const at::Tensor values = as_type(values_in, kind_type(kind)).contiguous();
-  const at::Tensor b = kernel_operand(as_type(b_in, kind_type(kind)), es);
   const int64_t M = a_transposed ? st.K : st.M, K = a_transposed ? st.M : st.K;
-  const int64_t N = b.size(linear ? 0 : 1);
-  if (b.size(linear ? 1 : 0) != K) fail("shape mismatch between the sparse matrix and the dense operand");
+  const int64_t N = b_in.size(linear ? 0 : 1);
+  if (b_in.size(linear ? 1 : 0) != K) fail("shape mismatch between the sparse matrix and the dense operand");
+  const bool copied = linear && copy_pays(kind, st.nnz, N, K);
+  const at::Tensor b_typed = as_type(b_in, kind_type(kind));
+  const at::Tensor b = copied ? transposed_copy(b_typed, es) : kernel_operand(b_typed, es);
   at::Tensor out = new_cuda({linear ? N : M, linear ? M : N}, b_in.scalar_type(), dev);
   at::Tensor store = new_cuda({std::max<int64_t>(st.nnz, 1) * 1024 * es + 1024}, at::kByte, dev);
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(store.data_ptr()) + 1023) & ~uintptr_t(1023));
@@ -694,7 +774,7 @@ at::Tensor product_of_values(const Structure& st, bool a_transposed, const at::T
   s.out_dtype = out_code(out.scalar_type());
   s.scale_mode = VOID_SCALE_ROW_MEAN;
   s.status = st.status.data_ptr<int32_t>();
-  s.transposed = linear ? 1 : 0;
+  s.transposed = copied ? 2 : (linear ? 1 : 0);
   check(void_spmm_fp(&s, kind, stream), "void_spmm_fp");
   return out;
 }
@@ -814,6 +894,7 @@ PyMethodDef kMethods[] = {
     FAST(packed_is_current),
     FAST(spmm),
     FAST(spmv),
+    FAST(mlp),
     FAST(quant_cols),
     FAST(dense_build),
     FAST(quant_tiles_i8),

@@ -239,7 +239,7 @@ __device__ __forceinline__ int stage_cap(const SpmmParams& p, int stage) {
 // claims its first ring stage and starts the bulk copy of that stage's tiles BEFORE the wait, while the
 // previous kernel is still draining; only the panels of B - typically that kernel's output - are
 // requested after it.
-template <class C, int ES, bool TR, bool TRACE>
+template <class C, int ES, int TR, bool TRACE>
 __device__ __forceinline__ void producer_loop(const SpmmParams& p, const CUtensorMap* tmap, PipeBars* bars,
                                               uint32_t ring_base, uint32_t stage_bytes, volatile int* ctl,
                                               int lane, int pw) {
@@ -259,7 +259,7 @@ __device__ __forceinline__ void producer_loop(const SpmmParams& p, const CUtenso
     if (i + step < end) seg_next = load_seg(p, i + step);
     const int npan = panels_in_chunk(p, s.chunk);
     const int n0 = s.chunk * p.np * kPanelN;
-    const uint32_t unit_bytes = (uint32_t)((kTileBytes * p.terms + ((p.use3d && !TR) ? p.np : npan) * kPanelBytes) * ES);
+    const uint32_t unit_bytes = (uint32_t)((kTileBytes * p.terms + ((p.use3d && TR != 1) ? p.np : npan) * kPanelBytes) * ES);
     if (TRACE && i == begin && pw == 0 && lane == 0) {
       asm volatile("" ::"r"(s.t1) : "memory");
       stamp<TRACE>(p, 57);   // the row's tile range has arrived
@@ -312,7 +312,7 @@ __device__ __forceinline__ void producer_loop(const SpmmParams& p, const CUtenso
         }
         if (TRACE && i == begin && pw == 0 && lane == 0 && k == 0) stamp<TRACE>(p, 60);   // past the wait on the previous kernel
         if (lane < gcnt && !drop) {
-          if (TR) {
+          if (TR == 1) {
             // B stored transposed ([N, K], k contiguous): one box of 128 rows of n x 32 k per panel
             for (int q = 0; q < npan; ++q)
               tma_load_2d(sbase + panel_off<ES>(p, lane, q), tmap, col * kTile, n0 + q * kPanelN, full);
@@ -404,7 +404,8 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[COLS]
   for (int c = 0; c < COLS; c += 16) tmem_ld_32x16p(taddr + (uint32_t)c, &r[c]);
 }
 
-template <int KIND, class C, bool TR = false, bool TRACE = false>
+// TR: 1 = B and C transposed ([N, K] and [N, M]), 2 = C alone
+template <int KIND, class C, int TR = 0, bool TRACE = false>
 __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel(const __grid_constant__ CUtensorMap tmap_b,
                                                                const __grid_constant__ CUtensorMap tmap_c,
                                                                const __grid_constant__ SpmmParams p) {
@@ -451,7 +452,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
       // one MMA covers 32 bytes of k: 32 / ES k-rows of the panel (8-row groups 1024 bytes apart) and two
       // 16-byte k-chunks of the packed tile (128 bytes apart)
       // (transposed B: the panel is K-major, 32 bytes of k lie inside one row of its swizzle atom)
-      constexpr uint64_t kPanelKStep = TR ? 2 : ((kPanelBytes / ES) >> 4), kTileKStep = 256 >> 4;
+      constexpr uint64_t kPanelKStep = TR == 1 ? 2 : ((kPanelBytes / ES) >> 4), kTileKStep = 256 >> 4;
       int begin, end, step;
       seg_range(p, begin, end, step);
       int stage = 0;
@@ -1014,7 +1015,7 @@ __global__ void __launch_bounds__(C::THREADS, (NP == 4) ? 1 : C::CTAS_PER_SM) sp
 // 90 % (13 tiles per row) fp16: N = 8 5.2 us against 9.6, N = 64 6.3 against 7.5, N = 128 10.7 against 7.6; at 16384^2, 90 %
 // (51 tiles) INT8: N = 16 12.9 against 23.8, N = 32 21.6 against 13.9.
 static bool few_columns(const void_spmm_args* a, int kind, int es, bool drain) {
-  if (drain || a->N > kPanelN || a->segs != nullptr || a->acc_out != nullptr || a->worker_partials != nullptr ||
+  if (drain || a->N > kPanelN || a->transposed == 2 || a->segs != nullptr || a->acc_out != nullptr || a->worker_partials != nullptr ||
       a->trace != nullptr || a->n_peers != 0 || a->test_hooks != 0 || a->panels_per_item != 0 || a->stages != 0 || a->grid != 0 ||
       a->tiles_per_stage != 0 || a->cta_shape != 0 || (a->flags & ~4) != 0)
     return false;
@@ -1037,15 +1038,15 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   if (a->segs != nullptr && a->partials_bytes > 0 && a->n_peers == 0 && (a->partials == nullptr || a->counters == nullptr))
     return VOID_ERR_BAD_ARG;
   if ((long long)a->nbr * kTile < a->M) return VOID_ERR_SHAPE;
-  const bool tr = a->transposed != 0;
-  if (a->transposed != 0 && a->transposed != 1) return VOID_ERR_BAD_ARG;
+  if (a->transposed < 0 || a->transposed > 2) return VOID_ERR_BAD_ARG;
+  const bool tr = a->transposed != 0, tr_b = a->transposed == 1;   // C ([N, M]), and B ([N, K]) with it
   if (a->ldc < (tr ? a->M : a->N)) return VOID_ERR_SHAPE;
   if ((reinterpret_cast<uintptr_t>(a->tiles) & 1023u) != 0) return VOID_ERR_ALIGN;
   if (kind < VOID_KIND_I8 || kind > VOID_KIND_TF32) return VOID_ERR_BAD_ARG;
   const int es = (kind == VOID_KIND_TF32) ? 4 : ((kind == VOID_KIND_F16 || kind == VOID_KIND_BF16) ? 2 : 1);
   const bool floating = es > 1;
   if ((reinterpret_cast<uintptr_t>(a->b) & 15u) != 0 || (a->ldb & 15) != 0 ||
-      a->ldb < (long long)(tr ? a->K : a->N) * es)
+      a->ldb < (long long)(tr_b ? a->K : a->N) * es)
     return VOID_ERR_ALIGN;
   // transposed operands: row-accumulate kernel without a plan or raw-accumulator outputs
   if (tr && (kind == VOID_KIND_F8E4M3 || a->scale_mode != VOID_SCALE_ROW_MEAN || a->segs != nullptr ||
@@ -1106,7 +1107,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   if (tr && np > 2) return VOID_ERR_BAD_ARG;
   if (tr && shape == 1 && kind == VOID_KIND_I8) return VOID_ERR_BAD_ARG;  // (8-bit transposed: the slim shape only)
   const long long n_items = (long long)a->nbr * n_chunks;
-  const bool short_rows = es == 2 && n_items > 2ll * dev.sms && a->nnz <= (tr ? 6ll : (n_items > 20ll * dev.sms ? 14ll : 10ll)) * a->nbr;
+  const bool short_rows = es == 2 && n_items > 2ll * dev.sms && a->nnz <= (tr_b ? 6ll : (n_items > 20ll * dev.sms ? 14ll : 10ll)) * a->nbr;
   if (shape == 0) shape = (!drain && np <= 2) ? ((floating && np == 1 && a->segs == nullptr && !short_rows) ? 1 : 2) : ((drain && np == 1) ? kDefaultDrainShape : 1);
   if (shape == 2 && (np > 2 || (drain && np > 1))) return VOID_ERR_BAD_ARG;
   if (shape >= 3 && (!drain || np != 1 || tr)) return VOID_ERR_BAD_ARG;  // shapes of the per-tile kernel
@@ -1128,7 +1129,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   // too often.  With fewer CTAs on the SM longer stages pay (1024 x 8192, 70 %, N = 256, one CTA per SM: INT8 3 x 3 12.4
   // us, 7 x 6 10.4; FP8 of two terms 17.4 -> 13.3; fp16 21.5 -> 13.4 with 6 x 3; fp32 41.2 -> 25.3 with 8 x 1).
   if (group == 0) {
-    if (floating) group = (es == 2 && np == 1) ? ((tr && share > 1) || shape == 2 ? 2 : 3) : 1;
+    if (floating) group = (es == 2 && np == 1) ? ((tr_b && share > 1) || shape == 2 ? 2 : 3) : 1;
     // (a tile stored as several terms is that much longer: 3 stages x 2 at four CTAs, headline 7.66 us, 2 x 3: 7.93)
     else if (a->tile_terms > 1) group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 3 : 2)) : 1;
     else group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 4 : 3)) : 2;
@@ -1228,7 +1229,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   p.group = group;
   p.stages = stages;
   p.last_group = last_group;
-  p.use3d = (!tr && a->N % (kPanelN / es) == 0) ? 1 : 0;
+  p.use3d = (!tr_b && a->N % (kPanelN / es) == 0) ? 1 : 0;
   p.tmem_cols = drain_tmem;
   p.tma_store = tma_store ? ((a->flags & 16) ? 1 : 2) : 0;   // 2: one store per epilogue warp; 1: one per tile
   p.n_items = a->nbr * n_chunks;
@@ -1266,8 +1267,8 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   }
   // Transposed B ([N, K], k contiguous) is a K-major operand: rows of 32 * es bytes (one swizzle span of 32,
   // 64 or 128 bytes), groups of 8 rows 256 * es bytes apart.
-  const uint32_t a_mn = tr ? 0u : 1u;
-  if (tr) p.desc_hi_a = smem_desc_hi(16, 256 * es, es == 4 ? kLayoutSw128 : (es == 2 ? kLayoutSw64 : kLayoutSw32));
+  const uint32_t a_mn = tr_b ? 0u : 1u;
+  if (tr_b) p.desc_hi_a = smem_desc_hi(16, 256 * es, es == 4 ? kLayoutSw128 : (es == 2 ? kLayoutSw64 : kLayoutSw32));
   if (kind == VOID_KIND_I8) p.idesc = instr_desc(/*c s32*/ 2, /*a s8*/ 1, /*b s8*/ 1, a_mn, /*b K*/ 0, 128, 32);
   else if (kind == VOID_KIND_F8E4M3) p.idesc = instr_desc(/*c f32*/ 1, /*a e4m3*/ 0, /*b e4m3*/ 0, a_mn, 0, 128, 32);
   else if (kind == VOID_KIND_F16) p.idesc = instr_desc(1, /*a f16*/ 0, /*b f16*/ 0, a_mn, 0, 128, 32);
@@ -1289,7 +1290,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   memset(&tmap, 0, sizeof(tmap));
   if (a->nnz > 0) {
     bool whole = p.use3d != 0;
-    const bool ok = tr ? panel_map_transposed(&tmap, a->b, a->ldb, a->K, a->N, es) : panel_map(&tmap, a->b, a->ldb, a->K, a->N, es, np, &whole);
+    const bool ok = tr_b ? panel_map_transposed(&tmap, a->b, a->ldb, a->K, a->N, es) : panel_map(&tmap, a->b, a->ldb, a->K, a->N, es, np, &whole);
     if (!ok) return VOID_ERR_TENSOR_MAP;
     p.use3d = whole ? 1 : 0;
   }
@@ -1311,12 +1312,18 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
     launch_pdl(KERNEL, grid, SHAPE::THREADS, smem_bytes, stream, tmap, tmap_c, p);            \
   } while (0)
   const bool traced = a->trace != nullptr;
-  if (tr) {
-    if (kind == VOID_KIND_TF32 && !slim) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_TF32, Wide, true>), Wide);
-    else if (kind == VOID_KIND_TF32) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_TF32, Slim, true>), Slim);
-    else if (kind != VOID_KIND_I8 && !slim) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_F16, Wide, true>), Wide);
-    else if (kind == VOID_KIND_I8) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_I8, Slim, true>), Slim);
-    else VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_F16, Slim, true>), Slim);
+#define VB_LAUNCH_TR(TR)                                                                                              \
+  do {                                                                                                                \
+    if (kind == VOID_KIND_I8) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_I8, Slim, TR>), Slim);                   \
+    else if (kind == VOID_KIND_TF32 && slim) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_TF32, Slim, TR>), Slim);  \
+    else if (kind == VOID_KIND_TF32) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_TF32, Wide, TR>), Wide);          \
+    else if (slim) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_F16, Slim, TR>), Slim);                             \
+    else VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_F16, Wide, TR>), Wide);                                       \
+  } while (0)
+  if (tr_b) {
+    VB_LAUNCH_TR(1);
+  } else if (tr) {
+    VB_LAUNCH_TR(2);
   } else if (floating) {
     if (kind == VOID_KIND_TF32) {
       if (slim) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_TF32, Slim>), Slim);
@@ -1327,7 +1334,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
     }
   } else if (!drain) {
     if (kind == VOID_KIND_I8) {
-      if (slim && traced) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_I8, Slim, false, true>), Slim);
+      if (slim && traced) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_I8, Slim, 0, true>), Slim);
       else if (slim) VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_I8, Slim>), Slim);
       else VB_LAUNCH_ROWACC((spmm_rowacc_kernel<VOID_KIND_I8, Wide>), Wide);
     } else {
@@ -1357,6 +1364,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   }
 #undef VB_LAUNCH
 #undef VB_LAUNCH_ROWACC
+#undef VB_LAUNCH_TR
   return cudaGetLastError() == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
 }
 

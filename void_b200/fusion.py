@@ -20,7 +20,7 @@ from . import _lib
 from .format import VOIDTensor
 from .fp8 import FP8VOIDTensor, void_spmm_fp8
 from .int_quant import Int8VOIDTensor, void_spmm_int8
-from .ops import void_linear, void_spmm
+from .ops import _KIND_DTYPE, packed_fp, product_kind, void_linear, void_spmm
 
 
 class FusedOpType(Enum):
@@ -108,11 +108,20 @@ def _void_spmm_activation_row_bias(a, b: torch.Tensor, bias: Optional[torch.Tens
 def fused_sparse_mlp(x: torch.Tensor, w1: VOIDTensor, w2: VOIDTensor, activation: str = "gelu",
                      bias1: Optional[torch.Tensor] = None, bias2: Optional[torch.Tensor] = None) -> torch.Tensor:
     """y = W2 @ activation(W1 @ x + b1) + b2 for x of shape [*, in_features] (void/fusion.py:557-602): two
-    launches, each with its bias and activation fused.  Activations stay [batch, features] throughout
-    (void_linear): none of the reference's three transposes is made."""
+    launches, each with its bias and activation fused.  Activations stay [batch, features] (void_linear), or, where
+    the layers are large enough to pay for one transposed copy of x, [features, batch] up to the result, which the
+    second product writes transposed: the reference makes three transposes."""
     code = get_activation_code(activation)
     if code > _lib.ACT_SILU:
         raise NotImplementedError("activation %r is not fused on B200 (none, relu, gelu, silu are)" % activation)
+    if isinstance(w1, VOIDTensor) and isinstance(w2, VOIDTensor) and x.is_cuda and x.dtype in _lib.OUT_DTYPE_CODE:
+        kind, (m1, k1), (m2, k2) = product_kind(w1, x), w1.shape, w2.shape
+        if (_KIND_DTYPE[kind] is x.dtype and product_kind(w2, x) == kind and x.dim() >= 2 and x.shape[-1] == k1 and m1 == k2
+                and (bias1 is None or bias1.shape == (m1,)) and (bias2 is None or bias2.shape == (m2,))):
+            y = _lib.native().mlp(packed_fp(w1, kind).native, packed_fp(w2, kind).native,
+                                  x if x.dim() == 2 else x.reshape(-1, k1), bias1, code, bias2)
+            return y if x.dim() == 2 else y.reshape(x.shape[:-1] + (m2,))
+    # mixed types, and the operands that an error has to be raised for
     hidden = void_linear(w1, x if x.dim() == 2 else x.reshape(-1, x.shape[-1]), bias1, code)
     out = void_linear(w2, hidden, bias2, 0)
     return out if x.dim() == 2 else out.reshape(x.shape[:-1] + (out.shape[-1],))
