@@ -369,7 +369,6 @@ __device__ __forceinline__ void pipeline_setup(const SpmmParams& p, const CUtens
     tmem_alloc(smem_u32(tmem_base_s), tmem_cols);
     tmem_relinquish();
   }
-  grid_launch_dependents();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -379,6 +378,10 @@ __device__ __forceinline__ void pipeline_setup(const SpmmParams& p, const CUtens
 template <class C, bool TRACE>
 __device__ __forceinline__ void pipeline_teardown(const SpmmParams& p, int* ctl_s, uint32_t tmem_base,
                                                   uint32_t tmem_cols) {
+  // The next kernel may start when every CTA is through with its work: started with this one, it settles beside CTAs that
+  // have yet to come, on few SMs, and keeps that placement (graphs of launches, 4096^2, N = 512: fp32 90 % 13.1 -> 12.8 us,
+  // its transposed form 14.1 -> 13.1; INT8 16384^2, 95 % 21.7 -> 20.6; not at all early: 15.5 and 23.5).
+  grid_launch_dependents();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
