@@ -386,6 +386,30 @@ typedef struct void_spmm_args {
   const int32_t* row_order;
 } void_spmm_args;
 
+/* ---------------------------------------------------------------------------------------
+ * Products of groups of tile rows that share B's panels, for large products.  The tiles of up to 8 tile rows are laid
+ * out in the order their block columns meet B: stages of at most max_entries block columns and max_tiles tiles, each a
+ * 128-byte header followed by its tiles.  void_group_build makes that store from a packed one (void_pack_tiles,
+ * void_pack_tiles_fp; tile_bytes = 1024 * element bytes):
+ *   group_rows [n_groups * 16], stage_ptr [n_groups + 1], records [8 * nnz], blob (nnz * (tile_bytes + 128) bytes,
+ *   128-byte aligned), ws [2 * n_groups + nnz]; row_order as in void_spmm_args (rows are dealt to the groups in that order
+ *   back and forth), or NULL; n_groups * 16 >= nbr and ceil(nbr / n_groups) <= 8, <= max_tiles <= 16; max_entries <= 6.
+ * void_spmm_grouped multiplies it: args as for void_spmm_i8 / _fp (tiles, tile_cols and tile_scales are not read; no
+ * plan, no raw accumulators); args->transposed 0 or 2.
+ * ------------------------------------------------------------------------------------- */
+typedef struct void_group_store {
+  const void* blob;
+  const int32_t* records;
+  const int32_t* stage_ptr;
+  const int32_t* group_rows;
+  int32_t n_groups, max_entries, max_tiles, reserved;
+} void_group_store;
+VOID_API int void_group_build(const int32_t* row_ptr, const int32_t* row_order, const int32_t* tile_cols, const void* tiles,
+                              int32_t nbr, int64_t nnz, int32_t elem_bytes, int32_t n_groups,
+                              int32_t max_entries, int32_t max_tiles, int32_t* group_rows, int32_t* stage_ptr, int32_t* records, void* blob,
+                              int32_t* ws, void_stream_t stream);
+VOID_API int void_spmm_grouped(const void_spmm_args* args, const void_group_store* store, int32_t kind, void_stream_t stream);
+
 VOID_API int void_spmm_i8(const void_spmm_args* args, void_stream_t stream);
 VOID_API int void_spmm_f8(const void_spmm_args* args, void_stream_t stream);
 

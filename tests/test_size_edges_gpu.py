@@ -247,3 +247,72 @@ def test_two_layers_are_exact_on_small_integers(dtype, m, k, n, density=0.3):
         y = void.fused_sparse_mlp(x.to(dtype), w1, w2, "relu", b1, b2)
         assert y.dtype == dtype and torch.equal(y.double(), ref.to(dtype).double())
     void.check_device_status()
+
+
+# ------------------------------------------------------------------------------------------ groups of tile rows
+@pytest.mark.parametrize("kind,dtype,out", [("I8", torch.int8, torch.float32), ("I8", torch.int8, torch.float16),
+                                            ("I8", torch.int8, torch.bfloat16), ("F16", torch.float16, torch.float16),
+                                            ("BF16", torch.bfloat16, torch.bfloat16), ("TF32", torch.float32, torch.float32)])
+@pytest.mark.parametrize("m,k,n,density,groups,entries,tiles", [
+    (40, 70, 40, 0.9, 1, 1, 2), (250, 300, 129, 0.6, 1, 1, 8), (2500, 333, 384, 0.4, 12, 2, 8), (1111, 2000, 200, 0.95, 18, 1, 2),
+    (10000, 640, 515, 0.1, 60, 2, 16)])
+def test_grouped_products_are_exact_on_small_integers(kind, dtype, out, m, k, n, density, groups, entries, tiles):
+    import ctypes
+    from void_b200 import _lib, _spmm
+    lib, kd = _lib.load(), getattr(_lib, "KIND_" + kind)
+    dense, gen = _integer_matrix(m, k, density, m + n)
+    a = void.dense_to_void(dense.cuda())
+    vals = a.values.to(dtype)
+    p = _spmm._mark_ready(_spmm.pack(vals, torch.ones(a.n_blocks, device="cuda") if kd == _lib.KIND_I8 else None, a.block_rows,
+                                     a.block_cols, (m, k), kd))
+    es, P = vals.element_size(), _lib.ptr
+    if es == 4:                                                           # (two stages have to fit a CTA's shared memory)
+        entries, tiles = 1, (p.nbr + groups - 1) // groups
+    ints = dict(dtype=torch.int32, device="cuda")
+    rows, stages = torch.empty(groups * 16, **ints), torch.empty(groups + 1, **ints)
+    records, ws = torch.empty(8 * p.nnz, **ints), torch.empty(2 * groups + p.nnz, **ints)
+    blob = torch.empty(p.nnz * (1024 * es + 128), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.void_group_build(P(p.row_ptr), P(p.row_order), P(p.tile_cols), P(p.tiles), p.nbr, p.nnz, es, groups, entries,
+                                    tiles, P(rows), P(stages), P(records), P(blob), P(ws), _lib.stream_ptr(blob.device)), "void_group_build")
+    s = _lib.GroupStore(blob.data_ptr(), records.data_ptr(), stages.data_ptr(), rows.data_ptr(), groups, entries, tiles, 0)
+    ld = (n * es + 15) // 16 * 16 // es
+    b = torch.zeros(k, ld, dtype=dtype, device="cuda")[:, :n]
+    x = torch.randint(-3, 4, (k, n), generator=gen).float().cuda()
+    b.view(torch.uint8).copy_(x.to(dtype).view(torch.uint8)) if es == 1 else b.copy_(x)
+    bias, rb = (torch.randint(-4, 5, (z,), generator=gen).float().cuda() for z in (n, m))
+    ref = (dense.cuda().double() @ x.double() + bias.double() + rb.double()[:, None]).clamp(min=0).to(out)
+    for tr in (0, 2):
+        c = torch.empty(n, m, dtype=out, device="cuda") if tr else torch.empty(m, n, dtype=out, device="cuda")
+        g = _lib.SpmmArgs()
+        g.row_ptr, g.row_scale = p.row_ptr.data_ptr(), p.row_scale.data_ptr() if es == 1 else None
+        g.nbr, g.nbc, g.nnz, g.tile_terms = p.nbr, p.nbc, p.nnz, 1
+        g.b, g.ldb, g.K, g.N, g.b_scale = b.data_ptr(), ld * es, k, n, 1.0
+        g.out, g.ldc, g.M, g.out_dtype, g.act, g.transposed = c.data_ptr(), c.stride(0), m, _lib.OUT_DTYPE_CODE[out], 1, tr
+        g.bias, g.row_bias, g.status = bias.data_ptr(), rb.data_ptr(), _lib.status_word(c.device).data_ptr()
+        _lib.check(lib.void_spmm_grouped(ctypes.byref(g), ctypes.byref(s), kd, _lib.stream_ptr(c.device)), "void_spmm_grouped")
+        assert torch.equal(c.t() if tr else c, ref), tr
+    void.check_device_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.int8, torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m,k,density", [(9473, 700, 0.5), (5000, 1930, 0.9)])
+def test_repeated_products_of_dense_tensors_stay_the_same(dtype, m, k, density):
+    dense, gen = _integer_matrix(m, k, density, m + k)
+    a = void.dense_to_void(dense.cuda())
+    if dtype == torch.int8:
+        q = void.quantize_void_tensor(a)
+        q.values, q.scales = a.values.to(torch.int8), torch.ones_like(q.scales)
+    else:
+        q = a.to_dtype(dtype)
+    for n in (1500, 520, 1030, 1500):
+        x = torch.randint(-3, 4, (k, n), generator=gen).float().cuda()
+        ref = dense.cuda().double() @ x.double()
+        for _ in range(4):
+            if dtype == torch.int8:
+                assert torch.equal(void.void_spmm_int8(q, x.to(dtype), 1.0, out_dtype=torch.float32).double(), ref)
+                y = void.void_linear(q, x.t().contiguous().to(dtype))
+            else:
+                assert torch.equal(void.void_spmm(q, x.to(dtype)).double(), ref.to(dtype).double())
+                y = void.void_linear(q, x.t().contiguous().to(dtype))
+            assert torch.equal(y.double(), ref.t().to(y.dtype).double())
+    void.check_device_status()

@@ -49,6 +49,12 @@ class SpmmArgs(ctypes.Structure):
     ]
 
 
+class GroupStore(ctypes.Structure):
+    """Mirror of ``struct void_group_store``."""
+    _fields_ = [("blob", c_vp), ("records", c_vp), ("stage_ptr", c_vp), ("group_rows", c_vp), ("n_groups", c_i32),
+                ("max_entries", c_i32), ("max_tiles", c_i32), ("reserved", c_i32)]
+
+
 _PROTOTYPES = {
     "void_strerror": (ctypes.c_char_p, [ctypes.c_int]),
     "void_b200_abi_version": (ctypes.c_int, []),
@@ -83,6 +89,8 @@ _PROTOTYPES = {
     "void_spmm_i8": (ctypes.c_int, [ctypes.POINTER(SpmmArgs), c_vp]),
     "void_spmm_f8": (ctypes.c_int, [ctypes.POINTER(SpmmArgs), c_vp]),
     "void_spmm_fp": (ctypes.c_int, [ctypes.POINTER(SpmmArgs), c_i32, c_vp]),
+    "void_group_build": (ctypes.c_int, [c_vp, c_vp, c_vp, c_vp, c_i32, c_i64, c_i32, c_i32, c_i32, c_i32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "void_spmm_grouped": (ctypes.c_int, [ctypes.POINTER(SpmmArgs), ctypes.POINTER(GroupStore), c_i32, c_vp]),
     "void_spmm_tile_grad": (ctypes.c_int, [c_vp, c_i64, c_vp, c_i64, c_i32, c_i32, c_i32, c_i32, c_vp, c_i32, c_vp, c_vp,
                                            c_vp, c_i32, c_vp, c_vp]),
     "void_linear_tile_grad": (ctypes.c_int, [c_vp, c_i64, c_vp, c_i64, c_i32, c_i32, c_i32, c_i32, c_vp, c_i32, c_vp, c_vp,

@@ -15,7 +15,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libvoid_b200.so")
 NATIVE_PATH = os.path.join(LIB_DIR, "_native.so")
-SOURCES = ["spmm.cu", "skinny.cu", "prep.cu", "plan.cu", "format.cu", "tile_grad.cu"]
+SOURCES = ["spmm.cu", "skinny.cu", "group.cu", "prep.cu", "plan.cu", "format.cu", "tile_grad.cu"]
 HOST_SOURCE = os.path.join(CSRC, "host.cpp")
 HEADERS = [os.path.join(CSRC, h) for h in ("ptx.cuh", "kinds.cuh", "epilogue.cuh", "launch.cuh", "skinny.cuh")] + [
     os.path.join(HERE, "..", "include", "void_b200.h")]

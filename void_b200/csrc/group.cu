@@ -1,0 +1,586 @@
+// Products of groups of tile rows that share B's panels:  C = act(dequant(A . B) + bias).
+//
+// The row-accumulate kernel of spmm.cu fetches a panel of B for every stored tile.  Its large products run at what an SM
+// takes in from L2 - measured 66 - 76 bytes per clock with every SM loading, whatever else it does - so only fewer bytes
+// make them faster.  Here a CTA (two per SM) owns up to eight tile rows at once, their accumulators for a panel of 128
+// columns in tensor memory, and walks the block columns that ANY of its rows stores: a panel is fetched once and multiplied
+// by the 1 ... R tiles of that column.  With density d a panel serves R d / (1 - (1 - d)^R) tiles: 1.3 at 90 % sparsity and
+// R = 7, 2.3 at 70 %, 3.5 at 50 %.  Measured against that kernel, 8192^2, N = 1024, us: fp16 50 % 132 -> 95, 70 % 84 -> 66,
+// 80 % 59 -> 53; fp32 50 % 261 -> 212, 70 % 163 -> 153; INT8 50 % 74 -> 54, 70 % 48 -> 39; slower from 90 % on.  What is left is
+// the issue of the products: one thread spends about 60 clocks on each and 240 - 490 per stage, against the tensor cores' 40 -
+// 64; two warps on alternate rows and two CTAs per SM hide most of it.
+//
+// The packed tiles are laid out in the order the CTA uses them: stages of up to E block columns and T tiles, a 128-byte
+// header (per MMA warp its tiles: accumulator, panel, whether it is the row's first) followed by the tiles, so that one bulk
+// copy brings header and tiles, and E tensor copies the panels.  Groups are made of rows of falling length dealt out back and
+// forth, so that they hold nearly the same number of tiles.
+//
+// Roles as in spmm.cu: two producer warps take the stages in turn, two warps issue the MMAs of alternate rows, four warps
+// finish rows, one per lane quadrant of tensor memory.  Every wait is bounded.
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cudaTypedefs.h>
+
+#include "../../include/void_b200.h"
+#include "epilogue.cuh"
+#include "kinds.cuh"
+#include "launch.cuh"
+#include "ptx.cuh"
+
+namespace vb {
+
+namespace {
+
+constexpr int kCtas = 2, kProducers = 2, kMmaWarps = 2, kMmaWarp0 = 2, kEpiWarp0 = 4, kEpiWarps = 4;
+constexpr int kMaxRows = 512 / kCtas / 32;   // tile rows of a group whose accumulators fit a CTA's tensor memory
+constexpr int kMaxGroupRows = 16;             // and the places group_rows has for them
+constexpr int kMaxEntries = 6;       // block columns per stage (what a record holds)
+constexpr int kMaxStageTiles = 16;   // tiles per stage (what a header holds)
+constexpr int kHeaderBytes = 128;   // per MMA warp: a word (first tile | tiles << 8), then its tiles' words
+constexpr int kClassWords = 32 / kMmaWarps;
+constexpr int kMaxRing = 12;
+constexpr int kThreads = 32 * (kProducers + kMmaWarps + kEpiWarps);
+constexpr int kNone = 0x7fffffff;
+
+constexpr int kPartPitch = 40, kPartBytes = 32 * kPartPitch * 2;   // staging of a 32 x 32 part, rows 80 bytes apart
+
+struct GroupParams {
+  const uint8_t* blob;
+  const int32_t* records;      // 8 per stage: blob offset / 128, tiles | entries << 8, block columns
+  const int32_t* stage_ptr;    // [groups + 1]
+  const int32_t* group_rows;   // [groups][16]: tile rows, -1 for none
+  const int32_t* row_ptr;
+  const float* row_scale;
+  const float* col_scale;
+  const float* bias;
+  float b_scale;
+  OutDesc out;
+  int32_t* status;
+  int n_groups, n_chunks, n_items, rows;
+  int panel_bytes;             // panels of a stage (their tiles follow)
+  int stage_bytes, stages;
+  int use3d, staged, out_tr, a_stable;
+  int wait_limit_ms;
+  unsigned long long desc_hi_a, desc_hi_b;
+  unsigned int idesc;
+};
+
+struct __align__(8) Bars {
+  uint64_t full[kMaxRing], empty[kMaxRing];
+  uint64_t acc_full[2], acc_empty[2];
+};
+
+template <int KIND>
+__global__ void __launch_bounds__(kThreads, kCtas) group_kernel(const __grid_constant__ CUtensorMap tmap_b,
+                                                            const __grid_constant__ GroupParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ Bars bars;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int ctl_s[2];   // abort flag, wait limit in ms
+  __shared__ int ok_s[2];
+  constexpr int ES = Elem<KIND>::ES;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  volatile int* ctl = ctl_s;
+  const int buf_cols = p.rows * 32;
+  const int n_buf = 2 * buf_cols <= 512 / kCtas ? 2 : 1;
+  uint32_t tmem_cols = 32;
+  while ((int)tmem_cols < n_buf * buf_cols) tmem_cols <<= 1;
+
+  if (threadIdx.x == 0) {
+    ctl_s[0] = 0;
+    ctl_s[1] = p.wait_limit_ms;
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(smem_u32(&bars.full[s]), 1);
+      mbar_init(smem_u32(&bars.empty[s]), kMmaWarps);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&bars.acc_full[b]), kMmaWarps);
+      mbar_init(smem_u32(&bars.acc_empty[b]), kEpiWarps);
+    }
+    fence_mbar_init();
+    prefetch_tmap(&tmap_b);
+  }
+  if (warp == kMmaWarp0) {
+    tmem_alloc(smem_u32(&tmem_base_s), tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_s;
+
+  if (warp < kProducers) {
+    bool waited = p.a_stable == 0;
+    if (waited) grid_dependency_wait();
+    const int S = p.stages;
+    int slot = warp, first = 0;   // ring slot of this warp's next stage; CTA stages before the current item, mod 4
+    uint32_t phase = 0;
+    while (slot >= S) { slot -= S; phase ^= 1u; }
+    bool ok = true;
+    for (int i = blockIdx.x; i < p.n_items && ok; i += gridDim.x) {
+      const int g = i / p.n_chunks, chunk = i - g * p.n_chunks;
+      const int s0 = __ldg(p.stage_ptr + g), s1 = __ldg(p.stage_ptr + g + 1);
+      int s = s0 + ((warp - first) & (kProducers - 1));
+      int rec_next = s < s1 && lane < 8 ? __ldg(p.records + (size_t)s * 8 + lane) : 0;
+      for (; s < s1; s += kProducers) {
+        const int rec = rec_next;
+        if (s + kProducers < s1 && lane < 8) rec_next = __ldg(p.records + (size_t)(s + kProducers) * 8 + lane);
+        const uint32_t off = (uint32_t)__shfl_sync(0xffffffffu, rec, 0);
+        const int meta = __shfl_sync(0xffffffffu, rec, 1);
+        const int tiles = meta & 0xff, entries = (meta >> 8) & 0xff;
+        const int col = __shfl_sync(0xffffffffu, rec, 2 + (lane < kMaxEntries ? lane : 0));
+        const uint32_t full = smem_u32(&bars.full[slot]), base = ring + (uint32_t)slot * (uint32_t)p.stage_bytes;
+        const uint32_t blob_bytes = (uint32_t)(kHeaderBytes + tiles * kTileBytes * ES);
+        int fine = 1;
+        if (lane == 0) {
+          fine = mbar_wait(smem_u32(&bars.empty[slot]), phase ^ 1u, ctl) ? 1 : 0;
+          if (fine) {
+            mbar_expect_tx(full, blob_bytes + (uint32_t)(entries * kPanelBytes * ES));
+            bulk_load(base + (uint32_t)p.panel_bytes, p.blob + (size_t)off * 128, blob_bytes, full);
+          }
+        }
+        fine = __shfl_sync(0xffffffffu, fine, 0);
+        if (!fine) { ok = false; break; }
+        if (!waited) {   // B may be the output of the previous kernel
+          grid_dependency_wait();
+          waited = true;
+        }
+        if (lane < entries) {
+          const uint32_t dst = base + (uint32_t)lane * (kPanelBytes * ES);
+          if (p.use3d) tma_load_3d(dst, &tmap_b, 0, col * kTile, chunk * ES, full);
+          else
+            for (int q = 0; q < ES; ++q)
+              tma_load_2d(dst + (uint32_t)q * kPanelBytes, &tmap_b, chunk * kPanelN + q * (kPanelN / ES), col * kTile, full);
+        }
+        slot += kProducers;
+        while (slot >= S) { slot -= S; phase ^= 1u; }
+      }
+      first = (first + (s1 - s0)) & (kProducers - 1);
+    }
+    if (!waited) grid_dependency_wait();
+  } else if (warp < kEpiWarp0) {
+    // Each MMA warp issues the products of its own rows of the group.  Operands differ from tile to tile, so nothing is
+    // gained by walking the loop as a warp.
+    if (!p.a_stable) grid_dependency_wait();
+    if (elect_one()) {
+      const int cls = warp - kMmaWarp0;
+      const uint32_t idesc = p.idesc;
+      constexpr uint32_t kTileStep = (kTileBytes * ES) >> 4;
+      constexpr uint32_t kPanelKStep = (kPanelBytes / ES) >> 4, kTileKStep = 256 >> 4;
+      const int S = p.stages;
+      const uint32_t a_hi = (uint32_t)(p.desc_hi_a >> 32), b_hi = (uint32_t)(p.desc_hi_b >> 32);
+      const uint32_t a_const = (uint32_t)p.desc_hi_a, b_const = (uint32_t)p.desc_hi_b;
+      int slot = 0;
+      uint32_t phase = 0, it = 0;
+      bool ok = true;
+      for (int i = blockIdx.x; i < p.n_items && ok; i += gridDim.x, ++it) {
+        const int g = i / p.n_chunks;
+        const int s0 = __ldg(p.stage_ptr + g), s1 = __ldg(p.stage_ptr + g + 1);
+        const uint32_t buf = n_buf == 2 ? (it & 1u) : 0u, use = n_buf == 2 ? (it >> 1) : it;
+        ok = mbar_wait(smem_u32(&bars.acc_empty[buf]), (use & 1u) ^ 1u, ctl);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d0 = tmem_base + buf * (uint32_t)buf_cols;
+        for (int s = s0; s < s1; ++s) {
+          ok = mbar_wait(smem_u32(&bars.full[slot]), phase, ctl);
+          if (!ok) break;
+          const uint32_t base = ring + (uint32_t)slot * (uint32_t)p.stage_bytes;
+          const uint32_t head = base + (uint32_t)p.panel_bytes + (uint32_t)cls * (kClassWords * 4);
+          uint32_t h[4];
+          ld_shared_v4(head, h);
+          const uint32_t n = h[0] >> 8;
+          if (n == 0) {
+            mbar_arrive(smem_u32(&bars.empty[slot]));
+          } else {
+            const uint32_t a0 = a_const | ((base >> 4) & 0x3fffu);
+            uint32_t bt = (b_const | (((base + (uint32_t)p.panel_bytes + kHeaderBytes) >> 4) & 0x3fffu)) + (h[0] & 0xffu) * kTileStep;
+            uint32_t word = h[1];
+#pragma unroll 1
+            for (uint32_t t = 0; t < n; ++t, bt += kTileStep) {
+              const uint32_t w = word;
+              asm volatile("ld.shared.u32 %0, [%1];" : "=r"(word) : "r"(head + 8u + t * 4u));   // (what follows the last is not used)
+              const uint32_t d = d0 + (w & 0x1ffu), a = a0 + ((w >> 12) & 0x3fffu), keep = 1u - (w >> 31);
+#pragma unroll
+              for (int kk = 0; kk < ES; ++kk)
+                mma_halves<KIND>(d, a + (uint32_t)(kk * kPanelKStep), a_hi, bt + (uint32_t)(kk * kTileKStep), b_hi, idesc, kk > 0 ? 1u : keep);
+            }
+            tc_commit(smem_u32(&bars.empty[slot]));
+          }
+          if (++slot == S) { slot = 0; phase ^= 1u; }
+        }
+        if (!ok) break;
+        if (s1 > s0) tc_commit(smem_u32(&bars.acc_full[buf]));
+        else mbar_arrive(smem_u32(&bars.acc_full[buf]));
+      }
+    }
+    __syncwarp();
+  } else {
+    const int quad = warp & 3;
+    const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
+    const OutDesc od = p.out;
+    const uint32_t part_u32 = ring + (uint32_t)p.stages * (uint32_t)p.stage_bytes + (uint32_t)(warp - kEpiWarp0) * kPartBytes;
+    uint16_t* part = reinterpret_cast<uint16_t*>(smem_raw + (part_u32 - smem_u32(smem_raw)));
+    grid_dependency_wait();
+    uint32_t it = 0;
+    for (int i = blockIdx.x; i < p.n_items; i += gridDim.x, ++it) {
+      const int g = i / p.n_chunks, chunk = i - g * p.n_chunks;
+      const uint32_t buf = n_buf == 2 ? (it & 1u) : 0u, use = n_buf == 2 ? (it >> 1) : it;
+      // this lane's row of the group, with what its epilogue needs; scales and biases of the columns
+      const int my_row = lane < p.rows ? __ldg(p.group_rows + g * kMaxGroupRows + lane) : -1;
+      int my_has = 0;
+      float my_scale = 1.0f;
+      if (my_row >= 0) {
+        my_has = __ldg(p.row_ptr + my_row + 1) > __ldg(p.row_ptr + my_row) ? 1 : 0;
+        if (p.row_scale != nullptr && my_has) my_scale = __ldg(p.row_scale + my_row);
+      }
+      // one thread waits and the named barrier passes its verdict on: eight polling warps slow the MMA warp down
+      if (threadIdx.x == 32 * kEpiWarp0) ok_s[it & 1u] = mbar_wait(smem_u32(&bars.acc_full[buf]), use & 1u, ctl) ? 1 : 0;
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
+      if (!ok_s[it & 1u]) break;
+      tc_fence_after();
+      const int n = chunk * kPanelN + quad * 32 + lane;
+      float cs = p.b_scale, bias = 0.0f;
+      if (n < od.N) {
+        if (p.col_scale != nullptr) cs *= __ldg(p.col_scale + n);
+        if (p.bias != nullptr) bias = __ldg(p.bias + n);
+      }
+#pragma unroll 1
+      for (int r = 0; r < p.rows; ++r) {
+        const int row = __shfl_sync(0xffffffffu, my_row, r);
+        if (row < 0) continue;
+        const int has = __shfl_sync(0xffffffffu, my_has, r);
+        const float rs = __shfl_sync(0xffffffffu, my_scale, r);
+        uint32_t v[32];
+        if (has) {
+          tmem_ld_32x32(tmem_base + lane_sel + buf * (uint32_t)buf_cols + (uint32_t)(r * 32), v);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int k = 0; k < 32; ++k) v[k] = 0u;
+        }
+        if (p.staged) {
+          // 16-bit results: the warp's 32 x 32 part is put together in shared memory and leaves in 16-byte pieces, four
+          // lanes per row.  (A tiled store by the copy engine waits there behind the panels' loads: 2.4 us per part.)
+          finish16_stage<KIND, kPartPitch>(od, row, n, 0, &v[0], rs, cs, bias, part + lane);
+          finish16_stage<KIND, kPartPitch>(od, row, n, 16, &v[16], rs, cs, bias, part + lane);
+          __syncwarp();
+          const int c = chunk * kPanelN + quad * 32 + (lane & 3) * 8;
+          uint16_t* dst = reinterpret_cast<uint16_t*>(od.out) + (size_t)row * kTile * (size_t)od.ldc + c;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int m = k * 8 + (lane >> 2);
+            const uint4 x = *reinterpret_cast<const uint4*>(part + m * kPartPitch + (lane & 3) * 8);
+            if (c < od.N && row * kTile + m < od.M) *reinterpret_cast<uint4*>(dst + (size_t)m * od.ldc) = x;
+          }
+          __syncwarp();
+        } else if (p.out_tr) {
+          finish16_tr<KIND>(od, row, n, 0, &v[0], rs, cs, bias);
+          finish16_tr<KIND>(od, row, n, 16, &v[16], rs, cs, bias);
+        } else {
+          finish16<KIND>(od, row, n, 0, &v[0], rs, cs, bias);
+          finish16<KIND>(od, row, n, 16, &v[16], rs, cs, bias);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&bars.acc_empty[buf]));
+    }
+  }
+
+  grid_launch_dependents();   // (late, see pipeline_teardown in spmm.cu)
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (ctl_s[0]) {
+    const uint64_t t0 = globaltimer_ns();   // let copies still in flight land before shared memory is given back
+    while (globaltimer_ns() - t0 < 200000ull) {
+    }
+    if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, 1);
+    __syncthreads();
+  }
+  if (warp == kMmaWarp0) tmem_dealloc(tmem_base, tmem_cols);
+}
+
+// ------------------------------------------------------------------------------------------ building a group store
+// Rows of falling length (row_order, or their own order) dealt to the groups back and forth.
+__global__ void group_rows_kernel(const int32_t* __restrict__ row_order, int nbr, int n_groups, int32_t* __restrict__ group_rows) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_groups * kMaxGroupRows) return;
+  const int g = i / kMaxGroupRows, slot = i - g * kMaxGroupRows;
+  const long long k = (long long)slot * n_groups + ((slot & 1) ? n_groups - 1 - g : g);
+  int row = -1;
+  if (k < nbr) {
+    row = row_order != nullptr ? row_order[k] : (int)k;
+    if (row < 0 || row >= nbr) row = -1;
+  }
+  group_rows[i] = row;
+}
+
+__device__ __forceinline__ unsigned class_lanes(int k) {   // rows of a group whose products MMA warp k issues
+  unsigned m = 0;
+  for (int r = k; r < kMaxGroupRows; r += kMmaWarps) m |= 1u << r;
+  return m;
+}
+// One warp per group merges its rows' sorted column lists, lane r holding row r's place.  Pass 1 counts the group's stages;
+// pass 2 writes their records and headers and where every tile goes.
+template <bool EMIT>
+__global__ void __launch_bounds__(128) group_walk_kernel(const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ tile_cols,
+                                                         const int32_t* __restrict__ group_rows, int n_groups, int max_entries,
+                                                         int max_tiles, int tile_units, int panel_units,
+                                                         const int32_t* __restrict__ stage_ptr,
+                                                         const int32_t* __restrict__ blob_base, int32_t* __restrict__ counts,
+                                                         int32_t* __restrict__ records, uint8_t* __restrict__ blob,
+                                                         int32_t* __restrict__ tile_at) {
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (g >= n_groups) return;
+  int at = 0, end = 0, begin = 0;
+  if (lane < kMaxGroupRows) {
+    const int row = group_rows[g * kMaxGroupRows + lane];
+    if (row >= 0) { begin = at = row_ptr[row]; end = row_ptr[row + 1]; }
+  }
+  int stage = EMIT ? stage_ptr[g] : 0;
+  long long unit = EMIT ? blob_base[g] : 0;   // 128-byte units
+  int entries = 0, tiles = 0;
+  int rec = 0;                      // lane k < 8: word k of the open stage's record
+  uint32_t word = 0;                // lane k < tiles: the k-th tile of the open stage, its packed position and its class
+  int src = 0, cls = kMmaWarps;
+  int in_class = 0;                 // lane k < classes: tiles of class k in the open stage
+  auto close = [&]() {
+    if (EMIT) {
+      // tiles go class by class: a tile's place is the number of tiles of lower classes and of its own before it
+      uint32_t* head = reinterpret_cast<uint32_t*>(blob + unit * 128);
+      int before = 0;
+      for (int c = 0; c < kMmaWarps; ++c) {
+        const unsigned m = __ballot_sync(0xffffffffu, cls == c);
+        const int mine = __popc(m & ((1u << lane) - 1u)), n = __popc(m);
+        if (cls == c) {
+          head[c * kClassWords + 1 + mine] = word;
+          tile_at[src] = (int)(unit + 1 + (long long)(before + mine) * tile_units);
+        }
+        if (lane == 0) head[c * kClassWords] = (uint32_t)(before | n << 8);
+        before += n;
+      }
+      if (lane == 0) rec = (int)unit;
+      if (lane == 1) rec = tiles | entries << 8;
+      if (lane < 8) records[(size_t)stage * 8 + lane] = rec;
+      unit += 1 + (long long)tiles * tile_units;
+    }
+    ++stage;
+    entries = tiles = 0;
+    rec = 0;
+    cls = kMmaWarps;
+  };
+  while (true) {
+    const int col = at < end ? tile_cols[at] : kNone;
+    const int c = __reduce_min_sync(0xffffffffu, col);
+    if (c == kNone) break;
+    const unsigned mask = __ballot_sync(0xffffffffu, col == c);
+    const int n = __popc(mask);
+    // (a class's tiles have to fit its words of the header)
+    bool full = entries == max_entries || tiles + n > max_tiles;
+    for (int k = 0; k < kMmaWarps; ++k) {
+      const int of_class = __popc(mask & class_lanes(k));
+      if (__shfl_sync(0xffffffffu, in_class, k) + of_class > kClassWords - 1) full = true;
+    }
+    if (full) {
+      close();
+      in_class = 0;
+    }
+    if (lane < kMmaWarps) in_class += __popc(mask & class_lanes(lane));
+    if (EMIT) {
+      // a word per tile: its accumulator's column, its panel's place in the stage (16-byte units), bit 31: the row's first tile
+      const uint32_t mine = (uint32_t)(lane * 32) | (uint32_t)(entries * panel_units) << 12 | (at == begin ? 0x80000000u : 0u);
+      for (unsigned m = mask; m != 0u; m &= m - 1u) {
+        const int from = __ffs(m) - 1;
+        const uint32_t b = __shfl_sync(0xffffffffu, mine, from);
+        const int place = __shfl_sync(0xffffffffu, at, from);
+        if (lane == tiles) { word = b; src = place; cls = from % kMmaWarps; }
+        ++tiles;
+      }
+      if (lane == 2 + entries) rec = c;
+    } else {
+      tiles += n;
+    }
+    ++entries;
+    if (col == c) ++at;
+  }
+  if (entries > 0) close();
+  if (!EMIT && lane == 0) counts[g] = stage;
+}
+
+// stage_ptr and blob_base from the groups' stage and tile counts, by one block
+__global__ void __launch_bounds__(1024) group_scan_kernel(const int32_t* __restrict__ counts, const int32_t* __restrict__ row_ptr,
+                                                          const int32_t* __restrict__ group_rows, int n_groups, int tile_units,
+                                                          int32_t* __restrict__ stage_ptr, int32_t* __restrict__ blob_base) {
+  __shared__ int s_sum[1024], u_sum[1024];
+  const int tid = threadIdx.x, per = (n_groups + 1023) / 1024;
+  const int lo = tid * per < n_groups ? tid * per : n_groups, hi = lo + per < n_groups ? lo + per : n_groups;
+  auto units = [&](int g) {
+    int t = 0;
+    for (int r = 0; r < kMaxGroupRows; ++r) {
+      const int row = group_rows[g * kMaxGroupRows + r];
+      if (row >= 0) t += row_ptr[row + 1] - row_ptr[row];
+    }
+    return counts[g] + t * tile_units;
+  };
+  int s = 0, u = 0;
+  for (int g = lo; g < hi; ++g) { s += counts[g]; u += units(g); }
+  s_sum[tid] = s;
+  u_sum[tid] = u;
+  __syncthreads();
+  for (int o = 1; o < 1024; o <<= 1) {
+    const int a = tid >= o ? s_sum[tid - o] : 0, b = tid >= o ? u_sum[tid - o] : 0;
+    __syncthreads();
+    s_sum[tid] += a;
+    u_sum[tid] += b;
+    __syncthreads();
+  }
+  s = s_sum[tid] - s;
+  u = u_sum[tid] - u;
+  for (int g = lo; g < hi; ++g) {
+    stage_ptr[g] = s;
+    blob_base[g] = u;
+    s += counts[g];
+    u += units(g);
+  }
+  if (tid == 1023) stage_ptr[n_groups] = s_sum[1023];
+}
+
+__global__ void __launch_bounds__(256) group_copy_kernel(const uint4* __restrict__ tiles, const int32_t* __restrict__ tile_at,
+                                                         int64_t nnz, int pieces, uint4* __restrict__ blob) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t t = i / pieces;
+  if (t >= nnz) return;
+  blob[(size_t)tile_at[t] * 8 + (size_t)(i - t * pieces)] = tiles[i];
+}
+
+template <int KIND>
+int launch_group(const GroupParams& p, const CUtensorMap& mb, int grid, int smem, cudaStream_t st) {
+  auto kernel = group_kernel<KIND>;
+  if (ensure_smem((const void*)kernel, smem)) return VOID_ERR_CUDA;
+  launch_pdl(kernel, grid, kThreads, smem, st, mb, p);
+  return cudaGetLastError() == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
+}
+
+}  // namespace
+
+}  // namespace vb
+
+extern "C" {
+
+int void_group_build(const int32_t* row_ptr, const int32_t* row_order, const int32_t* tile_cols, const void* tiles, int32_t nbr,
+                     int64_t nnz, int32_t elem_bytes, int32_t n_groups, int32_t max_entries, int32_t max_tiles,
+                     int32_t* group_rows, int32_t* stage_ptr, int32_t* records, void* blob, int32_t* ws, void_stream_t stream) {
+  using namespace vb;
+  if (nbr <= 0 || nnz <= 0 || n_groups <= 0 || (long long)n_groups * kMaxGroupRows < nbr) return VOID_ERR_BAD_ARG;
+  if ((elem_bytes != 1 && elem_bytes != 2 && elem_bytes != 4)) return VOID_ERR_BAD_ARG;
+  const int tile_bytes = kTileBytes * elem_bytes, panel_units = kPanelBytes * elem_bytes / 16;
+  if (max_entries < 1 || max_entries > kMaxEntries || max_tiles < 1 ||
+      max_tiles > kMaxStageTiles || (nbr + n_groups - 1) / n_groups > max_tiles || (nbr + n_groups - 1) / n_groups > kMaxRows)
+    return VOID_ERR_BAD_ARG;
+  if (nnz * (tile_bytes / 128 + 1) > 0x7fffffffLL) return VOID_ERR_TOO_LARGE;
+  if (row_ptr == nullptr || tile_cols == nullptr || tiles == nullptr || group_rows == nullptr || stage_ptr == nullptr ||
+      records == nullptr || blob == nullptr || ws == nullptr)
+    return VOID_ERR_BAD_ARG;
+  if ((reinterpret_cast<uintptr_t>(tiles) & 15u) != 0 || (reinterpret_cast<uintptr_t>(blob) & 127u) != 0) return VOID_ERR_ALIGN;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  int32_t *counts = ws, *blob_base = ws + n_groups, *tile_at = ws + 2 * (size_t)n_groups;
+  const int units = tile_bytes / 128, blocks = (n_groups + 3) / 4;
+  group_rows_kernel<<<(n_groups * kMaxGroupRows + 255) / 256, 256, 0, st>>>(row_order, nbr, n_groups, group_rows);
+  group_walk_kernel<false><<<blocks, 128, 0, st>>>(row_ptr, tile_cols, group_rows, n_groups, max_entries, max_tiles, units, panel_units, nullptr,
+                                                   nullptr, counts, nullptr, nullptr, nullptr);
+  group_scan_kernel<<<1, 1024, 0, st>>>(counts, row_ptr, group_rows, n_groups, units, stage_ptr, blob_base);
+  group_walk_kernel<true><<<blocks, 128, 0, st>>>(row_ptr, tile_cols, group_rows, n_groups, max_entries, max_tiles, units, panel_units, stage_ptr,
+                                                  blob_base, counts, records, reinterpret_cast<uint8_t*>(blob), tile_at);
+  const int64_t pieces = nnz * (tile_bytes / 16);
+  group_copy_kernel<<<(unsigned)((pieces + 255) / 256), 256, 0, st>>>(reinterpret_cast<const uint4*>(tiles), tile_at, nnz,
+                                                                      tile_bytes / 16, reinterpret_cast<uint4*>(blob));
+  return cudaGetLastError() == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
+}
+
+int void_spmm_grouped(const void_spmm_args* a, const void_group_store* s, int32_t kind, void_stream_t stream) {
+  using namespace vb;
+  if (a == nullptr || s == nullptr || kind < VOID_KIND_I8 || kind > VOID_KIND_TF32 || kind == VOID_KIND_F8E4M3) return VOID_ERR_BAD_ARG;
+  if (a->M <= 0 || a->N <= 0 || a->K <= 0 || a->nbr <= 0) return VOID_ERR_BAD_ARG;
+  if (a->out == nullptr || a->b == nullptr || a->row_ptr == nullptr || s->blob == nullptr || s->records == nullptr ||
+      s->stage_ptr == nullptr || s->group_rows == nullptr)
+    return VOID_ERR_BAD_ARG;
+  if (a->out_dtype < VOID_OUT_F32 || a->out_dtype > VOID_OUT_BF16 || a->act < VOID_ACT_NONE || a->act > VOID_ACT_SILU ||
+      a->scale_mode != VOID_SCALE_ROW_MEAN || a->acc_out != nullptr || a->segs != nullptr || a->worker_partials != nullptr ||
+      a->n_peers != 0 || a->trace != nullptr)
+    return VOID_ERR_BAD_ARG;
+  const int es = (kind == VOID_KIND_TF32) ? 4 : ((kind == VOID_KIND_F16 || kind == VOID_KIND_BF16) ? 2 : 1);
+  if (a->tile_terms > 1 || (es > 1 && a->row_scale != nullptr)) return VOID_ERR_BAD_ARG;
+  if (a->transposed != 0 && a->transposed != 2) return VOID_ERR_BAD_ARG;
+  const bool tr = a->transposed != 0;
+  if ((long long)a->nbr * kTile < a->M || a->ldc < (tr ? a->M : a->N)) return VOID_ERR_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(a->b) & 15u) != 0 || (a->ldb & 15) != 0 || a->ldb < (long long)a->N * es) return VOID_ERR_ALIGN;
+  const int rows = (a->nbr + s->n_groups - 1) / (s->n_groups > 0 ? s->n_groups : 1);
+  if (s->n_groups <= 0 || rows < 1 || rows > kMaxRows) return VOID_ERR_BAD_ARG;
+  if (s->max_entries < 1 || s->max_entries > kMaxEntries || s->max_tiles < 1 || s->max_tiles > kMaxStageTiles) return VOID_ERR_BAD_ARG;
+  const DeviceInfo dev = device_info();
+  if (!dev.ok) return VOID_ERR_CUDA;
+  if (dev.cc_major != 10) return VOID_ERR_ARCH;
+
+  GroupParams p;
+  p.blob = reinterpret_cast<const uint8_t*>(s->blob);
+  p.records = s->records;
+  p.stage_ptr = s->stage_ptr;
+  p.group_rows = s->group_rows;
+  p.row_ptr = a->row_ptr;
+  p.row_scale = a->row_scale;
+  p.col_scale = a->col_scale;
+  p.bias = a->bias;
+  p.b_scale = a->b_scale;
+  p.out.out = a->out;
+  p.out.ldc = a->ldc;
+  p.out.acc_out = nullptr;
+  p.out.row_bias = a->row_bias;
+  p.out.M = a->M;
+  p.out.N = a->N;
+  p.out.dtype = a->out_dtype;
+  p.out.act = a->act;
+  p.status = a->status;
+  p.n_groups = s->n_groups;
+  p.n_chunks = (a->N + kPanelN - 1) / kPanelN;
+  if ((long long)p.n_groups * p.n_chunks > 0x7fffffffLL) return VOID_ERR_TOO_LARGE;
+  p.n_items = p.n_groups * p.n_chunks;
+  p.rows = rows;
+  p.out_tr = tr ? 1 : 0;
+  p.staged = (!tr && a->out_dtype != VOID_OUT_F32 && a->N % 8 == 0 && a->ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(a->out) & 15u) == 0) ? 1 : 0;
+  p.a_stable = (a->flags & 4) ? 1 : 0;
+  p.wait_limit_ms = (a->test_hooks & 0xffff) ? (a->test_hooks & 0xffff) : kDefaultWaitLimitMs;
+  p.panel_bytes = s->max_entries * kPanelBytes * es;
+  p.stage_bytes = (p.panel_bytes + kHeaderBytes + s->max_tiles * kTileBytes * es + 1023) / 1024 * 1024;
+  const int staging = p.staged ? kEpiWarps * kPartBytes : 0;
+  const int room = dev.smem_per_sm / kCtas - 1024 - 1024 - 1024 - staging;   // less alignment slack and the kernel's static variables
+  p.stages = room / p.stage_bytes;
+  if (p.stages > kMaxRing) p.stages = kMaxRing;
+  if (p.stages < kProducers) return VOID_ERR_SHAPE;   // (a producer warp may run that many stages ahead, see spmm.cu)
+  const int smem = p.stages * p.stage_bytes + staging + 1024;
+  p.desc_hi_b = smem_desc_hi(128, 256 * es, kLayoutNone);
+  p.desc_hi_a = es == 4 ? smem_desc_hi(4096, 512, kLayoutSw128Base32)
+                        : (es == 2 ? smem_desc_hi(4096, 1024, kLayoutSw128) : smem_desc_hi(1024, 1024, kLayoutSw128));
+  if (kind == VOID_KIND_I8) p.idesc = instr_desc(/*c s32*/ 2, /*s8*/ 1, 1, /*a MN*/ 1, /*b K*/ 0, 128, 32);
+  else if (kind == VOID_KIND_F16) p.idesc = instr_desc(1, 0, 0, 1, 0, 128, 32);
+  else if (kind == VOID_KIND_BF16) p.idesc = instr_desc(1, 1, 1, 1, 0, 128, 32);
+  else p.idesc = instr_desc(1, 2, 2, 1, 0, 128, 32);
+
+  CUtensorMap mb;
+  memset(&mb, 0, sizeof(mb));
+  bool whole = a->N % (kPanelN / es) == 0;
+  if (!panel_map(&mb, a->b, a->ldb, a->K, a->N, es, 1, &whole)) return VOID_ERR_TENSOR_MAP;
+  p.use3d = whole ? 1 : 0;
+  int grid = a->grid > 0 ? a->grid : dev.sms * kCtas;
+  if (grid > p.n_items) grid = p.n_items;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  switch (kind) {
+    case VOID_KIND_I8: return launch_group<VOID_KIND_I8>(p, mb, grid, smem, st);
+    case VOID_KIND_TF32: return launch_group<VOID_KIND_TF32>(p, mb, grid, smem, st);
+    default: return launch_group<VOID_KIND_F16>(p, mb, grid, smem, st);
+  }
+}
+
+}  // extern "C"
+

@@ -15,6 +15,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 
+#include <cmath>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -97,6 +98,12 @@ Identity identity(PyObject* o) {
   id.version = t.is_inference() ? 0 : (int64_t)t._version();
   return id;
 }
+// The tiles of a packed tensor laid out once more for products of groups of tile rows (csrc/group.cu).
+struct GroupStore {
+  at::Tensor index, blob;
+  void_group_store store = {};
+};
+constexpr int kMaxGroupStores = 2;
 struct PackedObject {
   PyObject_HEAD
   void_spmm_args args;   // the fields of A; everything of a launch is filled into a copy
@@ -107,6 +114,8 @@ struct PackedObject {
   int32_t kind;
   int32_t stable;
   c10::DeviceIndex device;
+  GroupStore* groups[kMaxGroupStores];   // null: not built
+  int32_t group_calls;                   // products a group store would have served since the last build; -1: none is to be built
 };
 PyTypeObject* g_packed_type = nullptr;
 
@@ -234,6 +243,121 @@ at::Tensor fp32_vector(PyObject* o, c10::Device dev, const char* what) {
   return t.to(dev, at::kFloat).contiguous();
 }
 
+// ------------------------------------------------------------------------------------------ groups of tile rows
+// How the tile rows are dealt to groups for N columns, and what that saves.  In units of a row-accumulate launch's bytes: a
+// CTA slot (two per SM) takes `turns` groups, each the panels of the block columns that any of its rows stores and its tiles;
+// the other kernel takes a panel with every tile.  More than four rows leave no second accumulator set, which costs where a
+// slot has more than one group (16384 x 4096, N = 2048, INT8 70 %: 7 rows 87.1 us, 4 rows 80.6).
+struct GroupShape {
+  int groups = 0, entries = 0, tiles = 0;
+  double saves = 0.0;
+};
+double group_saves(const PackedObject* p, int64_t N, int groups, int slots) {
+  const int es = elem_bytes(p->kind);
+  const double chunks = (double)((N + 127) / 128), nbr = p->args.nbr, nbc = p->args.nbc, nnz = (double)p->args.nnz;
+  const double d = nnz / (nbr * nbc), panel = 4.0 * es, tile = es;
+  const double rows = std::ceil(nbr / groups), turns = std::ceil(groups * chunks / slots);
+  double cost = turns * nbc * ((1.0 - std::pow(1.0 - d, rows)) * panel + d * rows * tile);
+  if (rows > 4 && turns > 1) cost *= 1.1;
+  return nnz * chunks / slots * (panel + tile) / cost;
+}
+GroupShape group_shape(const PackedObject* p, int64_t N, int slots) {
+  GroupShape best;
+  const int es = elem_bytes(p->kind);
+  const int64_t chunks = (N + 127) / 128, nbr = p->args.nbr;
+  const double d = (double)p->args.nnz / ((double)nbr * p->args.nbc);
+  // 32-bit stages hold one block column, so that rows which rarely store it leave the room of their tiles unused
+  const int64_t most = es == 4 ? (d >= 0.4 ? 4 : 2) : 8;
+  for (int64_t turns = 1; turns <= 256; ++turns) {
+    const int64_t groups = turns * slots / chunks;
+    if (groups < 1) continue;
+    const int64_t rows = (nbr + groups - 1) / groups;
+    if (rows > most) continue;
+    if (rows < 2) break;
+    const double saves = group_saves(p, N, (int)groups, slots);
+    if (saves > best.saves) {
+      best.saves = saves;
+      best.groups = (int)groups;
+      best.entries = es == 4 ? 1 : (es == 2 ? 2 : 4);
+      best.tiles = es == 4 ? (int)rows : (p->kind == VOID_KIND_I8 && rows * d > 2.2 * (1.0 - std::pow(1.0 - d, (double)rows)) ? 16 : 8);
+    }
+  }
+  return best;
+}
+// The saving from which the grouped kernel is the faster one; swept at 2048^2 ... 16384 x 4096, N = 256 ... 2048, 50 - 90 %
+// sparsity.  Predicted saving and measured gain, fp16: 1.25 0.97, 1.41 1.05, 1.74 1.17, 2.34 1.35; INT8 1.41 0.97 - 1.03,
+// 1.53 1.0 (25 tiles per row) and 1.14 (51), 1.82 1.10 - 1.23; fp32 1.14 1.06, 1.25 1.14, 1.74 1.3.
+double group_line(const PackedObject* p) {
+  const bool long_rows = p->args.nnz >= 48ll * p->args.nbr;
+  switch (p->kind) {
+    case VOID_KIND_I8: return long_rows ? 1.5 : 1.75;
+    case VOID_KIND_TF32: return 1.15;
+    default: return 1.45;
+  }
+}
+bool capturing(void_stream_t st);
+void wait_for(void_stream_t st);
+// The group store that serves this product, or null.  It is built on the third product it would have served - a tensor that is
+// multiplied once or twice does not pay for it - once for each of up to two widths; the host waits until it is complete.
+const GroupStore* group_store(PackedObject* p, int64_t N, void_stream_t st) {
+  if (N <= 64 || p->args.nnz < 4096 || p->kind == VOID_KIND_F8E4M3) return nullptr;   // (FP8 of two terms: within 5 % either way)
+  const int slots = 2 * void_device_sm_count();
+  if ((int64_t)p->args.nbr * ((N + 127) / 128) < 2ll * slots) return nullptr;
+  const double line = group_line(p);
+  const GroupShape shape = group_shape(p, N, slots);
+  if (shape.saves < line) return nullptr;
+  const GroupStore* hit = nullptr;
+  double hit_saves = 0.0;
+  int n = 0;
+  for (; n < kMaxGroupStores && p->groups[n] != nullptr; ++n) {
+    const double saves = group_saves(p, N, p->groups[n]->store.n_groups, slots);
+    if (saves > hit_saves) { hit = p->groups[n]; hit_saves = saves; }
+  }
+  const int64_t es = elem_bytes(p->kind), tile_bytes = 1024 * es, bytes = p->args.nnz * (tile_bytes + 128);
+  if (hit_saves < 0.93 * shape.saves && n < kMaxGroupStores && p->stable && bytes <= (4ll << 30) && !capturing(st) && p->group_calls >= 0 &&
+      ++p->group_calls >= 3) {
+    p->group_calls = -1;   // while this one is built, and for good if there is no room for it
+    std::unique_ptr<GroupStore> g(new GroupStore);
+    const int64_t G = shape.groups, nnz = p->args.nnz;
+    try {
+      const c10::Device dev(c10::kCUDA, p->device);
+      g->index = new_cuda({16 * G + (G + 4) / 4 * 4 + 8 * nnz}, at::kInt, dev);
+      g->blob = new_cuda({bytes + 128}, at::kByte, dev);
+      const at::Tensor ws = new_cuda({2 * G + nnz}, at::kInt, dev);
+      int32_t *rows = g->index.data_ptr<int32_t>(), *stages = rows + 16 * G, *records = stages + (G + 4) / 4 * 4;
+      uint8_t* blob = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(g->blob.data_ptr()) + 127) & ~uintptr_t(127));
+      g->store.blob = blob;
+      g->store.records = records;
+      g->store.stage_ptr = stages;
+      g->store.group_rows = rows;
+      g->store.n_groups = (int32_t)G;
+      g->store.max_entries = shape.entries;
+      g->store.max_tiles = shape.tiles;
+      if (void_group_build(p->args.row_ptr, p->row_order, p->args.tile_cols, p->args.tiles, p->args.nbr, nnz, (int32_t)es,
+                           (int32_t)G, shape.entries, shape.tiles, rows, stages, records, blob, ws.data_ptr<int32_t>(), st) != VOID_OK)
+        return hit_saves >= line ? hit : nullptr;
+      wait_for(st);
+    } catch (const c10::OutOfMemoryError&) {
+      return hit_saves >= line ? hit : nullptr;
+    }
+    p->group_calls = 0;
+    return p->groups[n] = g.release();
+  }
+  return hit_saves >= line ? hit : nullptr;
+}
+// A plain product with everything filled in.
+void launch_product(PackedObject* p, const void_spmm_args& s, void_stream_t st) {
+  if (s.transposed != 1 && s.scale_mode == VOID_SCALE_ROW_MEAN) {
+    const GroupStore* g = group_store(p, s.N, st);
+    if (g != nullptr) {
+      check(void_spmm_grouped(&s, &g->store, p->kind, st), "void_spmm_grouped");
+      return;
+    }
+  }
+  if (elem_bytes(p->kind) > 1) check(void_spmm_fp(&s, p->kind, st), "void_spmm_fp");
+  else check(p->kind == VOID_KIND_I8 ? void_spmm_i8(&s, st) : void_spmm_f8(&s, st), "void_spmm");
+}
+
 // spmm(handle, b, out | None, out_dtype | None, per_tile, col_scale | None, b_scale, bias | None, row_bias | None, act,
 //      transposed, options | None) -> out
 // options: (plan | None, acc_out, worker_partials, panels, stages, grid, tiles_per_stage, cta_shape, trace, flags,
@@ -241,7 +365,7 @@ at::Tensor fp32_vector(PyObject* o, c10::Device dev, const char* what) {
 PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_BEGIN
   if (n != 12) throw torch::TypeError("spmm takes 12 arguments");
-  const PackedObject* pk = packed_of(a[0]);
+  PackedObject* pk = packed_of(a[0]);
   const at::Tensor& b_in = cuda_tensor(a[1], "B");
   const c10::Device dev = b_in.device();
   const bool tr = PyObject_IsTrue(a[10]) == 1;
@@ -340,7 +464,8 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   // before it waits for the previous kernel; bit 30 (measurements) keeps it from doing so
   s.flags = (int32_t)(flags & 0xffff) | ((pk->stable && !(flags & (1ll << 30))) ? 4 : 0);
   const void_stream_t st = stream_of(dev.index());
-  if (es > 1) check(void_spmm_fp(&s, pk->kind, st), "void_spmm_fp");
+  if (none(a[11])) launch_product(pk, s, st);
+  else if (es > 1) check(void_spmm_fp(&s, pk->kind, st), "void_spmm_fp");
   else check(pk->kind == VOID_KIND_I8 ? void_spmm_i8(&s, st) : void_spmm_f8(&s, st), "void_spmm");
   if (!none(a[2])) {
     Py_INCREF(a[2]);
@@ -356,7 +481,7 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_BEGIN
   if (n != 6) throw torch::TypeError("mlp takes 6 arguments");
-  const PackedObject* pk[2] = {packed_of(a[0]), packed_of(a[1])};
+  PackedObject* pk[2] = {packed_of(a[0]), packed_of(a[1])};
   const at::Tensor& x = cuda_tensor(a[2], "x");
   const c10::Device dev = x.device();
   if (x.dim() != 2 || x.size(1) != pk[0]->K || pk[1]->K != pk[0]->M) fail("shape mismatch between the layers and their input");
@@ -370,7 +495,7 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const void_stream_t st = stream_of(dev.index());
   at::Tensor in = columns ? transposed_copy(x, es) : kernel_operand(x, es), bias[2], out;
   for (int layer = 0; layer < 2; ++layer) {
-    const PackedObject* p = pk[layer];
+    PackedObject* p = pk[layer];
     void_spmm_args s = p->args;
     s.scale_mode = VOID_SCALE_ROW_MEAN;
     s.row_order = p->row_order;
@@ -391,7 +516,7 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
     s.act = layer == 0 ? (int32_t)integer(a[4]) : VOID_ACT_NONE;
     s.transposed = columns ? (layer == 0 ? 0 : 2) : 1;
     s.flags = p->stable ? 4 : 0;
-    check(void_spmm_fp(&s, kind, st), "void_spmm_fp");
+    launch_product(p, s, st);
     in = out;
   }
   return THPVariable_Wrap(out);
@@ -909,6 +1034,7 @@ PyMethodDef kMethods[] = {
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 void packed_dealloc(PyObject* self) {
+  for (GroupStore* g : reinterpret_cast<PackedObject*>(self)->groups) delete g;
   PyTypeObject* type = Py_TYPE(self);
   type->tp_free(self);
   Py_DECREF(type);

@@ -22,4 +22,20 @@ __device__ __forceinline__ void issue_mma(uint32_t d, uint64_t a, uint64_t b, ui
   else mma_f16(d, a, b, idesc, acc);
 }
 
+// The same with the descriptors in halves (their upper halves do not change from one instruction to the next).
+template <int KIND>
+__device__ __forceinline__ void mma_halves(uint32_t d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                           uint32_t acc) {
+#define VB_MMA(NAME)                                                                                                   \
+  asm volatile(                                                                                                        \
+      "{\n .reg .pred p;\n .reg .b64 a, b;\n mov.b64 a, {%1, %2};\n mov.b64 b, {%3, %4};\n setp.ne.b32 p, %6, 0;\n"    \
+      " tcgen05.mma.cta_group::1." NAME " [%0], a, b, %5, p;\n}\n"                                                      \
+      ::"r"(d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc) : "memory")
+  if constexpr (KIND == VOID_KIND_I8) VB_MMA("kind::i8");
+  else if constexpr (KIND == VOID_KIND_F8E4M3) VB_MMA("kind::f8f6f4");
+  else if constexpr (KIND == VOID_KIND_TF32) VB_MMA("kind::tf32");
+  else VB_MMA("kind::f16");
+#undef VB_MMA
+}
+
 }  // namespace vb

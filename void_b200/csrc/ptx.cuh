@@ -46,6 +46,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+__device__ __forceinline__ void ld_shared_v4(uint32_t addr, uint32_t (&v)[4]) {
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr) : "memory");
+}
+
 // Additions to global memory whose old value nobody reads (no reply travels back), and the arrival count of a
 // split tile row: an add that releases this thread's earlier writes - and, after a barrier, those of the threads
 // that met it there - and acquires what earlier arrivers released.
