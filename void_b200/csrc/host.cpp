@@ -812,7 +812,7 @@ PyObject* finish_store(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // ------------------------------------------------------------------------------------------ training
 // The index arrays of one sparsity structure, both ways round; they outlive the values that train over them.
 struct Structure {
-  at::Tensor row_ptr[2], block_indices[2], tile_cols[2];   // of A, of A^T
+  at::Tensor row_ptr[2], block_indices[2], tile_cols[2], row_order[2];   // of A, of A^T
   at::Tensor items, status;
   int64_t M = 0, K = 0, nnz = 0;
 };
@@ -822,15 +822,17 @@ struct StructureObject {
 };
 PyTypeObject* g_structure_type = nullptr;
 
-// structure(row_ptr, block_indices, tile_cols, row_ptr_t, block_indices_t, tile_cols_t, items, status, M, K, n_blocks)
+// structure(row_ptr, block_indices, tile_cols, row_ptr_t, block_indices_t, tile_cols_t, items, status, M, K, n_blocks,
+//           row_order | None, row_order_t | None)
 PyObject* structure(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_BEGIN
-  if (n != 11) throw torch::TypeError("structure takes 11 arguments");
+  if (n != 13) throw torch::TypeError("structure takes 13 arguments");
   auto st = std::make_shared<Structure>();
   for (int i = 0; i < 2; ++i) {
     st->row_ptr[i] = cuda_tensor(a[3 * i], "row_ptr");
     st->block_indices[i] = cuda_tensor(a[3 * i + 1], "block_indices");
     st->tile_cols[i] = cuda_tensor(a[3 * i + 2], "tile_cols");
+    if (!none(a[11 + i])) st->row_order[i] = cuda_tensor(a[11 + i], "row_order");
   }
   st->items = cuda_tensor(a[6], "items");
   st->status = cuda_tensor(a[7], "status");
@@ -879,6 +881,7 @@ at::Tensor product_of_values(const Structure& st, bool a_transposed, const at::T
   s.tiles = tiles;
   s.tile_cols = st.tile_cols[way].const_data_ptr<int32_t>();
   s.row_ptr = st.row_ptr[way].const_data_ptr<int32_t>();
+  if (st.row_order[way].defined()) s.row_order = st.row_order[way].const_data_ptr<int32_t>();
   s.nbr = (int32_t)((M + 31) / 32);
   s.nbc = (int32_t)((K + 31) / 32);
   s.nnz = st.nnz;
