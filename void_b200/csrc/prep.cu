@@ -849,11 +849,17 @@ template <int KIND, bool VEC>
 static bool launch_quant_cols_fused(const float* b, int64_t ldb, int K, int N, void* q, int64_t ldq, float* scale,
                                     float* scale_inv, cudaStream_t st) {
   auto kernel = quant_cols_fused_kernel<KIND, VEC>;
-  const int smem = (K + kFusedCtas - 1) / kFusedCtas * kFusedCols * 4;
+  const unsigned ctas = (unsigned)((ldq + kFusedCols - 1) / kFusedCols) * kFusedCtas;
+  int smem = (K + kFusedCtas - 1) / kFusedCtas * kFusedCols * 4;
+  // The launch may start beside the end of the kernel before it, whose SMs come free one after the other: a grid that needs two
+  // CTAs per SM would fill the first ones with as many as fit and leave others idle.  It asks for the shared memory that keeps
+  // it to two (quantise and multiply in turn: INT8 4096^2, N = 512 14.0 -> 12.1 us, FP8 2048 x 4096, N = 384 15.9 -> 13.9;
+  // launched only after that kernel 13.7 and 15.7).  From 48 KB a CTA on there is nothing to gain (8192^2: 38.8 -> 39.4).
+  if (ctas > 128 && ctas <= 256 && smem <= 48 * 1024) smem = kFusedMaxSmem / 2;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedMaxSmem) != cudaSuccess)
     return false;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((ldq + kFusedCols - 1) / kFusedCols) * kFusedCtas);
+  cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(kFusedThreads);
   cfg.dynamicSmemBytes = (size_t)smem;
   cfg.stream = st;
@@ -862,10 +868,7 @@ static bool launch_quant_cols_fused(const float* b, int64_t ldb, int K, int N, v
   attr[0].val.clusterDim.x = kFusedCtas;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  // Grids that leave SMs free start beside the end of the kernel before; larger ones only take the places of its last CTAs
-  // (quantise and multiply in turn, 4096^2, N = 512: INT8 90 % 13.7 us early, 12.0 not; FP8 80 % 17.6, 16.7; 512^2, N = 128, a
-  // grid of 64: 7.0 early, 7.2 not; 2048^2, N = 256, a grid of 128: FP8 11.6 and 10.1).
-  attr[1].val.programmaticStreamSerializationAllowed = cfg.gridDim.x <= 64 ? 1 : 0;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kernel, b, ldb, K, N, reinterpret_cast<uint8_t*>(q), ldq, scale, scale_inv) == cudaSuccess;
