@@ -1015,8 +1015,8 @@ __global__ void __launch_bounds__(C::THREADS, (NP == 4) ? 1 : C::CTAS_PER_SM) sp
 // with little enough work.  That kernel's time grows with the (tile, 32 columns) pairs, about 0.7 / 0.9 / 1.4 ns each for 8- /
 // 16- / 32-bit tiles; the tensor-memory kernel's with the length of a tile row, which one CTA streams through its ring, about
 // 0.13 / 0.22 / 0.42 us per tile.  The lines were swept at 16 ... 512 tile rows of 2 ... 64 tiles, N = 1 ... 128; at 4096^2,
-// 90 % (13 tiles per row) fp16: N = 8 5.2 us against 9.6, N = 64 6.3 against 7.5, N = 128 10.7 against 7.6; at 16384^2, 90 %
-// (51 tiles) INT8: N = 16 12.9 against 23.8, N = 32 21.6 against 13.9.
+// 90 % (13 tiles per row) fp16: N = 8 4.8 us against 9.6, N = 64 6.0 against 5.2; 2048 x 8192, 80 % (51 tiles), N = 64 7.3
+// against 10.3; 16384^2, 90 % (51 tiles) INT8: N = 16 12.9 against 23.8, N = 32 21.6 against 13.9.
 static bool few_columns(const void_spmm_args* a, int kind, int es, bool drain) {
   if (drain || a->N > kPanelN || a->transposed == 2 || a->segs != nullptr || a->acc_out != nullptr || a->worker_partials != nullptr ||
       a->trace != nullptr || a->n_peers != 0 || a->test_hooks != 0 || a->panels_per_item != 0 || a->stages != 0 || a->grid != 0 ||
@@ -1025,7 +1025,7 @@ static bool few_columns(const void_spmm_args* a, int kind, int es, bool drain) {
   if (a->N <= 16) return true;
   const long long pairs = a->nnz * ((a->N + 31) / 32), rows = a->nbr > 0 ? a->nbr : 1;
   if (kind == VOID_KIND_F8E4M3 && a->tile_terms > 1) return pairs * rows < 150 * (a->nnz - 10 * rows);
-  return pairs * rows < (es == 1 ? 180 : 270) * (a->nnz + rows);
+  return pairs * rows < (es == 1 ? 180 : 160) * (a->nnz + rows);
 }
 
 static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
