@@ -36,6 +36,7 @@ class PackedTiles:
     terms: int = 1             # packed tiles per stored tile (2 / 3: FP8 tiles stored as sums of E4M3 terms)
     stable: bool = False       # the kernels that wrote the arrays above are known to have finished
     row_order: Optional[torch.Tensor] = None   # int32 [nbr]: tile rows by falling tile count (launches without a plan)
+    home: Optional[int] = None                 # the stream the arrays were allocated on, if one and known
     native: object = field(default=None, init=False, repr=False, compare=False)   # the native host path's view of this store (handle())
 
     def is_stable(self) -> bool:
@@ -51,7 +52,7 @@ class PackedTiles:
         """What the native host path launches products of this store from, as its fields are now."""
         return _lib.native().packed_handle(
             self.shape[0], self.shape[1], self.kind, self.terms, self.nnz, self.stable, _lib.status_word(self.tiles.device),
-            self.tiles, self.tile_cols, self.tile_scales, self.row_ptr, self.row_scale, self.row_order)
+            self.tiles, self.tile_cols, self.tile_scales, self.row_ptr, self.row_scale, self.row_order, self.home)
 
     def handle(self):
         """The handle the operators use, made once."""
@@ -72,10 +73,10 @@ def pack(values: torch.Tensor, scales: Optional[torch.Tensor], block_rows: torch
     if values.dim() != 3 or values.shape[1] != TILE or values.shape[2] != TILE or values.element_size() != es:
         raise _lib.VoidB200Error("void_b200 kernels need 32x32 tiles of %d-byte elements here, got %s %s"
                                  % (es, tuple(values.shape), values.dtype))
-    tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale = _lib.native().pack_store(
+    tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale, home = _lib.native().pack_store(
         values, scales, block_rows, block_cols, M, K, kind, terms, row_ptr, block_indices)
     return PackedTiles(tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale, (M + TILE - 1) // TILE,
-                       (K + TILE - 1) // TILE, values.shape[0], (M, K), kind, terms)
+                       (K + TILE - 1) // TILE, values.shape[0], (M, K), kind, terms, home=home)
 
 
 def pack_f8_split(values: torch.Tensor, scales: Optional[torch.Tensor], block_rows: torch.Tensor,

@@ -6,6 +6,7 @@
 // arguments by position (METH_FASTCALL) from the Python operators, which keep the public signatures.
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
@@ -15,10 +16,12 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 
+#include <algorithm>
 #include <cmath>
 #include <memory>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "../../include/void_b200.h"
 
@@ -72,6 +75,26 @@ at::Tensor new_cuda(at::IntArrayRef size, at::ScalarType type, c10::Device dev) 
 at::Tensor as_type(const at::Tensor& t, at::ScalarType type) { return t.scalar_type() == type ? t : t.to(type); }
 void_stream_t stream_of(c10::DeviceIndex dev) { return c10::cuda::getCurrentCUDAStream(dev).stream(); }
 
+// The streams that have read the arrays of a store.  The allocator knows the stream an array was allocated on; that another
+// one reads it has to be said, or the memory is handed out again when the tensor is dropped while that stream's kernel still
+// runs.  Callers cannot say it for arrays they never see.
+class Readers {
+ public:
+  // the stream all arrays were allocated on, where that is known
+  void home(cudaStream_t stream) { seen_.push_back(stream); }
+  void add(c10::cuda::CUDAStream stream, std::initializer_list<const at::Tensor*> arrays) {
+    const std::lock_guard<std::mutex> lock(mutex_);
+    if (std::find(seen_.begin(), seen_.end(), stream.stream()) != seen_.end()) return;
+    for (const at::Tensor* t : arrays)
+      if (t->defined()) c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), stream);
+    seen_.push_back(stream.stream());
+  }
+
+ private:
+  std::mutex mutex_;
+  std::vector<cudaStream_t> seen_;
+};
+
 #define NATIVE_BEGIN                                    \
   HANDLE_TH_ERRORS                                      \
   try {
@@ -104,38 +127,46 @@ struct GroupStore {
   void_group_store store = {};
 };
 constexpr int kMaxGroupStores = 2;
+struct Packed {
+  void_spmm_args args = {};   // the fields of A; everything of a launch is filled into a copy
+  at::Tensor tiles, tile_cols, tile_scales, row_ptr, row_scale_array, row_order_array;   // what those fields point into
+  const int32_t* row_order = nullptr;
+  const float* row_scale = nullptr;
+  Identity made_from[4];      // values, scales, block rows, block columns
+  int64_t M = 0, K = 0;
+  int32_t kind = 0;
+  int32_t stable = 0;
+  c10::DeviceIndex device = 0;
+  Readers readers;
+  std::unique_ptr<GroupStore> groups[kMaxGroupStores];   // null: not built
+  int32_t group_calls = 0;    // products a group store would have served since the last build; -1: none is to be built
+};
 struct PackedObject {
   PyObject_HEAD
-  void_spmm_args args;   // the fields of A; everything of a launch is filled into a copy
-  const int32_t* row_order;
-  const float* row_scale;
-  Identity made_from[4]; // values, scales, block rows, block columns
-  int64_t M, K;
-  int32_t kind;
-  int32_t stable;
-  c10::DeviceIndex device;
-  GroupStore* groups[kMaxGroupStores];   // null: not built
-  int32_t group_calls;                   // products a group store would have served since the last build; -1: none is to be built
+  Packed* packed;
 };
 PyTypeObject* g_packed_type = nullptr;
 
-PackedObject* packed_of(PyObject* o) {
+Packed* packed_of(PyObject* o) {
   if (Py_TYPE(o) != g_packed_type) throw torch::TypeError("expected a packed tensor handle");
-  return reinterpret_cast<PackedObject*>(o);
+  return reinterpret_cast<PackedObject*>(o)->packed;
 }
 template <typename T>
 T* data_or_null(PyObject* o) {
   return none(o) ? nullptr : static_cast<T*>(tensor(o, "operand").data_ptr());
 }
+// The stream a product of this store is launched on, noted as one of its readers.
+void_stream_t launch_stream(Packed* p) {
+  const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(p->device);
+  p->readers.add(stream, {&p->tiles, &p->tile_cols, &p->tile_scales, &p->row_ptr, &p->row_scale_array, &p->row_order_array});
+  return stream.stream();
+}
 
-// packed_handle(M, K, kind, terms, nnz, stable, status, tiles, tile_cols, tile_scales, row_ptr, row_scale, row_order)
+// packed_handle(M, K, kind, terms, nnz, stable, status, tiles, tile_cols, tile_scales, row_ptr, row_scale, row_order, home | None)
 PyObject* packed_handle(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_BEGIN
-  if (n != 13) throw torch::TypeError("packed_handle takes 13 arguments");
-  PyObject* self = PyType_GenericAlloc(g_packed_type, 0);
-  if (self == nullptr) return nullptr;
-  PackedObject* p = reinterpret_cast<PackedObject*>(self);
-  p->args = void_spmm_args();
+  if (n != 14) throw torch::TypeError("packed_handle takes 14 arguments");
+  std::unique_ptr<Packed> p(new Packed);
   p->M = integer(a[0]);
   p->K = integer(a[1]);
   p->kind = (int32_t)integer(a[2]);
@@ -143,6 +174,9 @@ PyObject* packed_handle(PyObject*, PyObject* const* a, Py_ssize_t n) {
   p->args.nnz = integer(a[4]);
   p->stable = (int32_t)integer(a[5]);
   p->args.status = data_or_null<int32_t>(a[6]);
+  at::Tensor* arrays[6] = {&p->tiles, &p->tile_cols, &p->tile_scales, &p->row_ptr, &p->row_scale_array, &p->row_order_array};
+  for (int i = 0; i < 6; ++i)
+    if (!none(a[7 + i])) *arrays[i] = cuda_tensor(a[7 + i], "packed array");
   p->args.tiles = data_or_null<void>(a[7]);
   p->args.tile_cols = data_or_null<int32_t>(a[8]);
   p->args.tile_scales = data_or_null<float>(a[9]);
@@ -153,7 +187,11 @@ PyObject* packed_handle(PyObject*, PyObject* const* a, Py_ssize_t n) {
   p->args.nbc = (int32_t)((p->K + 31) / 32);
   p->args.M = (int32_t)p->M;
   p->args.K = (int32_t)p->K;
-  p->device = tensor(a[7], "tiles").device().index();
+  p->device = p->tiles.device().index();
+  if (!none(a[13])) p->readers.home(reinterpret_cast<cudaStream_t>((intptr_t)integer(a[13])));
+  PyObject* self = PyType_GenericAlloc(g_packed_type, 0);
+  if (self == nullptr) return nullptr;
+  reinterpret_cast<PackedObject*>(self)->packed = p.release();
   return self;
   NATIVE_END
 }
@@ -162,7 +200,7 @@ PyObject* packed_handle(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* packed_made_from(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_BEGIN
   if (n != 5) throw torch::TypeError("packed_made_from takes 5 arguments");
-  PackedObject* p = packed_of(a[0]);
+  Packed* p = packed_of(a[0]);
   for (int i = 0; i < 4; ++i) p->made_from[i] = identity(a[1 + i]);
   Py_RETURN_NONE;
   NATIVE_END
@@ -171,7 +209,7 @@ PyObject* packed_made_from(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* packed_is_current(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_BEGIN
   if (n != 6) throw torch::TypeError("packed_is_current takes 6 arguments");
-  const PackedObject* p = packed_of(a[0]);
+  const Packed* p = packed_of(a[0]);
   for (int i = 0; i < 4; ++i)
     if (!(p->made_from[i] == identity(a[1 + i]))) Py_RETURN_FALSE;
   PyObject* shape = a[5];
@@ -259,7 +297,7 @@ struct GroupShape {
   int groups = 0, entries = 0, tiles = 0;
   double saves = 0.0;
 };
-double group_saves(const PackedObject* p, int64_t N, int groups, int slots) {
+double group_saves(const Packed* p, int64_t N, int groups, int slots) {
   const int es = elem_bytes(p->kind);
   const double chunks = (double)((N + 127) / 128), nbr = p->args.nbr, nbc = p->args.nbc, nnz = (double)p->args.nnz;
   const double d = nnz / (nbr * nbc), panel = 4.0 * es, tile = es;
@@ -268,7 +306,7 @@ double group_saves(const PackedObject* p, int64_t N, int groups, int slots) {
   if (rows > 4 && turns > 1) cost *= 1.1;
   return nnz * chunks / slots * (panel + tile) / cost;
 }
-GroupShape group_shape(const PackedObject* p, int64_t N, int slots) {
+GroupShape group_shape(const Packed* p, int64_t N, int slots) {
   GroupShape best;
   const int es = elem_bytes(p->kind);
   const int64_t chunks = (N + 127) / 128, nbr = p->args.nbr;
@@ -294,7 +332,7 @@ GroupShape group_shape(const PackedObject* p, int64_t N, int slots) {
 // The saving from which the grouped kernel is the faster one; swept at 2048^2 ... 16384 x 4096, N = 256 ... 2048, 50 - 90 %
 // sparsity.  Predicted saving and measured gain, fp16: 1.25 0.97, 1.41 1.05, 1.74 1.17, 2.34 1.35; INT8 1.41 0.97 - 1.03,
 // 1.53 1.0 (25 tiles per row) and 1.14 (51), 1.82 1.10 - 1.23; fp32 1.14 1.06, 1.25 1.14, 1.74 1.3.
-double group_line(const PackedObject* p) {
+double group_line(const Packed* p) {
   const bool long_rows = p->args.nnz >= 48ll * p->args.nbr;
   switch (p->kind) {
     case VOID_KIND_I8: return long_rows ? 1.5 : 1.75;
@@ -306,7 +344,7 @@ bool capturing(void_stream_t st);
 void wait_for(void_stream_t st);
 // The group store that serves this product, or null.  It is built on the third product it would have served - a tensor that is
 // multiplied once or twice does not pay for it - once for each of up to two widths; the host waits until it is complete.
-const GroupStore* group_store(PackedObject* p, int64_t N, void_stream_t st) {
+const GroupStore* group_store(Packed* p, int64_t N, void_stream_t st) {
   if (N <= 64 || p->args.nnz < 4096 || p->kind == VOID_KIND_F8E4M3) return nullptr;   // (FP8 of two terms: within 5 % either way)
   const int slots = 2 * void_device_sm_count();
   if ((int64_t)p->args.nbr * ((N + 127) / 128) < 2ll * slots) return nullptr;
@@ -318,7 +356,7 @@ const GroupStore* group_store(PackedObject* p, int64_t N, void_stream_t st) {
   int n = 0;
   for (; n < kMaxGroupStores && p->groups[n] != nullptr; ++n) {
     const double saves = group_saves(p, N, p->groups[n]->store.n_groups, slots);
-    if (saves > hit_saves) { hit = p->groups[n]; hit_saves = saves; }
+    if (saves > hit_saves) { hit = p->groups[n].get(); hit_saves = saves; }
   }
   const int64_t es = elem_bytes(p->kind), tile_bytes = 1024 * es, bytes = p->args.nnz * (tile_bytes + 128);
   if (hit_saves < 0.93 * shape.saves && n < kMaxGroupStores && p->stable && bytes <= (4ll << 30) && !capturing(st) && p->group_calls >= 0 &&
@@ -348,12 +386,13 @@ const GroupStore* group_store(PackedObject* p, int64_t N, void_stream_t st) {
       return hit_saves >= line ? hit : nullptr;
     }
     p->group_calls = 0;
-    return p->groups[n] = g.release();
+    p->groups[n] = std::move(g);
+    return p->groups[n].get();
   }
   return hit_saves >= line ? hit : nullptr;
 }
 // A plain product with everything filled in.
-void launch_product(PackedObject* p, const void_spmm_args& s, void_stream_t st) {
+void launch_product(Packed* p, const void_spmm_args& s, void_stream_t st) {
   if (s.transposed != 1 && s.scale_mode == VOID_SCALE_ROW_MEAN) {
     const GroupStore* g = group_store(p, s.N, st);
     if (g != nullptr) {
@@ -372,7 +411,7 @@ void launch_product(PackedObject* p, const void_spmm_args& s, void_stream_t st) 
 PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_BEGIN
   if (n != 12) throw torch::TypeError("spmm takes 12 arguments");
-  PackedObject* pk = packed_of(a[0]);
+  Packed* pk = packed_of(a[0]);
   const at::Tensor& b_in = cuda_tensor(a[1], "B");
   const c10::Device dev = b_in.device();
   const bool tr = PyObject_IsTrue(a[10]) == 1;
@@ -470,7 +509,7 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   // bit 2: the packed store (and the plan, whose builder synchronises) is complete, so the kernel may read it
   // before it waits for the previous kernel; bit 30 (measurements) keeps it from doing so
   s.flags = (int32_t)(flags & 0xffff) | ((pk->stable && !(flags & (1ll << 30))) ? 4 : 0);
-  const void_stream_t st = stream_of(dev.index());
+  const void_stream_t st = launch_stream(pk);
   if (none(a[11])) launch_product(pk, s, st);
   else if (es > 1) check(void_spmm_fp(&s, pk->kind, st), "void_spmm_fp");
   else check(pk->kind == VOID_KIND_I8 ? void_spmm_i8(&s, st) : void_spmm_f8(&s, st), "void_spmm");
@@ -488,7 +527,7 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_BEGIN
   if (n != 6) throw torch::TypeError("mlp takes 6 arguments");
-  PackedObject* pk[2] = {packed_of(a[0]), packed_of(a[1])};
+  Packed* pk[2] = {packed_of(a[0]), packed_of(a[1])};
   const at::Tensor& x = cuda_tensor(a[2], "x");
   const c10::Device dev = x.device();
   if (x.dim() != 2 || x.size(1) != pk[0]->K || pk[1]->K != pk[0]->M) fail("shape mismatch between the layers and their input");
@@ -499,10 +538,11 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int kind = pk[0]->kind, es = elem_bytes(kind);
   const int64_t N = x.size(0);
   const bool columns = N > 128 && copy_saves_ns(kind, pk[0]->args.nnz + pk[1]->args.nnz, N) > copy_costs_ns(N, pk[0]->K, es);
-  const void_stream_t st = stream_of(dev.index());
+  const void_stream_t st = launch_stream(pk[0]);
+  launch_stream(pk[1]);
   at::Tensor in = columns ? transposed_copy(x, es) : kernel_operand(x, es), bias[2], out;
   for (int layer = 0; layer < 2; ++layer) {
-    PackedObject* p = pk[layer];
+    Packed* p = pk[layer];
     void_spmm_args s = p->args;
     s.scale_mode = VOID_SCALE_ROW_MEAN;
     s.row_order = p->row_order;
@@ -534,7 +574,7 @@ PyObject* mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* spmv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_BEGIN
   if (n != 4) throw torch::TypeError("spmv takes 4 arguments");
-  const PackedObject* pk = packed_of(a[0]);
+  Packed* pk = packed_of(a[0]);
   at::Tensor x = cuda_tensor(a[1], "x");
   const c10::Device dev = x.device();
   const int es = elem_bytes(pk->kind);
@@ -556,7 +596,7 @@ PyObject* spmv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   s.out_dtype = out_code(out.scalar_type());
   s.transposed = 1;
   s.flags = pk->stable ? 4 : 0;
-  check(void_spmm_fp(&s, pk->kind, stream_of(dev.index())), "void_spmm_fp");
+  check(void_spmm_fp(&s, pk->kind, launch_stream(pk)), "void_spmm_fp");
   if (!none(a[2])) {
     Py_INCREF(a[2]);
     return a[2];
@@ -746,7 +786,8 @@ PyObject* tile_index(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // pack_store(values, scales | None, block_rows, block_cols, M, K, kind, terms, row_ptr | None, block_indices | None)
-//   -> (tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale)
+//   -> (tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale, home): home is the stream all of them were allocated
+//   on, None with an index that was given
 // The packed store of a tensor, its tile index built on the way when it is not given.  The caller waits for it
 // and checks the index (finish_store); until then a list that is not valid is packed without leaving its arrays.
 PyObject* pack_store(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -787,7 +828,11 @@ PyObject* pack_store(PyObject*, PyObject* const* a, Py_ssize_t n) {
           "void_pack_tiles_f8_split");
   else
     check(void_pack_tiles(values.const_data_ptr(), sc, n_sc, bc, bi, rp, count, nbr, tiles.data_ptr(), tc, ts, rs, st), "void_pack_tiles");
-  return pack_tuple({tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale});
+  PyObject* home = Py_None;
+  if (none(a[8]) || none(a[9])) home = PyLong_FromLongLong((long long)reinterpret_cast<intptr_t>(st));
+  else Py_INCREF(home);
+  return Py_BuildValue("NNNNNNN", THPVariable_Wrap(tiles), THPVariable_Wrap(tile_cols), THPVariable_Wrap(tile_scales), THPVariable_Wrap(row_ptr),
+                       THPVariable_Wrap(block_indices), THPVariable_Wrap(row_scale), home);
   NATIVE_END
 }
 
@@ -822,6 +867,7 @@ struct Structure {
   at::Tensor row_ptr[2], block_indices[2], tile_cols[2], row_order[2];   // of A, of A^T
   at::Tensor items, status;
   int64_t M = 0, K = 0, nnz = 0;
+  mutable Readers readers;
 };
 struct StructureObject {
   PyObject_HEAD
@@ -852,6 +898,12 @@ PyObject* structure(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return self;
   NATIVE_END
 }
+void_stream_t launch_stream(const Structure& st, c10::Device dev) {
+  const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  st.readers.add(stream, {&st.row_ptr[0], &st.row_ptr[1], &st.block_indices[0], &st.block_indices[1], &st.tile_cols[0], &st.tile_cols[1],
+                          &st.row_order[0], &st.row_order[1], &st.items});
+  return stream.stream();
+}
 std::shared_ptr<const Structure> structure_of(PyObject* o) {
   if (Py_TYPE(o) != g_structure_type) throw torch::TypeError("expected a structure handle");
   return reinterpret_cast<StructureObject*>(o)->st;
@@ -880,7 +932,7 @@ at::Tensor product_of_values(const Structure& st, bool a_transposed, const at::T
   at::Tensor out = new_cuda({linear ? N : M, linear ? M : N}, b_in.scalar_type(), dev);
   at::Tensor store = new_cuda({std::max<int64_t>(st.nnz, 1) * 1024 * es + 1024}, at::kByte, dev);
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(store.data_ptr()) + 1023) & ~uintptr_t(1023));
-  const void_stream_t stream = stream_of(dev.index());
+  const void_stream_t stream = launch_stream(st, dev);
   const int way = a_transposed ? 1 : 0;
   check(void_repack_tiles_fp(values.const_data_ptr(), es, st.block_indices[way].const_data_ptr<int32_t>(), st.nnz, way, tiles, stream),
         "void_repack_tiles_fp");
@@ -928,7 +980,7 @@ at::Tensor gradient_of_values(const Structure& st, const at::Tensor& g_in, const
             g.const_data_ptr(), row_pitch(g, es), x.const_data_ptr(), row_pitch(x, es), (int32_t)st.M, (int32_t)st.K, (int32_t)N,
             kind, st.items.const_data_ptr<int32_t>(), (int32_t)st.items.size(0), st.tile_cols[0].const_data_ptr<int32_t>(),
             st.block_indices[0].const_data_ptr<int32_t>(), grad.data_ptr(), out_code(type), st.status.data_ptr<int32_t>(),
-            stream_of(dev.index())),
+            launch_stream(st, dev)),
         "void_spmm_tile_grad");
   return grad;
 }
@@ -1044,7 +1096,7 @@ PyMethodDef kMethods[] = {
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 void packed_dealloc(PyObject* self) {
-  for (GroupStore* g : reinterpret_cast<PackedObject*>(self)->groups) delete g;
+  delete reinterpret_cast<PackedObject*>(self)->packed;
   PyTypeObject* type = Py_TYPE(self);
   type->tp_free(self);
   Py_DECREF(type);
