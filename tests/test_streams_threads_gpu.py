@@ -69,3 +69,166 @@ def test_index_arrays_of_a_dropped_layer_wait_for_the_other_stream_that_reads_th
     side.synchronize()
     assert torch.equal(got, want)
     void.check_device_status()
+
+
+# ------------------------------------------------------------------------------------------ group stores
+GROUPED = [torch.int8, torch.float16, torch.bfloat16, torch.float32]
+
+
+def _grouped_case(dtype, seed):
+    """A tensor and an operand whose products a group store serves, of random values: a changed order of additions shows."""
+    w = workloads.block_sparse(workloads.uniform_mask(157, 61, 0.1, seed=seed), 1500, seed=seed)
+    if dtype == torch.int8:
+        q = void.quantize_void_tensor(w.a)
+        bq, bs = void.quantize_cols_int8(w.b)
+        return q, lambda out=None: void.void_spmm_int8(q, bq, bs, out, out_dtype=torch.float32), lambda: q.packed()
+    from void_b200 import ops
+    a, b = w.a.to_dtype(dtype), w.b.to(dtype)
+    return a, lambda out=None: void.void_spmm(a, b, out), lambda: ops.packed_fp(a, ops.product_kind(a, b))
+
+
+def _stores(packed, allowed=None):
+    from void_b200 import _lib
+    return _lib.native().packed_grouped(packed().native, allowed)
+
+
+@pytest.mark.parametrize("dtype", GROUPED)
+def test_a_group_store_is_built_behind_a_product_and_changes_no_bit(dtype):
+    warm, product, _ = _grouped_case(dtype, 2)              # kernels loaded, and memory for a store at hand
+    for _ in range(4):
+        product()
+        torch.cuda.synchronize()
+    del warm, product, _
+    a, product, packed = _grouped_case(dtype, 3)
+    want = product()
+    product()
+    torch.cuda.synchronize()
+    assert _stores(packed) == (True, 0, 0)
+    torch.cuda._sleep(BUSY)
+    third, fourth = product(), product()
+    assert not torch.cuda.current_stream().query()          # the host did not wait for the store
+    assert _stores(packed) == (True, 1, 0)                  # and the products did not use it
+    torch.cuda.synchronize()
+    fifth = product()
+    assert _stores(packed) == (True, 1, 1)
+    for got in (third, fourth, fifth):
+        assert torch.equal(got, want)
+    void.check_device_status()
+
+
+@pytest.mark.parametrize("dtype", GROUPED)
+def test_group_stores_can_be_refused_and_are_given_back(dtype):
+    a, product, packed = _grouped_case(dtype, 4)
+    want = product()
+    for _ in range(4):
+        product()
+    torch.cuda.synchronize()
+    product()
+    assert _stores(packed) == (True, 1, 1)
+    before = torch.cuda.memory_allocated()
+    void.allow_group_stores(a, False)
+    assert _stores(packed) == (False, 0, 0) and before - torch.cuda.memory_allocated() > a.values.numel() * a.values.element_size()
+    for _ in range(4):
+        assert torch.equal(product(), want)
+    assert _stores(packed) == (False, 0, 0)
+    void.allow_group_stores(a, True)
+    for _ in range(4):
+        product()
+    torch.cuda.synchronize()
+    assert torch.equal(product(), want) and _stores(packed) == (True, 1, 1)
+    c, again, packed_c = _grouped_case(dtype, 4)            # refused before anything is packed
+    void.allow_group_stores(c, False)
+    for _ in range(4):
+        assert torch.equal(again(), want)
+    assert _stores(packed_c) == (False, 0, 0)
+    void.check_device_status()
+
+
+@pytest.mark.parametrize("dtype", GROUPED)
+def test_group_stores_with_two_streams(dtype):
+    a, product, packed = _grouped_case(dtype, 5)
+    void.allow_group_stores(a, False)
+    want = product()
+    void.allow_group_stores(a, True)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got = []
+    for i in range(12):                                     # the build falls between products of both streams
+        with torch.cuda.stream(streams[i % 2]):
+            if i < 4:
+                torch.cuda._sleep(1_000_000)
+            got.append(product())
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, want) for g in got)
+    with torch.cuda.stream(streams[1]):                     # dropped while a product on the other stream reads it
+        torch.cuda._sleep(BUSY)
+        last = product()
+    assert _stores(packed) == (True, 1, 1)
+    before = torch.cuda.memory_allocated()
+    void.allow_group_stores(a, False)
+    kept, _ = _blocks_handed_out(before - torch.cuda.memory_allocated(), 2)
+    for t in kept:
+        t.fill_(0)
+    torch.cuda.synchronize()
+    assert torch.equal(last, want)
+    void.check_device_status()
+
+
+@pytest.mark.parametrize("dtype", GROUPED)
+def test_group_stores_with_two_threads(dtype):
+    a, product, packed = _grouped_case(dtype, 6)
+    void.allow_group_stores(a, False)
+    want = product()
+    void.allow_group_stores(a, True)
+    torch.cuda.synchronize()
+    got, failed = [[], []], []
+
+    def work(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(20):
+                    got[k].append(product())
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:          # noqa: BLE001 - reported below
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed and all(torch.equal(g, want) for g in got[0] + got[1])
+    assert _stores(packed)[1] == 1
+    void.check_device_status()
+
+
+@pytest.mark.parametrize("dtype", GROUPED)
+def test_group_stores_and_captures(dtype):
+    a, product, packed = _grouped_case(dtype, 7)
+    want = product()
+    out = [torch.empty_like(want) for _ in range(2)]
+    torch.cuda.synchronize()
+
+    def capture(o):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for _ in range(4):
+                product(o)
+        return g
+
+    before = capture(out[0])                                # nothing is built while a stream is captured
+    assert _stores(packed) == (True, 0, 0)
+    for _ in range(4):
+        product()
+    torch.cuda.synchronize()
+    during = capture(out[1])                                # built, but not yet known to be complete: not used
+    assert _stores(packed)[1] == 1
+    product()
+    after_out = torch.empty_like(want)
+    after = capture(after_out)
+    assert _stores(packed) == (True, 1, 1)
+    for g in (before, during, after):
+        g.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o in out + [after_out])
+    void.check_device_status()

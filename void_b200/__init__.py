@@ -24,5 +24,6 @@ from .scheduler import WorkloadProfile, analyze_workload
 from .distributed import (ShardingStrategy, DistributedVOIDTensor, shard_void_tensor, distributed_void_spmm,
                           broadcast_b, broadcast_spmm_overlapped)
 from ._lib import VoidB200Error, check_device_status
+from ._spmm import allow_group_stores
 
 __version__ = "0.1.0"

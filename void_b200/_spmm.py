@@ -99,12 +99,32 @@ def _mark_ready(p: PackedTiles) -> PackedTiles:
     return p
 
 
+def allow_group_stores(a, allowed: bool) -> None:
+    """Whether products of ``a`` (VOIDTensor, Int8VOIDTensor) may keep its tiles a second time, laid out for groups of tile
+    rows (by default they may).  From the third large product of a rather dense tensor on, such a store - as large as the
+    packed tiles and an eighth more for 8-bit tiles, at most 4 GB, for up to two widths of B - is built behind a product and
+    used once it is complete.  False gives the stores of ``a`` back and keeps further ones from being built."""
+    a._group_stores = bool(allowed)
+    d = a.__dict__
+    for p in (d.get("_packed_cache"), *d.get("_packed_fp_cache", {}).values()):
+        if p is not None:
+            _lib.native().packed_grouped(p.handle(), bool(allowed))
+
+
+def new_store(owner, p: PackedTiles, *made_from) -> PackedTiles:
+    """A store that was just packed for ``owner``, ready to be launched from: it knows what it was made from."""
+    p = _mark_ready(p)
+    _lib.native().packed_made_from(p.handle(), *made_from)
+    if not owner.__dict__.get("_group_stores", True):
+        _lib.native().packed_grouped(p.native, False)
+    return p
+
+
 def cached_pack(owner, values, scales, block_rows, block_cols, shape, kind) -> PackedTiles:
     """Packed store cached on the tensor object, rebuilt when its storage or contents change."""
     p = owner.__dict__.get("_packed_cache")
     if p is None or not _lib.native().packed_is_current(p.native, values, scales, block_rows, block_cols, shape):
-        p = _mark_ready(pack(values, scales, block_rows, block_cols, shape, kind))
-        _lib.native().packed_made_from(p.handle(), values, scales, block_rows, block_cols)
+        p = new_store(owner, pack(values, scales, block_rows, block_cols, shape, kind), values, scales, block_rows, block_cols)
         owner._packed_cache = p
         owner._plan_cache = {}
     return p

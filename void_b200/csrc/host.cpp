@@ -7,6 +7,7 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
@@ -125,6 +126,14 @@ Identity identity(PyObject* o) {
 struct GroupStore {
   at::Tensor index, blob;
   void_group_store store = {};
+  cudaEvent_t built = nullptr;   // behind the kernels that write it; null once it is known to be complete
+  Readers readers;
+  GroupStore() = default;
+  GroupStore(const GroupStore&) = delete;
+  GroupStore& operator=(const GroupStore&) = delete;
+  ~GroupStore() {
+    if (built != nullptr) cudaEventDestroy(built);
+  }
 };
 constexpr int kMaxGroupStores = 2;
 struct Packed {
@@ -139,7 +148,8 @@ struct Packed {
   c10::DeviceIndex device = 0;
   Readers readers;
   std::unique_ptr<GroupStore> groups[kMaxGroupStores];   // null: not built
-  int32_t group_calls = 0;    // products a group store would have served since the last build; -1: none is to be built
+  int32_t group_calls = 0;    // products a group store would have served since the last build; -1: there was no room for one
+  bool grouped = true;        // whether group stores may be built and used
 };
 struct PackedObject {
   PyObject_HEAD
@@ -217,6 +227,29 @@ PyObject* packed_is_current(PyObject*, PyObject* const* a, Py_ssize_t n) {
       integer(PyTuple_GET_ITEM(shape, 1)) != p->K)
     Py_RETURN_FALSE;
   Py_RETURN_TRUE;
+  NATIVE_END
+}
+
+// packed_grouped(handle, allowed | None) -> (allowed, group stores, of them complete): whether products may use tiles laid out
+// for groups of tile rows; the stores there are, are given back when they may not
+PyObject* packed_grouped(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 2) throw torch::TypeError("packed_grouped takes 2 arguments");
+  Packed* p = packed_of(a[0]);
+  if (!none(a[1])) {
+    p->grouped = PyObject_IsTrue(a[1]) == 1;
+    if (!p->grouped) {
+      for (std::unique_ptr<GroupStore>& g : p->groups) g.reset();
+      p->group_calls = 0;
+    }
+  }
+  int stores = 0, done = 0;
+  for (const std::unique_ptr<GroupStore>& g : p->groups)
+    if (g != nullptr) {
+      ++stores;
+      done += g->built == nullptr ? 1 : 0;
+    }
+  return Py_BuildValue("Oii", p->grouped ? Py_True : Py_False, stores, done);
   NATIVE_END
 }
 
@@ -341,61 +374,82 @@ double group_line(const Packed* p) {
   }
 }
 bool capturing(void_stream_t st);
-void wait_for(void_stream_t st);
-// The group store that serves this product, or null.  It is built on the third product it would have served - a tensor that is
-// multiplied once or twice does not pay for it - once for each of up to two widths; the host waits until it is complete.
-const GroupStore* group_store(Packed* p, int64_t N, void_stream_t st) {
-  if (N <= 64 || p->args.nnz < 4096 || p->kind == VOID_KIND_F8E4M3) return nullptr;   // (FP8 of two terms: within 5 % either way)
+// Whether the kernels that write the store are through.  Asked without waiting; not while the stream is captured, where the
+// store then is not used.  (Another thread may be capturing: relaxed mode keeps the question from ending its capture.)
+bool complete(GroupStore* g, void_stream_t st) {
+  if (g->built == nullptr) return true;
+  if (capturing(st)) return false;
+  const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+  if (cudaEventQuery(g->built) != cudaSuccess) {
+    (void)cudaGetLastError();   // "not ready" is no error of the launch that follows
+    return false;
+  }
+  cudaEventDestroy(g->built);
+  g->built = nullptr;
+  return true;
+}
+// Queues the kernels that lay the tiles out for `shape`; null where there is no memory for it.
+std::unique_ptr<GroupStore> build_group_store(const Packed* p, const GroupShape& shape, void_stream_t st) {
+  std::unique_ptr<GroupStore> g(new GroupStore);
+  const int64_t G = shape.groups, nnz = p->args.nnz, es = elem_bytes(p->kind);
+  at::Tensor ws;
+  try {
+    const c10::Device dev(c10::kCUDA, p->device);
+    g->index = new_cuda({16 * G + (G + 4) / 4 * 4 + 8 * nnz}, at::kInt, dev);
+    g->blob = new_cuda({nnz * (1024 * es + 128) + 128}, at::kByte, dev);
+    ws = new_cuda({2 * G + nnz}, at::kInt, dev);
+  } catch (const c10::OutOfMemoryError&) {
+    return nullptr;
+  }
+  int32_t *rows = g->index.data_ptr<int32_t>(), *stages = rows + 16 * G, *records = stages + (G + 4) / 4 * 4;
+  uint8_t* blob = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(g->blob.data_ptr()) + 127) & ~uintptr_t(127));
+  g->store.blob = blob;
+  g->store.records = records;
+  g->store.stage_ptr = stages;
+  g->store.group_rows = rows;
+  g->store.n_groups = (int32_t)G;
+  g->store.max_entries = shape.entries;
+  g->store.max_tiles = shape.tiles;
+  if (cudaEventCreateWithFlags(&g->built, cudaEventDisableTiming) != cudaSuccess) return nullptr;
+  check(void_group_build(p->args.row_ptr, p->row_order, p->args.tile_cols, p->args.tiles, p->args.nbr, nnz, (int32_t)es, (int32_t)G,
+                         shape.entries, shape.tiles, rows, stages, records, blob, ws.data_ptr<int32_t>(), st),
+        "void_group_build");
+  if (cudaEventRecord(g->built, reinterpret_cast<cudaStream_t>(st)) != cudaSuccess) throw std::runtime_error("CUDA error: recording an event failed");
+  return g;
+}
+// The group store that serves this product, or null.  Its build is queued behind the third product it would have served - a
+// tensor that is multiplied once or twice does not pay for it - once for each of up to two widths.  Nothing waits for it:
+// products go to the other kernel until it is complete, and then read it on any stream and ahead of their stream's order.
+GroupStore* group_store(Packed* p, int64_t N, void_stream_t st) {
+  if (!p->grouped || N <= 64 || p->args.nnz < 4096 || p->kind == VOID_KIND_F8E4M3) return nullptr;   // (FP8 of two terms: within 5 % either way)
   const int slots = 2 * void_device_sm_count();
   if ((int64_t)p->args.nbr * ((N + 127) / 128) < 2ll * slots) return nullptr;
   const double line = group_line(p);
   const GroupShape shape = group_shape(p, N, slots);
   if (shape.saves < line) return nullptr;
-  const GroupStore* hit = nullptr;
-  double hit_saves = 0.0;
+  GroupStore* hit = nullptr;
+  double hit_saves = 0.0, best = 0.0;   // best: of those that are still being built, too
   int n = 0;
   for (; n < kMaxGroupStores && p->groups[n] != nullptr; ++n) {
     const double saves = group_saves(p, N, p->groups[n]->store.n_groups, slots);
-    if (saves > hit_saves) { hit = p->groups[n].get(); hit_saves = saves; }
+    best = std::max(best, saves);
+    if (saves > hit_saves && complete(p->groups[n].get(), st)) { hit = p->groups[n].get(); hit_saves = saves; }
   }
-  const int64_t es = elem_bytes(p->kind), tile_bytes = 1024 * es, bytes = p->args.nnz * (tile_bytes + 128);
-  if (hit_saves < 0.93 * shape.saves && n < kMaxGroupStores && p->stable && bytes <= (4ll << 30) && !capturing(st) && p->group_calls >= 0 &&
+  const int64_t bytes = p->args.nnz * (1024 * (int64_t)elem_bytes(p->kind) + 128);
+  if (best < 0.93 * shape.saves && n < kMaxGroupStores && p->stable && bytes <= (4ll << 30) && p->group_calls >= 0 && !capturing(st) &&
       ++p->group_calls >= 3) {
-    p->group_calls = -1;   // while this one is built, and for good if there is no room for it
-    std::unique_ptr<GroupStore> g(new GroupStore);
-    const int64_t G = shape.groups, nnz = p->args.nnz;
-    try {
-      const c10::Device dev(c10::kCUDA, p->device);
-      g->index = new_cuda({16 * G + (G + 4) / 4 * 4 + 8 * nnz}, at::kInt, dev);
-      g->blob = new_cuda({bytes + 128}, at::kByte, dev);
-      const at::Tensor ws = new_cuda({2 * G + nnz}, at::kInt, dev);
-      int32_t *rows = g->index.data_ptr<int32_t>(), *stages = rows + 16 * G, *records = stages + (G + 4) / 4 * 4;
-      uint8_t* blob = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(g->blob.data_ptr()) + 127) & ~uintptr_t(127));
-      g->store.blob = blob;
-      g->store.records = records;
-      g->store.stage_ptr = stages;
-      g->store.group_rows = rows;
-      g->store.n_groups = (int32_t)G;
-      g->store.max_entries = shape.entries;
-      g->store.max_tiles = shape.tiles;
-      if (void_group_build(p->args.row_ptr, p->row_order, p->args.tile_cols, p->args.tiles, p->args.nbr, nnz, (int32_t)es,
-                           (int32_t)G, shape.entries, shape.tiles, rows, stages, records, blob, ws.data_ptr<int32_t>(), st) != VOID_OK)
-        return hit_saves >= line ? hit : nullptr;
-      wait_for(st);
-    } catch (const c10::OutOfMemoryError&) {
-      return hit_saves >= line ? hit : nullptr;
-    }
-    p->group_calls = 0;
-    p->groups[n] = std::move(g);
-    return p->groups[n].get();
+    p->group_calls = -1;   // for good, if there is no room for it
+    p->groups[n] = build_group_store(p, shape, st);
+    if (p->groups[n] != nullptr) p->group_calls = 0;
   }
   return hit_saves >= line ? hit : nullptr;
 }
 // A plain product with everything filled in.
 void launch_product(Packed* p, const void_spmm_args& s, void_stream_t st) {
   if (s.transposed != 1 && s.scale_mode == VOID_SCALE_ROW_MEAN) {
-    const GroupStore* g = group_store(p, s.N, st);
+    GroupStore* g = group_store(p, s.N, st);
     if (g != nullptr) {
+      g->readers.add(c10::cuda::getCurrentCUDAStream(p->device), {&g->index, &g->blob});
       check(void_spmm_grouped(&s, &g->store, p->kind, st), "void_spmm_grouped");
       return;
     }
@@ -1079,6 +1133,7 @@ PyMethodDef kMethods[] = {
     FAST(packed_handle),
     FAST(packed_made_from),
     FAST(packed_is_current),
+    FAST(packed_grouped),
     FAST(spmm),
     FAST(spmv),
     FAST(mlp),

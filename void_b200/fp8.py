@@ -237,10 +237,9 @@ class FP8VOIDTensor:
         cache = self.__dict__.setdefault("_packed_split_cache", {})
         p = cache.get(terms)
         if p is None or not _lib.native().packed_is_current(p.native, v, sc, self.block_rows, self.block_cols, self.shape):
-            p = _spmm._mark_ready(_spmm.pack_f8_split(v.view(torch.uint8), sc, self.block_rows, self.block_cols, self.shape,
-                                                      terms))
-            _lib.native().packed_made_from(p.handle(), v, sc, self.block_rows, self.block_cols)
-            cache[terms] = p
+            p = cache[terms] = _spmm.new_store(
+                self, _spmm.pack_f8_split(v.view(torch.uint8), sc, self.block_rows, self.block_cols, self.shape, terms),
+                v, sc, self.block_rows, self.block_cols)
         return p
 
     def __repr__(self) -> str:

@@ -43,9 +43,9 @@ def packed_fp(a: VOIDTensor, kind: int) -> _spmm.PackedTiles:
     row_ptr, block_indices = getattr(a, "_row_ptr_cache", None), getattr(a, "_block_indices_cache", None)
     if row_ptr is not None and row_ptr.device != a.block_rows.device:
         row_ptr = None
-    p = _spmm._mark_ready(_spmm.pack(vals, None, a.block_rows, a.block_cols, a.shape, kind, row_ptr, block_indices))
+    p = _spmm.new_store(a, _spmm.pack(vals, None, a.block_rows, a.block_cols, a.shape, kind, row_ptr, block_indices),
+                        a.values, None, a.block_rows, a.block_cols)
     a._row_ptr_cache, a._block_indices_cache = p.row_ptr, p.block_indices
-    _lib.native().packed_made_from(p.handle(), a.values, None, a.block_rows, a.block_cols)
     cache[kind] = p
     a._plan_cache = {}
     return p
