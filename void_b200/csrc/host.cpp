@@ -21,6 +21,7 @@
 #include <cmath>
 #include <memory>
 #include <mutex>
+#include <optional>
 #include <string>
 #include <vector>
 
@@ -108,20 +109,37 @@ class Readers {
   END_HANDLE_TH_ERRORS
 
 // ------------------------------------------------------------------------------------------ packed A
-// The C ABI's view of a packed tensor and the identity (address and version) of the tensors it was made from.
+// What a store was made from, so that it is made again when its tensor has changed: the storage (held weakly, so that its
+// address cannot come back as another one's), the version of its contents and how the tensor lies in it.
 struct Identity {
+  std::optional<c10::weak_intrusive_ptr<c10::StorageImpl>> storage;   // none: no tensor
   const void* ptr = nullptr;
   int64_t version = 0;
-  bool operator==(const Identity& o) const { return ptr == o.ptr && version == o.version; }
+  at::ScalarType type = at::kFloat;
+  c10::SmallVector<int64_t, 6> layout;   // sizes, then strides
+
+  Identity() = default;
+  explicit Identity(PyObject* o) {
+    if (none(o)) return;
+    const at::Tensor& t = tensor(o, "operand");
+    storage = t.storage().getWeakStorageImpl();
+    ptr = t.const_data_ptr();
+    version = t.is_inference() ? -1 : (int64_t)t._version();
+    type = t.scalar_type();
+    layout.append(t.sizes().begin(), t.sizes().end());
+    layout.append(t.strides().begin(), t.strides().end());
+  }
+  // Inference tensors have no version: their contents may have changed at any time.
+  bool still(PyObject* o) const {
+    if (none(o)) return !storage.has_value();
+    const at::Tensor& t = tensor(o, "operand");
+    const size_t dims = (size_t)t.dim();
+    return storage.has_value() && storage->_unsafe_get_target() == t.storage().unsafeGetStorageImpl() && ptr == t.const_data_ptr() &&
+           !t.is_inference() && version == (int64_t)t._version() && type == t.scalar_type() && layout.size() == 2 * dims &&
+           std::equal(t.sizes().begin(), t.sizes().end(), layout.begin()) &&
+           std::equal(t.strides().begin(), t.strides().end(), layout.begin() + (std::ptrdiff_t)dims);
+  }
 };
-Identity identity(PyObject* o) {
-  Identity id;
-  if (none(o)) return id;
-  const at::Tensor& t = tensor(o, "operand");
-  id.ptr = t.const_data_ptr();
-  id.version = t.is_inference() ? 0 : (int64_t)t._version();
-  return id;
-}
 // The tiles of a packed tensor laid out once more for products of groups of tile rows (csrc/group.cu).
 struct GroupStore {
   at::Tensor index, blob;
@@ -211,7 +229,7 @@ PyObject* packed_made_from(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_BEGIN
   if (n != 5) throw torch::TypeError("packed_made_from takes 5 arguments");
   Packed* p = packed_of(a[0]);
-  for (int i = 0; i < 4; ++i) p->made_from[i] = identity(a[1 + i]);
+  for (int i = 0; i < 4; ++i) p->made_from[i] = Identity(a[1 + i]);
   Py_RETURN_NONE;
   NATIVE_END
 }
@@ -221,12 +239,37 @@ PyObject* packed_is_current(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 6) throw torch::TypeError("packed_is_current takes 6 arguments");
   const Packed* p = packed_of(a[0]);
   for (int i = 0; i < 4; ++i)
-    if (!(p->made_from[i] == identity(a[1 + i]))) Py_RETURN_FALSE;
+    if (!p->made_from[i].still(a[1 + i])) Py_RETURN_FALSE;
   PyObject* shape = a[5];
   if (!PyTuple_Check(shape) || PyTuple_GET_SIZE(shape) != 2 || integer(PyTuple_GET_ITEM(shape, 0)) != p->M ||
       integer(PyTuple_GET_ITEM(shape, 1)) != p->K)
     Py_RETURN_FALSE;
   Py_RETURN_TRUE;
+  NATIVE_END
+}
+
+// identity(tensor | None, ...) -> what the tensors are now; unchanged(identity, tensor | None, ...) -> whether they still are:
+// for what the Python layer derives from a tensor's fields and keeps
+constexpr const char* kIdentityName = "void_b200.identity";
+PyObject* identity(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  std::unique_ptr<std::vector<Identity>> ids(new std::vector<Identity>);
+  for (Py_ssize_t i = 0; i < n; ++i) ids->emplace_back(a[i]);
+  PyObject* c = PyCapsule_New(ids.get(), kIdentityName, [](PyObject* o) {
+    delete static_cast<std::vector<Identity>*>(PyCapsule_GetPointer(o, kIdentityName));
+  });
+  if (c != nullptr) ids.release();
+  return c;
+  NATIVE_END
+}
+PyObject* unchanged(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n < 1) throw torch::TypeError("unchanged takes an identity and its tensors");
+  const auto* ids = static_cast<const std::vector<Identity>*>(PyCapsule_GetPointer(a[0], kIdentityName));
+  if (ids == nullptr) return nullptr;
+  bool same = ids->size() == (size_t)n - 1;
+  for (Py_ssize_t i = 1; same && i < n; ++i) same = (*ids)[(size_t)i - 1].still(a[i]);
+  return PyBool_FromLong(same);
   NATIVE_END
 }
 
@@ -1134,6 +1177,8 @@ PyMethodDef kMethods[] = {
     FAST(packed_made_from),
     FAST(packed_is_current),
     FAST(packed_grouped),
+    FAST(identity),
+    FAST(unchanged),
     FAST(spmm),
     FAST(spmv),
     FAST(mlp),

@@ -286,10 +286,10 @@ def void_spmm_fp8(a: FP8VOIDTensor, b: torch.Tensor, output_dtype: torch.dtype =
             raise ValueError("b_scale belongs to an FP8 B")
         dt = b.dtype if b.dtype in (torch.float16, torch.bfloat16) else torch.float32
         cache = a.__dict__.setdefault("_dequantised", {})
-        key = (a.values_fp8.data_ptr(), a.values_fp8._version, a.scaling_info.scale.data_ptr(), a.scaling_info.scale._version)
+        made_from = _lib.native().identity(a.values_fp8, a.scaling_info.scale, a.block_rows, a.block_cols)
         hit = cache.get(dt)
-        if hit is None or hit[0] != key:
-            hit = cache[dt] = (key, a.to_void_tensor(dt))
+        if hit is None or not _lib.native().unchanged(hit[0], a.values_fp8, a.scaling_info.scale, a.block_rows, a.block_cols):
+            hit = cache[dt] = (made_from, a.to_void_tensor(dt))
         if out is None:
             out = torch.empty(a.shape[0], b.shape[1], dtype=output_dtype, device=b.device)
         return void_spmm(hit[1], b if b.dtype == dt else b.to(dt), out, activation=activation, bias=bias)
