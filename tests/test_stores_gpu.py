@@ -54,3 +54,57 @@ def test_tensors_without_versions_are_packed_for_every_product():
             a.values.mul_(2)
             q.scales.mul_(2)
             assert torch.equal(make(), want)
+
+
+def _swap_rows(t):
+    """Tile list of the matrix with its tile rows reversed, edited in place."""
+    nbr = t.block_grid[0]
+    t.block_rows.mul_(-1).add_(nbr - 1)
+
+
+@pytest.mark.parametrize("kind", ["fp32", "fp16", "int8", "streamk", "streamk_int8", "linear"])
+def test_an_edited_tile_list_is_indexed_again(kind):
+    w = _case(4, nbr=12, nbc=20, n=130)
+    a, b = w.a, w.b
+    if kind == "fp16":
+        a, b = a.half(), b.half()
+    if kind.endswith("int8"):
+        a = void.quantize_void_tensor(a)
+        bq, bs = void.quantize_cols_int8(b)
+    product = {"fp32": lambda t: void.void_spmm(t, b), "fp16": lambda t: void.void_spmm(t, b),
+               "int8": lambda t: void.void_spmm_int8(t, bq, bs), "streamk": lambda t: void.void_spmm_stream_k(t, b, n_cta=16),
+               "streamk_int8": lambda t: void.void_spmm_stream_k(t, bq, b_scale=bs, n_cta=16),
+               "linear": lambda t: void.void_linear(t, b.t().contiguous()).t()}[kind]
+    product(a)
+    a.get_row_block_info()
+    _swap_rows(a)
+    got = product(a)
+    fresh = a.to(a.values.device)                      # the same fields, nothing kept
+    fresh.block_rows, fresh.block_cols = a.block_rows.clone(), a.block_cols.clone()
+    if kind == "streamk":                              # (sums of split rows depend on the order of arrival)
+        torch.testing.assert_close(got, product(fresh), rtol=1e-5, atol=1e-4)
+    else:
+        assert torch.equal(got, product(fresh))
+    assert torch.equal(a.get_row_block_info()[0], fresh.get_row_block_info()[0])
+    a.block_rows[0] = 100                              # no longer a valid list: refused as it was before anything was kept
+    with pytest.raises(ValueError, match="invalid VOID tile list"):
+        product(a)
+    void.check_device_status()
+
+
+def test_a_layer_whose_tile_list_is_another_view_of_the_same_memory():
+    w = _case(5, nbr=6, nbc=6, n=8)
+    n = w.a.n_blocks
+    cols = torch.arange(n, dtype=torch.int32, device="cuda") % 6
+    rows = torch.arange(n, dtype=torch.int32, device="cuda") // 6
+    both = torch.stack([rows, (n - 1) // 6 - rows], 1).reshape(-1).contiguous()                  # rows and reversed rows in turn
+    x = torch.randn(5, 192, device="cuda")
+
+    def dense(r):
+        out = torch.zeros(6, 6, 32, 32, device="cuda")
+        out[r.long(), cols.long()] = w.a.values
+        return out.permute(0, 2, 1, 3).reshape(192, 192)
+
+    for r in (both[0::2], both[1::2]):
+        y = void.VOIDLinearFunction.apply(w.a.values, r, cols, (192, 192), (32, 32), n, x, None)
+        torch.testing.assert_close(y, x @ dense(r).t(), rtol=2e-3, atol=2e-3 * float(y.abs().max()))

@@ -11,6 +11,7 @@ from typing import Optional
 import torch
 
 from . import _lib
+from .format import check_indexed
 
 TILE = 32
 PANEL = 128
@@ -91,7 +92,6 @@ def _mark_ready(p: PackedTiles) -> PackedTiles:
     # capture nothing can be waited for; a store built there is simply never read early.
     # The CTAs that start first take the first work items: with the tile rows sorted by falling tile count the
     # longest rows start earliest and the shortest are left for the CTAs that share an SM with the most others.
-    from .format import check_indexed
     p.row_order, indexed = _lib.native().finish_store(p.row_ptr, p.nbr)
     if indexed is not None:
         check_indexed(indexed, p.nnz)

@@ -13,7 +13,7 @@ import torch
 from torch.autograd import Function
 
 from . import _lib
-from .format import VOIDTensor
+from .format import VOIDTensor, note_index
 
 
 # Index arrays per sparsity structure: tile index and column list of A and of A^T, work items of the tile gradient.  The
@@ -25,7 +25,8 @@ _STRUCTURE_MAX = 64
 
 def _structure(block_rows, block_cols, shape, n_blocks):
     """The native path's structure handle (csrc/host.cpp)."""
-    key = (block_rows.data_ptr(), block_cols.data_ptr(), block_rows._version, block_cols._version, shape[0], shape[1], n_blocks)
+    key = (block_rows.data_ptr(), block_cols.data_ptr(), block_rows._version, block_cols._version, shape[0], shape[1], n_blocks,
+           block_rows.is_contiguous() or block_rows.stride(), block_cols.is_contiguous() or block_cols.stride())
     hit = _STRUCTURE.get(key)
     if hit is None:
         from .format import build_tile_index
@@ -62,6 +63,7 @@ def _bare_void(values, block_rows, block_cols, shape, tile_size, n_blocks) -> VO
     if values.is_cuda and tuple(tile_size) == (32, 32):
         st = _structure(block_rows, block_cols, shape, n_blocks)
         v._row_ptr_cache, v._block_indices_cache = st[1], st[2]
+        note_index(v)
     return v
 
 

@@ -73,6 +73,19 @@ def check_tile_index(row_ptr: torch.Tensor, nnz: int) -> None:
     check_indexed(int(row_ptr[-1].item()), nnz)
 
 
+def index_is_current(owner, row_ptr) -> bool:
+    """Whether the tile index kept on a tensor still belongs to its tile list, which may have been edited or replaced."""
+    if row_ptr is None or row_ptr.device != owner.block_rows.device:
+        return False
+    known = owner.__dict__.get("_index_made_from")     # none: an index the caller handed in
+    return known is None or _lib.native().unchanged(known, owner.block_rows, owner.block_cols)
+
+
+def note_index(owner) -> None:
+    """The tile index kept on a tensor was made from its tile list as it is now."""
+    owner._index_made_from = _lib.native().identity(owner.block_rows, owner.block_cols)
+
+
 @dataclass
 class VOIDTensor:
     """VOID sparse matrix (field for field the dataclass of void/format.py:54-80)."""
@@ -153,14 +166,12 @@ class VOIDTensor:
         return out[:self.shape[0], :self.shape[1]]
 
     def get_row_block_info(self) -> Tuple[torch.Tensor, torch.Tensor]:
-        """(row_ptr, block_indices) as in void/format.py:201-237; cached on the object."""
-        cached = getattr(self, "_row_ptr_cache", None)
-        if cached is not None and cached.device == self.block_rows.device:
-            return self._row_ptr_cache, self._block_indices_cache
-        nbr, nbc = self.block_grid
-        row_ptr, block_indices = build_tile_index(self.block_rows, self.block_cols, nbr, nbc)
-        self._row_ptr_cache, self._block_indices_cache = row_ptr, block_indices
-        return row_ptr, block_indices
+        """(row_ptr, block_indices) as in void/format.py:201-237; cached on the object while its tile list stays the same."""
+        if not index_is_current(self, getattr(self, "_row_ptr_cache", None)):
+            nbr, nbc = self.block_grid
+            self._row_ptr_cache, self._block_indices_cache = build_tile_index(self.block_rows, self.block_cols, nbr, nbc)
+            note_index(self)
+        return self._row_ptr_cache, self._block_indices_cache
 
     def __repr__(self) -> str:
         return (f"VOIDTensor(shape={self.shape}, tile_size={self.tile_size}, n_blocks={self.n_blocks}, "

@@ -187,9 +187,9 @@ class FusedSparseLinear(torch.nn.Module):
 
     def get_void_tensor(self) -> VOIDTensor:
         """The VOIDTensor over the module's buffers; kept between calls so that its packed copy is reused
-        (rebuilt when the buffers move or change)."""
+        (rebuilt when the buffers are replaced)."""
         v = self._void
-        if v is None or v.values.data_ptr() != self.values.data_ptr():
+        if v is None or v.values is not self.values or v.block_rows is not self.block_rows or v.block_cols is not self.block_cols:
             v = self._void = VOIDTensor(values=self.values, block_rows=self.block_rows, block_cols=self.block_cols,
                                         morton_codes=self.morton_codes, shape=self.shape, tile_size=self.tile_size,
                                         nnz_original=0, n_blocks=self.n_blocks, density=0.0, dtype=self.values.dtype)

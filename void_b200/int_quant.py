@@ -21,6 +21,7 @@ from typing import Literal, Optional, Tuple, Union
 import torch
 
 from . import _lib, _spmm
+from .format import build_tile_index, index_is_current, note_index
 
 
 class IntFormat(Enum):
@@ -118,11 +119,11 @@ class Int8VOIDTensor:
         return self.to("cuda")
 
     def get_row_block_info(self) -> Tuple[torch.Tensor, torch.Tensor]:
-        """(row_ptr, block_indices), cached (void/int_quant.py:158-175)."""
-        if self._row_ptr is None or self._block_indices is None or self._row_ptr.device != self.block_rows.device:
-            from .format import build_tile_index
+        """(row_ptr, block_indices), cached while the tile list stays the same (void/int_quant.py:158-175)."""
+        if self._block_indices is None or not index_is_current(self, self._row_ptr):
             nbr, nbc = self.block_grid
             self._row_ptr, self._block_indices = build_tile_index(self.block_rows, self.block_cols, nbr, nbc)
+            note_index(self)
         return self._row_ptr, self._block_indices
 
     def packed(self) -> _spmm.PackedTiles:
@@ -132,6 +133,7 @@ class Int8VOIDTensor:
                                                             self.block_cols, self.shape):
             p = _spmm.cached_pack(self, self.values, self.scales, self.block_rows, self.block_cols, self.shape, _lib.KIND_I8)
             self._row_ptr, self._block_indices = p.row_ptr, p.block_indices
+            note_index(self)
         return p
 
 

@@ -12,7 +12,7 @@ from typing import Optional
 import torch
 
 from . import _lib, _spmm
-from .format import VOIDTensor
+from .format import VOIDTensor, index_is_current, note_index
 from .int_quant import Int8VOIDTensor
 
 _KIND_DTYPE = {_lib.KIND_F16: torch.float16, _lib.KIND_BF16: torch.bfloat16, _lib.KIND_TF32: torch.float32}
@@ -41,11 +41,13 @@ def packed_fp(a: VOIDTensor, kind: int) -> _spmm.PackedTiles:
         raise NotImplementedError("void_b200 kernels are built for 32x32 tiles, got tile_size=%s" % (a.tile_size,))
     vals = a.values if a.values.dtype == _KIND_DTYPE[kind] else a.values.to(_KIND_DTYPE[kind])
     row_ptr, block_indices = getattr(a, "_row_ptr_cache", None), getattr(a, "_block_indices_cache", None)
-    if row_ptr is not None and row_ptr.device != a.block_rows.device:
+    if not index_is_current(a, row_ptr):
         row_ptr = None
     p = _spmm.new_store(a, _spmm.pack(vals, None, a.block_rows, a.block_cols, a.shape, kind, row_ptr, block_indices),
                         a.values, None, a.block_rows, a.block_cols)
-    a._row_ptr_cache, a._block_indices_cache = p.row_ptr, p.block_indices
+    if row_ptr is None:
+        a._row_ptr_cache, a._block_indices_cache = p.row_ptr, p.block_indices
+        note_index(a)
     cache[kind] = p
     a._plan_cache = {}
     return p

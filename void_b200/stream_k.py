@@ -91,18 +91,18 @@ def void_spmm_stream_k(a: Int8VOIDTensor, b: torch.Tensor, workload: Optional[St
     opts = None
     if a.n_blocks != 0:
         if workload is None:
-            workload = _cached_workload(a)
+            workload = _cached_workload(a, packed)
         opts = _plan_for(a, packed, b.shape[1], workload, worker_partials is not None, n_cta).options(acc_out, worker_partials)
     return _lib.native().spmm(packed.native, b_q, out, out_dtype or torch.float32, False, col_scale, scalar, bias, None,
                               activation, False, opts)
 
 
-def _cached_workload(a) -> StreamKWorkload:
-    """The table depends on A's structure only: built once per tensor, then reused."""
-    workload = getattr(a, "_streamk_workload_cache", None)
-    if workload is None or workload.total_work != a.n_blocks:
+def _cached_workload(a, packed) -> StreamKWorkload:
+    """The table depends on A's structure only: built once per tile index, then reused."""
+    row_ptr, workload = getattr(a, "_streamk_workload_cache", (None, None))
+    if row_ptr is not packed.row_ptr or workload.total_work != a.n_blocks:
         workload = compute_stream_k_workload(a)
-        a._streamk_workload_cache = workload
+        a._streamk_workload_cache = packed.row_ptr, workload
     return workload
 
 
@@ -111,9 +111,9 @@ def _stream_k_fp(a: VOIDTensor, b, workload, out, activation, bias, worker_parti
     from . import ops
     if a.n_blocks == 0:
         return ops.void_spmm(a, b, out, activation=activation, bias=bias)
-    if workload is None:
-        workload = _cached_workload(a)
     packed = ops.packed_fp(a, ops.product_kind(a, b))
+    if workload is None:
+        workload = _cached_workload(a, packed)
     plan = _plan_for(a, packed, b.shape[1], workload, worker_partials is not None, n_cta)
     return ops.void_spmm(a, b, out, activation=activation, bias=bias, plan=plan, acc_out=acc_out,
                          worker_partials=worker_partials)
