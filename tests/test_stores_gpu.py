@@ -108,3 +108,32 @@ def test_a_layer_whose_tile_list_is_another_view_of_the_same_memory():
     for r in (both[0::2], both[1::2]):
         y = void.VOIDLinearFunction.apply(w.a.values, r, cols, (192, 192), (32, 32), n, x, None)
         torch.testing.assert_close(y, x @ dense(r).t(), rtol=2e-3, atol=2e-3 * float(y.abs().max()))
+
+
+@pytest.mark.parametrize("kind", ["fp32", "int8", "fp8", "fp8_exact", "fp8_floating", "linear", "mlp"])
+def test_a_tensor_first_used_inside_a_capture(kind):
+    w = _case(6)
+    a, b = w.a, w.b
+    q = {"int8": lambda: void.quantize_void_tensor(a), "fp8": lambda: void.void_tensor_to_fp8(a),
+         "fp8_exact": lambda: void.void_tensor_to_fp8(a), "fp8_floating": lambda: void.void_tensor_to_fp8(a)}.get(kind, lambda: a.to(a.values.device))
+    bq, bs = void.quantize_cols_int8(b) if kind == "int8" else void.quantize_cols_fp8(b)[:2]
+    back = void.VOIDTensor(a.values, a.block_cols, a.block_rows, a.morton_codes, a.shape[::-1], (32, 32), 0, a.n_blocks, 0.0)
+    product = {"fp32": lambda t: void.void_spmm(t, b), "int8": lambda t: void.void_spmm_int8(t, bq, bs),
+               "fp8": lambda t: void.void_spmm_fp8(t, bq, b_scale=bs),
+               "fp8_exact": lambda t: void.void_spmm_fp8(t, bq, b_scale=bs, scale_terms=0),
+               "fp8_floating": lambda t: void.void_spmm_fp8(t, b),
+               "linear": lambda t: void.void_linear(t, b.t().contiguous()),
+               "mlp": lambda t: void.fused_sparse_mlp(b.t().contiguous(), t, back)}[kind]
+    want = product(q())
+    t = q()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        first, second = product(t), product(t)
+    assert torch.equal(product(t), want)               # before the graph has run, its arrays hold nothing
+    for _ in range(2):
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(first, want) and torch.equal(second, want)
+    assert torch.equal(product(t), want)
+    void.check_device_status()

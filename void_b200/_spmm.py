@@ -89,7 +89,8 @@ def pack_f8_split(values: torch.Tensor, scales: Optional[torch.Tensor], block_ro
 def _mark_ready(p: PackedTiles) -> PackedTiles:
     # Building a packed store is a one-time set-up step of a tensor (a weight): the host waits here until the
     # store is complete, so that every later launch may read it ahead of its stream order.  Inside a stream
-    # capture nothing can be waited for; a store built there is simply never read early.
+    # capture nothing can be waited for, and the arrays hold nothing before the graph is replayed: a store built
+    # there is not stable, is never read early, and serves the one product it was built for (it is not kept).
     # The CTAs that start first take the first work items: with the tile rows sorted by falling tile count the
     # longest rows start earliest and the shortest are left for the CTAs that share an SM with the most others.
     p.row_order, indexed = _lib.native().finish_store(p.row_ptr, p.nbr)
@@ -125,8 +126,9 @@ def cached_pack(owner, values, scales, block_rows, block_cols, shape, kind) -> P
     p = owner.__dict__.get("_packed_cache")
     if p is None or not _lib.native().packed_is_current(p.native, values, scales, block_rows, block_cols, shape):
         p = new_store(owner, pack(values, scales, block_rows, block_cols, shape, kind), values, scales, block_rows, block_cols)
-        owner._packed_cache = p
-        owner._plan_cache = {}
+        if p.stable:
+            owner._packed_cache = p
+            owner._plan_cache = {}
     return p
 
 

@@ -237,9 +237,11 @@ class FP8VOIDTensor:
         cache = self.__dict__.setdefault("_packed_split_cache", {})
         p = cache.get(terms)
         if p is None or not _lib.native().packed_is_current(p.native, v, sc, self.block_rows, self.block_cols, self.shape):
-            p = cache[terms] = _spmm.new_store(
+            p = _spmm.new_store(
                 self, _spmm.pack_f8_split(v.view(torch.uint8), sc, self.block_rows, self.block_cols, self.shape, terms),
                 v, sc, self.block_rows, self.block_cols)
+            if p.stable:
+                cache[terms] = p
         return p
 
     def __repr__(self) -> str:
@@ -286,10 +288,12 @@ def void_spmm_fp8(a: FP8VOIDTensor, b: torch.Tensor, output_dtype: torch.dtype =
             raise ValueError("b_scale belongs to an FP8 B")
         dt = b.dtype if b.dtype in (torch.float16, torch.bfloat16) else torch.float32
         cache = a.__dict__.setdefault("_dequantised", {})
-        made_from = _lib.native().identity(a.values_fp8, a.scaling_info.scale, a.block_rows, a.block_cols)
+        fields = a.values_fp8, a.scaling_info.scale, a.block_rows, a.block_cols
         hit = cache.get(dt)
-        if hit is None or not _lib.native().unchanged(hit[0], a.values_fp8, a.scaling_info.scale, a.block_rows, a.block_cols):
-            hit = cache[dt] = (made_from, a.to_void_tensor(dt))
+        if hit is None or not _lib.native().unchanged(hit[0], *fields):
+            hit = _lib.native().identity(*fields), a.to_void_tensor(dt)
+            if not torch.cuda.is_current_stream_capturing():     # (a captured copy holds nothing before the graph is replayed)
+                cache[dt] = hit
         if out is None:
             out = torch.empty(a.shape[0], b.shape[1], dtype=output_dtype, device=b.device)
         return void_spmm(hit[1], b if b.dtype == dt else b.to(dt), out, activation=activation, bias=bias)

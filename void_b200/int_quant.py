@@ -132,8 +132,9 @@ class Int8VOIDTensor:
         if p is None or not _lib.native().packed_is_current(p.native, self.values, self.scales, self.block_rows,
                                                             self.block_cols, self.shape):
             p = _spmm.cached_pack(self, self.values, self.scales, self.block_rows, self.block_cols, self.shape, _lib.KIND_I8)
-            self._row_ptr, self._block_indices = p.row_ptr, p.block_indices
-            note_index(self)
+            if p.stable:
+                self._row_ptr, self._block_indices = p.row_ptr, p.block_indices
+                note_index(self)
         return p
 
 

@@ -45,6 +45,8 @@ def packed_fp(a: VOIDTensor, kind: int) -> _spmm.PackedTiles:
         row_ptr = None
     p = _spmm.new_store(a, _spmm.pack(vals, None, a.block_rows, a.block_cols, a.shape, kind, row_ptr, block_indices),
                         a.values, None, a.block_rows, a.block_cols)
+    if not p.stable:
+        return p
     if row_ptr is None:
         a._row_ptr_cache, a._block_indices_cache = p.row_ptr, p.block_indices
         note_index(a)
