@@ -358,8 +358,10 @@ at::Tensor transposed_copy(const at::Tensor& x_in, int es) {
         "void_transpose");
   return out;
 }
-at::Tensor fp32_vector(PyObject* o, c10::Device dev, const char* what) {
+at::Tensor fp32_vector(PyObject* o, c10::Device dev, const char* what, int64_t at_least = 0) {
   const at::Tensor& t = tensor(o, what);
+  if (t.numel() < at_least)
+    fail(std::string(what) + " must have " + std::to_string(at_least) + " elements, got " + std::to_string(t.numel()));
   if (t.scalar_type() == at::kFloat && t.device() == dev && t.is_contiguous()) return t;
   return t.to(dev, at::kFloat).contiguous();
 }
@@ -501,6 +503,15 @@ void launch_product(Packed* p, const void_spmm_args& s, void_stream_t st) {
   else check(p->kind == VOID_KIND_I8 ? void_spmm_i8(&s, st) : void_spmm_f8(&s, st), "void_spmm");
 }
 
+// An array for raw sums of four bytes each; null for None.
+void* raw_sums(PyObject* o, c10::Device dev, int64_t at_least, const char* what) {
+  if (none(o)) return nullptr;
+  const at::Tensor& t = cuda_tensor(o, what);
+  if (t.device() != dev || t.element_size() != 4 || !t.is_contiguous() || t.numel() < at_least)
+    fail(std::string(what) + " must be a contiguous tensor of at least " + std::to_string(at_least) + " 32-bit elements on B's device");
+  return t.data_ptr();
+}
+
 // spmm(handle, b, out | None, out_dtype | None, per_tile, col_scale | None, b_scale, bias | None, row_bias | None, act,
 //      transposed, options | None) -> out
 // options: (plan | None, acc_out, worker_partials, panels, stages, grid, tiles_per_stage, cta_shape, trace, flags,
@@ -532,6 +543,7 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     out = cuda_tensor(a[2], "out");
     if (out.dim() != 2 || out.size(0) != rows || out.size(1) != cols || out.stride(1) != 1)
       fail("out must be a row-major [" + std::to_string(rows) + ", " + std::to_string(cols) + "] tensor");
+    if (out.device() != dev) fail("out and B are on different devices");
   }
   const bool copied = tr && none(a[11]) && copy_pays(pk->kind, pk->args.nnz, N, pk->K);
   const at::Tensor b = copied ? transposed_copy(b_in, es) : kernel_operand(b_in, es, tr ? 0 : pk->args.nnz * ((N + 127) / 128));
@@ -545,12 +557,12 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   s.N = (int32_t)N;
   at::Tensor col_scale, bias, row_bias;   // keep converted copies alive until the launch is queued
   if (!none(a[5])) {
-    col_scale = fp32_vector(a[5], dev, "col_scale");
+    col_scale = fp32_vector(a[5], dev, "col_scale", N);
     s.col_scale = col_scale.const_data_ptr<float>();
   }
   s.b_scale = (float)real(a[6]);
   if (!none(a[7])) {
-    bias = fp32_vector(a[7], dev, "bias");
+    bias = fp32_vector(a[7], dev, "bias", N);
     s.bias = bias.const_data_ptr<float>();
   }
   if (!none(a[8])) {
@@ -589,8 +601,8 @@ PyObject* spmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
       s.counters = data_or_null<int32_t>(PyTuple_GET_ITEM(plan, 4));
       s.panels_per_item = (int32_t)integer(PyTuple_GET_ITEM(plan, 5));
     }
-    s.acc_out = data_or_null<void>(PyTuple_GET_ITEM(o, 1));
-    s.worker_partials = data_or_null<void>(PyTuple_GET_ITEM(o, 2));
+    s.acc_out = raw_sums(PyTuple_GET_ITEM(o, 1), dev, (int64_t)pk->args.nbr * 32 * N, "acc_out");
+    s.worker_partials = raw_sums(PyTuple_GET_ITEM(o, 2), dev, 0, "worker_partials");
     s.stages = (int32_t)integer(PyTuple_GET_ITEM(o, 4));
     s.grid = (int32_t)integer(PyTuple_GET_ITEM(o, 5));
     s.tiles_per_stage = (int32_t)integer(PyTuple_GET_ITEM(o, 6));
@@ -682,6 +694,7 @@ PyObject* spmv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (x.stride(0) != 1 || (reinterpret_cast<uintptr_t>(x.const_data_ptr()) & 15u) != 0) x = x.clone(at::MemoryFormat::Contiguous);
   at::Tensor out = none(a[2]) ? new_cuda({pk->M}, reinterpret_cast<THPDtype*>(a[3])->scalar_type, dev) : cuda_tensor(a[2], "out");
   if (out.dim() != 1 || out.size(0) != pk->M || out.stride(0) != 1) fail("out must be a contiguous vector of M elements");
+  if (out.device() != dev) fail("out and x are on different devices");
   void_spmm_args s = pk->args;
   s.scale_mode = VOID_SCALE_ROW_MEAN;
   s.b = x.const_data_ptr();
@@ -823,6 +836,7 @@ PyObject* quant_tiles_i8(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::ScalarType t = in.scalar_type();
   const at::Tensor v = (t == at::kFloat || t == at::kHalf || t == at::kBFloat16 ? in : in.to(at::kFloat)).contiguous();
   const int64_t count = v.size(0);
+  if (v.dim() != 3 || v.numel() != count * 1024) fail("void_b200 kernels are built for 32x32 tiles");
   at::Tensor q = new_cuda(v.sizes(), at::kChar, dev), scales = new_cuda({count}, at::kFloat, dev);
   at::Tensor zeros = new_cuda({count}, at::kChar, dev);
   at::Tensor copy[2];
@@ -845,6 +859,16 @@ PyObject* quant_tiles_i8(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_END
 }
 
+// A tile list names every stored tile once; kernels read as many coordinates as there are tiles.
+void check_list(const at::Tensor& rows, const at::Tensor& cols, int64_t tiles) {
+  TORCH_CHECK_VALUE(rows.numel() == tiles && cols.numel() == tiles, "invalid VOID tile list: ", rows.numel(), " block rows and ",
+                    cols.numel(), " block columns for ", tiles, " tiles");
+}
+void check_index(const at::Tensor& row_ptr, const at::Tensor& block_indices, int64_t nbr, int64_t tiles) {
+  TORCH_CHECK_VALUE(row_ptr.is_cuda() && block_indices.is_cuda() && row_ptr.scalar_type() == at::kInt && block_indices.scalar_type() == at::kInt &&
+                        row_ptr.is_contiguous() && block_indices.is_contiguous() && row_ptr.numel() == nbr + 1 && block_indices.numel() == tiles,
+                    "invalid VOID tile index: it does not belong to ", tiles, " tiles in ", nbr, " tile rows");
+}
 void build_index(const at::Tensor& rows, const at::Tensor& cols, int32_t nbr, int32_t nbc, at::Tensor& row_ptr, at::Tensor& block_indices,
                  void_stream_t st) {
   const c10::Device dev = rows.device();
@@ -875,6 +899,7 @@ PyObject* tile_index(PyObject*, PyObject* const* a, Py_ssize_t n) {
   c10::cuda::OptionalCUDAGuard guard(rows.device());
   const void_stream_t st = stream_of(rows.device().index());
   const int32_t nbr = (int32_t)integer(a[2]), nbc = (int32_t)integer(a[3]);
+  check_list(rows, cols, rows.numel());
   at::Tensor row_ptr, block_indices;
   build_index(rows, cols, nbr, nbc, row_ptr, block_indices, st);
   const long long indexed = indexed_tiles(row_ptr, nbr, st);
@@ -898,12 +923,14 @@ PyObject* pack_store(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t M = integer(a[4]), K = integer(a[5]), count = values.size(0);
   const int kind = (int)integer(a[6]), terms = (int)integer(a[7]), es = elem_bytes(kind);
   const int32_t nbr = (int32_t)((M + 31) / 32), nbc = (int32_t)((K + 31) / 32);
+  check_list(rows, cols, count);
   at::Tensor row_ptr, block_indices, scales;
   if (none(a[8]) || none(a[9])) {
     build_index(rows, cols, nbr, nbc, row_ptr, block_indices, st);
   } else {
     row_ptr = tensor(a[8], "row_ptr");
     block_indices = tensor(a[9], "block_indices");
+    check_index(row_ptr, block_indices, nbr, count);
   }
   if (!none(a[1])) scales = as_type(tensor(a[1], "scales"), at::kFloat).contiguous();
   const float* sc = scales.defined() ? scales.const_data_ptr<float>() : nullptr;
@@ -989,6 +1016,8 @@ PyObject* structure(PyObject*, PyObject* const* a, Py_ssize_t n) {
   st->M = integer(a[8]);
   st->K = integer(a[9]);
   st->nnz = integer(a[10]);
+  check_index(st->row_ptr[0], st->block_indices[0], (st->M + 31) / 32, st->nnz);
+  check_index(st->row_ptr[1], st->block_indices[1], (st->K + 31) / 32, st->nnz);
   PyObject* self = PyType_GenericAlloc(g_structure_type, 0);
   if (self == nullptr) return nullptr;
   new (&reinterpret_cast<StructureObject*>(self)->st) std::shared_ptr<const Structure>(std::move(st));
@@ -1012,6 +1041,10 @@ int common_kind(at::ScalarType a, at::ScalarType b) {   // their common 16-bit t
 }
 at::ScalarType kind_type(int kind) { return kind == VOID_KIND_F16 ? at::kHalf : (kind == VOID_KIND_BF16 ? at::kBFloat16 : at::kFloat); }
 
+void check_tiles(const Structure& st, const at::Tensor& values) {
+  if (values.dim() != 3 || values.size(0) != st.nnz || values.size(1) != 32 || values.size(2) != 32)
+    fail("the sparse matrix stores " + std::to_string(st.nnz) + " tiles of 32x32, got values of another shape");
+}
 // Product with tiles that change from call to call: they are packed (their transposes for A^T) and multiplied at once.
 // linear: b is x [N, K] and the result x A^T [N, M]; otherwise b is [K, N] and the result A b [M, N].
 at::Tensor product_of_values(const Structure& st, bool a_transposed, const at::Tensor& values_in, const at::Tensor& b_in,
@@ -1022,7 +1055,8 @@ at::Tensor product_of_values(const Structure& st, bool a_transposed, const at::T
   const at::Tensor values = as_type(values_in, kind_type(kind)).contiguous();
   const int64_t M = a_transposed ? st.K : st.M, K = a_transposed ? st.M : st.K;
   const int64_t N = b_in.size(linear ? 0 : 1);
-  if (b_in.size(linear ? 1 : 0) != K) fail("shape mismatch between the sparse matrix and the dense operand");
+  if (b_in.dim() != 2 || b_in.size(linear ? 1 : 0) != K) fail("shape mismatch between the sparse matrix and the dense operand");
+  check_tiles(st, values);
   const bool copied = linear && copy_pays(kind, st.nnz, N, K);
   const at::Tensor b_typed = as_type(b_in, kind_type(kind));
   const at::Tensor b = copied ? transposed_copy(b_typed, es) : kernel_operand(b_typed, es, linear ? 0 : st.nnz * ((N + 127) / 128));
@@ -1067,6 +1101,8 @@ at::Tensor product_of_values(const Structure& st, bool a_transposed, const at::T
 at::Tensor gradient_of_values(const Structure& st, const at::Tensor& g_in, const at::Tensor& x_in, at::ScalarType type, bool linear) {
   const c10::Device dev = x_in.device();
   const int64_t N = x_in.size(linear ? 0 : 1);
+  if (g_in.dim() != 2 || x_in.dim() != 2 || g_in.size(linear ? 0 : 1) != N || g_in.size(linear ? 1 : 0) != st.M || x_in.size(linear ? 1 : 0) != st.K)
+    fail("shape mismatch between the gradient, the dense operand and the sparse matrix");
   if (st.nnz == 0 || N == 0) return at::zeros({st.nnz, 32, 32}, x_in.options().dtype(type));
   const int kind = common_kind(g_in.scalar_type(), x_in.scalar_type());
   const int es = elem_bytes(kind);

@@ -67,6 +67,13 @@ def _plan_for(a, packed, N: int, workload: StreamKWorkload, per_worker: bool, n_
     return plan
 
 
+def _require_room(worker_partials, plan, N: int) -> None:
+    """Every segment of the plan writes its sums, 32 rows of N."""
+    if worker_partials is not None and worker_partials.numel() < plan.n_segs * _spmm.TILE * N:
+        raise _lib.VoidB200Error("worker_partials must have %d elements (%d segments), got %d"
+                                 % (plan.n_segs * _spmm.TILE * N, plan.n_segs, worker_partials.numel()))
+
+
 def void_spmm_stream_k(a: Int8VOIDTensor, b: torch.Tensor, workload: Optional[StreamKWorkload] = None,
                        out: Optional[torch.Tensor] = None, *, b_scale=None, out_dtype: Optional[torch.dtype] = None,
                        activation: int = 0, bias: Optional[torch.Tensor] = None,
@@ -92,7 +99,9 @@ def void_spmm_stream_k(a: Int8VOIDTensor, b: torch.Tensor, workload: Optional[St
     if a.n_blocks != 0:
         if workload is None:
             workload = _cached_workload(a, packed)
-        opts = _plan_for(a, packed, b.shape[1], workload, worker_partials is not None, n_cta).options(acc_out, worker_partials)
+        plan = _plan_for(a, packed, b.shape[1], workload, worker_partials is not None, n_cta)
+        _require_room(worker_partials, plan, b.shape[1])
+        opts = plan.options(acc_out, worker_partials)
     return _lib.native().spmm(packed.native, b_q, out, out_dtype or torch.float32, False, col_scale, scalar, bias, None,
                               activation, False, opts)
 
@@ -115,6 +124,7 @@ def _stream_k_fp(a: VOIDTensor, b, workload, out, activation, bias, worker_parti
     if workload is None:
         workload = _cached_workload(a, packed)
     plan = _plan_for(a, packed, b.shape[1], workload, worker_partials is not None, n_cta)
+    _require_room(worker_partials, plan, b.shape[1])
     return ops.void_spmm(a, b, out, activation=activation, bias=bias, plan=plan, acc_out=acc_out,
                          worker_partials=worker_partials)
 
