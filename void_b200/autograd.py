@@ -47,6 +47,8 @@ def _structure(block_rows, block_cols, shape, n_blocks):
 
 
 def _require_operands(values, tile_size, dense):
+    if torch._C._are_functorch_transforms_active():
+        raise RuntimeError("the sparse product cannot be used inside torch.func transforms (vmap, grad, jvp, ...)")
     _lib.require_cuda(values, dense)
     if tuple(tile_size) != (32, 32):
         raise NotImplementedError("void_b200 kernels are built for 32x32 tiles, got tile_size=%s" % (tile_size,))

@@ -1141,16 +1141,19 @@ struct ProductBackward : torch::autograd::Node {
   }
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
-    at::AutoDispatchBelowADInplaceOrView below;
     torch::autograd::variable_list out(3);
     if (!grads[0].defined()) return out;
+    // Unpacked with autograd on: a hook may run the user's code here, such as a checkpoint's second forward pass.
     const at::Tensor v = values.unpack(), b = dense.unpack(), g = grads[0].contiguous();
     c10::cuda::OptionalCUDAGuard guard(b.device());
+    // (a backward pass that is recorded itself gets the bias gradient from an operator that can be differentiated)
+    if (task_should_compute_output(2) && at::GradMode::is_enabled()) out[2] = g.sum(0);
+    at::AutoDispatchBelowADInplaceOrView below;
     try {
       if (task_should_compute_output(1))
         out[1] = st->nnz ? product_of_values(*st, true, v, as_type(g, b.scalar_type()), linear, nullptr) : at::zeros_like(b);
       if (task_should_compute_output(0)) out[0] = gradient_of_values(*st, g, b, v.scalar_type(), linear);
-      if (task_should_compute_output(2)) out[2] = column_sums(g);
+      if (task_should_compute_output(2) && !out[2].defined()) out[2] = column_sums(g);
     } catch (const Failure& f) {
       TORCH_CHECK(false, f.text);
     }
@@ -1169,6 +1172,9 @@ PyObject* values_product(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const bool linear = PyObject_IsTrue(a[3]) == 1;
   const at::Tensor none_given;
   const at::Tensor& bias = none(a[4]) ? none_given : tensor(a[4], "bias");
+  for (const at::Tensor* t : {&values, &b, &bias})
+    TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined(*t),
+                                "the sparse product has no forward-mode derivative: an operand carries a tangent");
   at::Tensor out;
   {
     at::AutoDispatchBelowADInplaceOrView below;
