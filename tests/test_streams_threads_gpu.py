@@ -232,3 +232,68 @@ def test_group_stores_and_captures(dtype):
     torch.cuda.synchronize()
     assert all(torch.equal(o, want) for o in out + [after_out])
     void.check_device_status()
+
+
+# ------------------------------------------------------------------------------------------ split rows of a work plan
+def _split_case(floating=False):
+    mask = workloads.zipf_mask(64, 256, 1.5, 200, 10.0, seed=7)
+    w = workloads.block_sparse(mask, 256, seed=7)
+    if floating:
+        return w.a, lambda out=None: void.void_spmm_stream_k(w.a, w.b, out=out, n_cta=48)
+    q = void.quantize_void_tensor(w.a)
+    bq, bs = void.quantize_cols_int8(w.b)
+    return q, lambda out=None: void.void_spmm_stream_k(q, bq, b_scale=bs, out=out, out_dtype=torch.float16, n_cta=48)
+
+
+@pytest.mark.parametrize("floating", [False, True])
+def test_split_rows_on_two_streams_at_once(floating):
+    a, product = _split_case(floating)
+    want = product()
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got = []
+    for _ in range(2):
+        start = torch.cuda.Event()
+        torch.cuda._sleep(20_000_000)                       # both streams have their launches queued when they start
+        start.record()
+        for s in streams:
+            s.wait_event(start)
+        for _ in range(50):
+            for s in streams:
+                with torch.cuda.stream(s):
+                    got.append(product())
+    torch.cuda.synchronize()
+    for g in got:
+        if floating:                                        # (fp32 sums of split rows depend on the order of arrival)
+            torch.testing.assert_close(g, want, rtol=1e-5, atol=1e-5 * float(want.abs().max()))
+        else:
+            assert torch.equal(g, want)
+    (plan,) = a._plan_cache.values()
+    assert len(plan.scratch) == 3 and not any(bool(c.any()) or bool(p.any()) for p, c in plan.scratch.values())
+    void.check_device_status()
+
+
+def test_split_rows_in_a_graph_beside_launches_on_other_streams():
+    q, product = _split_case()
+    want = product()
+    torch.cuda.synchronize()
+    out = torch.empty_like(want)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        for _ in range(20):
+            product(out)
+    side = torch.cuda.Stream()
+    got = []
+    for _ in range(5):
+        torch.cuda._sleep(5_000_000)
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            g.replay()
+        got += [product() for _ in range(20)]
+        side.synchronize()
+        assert torch.equal(out, want)
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, want) for x in got)
+    (plan,) = q._plan_cache.values()
+    assert len(plan.scratch) == 2 and not any(bool(c.any()) or bool(p.any()) for p, c in plan.scratch.values())
+    void.check_device_status()

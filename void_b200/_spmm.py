@@ -15,6 +15,7 @@ from .format import check_indexed
 
 TILE = 32
 PANEL = 128
+CAPTURED = -1   # launch key of a stream that is being captured; others have their stream's
 FLAG_DIRECT_STORES, FLAG_A_STABLE, FLAG_STORE_PER_TILE = 2, 4, 16   # bits of void_spmm_args.flags
 FLAG_NO_EARLY_A = 1 << 30   # host side only: never set FLAG_A_STABLE (measurements)
 
@@ -142,14 +143,18 @@ def reset_plan_scratch(device) -> None:
     dev = torch.device(device)
     for plan in list(_LIVE_PLANS):
         if plan.counters.device == dev:
-            plan.counters.zero_()
-            if plan.partials is not None:
-                plan.partials.zero_()
+            for partials, counters in list(plan.scratch.values()):
+                counters.zero_()
+                if partials is not None:
+                    partials.zero_()
 
 
 @dataclass(eq=False)
 class Plan:
-    """Work plan of void_plan_segments for one (packed tensor, column chunking, CTA count)."""
+    """Work plan of void_plan_segments for one (packed tensor, column chunking, CTA count).  The accumulators and counters of
+    split rows belong to one launch at a time, so every stream has its own (``partials`` and ``counters`` are those of the
+    stream the plan was built on).  Captured launches share one further set: graphs that hold products of the same tensor are
+    to be replayed one after the other."""
     segs: torch.Tensor
     cta_seg_ptr: torch.Tensor
     n_cta: int
@@ -162,9 +167,29 @@ class Plan:
     counters: torch.Tensor
     mode: int
     chunk_tiles: int
+    scratch: dict = field(default_factory=dict, init=False, repr=False)   # launch key: (partials, counters)
+
+    def __post_init__(self):
+        self.scratch[_lib.native().launch_key(self.counters.device.index)] = self.partials, self.counters
 
     def native_args(self) -> tuple:
-        return self.segs, self.cta_seg_ptr, self.n_cta, self.partials, self.counters, self.np
+        key = _lib.native().launch_key(self.counters.device.index)
+        partials, counters = self.scratch.get(key) or self._new_scratch(key)
+        return self.segs, self.cta_seg_ptr, self.n_cta, partials, counters, self.np
+
+    def _new_scratch(self, key: int) -> tuple:
+        """Zeroed accumulators and counters for the current stream (CAPTURED: for captured launches)."""
+        if self.partials is None:
+            return None, self.counters
+        dev, n = self.counters.device, self.partials.numel()
+        if key == CAPTURED:      # filled before the graph can run, and not by the graph: a replay leaves them zero again
+            both = _lib.native().zeroed_words(n + self.counters.numel(), dev.index)
+        else:
+            both = torch.zeros(n + self.counters.numel(), dtype=torch.int32, device=dev)
+            for t in (self.segs, self.cta_seg_ptr):
+                t.record_stream(torch.cuda.current_stream(dev))
+        self.scratch[key] = made = both[:n], both[n:]
+        return made
 
     def options(self, acc_out=None, worker_partials=None) -> tuple:
         """The native product call's options for a launch with this plan."""

@@ -765,6 +765,31 @@ bool capturing(void_stream_t st) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(reinterpret_cast<cudaStream_t>(st), &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
 }
+// launch_key(device) -> the current stream, as a key for what belongs to one stream; -1 while it is being captured
+PyObject* launch_key(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 1) throw torch::TypeError("launch_key takes 1 argument");
+  const void_stream_t st = stream_of((c10::DeviceIndex)integer(a[0]));
+  return PyLong_FromLongLong(capturing(st) ? -1 : (long long)reinterpret_cast<intptr_t>(st));
+  NATIVE_END
+}
+// zeroed_words(n, device) -> int32 [n], zero before the call returns, whatever the current stream is capturing: it is
+// allocated and cleared on another stream
+PyObject* zeroed_words(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 2) throw torch::TypeError("zeroed_words takes 2 arguments");
+  const int64_t words = integer(a[0]);
+  const c10::Device dev(c10::kCUDA, (c10::DeviceIndex)integer(a[1]));
+  c10::cuda::CUDAStream side = c10::cuda::getStreamFromPool(false, dev.index());
+  for (int i = 0; i < 64 && capturing(side.stream()); ++i) side = c10::cuda::getStreamFromPool(false, dev.index());
+  const c10::cuda::CUDAStreamGuard on_side(side);
+  const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+  const at::Tensor t = new_cuda({words}, at::kInt, dev);
+  if (cudaMemsetAsync(t.data_ptr(), 0, (size_t)words * 4, side.stream()) != cudaSuccess || cudaStreamSynchronize(side.stream()) != cudaSuccess)
+    throw std::runtime_error("CUDA error: clearing scratch memory failed");
+  return THPVariable_Wrap(t);
+  NATIVE_END
+}
 // Host memory the GPU writes a few integers to (the caching host allocator hands the same block out again).
 at::Tensor host_words(int64_t n) {
   return at::empty({n}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
@@ -1220,6 +1245,8 @@ PyMethodDef kMethods[] = {
     FAST(packed_is_current),
     FAST(packed_grouped),
     FAST(identity),
+    FAST(launch_key),
+    FAST(zeroed_words),
     FAST(unchanged),
     FAST(spmm),
     FAST(spmv),
