@@ -122,7 +122,7 @@ def load():
         if _LIB is not None:
             return _LIB
         path = _build.LIB_PATH
-        if not (os.path.exists(path) and os.path.exists(_build.NATIVE_PATH)) or (_build.needs_build() and _build.have_nvcc()):
+        if not (os.path.exists(path) and os.path.exists(_build.native_path())) or (_build.needs_build() and _build.have_nvcc()):
             path = _build.build()
         if not os.path.exists(path):
             raise VoidB200Error(
@@ -149,10 +149,11 @@ def native():
         load()
         with _LOCK:
             if _NATIVE is None:
-                if not os.path.exists(_build.NATIVE_PATH):
-                    raise VoidB200Error("void_b200: the native host library %s is missing and could not be built"
-                                        % _build.NATIVE_PATH)
-                spec = importlib.util.spec_from_file_location("void_b200._native", _build.NATIVE_PATH)
+                path = _build.native_path()
+                if not os.path.exists(path):
+                    raise VoidB200Error("void_b200: the native host library %s (for this torch, this Python and these sources) is "
+                                        "missing and could not be built" % path)
+                spec = importlib.util.spec_from_file_location("void_b200._native", path)
                 mod = importlib.util.module_from_spec(spec)
                 spec.loader.exec_module(mod)
                 mod.set_error(VoidB200Error)
