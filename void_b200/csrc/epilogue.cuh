@@ -23,6 +23,13 @@ __device__ __forceinline__ float gelu_tanh_sigmoid(float x) {
   const float two_u = 1.5957691216f * x * fmaf(0.044715f * x, x, 1.0f);
   return x * fast_sigmoid(two_u);
 }
+// One value, for the kernels whose epilogue is no loop over registers.
+__device__ __forceinline__ float activate(float x, int act) {
+  if (act == VOID_ACT_RELU) return fmaxf(x, 0.0f);
+  if (act == VOID_ACT_GELU) return gelu_tanh_sigmoid(x);
+  if (act == VOID_ACT_SILU) return x * fast_sigmoid(x);
+  return x;
+}
 // What an epilogue thread needs to know about C, read from the kernel parameters once.
 struct OutDesc {
   void* out;

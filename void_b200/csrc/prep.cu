@@ -11,6 +11,8 @@
 #include <stdlib.h>
 
 #include "../../include/void_b200.h"
+#include "epilogue.cuh"
+#include "launch.cuh"
 
 namespace vb {
 
@@ -236,15 +238,6 @@ __global__ void pack_tiles_f8_split_kernel(const uint4* __restrict__ values, con
 // (owned tile row, 128-column panel), one thread per column n: the slots hold int32 tiles [32 m][128 n], so a
 // warp reads 128 contiguous bytes per m.  contrib[row] has bit r set when rank r stored a tile for the row
 // (a rank without tiles in the row stores nothing and its slot is not read).
-__device__ __forceinline__ float reduce_act(float x, int act) {
-  if (act == VOID_ACT_RELU) return fmaxf(x, 0.0f);
-  if (act == VOID_ACT_GELU) {
-    const float two_u = 1.5957691216f * x * fmaf(0.044715f * x, x, 1.0f);
-    return x * __fdividef(1.0f, 1.0f + __expf(-two_u));
-  }
-  if (act == VOID_ACT_SILU) return x * __fdividef(1.0f, 1.0f + __expf(-x));
-  return x;
-}
 __global__ void __launch_bounds__(128) reduce_slots_kernel(const int32_t* __restrict__ slots, const uint8_t* __restrict__ contrib,
                                                            int n_ranks, int rows_owned, int row0, int n_panels,
                                                            int np, const float* __restrict__ row_scale,
@@ -276,7 +269,7 @@ __global__ void __launch_bounds__(128) reduce_slots_kernel(const int32_t* __rest
   for (int m = 0; m < 32; ++m) {
     const long long gm = (long long)grow * 32 + m;
     if (gm >= M) break;
-    const float v = reduce_act((__int2float_rn(acc[m]) * rs) * cs + bi, act);
+    const float v = activate((__int2float_rn(acc[m]) * rs) * cs + bi, act);
     const size_t o = (size_t)(lr * 32 + m) * ldc + n;
     if (out_dtype == VOID_OUT_F16) reinterpret_cast<__half*>(out)[o] = __float2half_rn(v);
     else if (out_dtype == VOID_OUT_BF16) reinterpret_cast<__nv_bfloat16*>(out)[o] = __float2bfloat16_rn(v);

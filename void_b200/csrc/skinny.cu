@@ -20,6 +20,9 @@
 #include <stdint.h>
 
 #include "../../include/void_b200.h"
+#include "epilogue.cuh"
+#include "kinds.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "skinny.cuh"
 
@@ -27,10 +30,6 @@ namespace vb {
 
 namespace {
 
-template <int KIND>
-struct Bytes {
-  static constexpr int ES = (KIND == VOID_KIND_TF32) ? 4 : ((KIND == VOID_KIND_F16 || KIND == VOID_KIND_BF16) ? 2 : 1);
-};
 template <int KIND>
 struct AccType { using T = float; };
 template <>
@@ -171,19 +170,9 @@ __device__ __forceinline__ void load_b(const uint8_t* b, long long ldb, int k0, 
   }
 }
 
-__device__ __forceinline__ float activate(float x, int act) {
-  if (act == VOID_ACT_RELU) return fmaxf(x, 0.0f);
-  if (act == VOID_ACT_GELU) {   // x sigmoid(2u) with the hardware exponential, as in spmm.cu
-    const float two_u = 1.5957691216f * x * fmaf(0.044715f * x, x, 1.0f);
-    return x * __fdividef(1.0f, 1.0f + __expf(-two_u));
-  }
-  if (act == VOID_ACT_SILU) return x * __fdividef(1.0f, 1.0f + __expf(-x));
-  return x;
-}
-
 template <int KIND, bool TR, int NG>
 __global__ void __launch_bounds__(512) skinny_kernel(const __grid_constant__ SkinnyParams p) {
-  constexpr int ES = Bytes<KIND>::ES, NB = 8 * NG;
+  constexpr int ES = Elem<KIND>::ES, NB = 8 * NG;
   using T = typename AccType<KIND>::T;
   extern __shared__ __align__(16) uint8_t smem_raw[];
   T* red = reinterpret_cast<T*>(smem_raw);   // [warps][32][NB + 1]
@@ -278,10 +267,7 @@ template <int KIND, bool TR, int NG>
 cudaError_t launch(const SkinnyParams& p, int nbr, int warps, cudaStream_t st) {
   auto kernel = skinny_kernel<KIND, TR, NG>;
   const int smem = warps * 32 * (8 * NG + 1) * 4;
-  if (smem > 48 * 1024) {
-    const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
-    if (rc != cudaSuccess) return rc;
-  }
+  if (smem > 48 * 1024 && ensure_smem((const void*)kernel, smem)) return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)nbr, (unsigned)((p.N + 8 * NG - 1) / (8 * NG)));
   cfg.blockDim = dim3((unsigned)(32 * warps));

@@ -29,16 +29,15 @@
 #include <cuda_fp16.h>
 #include <cudaTypedefs.h>
 
-#include <mutex>
-
 #include "../../include/void_b200.h"
+#include "kinds.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace vbg {
 
 using namespace vb;
 
-constexpr int kTile = 32;
 constexpr int kBlockBytes = 4096;          // 32 rows x 128 bytes: one row block, one slice of n
 constexpr int kStageBytes = 5 * kBlockBytes;
 constexpr int kStages = 4;
@@ -65,12 +64,6 @@ struct __align__(8) Bars {
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
 };
-
-template <int KIND>
-__device__ __forceinline__ void issue(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  if (KIND == VOID_KIND_TF32) mma_tf32(d, a, b, idesc, acc);
-  else mma_f16(d, a, b, idesc, acc);
-}
 
 template <int KIND, bool MN>
 __global__ void __launch_bounds__(kThreads, 2) tile_grad_kernel(const __grid_constant__ CUtensorMap tmap_b,
@@ -166,7 +159,7 @@ __global__ void __launch_bounds__(kThreads, 2) tile_grad_kernel(const __grid_con
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {  // 32 bytes of n per MMA (inside the swizzle atom), or 1024 bytes of its rows
             constexpr uint64_t kStep = MN ? (1024u >> 4) : 2u;
-            if (leader) issue<KIND>(d, ad + kStep * kk, bd + kStep * kk, idesc, acc);
+            if (leader) issue_mma<KIND>(d, ad + kStep * kk, bd + kStep * kk, idesc, acc);
             acc = 1u;
           }
           if (leader) tc_commit(smem_u32(&bars.empty[stage]));
@@ -238,23 +231,10 @@ __global__ void __launch_bounds__(kThreads, 2) tile_grad_kernel(const __grid_con
   if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
 }
 
-static PFN_cuTensorMapEncodeTiled_v12000 encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
-  });
-  return fn;
-}
-
 // A row-major matrix [rows, cols] as a tensor of 4 KB boxes: 32 rows of 128 bytes (K-major form), or 128 / es rows of 32
 // columns (MN-major form).
 static bool row_block_map(CUtensorMap* m, const void* base, int64_t ld_bytes, int rows, int cols, int es, bool mn) {
-  PFN_cuTensorMapEncodeTiled_v12000 enc = encoder();
+  PFN_cuTensorMapEncodeTiled_v12000 enc = get_encode();
   if (enc == nullptr) return false;
   const CUtensorMapDataType dt = (es == 2) ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT32;
   const cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
@@ -271,7 +251,7 @@ template <int KIND, bool MN>
 static int launch(const GradParams& p, const CUtensorMap& map_b, const CUtensorMap& map_g, int sms, cudaStream_t st) {
   auto kernel = tile_grad_kernel<KIND, MN>;
   const int smem = kStages * kStageBytes + 1024;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return VOID_ERR_CUDA;
+  if (ensure_smem((const void*)kernel, smem)) return VOID_ERR_CUDA;
   int grid = 2 * sms;
   if (grid > p.n_items) grid = p.n_items;
   kernel<<<grid, kThreads, smem, st>>>(map_b, map_g, p);
@@ -293,11 +273,9 @@ static int tile_grad(const void* grad_out, int64_t ldg, const void* b, int64_t l
         ldg < (int64_t)(mn ? M : N) * es || ldb < (int64_t)(mn ? K : N) * es)
       return VOID_ERR_ALIGN;
   }
-  int dev = 0, cc = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return VOID_ERR_CUDA;
-  cudaDeviceGetAttribute(&cc, cudaDevAttrComputeCapabilityMajor, dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cc != 10) return VOID_ERR_ARCH;
+  const DeviceInfo dev = device_info();
+  if (!dev.ok) return VOID_ERR_CUDA;
+  if (dev.cc_major != 10) return VOID_ERR_ARCH;
 
   GradParams p;
   p.items = items;
@@ -322,8 +300,8 @@ static int tile_grad(const void* grad_out, int64_t ldg, const void* b, int64_t l
     if (!row_block_map(&map_b, b, ldb, mn ? N : K, mn ? K : N, es, mn) || !row_block_map(&map_g, grad_out, ldg, mn ? N : M, mn ? M : N, es, mn))
       return VOID_ERR_TENSOR_MAP;
   }
-  if (kind == VOID_KIND_TF32) return mn ? launch<VOID_KIND_TF32, true>(p, map_b, map_g, sms, st) : launch<VOID_KIND_TF32, false>(p, map_b, map_g, sms, st);
-  return mn ? launch<VOID_KIND_F16, true>(p, map_b, map_g, sms, st) : launch<VOID_KIND_F16, false>(p, map_b, map_g, sms, st);
+  if (kind == VOID_KIND_TF32) return mn ? launch<VOID_KIND_TF32, true>(p, map_b, map_g, dev.sms, st) : launch<VOID_KIND_TF32, false>(p, map_b, map_g, dev.sms, st);
+  return mn ? launch<VOID_KIND_F16, true>(p, map_b, map_g, dev.sms, st) : launch<VOID_KIND_F16, false>(p, map_b, map_g, dev.sms, st);
 }
 
 }  // namespace vbg
