@@ -10,6 +10,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <atomic>
+
 #include "../../include/void_b200.h"
 #include "epilogue.cuh"
 #include "launch.cuh"
@@ -838,19 +840,62 @@ __global__ void streamk_fill_kernel(const int32_t* __restrict__ row_ptr, int nbr
   }
 }
 
+// Clusters of the column quantiser that run at once when its shared memory lets one and two CTAs share an SM.  A cluster
+// stays inside one group of SMs, and the groups differ from device to device, so the driver is asked, once per device.
+struct ClusterRoom { int one_per_sm = 0, two_per_sm = 0; };
+template <int KIND, bool VEC>
+static ClusterRoom cluster_room() {
+  static std::atomic<uint32_t> rooms[64];   // 1 + (two_per_sm << 16 | one_per_sm); 0: not asked yet
+  int dev = 0;
+  ClusterRoom r;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return r;
+  uint32_t packed = rooms[dev].load(std::memory_order_relaxed);
+  if (packed == 0) {
+    auto kernel = quant_cols_fused_kernel<KIND, VEC>;
+    if (ensure_smem((const void*)kernel, kFusedMaxSmem)) return r;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kFusedCtas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kFusedCtas);
+    cfg.blockDim = dim3(kFusedThreads);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int room[2] = {0, 0};
+    for (int ctas = 1; ctas <= 2; ++ctas) {
+      cfg.dynamicSmemBytes = (size_t)(kFusedMaxSmem / ctas);
+      if (cudaOccupancyMaxActiveClusters(&room[ctas - 1], kernel, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();   // no error of the launch
+        return r;
+      }
+    }
+    packed = 1u + ((uint32_t)room[1] << 16 | (uint32_t)room[0]);
+    rooms[dev].store(packed, std::memory_order_relaxed);   // (threads that ask at once store the same)
+  }
+  r.one_per_sm = (int)((packed - 1u) & 0xffffu);
+  r.two_per_sm = (int)((packed - 1u) >> 16);
+  return r;
+}
 template <int KIND, bool VEC>
 static bool launch_quant_cols_fused(const float* b, int64_t ldb, int K, int N, void* q, int64_t ldq, float* scale,
                                     float* scale_inv, cudaStream_t st) {
   auto kernel = quant_cols_fused_kernel<KIND, VEC>;
-  const unsigned ctas = (unsigned)((ldq + kFusedCols - 1) / kFusedCols) * kFusedCtas;
+  const unsigned clusters = (unsigned)((ldq + kFusedCols - 1) / kFusedCols), ctas = clusters * kFusedCtas;
   int smem = (K + kFusedCtas - 1) / kFusedCtas * kFusedCols * 4;
-  // The launch may start beside the end of the kernel before it, whose SMs come free one after the other: a grid that needs two
-  // CTAs per SM would fill the first ones with as many as fit and leave others idle.  It asks for the shared memory that keeps
-  // it to two (quantise and multiply in turn: INT8 4096^2, N = 512 14.0 -> 12.1 us, FP8 2048 x 4096, N = 384 15.9 -> 13.9;
-  // launched only after that kernel 13.7 and 15.7).  From 48 KB a CTA on there is nothing to gain (8192^2: 38.8 -> 39.4).
-  if (ctas > 128 && ctas <= 256 && smem <= 48 * 1024) smem = kFusedMaxSmem / 2;
-  if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedMaxSmem) != cudaSuccess)
-    return false;
+  if (smem > 48 * 1024 && ensure_smem((const void*)kernel, kFusedMaxSmem)) return false;
+  // The launch may start beside the end of the kernel before it, whose SMs come free one after the other: a grid that needs
+  // two CTAs per SM would fill the first ones with as many as fit and leave others idle.  It asks for the shared memory that
+  // keeps it to two, while all its clusters then still run at once: from more than fit one CTA per SM (15 here, 240 columns) to
+  // fewer than fit two (33).  Columns quantised and multiplied in turn, without and with it, us: INT8 4096^2, 90 %, N = 256
+  // 10.9 / 10.3, 384 12.8 / 11.4, 496 15.7 / 13.9, 512 14.4 / 12.6; FP8 2048 x 4096 256 13.0 / 10.6, 384 11.7 / 11.4, 512 13.7 / 12.4; FP8
+  // 4096^2 384 13.7 / 12.4, but 512 15.3 / 16.3.  Where the last cluster has just room, N = 528: INT8 16.0 / 15.0, FP8 2048 x 4096
+  // 13.0 / 15.7; where it waits for the first to end, N = 560: 16.8 / 19.3 and 13.2 / 16.3.  From 48 KB a CTA on there is nothing to
+  // gain (8192^2: 38.8 / 39.4).
+  if (smem <= 48 * 1024) {
+    const ClusterRoom room = cluster_room<KIND, VEC>();
+    if ((int)clusters > room.one_per_sm && (int)clusters < room.two_per_sm) smem = kFusedMaxSmem / 2;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(kFusedThreads);
