@@ -316,3 +316,15 @@ def test_repeated_products_of_dense_tensors_stay_the_same(dtype, m, k, density):
                 y = void.void_linear(q, x.t().contiguous().to(dtype))
             assert torch.equal(y.double(), ref.t().to(y.dtype).double())
     void.check_device_status()
+
+
+@pytest.mark.parametrize("n", [224, 240, 241, 256, 257, 512, 513, 528, 529, 544])
+def test_quantised_columns_around_the_widths_whose_grids_ask_for_more_shared_memory(n):
+    b = torch.randn(700, n, generator=torch.Generator().manual_seed(n))
+    q, s = void.quantize_cols_int8(b.cuda())
+    ref_q, ref_s = vo.quantize_int8_cols(b.numpy())
+    assert np.array_equal(s.cpu().numpy(), ref_s) and np.array_equal(q.cpu().numpy(), ref_q)
+    f, fs, fi = void.quantize_cols_fp8(b.cuda())
+    ref_f, ref_fs, ref_fi = vo.quantize_fp8_cols(b.numpy())
+    assert np.array_equal(fs.cpu().numpy(), ref_fs) and np.array_equal(fi.cpu().numpy(), ref_fi)
+    assert np.array_equal(f.view(torch.uint8).cpu().numpy(), ref_f)
