@@ -328,3 +328,16 @@ def test_quantised_columns_around_the_widths_whose_grids_ask_for_more_shared_mem
     ref_f, ref_fs, ref_fi = vo.quantize_fp8_cols(b.numpy())
     assert np.array_equal(fs.cpu().numpy(), ref_fs) and np.array_equal(fi.cpu().numpy(), ref_fi)
     assert np.array_equal(f.view(torch.uint8).cpu().numpy(), ref_f)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("off", [0, 1, 3, 8])
+def test_tiles_are_quantised_wherever_they_start(dtype, off):
+    n = 5
+    flat = torch.randn(n * 1024 + off, generator=torch.Generator().manual_seed(off)).to(dtype)
+    values = flat.cuda()[off:].view(n, 32, 32)
+    coords = torch.arange(n, dtype=torch.int32, device="cuda")
+    a = void.VOIDTensor(values, coords, coords, torch.zeros(n, dtype=torch.int64, device="cuda"), (n * 32, n * 32), (32, 32), 0, n, 0.0)
+    q = void.quantize_void_tensor(a)
+    ref_q, ref_s = vo.quantize_int8_tiles(flat[off:].view(n, 32, 32).float().numpy())
+    assert np.array_equal(q.values.cpu().numpy(), ref_q) and np.array_equal(q.scales.cpu().numpy(), ref_s)

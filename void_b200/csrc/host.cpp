@@ -859,7 +859,8 @@ PyObject* quant_tiles_i8(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const c10::Device dev = in.device();
   c10::cuda::OptionalCUDAGuard guard(dev);
   const at::ScalarType t = in.scalar_type();
-  const at::Tensor v = (t == at::kFloat || t == at::kHalf || t == at::kBFloat16 ? in : in.to(at::kFloat)).contiguous();
+  at::Tensor v = (t == at::kFloat || t == at::kHalf || t == at::kBFloat16 ? in : in.to(at::kFloat)).contiguous();
+  if ((reinterpret_cast<uintptr_t>(v.const_data_ptr()) & 15u) != 0) v = v.clone();   // the kernel loads 16 bytes at a time
   const int64_t count = v.size(0);
   if (v.dim() != 3 || v.numel() != count * 1024) fail("void_b200 kernels are built for 32x32 tiles");
   at::Tensor q = new_cuda(v.sizes(), at::kChar, dev), scales = new_cuda({count}, at::kFloat, dev);
