@@ -137,3 +137,39 @@ def test_a_tensor_first_used_inside_a_capture(kind):
         assert torch.equal(first, want) and torch.equal(second, want)
     assert torch.equal(product(t), want)
     void.check_device_status()
+
+
+@pytest.mark.parametrize("how", ["deepcopy", "copy", "file"])
+@pytest.mark.parametrize("kind", ["fp32", "int8", "fp8", "fp8_floating", "streamk", "module", "layer"])
+def test_tensors_that_were_multiplied_can_be_copied_and_saved(kind, how, tmp_path):
+    import copy
+    w = _case(7, n=130)
+    b, bt = w.b, w.b.t().contiguous()
+    bq, bs = void.quantize_cols_fp8(b)[:2] if kind == "fp8" else void.quantize_cols_int8(b)
+    t = {"int8": lambda: void.quantize_void_tensor(w.a), "streamk": lambda: void.quantize_void_tensor(w.a),
+         "fp8": lambda: void.void_tensor_to_fp8(w.a), "fp8_floating": lambda: void.void_tensor_to_fp8(w.a),
+         "module": lambda: void.FusedSparseLinear(224, 288, w.a), "layer": lambda: void.SparseLinear(224, 288, w.a)}.get(kind, lambda: w.a)()
+    product = {"fp32": lambda x: void.void_spmm(x, b), "int8": lambda x: void.void_spmm_int8(x, bq, bs),
+               "streamk": lambda x: void.void_spmm_stream_k(x, bq, b_scale=bs, n_cta=16),
+               "fp8": lambda x: void.void_spmm_fp8(x, bq, b_scale=bs), "fp8_floating": lambda x: void.void_spmm_fp8(x, b),
+               "module": lambda x: x(bt), "layer": lambda x: x(bt).detach()}[kind]
+    want = product(t)
+    if how == "file":
+        torch.save(t, tmp_path / "t.pt")
+        again = torch.load(tmp_path / "t.pt", weights_only=False)
+    else:
+        again = getattr(copy, how)(t)
+    assert torch.equal(product(again), want) and torch.equal(product(t), want)
+    if hasattr(again, "get_row_block_info"):
+        assert torch.equal(again.get_row_block_info()[0], t.get_row_block_info()[0])
+
+
+def test_states_of_earlier_versions_are_read_without_what_they_derived():
+    w = _case(8)
+    q = void.quantize_void_tensor(w.a)
+    bq, bs = void.quantize_cols_int8(w.b)
+    want = void.void_spmm_int8(q, bq, bs)
+    old = dict(q.__getstate__(), _packed_cache=object(), _plan_cache={1: 2}, _streamk_workload_cache=object())
+    again = void.Int8VOIDTensor.__new__(void.Int8VOIDTensor)
+    again.__setstate__(old)
+    assert torch.equal(void.void_spmm_int8(again, bq, bs), want)

@@ -7,7 +7,7 @@ device="cuda", the format itself (kept tiles, Morton order, tile values) are bui
 library; there is no CPU compute path.
 """
 import warnings
-from dataclasses import dataclass
+from dataclasses import dataclass, fields
 from typing import Tuple, Union
 
 import numpy as np
@@ -81,13 +81,30 @@ def index_is_current(owner, row_ptr) -> bool:
     return known is None or _lib.native().unchanged(known, owner.block_rows, owner.block_cols)
 
 
+class Derived:
+    """What tensors of tiles have in common: everything kept on one beside its fields (packed stores, plans, the tile index)
+    is derived from them, so copies and files carry the fields alone and derive it again."""
+
+    def __getstate__(self):
+        state = {f.name: getattr(self, f.name) for f in fields(self)}
+        if "_group_stores" in self.__dict__:           # what the user allowed (allow_group_stores)
+            state["_group_stores"] = self._group_stores
+        if "_index_made_from" in self.__dict__:        # an index that was built here, not handed in
+            state.update((name, None) for name in ("_row_ptr", "_block_indices") if name in state)
+        return state
+
+    def __setstate__(self, state):
+        names = {f.name for f in fields(self)} | {"_group_stores"}     # (files of earlier versions carry more)
+        self.__dict__.update((k, v) for k, v in state.items() if k in names)
+
+
 def note_index(owner) -> None:
     """The tile index kept on a tensor was made from its tile list as it is now."""
     owner._index_made_from = _lib.native().identity(owner.block_rows, owner.block_cols)
 
 
 @dataclass
-class VOIDTensor:
+class VOIDTensor(Derived):
     """VOID sparse matrix (field for field the dataclass of void/format.py:54-80)."""
     values: torch.Tensor          # [n_blocks, tile_m, tile_n]
     block_rows: torch.Tensor      # [n_blocks] int32

@@ -21,6 +21,7 @@ from typing import Literal, Optional, Tuple, Union
 import torch
 
 from . import _lib, _spmm
+from .format import Derived
 
 
 class FP8Format(Enum):
@@ -171,7 +172,7 @@ def dequantize_from_fp8(tensor: torch.Tensor, scaling_info: FP8ScalingInfo,
 
 
 @dataclass
-class FP8VOIDTensor:
+class FP8VOIDTensor(Derived):
     """VOID tensor with FP8 storage (void/fp8.py:438-570)."""
     values_fp8: torch.Tensor
     scaling_info: FP8ScalingInfo

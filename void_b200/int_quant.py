@@ -21,7 +21,7 @@ from typing import Literal, Optional, Tuple, Union
 import torch
 
 from . import _lib, _spmm
-from .format import build_tile_index, index_is_current, note_index
+from .format import Derived, build_tile_index, index_is_current, note_index
 
 
 class IntFormat(Enum):
@@ -83,7 +83,7 @@ class QuantizationParams:
 
 
 @dataclass
-class Int8VOIDTensor:
+class Int8VOIDTensor(Derived):
     """Quantised VOID tensor (void/int_quant.py:105-175)."""
     values: torch.Tensor        # int8 [n_blocks, tile_m, tile_k]
     scales: torch.Tensor        # float32 [n_blocks]
