@@ -1,8 +1,8 @@
 // Products of groups of tile rows that share B's panels:  C = act(dequant(A . B) + bias).
 //
-// The row-accumulate kernel of spmm.cu fetches a panel of B for every stored tile.  Its large products run at what an SM
-// takes in from L2 - measured 66 - 76 bytes per clock with every SM loading, whatever else it does - so only fewer bytes
-// make them faster.  Here a CTA (two per SM) owns up to eight tile rows at once, their accumulators for a panel of 128
+// The row-accumulate kernel of spmm.cu fetches a panel of B for every stored tile.  Its large products bring 52 - 64 bytes per
+// clock into an SM, where a kernel that does nothing but load from L2 reaches 66 - 70 with every SM loading, so fewer bytes are
+// what makes them faster.  Here a CTA (two per SM) owns up to eight tile rows at once, their accumulators for a panel of 128
 // columns in tensor memory, and walks the block columns that ANY of its rows stores: a panel is fetched once and multiplied
 // by the 1 ... R tiles of that column.  With density d a panel serves R d / (1 - (1 - d)^R) tiles: 1.3 at 90 % sparsity and
 // R = 7, 2.3 at 70 %, 3.5 at 50 %.  Measured against that kernel, 8192^2, N = 1024, us: fp16 50 % 132 -> 95, 70 % 84 -> 66,

@@ -302,7 +302,7 @@ PyObject* packed_grouped(PyObject*, PyObject* const* a, Py_ssize_t n) {
 int64_t padded_pitch(int64_t cols, int es) { return (cols * es + 63) / 64 * 64 / es; }
 // B with unit column stride and rows on 16-byte boundaries, as the copy engine needs them; others are copied (one pass).
 // A single row has no pitch, so only its start matters.  Whole panels (products: the (tile, 128 columns) pairs that read one) of
-// rows that start on 16 bytes but not on 32 load slower, by 0.2 ns a pair for 16-bit and 0.12 for 8-bit elements, so large
+// rows that start on 16 bytes but not on 32 load slower, by 0.17 ns a pair for 16-bit and 0.12 for 8-bit elements, so large
 // products have them copied too: N = 1000, 8192^2, 80 %: fp16 98 -> 75 us and 6.5 for the copy, INT8 49 -> 36 and 6.
 at::Tensor kernel_operand(const at::Tensor& b, int es, int64_t products = 0) {
   if (b.element_size() != es)
