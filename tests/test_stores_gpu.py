@@ -173,3 +173,57 @@ def test_states_of_earlier_versions_are_read_without_what_they_derived():
     again = void.Int8VOIDTensor.__new__(void.Int8VOIDTensor)
     again.__setstate__(old)
     assert torch.equal(void.void_spmm_int8(again, bq, bs), want)
+
+
+@pytest.mark.parametrize("kind", ["fp32", "int8", "fp8", "fp8_exact", "fp8_floating", "streamk", "spmv", "mlp"])
+def test_a_graph_keeps_reading_what_it_was_captured_with(kind):
+    w = _case(9, nbr=12, nbc=20, n=130)
+    a, b = w.a, w.b
+    bq, bs = void.quantize_cols_fp8(b)[:2] if kind.startswith("fp8") else void.quantize_cols_int8(b)
+    t = void.void_tensor_to_fp8(a) if kind.startswith("fp8") else (void.quantize_void_tensor(a) if kind in ("int8", "streamk") else a)
+    back = void.VOIDTensor(a.values.clone(), a.block_cols, a.block_rows, a.morton_codes, a.shape[::-1], (32, 32), 0, a.n_blocks, 0.0)
+    bt = b.t().contiguous()
+    product = {"fp32": lambda: void.void_spmm(t, b), "int8": lambda: void.void_spmm_int8(t, bq, bs),
+               "fp8": lambda: void.void_spmm_fp8(t, bq, b_scale=bs), "fp8_exact": lambda: void.void_spmm_fp8(t, bq, b_scale=bs, scale_terms=0),
+               "fp8_floating": lambda: void.void_spmm_fp8(t, b), "streamk": lambda: void.void_spmm_stream_k(t, bq, b_scale=bs, n_cta=16),
+               "spmv": lambda: void.void_spmv(t, b[:, 0].contiguous()), "mlp": lambda: void.fused_sparse_mlp(bt, t, back)}[kind]
+    want = product()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = product()
+    scale = t.scaling_info.scale if kind.startswith("fp8") else (t.scales if kind in ("int8", "streamk") else t.values)
+    for _ in range(2):
+        scale.mul_(2)                                  # the tensor's own products follow it ...
+        new = product()
+    assert not torch.equal(new, want)
+    junk = [torch.full((n,), 0x55, dtype=torch.uint8, device="cuda") for n in (512, 4096, 1 << 16, 1 << 18, 1 << 19, 1 << 20) for _ in range(40)]
+    g.replay()                                         # ... the graph multiplies what it was captured with
+    torch.cuda.synchronize()
+    assert torch.equal(out, want) and len(junk) == 240
+    assert len(t._captured_stores) == 1
+    void.check_device_status()
+
+
+def test_structures_that_a_graph_reads_are_not_dropped(monkeypatch):
+    from void_b200 import autograd
+    monkeypatch.setattr(autograd, "_STRUCTURE", {})
+    monkeypatch.setattr(autograd, "_STRUCTURE_MAX", 2)
+    layers = []
+    for seed in range(4):
+        w = _case(10 + seed)
+        layers.append(void.SparseLinear(224, 288, w.a))
+    x = torch.randn(40, 224, device="cuda")
+    with torch.no_grad():
+        want = layers[0](x)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            out = layers[0](x)
+        first = next(iter(autograd._STRUCTURE))
+        for layer in layers[1:]:
+            layer(x)
+        assert len(autograd._STRUCTURE) == 2 and first in autograd._STRUCTURE
+        g.replay()
+        assert torch.equal(out, want)
+    void.check_device_status()

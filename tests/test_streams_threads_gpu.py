@@ -297,3 +297,25 @@ def test_split_rows_in_a_graph_beside_launches_on_other_streams():
     (plan,) = q._plan_cache.values()
     assert len(plan.scratch) == 2 and not any(bool(c.any()) or bool(p.any()) for p, c in plan.scratch.values())
     void.check_device_status()
+
+
+@pytest.mark.parametrize("dtype", GROUPED)
+def test_a_refused_group_store_that_a_graph_reads_stays(dtype):
+    a, product, packed = _grouped_case(dtype, 8)
+    want = product()
+    for _ in range(4):
+        product()
+    torch.cuda.synchronize()
+    product()
+    assert _stores(packed) == (True, 1, 1)
+    out = torch.empty_like(want)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        product(out)
+    before = torch.cuda.memory_allocated()
+    void.allow_group_stores(a, False)
+    assert _stores(packed) == (False, 0, 0) and torch.cuda.memory_allocated() == before
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want) and torch.equal(product(), want)
+    void.check_device_status()

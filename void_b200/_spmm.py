@@ -105,12 +105,21 @@ def allow_group_stores(a, allowed: bool) -> None:
     """Whether products of ``a`` (VOIDTensor, Int8VOIDTensor) may keep its tiles a second time, laid out for groups of tile
     rows (by default they may).  From the third large product of a rather dense tensor on, such a store - as large as the
     packed tiles and an eighth more for 8-bit tiles, at most 4 GB, for up to two widths of B - is built behind a product and
-    used once it is complete.  False gives the stores of ``a`` back and keeps further ones from being built."""
+    used once it is complete.  False gives the stores of ``a`` back - those that a captured graph reads, with ``a`` itself - and
+    keeps further ones from being built."""
     a._group_stores = bool(allowed)
     d = a.__dict__
     for p in (d.get("_packed_cache"), *d.get("_packed_fp_cache", {}).values()):
         if p is not None:
             _lib.native().packed_grouped(p.handle(), bool(allowed))
+
+
+def retire(owner, *stores) -> None:
+    """Stores of ``owner`` whose place is being taken: those that a captured graph reads, and their plans, stay as long as
+    ``owner`` does, so that a replay reads what it was captured with."""
+    kept = [p for p in stores if p is not None and p.native is not None and _lib.native().packed_captured(p.native)]
+    if kept:
+        owner.__dict__.setdefault("_captured_stores", []).append((kept, owner.__dict__.get("_plan_cache")))
 
 
 def new_store(owner, p: PackedTiles, *made_from) -> PackedTiles:
@@ -126,8 +135,10 @@ def cached_pack(owner, values, scales, block_rows, block_cols, shape, kind) -> P
     """Packed store cached on the tensor object, rebuilt when its storage or contents change."""
     p = owner.__dict__.get("_packed_cache")
     if p is None or not _lib.native().packed_is_current(p.native, values, scales, block_rows, block_cols, shape):
-        p = new_store(owner, pack(values, scales, block_rows, block_cols, shape, kind), values, scales, block_rows, block_cols)
+        old, p = p, new_store(owner, pack(values, scales, block_rows, block_cols, shape, kind), values, scales, block_rows,
+                              block_cols)
         if p.stable:
+            retire(owner, old)
             owner._packed_cache = p
             owner._plan_cache = {}
     return p

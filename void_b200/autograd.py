@@ -40,8 +40,11 @@ def _structure(block_rows, block_cols, shape, n_blocks):
                                      tile_grad_items(row_ptr), _lib.status_word(block_rows.device), shape[0], shape[1], n_blocks,
                                      _lib.native().finish_store(row_ptr, nbr)[0], _lib.native().finish_store(row_ptr_t, nbc)[0])
         hit = (st, row_ptr, block_indices, block_rows, block_cols)     # keeps the keys alive
-        if len(_STRUCTURE) >= _STRUCTURE_MAX:
-            _STRUCTURE.pop(next(iter(_STRUCTURE)), None)
+        if len(_STRUCTURE) >= _STRUCTURE_MAX:              # the oldest that no captured graph reads
+            for old in list(_STRUCTURE):
+                if not _lib.native().structure_captured(_STRUCTURE[old][0]):
+                    _STRUCTURE.pop(old, None)
+                    break
         _STRUCTURE[key] = hit
     return hit
 

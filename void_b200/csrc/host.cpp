@@ -18,6 +18,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <memory>
 #include <mutex>
@@ -85,14 +86,19 @@ class Readers {
   // the stream all arrays were allocated on, where that is known
   void home(cudaStream_t stream) { seen_.push_back(stream); }
   void add(c10::cuda::CUDAStream stream, std::initializer_list<const at::Tensor*> arrays) {
+    const intptr_t key = reinterpret_cast<intptr_t>(stream.stream());
+    if (last_.load(std::memory_order_acquire) == key) return;
     const std::lock_guard<std::mutex> lock(mutex_);
-    if (std::find(seen_.begin(), seen_.end(), stream.stream()) != seen_.end()) return;
-    for (const at::Tensor* t : arrays)
-      if (t->defined()) c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), stream);
-    seen_.push_back(stream.stream());
+    if (std::find(seen_.begin(), seen_.end(), stream.stream()) == seen_.end()) {
+      for (const at::Tensor* t : arrays)
+        if (t->defined()) c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), stream);
+      seen_.push_back(stream.stream());
+    }
+    last_.store(key, std::memory_order_release);
   }
 
  private:
+  std::atomic<intptr_t> last_{-1};   // the last one added
   std::mutex mutex_;
   std::vector<cudaStream_t> seen_;
 };
@@ -145,6 +151,7 @@ struct GroupStore {
   at::Tensor index, blob;
   void_group_store store = {};
   cudaEvent_t built = nullptr;   // behind the kernels that write it; null once it is known to be complete
+  bool captured = false;         // a graph reads it
   Readers readers;
   GroupStore() = default;
   GroupStore(const GroupStore&) = delete;
@@ -168,6 +175,8 @@ struct Packed {
   std::unique_ptr<GroupStore> groups[kMaxGroupStores];   // null: not built
   int32_t group_calls = 0;    // products a group store would have served since the last build; -1: there was no room for one
   bool grouped = true;        // whether group stores may be built and used
+  bool captured = false;      // a graph was captured that reads these arrays, and may be replayed as long as the tensor lives
+  std::vector<std::unique_ptr<GroupStore>> retired;   // group stores that are no longer used, but read by a graph
 };
 struct PackedObject {
   PyObject_HEAD
@@ -183,10 +192,12 @@ template <typename T>
 T* data_or_null(PyObject* o) {
   return none(o) ? nullptr : static_cast<T*>(tensor(o, "operand").data_ptr());
 }
+bool capturing(void_stream_t st);
 // The stream a product of this store is launched on, noted as one of its readers.
 void_stream_t launch_stream(Packed* p) {
   const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(p->device);
   p->readers.add(stream, {&p->tiles, &p->tile_cols, &p->tile_scales, &p->row_ptr, &p->row_scale_array, &p->row_order_array});
+  if (capturing(stream.stream())) p->captured = true;
   return stream.stream();
 }
 
@@ -273,8 +284,16 @@ PyObject* unchanged(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_END
 }
 
+// packed_captured(handle) -> whether a graph reads this store: then it is kept when another takes its place
+PyObject* packed_captured(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 1) throw torch::TypeError("packed_captured takes 1 argument");
+  return PyBool_FromLong(packed_of(a[0])->captured);
+  NATIVE_END
+}
+
 // packed_grouped(handle, allowed | None) -> (allowed, group stores, of them complete): whether products may use tiles laid out
-// for groups of tile rows; the stores there are, are given back when they may not
+// for groups of tile rows; the stores there are, are given back when they may not (those a graph reads with the tensor)
 PyObject* packed_grouped(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_BEGIN
   if (n != 2) throw torch::TypeError("packed_grouped takes 2 arguments");
@@ -282,7 +301,10 @@ PyObject* packed_grouped(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!none(a[1])) {
     p->grouped = PyObject_IsTrue(a[1]) == 1;
     if (!p->grouped) {
-      for (std::unique_ptr<GroupStore>& g : p->groups) g.reset();
+      for (std::unique_ptr<GroupStore>& g : p->groups) {
+        if (g != nullptr && g->captured) p->retired.push_back(std::move(g));
+        g.reset();
+      }
       p->group_calls = 0;
     }
   }
@@ -418,7 +440,6 @@ double group_line(const Packed* p) {
     default: return 1.45;
   }
 }
-bool capturing(void_stream_t st);
 // Whether the kernels that write the store are through.  Asked without waiting; not while the stream is captured, where the
 // store then is not used.  (Another thread may be capturing: relaxed mode keeps the question from ending its capture.)
 bool complete(GroupStore* g, void_stream_t st) {
@@ -495,6 +516,7 @@ void launch_product(Packed* p, const void_spmm_args& s, void_stream_t st) {
     GroupStore* g = group_store(p, s.N, st);
     if (g != nullptr) {
       g->readers.add(c10::cuda::getCurrentCUDAStream(p->device), {&g->index, &g->blob});
+      if (p->captured && capturing(st)) g->captured = true;
       check(void_spmm_grouped(&s, &g->store, p->kind, st), "void_spmm_grouped");
       return;
     }
@@ -762,6 +784,7 @@ void wait_for(void_stream_t st) {
   if (rc != cudaSuccess) throw std::runtime_error(std::string("CUDA error: ") + cudaGetErrorString(rc));
 }
 bool capturing(void_stream_t st) {
+  if (st == nullptr) return false;   // the legacy default stream is never captured; asking costs 0.3 us
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(reinterpret_cast<cudaStream_t>(st), &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
 }
@@ -1018,6 +1041,7 @@ struct Structure {
   at::Tensor items, status;
   int64_t M = 0, K = 0, nnz = 0;
   mutable Readers readers;
+  mutable std::atomic<bool> captured{false};   // a graph reads these arrays
 };
 struct StructureObject {
   PyObject_HEAD
@@ -1054,11 +1078,19 @@ void_stream_t launch_stream(const Structure& st, c10::Device dev) {
   const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(dev.index());
   st.readers.add(stream, {&st.row_ptr[0], &st.row_ptr[1], &st.block_indices[0], &st.block_indices[1], &st.tile_cols[0], &st.tile_cols[1],
                           &st.row_order[0], &st.row_order[1], &st.items});
+  if (capturing(stream.stream())) st.captured.store(true, std::memory_order_relaxed);
   return stream.stream();
 }
 std::shared_ptr<const Structure> structure_of(PyObject* o) {
   if (Py_TYPE(o) != g_structure_type) throw torch::TypeError("expected a structure handle");
   return reinterpret_cast<StructureObject*>(o)->st;
+}
+// structure_captured(structure) -> whether a graph reads its arrays
+PyObject* structure_captured(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  NATIVE_BEGIN
+  if (n != 1) throw torch::TypeError("structure_captured takes 1 argument");
+  return PyBool_FromLong(structure_of(a[0])->captured.load(std::memory_order_relaxed));
+  NATIVE_END
 }
 int common_kind(at::ScalarType a, at::ScalarType b) {   // their common 16-bit type, else fp32 operands (TF32)
   if (a == b && a == at::kHalf) return VOID_KIND_F16;
@@ -1244,6 +1276,7 @@ PyMethodDef kMethods[] = {
     FAST(packed_handle),
     FAST(packed_made_from),
     FAST(packed_is_current),
+    FAST(packed_captured),
     FAST(packed_grouped),
     FAST(identity),
     FAST(launch_key),
@@ -1259,6 +1292,7 @@ PyMethodDef kMethods[] = {
     FAST(pack_store),
     FAST(finish_store),
     FAST(structure),
+    FAST(structure_captured),
     FAST(values_product),
     FAST(tile_gradient),
     {nullptr, nullptr, 0, nullptr},

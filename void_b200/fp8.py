@@ -238,10 +238,11 @@ class FP8VOIDTensor(Derived):
         cache = self.__dict__.setdefault("_packed_split_cache", {})
         p = cache.get(terms)
         if p is None or not _lib.native().packed_is_current(p.native, v, sc, self.block_rows, self.block_cols, self.shape):
-            p = _spmm.new_store(
+            old, p = p, _spmm.new_store(
                 self, _spmm.pack_f8_split(v.view(torch.uint8), sc, self.block_rows, self.block_cols, self.shape, terms),
                 v, sc, self.block_rows, self.block_cols)
             if p.stable:
+                _spmm.retire(self, old)
                 cache[terms] = p
         return p
 
@@ -292,6 +293,8 @@ def void_spmm_fp8(a: FP8VOIDTensor, b: torch.Tensor, output_dtype: torch.dtype =
         fields = a.values_fp8, a.scaling_info.scale, a.block_rows, a.block_cols
         hit = cache.get(dt)
         if hit is None or not _lib.native().unchanged(hit[0], *fields):
+            if hit is not None:
+                _spmm.retire(a, *hit[1].__dict__.get("_packed_fp_cache", {}).values())
             hit = _lib.native().identity(*fields), a.to_void_tensor(dt)
             if not torch.cuda.is_current_stream_capturing():     # (a captured copy holds nothing before the graph is replayed)
                 cache[dt] = hit

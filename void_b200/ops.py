@@ -47,6 +47,7 @@ def packed_fp(a: VOIDTensor, kind: int) -> _spmm.PackedTiles:
                         a.values, None, a.block_rows, a.block_cols)
     if not p.stable:
         return p
+    _spmm.retire(a, hit)
     if row_ptr is None:
         a._row_ptr_cache, a._block_indices_cache = p.row_ptr, p.block_indices
         note_index(a)
