@@ -11,7 +11,7 @@ from void_b200 import workloads
 
 pytestmark = pytest.mark.gpu
 
-BUSY = 400_000_000     # clocks a stream is kept busy: 0.2 s, far longer than the host work behind it takes
+BUSY = 1_000_000_000     # clocks a stream is kept busy: half a second, far longer than the host work behind it takes
 
 
 def _blocks_handed_out(nbytes, count):
