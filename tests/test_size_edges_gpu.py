@@ -341,3 +341,40 @@ def test_tiles_are_quantised_wherever_they_start(dtype, off):
     q = void.quantize_void_tensor(a)
     ref_q, ref_s = vo.quantize_int8_tiles(flat[off:].view(n, 32, 32).float().numpy())
     assert np.array_equal(q.values.cpu().numpy(), ref_q) and np.array_equal(q.scales.cpu().numpy(), ref_s)
+
+
+# ------------------------------------------------------------------------------------------ passes over the columns of B
+@pytest.mark.parametrize("dtype,k,n,linear", [
+    ("int8", 65536, 512, False), ("int8", 65536, 600, False), ("int8", 65536, 1153, False), ("fp8", 65536, 641, False),
+    (torch.bfloat16, 32768, 600, False), (torch.float16, 32768, 600, True), (torch.float32, 16384, 513, False),
+    (torch.float32, 16384, 600, True)])
+def test_products_in_passes_equal_products_of_few_columns(dtype, k, n, linear):
+    """A B above three tenths of the L2 is multiplied in passes over its columns (the last one shorter), every product as in
+    one of a few columns.  Small integers for the floating kinds, whose sums in any order are exact."""
+    m, step, floating = 90, 256, isinstance(dtype, torch.dtype)
+    gen = torch.Generator(device="cuda").manual_seed(k + n)
+    mask = torch.rand(3, k // 32, generator=gen, device="cuda") < 0.05
+    mask[1] = False
+    numbers = lambda *size: (torch.randint(-2, 3, size, generator=gen, device="cuda").float() if floating
+                             else torch.randn(*size, generator=gen, device="cuda"))
+    a = void.void_from_block_mask(mask.cpu().numpy(), numbers(int(mask.sum()), 32, 32), shape=(m, k))
+    a.values[a.block_rows == m // 32, m % 32:, :] = 0
+    b = numbers(k, n)
+    if dtype == "int8":
+        q = void.quantize_void_tensor(a)
+        bq, scale = void.quantize_cols_int8(b)
+        product = lambda lo, hi: void.void_spmm_int8(q, bq[:, lo:hi], scale[lo:hi], out_dtype=torch.float16)
+    elif dtype == "fp8":
+        q = void.void_tensor_to_fp8(a)
+        bq, scale = void.quantize_cols_fp8(b)[:2]
+        product = lambda lo, hi: void.void_spmm_fp8(q, bq[:, lo:hi], torch.float16, b_scale=scale[lo:hi])
+    elif linear:
+        q, x = a.to_dtype(dtype), b.t().contiguous().to(dtype)
+        product = lambda lo, hi: void.void_linear(q, x[lo:hi]).t()
+    else:
+        q, x = a.to_dtype(dtype), b.to(dtype)
+        product = lambda lo, hi: void.void_spmm(q, x[:, lo:hi])
+    whole = product(0, n)
+    parts = [product(lo, min(n, lo + step)) for lo in range(0, n, step)]
+    void.check_device_status()
+    assert torch.equal(whole, torch.cat(parts, 1))

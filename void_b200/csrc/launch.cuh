@@ -25,7 +25,7 @@ inline PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
 }
 
 struct DeviceInfo {
-  int sms = 0, cc_major = 0, cc_minor = 0, max_smem = 0, smem_per_sm = 0;
+  int sms = 0, cc_major = 0, cc_minor = 0, max_smem = 0, smem_per_sm = 0, l2_bytes = 0;
   bool ok = false;
 };
 inline DeviceInfo device_info() {
@@ -42,6 +42,7 @@ inline DeviceInfo device_info() {
     cudaDeviceGetAttribute(&d.cc_minor, cudaDevAttrComputeCapabilityMinor, dev);
     cudaDeviceGetAttribute(&d.max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaDeviceGetAttribute(&d.smem_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+    cudaDeviceGetAttribute(&d.l2_bytes, cudaDevAttrL2CacheSize, dev);
     d.ok = true;
     cache[dev] = d;
   }
