@@ -20,9 +20,9 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libvoid_b200.so")
-SOURCES = ["spmm.cu", "skinny.cu", "group.cu", "prep.cu", "plan.cu", "format.cu", "tile_grad.cu"]
+SOURCES = ["spmm.cu", "rowacc_i8.cu", "rowacc_f8.cu", "rowacc_f16.cu", "rowacc_tf32.cu", "skinny.cu", "group.cu", "prep.cu", "plan.cu", "format.cu", "tile_grad.cu"]
 HOST_SOURCE = os.path.join(CSRC, "host.cpp")
-HEADERS = [os.path.join(CSRC, h) for h in ("ptx.cuh", "kinds.cuh", "epilogue.cuh", "launch.cuh", "skinny.cuh")] + [
+HEADERS = [os.path.join(CSRC, h) for h in ("ptx.cuh", "kinds.cuh", "epilogue.cuh", "launch.cuh", "pipeline.cuh", "rowacc.cuh", "skinny.cuh")] + [
     os.path.join(HERE, "..", "include", "void_b200.h")]
 
 HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)]

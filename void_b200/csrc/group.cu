@@ -1,6 +1,6 @@
 // Products of groups of tile rows that share B's panels:  C = act(dequant(A . B) + bias).
 //
-// The row-accumulate kernel of spmm.cu fetches a panel of B for every stored tile.  Its large products bring 52 - 64 bytes per
+// The row-accumulate kernel of rowacc.cuh fetches a panel of B for every stored tile.  Its large products bring 52 - 64 bytes per
 // clock into an SM, where a kernel that does nothing but load from L2 reaches 66 - 70 with every SM loading, so fewer bytes are
 // what makes them faster.  Here a CTA (two per SM) owns up to eight tile rows at once, their accumulators for a panel of 128
 // columns in tensor memory, and walks the block columns that ANY of its rows stores: a panel is fetched once and multiplied
@@ -15,7 +15,7 @@
 // copy brings header and tiles, and E tensor copies the panels.  Groups are made of rows of falling length dealt out back and
 // forth, so that they hold nearly the same number of tiles.
 //
-// Roles as in spmm.cu: two producer warps take the stages in turn, two warps issue the MMAs of alternate rows, four warps
+// Roles as in pipeline.cuh: two producer warps take the stages in turn, two warps issue the MMAs of alternate rows, four warps
 // finish rows, one per lane quadrant of tensor memory.  Every wait is bounded.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(kThreads, kCtas) group_kernel(const __grid_con
     }
   }
 
-  grid_launch_dependents();   // (late, see pipeline_teardown in spmm.cu)
+  grid_launch_dependents();   // (late, see pipeline_teardown in pipeline.cuh)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -557,7 +557,7 @@ int void_spmm_grouped(const void_spmm_args* a, const void_group_store* s, int32_
   const int room = dev.smem_per_sm / kCtas - 1024 - 1024 - 1024 - staging;   // less alignment slack and the kernel's static variables
   p.stages = room / p.stage_bytes;
   if (p.stages > kMaxRing) p.stages = kMaxRing;
-  if (p.stages < kProducers) return VOID_ERR_SHAPE;   // (a producer warp may run that many stages ahead, see spmm.cu)
+  if (p.stages < kProducers) return VOID_ERR_SHAPE;   // (a producer warp may run that many stages ahead, see pipeline.cuh)
   const int smem = p.stages * p.stage_bytes + staging + 1024;
   p.desc_hi_b = smem_desc_hi(128, 256 * es, kLayoutNone);
   p.desc_hi_a = es == 4 ? smem_desc_hi(4096, 512, kLayoutSw128Base32)

@@ -1,0 +1,8 @@
+// Row-accumulate kernels for fp32 (TF32) tiles.
+#include "rowacc.cuh"
+
+namespace vb {
+
+template int launch_rowacc<VOID_KIND_TF32>(const RowaccLaunch&, const CUtensorMap&, const CUtensorMap&, const SpmmParams&);
+
+}  // namespace vb

@@ -1,12 +1,12 @@
 // Products with few columns (one token, a handful of activations):  C = act(dequant(A . B) + bias), N small.
 //
-// The tensor-memory kernels of spmm.cu multiply 128 columns of B whatever N is and stream a tile row through one CTA's
+// The tensor-memory kernels of pipeline.cuh multiply 128 columns of B whatever N is and stream a tile row through one CTA's
 // ring, a stage's round trip (1.2 us) at a time: 15 us for a decode step whose bytes take 2.  Here a CTA takes one tile
 // row and up to 32 columns, its warps share the row's tiles, every warp keeps its sums in registers (mma.sync,
 // D[32 x 8 NG] += tile[32 x 32] . B[32 x 8 NG]) and the warps' sums meet in shared memory once, before the epilogue.
 // The time is a chain of four memory latencies (row range, block columns, B, store) plus A's bytes.
 //
-// A is the packed store of spmm.cu, read straight into fragments: which k a lane holds in which register is free as long
+// A is the packed store of pipeline.cuh, read straight into fragments: which k a lane holds in which register is free as long
 // as A and B agree, so lane (g, t) = (lane / 4, lane % 4) takes the t-th contiguous piece of row g's 32 k:
 //   8-bit   8 k   (8 bytes: one mma.m16n8k32 per 16 rows)
 //   16-bit  8 k   (16 bytes: two mma.m16n8k16)
