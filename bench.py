@@ -315,7 +315,6 @@ def launch_floor(args, torch, void, workloads, _lib, _spmm, dev):
         "null_kernel_us": timed(lambda i: lib.void_launch_floor(512, 224, 50176, _lib.stream_ptr(dev))),
         "empty_a_us": timed(spmm(lambda i: empty)),
         "spmm_us": timed(spmm(own)),
-        "spmm_one_store_per_tile_us": timed(spmm(own, flags=_spmm.FLAG_STORE_PER_TILE)),
         "spmm_direct_stores_us": timed(spmm(own, flags=_spmm.FLAG_DIRECT_STORES)),
         "spmm_a_not_read_early_us": timed(spmm(own, flags=_spmm.FLAG_NO_EARLY_A)),
     }

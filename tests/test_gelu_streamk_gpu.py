@@ -171,3 +171,58 @@ def test_stream_k_power_law_benchmark_size():
     assert torch.equal(c, void.void_spmm_int8(q, bq, bs, out_dtype=torch.bfloat16, activation=2))
     prof = void.analyze_workload(q)
     assert prof.use_stream_k and prof.imbalance_ratio > 5
+
+
+@pytest.mark.parametrize("n", [256, 8])
+@pytest.mark.parametrize("name", ["gelu", "silu"])
+def test_activations_against_64_bits(name, n):
+    """Both epilogues (tensor-memory kernel, kernel for few columns) on |x| <= 6.  x * sigmoid(v): the argument of the
+    exponential has three roundings of at most 2^-24 each, which its size (GELU 25, SiLU 6 natural units) turns into relative
+    errors of the result; exponential, sum, reciprocal and two products add 2^-21 together."""
+    q = void.quantize_void_tensor(void.dense_to_void(torch.eye(128, device="cuda")))
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    b = torch.randint(-128, 128, (128, n), dtype=torch.int8, device="cuda", generator=gen)
+    scale = 6.0 / 127 * 10.0 ** (-3 * torch.arange(n, device="cuda") / n)
+    x = void.void_spmm_int8(q, b, scale, out_dtype=torch.float32).double()
+    y = void.void_spmm_int8(q, b, scale, out_dtype=torch.float32, activation=void.get_activation_code(name)).double()
+    assert 5.0 < x.abs().max() < 6.1
+    v = 1.5957691216 * (x + 0.044715 * x ** 3) if name == "gelu" else x
+    ref = x * torch.sigmoid(v)
+    keep = ref != 0
+    worst = ((y - ref).abs() / ref.abs())[keep].max().item()
+    assert worst < v.abs().max().item() * 3 * 2.0 ** -24 + 2.0 ** -21
+    assert bool((y[~keep] == 0).all())
+
+
+@pytest.mark.parametrize("kind", ["int8", "fp8", torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m,n,biased", [(32, 136, False), (95, 200, True), (160, 384, True), (64, 264, False)])
+def test_staged_results_of_slim_ctas_equal_direct_stores(kind, m, n, biased):
+    """16-bit results without an activation: matrix stores into the staging tile and a clipped tiled store, every operand
+    type, edges of C inside a part."""
+    from void_b200 import _lib, _spmm, ops
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    mask = torch.rand((m + 31) // 32, 12, generator=gen, device="cuda") < 0.7
+    mask[0, :2] = True
+    if m > 32:
+        mask[1] = False
+    values = torch.randn(int(mask.sum()), 32, 32, generator=gen, device="cuda")
+    a = void.void_from_block_mask(mask.cpu().numpy(), values, shape=(m, 384))
+    b = torch.randn(384, n, generator=gen, device="cuda")
+    kw = {"bias": torch.randn(n, generator=gen, device="cuda") if biased else None}
+    if kind == "int8":
+        p = void.quantize_void_tensor(a).packed()
+        b, kw["col_scale"] = void.quantize_cols_int8(b)
+    elif kind == "fp8":
+        p = void.void_tensor_to_fp8(a).packed()
+        b, kw["col_scale"] = void.quantize_cols_fp8(b)[:2]
+    else:
+        a, b = a.to_dtype(kind), b.to(kind)
+        p = ops.packed_fp(a, ops.product_kind(a, b))
+    for dtype in (torch.float16, torch.bfloat16):
+        outs = []
+        for flags in (0, _spmm.FLAG_DIRECT_STORES):
+            out = torch.full((m, n), 7.0, dtype=dtype, device="cuda")
+            _spmm.spmm(p, b, out, scale_mode=_lib.SCALE_ROW_MEAN, cta_shape=2, flags=flags, **kw)
+            outs.append(out)
+        assert torch.equal(*outs)
+    void.check_device_status()

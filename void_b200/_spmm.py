@@ -16,7 +16,7 @@ from .format import check_indexed
 TILE = 32
 PANEL = 128
 CAPTURED = -1   # launch key of a stream that is being captured; others have their stream's
-FLAG_DIRECT_STORES, FLAG_A_STABLE, FLAG_STORE_PER_TILE = 2, 4, 16   # bits of void_spmm_args.flags
+FLAG_DIRECT_STORES, FLAG_A_STABLE = 2, 4   # bits of void_spmm_args.flags
 FLAG_NO_EARLY_A = 1 << 30   # host side only: never set FLAG_A_STABLE (measurements)
 
 

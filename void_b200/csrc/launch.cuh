@@ -130,16 +130,16 @@ inline bool panel_map_transposed(CUtensorMap* m, const void* b, int64_t ldb, int
   return enc(m, dt, 2, const_cast<void*>(b), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// C of 16-bit elements for tiled stores of 32 rows x box_cols columns
-inline bool store_map(CUtensorMap* m, void* out, int64_t ldc, int M, int N, int box_cols) {
+// C of 16-bit elements for tiled stores of 32 rows x 32 columns, 64-byte swizzle
+inline bool store_map(CUtensorMap* m, void* out, int64_t ldc, int M, int N) {
   PFN_cuTensorMapEncodeTiled_v12000 enc = get_encode();
   if (enc == nullptr) return false;
   const cuuint64_t gdim[2] = {(cuuint64_t)N, (cuuint64_t)M};
   const cuuint64_t gstride[1] = {(cuuint64_t)ldc * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)kTile};
+  const cuuint32_t box[2] = {32, (cuuint32_t)kTile};
   const cuuint32_t estride[2] = {1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, out, gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+             CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace vb

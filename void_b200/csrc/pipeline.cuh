@@ -153,7 +153,6 @@ struct SpmmParams {
   int stages;   // ring depth
   int last_group;   // tiles of the ring's last stage (1 .. group): the shared memory left over by the full stages
   int use3d;    // B panels of a tile fetched by one 3-D TMA
-  int tma_store;  // 16-bit outputs leave through a staging tile in shared memory and a tiled TMA store
   int tmem_cols;  // tensor-memory columns of the drain kernel (256: two CTAs per SM, 512: one)
   int n_items;  // without a plan: nbr * n_chunks
   Passes passes;  // and the order they are taken in
@@ -180,9 +179,11 @@ struct Seg {
   int row, chunk, t0, t1, nseg, slot0, my_idx, ctr;
 };
 
+// PLAN: the launch may come with a work plan.
+template <bool PLAN>
 __device__ __forceinline__ Seg load_seg(const SpmmParams& p, int i) {
   Seg s;
-  if (p.segs != nullptr) {
+  if (PLAN && p.segs != nullptr) {
     const int4* q = reinterpret_cast<const int4*>(p.segs) + 2 * (size_t)i;
     const int4 a = __ldg(q), b = __ldg(q + 1);
     s.row = a.x; s.chunk = a.y; s.t0 = a.z; s.t1 = a.w;
@@ -202,9 +203,26 @@ __device__ __forceinline__ Seg load_seg(const SpmmParams& p, int i) {
   return s;
 }
 
+// The same for a warp that waits with many values in registers: lane k holds word k (in the order of Seg's fields).
+template <bool PLAN>
+__device__ __forceinline__ int load_seg_word(const SpmmParams& p, int i, int lane) {
+  if (PLAN && p.segs != nullptr) return lane < 8 ? __ldg(p.segs + 8 * (size_t)i + lane) : 0;
+  int k, chunk;
+  p.passes.item(i, k, chunk);
+  int row = k;
+  if (p.row_order != nullptr) {
+    const int r = __ldg(p.row_order + k);
+    row = r < 0 ? 0 : (r >= p.nbr ? p.nbr - 1 : r);
+  }
+  if (lane == 2 || lane == 3) return __ldg(p.row_ptr + row + lane - 2);
+  return lane == 0 ? row : (lane == 1 ? chunk : (lane == 4 ? 1 : 0));
+}
+__device__ __forceinline__ int word_of(int words, int k) { return __shfl_sync(0xffffffffu, words, k); }
+
 // Range of segment indices of this CTA: [begin, end) with stride step.
+template <bool PLAN>
 __device__ __forceinline__ void seg_range(const SpmmParams& p, int& begin, int& end, int& step) {
-  if (p.segs != nullptr) {
+  if (PLAN && p.segs != nullptr) {
     begin = __ldg(p.cta_seg_ptr + blockIdx.x);
     end = __ldg(p.cta_seg_ptr + blockIdx.x + 1);
     step = 1;
@@ -260,7 +278,7 @@ __device__ __forceinline__ int stage_cap(const SpmmParams& p, int stage) {
 // claims its first ring stage and starts the bulk copy of that stage's tiles BEFORE the wait, while the
 // previous kernel is still draining; only the panels of B - typically that kernel's output - are
 // requested after it.
-template <class C, int ES, int TR, bool TRACE>
+template <class C, int ES, int TR, bool PLAN, bool TRACE>
 __device__ __forceinline__ void producer_loop(const SpmmParams& p, const CUtensorMap* tmap, PipeBars* bars,
                                               uint32_t ring_base, uint32_t stage_bytes, volatile int* ctl,
                                               int lane, int pw) {
@@ -268,16 +286,16 @@ __device__ __forceinline__ void producer_loop(const SpmmParams& p, const CUtenso
   if (waited) grid_dependency_wait();
   if (TRACE && pw == 0 && lane == 0) stamp<TRACE>(p, 56);   // producer starts
   int begin, end, step;
-  seg_range(p, begin, end, step);
+  seg_range<PLAN>(p, begin, end, step);
   const int S = p.stages;
   // position of the next group in the ring: its stage, the parity of the stage's use, the warp it belongs to
   int stage = 0, owner = 0, gcount = 0;
   uint32_t phase = 0;
   Seg seg_next = {};  // the next segment's descriptor is fetched one item ahead
-  if (begin < end) seg_next = load_seg(p, begin);
+  if (begin < end) seg_next = load_seg<PLAN>(p, begin);
   for (int i = begin; i < end; i += step) {
     const Seg s = seg_next;
-    if (i + step < end) seg_next = load_seg(p, i + step);
+    if (i + step < end) seg_next = load_seg<PLAN>(p, i + step);
     const int npan = panels_in_chunk(p, s.chunk);
     const int n0 = s.chunk * p.np * kPanelN;
     const uint32_t unit_bytes = (uint32_t)((kTileBytes * p.terms + ((p.use3d && TR != 1) ? p.np : npan) * kPanelBytes) * ES);
@@ -418,11 +436,17 @@ __device__ __forceinline__ void pipeline_teardown(const SpmmParams& p, int* ctl_
   if ((threadIdx.x >> 5) == C::MMA) tmem_dealloc(tmem_base, tmem_cols);
 }
 
-// How a row-accumulate kernel is launched; defined in rowacc.cuh, built for one kind per source file.
+// How a row-accumulate kernel is launched; defined in rowacc.cuh, built for one kind per source file.  `epilogue`: what its
+// epilogue has to be able to do, a sum of
+//   kStaged  16-bit results through shared memory and tiled stores
+//   kSplit   a work plan, raw sums for the caller
+//   kActive  activation, row bias
+//   kTraced  time stamps (slim INT8 only, with kActive)
+constexpr int kStaged = 1, kSplit = 2, kActive = 4, kTraced = 8;
 struct RowaccLaunch {
   bool slim;
   int transposed;
-  bool traced;
+  int epilogue;
   int grid, smem_bytes;
   cudaStream_t stream;
 };

@@ -262,8 +262,55 @@ __device__ __forceinline__ void tmem_ld_32x16p(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
+// 32 lanes x 32 columns as fragments: thread t gets columns 8 g + 2 (t % 4) + {0, 1} of lanes t / 4 + {0, 8, 16, 24}, elements
+// [4 g + 2 (lane / 8 % 2) + {0, 1}] of `lo` (lanes 0 .. 15) and `hi` (lanes 16 .. 31).
+__device__ __forceinline__ void tmem_ld_fragments(uint32_t taddr, uint32_t (&lo)[16], uint32_t (&hi)[16]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t(&r)[16] = h ? hi : lo;
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr + ((uint32_t)(16 * h) << 16))
+        : "memory");
+  }
+}
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// Four 8 x 8 matrices of 16-bit elements to shared memory, transposed: thread t holds elements [t / 4][2 (t % 4) + {0, 1}] of
+// each, and gives the address of row t % 8 of what becomes of matrix t / 8.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
+
+// ---------------------------------------------------------------- pairs of floats
+// Two floats in a register pair: sm_100 multiplies and adds both in one instruction, each rounded as by itself.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pair(float a, float b) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ void unpair(f32x2 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
 }
 
 // ---------------------------------------------------------------- descriptors

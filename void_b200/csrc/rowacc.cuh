@@ -11,11 +11,22 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[COLS]
   for (int c = 0; c < COLS; c += 16) tmem_ld_32x16p(taddr + (uint32_t)c, &r[c]);
 }
 
-// TR: 1 = B and C transposed ([N, K] and [N, M]), 2 = C alone
-template <int KIND, class C, int TR = 0, bool TRACE = false>
+// The accumulator of a split row's panel q, [32 m][128 n]; with peers the owner's.
+__device__ __forceinline__ int32_t* row_sums(const SpmmParams& p, int seg_words, bool peers, int q) {
+  int32_t* base = peers ? p.peer_partials[word_of(seg_words, 5)] : p.partials;
+  return base + ((size_t)word_of(seg_words, 7) * p.np + q) * (kTile * kPanelN);
+}
+
+// TR: 1 = B and C transposed ([N, K] and [N, M]), 2 = C alone.  EPI: what the epilogue is asked for (kStaged ...).  One kernel
+// that could do all of it took 6.83 us for a launch that runs in 5.46 without activations and in 5.67 with them (INT8 4096^2,
+// 90 %, N = 512, fp16 results): what is not run costs too, in spilled registers and in instructions fetched around it.
+template <int KIND, class C, int TR, int EPI>
 __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel(const __grid_constant__ CUtensorMap tmap_b,
                                                                const __grid_constant__ CUtensorMap tmap_c,
                                                                const __grid_constant__ SpmmParams p) {
+  constexpr bool STAGED = (EPI & kStaged) != 0, SPLIT = (EPI & kSplit) != 0, ACT = (EPI & kActive) != 0, TRACE = (EPI & kTraced) != 0;
+  static_assert(!TR || (!STAGED && !SPLIT), "transposed results are stored directly, of whole rows");
+  static_assert(!STAGED || C::COLS == kTile, "an epilogue warp stages whole columns of a tile row");
   extern __shared__ uint8_t smem_raw[];
   __shared__ PipeBars bars;
   __shared__ uint32_t tmem_base_s;
@@ -40,7 +51,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
   const uint32_t tmem_base = tmem_base_s;
 
   if (warp < C::PW) {
-    producer_loop<C, ES, TR, TRACE>(p, &tmap_b, &bars, ring_base, stage_bytes, ctl, lane, warp);
+    producer_loop<C, ES, TR, SPLIT, TRACE>(p, &tmap_b, &bars, ring_base, stage_bytes, ctl, lane, warp);
     if (warp == 0 && lane == 0) stamp<TRACE>(p, 2);
   } else if (warp == C::MMA) {
     {
@@ -61,17 +72,17 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
       // (transposed B: the panel is K-major, 32 bytes of k lie inside one row of its swizzle atom)
       constexpr uint64_t kPanelKStep = TR == 1 ? 2 : ((kPanelBytes / ES) >> 4), kTileKStep = 256 >> 4;
       int begin, end, step;
-      seg_range(p, begin, end, step);
+      seg_range<SPLIT>(p, begin, end, step);
       int stage = 0;
       uint32_t phase = 0;
       uint32_t sbase = ring_base;
       uint32_t it = 0;
       bool ok = true;
       Seg seg_next = {};  // the next segment's descriptor is fetched one item ahead
-      if (begin < end) seg_next = load_seg(p, begin);
+      if (begin < end) seg_next = load_seg<SPLIT>(p, begin);
       for (int i = begin; i < end && ok; i += step, ++it) {
         const Seg s = seg_next;
-        if (i + step < end) seg_next = load_seg(p, i + step);
+        if (i + step < end) seg_next = load_seg<SPLIT>(p, i + step);
         const int npan = panels_in_chunk(p, s.chunk);
         const uint32_t buf = it & 1u, aph = (it >> 1) & 1u;
         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.acc_empty[buf]), aph ^ 1u, ctl));
@@ -133,45 +144,35 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
     const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
     const int m_first = half * C::COLS;
     const OutDesc od = out_desc(p);
-    // staging tile of the TMA-store epilogue: behind the ring
-    const uint32_t stage_u32 = ring_base + ring_bytes;
-    uint16_t* stage_tile = reinterpret_cast<uint16_t*>(smem_raw + (stage_u32 - smem_u32(smem_raw)));
+    // this warp's part of the staging tile behind the ring
+    const uint32_t part = ring_base + ring_bytes + (uint32_t)(warp - C::EPI0) * (32u * kTile * 2u);
     bool store_pending = false;
     // the column scales and biases this role reads and the C it writes may be the previous kernel's; the index
     // of A may be read ahead of it when the caller vouches for A
     if (!p.a_stable) grid_dependency_wait();
     int begin, end, step;
-    seg_range(p, begin, end, step);
+    seg_range<SPLIT>(p, begin, end, step);
     uint32_t it = 0;
-    Seg seg_next = {};  // the next segment's descriptor is fetched one item ahead
-    if (begin < end) seg_next = load_seg(p, begin);
+    int seg_next = 0;  // the next segment's descriptor is fetched one item ahead, a word per lane
+    if (begin < end) seg_next = load_seg_word<SPLIT>(p, begin, lane);
     if (p.a_stable) grid_dependency_wait();
     if (epi_tid == 0) stamp<TRACE>(p, 0);
     for (int i = begin; i < end; i += step, ++it) {
-      const Seg s = seg_next;
-      if (i + step < end) seg_next = load_seg(p, i + step);
-      const int npan = panels_in_chunk(p, s.chunk);
+      const int seg = seg_next;
+      if (i + step < end) seg_next = load_seg_word<SPLIT>(p, i + step, lane);
+      const int row = word_of(seg, 0), chunk = word_of(seg, 1), nseg = SPLIT ? word_of(seg, 4) : 1;
+      const int npan = panels_in_chunk(p, chunk);
       const uint32_t buf = it & 1u, aph = (it >> 1) & 1u;
-      const bool has = s.t1 > s.t0;
+      const bool has = word_of(seg, 3) > word_of(seg, 2);
       // an empty tile row is zeros (+ bias): nothing to scale, no scales to wait for
-      const float rs = (p.row_scale != nullptr && (has || s.nseg > 1)) ? __ldg(p.row_scale + s.row) : 1.0f;
-      const int n_base = s.chunk * p.np * kPanelN + quad * 32 + lane;
+      const float rs = (p.row_scale != nullptr && (has || nseg > 1)) ? __ldg(p.row_scale + row) : 1.0f;
+      const int n_base = chunk * p.np * kPanelN + quad * 32 + lane;
       // per-column scale and bias of the first panel are fetched before the accumulator is ready
       float cs = p.b_scale, bias = 0.0f;
       if (n_base < p.N) {
-        if (p.col_scale != nullptr && (has || s.nseg > 1)) cs = __ldg(p.col_scale + n_base) * p.b_scale;
+        if (p.col_scale != nullptr && (has || nseg > 1)) cs = __ldg(p.col_scale + n_base) * p.b_scale;
         if (p.bias != nullptr) bias = __ldg(p.bias + n_base);
       }
-      // a split row whose scratch index lies outside what the caller provided is skipped and reported
-      const bool peers = p.n_peers > 0 && s.nseg > 1;
-      const bool bad_split = s.nseg > 1 && (s.ctr < 0 || s.ctr >= p.ctr_limit || (peers && (unsigned)s.slot0 >= (unsigned)p.n_peers));
-      int32_t* split_partials = p.partials;
-      int32_t* split_counters = p.counters;
-      if (peers && !bad_split) {
-        split_partials = p.peer_partials[s.slot0];
-        split_counters = p.peer_counters[s.slot0];
-      }
-      if (bad_split && epi_tid == 0 && p.status != nullptr) atomicCAS(p.status, 0, kStatusBadPlan);
       // one thread waits, the named barrier hands its verdict to all epilogue warps, so that they
       // leave the loop together if the wait gave up (a warp that went on alone would wait at the next
       // named barrier for ever)
@@ -181,152 +182,78 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
       if (epi_tid == 0 && i == begin) stamp<TRACE>(p, 5);
       if (epi_tid == 0) stamp<TRACE>(p, 8);
       tc_fence_after();
-      const bool fast = s.nseg == 1 && od.acc_out == nullptr && p.worker_partials == nullptr;
+      // Everything but whole rows into C alone goes through here first: raw accumulators for the caller, pieces of split rows.
+      const bool whole = !SPLIT || (nseg == 1 && (STAGED || (od.acc_out == nullptr && p.worker_partials == nullptr)));
+      const bool peers = SPLIT && !STAGED && p.n_peers > 0 && nseg > 1;
+      if (!whole) {
+        const int owner = word_of(seg, 5), ctr = word_of(seg, 7);
+        // a split row whose scratch index lies outside what the caller provided is skipped and reported
+        const bool bad_split = nseg > 1 && (ctr < 0 || ctr >= p.ctr_limit || (peers && (unsigned)owner >= (unsigned)p.n_peers));
+        int32_t* split_partials = peers && !bad_split ? p.peer_partials[owner] : p.partials;
+        if (bad_split && epi_tid == 0 && p.status != nullptr) atomicCAS(p.status, 0, kStatusBadPlan);
 #pragma unroll 1
-      for (int q = 0; q < npan; ++q) {
-        const int n = n_base + q * kPanelN;
-        const uint32_t acc_addr = tmem_base + lane_sel + buf * acc_cols + (uint32_t)(q * 32 + m_first);
-        if (fast) {
-          // All of this warp's columns of the panel are requested at once and awaited once; the
-          // accumulator buffer goes back to the MMA warp as soon as the values sit in registers.
-          float csq = cs, biasq = bias;
-          if (q > 0) {
-            csq = p.b_scale; biasq = 0.0f;
-            if (n < p.N) {
-              if (p.col_scale != nullptr) csq = __ldg(p.col_scale + n) * p.b_scale;
-              if (p.bias != nullptr) biasq = __ldg(p.bias + n);
-            }
+        for (int q = 0; q < npan; ++q) {
+          const int n = n_base + q * kPanelN;
+          float csq = p.b_scale, biasq = 0.0f;
+          if (!STAGED && n < p.N) {
+            if (p.col_scale != nullptr) csq = __ldg(p.col_scale + n) * p.b_scale;
+            if (p.bias != nullptr) biasq = __ldg(p.bias + n);
           }
-          uint32_t r[C::COLS];
+          // all columns of the panel with one wait, then the accumulator buffer goes back to the MMA warp
+          uint32_t ra[C::COLS];
           if (has) {
-            tmem_ld_cols<C::COLS>(acc_addr, r);
+            tmem_ld_cols<C::COLS>(tmem_base + lane_sel + buf * acc_cols + (uint32_t)(q * 32 + m_first), ra);
             tmem_ld_wait();
           } else {
 #pragma unroll
-            for (int k = 0; k < C::COLS; ++k) r[k] = 0u;
+            for (int k = 0; k < C::COLS; ++k) ra[k] = 0u;
           }
-          if (epi_tid == 0 && q == 0) stamp<TRACE>(p, 9);
-          if (q == npan - 1) {  // this warp is done with the accumulator buffer
+          if (q == npan - 1) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bars.acc_empty[buf]));
           }
-          if (!TR && p.tma_store == 2) {
-            // 16-bit outputs, one store per epilogue warp: the warp puts its 32 x 32 part of the result tile
-            // together in its own 2 KB of shared memory and sends it off itself - no barrier between the warps.
-            // The copy engine clips at the edges of C; the part is free again once the previous store has read it.
-            if (store_pending) {
-              if (lane == 0) bulk_wait_read();
-              __syncwarp();
+#pragma unroll
+          for (int c = 0; c < C::COLS; c += 8) {
+            const int m0 = m_first + c;
+            uint32_t r[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) r[k] = ra[c + k];
+            if (!STAGED && p.worker_partials != nullptr && n < p.N) {
+              uint32_t* w = reinterpret_cast<uint32_t*>(p.worker_partials) + ((size_t)i * kTile + m0) * p.N + n;
+#pragma unroll
+              for (int k = 0; k < 8; ++k) w[(size_t)k * p.N] = r[k];
             }
-            uint16_t* part = stage_tile + quad * (32 * 32);
-            if (!has && p.bias == nullptr && p.row_bias == nullptr) {
-              // an empty tile row without bias is zeros under every activation: 2 KB of zero words, no conversions
-              uint4* z = reinterpret_cast<uint4*>(part) + lane;
+            if (!STAGED && nseg == 1) {
+              finish8<KIND>(od, row, n, m0, r, rs, csq, biasq);
+            } else if (!bad_split && has) {
+              // partial sum of a split row: added into the row's int32 accumulator in global memory
+              // (integer adds commute, so the total does not depend on which CTA - or which GPU - comes first)
+              int32_t* dst = split_partials + ((size_t)ctr * p.np + q) * (kTile * kPanelN) + (size_t)m0 * kPanelN +
+                             (quad * 32 + lane);
+              if (peers && p.peer_slots) {
+                // this rank's own slot of the row: nothing else writes it, plain stores (NVLink writes for a remote owner)
+                int32_t* slot = split_partials + (((size_t)ctr * p.n_peers + word_of(seg, 6)) * p.np + q) * (kTile * kPanelN) +
+                                (size_t)m0 * kPanelN + (quad * 32 + lane);
 #pragma unroll
-              for (int k = 0; k < 4; ++k) z[k * 32] = make_uint4(0u, 0u, 0u, 0u);
-            } else {
+                for (int k = 0; k < 8; ++k) slot[k * kPanelN] = (int32_t)r[k];
+              } else if (!STAGED && p.n_peers > 0) {   // the accumulator may be another GPU's: system-wide adds over NVLink
 #pragma unroll
-              for (int c = 0; c < C::COLS; c += 16)
-                finish16_stage<KIND, 32>(od, s.row, n, m_first + c, &r[c], rs, csq, biasq, part + lane);
-            }
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&tmap_c, stage_u32 + (uint32_t)quad * (32 * 32 * 2), (s.chunk * p.np + q) * kPanelN + quad * 32,
-                           s.row * kTile);
-              bulk_commit();
-            }
-            store_pending = true;
-          } else if (!TR && p.tma_store) {
-            // 16-bit outputs: the 32 x 128 result tile is put together in shared memory and leaves in one
-            // tiled store; the copy engine clips it at the edges of C.  The staging tile is free again once
-            // the previous store has read it.
-            if (store_pending) {
-              if (epi_tid == 0) bulk_wait_read();
-              asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_THREADS) : "memory");
-            }
+                for (int k = 0; k < 8; ++k) {
+                  if (KIND == VOID_KIND_I8) atomicAdd_system(dst + k * kPanelN, (int32_t)r[k]);
+                  else atomicAdd_system(reinterpret_cast<float*>(dst) + k * kPanelN, __uint_as_float(r[k]));
+                }
+              } else {
 #pragma unroll
-            for (int c = 0; c < C::COLS; c += 16)
-              finish16_stage<KIND, kPanelN>(od, s.row, n, m_first + c, &r[c], rs, csq, biasq, stage_tile + quad * 32 + lane);
-            fence_proxy_async_smem();
-            asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_THREADS) : "memory");
-            if (epi_tid == 0) {
-              tma_store_2d(&tmap_c, stage_u32, (s.chunk * p.np + q) * kPanelN, s.row * kTile);
-              bulk_commit();
-            }
-            store_pending = true;
-          } else {
-#pragma unroll
-            for (int c = 0; c < C::COLS; c += 16) {
-              if (TR) finish16_tr<KIND>(od, s.row, n, m_first + c, &r[c], rs, csq, biasq);
-              else finish16<KIND>(od, s.row, n, m_first + c, &r[c], rs, csq, biasq);
-            }
-          }
-          if (epi_tid == 0 && q == 0) stamp<TRACE>(p, 10);
-          continue;
-        }
-        float csq = p.b_scale, biasq = 0.0f;
-        if (n < p.N) {
-          if (p.col_scale != nullptr) csq = __ldg(p.col_scale + n) * p.b_scale;
-          if (p.bias != nullptr) biasq = __ldg(p.bias + n);
-        }
-        // (raw accumulators wanted, or a piece of a split row) all columns of the panel with one wait, then the
-        // accumulator buffer goes back to the MMA warp
-        uint32_t ra[C::COLS];
-        if (has) {
-          tmem_ld_cols<C::COLS>(acc_addr, ra);
-          tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int k = 0; k < C::COLS; ++k) ra[k] = 0u;
-        }
-        if (q == npan - 1) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&bars.acc_empty[buf]));
-        }
-#pragma unroll
-        for (int c = 0; c < C::COLS; c += 8) {
-          const int m0 = m_first + c;
-          uint32_t r[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) r[k] = ra[c + k];
-          if (p.worker_partials != nullptr && n < p.N) {
-            uint32_t* w = reinterpret_cast<uint32_t*>(p.worker_partials) + ((size_t)i * kTile + m0) * p.N + n;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) w[(size_t)k * p.N] = r[k];
-          }
-          if (s.nseg == 1) {
-            finish8<KIND>(od, s.row, n, m0, r, rs, csq, biasq);
-          } else if (!bad_split && has) {
-            // partial sum of a split row: added into the row's int32 accumulator in global memory
-            // (integer adds commute, so the total does not depend on which CTA - or which GPU - comes first)
-            int32_t* dst = split_partials + ((size_t)s.ctr * p.np + q) * (kTile * kPanelN) + (size_t)m0 * kPanelN +
-                           (quad * 32 + lane);
-            if (peers && p.peer_slots) {
-              // this rank's own slot of the row: nothing else writes it, plain stores (NVLink writes for a remote owner)
-              int32_t* slot = split_partials + (((size_t)s.ctr * p.n_peers + s.my_idx) * p.np + q) * (kTile * kPanelN) +
-                              (size_t)m0 * kPanelN + (quad * 32 + lane);
-#pragma unroll
-              for (int k = 0; k < 8; ++k) slot[k * kPanelN] = (int32_t)r[k];
-            } else if (p.n_peers > 0) {   // the accumulator may be another GPU's: system-wide adds over NVLink
-#pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                if (KIND == VOID_KIND_I8) atomicAdd_system(dst + k * kPanelN, (int32_t)r[k]);
-                else atomicAdd_system(reinterpret_cast<float*>(dst) + k * kPanelN, __uint_as_float(r[k]));
-              }
-            } else {
-#pragma unroll
-              for (int k = 0; k < 8; ++k) {
-                if (KIND == VOID_KIND_I8) red_add_s32(dst + k * kPanelN, (int32_t)r[k]);
-                else red_add_f32(reinterpret_cast<float*>(dst) + k * kPanelN, __uint_as_float(r[k]));
+                for (int k = 0; k < 8; ++k) {
+                  if (KIND == VOID_KIND_I8) red_add_s32(dst + k * kPanelN, (int32_t)r[k]);
+                  else red_add_f32(reinterpret_cast<float*>(dst) + k * kPanelN, __uint_as_float(r[k]));
+                }
               }
             }
           }
         }
-      }
-      if (s.nseg > 1 && !bad_split && !(peers && p.peer_slots)) {
+        if (nseg == 1 || bad_split || (peers && p.peer_slots)) continue;
         // the CTA that arrives last reads the completed sums back and finishes the row
         if (epi_tid == 0) stamp<TRACE>(p, 12);
         // The arrival is one release-acquire add by one thread after a barrier of the epilogue warps: the barrier
@@ -336,9 +263,10 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
         asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_THREADS) : "memory");
         if (epi_tid == 0) stamp<TRACE>(p, 13);
         if (epi_tid == 0) {
-          const int old = peers ? atomicAdd_system(split_counters + s.ctr, 1) : atom_add_acq_rel(split_counters + s.ctr, 1);
-          const int last = (old == s.nseg - 1) ? 1 : 0;
-          if (last) split_counters[s.ctr] = 0;  // left clean for the next launch
+          int32_t* counter = (peers ? p.peer_counters[owner] : p.counters) + ctr;
+          const int old = peers ? atomicAdd_system(counter, 1) : atom_add_acq_rel(counter, 1);
+          const int last = (old == nseg - 1) ? 1 : 0;
+          if (last) *counter = 0;  // left clean for the next launch
           last_s = last;
         }
         asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_THREADS) : "memory");
@@ -346,101 +274,160 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
         asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_THREADS) : "memory");
         if (epi_tid == 0) stamp<TRACE>(p, 14);
         if (TRACE && epi_tid == 0 && p.trace != nullptr) p.trace[(size_t)blockIdx.x * 64 + 15] = (unsigned long long)last;
-        if (last) {
-          if (peers) __threadfence_system();
-          if (epi_tid == 0) stamp<TRACE>(p, 28);
-          OutDesc od2 = od;
-          od2.acc_out = nullptr;
-          if (peers) od2.out = p.peer_out[s.slot0];   // the owner's rows of C
+        if (!last) continue;
+        if (peers) __threadfence_system();
+        if (epi_tid == 0) stamp<TRACE>(p, 28);
+      }
+      // Finished values, panel by panel: of a whole row from tensor memory, of a split row from its sums.  The values of a
+      // panel are requested at once and awaited once; an accumulator buffer goes back to the MMA warp as soon as they sit in
+      // registers, a row's sums in global memory are cleared for the next launch.
 #pragma unroll 1
-          for (int q = 0; q < npan; ++q) {
-            const int n = n_base + q * kPanelN;
-            float csq = cs, biasq = bias;   // the first panel's were read before the accumulator was ready
-            if (q > 0) {
-              csq = p.b_scale; biasq = 0.0f;
-              if (n < p.N) {
-                if (p.col_scale != nullptr) csq = __ldg(p.col_scale + n) * p.b_scale;
-                if (p.bias != nullptr) biasq = __ldg(p.bias + n);
-              }
-            }
-            // all of this warp's sums of the panel are requested at once (one L2 round trip), then
-            // the accumulator is cleared for the next launch
-            int32_t* src = split_partials + ((size_t)s.ctr * p.np + q) * (kTile * kPanelN) + (size_t)m_first * kPanelN +
-                           (quad * 32 + lane);
-            uint32_t rl[C::COLS];
-            if (TRACE && epi_tid == 0 && q == 0) { asm volatile("" ::"f"(csq), "f"(biasq) : "memory"); stamp<TRACE>(p, 29); }
-#pragma unroll
-            for (int k = 0; k < C::COLS; ++k)
-              rl[k] = (uint32_t)(peers ? __ldcv(src + k * kPanelN) : __ldcg(src + k * kPanelN));
-            if (TRACE && epi_tid == 0 && q == 0) { asm volatile("" ::"r"(rl[0]), "r"(rl[C::COLS - 1]) : "memory"); stamp<TRACE>(p, 30); }
-            if (epi_tid == 0 && q == 0) stamp<TRACE>(p, 31);
-            if (!TR && p.tma_store == 2 && !peers && od.acc_out == nullptr) {
-              // 16-bit outputs leave as in the unsplit case: the warp's 32 x 32 part through shared memory and one tiled store
-              if (store_pending) {
-                if (lane == 0) bulk_wait_read();
-                __syncwarp();
-              }
-              uint16_t* part = stage_tile + quad * (32 * 32);
-#pragma unroll
-              for (int c = 0; c < C::COLS; c += 16)
-                finish16_stage<KIND, 32>(od, s.row, n, m_first + c, &rl[c], rs, csq, biasq, part + lane);
-              fence_proxy_async_smem();
-              __syncwarp();
-              if (lane == 0) {
-                tma_store_2d(&tmap_c, stage_u32 + (uint32_t)quad * (32 * 32 * 2), (s.chunk * p.np + q) * kPanelN + quad * 32,
-                             s.row * kTile);
-                bulk_commit();
-              }
-              store_pending = true;
-              // (cleared after the store has been issued: the fence in front of it would wait for these writes)
-#pragma unroll
-              for (int k = 0; k < C::COLS; ++k) src[k * kPanelN] = 0;
-              continue;
-            }
-#pragma unroll
-            for (int k = 0; k < C::COLS; ++k) src[k * kPanelN] = 0;
-#pragma unroll
-            for (int c = 0; c < C::COLS; c += 16) {
-              if (od.acc_out != nullptr && n < od.N) {
-                uint32_t* a = reinterpret_cast<uint32_t*>(od.acc_out) + ((size_t)s.row * kTile + m_first + c) * od.N + n;
-#pragma unroll
-                for (int k = 0; k < 16; ++k) a[(size_t)k * od.N] = rl[c + k];
-              }
-              finish16<KIND>(od2, s.row, n, m_first + c, &rl[c], rs, csq, biasq);
-            }
+      for (int q = 0; q < npan; ++q) {
+        const int n = n_base + q * kPanelN;
+        const uint32_t acc_addr = tmem_base + lane_sel + buf * acc_cols + (uint32_t)(q * 32 + m_first);
+        float csq = cs, biasq = bias;   // the first panel's were read before the accumulator was ready
+        if (q > 0) {
+          csq = p.b_scale; biasq = 0.0f;
+          if (n < p.N) {
+            if (p.col_scale != nullptr) csq = __ldg(p.col_scale + n) * p.b_scale;
+            if (p.bias != nullptr) biasq = __ldg(p.bias + n);
           }
         }
+        if constexpr (STAGED) {
+          // 16-bit outputs: every epilogue warp puts its part of the result tile (32 columns of the tile row) together in its own
+          // piece of shared memory and sends it off itself - no barrier between the warps.  The copy engine clips at the
+          // edges of C; the part is free again once the previous store has read it.
+          uint32_t lo[16], hi[16];
+          if (!whole) {
+            const int32_t* from = row_sums(p, seg, peers, q) + quad * 32 + 2 * (lane & 3) * kPanelN + (lane >> 2);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {   // rows 8 (k / 4) + k % 2 further, columns 8 (k / 2 % 2), and 16 more
+              lo[k] = (uint32_t)__ldcg(from + (8 * (k >> 2) + (k & 1)) * kPanelN + 8 * ((k >> 1) & 1));
+              hi[k] = (uint32_t)__ldcg(from + (8 * (k >> 2) + (k & 1)) * kPanelN + 8 * ((k >> 1) & 1) + 16);
+            }
+          } else if (has) {
+            tmem_ld_fragments(acc_addr, lo, hi);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) lo[k] = hi[k] = 0u;
+          }
+          if (epi_tid == 0 && q == 0) stamp<TRACE>(p, 9);
+          if (whole && q == npan - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bars.acc_empty[buf]));
+          }
+          if (store_pending) {
+            if (lane == 0) bulk_wait_read();
+            __syncwarp();
+          }
+          if (whole && !has && p.bias == nullptr && p.row_bias == nullptr) {
+            // an empty tile row without bias is zeros under every activation: no conversions
+            uint4* z = reinterpret_cast<uint4*>(smem_raw + (part - smem_u32(smem_raw))) + lane;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) z[k * 32] = make_uint4(0u, 0u, 0u, 0u);
+          } else {
+            finish_fragments<KIND, ACT>(od, row * kTile, lo, hi, rs, csq, biasq, p.bias != nullptr, part, lane);
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(&tmap_c, part, (chunk * p.np + q) * kPanelN + quad * 32, row * kTile);
+            bulk_commit();
+          }
+          store_pending = true;
+          // (after the store has been issued: the fence in front of it would wait for these writes)
+          if (!whole) {
+            int32_t* sums = row_sums(p, seg, peers, q) + m_first * kPanelN + quad * 32;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) reinterpret_cast<int4*>(sums)[(lane >> 3) * 32 + k * 128 + (lane & 7)] = make_int4(0, 0, 0, 0);
+          }
+        } else {
+          uint32_t r[C::COLS];
+          OutDesc to = od;
+          if (!whole) {
+            int32_t* sums = row_sums(p, seg, peers, q) + m_first * kPanelN + quad * 32;
+#pragma unroll
+            for (int k = 0; k < C::COLS; ++k) r[k] = (uint32_t)(peers ? __ldcv(sums + k * kPanelN + lane) : __ldcg(sums + k * kPanelN + lane));
+#pragma unroll
+            for (int k = 0; k < C::COLS; ++k) sums[k * kPanelN + lane] = 0;
+            if (od.acc_out != nullptr && n < od.N) {
+              uint32_t* a = reinterpret_cast<uint32_t*>(od.acc_out) + ((size_t)row * kTile + m_first) * od.N + n;
+#pragma unroll
+              for (int k = 0; k < C::COLS; ++k) a[(size_t)k * od.N] = r[k];
+            }
+            if (peers) to.out = p.peer_out[word_of(seg, 5)];   // the owner's rows of C
+          } else if (has) {
+            tmem_ld_cols<C::COLS>(acc_addr, r);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int k = 0; k < C::COLS; ++k) r[k] = 0u;
+          }
+          if (whole && q == npan - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bars.acc_empty[buf]));
+          }
+#pragma unroll
+          for (int c = 0; c < C::COLS; c += 16) {
+            if (TR) finish16_tr<KIND, ACT>(to, row, n, m_first + c, &r[c], rs, csq, biasq);
+            else finish16<KIND, ACT>(to, row, n, m_first + c, &r[c], rs, csq, biasq);
+          }
+        }
+        if (epi_tid == 0 && q == 0) stamp<TRACE>(p, 10);
       }
     }
-    // the staging tile must have been read before shared memory is given back; the writes themselves
+    // a part must have been read before shared memory is given back; the writes themselves
     // complete with the kernel
-    if (store_pending && (p.tma_store == 2 ? lane == 0 : epi_tid == 0)) bulk_wait_read();
+    if (store_pending && lane == 0) bulk_wait_read();
     if (epi_tid == 0) stamp<TRACE>(p, 6);
   }
   pipeline_teardown<C, TRACE>(p, ctl_s, tmem_base, tmem_cols);
 }
 
-template <class C, typename Kernel>
-int launch_rowacc(Kernel kernel, const RowaccLaunch& l, const CUtensorMap& b, const CUtensorMap& c, const SpmmParams& p) {
+template <int KIND, class C, int TR, int EPI>
+int launch_rowacc(const RowaccLaunch& l, const CUtensorMap& b, const CUtensorMap& c, const SpmmParams& p) {
+  auto kernel = spmm_rowacc_kernel<KIND, C, TR, EPI>;
   if (ensure_smem((const void*)kernel, l.smem_bytes)) return VOID_ERR_CUDA;
   launch_pdl(kernel, l.grid, C::THREADS, l.smem_bytes, l.stream, b, c, p);
   return VOID_OK;
 }
-template <int KIND, int TR>
-int launch_rowacc_tr(const RowaccLaunch& l, const CUtensorMap& b, const CUtensorMap& c, const SpmmParams& p) {
-  if constexpr (KIND != VOID_KIND_I8)
-    if (!l.slim) return launch_rowacc<Wide>(spmm_rowacc_kernel<KIND, Wide, TR>, l, b, c, p);
-  return launch_rowacc<Slim>(spmm_rowacc_kernel<KIND, Slim, TR>, l, b, c, p);
+template <int KIND, class C>
+int launch_rowacc(const RowaccLaunch& l, const CUtensorMap& b, const CUtensorMap& c, const SpmmParams& p) {
+  if constexpr (KIND != VOID_KIND_F8E4M3 && (KIND != VOID_KIND_I8 || C::COLS == kTile)) {
+    if (l.transposed)
+      return l.transposed == 1
+                 ? (l.epilogue & kActive ? launch_rowacc<KIND, C, 1, kActive>(l, b, c, p) : launch_rowacc<KIND, C, 1, 0>(l, b, c, p))
+                 : (l.epilogue & kActive ? launch_rowacc<KIND, C, 2, kActive>(l, b, c, p) : launch_rowacc<KIND, C, 2, 0>(l, b, c, p));
+  }
+  switch (l.epilogue) {
+    case 0: return launch_rowacc<KIND, C, 0, 0>(l, b, c, p);
+    case kActive: return launch_rowacc<KIND, C, 0, kActive>(l, b, c, p);
+    case kSplit | kActive: return launch_rowacc<KIND, C, 0, kSplit | kActive>(l, b, c, p);
+    default: break;
+  }
+  if constexpr (C::COLS == kTile) {   // slim
+    if (l.epilogue == kStaged) return launch_rowacc<KIND, C, 0, kStaged>(l, b, c, p);
+    if (l.epilogue == (kStaged | kActive)) return launch_rowacc<KIND, C, 0, kStaged | kActive>(l, b, c, p);
+    if constexpr (KIND != VOID_KIND_F8E4M3)
+      if (l.epilogue == (kStaged | kSplit | kActive)) return launch_rowacc<KIND, C, 0, kStaged | kSplit | kActive>(l, b, c, p);
+  }
+  if constexpr (KIND == VOID_KIND_I8 && C::COLS == kTile) {
+    constexpr int T = kTraced | kActive;
+    switch (l.epilogue) {
+      case T: return launch_rowacc<KIND, C, 0, T>(l, b, c, p);
+      case T | kStaged: return launch_rowacc<KIND, C, 0, T | kStaged>(l, b, c, p);
+      case T | kSplit: return launch_rowacc<KIND, C, 0, T | kSplit>(l, b, c, p);
+      case T | kStaged | kSplit: return launch_rowacc<KIND, C, 0, T | kStaged | kSplit>(l, b, c, p);
+    }
+  }
+  return VOID_ERR_BAD_ARG;
 }
 template <int KIND>
 int launch_rowacc(const RowaccLaunch& l, const CUtensorMap& b, const CUtensorMap& c, const SpmmParams& p) {
-  if constexpr (KIND != VOID_KIND_F8E4M3) {
-    if (l.transposed == 1) return launch_rowacc_tr<KIND, 1>(l, b, c, p);
-    if (l.transposed == 2) return launch_rowacc_tr<KIND, 2>(l, b, c, p);
-  }
-  if constexpr (KIND == VOID_KIND_I8)
-    if (l.slim && l.traced) return launch_rowacc<Slim>(spmm_rowacc_kernel<KIND, Slim, 0, true>, l, b, c, p);
-  return l.slim ? launch_rowacc<Slim>(spmm_rowacc_kernel<KIND, Slim>, l, b, c, p) : launch_rowacc<Wide>(spmm_rowacc_kernel<KIND, Wide>, l, b, c, p);
+  return l.slim ? launch_rowacc<KIND, Slim>(l, b, c, p) : launch_rowacc<KIND, Wide>(l, b, c, p);
 }
 
 }  // namespace vb

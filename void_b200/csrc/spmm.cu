@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(C::THREADS, (NP == 4) ? 1 : C::CTAS_PER_SM) sp
   const uint32_t tmem_base = tmem_base_s;
 
   if (warp < C::PW) {
-    producer_loop<C, 1, false, TRACE>(p, &tmap_b, &bars, ring_base, stage_bytes, ctl, lane, warp);
+    producer_loop<C, 1, 0, false, TRACE>(p, &tmap_b, &bars, ring_base, stage_bytes, ctl, lane, warp);
     if (warp == 0 && lane == 0) stamp<TRACE>(p, 2);
   } else if (warp == C::MMA) {
     {
@@ -54,16 +54,16 @@ __global__ void __launch_bounds__(C::THREADS, (NP == 4) ? 1 : C::CTAS_PER_SM) sp
       const uint32_t tiles_at = (uint32_t)(G * NP) * kPanelBytes;
       constexpr uint64_t kPanelStep = kPanelBytes >> 4, kTileStep = kTileBytes >> 4;
       int begin, end, step;
-      seg_range(p, begin, end, step);
+      seg_range<false>(p, begin, end, step);
       int stage = 0, slot = 0;
       uint32_t phase = 0, sphase = 0;
       uint32_t sbase = ring_base;
       bool ok = true;
       Seg seg_next = {};  // the next segment's descriptor is fetched one item ahead
-      if (begin < end) seg_next = load_seg(p, begin);
+      if (begin < end) seg_next = load_seg<false>(p, begin);
       for (int i = begin; i < end && ok; i += step) {
         const Seg s = seg_next;
-        if (i + step < end) seg_next = load_seg(p, i + step);
+        if (i + step < end) seg_next = load_seg<false>(p, i + step);
         const int npan = panels_in_chunk(p, s.chunk);
         for (int t = s.t0; t < s.t1; t += G) {
           const int gcnt = (s.t1 - t) < G ? (s.t1 - t) : G;
@@ -107,15 +107,15 @@ __global__ void __launch_bounds__(C::THREADS, (NP == 4) ? 1 : C::CTAS_PER_SM) sp
     const int G = p.group;
     grid_dependency_wait();
     int begin, end, step;
-    seg_range(p, begin, end, step);
+    seg_range<false>(p, begin, end, step);
     int slot = 0;
     uint32_t sphase = 0;
     bool alive = true;
     Seg seg_next = {};  // the next segment's descriptor is fetched one item ahead
-    if (begin < end) seg_next = load_seg(p, begin);
+    if (begin < end) seg_next = load_seg<false>(p, begin);
     for (int i = begin; i < end && alive; i += step) {
       const Seg s = seg_next;
-      if (i + step < end) seg_next = load_seg(p, i + step);
+      if (i + step < end) seg_next = load_seg<false>(p, i + step);
       const int npan = panels_in_chunk(p, s.chunk);
       float acc[NP][CW];
 #pragma unroll
@@ -354,12 +354,12 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   // 16-bit outputs of the slim row-accumulate kernel leave through a staging tile (32 x 128 x 2 bytes behind the
   // ring) and a tiled TMA store, when C qualifies as a tensor for the copy engine (16-byte aligned base and pitch)
   // (with a plan, whole-row segments take this route and the pieces of split rows the ordinary one)
-  const bool tma_store = !drain && !tr && slim && a->acc_out == nullptr &&
+  const bool staged = !drain && !tr && slim && a->acc_out == nullptr && a->n_peers == 0 &&
                          a->worker_partials == nullptr && (a->flags & 2) == 0 &&
                          (a->out_dtype == VOID_OUT_F16 || a->out_dtype == VOID_OUT_BF16) &&
                          (reinterpret_cast<uintptr_t>(a->out) & 15u) == 0 && ((a->ldc * 2) & 15) == 0;
   const int stage_bytes = group * (np * kPanelBytes + kTileBytes * terms) * es;
-  const int staging_bytes = tma_store ? kTile * kPanelN * 2 : 0;
+  const int staging_bytes = staged ? kTile * kPanelN * 2 : 0;
   int stages = a->stages;
   if (stages == 0) {
     // dynamic shared memory a CTA may use so that its share of them fits an SM: the SM's bytes less the kilobyte
@@ -440,7 +440,6 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   p.last_group = last_group;
   p.use3d = (!tr_b && a->N % (kPanelN / es) == 0) ? 1 : 0;
   p.tmem_cols = drain_tmem;
-  p.tma_store = tma_store ? ((a->flags & 16) ? 1 : 2) : 0;   // 2: one store per epilogue warp; 1: one per tile
   p.n_items = a->nbr * n_chunks;
   p.passes = make_passes(dev, a->nbr, n_chunks, a->K, np * kPanelN * es);
   p.a_stable = (a->flags & 4) ? 1 : 0;
@@ -507,9 +506,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
 
   CUtensorMap tmap_c;
   memset(&tmap_c, 0, sizeof(tmap_c));
-  if (tma_store) {
-    if (!store_map(&tmap_c, a->out, a->ldc, a->M, a->N, (a->flags & 16) ? kPanelN : 32)) return VOID_ERR_TENSOR_MAP;
-  }
+  if (staged && !store_map(&tmap_c, a->out, a->ldc, a->M, a->N)) return VOID_ERR_TENSOR_MAP;
 
 #define VB_LAUNCH(KERNEL, SHAPE)                                                               \
   do {                                                                                        \
@@ -518,7 +515,10 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   } while (0)
   const bool traced = a->trace != nullptr;
   if (!drain) {
-    const RowaccLaunch l = {slim, a->transposed, traced, grid, smem_bytes, stream};
+    const bool split = a->segs != nullptr || a->acc_out != nullptr || a->worker_partials != nullptr;
+    const bool active = split || traced || a->act != VOID_ACT_NONE || a->row_bias != nullptr;
+    const int epilogue = (staged ? kStaged : 0) | (split ? kSplit : 0) | (active ? kActive : 0) | (traced ? kTraced : 0);
+    const RowaccLaunch l = {slim, a->transposed, epilogue, grid, smem_bytes, stream};
     const int st = kind == VOID_KIND_I8       ? launch_rowacc<VOID_KIND_I8>(l, tmap, tmap_c, p)
                    : kind == VOID_KIND_F8E4M3 ? launch_rowacc<VOID_KIND_F8E4M3>(l, tmap, tmap_c, p)
                    : kind == VOID_KIND_TF32   ? launch_rowacc<VOID_KIND_TF32>(l, tmap, tmap_c, p)
