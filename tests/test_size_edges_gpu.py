@@ -378,3 +378,23 @@ def test_products_in_passes_equal_products_of_few_columns(dtype, k, n, linear):
     parts = [product(lo, min(n, lo + step)) for lo in range(0, n, step)]
     void.check_device_status()
     assert torch.equal(whole, torch.cat(parts, 1))
+
+
+# ------------------------------------------------------------------------------------------ panels per item and CTA shapes
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m,k,n,density,linear", [
+    (2110, 300, 5700, 0.95, False),     # two panels per item (16 bits), an odd number of them
+    (2080, 300, 5633, 0.7, False),      # rows too short for it
+    (4250, 300, 5800, 0.95, True),      # two panels per item, x as it lies
+    (2110, 640, 5700, 0.95, True),      # ... with fewer items and longer rows
+    (16390, 640, 1100, 0.95, True),     # ... and x transposed first
+    (9000, 300, 515, 0.5, True)])       # one panel, slim CTAs for every type
+def test_large_floating_products_are_exact_on_small_integers(dtype, m, k, n, density, linear):
+    dense, gen = _integer_matrix(m, k, density, m + n)
+    a = void.dense_to_void(dense.cuda()).to_dtype(dtype)
+    b = torch.randint(-2, 3, (n, k) if linear else (k, n), generator=gen).cuda().to(dtype)
+    ref = b.double() @ dense.cuda().double().t() if linear else dense.cuda().double() @ b.double()
+    for _ in range(2):
+        y = void.void_linear(a, b) if linear else void.void_spmm(a, b)
+        assert torch.equal(y.double(), ref.to(dtype).double())
+    void.check_device_status()

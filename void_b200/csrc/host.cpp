@@ -354,10 +354,11 @@ int64_t row_pitch(const at::Tensor& b, int es) {
 // A linear layer on x [N, K] either reads x as it lies (its 32-element pieces of rows load at a fraction of the rate of
 // whole panels) or has it transposed to [K, N] first and its result written transposed.  The copy costs two passes over x
 // and a launch that nothing overlaps; what it saves grows with the (tile, 128 columns) products: INT8 0.36 ns each (8192^2,
-// N = 1024, 80 %: 73.4 -> 40.6 us), 16 bits 0.1 (70 %: 98.0 -> 92.9; 4096^2, N = 4096, 60 %: 134 -> 127), fp32 no more than
-// the copy takes (8192^2, N = 1024, 50 %: 298.5 against 298.8).
+// N = 1024, 80 %: 73.4 -> 40.6 us), 16 bits 0.15 (16384 rows of 13 / 26 / 51 tiles, N = 2048: 83.6 -> 78.0, 142 -> 130, 260 -> 233;
+// 8192 rows, N = 4096: 85.4 -> 83.0, 150 -> 150, 270 -> 259), fp32 no more than the copy takes (8192^2, N = 1024, 50 %: 298.5
+// against 298.8).
 double copy_saves_ns(int kind, int64_t nnz, int64_t N) {
-  const double per = kind == VOID_KIND_I8 ? 0.36 : (kind == VOID_KIND_TF32 ? 0.0 : 0.1);
+  const double per = kind == VOID_KIND_I8 ? 0.36 : (kind == VOID_KIND_TF32 ? 0.0 : 0.15);
   return per * (double)nnz * (double)((N + 127) / 128);
 }
 double copy_costs_ns(int64_t N, int64_t K, int es) { return 5000.0 + 2.0 * (double)N * (double)K * es / 4500.0; }

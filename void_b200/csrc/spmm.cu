@@ -294,7 +294,17 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   int np = a->panels_per_item;
   if (np != 0 && np != 1 && np != 2 && np != 4) return VOID_ERR_BAD_ARG;
   if (floating && np > 2) return VOID_ERR_BAD_ARG;  // ring stages of wider items do not fit
-  if (np == 0 && floating) np = 1;
+  // Floating products: one panel per item, and the CTA shape that goes with the length of the tile rows (below); of 16-bit
+  // tiles two panels per item, in slim CTAs, where there are twenty items per SM: a tile then comes in once for both and an SM
+  // keeps more in flight (8 x 18 KB against 11 x 10 KB).  us, one panel in the better shape and two: 16384 x 4096, 13 tiles per
+  // row, N = 2048 69.6, 64.3; C transposed 16384 x 13056, 51 tiles 256, 231; both transposed, N = 4096, 8192 x 3328 89.4, 85.4,
+  // 8192 x 6656 156, 150.  Not for rows of under 8 tiles (4096 items, B and C as they are: 23.6 against 24.4) nor, with B
+  // transposed, under 16 and forty items per SM (45.2 against 44.8 - 46.5).
+  const long long row_panels = (long long)a->nbr * total_panels;
+  const bool by_rule = floating && np == 0 && a->cta_shape == 0 && a->segs == nullptr && es == 2;
+  const bool two_panels = by_rule && row_panels >= 20ll * dev.sms &&
+                          (tr_b ? row_panels >= 40ll * dev.sms || a->nnz > 16ll * a->nbr : a->nnz >= 8ll * a->nbr);
+  if (np == 0 && floating) np = two_panels ? 2 : 1;
   if (np == 0) {
     // two panels per item keep two CTAs on an SM, which measured faster than four panels with one
     np = total_panels >= 2 ? 2 : 1;
@@ -308,15 +318,22 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   // for its row is the row's tiles times the ring's round trip, and a slim ring holds two 32-bit tiles or four 16-bit
   // ones; 4096^2, 90 %, N = 512: fp32 15.7 -> 13.1 us, fp16 9.1 -> 8.8; 2048^2, 80 %, N = 256 fp32 12.1 -> 8.1), for the
   // per-tile kernel and for four-panel items (TMEM: 2 x np x 32 columns per row-accumulate CTA, 512 per SM).  Short tile
-  // rows of 16-bit tiles are bound by what an item costs besides its stream, which four CTAs hide better where the SM has
-  // more than two items: 16384 x 4096, N = 2048 at 4 / 8 / 13 tiles per row: slim 41 / 53 / 74 us, wide 60 / 67 / 82; N = 512:
-  // 12 / 16.5 / 22.5 against 16 / 18 / 21.9.  Transposed, N = 2048, 4 tiles: 55 against 61, and even from 6 tiles on.
+  // rows are bound by what an item costs besides its stream, which four CTAs hide better where the SM has more than two
+  // items.  16-bit tiles, wide and slim, us: 8192 rows, N = 512, 6 / 13 / 20 tiles per row 8.7 7.8, 12.4 12.1, 16.0 16.4; N = 2048
+  // 26.4 20.6, 39.2 37.1, 55.6 52.2; B transposed, N = 1024 6 / 9 / 13 / 20 tiles 19.0 18.4, 21.6 20.2, 25.0 24.8, 33.0 33.6; 2048 rows,
+  // N = 1024 (512 items) 9 tiles 7.85 8.03.  32-bit tiles with B transposed, N = 1024, 3 / 6 / 9 / 13 tiles: 22.8 22.3, 27.4 25.5,
+  // 33.0 31.9, 41.6 40.9; 2048 rows, N = 512 26 tiles 21.7 22.1; as they are slim is no faster from 6 tiles on.
   int shape = a->cta_shape;
   if (shape < 0 || shape > 5) return VOID_ERR_BAD_ARG;
   if (tr && np > 2) return VOID_ERR_BAD_ARG;
   if (tr && shape == 1 && kind == VOID_KIND_I8) return VOID_ERR_BAD_ARG;  // (8-bit transposed: the slim shape only)
   const long long n_items = (long long)a->nbr * n_chunks;
-  const bool short_rows = es == 2 && n_items > 2ll * dev.sms && a->nnz <= (tr_b ? 6ll : (n_items > 20ll * dev.sms ? 14ll : 10ll)) * a->nbr;
+  long long short_row = 0;   // tiles per row up to which rows are short
+  if (n_items > 2ll * dev.sms) {
+    if (es == 2) short_row = tr_b ? (n_items > 6ll * dev.sms ? 16 : 6) : (n_items > 20ll * dev.sms ? 14 : 10);
+    else if (tr_b) short_row = 10;
+  }
+  const bool short_rows = a->nnz <= short_row * a->nbr;
   if (shape == 0) shape = (!drain && np <= 2) ? ((floating && np == 1 && a->segs == nullptr && !short_rows) ? 1 : 2) : ((drain && np == 1) ? kDefaultDrainShape : 1);
   if (shape == 2 && (np > 2 || (drain && np > 1))) return VOID_ERR_BAD_ARG;
   if (shape >= 3 && (!drain || np != 1 || tr)) return VOID_ERR_BAD_ARG;  // shapes of the per-tile kernel
