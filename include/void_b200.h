@@ -99,7 +99,8 @@ VOID_API int void_build_tile_index(const int32_t* block_rows, const int32_t* blo
  *      tiles and, for the dense form, the number of nonzero elements (nnz_original, :429).
  *   2. the caller reads counts[0], allocates, and calls void_morton_emit: block_rows,
  *      block_cols, morton_codes [n_blocks] in ascending Morton order.
- *   3. void_dense_gather copies the kept tiles (zero padding outside the matrix, :374-378);
+ *   3. void_dense_gather copies the kept tiles (zero padding outside the matrix, :374-378), or
+ *      void_dense_emit does 2 and 3 in one launch;
  *      void_csr_scatter zero-fills values [n_blocks, 32, 32] and places every stored entry
  *      (entries with equal coordinates race; the reference keeps the later one).
  * ------------------------------------------------------------------------------------- */
@@ -116,6 +117,9 @@ VOID_API int void_morton_emit(const void* ws, int32_t nbr, int32_t nbc, int64_t 
 VOID_API int void_dense_gather(const void* matrix, int32_t elem, int64_t ld, int32_t M, int32_t N,
                                const int32_t* block_rows, const int32_t* block_cols,
                                int64_t n_blocks, void* values, void_stream_t stream);
+VOID_API int void_dense_emit(const void* ws, const void* matrix, int32_t elem, int64_t ld, int32_t M, int32_t N,
+                             int64_t n_blocks, int32_t* block_rows, int32_t* block_cols, int64_t* morton_codes,
+                             void* values, void_stream_t stream);
 VOID_API int void_csr_scatter(const int32_t* crow, const int32_t* col, const float* data, int32_t M,
                               int32_t N, const void* ws, int64_t n_blocks, float* values,
                               void_stream_t stream);

@@ -66,7 +66,8 @@ def test_linear_gradients_exact_on_small_integers(dtype, m, k, n):
 @pytest.mark.parametrize("m,n,off,dtype,threshold", [
     (1, 1, 0, torch.float32, 0.0), (31, 33, 0, torch.float32, 0.0), (64, 126, 1, torch.float32, 0.0),
     (100, 130, 0, torch.float16, 2.0), (65, 257, 0, torch.bfloat16, 0.0), (33, 264, 1, torch.bfloat16, 1.5),
-    (64, 256, 0, torch.float32, -1.0), (32, 32800, 0, torch.float16, 0.0)])
+    (64, 256, 0, torch.float32, -1.0), (32, 32800, 0, torch.float16, 0.0), (70, 16384, 0, torch.float32, 0.0),
+    (70, 16385, 0, torch.bfloat16, 0.0)])
 def test_dense_to_void_widths_and_alignments(m, n, off, dtype, threshold):
     gen = torch.Generator().manual_seed(m * 7 + n)
     full = (torch.randn(m, n, generator=gen) * (torch.rand(m, n, generator=gen) < 0.01)).to(dtype)
@@ -100,6 +101,18 @@ def test_packed_store_of_grids_of_every_size(nbr, nbc):
     assert np.array_equal(p.tile_cols.cpu().numpy(), cols[ref_bi]) and np.array_equal(p.tile_scales.cpu().numpy(), ref_s[ref_bi])
     order = np.argsort(-np.diff(ref_rp), kind="stable")
     assert np.array_equal(p.row_order.cpu().numpy(), order)
+
+
+@pytest.mark.parametrize("nbr,nbc,nnz", [(1, 1, 1), (1, 1, 0), (3, 33, 60), (4000, 64, 16384), (4001, 64, 900), (363, 1024, 16384),
+                                         (363, 1024, 16385), (364, 1024, 1000), (1024, 256, 16000)])
+def test_tile_index_around_the_limits_of_one_block(nbr, nbc, nnz):
+    from void_b200.format import build_tile_index
+    gen = torch.Generator().manual_seed(nbr + nbc + nnz)
+    cells = torch.randperm(nbr * nbc, generator=gen)[:nnz]
+    rows, cols = (cells // nbc).int(), (cells % nbc).int()
+    row_ptr, indices = build_tile_index(rows.cuda(), cols.cuda(), nbr, nbc)
+    assert torch.equal(row_ptr.cpu(), torch.cat([torch.zeros(1), torch.bincount(rows.long(), minlength=nbr).cumsum(0)]).int())
+    assert torch.equal(indices.cpu(), cells.argsort().int())
 
 
 def test_tile_lists_that_are_not_valid_are_refused():

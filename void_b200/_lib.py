@@ -66,6 +66,7 @@ _PROTOTYPES = {
     "void_dense_mark": (ctypes.c_int, [c_vp, c_i32, c_i64, c_i32, c_i32, c_f32, c_vp, c_sz, c_vp, c_vp]),
     "void_csr_mark": (ctypes.c_int, [c_vp, c_vp, c_i32, c_i32, c_vp, c_sz, c_vp, c_vp]),
     "void_morton_emit": (ctypes.c_int, [c_vp, c_i32, c_i32, c_i64, c_vp, c_vp, c_vp, c_vp]),
+    "void_dense_emit": (ctypes.c_int, [c_vp, c_vp, c_i32, c_i64, c_i32, c_i32, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "void_dense_gather": (ctypes.c_int, [c_vp, c_i32, c_i64, c_i32, c_i32, c_vp, c_vp, c_i64, c_vp, c_vp]),
     "void_csr_scatter": (ctypes.c_int, [c_vp, c_vp, c_vp, c_i32, c_i32, c_vp, c_i64, c_vp, c_vp]),
     "void_row_order": (ctypes.c_int, [c_vp, c_i32, c_vp, c_vp]),

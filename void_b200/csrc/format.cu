@@ -13,6 +13,8 @@
 #include <stdint.h>
 
 #include "../../include/void_b200.h"
+#include "launch.cuh"
+#include "ptx.cuh"
 
 namespace vbf {
 
@@ -144,6 +146,7 @@ __global__ void __launch_bounds__(256) dense_mark_kernel(const T* __restrict__ a
     atomicOr(bitmap + (code >> 5), 1u << (code & 31));
   }
   if (lane == 0 && nz) atomicAdd(&block_nz, nz);
+  vb::grid_launch_dependents();   // the ranking waits on an SM until all blocks are through
   __syncthreads();
   if (threadIdx.x == 0 && block_nz) atomicAdd(counts + 1, (unsigned long long)block_nz);
 }
@@ -171,6 +174,7 @@ __global__ void __launch_bounds__(1024) rank_bitmap_kernel(const uint32_t* __res
                                                            const unsigned long long* __restrict__ counts,
                                                            int64_t* __restrict__ counts_out) {
   __shared__ int32_t warp_sum[32];
+  vb::grid_dependency_wait();
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int per = (words + 1023) / 1024;
   const int lo = tid * per < words ? tid * per : words, hi = lo + per < words ? lo + per : words;
@@ -323,6 +327,52 @@ __global__ void dense_gather_kernel(const T* __restrict__ a, int64_t ld, int M, 
   for (int k = 0; k < 8; ++k) dst[k * 128] = v[k];
 }
 
+// Both for the grids that most matrices have: a block takes a word of the bitmap, each of its eight warps four bits of it, and
+// copies the tiles that are set, writing their coordinates on the way.  V elements are a 16-byte piece of a row, or 1.
+// 4096^2, 80 %, fp32 (13 MB each way, cold): 7.1 us against 3.8 + 5.1 and the gap between two launches.
+constexpr int kFusedWords = 8192;   // a grid side of 512 tiles
+template <typename T, int V>
+__global__ void __launch_bounds__(256) emit_tiles_kernel(const uint32_t* __restrict__ bitmap, const int32_t* __restrict__ word_prefix,
+                                                         const T* __restrict__ a, int64_t ld, int M, int N, int64_t n_blocks,
+                                                         int32_t* __restrict__ brow, int32_t* __restrict__ bcol,
+                                                         int64_t* __restrict__ codes, T* __restrict__ values) {
+  constexpr int PER_ROW = kTile / V, ROWS = 32 / PER_ROW;   // lanes of a tile row, rows a warp reads at once
+  const int lane = threadIdx.x & 31, first = (int)(threadIdx.x >> 5) * 4;
+  const uint32_t word = bitmap[blockIdx.x];
+  const int row = lane / PER_ROW, col = lane % PER_ROW * V;
+  for (uint32_t bits = word & (0xfu << first); bits != 0u; bits &= bits - 1u) {
+    const int b = __ffs((int)bits) - 1;
+    const uint32_t code = blockIdx.x * 32u + (uint32_t)b;
+    const int64_t rank = word_prefix[blockIdx.x] + __popc(word & ((1u << b) - 1u));
+    if (rank >= n_blocks) return;
+    const int r = (int)compact16(code), c = (int)compact16(code >> 1);
+    if (lane == 0) {
+      brow[rank] = r;
+      bcol[rank] = c;
+      codes[rank] = (int64_t)code;
+    }
+    const T* src = a + (size_t)(r * kTile + row) * ld + c * kTile + col;
+    T* dst = values + rank * (kTile * kTile) + row * kTile + col;
+    if constexpr (V > 1) {
+      if ((r + 1) * kTile <= M && (c + 1) * kTile <= N) {
+        uint4 v[kTile / ROWS];
+#pragma unroll
+        for (int k = 0; k < kTile / ROWS; ++k) v[k] = *reinterpret_cast<const uint4*>(src + (size_t)(k * ROWS) * ld);
+#pragma unroll
+        for (int k = 0; k < kTile / ROWS; ++k) *reinterpret_cast<uint4*>(dst + k * ROWS * kTile) = v[k];
+        continue;
+      }
+    }
+#pragma unroll 8
+    for (int k = 0; k < kTile / ROWS; ++k)
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        const bool in = r * kTile + row + k * ROWS < M && c * kTile + col + e < N;
+        dst[k * ROWS * kTile + e] = in ? src[(size_t)(k * ROWS) * ld + e] : T(0.0f);
+      }
+  }
+}
+
 // One warp per matrix row of the CSR matrix: every stored entry goes to its place in its tile.
 // Two entries with the same coordinates (a non-canonical CSR) race; the reference keeps the later one.
 __global__ void csr_scatter_kernel(const int32_t* __restrict__ crow, const int32_t* __restrict__ col,
@@ -351,7 +401,7 @@ static int rank_bitmap(const WsLayout& w, unsigned char* ws, int64_t* counts_out
   int32_t* chunk_ptr = reinterpret_cast<int32_t*>(ws + w.off_chunk);
   const unsigned long long* counts = reinterpret_cast<const unsigned long long*>(ws);
   if (w.words <= kOneBlockWords) {
-    rank_bitmap_kernel<<<1, 1024, 0, st>>>(bitmap, (int)w.words, word_prefix, counts, counts_out);
+    vb::launch_pdl(rank_bitmap_kernel, 1, 1024, 0, st, bitmap, (int)w.words, word_prefix, counts, counts_out);
     return last_status();
   }
   chunk_count_kernel<<<(unsigned)w.chunks, kChunkWords, 0, st>>>(bitmap, w.words, chunk_ptr);
@@ -371,6 +421,17 @@ static void launch_dense_mark(const void* matrix, int64_t ld, int M, int N, floa
   unsigned long long* counts = static_cast<unsigned long long*>(ws);
   if (vec) dense_mark_kernel<T, kVec><<<blocks, 256, 0, st>>>(a, ld, M, N, nbr, strips, threshold, bitmap_of(ws), counts);
   else dense_mark_kernel<T, 1><<<blocks, 256, 0, st>>>(a, ld, M, N, nbr, strips, threshold, bitmap_of(ws), counts);
+}
+
+template <typename T>
+static void launch_emit_tiles(const WsLayout& w, const void* ws, const void* matrix, int64_t ld, int M, int N, int64_t n_blocks,
+                              int32_t* brow, int32_t* bcol, int64_t* codes, void* values, cudaStream_t st) {
+  constexpr int kVec = 16 / (int)sizeof(T);
+  const int32_t* prefix = reinterpret_cast<const int32_t*>(static_cast<const unsigned char*>(ws) + w.off_prefix);
+  const T* a = static_cast<const T*>(matrix);
+  const bool vec = ld % kVec == 0 && ((reinterpret_cast<uintptr_t>(matrix) | reinterpret_cast<uintptr_t>(values)) & 15u) == 0;
+  auto kernel = vec ? emit_tiles_kernel<T, kVec> : emit_tiles_kernel<T, 1>;
+  kernel<<<(unsigned)w.words, 256, 0, st>>>(bitmap_of(ws), prefix, a, ld, M, N, n_blocks, brow, bcol, codes, static_cast<T*>(values));
 }
 
 }  // namespace vbf
@@ -452,6 +513,27 @@ int void_dense_gather(const void* matrix, int32_t elem, int64_t ld, int32_t M, i
     vbf::dense_gather_kernel<__nv_bfloat16><<<blocks, tb, 0, st>>>(static_cast<const __nv_bfloat16*>(matrix), ld, M, N,
                                                                     block_rows, block_cols, n_blocks,
                                                                     static_cast<__nv_bfloat16*>(values));
+  return vbf::last_status();
+}
+
+int void_dense_emit(const void* ws, const void* matrix, int32_t elem, int64_t ld, int32_t M, int32_t N, int64_t n_blocks,
+                    int32_t* block_rows, int32_t* block_cols, int64_t* morton_codes, void* values, void_stream_t stream) {
+  if (n_blocks < 0 || M < 0 || N < 0 || ld < N || ws == nullptr) return VOID_ERR_BAD_ARG;
+  if (elem < VOID_ELEM_F32 || elem > VOID_ELEM_BF16) return VOID_ERR_BAD_ARG;
+  if (n_blocks == 0) return VOID_OK;
+  const int nbr = (M + vbf::kTile - 1) / vbf::kTile, nbc = (N + vbf::kTile - 1) / vbf::kTile;
+  vbf::WsLayout w;
+  if (!vbf::ws_layout(nbr, nbc, &w)) return VOID_ERR_TOO_LARGE;
+  if (w.words > vbf::kFusedWords) {
+    const int st = void_morton_emit(ws, nbr, nbc, n_blocks, block_rows, block_cols, morton_codes, stream);
+    return st != VOID_OK ? st : void_dense_gather(matrix, elem, ld, M, N, block_rows, block_cols, n_blocks, values, stream);
+  }
+  if (matrix == nullptr || block_rows == nullptr || block_cols == nullptr || morton_codes == nullptr || values == nullptr)
+    return VOID_ERR_BAD_ARG;
+  cudaStream_t st = vbf::as_stream(stream);
+  if (elem == VOID_ELEM_F32) vbf::launch_emit_tiles<float>(w, ws, matrix, ld, M, N, n_blocks, block_rows, block_cols, morton_codes, values, st);
+  else if (elem == VOID_ELEM_F16) vbf::launch_emit_tiles<__half>(w, ws, matrix, ld, M, N, n_blocks, block_rows, block_cols, morton_codes, values, st);
+  else vbf::launch_emit_tiles<__nv_bfloat16>(w, ws, matrix, ld, M, N, n_blocks, block_rows, block_cols, morton_codes, values, st);
   return vbf::last_status();
 }
 

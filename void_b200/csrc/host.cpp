@@ -864,12 +864,9 @@ PyObject* dense_build(PyObject*, PyObject* const* a, Py_ssize_t n) {
   at::Tensor values = new_cuda({kept, 32, 32}, m.scalar_type(), dev);
   at::Tensor rows = new_cuda({kept}, at::kInt, dev), cols = new_cuda({kept}, at::kInt, dev);
   at::Tensor codes = new_cuda({kept}, at::kLong, dev);
-  check(void_morton_emit(ws.const_data_ptr(), nbr, nbc, kept, rows.data_ptr<int32_t>(), cols.data_ptr<int32_t>(),
-                         codes.data_ptr<int64_t>(), st),
-        "void_morton_emit");
-  check(void_dense_gather(m.const_data_ptr(), elem, ld, (int32_t)M, (int32_t)N, rows.const_data_ptr<int32_t>(),
-                          cols.const_data_ptr<int32_t>(), kept, values.data_ptr(), st),
-        "void_dense_gather");
+  check(void_dense_emit(ws.const_data_ptr(), m.const_data_ptr(), elem, ld, (int32_t)M, (int32_t)N, kept, rows.data_ptr<int32_t>(),
+                        cols.data_ptr<int32_t>(), codes.data_ptr<int64_t>(), values.data_ptr(), st),
+        "void_dense_emit");
   return Py_BuildValue("NNNNLL", THPVariable_Wrap(values), THPVariable_Wrap(rows), THPVariable_Wrap(cols), THPVariable_Wrap(codes),
                        (long long)kept, (long long)nonzeros);
   NATIVE_END
