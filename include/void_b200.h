@@ -327,7 +327,7 @@ typedef struct void_spmm_args {
   void* trace;
   int32_t cta_shape;       /* 0 default; 1 wide CTAs (13 warps, 2 per SM); 2 slim (7 warps, 4 per SM);
                               per-tile kernel with one panel only: 3 = 7 warps, 3 per SM; 4 = 10 warps, 3 per SM;
-                              5 = 6 warps, 4 per SM */
+                              5 = 6 warps, 4 per SM; floating operands without a plan or raw sums: 6 = 7 warps, 3 per SM */
   int32_t flags;           /* bit 1: no staged TMA store of 16-bit outputs (direct stores);
                               bit 2: the caller vouches that the packed A (tiles, tile_cols, tile_scales,
                               row_ptr, row_scale) and the plan were completely written before any kernel

@@ -246,7 +246,7 @@ def streamk_table(row_ptr: torch.Tensor, nbr: int, nnz: int, n_workers: Optional
     return rows[:n], start[:n], end[:n], atomic[:n].to(torch.bool), woff, target
 
 
-ROW_COST = 12  # epilogue of one (tile row, chunk) in units of one tile of work, swept on B200 (power-law workload: 6 -> 22.0 us, 12 -> 19.9, 24 -> 21.4)
+ROW_COST = 8   # epilogue of one (tile row, chunk) in units of one tile of work, swept on B200 (power-law rows, N = 256 / 1024, us: 4 15.6 / 45.7, 6 14.4 / 39.4, 8 13.9 / 37.0, 12 14.0 / 37.4, 16 14.8 / 39.4)
 
 
 def make_plan(packed: PackedTiles, N: int, np_: int, n_cta: int, mode: int, chunk_tiles: int = 0,

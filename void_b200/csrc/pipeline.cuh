@@ -78,6 +78,7 @@ struct Shape {
 };
 using Wide = Shape<4, 8, 2>;
 using Slim = Shape<2, 4, 4>;
+using Mid = Shape<2, 4, 3>;   // slim warps, three CTAs per SM: large products of 16- and 32-bit tiles
 // Shapes of the per-tile kernel, three CTAs per SM so that an epilogue thread can hold 32 raw products in
 // registers next to its running sums: four epilogue warps with all 32 accumulator columns each, or eight
 // with 16 each (two tiles per round trip to tensor memory).
@@ -444,7 +445,7 @@ __device__ __forceinline__ void pipeline_teardown(const SpmmParams& p, int* ctl_
 //   kTraced  time stamps (slim INT8 only, with kActive)
 constexpr int kStaged = 1, kSplit = 2, kActive = 4, kTraced = 8;
 struct RowaccLaunch {
-  bool slim;
+  int shape;   // 1 wide, 2 slim, 6 mid
   int transposed;
   int epilogue;
   int grid, smem_bytes;

@@ -405,13 +405,15 @@ int launch_rowacc(const RowaccLaunch& l, const CUtensorMap& b, const CUtensorMap
   switch (l.epilogue) {
     case 0: return launch_rowacc<KIND, C, 0, 0>(l, b, c, p);
     case kActive: return launch_rowacc<KIND, C, 0, kActive>(l, b, c, p);
-    case kSplit | kActive: return launch_rowacc<KIND, C, 0, kSplit | kActive>(l, b, c, p);
     default: break;
   }
-  if constexpr (C::COLS == kTile) {   // slim
+  if constexpr (C::COLS == kTile) {   // slim and mid
     if (l.epilogue == kStaged) return launch_rowacc<KIND, C, 0, kStaged>(l, b, c, p);
     if (l.epilogue == (kStaged | kActive)) return launch_rowacc<KIND, C, 0, kStaged | kActive>(l, b, c, p);
-    if constexpr (KIND != VOID_KIND_F8E4M3)
+  }
+  if constexpr (C::CTAS_PER_SM != Mid::CTAS_PER_SM) {
+    if (l.epilogue == (kSplit | kActive)) return launch_rowacc<KIND, C, 0, kSplit | kActive>(l, b, c, p);
+    if constexpr (KIND != VOID_KIND_F8E4M3 && C::COLS == kTile)
       if (l.epilogue == (kStaged | kSplit | kActive)) return launch_rowacc<KIND, C, 0, kStaged | kSplit | kActive>(l, b, c, p);
   }
   if constexpr (KIND == VOID_KIND_I8 && C::COLS == kTile) {
@@ -427,7 +429,9 @@ int launch_rowacc(const RowaccLaunch& l, const CUtensorMap& b, const CUtensorMap
 }
 template <int KIND>
 int launch_rowacc(const RowaccLaunch& l, const CUtensorMap& b, const CUtensorMap& c, const SpmmParams& p) {
-  return l.slim ? launch_rowacc<KIND, Slim>(l, b, c, p) : launch_rowacc<KIND, Wide>(l, b, c, p);
+  if constexpr (KIND == VOID_KIND_F16 || KIND == VOID_KIND_TF32)
+    if (l.shape == 6) return launch_rowacc<KIND, Mid>(l, b, c, p);
+  return l.shape == 2 ? launch_rowacc<KIND, Slim>(l, b, c, p) : launch_rowacc<KIND, Wide>(l, b, c, p);
 }
 
 }  // namespace vb

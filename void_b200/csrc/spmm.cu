@@ -295,15 +295,15 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   if (np != 0 && np != 1 && np != 2 && np != 4) return VOID_ERR_BAD_ARG;
   if (floating && np > 2) return VOID_ERR_BAD_ARG;  // ring stages of wider items do not fit
   // Floating products: one panel per item, and the CTA shape that goes with the length of the tile rows (below); of 16-bit
-  // tiles two panels per item, in slim CTAs, where there are twenty items per SM: a tile then comes in once for both and an SM
-  // keeps more in flight (8 x 18 KB against 11 x 10 KB).  us, one panel in the better shape and two: 16384 x 4096, 13 tiles per
-  // row, N = 2048 69.6, 64.3; C transposed 16384 x 13056, 51 tiles 256, 231; both transposed, N = 4096, 8192 x 3328 89.4, 85.4,
-  // 8192 x 6656 156, 150.  Not for rows of under 8 tiles (4096 items, B and C as they are: 23.6 against 24.4) nor, with B
-  // transposed, under 16 and forty items per SM (45.2 against 44.8 - 46.5).
+  // tiles two panels per item where there are twenty items per SM: a tile then comes in once for both and an SM keeps more in
+  // flight (9 x 18 KB in mid CTAs, 8 x 18 KB in slim ones, against 11 x 10 KB).  us, one panel in the better shape and two:
+  // 16384 rows, N = 2048, 3 / 6 / 13 tiles per row 28.1 24.8, 38.9 36.3, 69.6 61.7; 8192^2, 80 %, N = 2048 117 112; C transposed,
+  // 51 tiles 256 231; both transposed, N = 4096, 8192 x 3328 89.4 85.4, 8192 x 6656 156 150.  With B transposed not for rows of
+  // up to 16 tiles under forty items per SM (6 tiles 30.9 32.4, 13 tiles 45.2 44.8).
   const long long row_panels = (long long)a->nbr * total_panels;
-  const bool by_rule = floating && np == 0 && a->cta_shape == 0 && a->segs == nullptr && es == 2;
-  const bool two_panels = by_rule && row_panels >= 20ll * dev.sms &&
-                          (tr_b ? row_panels >= 40ll * dev.sms || a->nnz > 16ll * a->nbr : a->nnz >= 8ll * a->nbr);
+  const bool plain = floating && a->cta_shape == 0 && a->segs == nullptr && a->acc_out == nullptr && a->worker_partials == nullptr;
+  const bool two_panels = plain && es == 2 && np == 0 && row_panels >= 20ll * dev.sms &&
+                          (!tr_b || row_panels >= 40ll * dev.sms || a->nnz > 16ll * a->nbr);
   if (np == 0 && floating) np = two_panels ? 2 : 1;
   if (np == 0) {
     // two panels per item keep two CTAs on an SM, which measured faster than four panels with one
@@ -322,9 +322,15 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   // items.  16-bit tiles, wide and slim, us: 8192 rows, N = 512, 6 / 13 / 20 tiles per row 8.7 7.8, 12.4 12.1, 16.0 16.4; N = 2048
   // 26.4 20.6, 39.2 37.1, 55.6 52.2; B transposed, N = 1024 6 / 9 / 13 / 20 tiles 19.0 18.4, 21.6 20.2, 25.0 24.8, 33.0 33.6; 2048 rows,
   // N = 1024 (512 items) 9 tiles 7.85 8.03.  32-bit tiles with B transposed, N = 1024, 3 / 6 / 9 / 13 tiles: 22.8 22.3, 27.4 25.5,
-  // 33.0 31.9, 41.6 40.9; 2048 rows, N = 512 26 tiles 21.7 22.1; as they are slim is no faster from 6 tiles on.
+  // 33.0 31.9, 41.6 40.9; 2048 rows, N = 512 26 tiles 21.7 22.1.
+  // Between them the mid shape, slim CTAs three to an SM with rings in between: 16-bit products of two panels with rows of 5
+  // tiles and more (10 with B transposed), and 32-bit ones from six items per SM on.  fp32, 8192 rows, wide, slim, mid: N = 512, 3 /
+  // 6 / 13 tiles per row 9.6 9.1 8.4, 12.1 12.4 12.1, 20.6 21.0 20.5; N = 2048 28.9 25.3 24.5, 40.1 37.9 37.6, 73.1 70.9 65.6; 20 tiles
+  // 101 to 105 in all; B transposed, N = 2048, 6 / 9 / 13 / 20 tiles 52.4 48.1 50.1, 67.6 60.4 63.2, 86.3 79.7 77.8, 116 104 104.  With 512
+  // items it holds one and a half per CTA: 4096^2, 90 %, N = 512 12.1 13.0 13.9.
   int shape = a->cta_shape;
-  if (shape < 0 || shape > 5) return VOID_ERR_BAD_ARG;
+  if (shape < 0 || shape > 6) return VOID_ERR_BAD_ARG;
+  if (shape == 6 && (!floating || a->segs != nullptr || a->acc_out != nullptr || a->worker_partials != nullptr)) return VOID_ERR_BAD_ARG;
   if (tr && np > 2) return VOID_ERR_BAD_ARG;
   if (tr && shape == 1 && kind == VOID_KIND_I8) return VOID_ERR_BAD_ARG;  // (8-bit transposed: the slim shape only)
   const long long n_items = (long long)a->nbr * n_chunks;
@@ -334,12 +340,14 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
     else if (tr_b) short_row = 10;
   }
   const bool short_rows = a->nnz <= short_row * a->nbr;
+  if (plain && np == 2 && two_panels) shape = a->nnz >= (tr_b ? 10ll : 5ll) * a->nbr ? 6 : 2;
+  if (plain && np == 1 && es == 4 && n_items > 6ll * dev.sms && !(tr_b && short_rows)) shape = 6;
   if (shape == 0) shape = (!drain && np <= 2) ? ((floating && np == 1 && a->segs == nullptr && !short_rows) ? 1 : 2) : ((drain && np == 1) ? kDefaultDrainShape : 1);
   if (shape == 2 && (np > 2 || (drain && np > 1))) return VOID_ERR_BAD_ARG;
-  if (shape >= 3 && (!drain || np != 1 || tr)) return VOID_ERR_BAD_ARG;  // shapes of the per-tile kernel
-  const bool slim = (shape == 2);
-  const int producer_warps = (shape == 1) ? Wide::PW : ((shape >= 4) ? 1 : Slim::PW);
-  const int ctas_per_sm = (slim || shape == 5) ? 4 : (shape >= 3 ? 3 : ((np == 4) ? 1 : Wide::CTAS_PER_SM));
+  if (shape >= 3 && shape <= 5 && (!drain || np != 1 || tr)) return VOID_ERR_BAD_ARG;  // shapes of the per-tile kernel
+  const bool slim = (shape == 2 || shape == 6);   // seven warps, results of 16 bits staged
+  const int producer_warps = (shape == 1) ? Wide::PW : ((shape == 4 || shape == 5) ? 1 : Slim::PW);
+  const int ctas_per_sm = (shape == 2 || shape == 5) ? 4 : (shape >= 3 ? 3 : ((np == 4) ? 1 : Wide::CTAS_PER_SM));
   // CTAs that will share an SM: fewer than fit it when there are not enough work items, and each then has more of its
   // shared memory for the ring
   int share = ctas_per_sm;
@@ -355,7 +363,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   // too often.  With fewer CTAs on the SM longer stages pay (1024 x 8192, 70 %, N = 256, one CTA per SM: INT8 3 x 3 12.4
   // us, 7 x 6 10.4; FP8 of two terms 17.4 -> 13.3; fp16 21.5 -> 13.4 with 6 x 3; fp32 41.2 -> 25.3 with 8 x 1).
   if (group == 0) {
-    if (floating) group = (es == 2 && np == 1) ? ((tr_b && share > 1) || shape == 2 ? 2 : 3) : 1;
+    if (floating) group = (es == 2 && np == 1) ? ((tr_b && share > 1) || slim ? 2 : 3) : 1;
     // (a tile stored as several terms is that much longer: 3 stages x 2 at four CTAs, headline 7.66 us, 2 x 3: 7.93)
     else if (a->tile_terms > 1) group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 3 : 2)) : 1;
     else group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 4 : 3)) : 2;
@@ -535,7 +543,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
     const bool split = a->segs != nullptr || a->acc_out != nullptr || a->worker_partials != nullptr;
     const bool active = split || traced || a->act != VOID_ACT_NONE || a->row_bias != nullptr;
     const int epilogue = (staged ? kStaged : 0) | (split ? kSplit : 0) | (active ? kActive : 0) | (traced ? kTraced : 0);
-    const RowaccLaunch l = {slim, a->transposed, epilogue, grid, smem_bytes, stream};
+    const RowaccLaunch l = {shape, a->transposed, epilogue, grid, smem_bytes, stream};
     const int st = kind == VOID_KIND_I8       ? launch_rowacc<VOID_KIND_I8>(l, tmap, tmap_c, p)
                    : kind == VOID_KIND_F8E4M3 ? launch_rowacc<VOID_KIND_F8E4M3>(l, tmap, tmap_c, p)
                    : kind == VOID_KIND_TF32   ? launch_rowacc<VOID_KIND_TF32>(l, tmap, tmap_c, p)
