@@ -55,7 +55,7 @@ inline DeviceInfo device_info() {
 // on every launch of the pairs that found no room (correct, a little slower).
 inline int ensure_smem(const void* kernel, int bytes) {
   struct Rec { const void* fn; int dev; int bytes; };
-  constexpr int kRecs = 96 * 16;
+  constexpr int kRecs = 192 * 16;
   static Rec recs[kRecs];
   static int n_recs = 0;
   static std::mutex mu;
@@ -72,10 +72,13 @@ inline int ensure_smem(const void* kernel, int bytes) {
   return 0;
 }
 
-template <typename Kernel, typename... Args>
-void launch_pdl(Kernel kernel, int grid, int threads, int smem_bytes, cudaStream_t stream, const Args&... args) {
+template <typename T>
+struct same_type { using type = T; };
+// A launch that may start beside the end of the kernel before it.
+template <typename... P>
+void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem_bytes, cudaStream_t stream, const typename same_type<P>::type&... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)threads);
   cfg.dynamicSmemBytes = (size_t)smem_bytes;
   cfg.stream = stream;

@@ -137,15 +137,9 @@ struct SpmmParams {
   int32_t* partials;
   int32_t* counters;
   int32_t* worker_partials;
-  // Split rows whose sums live on other GPUs (reduction across ranks): n_peers > 0 makes field slot0 of a
-  // segment the owner of its tile row; the row's accumulator, arrival counter and rows of C are the owner's,
-  // reached through peer pointers (peer_out is offset so that the GLOBAL tile row indexes it).
-  int n_peers;
+  int n_peers;      // sums over ranks: PeerParams below
   int peer_slots;   // 1: every contributing rank stores its partial tile into its own slot of the owner's scratch
                     // (plain stores, no counters); a second kernel on the owner adds the slots (void_reduce_slots)
-  int32_t* peer_partials[8];
-  int32_t* peer_counters[8];
-  void* peer_out[8];
   int32_t* status;
   unsigned long long* trace;  // diagnostic instantiations only: 64 timestamps per CTA
   int np;       // panels per work item
@@ -165,6 +159,15 @@ struct SpmmParams {
   unsigned long long desc_hi_a;  // B panel  (instruction operand A: MN-major, 128B swizzle)
   unsigned long long desc_hi_b;  // A tile   (instruction operand B: K-major, no swizzle)
   unsigned int idesc;
+};
+
+// Split rows whose sums live on other GPUs (reduction across ranks): n_peers > 0 makes field slot0 of a segment the owner of its
+// tile row; the row's accumulator, arrival counter and rows of C are the owner's, reached through peer pointers (out is
+// offset so that the GLOBAL tile row indexes it).
+struct PeerParams {
+  int32_t* partials[8];
+  int32_t* counters[8];
+  void* out[8];
 };
 
 // Time stamps exist in the diagnostic instantiations (TRACE) only; the kernels every ordinary launch runs
@@ -450,8 +453,12 @@ struct RowaccLaunch {
   int epilogue;
   int grid, smem_bytes;
   cudaStream_t stream;
+  const CUtensorMap& b;
+  const CUtensorMap& c;
+  const PeerParams& peers;
+  const SpmmParams& p;
 };
 template <int KIND>
-int launch_rowacc(const RowaccLaunch& l, const CUtensorMap& b, const CUtensorMap& c, const SpmmParams& p);
+int launch_rowacc(const RowaccLaunch& l);
 
 }  // namespace vb

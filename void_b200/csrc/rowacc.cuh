@@ -1,5 +1,7 @@
 // The row-accumulate kernel (pipeline.cuh): one accumulator per (tile row, column chunk).
 #pragma once
+#include <type_traits>
+
 #include "pipeline.cuh"
 
 namespace vb {
@@ -12,18 +14,27 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[COLS]
 }
 
 // The accumulator of a split row's panel q, [32 m][128 n]; with peers the owner's.
-__device__ __forceinline__ int32_t* row_sums(const SpmmParams& p, int seg_words, bool peers, int q) {
-  int32_t* base = peers ? p.peer_partials[word_of(seg_words, 5)] : p.partials;
+template <typename X>
+__device__ __forceinline__ int32_t* row_sums(const SpmmParams& p, const X& x, int seg_words, bool peers, int q) {
+  int32_t* base = p.partials;
+  if constexpr (std::is_same<X, PeerParams>::value)
+    if (peers) base = x.partials[word_of(seg_words, 5)];
   return base + ((size_t)word_of(seg_words, 7) * p.np + q) * (kTile * kPanelN);
 }
+
+// What a kernel is given besides B and the common parameters: C as a tensor, the peers of a sum over ranks, or nothing.  (A
+// launch takes longer by about a nanosecond for every four bytes of parameters.)
+struct Nothing {};
+template <int EPI>
+using ExtraOf = std::conditional_t<(EPI & kStaged) != 0, CUtensorMap, std::conditional_t<(EPI & kSplit) != 0, PeerParams, Nothing>>;
 
 // TR: 1 = B and C transposed ([N, K] and [N, M]), 2 = C alone.  EPI: what the epilogue is asked for (kStaged ...).  One kernel
 // that could do all of it took 6.83 us for a launch that runs in 5.46 without activations and in 5.67 with them (INT8 4096^2,
 // 90 %, N = 512, fp16 results): what is not run costs too, in spilled registers and in instructions fetched around it.
 template <int KIND, class C, int TR, int EPI>
 __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel(const __grid_constant__ CUtensorMap tmap_b,
-                                                               const __grid_constant__ CUtensorMap tmap_c,
-                                                               const __grid_constant__ SpmmParams p) {
+                                                                                 const __grid_constant__ ExtraOf<EPI> x,
+                                                                                 const __grid_constant__ SpmmParams p) {
   constexpr bool STAGED = (EPI & kStaged) != 0, SPLIT = (EPI & kSplit) != 0, ACT = (EPI & kActive) != 0, TRACE = (EPI & kTraced) != 0;
   static_assert(!TR || (!STAGED && !SPLIT), "transposed results are stored directly, of whole rows");
   static_assert(!STAGED || C::COLS == kTile, "an epilogue warp stages whole columns of a tile row");
@@ -189,7 +200,12 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
         const int owner = word_of(seg, 5), ctr = word_of(seg, 7);
         // a split row whose scratch index lies outside what the caller provided is skipped and reported
         const bool bad_split = nseg > 1 && (ctr < 0 || ctr >= p.ctr_limit || (peers && (unsigned)owner >= (unsigned)p.n_peers));
-        int32_t* split_partials = peers && !bad_split ? p.peer_partials[owner] : p.partials;
+        int32_t *split_partials = p.partials, *counter = p.counters + ctr;
+        if constexpr (SPLIT && !STAGED)
+          if (peers && !bad_split) {
+            split_partials = x.partials[owner];
+            counter = x.counters[owner] + ctr;
+          }
         if (bad_split && epi_tid == 0 && p.status != nullptr) atomicCAS(p.status, 0, kStatusBadPlan);
 #pragma unroll 1
         for (int q = 0; q < npan; ++q) {
@@ -263,7 +279,6 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
         asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_THREADS) : "memory");
         if (epi_tid == 0) stamp<TRACE>(p, 13);
         if (epi_tid == 0) {
-          int32_t* counter = (peers ? p.peer_counters[owner] : p.counters) + ctr;
           const int old = peers ? atomicAdd_system(counter, 1) : atom_add_acq_rel(counter, 1);
           const int last = (old == nseg - 1) ? 1 : 0;
           if (last) *counter = 0;  // left clean for the next launch
@@ -299,7 +314,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
           // edges of C; the part is free again once the previous store has read it.
           uint32_t lo[16], hi[16];
           if (!whole) {
-            const int32_t* from = row_sums(p, seg, peers, q) + quad * 32 + 2 * (lane & 3) * kPanelN + (lane >> 2);
+            const int32_t* from = row_sums(p, x, seg, peers, q) + quad * 32 + 2 * (lane & 3) * kPanelN + (lane >> 2);
 #pragma unroll
             for (int k = 0; k < 16; ++k) {   // rows 8 (k / 4) + k % 2 further, columns 8 (k / 2 % 2), and 16 more
               lo[k] = (uint32_t)__ldcg(from + (8 * (k >> 2) + (k & 1)) * kPanelN + 8 * ((k >> 1) & 1));
@@ -333,13 +348,13 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            tma_store_2d(&tmap_c, part, (chunk * p.np + q) * kPanelN + quad * 32, row * kTile);
+            tma_store_2d(&x, part, (chunk * p.np + q) * kPanelN + quad * 32, row * kTile);
             bulk_commit();
           }
           store_pending = true;
           // (after the store has been issued: the fence in front of it would wait for these writes)
           if (!whole) {
-            int32_t* sums = row_sums(p, seg, peers, q) + m_first * kPanelN + quad * 32;
+            int32_t* sums = row_sums(p, x, seg, peers, q) + m_first * kPanelN + quad * 32;
 #pragma unroll
             for (int k = 0; k < 8; ++k) reinterpret_cast<int4*>(sums)[(lane >> 3) * 32 + k * 128 + (lane & 7)] = make_int4(0, 0, 0, 0);
           }
@@ -347,7 +362,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
           uint32_t r[C::COLS];
           OutDesc to = od;
           if (!whole) {
-            int32_t* sums = row_sums(p, seg, peers, q) + m_first * kPanelN + quad * 32;
+            int32_t* sums = row_sums(p, x, seg, peers, q) + m_first * kPanelN + quad * 32;
 #pragma unroll
             for (int k = 0; k < C::COLS; ++k) r[k] = (uint32_t)(peers ? __ldcv(sums + k * kPanelN + lane) : __ldcg(sums + k * kPanelN + lane));
 #pragma unroll
@@ -357,7 +372,8 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
 #pragma unroll
               for (int k = 0; k < C::COLS; ++k) a[(size_t)k * od.N] = r[k];
             }
-            if (peers) to.out = p.peer_out[word_of(seg, 5)];   // the owner's rows of C
+            if constexpr (SPLIT && !STAGED)
+              if (peers) to.out = x.out[word_of(seg, 5)];   // the owner's rows of C
           } else if (has) {
             tmem_ld_cols<C::COLS>(acc_addr, r);
             tmem_ld_wait();
@@ -388,50 +404,52 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
 }
 
 template <int KIND, class C, int TR, int EPI>
-int launch_rowacc(const RowaccLaunch& l, const CUtensorMap& b, const CUtensorMap& c, const SpmmParams& p) {
+int launch_rowacc(const RowaccLaunch& l) {
   auto kernel = spmm_rowacc_kernel<KIND, C, TR, EPI>;
   if (ensure_smem((const void*)kernel, l.smem_bytes)) return VOID_ERR_CUDA;
-  launch_pdl(kernel, l.grid, C::THREADS, l.smem_bytes, l.stream, b, c, p);
+  if constexpr ((EPI & kStaged) != 0) launch_pdl(kernel, l.grid, C::THREADS, l.smem_bytes, l.stream, l.b, l.c, l.p);
+  else if constexpr ((EPI & kSplit) != 0) launch_pdl(kernel, l.grid, C::THREADS, l.smem_bytes, l.stream, l.b, l.peers, l.p);
+  else launch_pdl(kernel, l.grid, C::THREADS, l.smem_bytes, l.stream, l.b, Nothing{}, l.p);
   return VOID_OK;
 }
 template <int KIND, class C>
-int launch_rowacc(const RowaccLaunch& l, const CUtensorMap& b, const CUtensorMap& c, const SpmmParams& p) {
+int launch_rowacc(const RowaccLaunch& l) {
   if constexpr (KIND != VOID_KIND_F8E4M3 && (KIND != VOID_KIND_I8 || C::COLS == kTile)) {
     if (l.transposed)
       return l.transposed == 1
-                 ? (l.epilogue & kActive ? launch_rowacc<KIND, C, 1, kActive>(l, b, c, p) : launch_rowacc<KIND, C, 1, 0>(l, b, c, p))
-                 : (l.epilogue & kActive ? launch_rowacc<KIND, C, 2, kActive>(l, b, c, p) : launch_rowacc<KIND, C, 2, 0>(l, b, c, p));
+                 ? (l.epilogue & kActive ? launch_rowacc<KIND, C, 1, kActive>(l) : launch_rowacc<KIND, C, 1, 0>(l))
+                 : (l.epilogue & kActive ? launch_rowacc<KIND, C, 2, kActive>(l) : launch_rowacc<KIND, C, 2, 0>(l));
   }
   switch (l.epilogue) {
-    case 0: return launch_rowacc<KIND, C, 0, 0>(l, b, c, p);
-    case kActive: return launch_rowacc<KIND, C, 0, kActive>(l, b, c, p);
+    case 0: return launch_rowacc<KIND, C, 0, 0>(l);
+    case kActive: return launch_rowacc<KIND, C, 0, kActive>(l);
     default: break;
   }
   if constexpr (C::COLS == kTile) {   // slim and mid
-    if (l.epilogue == kStaged) return launch_rowacc<KIND, C, 0, kStaged>(l, b, c, p);
-    if (l.epilogue == (kStaged | kActive)) return launch_rowacc<KIND, C, 0, kStaged | kActive>(l, b, c, p);
+    if (l.epilogue == kStaged) return launch_rowacc<KIND, C, 0, kStaged>(l);
+    if (l.epilogue == (kStaged | kActive)) return launch_rowacc<KIND, C, 0, kStaged | kActive>(l);
   }
   if constexpr (C::CTAS_PER_SM != Mid::CTAS_PER_SM) {
-    if (l.epilogue == (kSplit | kActive)) return launch_rowacc<KIND, C, 0, kSplit | kActive>(l, b, c, p);
+    if (l.epilogue == (kSplit | kActive)) return launch_rowacc<KIND, C, 0, kSplit | kActive>(l);
     if constexpr (KIND != VOID_KIND_F8E4M3 && C::COLS == kTile)
-      if (l.epilogue == (kStaged | kSplit | kActive)) return launch_rowacc<KIND, C, 0, kStaged | kSplit | kActive>(l, b, c, p);
+      if (l.epilogue == (kStaged | kSplit | kActive)) return launch_rowacc<KIND, C, 0, kStaged | kSplit | kActive>(l);
   }
   if constexpr (KIND == VOID_KIND_I8 && C::COLS == kTile) {
     constexpr int T = kTraced | kActive;
     switch (l.epilogue) {
-      case T: return launch_rowacc<KIND, C, 0, T>(l, b, c, p);
-      case T | kStaged: return launch_rowacc<KIND, C, 0, T | kStaged>(l, b, c, p);
-      case T | kSplit: return launch_rowacc<KIND, C, 0, T | kSplit>(l, b, c, p);
-      case T | kStaged | kSplit: return launch_rowacc<KIND, C, 0, T | kStaged | kSplit>(l, b, c, p);
+      case T: return launch_rowacc<KIND, C, 0, T>(l);
+      case T | kStaged: return launch_rowacc<KIND, C, 0, T | kStaged>(l);
+      case T | kSplit: return launch_rowacc<KIND, C, 0, T | kSplit>(l);
+      case T | kStaged | kSplit: return launch_rowacc<KIND, C, 0, T | kStaged | kSplit>(l);
     }
   }
   return VOID_ERR_BAD_ARG;
 }
 template <int KIND>
-int launch_rowacc(const RowaccLaunch& l, const CUtensorMap& b, const CUtensorMap& c, const SpmmParams& p) {
+int launch_rowacc(const RowaccLaunch& l) {
   if constexpr (KIND == VOID_KIND_F16 || KIND == VOID_KIND_TF32)
-    if (l.shape == 6) return launch_rowacc<KIND, Mid>(l, b, c, p);
-  return l.shape == 2 ? launch_rowacc<KIND, Slim>(l, b, c, p) : launch_rowacc<KIND, Wide>(l, b, c, p);
+    if (l.shape == 6) return launch_rowacc<KIND, Mid>(l);
+  return l.shape == 2 ? launch_rowacc<KIND, Slim>(l) : launch_rowacc<KIND, Wide>(l);
 }
 
 }  // namespace vb

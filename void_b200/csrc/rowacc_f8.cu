@@ -3,6 +3,6 @@
 
 namespace vb {
 
-template int launch_rowacc<VOID_KIND_F8E4M3>(const RowaccLaunch&, const CUtensorMap&, const CUtensorMap&, const SpmmParams&);
+template int launch_rowacc<VOID_KIND_F8E4M3>(const RowaccLaunch&);
 
 }  // namespace vb

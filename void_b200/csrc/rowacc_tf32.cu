@@ -3,6 +3,6 @@
 
 namespace vb {
 
-template int launch_rowacc<VOID_KIND_TF32>(const RowaccLaunch&, const CUtensorMap&, const CUtensorMap&, const SpmmParams&);
+template int launch_rowacc<VOID_KIND_TF32>(const RowaccLaunch&);
 
 }  // namespace vb

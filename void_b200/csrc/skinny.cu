@@ -285,17 +285,8 @@ cudaError_t launch(const SkinnyParams& p, int nbr, int warps, cudaStream_t st) {
   auto kernel = skinny_kernel<KIND, TR, NG, ACT>;
   const int smem = warps * 32 * (8 * NG + 1) * 4;
   if (smem > 48 * 1024 && ensure_smem((const void*)kernel, smem)) return cudaErrorInvalidValue;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)nbr, (unsigned)((p.N + 8 * NG - 1) / (8 * NG)));
-  cfg.blockDim = dim3((unsigned)(32 * warps));
-  cfg.dynamicSmemBytes = (size_t)smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, p);
+  launch_pdl(kernel, dim3((unsigned)nbr, (unsigned)((p.N + 8 * NG - 1) / (8 * NG))), 32 * warps, smem, st, p);
+  return cudaGetLastError();
 }
 template <int KIND, bool TR, int NG>
 cudaError_t launch(const SkinnyParams& p, int nbr, int warps, cudaStream_t st) {

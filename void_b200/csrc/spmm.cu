@@ -445,6 +445,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   p.n_peers = a->n_peers;
   p.peer_slots = a->peer_slots ? 1 : 0;
   if (a->n_peers < 0 || a->n_peers > 8) return VOID_ERR_BAD_ARG;
+  PeerParams peers;
   if (a->peer_slots != 0 && (a->n_peers == 0 || kind != VOID_KIND_I8)) return VOID_ERR_BAD_ARG;
   if (a->n_peers > 0) {
     // reduction across GPUs: a plan whose segments name the owner of their tile row; INT8 / floating row-accumulate
@@ -452,9 +453,9 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
     for (int r = 0; r < a->n_peers; ++r) {
       if (a->peer_partials[r] == nullptr) return VOID_ERR_BAD_ARG;
       if (!a->peer_slots && (a->peer_counters[r] == nullptr || a->peer_out[r] == nullptr)) return VOID_ERR_BAD_ARG;
-      p.peer_partials[r] = reinterpret_cast<int32_t*>(a->peer_partials[r]);
-      p.peer_counters[r] = a->peer_counters[r];
-      p.peer_out[r] = a->peer_out[r];
+      peers.partials[r] = reinterpret_cast<int32_t*>(a->peer_partials[r]);
+      peers.counters[r] = a->peer_counters[r];
+      peers.out[r] = a->peer_out[r];
     }
   }
   p.trace = reinterpret_cast<unsigned long long*>(a->trace);
@@ -530,7 +531,6 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   }
 
   CUtensorMap tmap_c;
-  memset(&tmap_c, 0, sizeof(tmap_c));
   if (staged && !store_map(&tmap_c, a->out, a->ldc, a->M, a->N)) return VOID_ERR_TENSOR_MAP;
 
 #define VB_LAUNCH(KERNEL, SHAPE)                                                               \
@@ -543,11 +543,11 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
     const bool split = a->segs != nullptr || a->acc_out != nullptr || a->worker_partials != nullptr;
     const bool active = split || traced || a->act != VOID_ACT_NONE || a->row_bias != nullptr;
     const int epilogue = (staged ? kStaged : 0) | (split ? kSplit : 0) | (active ? kActive : 0) | (traced ? kTraced : 0);
-    const RowaccLaunch l = {shape, a->transposed, epilogue, grid, smem_bytes, stream};
-    const int st = kind == VOID_KIND_I8       ? launch_rowacc<VOID_KIND_I8>(l, tmap, tmap_c, p)
-                   : kind == VOID_KIND_F8E4M3 ? launch_rowacc<VOID_KIND_F8E4M3>(l, tmap, tmap_c, p)
-                   : kind == VOID_KIND_TF32   ? launch_rowacc<VOID_KIND_TF32>(l, tmap, tmap_c, p)
-                                              : launch_rowacc<VOID_KIND_F16>(l, tmap, tmap_c, p);   // fp16 and bf16 differ in the descriptor only
+    const RowaccLaunch l = {shape, a->transposed, epilogue, grid, smem_bytes, stream, tmap, tmap_c, peers, p};
+    const int st = kind == VOID_KIND_I8       ? launch_rowacc<VOID_KIND_I8>(l)
+                   : kind == VOID_KIND_F8E4M3 ? launch_rowacc<VOID_KIND_F8E4M3>(l)
+                   : kind == VOID_KIND_TF32   ? launch_rowacc<VOID_KIND_TF32>(l)
+                                              : launch_rowacc<VOID_KIND_F16>(l);   // fp16 and bf16 differ in the descriptor only
     if (st != VOID_OK) return st;
   } else if (kind == VOID_KIND_I8) {
     if (np == 1 && shape == 2) VB_LAUNCH((spmm_drain_kernel<VOID_KIND_I8, 1, Slim>), Slim);
