@@ -82,6 +82,10 @@ VOID_API size_t void_tile_index_ws_bytes(int32_t nbr, int32_t nbc);
 VOID_API int void_build_tile_index(const int32_t* block_rows, const int32_t* block_cols, int64_t nnz,
                           int32_t nbr, int32_t nbc, int32_t* row_ptr, int32_t* block_indices,
                           void* ws, size_t ws_bytes, void_stream_t stream);
+/* The same with the tile rows by falling tile count (void_row_order), for small grids in one launch. */
+VOID_API int void_build_tile_index_order(const int32_t* block_rows, const int32_t* block_cols, int64_t nnz,
+                          int32_t nbr, int32_t nbc, int32_t* row_ptr, int32_t* block_indices,
+                          int32_t* row_order, void* ws, size_t ws_bytes, void_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------
  * Format construction on the device.  Replaces the host-side work of dense_to_void,

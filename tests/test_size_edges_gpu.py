@@ -81,7 +81,7 @@ def test_dense_to_void_widths_and_alignments(m, n, off, dtype, threshold):
     assert np.array_equal(v.values.float().cpu().numpy(), f["values"])
 
 
-@pytest.mark.parametrize("nbr,nbc", [(1, 1), (1, 70), (1023, 33), (1025, 2), (4096, 3), (4097, 3), (600, 2100)])
+@pytest.mark.parametrize("nbr,nbc", [(1, 1), (1, 70), (256, 40), (257, 40), (1023, 33), (1025, 2), (4096, 3), (4097, 3), (600, 2100)])
 def test_packed_store_of_grids_of_every_size(nbr, nbc):
     gen = torch.Generator().manual_seed(nbr + nbc)
     mask = (torch.rand(nbr, nbc, generator=gen) < min(0.4, 3000 / (nbr * nbc))).numpy()

@@ -61,6 +61,7 @@ _PROTOTYPES = {
     "void_device_sm_count": (ctypes.c_int, []),
     "void_launch_floor": (ctypes.c_int, [c_i32, c_i32, c_i32, c_vp]),
     "void_tile_index_ws_bytes": (c_sz, [c_i32, c_i32]),
+    "void_build_tile_index_order": (ctypes.c_int, [c_vp, c_vp, c_i64, c_i32, c_i32, c_vp, c_vp, c_vp, c_vp, c_sz, c_vp]),
     "void_build_tile_index": (ctypes.c_int, [c_vp, c_vp, c_i64, c_i32, c_i32, c_vp, c_vp, c_vp, c_sz, c_vp]),
     "void_format_ws_bytes": (c_sz, [c_i32, c_i32]),
     "void_dense_mark": (ctypes.c_int, [c_vp, c_i32, c_i64, c_i32, c_i32, c_f32, c_vp, c_sz, c_vp, c_vp]),

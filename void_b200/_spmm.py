@@ -75,10 +75,10 @@ def pack(values: torch.Tensor, scales: Optional[torch.Tensor], block_rows: torch
     if values.dim() != 3 or values.shape[1] != TILE or values.shape[2] != TILE or values.element_size() != es:
         raise _lib.VoidB200Error("void_b200 kernels need 32x32 tiles of %d-byte elements here, got %s %s"
                                  % (es, tuple(values.shape), values.dtype))
-    tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale, home = _lib.native().pack_store(
+    tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale, row_order, home = _lib.native().pack_store(
         values, scales, block_rows, block_cols, M, K, kind, terms, row_ptr, block_indices)
     return PackedTiles(tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale, (M + TILE - 1) // TILE,
-                       (K + TILE - 1) // TILE, values.shape[0], (M, K), kind, terms, home=home)
+                       (K + TILE - 1) // TILE, values.shape[0], (M, K), kind, terms, row_order=row_order, home=home)
 
 
 def pack_f8_split(values: torch.Tensor, scales: Optional[torch.Tensor], block_rows: torch.Tensor,
@@ -94,7 +94,7 @@ def _mark_ready(p: PackedTiles) -> PackedTiles:
     # there is not stable, is never read early, and serves the one product it was built for (it is not kept).
     # The CTAs that start first take the first work items: with the tile rows sorted by falling tile count the
     # longest rows start earliest and the shortest are left for the CTAs that share an SM with the most others.
-    p.row_order, indexed = _lib.native().finish_store(p.row_ptr, p.nbr)
+    p.row_order, indexed = _lib.native().finish_store(p.row_ptr, p.nbr, p.row_order)
     if indexed is not None:
         check_indexed(indexed, p.nnz)
         p.stable = True

@@ -38,7 +38,7 @@ def _structure(block_rows, block_cols, shape, n_blocks):
         tile_cols_t = block_rows.to(torch.int32)[block_indices_t.long()].contiguous()
         st = _lib.native().structure(row_ptr, block_indices, tile_cols, row_ptr_t, block_indices_t, tile_cols_t,
                                      tile_grad_items(row_ptr), _lib.status_word(block_rows.device), shape[0], shape[1], n_blocks,
-                                     _lib.native().finish_store(row_ptr, nbr)[0], _lib.native().finish_store(row_ptr_t, nbc)[0])
+                                     _lib.native().finish_store(row_ptr, nbr, None)[0], _lib.native().finish_store(row_ptr_t, nbc, None)[0])
         hit = (st, row_ptr, block_indices, block_rows, block_cols)     # keeps the keys alive
         if len(_STRUCTURE) >= _STRUCTURE_MAX:              # the oldest that no captured graph reads
             for old in list(_STRUCTURE):

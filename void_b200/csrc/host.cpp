@@ -916,17 +916,27 @@ void check_index(const at::Tensor& row_ptr, const at::Tensor& block_indices, int
                         row_ptr.is_contiguous() && block_indices.is_contiguous() && row_ptr.numel() == nbr + 1 && block_indices.numel() == tiles,
                     "invalid VOID tile index: it does not belong to ", tiles, " tiles in ", nbr, " tile rows");
 }
+constexpr int32_t kMaxOrderRows = 4096;   // tile rows that are put in order by comparing all pairs
+// order: null, or the tile rows by falling tile count (left undefined for more rows than that)
 void build_index(const at::Tensor& rows, const at::Tensor& cols, int32_t nbr, int32_t nbc, at::Tensor& row_ptr, at::Tensor& block_indices,
-                 void_stream_t st) {
+                 at::Tensor* order, void_stream_t st) {
   const c10::Device dev = rows.device();
   const int64_t count = rows.numel();
   row_ptr = new_cuda({nbr + 1}, at::kInt, dev);
   block_indices = new_cuda({count}, at::kInt, dev);
   const size_t ws_bytes = void_tile_index_ws_bytes(nbr, nbc);
   const at::Tensor ws = new_cuda({(int64_t)ws_bytes}, at::kByte, dev);
-  check(void_build_tile_index(rows.const_data_ptr<int32_t>(), cols.const_data_ptr<int32_t>(), count, nbr, nbc, row_ptr.data_ptr<int32_t>(),
-                              block_indices.data_ptr<int32_t>(), ws.data_ptr(), ws_bytes, st),
-        "void_build_tile_index");
+  const int32_t *r = rows.const_data_ptr<int32_t>(), *c = cols.const_data_ptr<int32_t>();
+  if (order != nullptr && nbr > 0 && nbr <= kMaxOrderRows) {
+    *order = new_cuda({nbr}, at::kInt, dev);
+    check(void_build_tile_index_order(r, c, count, nbr, nbc, row_ptr.data_ptr<int32_t>(), block_indices.data_ptr<int32_t>(),
+                                      order->data_ptr<int32_t>(), ws.data_ptr(), ws_bytes, st),
+          "void_build_tile_index_order");
+  } else {
+    check(void_build_tile_index(r, c, count, nbr, nbc, row_ptr.data_ptr<int32_t>(), block_indices.data_ptr<int32_t>(), ws.data_ptr(),
+                                ws_bytes, st),
+          "void_build_tile_index");
+  }
 }
 // Waits for the index and reads how many tiles it holds: one read of one integer per built index.
 long long indexed_tiles(const at::Tensor& row_ptr, int32_t nbr, void_stream_t st) {
@@ -948,15 +958,15 @@ PyObject* tile_index(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int32_t nbr = (int32_t)integer(a[2]), nbc = (int32_t)integer(a[3]);
   check_list(rows, cols, rows.numel());
   at::Tensor row_ptr, block_indices;
-  build_index(rows, cols, nbr, nbc, row_ptr, block_indices, st);
+  build_index(rows, cols, nbr, nbc, row_ptr, block_indices, nullptr, st);
   const long long indexed = indexed_tiles(row_ptr, nbr, st);
   return Py_BuildValue("NNL", THPVariable_Wrap(row_ptr), THPVariable_Wrap(block_indices), indexed);
   NATIVE_END
 }
 
 // pack_store(values, scales | None, block_rows, block_cols, M, K, kind, terms, row_ptr | None, block_indices | None)
-//   -> (tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale, home): home is the stream all of them were allocated
-//   on, None with an index that was given
+//   -> (tiles, tile_cols, tile_scales, row_ptr, block_indices, row_scale, row_order, home): row_order where it came with the
+//   index, else None; home is the stream all of them were allocated on, None with an index that was given
 // The packed store of a tensor, its tile index built on the way when it is not given.  The caller waits for it
 // and checks the index (finish_store); until then a list that is not valid is packed without leaving its arrays.
 PyObject* pack_store(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -971,9 +981,9 @@ PyObject* pack_store(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int kind = (int)integer(a[6]), terms = (int)integer(a[7]), es = elem_bytes(kind);
   const int32_t nbr = (int32_t)((M + 31) / 32), nbc = (int32_t)((K + 31) / 32);
   check_list(rows, cols, count);
-  at::Tensor row_ptr, block_indices, scales;
+  at::Tensor row_ptr, block_indices, order, scales;
   if (none(a[8]) || none(a[9])) {
-    build_index(rows, cols, nbr, nbc, row_ptr, block_indices, st);
+    build_index(rows, cols, nbr, nbc, row_ptr, block_indices, &order, st);
   } else {
     row_ptr = tensor(a[8], "row_ptr");
     block_indices = tensor(a[9], "block_indices");
@@ -1002,23 +1012,29 @@ PyObject* pack_store(PyObject*, PyObject* const* a, Py_ssize_t n) {
   PyObject* home = Py_None;
   if (none(a[8]) || none(a[9])) home = PyLong_FromLongLong((long long)reinterpret_cast<intptr_t>(st));
   else Py_INCREF(home);
-  return Py_BuildValue("NNNNNNN", THPVariable_Wrap(tiles), THPVariable_Wrap(tile_cols), THPVariable_Wrap(tile_scales), THPVariable_Wrap(row_ptr),
-                       THPVariable_Wrap(block_indices), THPVariable_Wrap(row_scale), home);
+  PyObject* by_length = Py_None;
+  if (order.defined()) by_length = THPVariable_Wrap(order);
+  else Py_INCREF(by_length);
+  return Py_BuildValue("NNNNNNNN", THPVariable_Wrap(tiles), THPVariable_Wrap(tile_cols), THPVariable_Wrap(tile_scales), THPVariable_Wrap(row_ptr),
+                       THPVariable_Wrap(block_indices), THPVariable_Wrap(row_scale), by_length, home);
   NATIVE_END
 }
 
-// finish_store(row_ptr, nbr) -> (row_order, indexed tiles | None): the order of the tile rows, then - outside a stream
-// capture, where nothing can be waited for - the wait until the store is complete and the size of its index
+// finish_store(row_ptr, nbr, row_order | None) -> (row_order, indexed tiles | None): the order of the tile rows, unless there is
+// one, then - outside a stream capture, where nothing can be waited for - the wait until the store is complete and the size of
+// its index
 PyObject* finish_store(PyObject*, PyObject* const* a, Py_ssize_t n) {
   NATIVE_BEGIN
-  if (n != 2) throw torch::TypeError("finish_store takes 2 arguments");
+  if (n != 3) throw torch::TypeError("finish_store takes 3 arguments");
   const at::Tensor& row_ptr = cuda_tensor(a[0], "row_ptr");
   const int32_t nbr = (int32_t)integer(a[1]);
   const c10::Device dev = row_ptr.device();
   c10::cuda::OptionalCUDAGuard guard(dev);
   const void_stream_t st = stream_of(dev.index());
   at::Tensor order;
-  if (nbr > 0 && nbr <= 4096) {
+  if (!none(a[2])) {
+    order = cuda_tensor(a[2], "row_order");
+  } else if (nbr > 0 && nbr <= kMaxOrderRows) {
     order = new_cuda({nbr}, at::kInt, dev);
     check(void_row_order(row_ptr.const_data_ptr<int32_t>(), nbr, order.data_ptr<int32_t>(), st), "void_row_order");
   } else if (nbr > 0) {   // beyond a few thousand rows a sort does less work than comparing all pairs

@@ -109,9 +109,10 @@ __global__ void rank_tiles_kernel(const int32_t* __restrict__ brow, const int32_
 // three passes over the list: 4096^2, 80 % (3277 tiles) 5.6 us, against 8.6 for a memset and three launches and the gaps
 // between them.
 constexpr int kOneBlockTiles = 16384, kOneBlockWords = 12000;   // words: those of the bitmap and one per tile row (48 KB)
+constexpr int kOneBlockOrder = 256;   // tile rows one block puts in order by comparing all pairs (0.3 us of 128 rows, 1.3 of 256)
 __global__ void __launch_bounds__(1024) tile_index_kernel(const int32_t* __restrict__ brow, const int32_t* __restrict__ bcol, int nnz,
                                                           int nbr, int nbc, int wpr, int32_t* __restrict__ row_ptr,
-                                                          int32_t* __restrict__ block_indices) {
+                                                          int32_t* __restrict__ block_indices, int32_t* __restrict__ row_order) {
   extern __shared__ uint32_t bits[];   // [nbr][wpr], then the rows' first tiles
   __shared__ int32_t warp_sum[32];
   int32_t* first = reinterpret_cast<int32_t*>(bits + nbr * wpr);
@@ -155,7 +156,19 @@ __global__ void __launch_bounds__(1024) tile_index_kernel(const int32_t* __restr
     row_ptr[r] = first[r];
   }
   if (tid == 1023) row_ptr[nbr] = before + sum;
+  if (tid == 1023) first[nbr] = before + sum;
   __syncthreads();
+  if (row_order != nullptr)   // as row_order_kernel
+    for (int r = wid; r < nbr; r += 32) {
+      const int mine = first[r + 1] - first[r];
+      int ahead = 0;
+      for (int i = lane; i < nbr; i += 32) {
+        const int c = first[i + 1] - first[i];
+        ahead += (c > mine || (c == mine && i < r)) ? 1 : 0;
+      }
+      ahead = __reduce_add_sync(0xffffffffu, ahead);
+      if (lane == 0) row_order[ahead] = r;
+    }
 #pragma unroll 4
   for (int i = tid; i < nnz; i += 1024) {
     const int r = brow[i], c = bcol[i];
@@ -684,14 +697,16 @@ __global__ void __launch_bounds__(kFusedThreads) quant_cols_fused_kernel(const f
       if (scale_inv_out != nullptr) scale_inv_out[n0 + tid] = inv;
     }
   }
-  cluster.sync();   // the scales for this CTA; and no CTA leaves while another still reads its maxima
+  // No CTA leaves while another still reads its maxima, so the second meeting of the cluster is waited for at the end.
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  __syncthreads();   // the scales for this CTA
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // late, see copy_rows_kernel
-  if (n >= ldq) return;
+  const int mine = n < ldq ? rows : 0;
   uint8_t* dst = q + (size_t)k0 * ldq + n;
   if constexpr (VEC) {
     const float4 sc = *reinterpret_cast<const float4*>(s_scale + col), si = *reinterpret_cast<const float4*>(s_inv + col);
 #pragma unroll 4
-    for (int r = r0; r < rows; r += ROWS) {
+    for (int r = r0; r < mine; r += ROWS) {
       const float4 x = *reinterpret_cast<const float4*>(slab + r * W + col);
       *reinterpret_cast<uint32_t*>(dst + (size_t)r * ldq) = KIND == VOID_KIND_I8 ? quant_i8x4(x, sc, si) : quant_e4m3x4(x, si);
     }
@@ -699,17 +714,18 @@ __global__ void __launch_bounds__(kFusedThreads) quant_cols_fused_kernel(const f
     const float sc = s_scale[col], si = s_inv[col];
     const float4 sc4 = make_float4(sc, sc, sc, sc), si4 = make_float4(si, si, si, si);
     int r = r0;
-    for (; r + 3 * ROWS < rows; r += 4 * ROWS) {   // (four rows at once: the form that divides only where rounding hangs on it)
+    for (; r + 3 * ROWS < mine; r += 4 * ROWS) {   // (four rows at once: the form that divides only where rounding hangs on it)
       const float4 x = make_float4(slab[r * W + col], slab[(r + ROWS) * W + col], slab[(r + 2 * ROWS) * W + col], slab[(r + 3 * ROWS) * W + col]);
       const uint32_t o = KIND == VOID_KIND_I8 ? quant_i8x4(x, sc4, si4) : quant_e4m3x4(x, si4);
 #pragma unroll
       for (int k = 0; k < 4; ++k) dst[(size_t)(r + k * ROWS) * ldq] = (uint8_t)(o >> (8 * k));
     }
-    for (; r < rows; r += ROWS) {
+    for (; r < mine; r += ROWS) {
       const float x = slab[r * W + col];
       dst[(size_t)r * ldq] = KIND == VOID_KIND_I8 ? (uint8_t)quant_i8(x, sc) : quant_e4m3(x, si);
     }
   }
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 
 // absmax of a whole row-major [K, N] matrix into amax[0] (zero before the launch)
@@ -1041,9 +1057,10 @@ size_t void_tile_index_ws_bytes(int32_t nbr, int32_t nbc) {
   return (size_t)nbr * wpr * 4 + (size_t)nbr * 4 + 16;
 }
 
-int void_build_tile_index(const int32_t* block_rows, const int32_t* block_cols, int64_t nnz, int32_t nbr,
-                          int32_t nbc, int32_t* row_ptr, int32_t* block_indices, void* ws, size_t ws_bytes,
-                          void_stream_t stream) {
+// row_order: null, or written as void_row_order writes it where that costs no launch (*ordered is set then)
+static int build_tile_index(const int32_t* block_rows, const int32_t* block_cols, int64_t nnz, int32_t nbr, int32_t nbc,
+                            int32_t* row_ptr, int32_t* block_indices, int32_t* row_order, bool* ordered, void* ws, size_t ws_bytes,
+                            void_stream_t stream) {
   if (nnz < 0 || nbr < 0 || nbc < 0 || row_ptr == nullptr) return VOID_ERR_BAD_ARG;
   cudaStream_t st = as_stream(stream);
   if (nbr == 0) return cudaMemsetAsync(row_ptr, 0, 4, st) == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
@@ -1052,7 +1069,9 @@ int void_build_tile_index(const int32_t* block_rows, const int32_t* block_cols, 
   if (ws == nullptr || ws_bytes < void_tile_index_ws_bytes(nbr, nbc)) return VOID_ERR_WORKSPACE;
   const int wpr = (nbc + 31) / 32;
   if (nnz <= kOneBlockTiles && (int64_t)nbr * (wpr + 1) <= kOneBlockWords) {
-    launch_pdl(tile_index_kernel, 1, 1024, nbr * (wpr + 1) * 4, st, block_rows, block_cols, (int)nnz, nbr, nbc, wpr, row_ptr, block_indices);
+    *ordered = row_order != nullptr && nbr <= kOneBlockOrder;
+    launch_pdl(tile_index_kernel, 1, 1024, (nbr * (wpr + 1) + 1) * 4, st, block_rows, block_cols, (int)nnz, nbr, nbc, wpr, row_ptr, block_indices,
+               *ordered ? row_order : nullptr);
     return last_status();
   }
   uint32_t* bitmap = reinterpret_cast<uint32_t*>(ws);
@@ -1072,6 +1091,22 @@ int void_build_tile_index(const int32_t* block_rows, const int32_t* block_cols, 
     rank_tiles_kernel<<<(unsigned)((nnz + tb - 1) / tb), tb, 0, st>>>(block_rows, block_cols, nnz, nbr, nbc, wpr, bitmap,
                                                                      row_ptr, block_indices);
   return last_status();
+}
+
+int void_build_tile_index(const int32_t* block_rows, const int32_t* block_cols, int64_t nnz, int32_t nbr,
+                          int32_t nbc, int32_t* row_ptr, int32_t* block_indices, void* ws, size_t ws_bytes,
+                          void_stream_t stream) {
+  bool ordered = false;
+  return build_tile_index(block_rows, block_cols, nnz, nbr, nbc, row_ptr, block_indices, nullptr, &ordered, ws, ws_bytes, stream);
+}
+
+int void_build_tile_index_order(const int32_t* block_rows, const int32_t* block_cols, int64_t nnz, int32_t nbr, int32_t nbc,
+                                int32_t* row_ptr, int32_t* block_indices, int32_t* row_order, void* ws, size_t ws_bytes,
+                                void_stream_t stream) {
+  if (nbr > 0 && row_order == nullptr) return VOID_ERR_BAD_ARG;
+  bool ordered = false;
+  const int st = build_tile_index(block_rows, block_cols, nnz, nbr, nbc, row_ptr, block_indices, row_order, &ordered, ws, ws_bytes, stream);
+  return st != VOID_OK || ordered ? st : void_row_order(row_ptr, nbr, row_order, stream);
 }
 
 int void_row_order(const int32_t* row_ptr, int32_t nbr, int32_t* order, void_stream_t stream) {
