@@ -625,7 +625,7 @@ template <int KIND, bool VEC>
 __global__ void __launch_bounds__(kFusedThreads) quant_cols_fused_kernel(const float* __restrict__ b, int64_t ldb, int K, int N,
                                                                          uint8_t* __restrict__ q, int64_t ldq,
                                                                          float* __restrict__ scale_out,
-                                                                         float* __restrict__ scale_inv_out) {
+                                                                         float* __restrict__ scale_inv_out, int early) {
   namespace cg = cooperative_groups;
   constexpr int W = kFusedCols;
   constexpr int E = VEC ? 4 : 1;                        // columns a thread owns
@@ -655,6 +655,7 @@ __global__ void __launch_bounds__(kFusedThreads) quant_cols_fused_kernel(const f
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src + (size_t)r * ldb), "r"(bytes) : "memory");
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
+  if (early) grid_launch_dependents();
   float m[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) m[e] = 0.0f;
@@ -700,7 +701,7 @@ __global__ void __launch_bounds__(kFusedThreads) quant_cols_fused_kernel(const f
   // No CTA leaves while another still reads its maxima, so the second meeting of the cluster is waited for at the end.
   asm volatile("barrier.cluster.arrive.release;" ::: "memory");
   __syncthreads();   // the scales for this CTA
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // late, see copy_rows_kernel
+  if (!early) grid_launch_dependents();
   const int mine = n < ldq ? rows : 0;
   uint8_t* dst = q + (size_t)k0 * ldq + n;
   if constexpr (VEC) {
@@ -831,13 +832,16 @@ static bool launch_column_sum(const void* in, int64_t ld, int rows, int cols, vo
 // padding is written as zeros.
 // The product that follows may start only when every block is about to write its result.  Started with the first loads, a
 // persistent product settles on the SMs unevenly beside the blocks still running and stays so: INT8 columns quantised and
-// multiplied, 16384 x 4096, N = 2048: 75.7 us, started late 59.7 (15.3 + 42.6 alone); 4096 x 4096, N = 512 13.7 -> 13.6.
+// multiplied, 16384 x 4096, N = 2048: 75.7 us, started late 59.7 (15.3 + 42.6 alone).  Where all blocks run at once there is nothing
+// to settle beside, and it may start with them: bf16 GELU 3001 x 5003, N = 333 (821 blocks) 11.7 -> 10.5 us, 4096 x 1111, N = 777
+// 12.9 -> 11.5; started early behind 4032 blocks 47.1 -> 47.4 (fp16 8192^2, 90 %, N = 1001).
 template <typename T>
 __global__ void __launch_bounds__(256) copy_rows_kernel(const T* __restrict__ in, int64_t ld_in, uint4* __restrict__ out,
-                                                        int64_t pieces, int64_t rows, int cols) {
+                                                        int64_t pieces, int64_t rows, int cols, int early) {
   constexpr int E = 16 / (int)sizeof(T);
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (early) grid_launch_dependents();
   if (i >= rows * pieces) return;
   const int64_t r = i / pieces;
   const int c0 = (int)(i - r * pieces) * E;
@@ -845,7 +849,7 @@ __global__ void __launch_bounds__(256) copy_rows_kernel(const T* __restrict__ in
   union { uint4 v; T e[E]; } o;
 #pragma unroll
   for (int k = 0; k < E; ++k) o.e[k] = c0 + k < cols ? src[k] : T(0);
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (!early) grid_launch_dependents();
   out[i] = o.v;
 }
 
@@ -991,8 +995,15 @@ static bool launch_quant_cols_fused(const float* b, int64_t ldb, int K, int N, v
   // 4096^2 384 13.7 / 12.4, but 512 15.3 / 16.3.  Where the last cluster has just room, N = 528: INT8 16.0 / 15.0, FP8 2048 x 4096
   // 13.0 / 15.7; where it waits for the first to end, N = 560: 16.8 / 19.3 and 13.2 / 16.3.  From 48 KB a CTA on there is nothing to
   // gain (8192^2: 38.8 / 39.4).
+  // The kernel behind it may start with the first maxima where all clusters run at once, two CTAs per SM at most: its own CTAs
+  // then only wait for the places.  With more, they would take the places of clusters still to come and settle unevenly (INT8
+  // 16384 x 4096, N = 2048 55 us late, 62 early).  us with their products, late and early: FP8 4096^2, 80 %, N = 512 16.9 16.0,
+  // 4096 x 2048, N = 128 10.7 8.96, INT8 4096^2, 90 %, N = 512 10.7 10.5, 512^2, N = 128 6.59 6.49; slabs of 64 KB (8192^2, N = 512) 21.8
+  // 21.9, as they were.
+  int early = 0;
   if (smem <= 48 * 1024) {
     const ClusterRoom room = cluster_room<KIND, VEC>();
+    early = (int)clusters <= room.two_per_sm ? 1 : 0;
     if ((int)clusters > room.one_per_sm && (int)clusters < room.two_per_sm) smem = kFusedMaxSmem / 2;
   }
   cudaLaunchConfig_t cfg = {};
@@ -1008,7 +1019,7 @@ static bool launch_quant_cols_fused(const float* b, int64_t ldb, int K, int N, v
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, kernel, b, ldb, K, N, reinterpret_cast<uint8_t*>(q), ldq, scale, scale_inv) == cudaSuccess;
+  return cudaLaunchKernelEx(&cfg, kernel, b, ldb, K, N, reinterpret_cast<uint8_t*>(q), ldq, scale, scale_inv, early) == cudaSuccess;
 }
 // The one-launch form; false: not taken.  It is the faster one while three of its CTAs fit an SM (64 KB of rows each, K up
 // to 8192), and beyond that only where one CTA per SM holds everything at once (16384 x 256: 13.8 us against 15.7, but
@@ -1255,9 +1266,10 @@ int void_copy_rows(const void* in, int64_t ld_in, void* out, int64_t ld_out, int
   cfg.numAttrs = 1;
   uint4* dst = reinterpret_cast<uint4*>(out);
   cudaError_t rc;
-  if (elem_bytes == 1) rc = cudaLaunchKernelEx(&cfg, copy_rows_kernel<uint8_t>, reinterpret_cast<const uint8_t*>(in), ld_in, dst, pieces, rows, cols);
-  else if (elem_bytes == 2) rc = cudaLaunchKernelEx(&cfg, copy_rows_kernel<uint16_t>, reinterpret_cast<const uint16_t*>(in), ld_in / 2, dst, pieces, rows, cols);
-  else rc = cudaLaunchKernelEx(&cfg, copy_rows_kernel<uint32_t>, reinterpret_cast<const uint32_t*>(in), ld_in / 4, dst, pieces, rows, cols);
+  const int early = blocks <= 8ll * device_info().sms ? 1 : 0;   // 2048 threads per SM
+  if (elem_bytes == 1) rc = cudaLaunchKernelEx(&cfg, copy_rows_kernel<uint8_t>, reinterpret_cast<const uint8_t*>(in), ld_in, dst, pieces, rows, cols, early);
+  else if (elem_bytes == 2) rc = cudaLaunchKernelEx(&cfg, copy_rows_kernel<uint16_t>, reinterpret_cast<const uint16_t*>(in), ld_in / 2, dst, pieces, rows, cols, early);
+  else rc = cudaLaunchKernelEx(&cfg, copy_rows_kernel<uint32_t>, reinterpret_cast<const uint32_t*>(in), ld_in / 4, dst, pieces, rows, cols, early);
   return rc == cudaSuccess ? last_status() : VOID_ERR_CUDA;
 }
 
