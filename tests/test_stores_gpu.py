@@ -139,6 +139,27 @@ def test_a_tensor_first_used_inside_a_capture(kind):
     void.check_device_status()
 
 
+@pytest.mark.parametrize("n", [8, 40, 300])
+@pytest.mark.parametrize("kind", ["int8", "fp8_exact"])
+def test_first_replays_of_products_packed_inside_a_capture(kind, n):
+    """Only the first replay finds arrays that nothing has written: new graphs, their first replay right behind a product."""
+    w = _case(8, n=n)
+    make, quantise = (void.quantize_void_tensor, void.quantize_cols_int8) if kind == "int8" else (void.void_tensor_to_fp8, void.quantize_cols_fp8)
+    bq, bs = quantise(w.b)[:2]
+    product = (lambda t: void.void_spmm_int8(t, bq, bs)) if kind == "int8" else (lambda t: void.void_spmm_fp8(t, bq, b_scale=bs, scale_terms=0))
+    want, keep = product(make(w.a)), []
+    for _ in range(12):
+        t, g = make(w.a), torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g):
+            out = product(t)
+        product(make(w.a))
+        g.replay()
+        keep.append((g, t, out))
+    assert all(torch.equal(out, want) for _, _, out in keep)
+    void.check_device_status()
+
+
 @pytest.mark.parametrize("how", ["deepcopy", "copy", "file"])
 @pytest.mark.parametrize("kind", ["fp32", "int8", "fp8", "fp8_floating", "streamk", "module", "layer"])
 def test_tensors_that_were_multiplied_can_be_copied_and_saved(kind, how, tmp_path):

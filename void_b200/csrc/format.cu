@@ -146,7 +146,6 @@ __global__ void __launch_bounds__(256) dense_mark_kernel(const T* __restrict__ a
     atomicOr(bitmap + (code >> 5), 1u << (code & 31));
   }
   if (lane == 0 && nz) atomicAdd(&block_nz, nz);
-  vb::grid_launch_dependents();   // the ranking waits on an SM until all blocks are through
   __syncthreads();
   if (threadIdx.x == 0 && block_nz) atomicAdd(counts + 1, (unsigned long long)block_nz);
 }
@@ -169,10 +168,10 @@ __global__ void csr_mark_kernel(const int32_t* __restrict__ crow, const int32_t*
 
 // Rank of the first set bit of every word and the counts, by one block: the three levels below in one launch for the
 // grids that most matrices have.
-__global__ void __launch_bounds__(1024) rank_bitmap_kernel(const uint32_t* __restrict__ bitmap, int words,
-                                                           int32_t* __restrict__ word_prefix,
-                                                           const unsigned long long* __restrict__ counts,
-                                                           int64_t* __restrict__ counts_out) {
+__global__ void __launch_bounds__(1024) rank_bitmap_kernel(const uint32_t* bitmap, int words,
+                                                           int32_t* word_prefix,
+                                                           const unsigned long long* counts,
+                                                           int64_t* counts_out) {
   __shared__ int32_t warp_sum[32];
   vb::grid_dependency_wait();
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;

@@ -110,15 +110,14 @@ __global__ void rank_tiles_kernel(const int32_t* __restrict__ brow, const int32_
 // between them.
 constexpr int kOneBlockTiles = 16384, kOneBlockWords = 12000;   // words: those of the bitmap and one per tile row (48 KB)
 constexpr int kOneBlockOrder = 256;   // tile rows one block puts in order by comparing all pairs (0.3 us of 128 rows, 1.3 of 256)
-__global__ void __launch_bounds__(1024) tile_index_kernel(const int32_t* __restrict__ brow, const int32_t* __restrict__ bcol, int nnz,
-                                                          int nbr, int nbc, int wpr, int32_t* __restrict__ row_ptr,
-                                                          int32_t* __restrict__ block_indices, int32_t* __restrict__ row_order) {
+__global__ void __launch_bounds__(1024) tile_index_kernel(const int32_t* brow, const int32_t* bcol, int nnz,
+                                                          int nbr, int nbc, int wpr, int32_t* row_ptr,
+                                                          int32_t* block_indices, int32_t* row_order) {
   extern __shared__ uint32_t bits[];   // [nbr][wpr], then the rows' first tiles
   __shared__ int32_t warp_sum[32];
   int32_t* first = reinterpret_cast<int32_t*>(bits + nbr * wpr);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   for (int i = tid; i < nbr * wpr; i += 1024) bits[i] = 0u;
-  grid_launch_dependents();
   grid_dependency_wait();
   __syncthreads();
 #pragma unroll 4
@@ -206,7 +205,7 @@ struct RowScales {
   int nbr;
   unsigned pack_blocks;
 };
-__device__ __forceinline__ void mean_scale(const RowScales& rows, const TileMeta& meta, const int32_t* __restrict__ block_indices) {
+__device__ __forceinline__ void mean_scale(const RowScales& rows, const TileMeta& meta, const int32_t* block_indices) {
   const int r = (int)(((blockIdx.x - rows.pack_blocks) * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (r >= rows.nbr) return;
   const int t0 = rows.row_ptr[r], t1 = rows.row_ptr[r + 1];
@@ -218,9 +217,11 @@ __device__ __forceinline__ void mean_scale(const RowScales& rows, const TileMeta
   }
   if (lane == 0) rows.row_scale[r] = t1 > t0 ? __fdiv_rn(s, (float)(t1 - t0)) : 0.0f;
 }
-__global__ void __launch_bounds__(256) pack_tiles_kernel(const uint4* __restrict__ values, const int32_t* __restrict__ block_indices,
-                                                         int64_t nnz, uint4* __restrict__ packed, TileMeta meta, RowScales rows) {
-  grid_launch_dependents();
+// The kernels of a store's set-up (quantised tiles, index, packing, row order) start when the one before is complete and let the
+// next start when they are: a product packed inside a stream capture follows them without a host's wait in between, and with each
+// let in before the one ahead was through, a first replay was seen to multiply with arrays that had not been written yet.
+__global__ void __launch_bounds__(256) pack_tiles_kernel(const uint4* values, const int32_t* block_indices, int64_t nnz, uint4* packed,
+                                                         TileMeta meta, RowScales rows) {
   grid_dependency_wait();
   if (blockIdx.x >= rows.pack_blocks) {
     mean_scale(rows, meta, block_indices);
@@ -404,9 +405,8 @@ __global__ void gather_tile_meta_kernel(const int32_t* __restrict__ bcol, const 
 
 // Tile rows by falling tile count, ties in their own order: a row's place is the number of rows that come before it.  One
 // warp per row counts them, which for the few thousand rows of a matrix takes less than a sort's launches.
-__global__ void row_order_kernel(const int32_t* __restrict__ row_ptr, int nbr, int32_t* __restrict__ order) {
+__global__ void row_order_kernel(const int32_t* row_ptr, int nbr, int32_t* order) {
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  grid_launch_dependents();
   grid_dependency_wait();
   if (r >= nbr) return;
   const int mine = row_ptr[r + 1] - row_ptr[r];
@@ -493,12 +493,11 @@ __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
 }
 // One warp per tile: 1024 values, 32 per lane, read once and in their own type.
 template <int KIND, typename T>
-__global__ void __launch_bounds__(256) quant_tiles_kernel(const T* __restrict__ values, int64_t nnz, uint8_t* __restrict__ q,
+__global__ void __launch_bounds__(256) quant_tiles_kernel(const T* values, int64_t nnz, uint8_t* __restrict__ q,
                                                           float* __restrict__ scale_out, float* __restrict__ scale_inv_out,
                                                           float* __restrict__ amax_out, StoreExtras x) {
   const int64_t tile = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  grid_launch_dependents();
   grid_dependency_wait();
   if (tile >= nnz) return;
   const T* src = values + tile * 1024;
