@@ -76,7 +76,7 @@ template <typename T>
 struct same_type { using type = T; };
 // A launch that may start beside the end of the kernel before it.
 template <typename... P>
-void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem_bytes, cudaStream_t stream, const typename same_type<P>::type&... args) {
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem_bytes, cudaStream_t stream, const typename same_type<P>::type&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)threads);
@@ -87,7 +87,7 @@ void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem_bytes, cu
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, args...);
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 // B as a tensor for the copy engine, 128-byte swizzle, zero fill outside [K, N].  Elements of es bytes: every box is 128

@@ -285,8 +285,7 @@ cudaError_t launch(const SkinnyParams& p, int nbr, int warps, cudaStream_t st) {
   auto kernel = skinny_kernel<KIND, TR, NG, ACT>;
   const int smem = warps * 32 * (8 * NG + 1) * 4;
   if (smem > 48 * 1024 && ensure_smem((const void*)kernel, smem)) return cudaErrorInvalidValue;
-  launch_pdl(kernel, dim3((unsigned)nbr, (unsigned)((p.N + 8 * NG - 1) / (8 * NG))), 32 * warps, smem, st, p);
-  return cudaGetLastError();
+  return launch_pdl(kernel, dim3((unsigned)nbr, (unsigned)((p.N + 8 * NG - 1) / (8 * NG))), 32 * warps, smem, st, p);
 }
 template <int KIND, bool TR, int NG>
 cudaError_t launch(const SkinnyParams& p, int nbr, int warps, cudaStream_t st) {
