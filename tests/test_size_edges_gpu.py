@@ -411,3 +411,46 @@ def test_large_floating_products_are_exact_on_small_integers(dtype, m, k, n, den
         y = void.void_linear(a, b) if linear else void.void_spmm(a, b)
         assert torch.equal(y.double(), ref.to(dtype).double())
     void.check_device_status()
+
+
+# ------------------------------------------------------------------------------------------ products behind what prepares B
+@pytest.mark.parametrize("dtype,k,n", [
+    (torch.bfloat16, 6880, 333), (torch.bfloat16, 6912, 333), (torch.float32, 64, 33),     # row copies: 1183, 1188 and 3 blocks
+    ("int8", 512, 16), ("int8", 4096, 528), ("int8", 4096, 544), ("fp8", 2080, 528), ("fp8", 2080, 529)])   # 1, 33 and 34 clusters
+def test_products_wait_for_the_kernel_that_prepares_their_operand(dtype, k, n):
+    """The product's launch starts beside a kernel that copies or quantises B.  New values in the same buffers every time, so
+    that a product which read too early would use those of the time before."""
+    gen = torch.Generator(device="cuda").manual_seed(k + n)
+    nbc = (k + 31) // 32
+    mask = torch.rand(5, nbc, generator=gen, device="cuda") < 0.3
+    mask[:, nbc - 1] = True
+    values = torch.randint(-2, 3, (int(mask.sum()), 32, 32), generator=gen, device="cuda").float()
+    a = void.void_from_block_mask(mask.cpu().numpy(), values, shape=(160, nbc * 32))
+    q = {"int8": void.quantize_void_tensor, "fp8": void.void_tensor_to_fp8}.get(dtype, lambda t: t.to_dtype(dtype))(a)
+    quantise = {"int8": void.quantize_cols_int8, "fp8": void.quantize_cols_fp8}.get(dtype)
+
+    def product(b):
+        if quantise is None:
+            return void.void_spmm(q, b)
+        c, scale = quantise(b)[:2]
+        if dtype == "int8":
+            return void.void_spmm_int8(q, c, scale, out_dtype=torch.float32)
+        return void.void_spmm_fp8(q, c, torch.float32, b_scale=scale)
+
+    inputs = [torch.randint(-4, 5, (nbc * 32, n), generator=gen, device="cuda").float() * 2.0 ** i for i in range(6)]
+    if quantise is None:
+        inputs = [b.to(dtype) for b in inputs]
+    for b in inputs:
+        product(b)                      # plans and stores are built
+    torch.cuda.synchronize()
+    for b, c in zip(inputs, [product(b) for b in inputs]):
+        if quantise is None:
+            ref = a.to_dense().double() @ b.double()
+            assert torch.equal(c.double(), ref.to(dtype).double())
+        else:
+            x, scale = quantise(b)[:2]
+            torch.cuda.synchronize()
+            alone = (void.void_spmm_int8(q, x, scale, out_dtype=torch.float32) if dtype == "int8"
+                     else void.void_spmm_fp8(q, x, torch.float32, b_scale=scale))
+            assert torch.equal(c, alone)
+    void.check_device_status()
