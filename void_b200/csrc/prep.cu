@@ -105,34 +105,45 @@ __global__ void rank_tiles_kernel(const int32_t* __restrict__ brow, const int32_
   block_indices[row_ptr[r] + rank] = (int32_t)i;
 }
 
-// All of the above by one block, bitmap and row counts in shared memory, for the lists that most matrices have.  A chain of
-// three passes over the list: 4096^2, 80 % (3277 tiles) 5.6 us, against 8.6 for a memset and three launches and the gaps
-// between them.
-constexpr int kOneBlockTiles = 16384, kOneBlockWords = 12000;   // words: those of the bitmap and one per tile row (48 KB)
-constexpr int kOneBlockOrder = 256;   // tile rows one block puts in order by comparing all pairs (0.3 us of 128 rows, 1.3 of 256)
+// All of the above by one block, the bitmap in shared memory beside the number of tiles ahead of each of its words (16 bits), for
+// the lists that most matrices have.  A tile's place is one word's sum and one word's bits, however wide the grid; rows lie an odd
+// number of words apart, so that neighbouring ones start on different banks.  (Adding up a row's words for every tile took 58 us for
+// 8000 tiles of a 363 x 1024 grid, now 8.1, and 353 for 16384 of 93 x 4096.)
+// Bound by one SM's two passes over the list, about 0.4 us per thousand tiles, so longer lists go to the kernels above, which
+// spread over the device.  us for the index, this kernel and those: 128 x 128 grid, 3277 tiles 4.2 10.4, 8000 5.2 10.5; 256 x 256,
+// 8192 6.1 7.8, 16384 9.4 8.0; 512 x 512, 8192 7.3 10.3, 16384 11.5 10.3; 1000 x 333, 8192 7.7 8.8, 16384 11.8 9.1; 363 x 1024,
+// 8192 8.1 16.0; 960 x 512, 8192 8.5 12.3.  Where the bitmap is small those are slow with 16384 as well: 128 x 128 8.4 11.2, 64 x 512
+// 8.6 12.4, but 160 x 256 (1440 words) 9.1 8.4.
+constexpr int kOneBlockTiles = 8192, kOneBlockWords = 16384;                // words: those of the bitmap, rows padded
+constexpr int kOneBlockManyTiles = 16384, kOneBlockFewWords = 1100;
+constexpr int kOneBlockOrder = 256;   // tile rows one block puts in order, a quarter of its threads: 128 rows 0.9 us, 256 1.3
+static bool one_block_index(int64_t nnz, int64_t words) {
+  return words <= kOneBlockWords && nnz <= (words <= kOneBlockFewWords ? kOneBlockManyTiles : kOneBlockTiles);
+}
+constexpr int one_block_pitch(int wpr) { return wpr | 1; }
+constexpr int one_block_smem(int words) { return words * 4 + (words + 2) / 2 * 4; }
 __global__ void __launch_bounds__(1024) tile_index_kernel(const int32_t* brow, const int32_t* bcol, int nnz,
-                                                          int nbr, int nbc, int wpr, int32_t* row_ptr,
+                                                          int nbr, int nbc, int pitch, int32_t* row_ptr,
                                                           int32_t* block_indices, int32_t* row_order) {
-  extern __shared__ uint32_t bits[];   // [nbr][wpr], then the rows' first tiles
+  extern __shared__ uint32_t bits[];   // [nbr][pitch], then the tiles ahead of every word and of the end
   __shared__ int32_t warp_sum[32];
-  int32_t* first = reinterpret_cast<int32_t*>(bits + nbr * wpr);
+  __shared__ __align__(16) uint32_t key[kOneBlockOrder];
+  const int words = nbr * pitch;
+  uint16_t* ahead = reinterpret_cast<uint16_t*>(bits + words);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  for (int i = tid; i < nbr * wpr; i += 1024) bits[i] = 0u;
+  for (int i = tid; i < words; i += 1024) bits[i] = 0u;
   grid_dependency_wait();
   __syncthreads();
 #pragma unroll 4
   for (int i = tid; i < nnz; i += 1024) {
     const int r = brow[i], c = bcol[i];
     block_indices[i] = 0;   // every entry is a valid position even when the list is rejected afterwards
-    if ((unsigned)r < (unsigned)nbr && (unsigned)c < (unsigned)nbc) atomicOr(bits + r * wpr + (c >> 5), 1u << (c & 31));
+    if ((unsigned)r < (unsigned)nbr && (unsigned)c < (unsigned)nbc) atomicOr(bits + r * pitch + (c >> 5), 1u << (c & 31));
   }
   __syncthreads();
-  const int per = (nbr + 1023) / 1024, lo = tid * per < nbr ? tid * per : nbr, hi = lo + per < nbr ? lo + per : nbr;
+  const int per = (words + 1023) / 1024 | 1, lo = tid * per < words ? tid * per : words, hi = lo + per < words ? lo + per : words;
   int sum = 0;
-  for (int r = lo; r < hi; ++r) {
-    first[r] = sum;
-    for (int w = 0; w < wpr; ++w) sum += __popc(bits[r * wpr + w]);
-  }
+  for (int w = lo; w < hi; ++w) sum += __popc(bits[w]);
   int incl = sum;
   for (int o = 1; o < 32; o <<= 1) {
     const int v = __shfl_up_sync(0xffffffffu, incl, o);
@@ -149,32 +160,34 @@ __global__ void __launch_bounds__(1024) tile_index_kernel(const int32_t* brow, c
     warp_sum[lane] = v;
   }
   __syncthreads();
-  const int before = (wid ? warp_sum[wid - 1] : 0) + incl - sum;
-  for (int r = lo; r < hi; ++r) {
-    first[r] += before;
-    row_ptr[r] = first[r];
+  int run = (wid ? warp_sum[wid - 1] : 0) + incl - sum;
+  for (int w = lo; w < hi; ++w) {
+    ahead[w] = (uint16_t)run;
+    run += __popc(bits[w]);
   }
-  if (tid == 1023) row_ptr[nbr] = before + sum;
-  if (tid == 1023) first[nbr] = before + sum;
+  if (tid == 1023) ahead[words] = (uint16_t)run;
   __syncthreads();
-  if (row_order != nullptr)   // as row_order_kernel
-    for (int r = wid; r < nbr; r += 32) {
-      const int mine = first[r + 1] - first[r];
-      int ahead = 0;
-      for (int i = lane; i < nbr; i += 32) {
-        const int c = first[i + 1] - first[i];
-        ahead += (c > mine || (c == mine && i < r)) ? 1 : 0;
-      }
-      ahead = __reduce_add_sync(0xffffffffu, ahead);
-      if (lane == 0) row_order[ahead] = r;
+  for (int r = tid; r <= nbr; r += 1024) row_ptr[r] = ahead[r * pitch];
+  if (row_order != nullptr) {   // as row_order_kernel: a row comes after all rows with a larger key, four threads count them
+    if (tid < kOneBlockOrder) key[tid] = tid < nbr ? (uint32_t)(ahead[(tid + 1) * pitch] - ahead[tid * pitch]) * kOneBlockOrder + (kOneBlockOrder - 1 - tid) : 0u;
+    __syncthreads();
+    const int r = tid >> 2;
+    const uint32_t mine = key[r];
+    int before = 0;
+    for (int i = tid & 3; i < (nbr + 3) / 4; i += 4) {
+      const uint4 k = reinterpret_cast<const uint4*>(key)[i];
+      before += (k.x > mine ? 1 : 0) + (k.y > mine ? 1 : 0) + (k.z > mine ? 1 : 0) + (k.w > mine ? 1 : 0);
     }
+    before += __shfl_xor_sync(0xffffffffu, before, 1);
+    before += __shfl_xor_sync(0xffffffffu, before, 2);
+    if ((tid & 3) == 0 && r < nbr) row_order[before] = r;
+  }
 #pragma unroll 4
   for (int i = tid; i < nnz; i += 1024) {
     const int r = brow[i], c = bcol[i];
     if ((unsigned)r >= (unsigned)nbr || (unsigned)c >= (unsigned)nbc) continue;
-    int at = first[r] + __popc(bits[r * wpr + (c >> 5)] & ((1u << (c & 31)) - 1u));
-    for (int w = 0; w < (c >> 5); ++w) at += __popc(bits[r * wpr + w]);
-    block_indices[at] = i;
+    const int w = r * pitch + (c >> 5);
+    block_indices[ahead[w] + __popc(bits[w] & ((1u << (c & 31)) - 1u))] = i;
   }
 }
 
@@ -1078,9 +1091,12 @@ static int build_tile_index(const int32_t* block_rows, const int32_t* block_cols
   if (nnz > 0x7fffffffLL) return VOID_ERR_TOO_LARGE;
   if (ws == nullptr || ws_bytes < void_tile_index_ws_bytes(nbr, nbc)) return VOID_ERR_WORKSPACE;
   const int wpr = (nbc + 31) / 32;
-  if (nnz <= kOneBlockTiles && (int64_t)nbr * (wpr + 1) <= kOneBlockWords) {
+  const int pitch = one_block_pitch(wpr);
+  if (one_block_index(nnz, (int64_t)nbr * pitch)) {
+    const int smem = one_block_smem(nbr * pitch);
+    if (smem > 48 * 1024 && ensure_smem((const void*)tile_index_kernel, one_block_smem(kOneBlockWords))) return VOID_ERR_CUDA;
     *ordered = row_order != nullptr && nbr <= kOneBlockOrder;
-    launch_pdl(tile_index_kernel, 1, 1024, (nbr * (wpr + 1) + 1) * 4, st, block_rows, block_cols, (int)nnz, nbr, nbc, wpr, row_ptr, block_indices,
+    launch_pdl(tile_index_kernel, 1, 1024, smem, st, block_rows, block_cols, (int)nnz, nbr, nbc, pitch, row_ptr, block_indices,
                *ordered ? row_order : nullptr);
     return last_status();
   }
