@@ -73,3 +73,49 @@ def test_plan_that_points_outside_its_scratch_is_reported_not_followed():
     assert not guard[(plan.n_counters - 1) * per_row:].any()      # nothing was written behind the scratch
     with pytest.raises(void.VoidB200Error, match="does not fit"):
         void.check_device_status()
+
+
+def _earlier_failure():
+    """A call that fails on the host: more shared memory than a block can have.  The runtime remembers its error."""
+    assert _lib.load().void_launch_floor(1, 128, 10_000_000, torch.cuda.current_stream().cuda_stream) != 0
+
+
+@pytest.mark.parametrize("what", ["product", "store", "fp8_exact", "few_columns", "grouped", "stream_k", "columns", "tiles", "index", "long_index", "convert", "linear"])
+def test_a_launch_reports_its_own_status_and_no_earlier_calls(what):
+    q, bq, bs = _small()
+    gen = torch.Generator().manual_seed(5)
+    a = void.dense_to_void(torch.randn(512, 512, generator=gen).cuda())
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    if what == "linear":
+        layer, x = void.SparseLinear(512, 512, a, bias=True), torch.randn(64, 512, generator=gen).cuda().requires_grad_(True)
+        call = lambda: layer(x).sum().backward()
+    elif what == "grouped":
+        big = workloads.block_sparse(workloads.uniform_mask(128, 128, 0.5, seed=1), 2048, seed=1)
+        t, b = big.a.to_dtype(torch.float16), big.b.half()
+        for _ in range(5):      # the fifth runs the grouped kernel, whose first launch sets its attributes
+            torch.cuda.synchronize()
+            void.void_spmm(t, b)
+        call = lambda: void.void_spmm(t, b)
+    else:
+        rows, cols = a.block_rows, a.block_cols
+        f8 = void.void_tensor_to_fp8(a)
+        b8, b8s, _ = void.quantize_cols_fp8(torch.randn(512, 256, generator=gen).cuda())
+        b8q, b8qs = void.quantize_cols_int8(torch.randn(512, 256, generator=gen).cuda())
+        wide = torch.randperm(700 * 700, generator=gen)[:20000]
+        wide_rows, wide_cols = (wide // 700).int().cuda(), (wide % 700).int().cuda()
+        from void_b200.format import build_tile_index
+        call = {"product": lambda: void.void_spmm_int8(q, bq, bs), "store": lambda: void.void_spmm_int8(void.quantize_void_tensor(a), b8q, b8qs),
+                "fp8_exact": lambda: void.void_spmm_fp8(f8, b8, b_scale=b8s, scale_terms=0),
+                "few_columns": lambda: void.void_spmv(a, torch.ones(512, device="cuda")),
+                "stream_k": lambda: void.void_spmm_stream_k(q, bq, b_scale=bs),
+                "columns": lambda: void.quantize_cols_int8(torch.randn(20000, 40, generator=gen).cuda()),
+                "tiles": lambda: void.void_tensor_to_fp8(a),
+                "index": lambda: build_tile_index(rows, cols, 16, 16),
+                "long_index": lambda: build_tile_index(wide_rows, wide_cols, 700, 700),
+                "convert": lambda: void.quantize_void_tensor(void.dense_to_void(torch.ones(96, 96, device="cuda"))).packed()}[what]
+    call()
+    for _ in range(2):          # what the first call builds, and what every one launches
+        _earlier_failure()
+        call()
+    torch.cuda.synchronize()
+    void.check_device_status()

@@ -24,7 +24,7 @@ constexpr int kOneBlockWords = 32768;  // up to this many words (a grid side of 
 constexpr size_t kBitmapAt = 256;  // workspace: unsigned long long counts[2] (kept tiles, nonzero elements), then the bitmap
 
 static inline cudaStream_t as_stream(void_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
-static inline int last_status() { return cudaGetLastError() == cudaSuccess ? VOID_OK : VOID_ERR_CUDA; }
+using vb::Launches;
 
 // morton(r, c): bits of r on the even positions, bits of c on the odd ones (void/format.py:41-51)
 __host__ __device__ inline uint32_t spread16(uint32_t v) {
@@ -400,17 +400,17 @@ static int rank_bitmap(const WsLayout& w, unsigned char* ws, int64_t* counts_out
   int32_t* chunk_ptr = reinterpret_cast<int32_t*>(ws + w.off_chunk);
   const unsigned long long* counts = reinterpret_cast<const unsigned long long*>(ws);
   if (w.words <= kOneBlockWords) {
-    vb::launch_pdl(rank_bitmap_kernel, 1, 1024, 0, st, bitmap, (int)w.words, word_prefix, counts, counts_out);
-    return last_status();
+    return vb::status_of(vb::launch_pdl(rank_bitmap_kernel, 1, 1024, 0, st, bitmap, (int)w.words, word_prefix, counts, counts_out));
   }
-  chunk_count_kernel<<<(unsigned)w.chunks, kChunkWords, 0, st>>>(bitmap, w.words, chunk_ptr);
-  chunk_scan_kernel<<<1, 1024, 0, st>>>(chunk_ptr, w.chunks, counts, counts_out);
-  word_prefix_kernel<<<(unsigned)w.chunks, kChunkWords, 0, st>>>(bitmap, w.words, chunk_ptr, word_prefix);
-  return last_status();
+  Launches on(st);
+  on.run(chunk_count_kernel, (unsigned)w.chunks, kChunkWords, bitmap, w.words, chunk_ptr);
+  on.run(chunk_scan_kernel, 1, 1024, chunk_ptr, w.chunks, counts, counts_out);
+  on.run(word_prefix_kernel, (unsigned)w.chunks, kChunkWords, bitmap, w.words, chunk_ptr, word_prefix);
+  return on.status();
 }
 
 template <typename T>
-static void launch_dense_mark(const void* matrix, int64_t ld, int M, int N, float threshold, void* ws, cudaStream_t st) {
+static int launch_dense_mark(const void* matrix, int64_t ld, int M, int N, float threshold, void* ws, cudaStream_t st) {
   constexpr int kVec = 16 / (int)sizeof(T);
   const int nbr = (M + kTile - 1) / kTile;
   const T* a = static_cast<const T*>(matrix);
@@ -418,19 +418,22 @@ static void launch_dense_mark(const void* matrix, int64_t ld, int M, int N, floa
   const int strips = (N + 32 * (vec ? kVec : 1) - 1) / (32 * (vec ? kVec : 1));
   const unsigned blocks = (unsigned)(((int64_t)nbr * strips + 7) / 8);
   unsigned long long* counts = static_cast<unsigned long long*>(ws);
-  if (vec) dense_mark_kernel<T, kVec><<<blocks, 256, 0, st>>>(a, ld, M, N, nbr, strips, threshold, bitmap_of(ws), counts);
-  else dense_mark_kernel<T, 1><<<blocks, 256, 0, st>>>(a, ld, M, N, nbr, strips, threshold, bitmap_of(ws), counts);
+  Launches on(st);
+  on.run(vec ? dense_mark_kernel<T, kVec> : dense_mark_kernel<T, 1>, blocks, 256, a, ld, M, N, nbr, strips, threshold, bitmap_of(ws), counts);
+  return on.status();
 }
 
 template <typename T>
-static void launch_emit_tiles(const WsLayout& w, const void* ws, const void* matrix, int64_t ld, int M, int N, int64_t n_blocks,
-                              int32_t* brow, int32_t* bcol, int64_t* codes, void* values, cudaStream_t st) {
+static int launch_emit_tiles(const WsLayout& w, const void* ws, const void* matrix, int64_t ld, int M, int N, int64_t n_blocks,
+                             int32_t* brow, int32_t* bcol, int64_t* codes, void* values, cudaStream_t st) {
   constexpr int kVec = 16 / (int)sizeof(T);
   const int32_t* prefix = reinterpret_cast<const int32_t*>(static_cast<const unsigned char*>(ws) + w.off_prefix);
   const T* a = static_cast<const T*>(matrix);
   const bool vec = ld % kVec == 0 && ((reinterpret_cast<uintptr_t>(matrix) | reinterpret_cast<uintptr_t>(values)) & 15u) == 0;
-  auto kernel = vec ? emit_tiles_kernel<T, kVec> : emit_tiles_kernel<T, 1>;
-  kernel<<<(unsigned)w.words, 256, 0, st>>>(bitmap_of(ws), prefix, a, ld, M, N, n_blocks, brow, bcol, codes, static_cast<T*>(values));
+  Launches on(st);
+  on.run(vec ? emit_tiles_kernel<T, kVec> : emit_tiles_kernel<T, 1>, (unsigned)w.words, 256, bitmap_of(ws), prefix, a, ld, M, N, n_blocks, brow, bcol,
+         codes, static_cast<T*>(values));
+  return on.status();
 }
 
 }  // namespace vbf
@@ -454,9 +457,10 @@ int void_dense_mark(const void* matrix, int32_t elem, int64_t ld, int32_t M, int
   cudaStream_t st = vbf::as_stream(stream);
   if (cudaMemsetAsync(ws, 0, w.clear_bytes, st) != cudaSuccess) return VOID_ERR_CUDA;
   if ((int64_t)nbr * nbc > 0) {
-    if (elem == VOID_ELEM_F32) vbf::launch_dense_mark<float>(matrix, ld, M, N, threshold, ws, st);
-    else if (elem == VOID_ELEM_F16) vbf::launch_dense_mark<__half>(matrix, ld, M, N, threshold, ws, st);
-    else vbf::launch_dense_mark<__nv_bfloat16>(matrix, ld, M, N, threshold, ws, st);
+    const int rc = elem == VOID_ELEM_F32   ? vbf::launch_dense_mark<float>(matrix, ld, M, N, threshold, ws, st)
+                   : elem == VOID_ELEM_F16 ? vbf::launch_dense_mark<__half>(matrix, ld, M, N, threshold, ws, st)
+                                           : vbf::launch_dense_mark<__nv_bfloat16>(matrix, ld, M, N, threshold, ws, st);
+    if (rc != VOID_OK) return rc;
   }
   return vbf::rank_bitmap(w, static_cast<unsigned char*>(ws), counts_out, st);
 }
@@ -472,8 +476,9 @@ int void_csr_mark(const int32_t* crow, const int32_t* col, int32_t M, int32_t N,
   cudaStream_t st = vbf::as_stream(stream);
   if (cudaMemsetAsync(ws, 0, w.clear_bytes, st) != cudaSuccess) return VOID_ERR_CUDA;
   if (M > 0) {
-    const int tb = 256;
-    vbf::csr_mark_kernel<<<(unsigned)(((int64_t)M * 32 + tb - 1) / tb), tb, 0, st>>>(crow, col, M, vbf::bitmap_of(ws));
+    vbf::Launches on(st);
+    on.run(vbf::csr_mark_kernel, (unsigned)(((int64_t)M * 32 + 255) / 256), 256, crow, col, M, vbf::bitmap_of(ws));
+    if (on.status() != VOID_OK) return on.status();
   }
   return vbf::rank_bitmap(w, static_cast<unsigned char*>(ws), counts_out, st);
 }
@@ -486,11 +491,10 @@ int void_morton_emit(const void* ws, int32_t nbr, int32_t nbc, int64_t n_blocks,
   if (n_blocks == 0) return VOID_OK;
   if (block_rows == nullptr || block_cols == nullptr || morton_codes == nullptr) return VOID_ERR_BAD_ARG;
   const unsigned char* base = static_cast<const unsigned char*>(ws);
-  const int tb = 256;
-  vbf::emit_index_kernel<<<(unsigned)((w.words + tb - 1) / tb), tb, 0, vbf::as_stream(stream)>>>(
-      vbf::bitmap_of(ws), reinterpret_cast<const int32_t*>(base + w.off_prefix), w.words,
-      block_rows, block_cols, morton_codes);
-  return vbf::last_status();
+  vbf::Launches on(vbf::as_stream(stream));
+  on.run(vbf::emit_index_kernel, (unsigned)((w.words + 255) / 256), 256, vbf::bitmap_of(ws), reinterpret_cast<const int32_t*>(base + w.off_prefix),
+         w.words, block_rows, block_cols, morton_codes);
+  return on.status();
 }
 
 int void_dense_gather(const void* matrix, int32_t elem, int64_t ld, int32_t M, int32_t N, const int32_t* block_rows,
@@ -499,20 +503,18 @@ int void_dense_gather(const void* matrix, int32_t elem, int64_t ld, int32_t M, i
   if (elem < VOID_ELEM_F32 || elem > VOID_ELEM_BF16) return VOID_ERR_BAD_ARG;
   if (n_blocks == 0) return VOID_OK;
   if (matrix == nullptr || block_rows == nullptr || block_cols == nullptr || values == nullptr) return VOID_ERR_BAD_ARG;
-  cudaStream_t st = vbf::as_stream(stream);
-  const int tb = 256;
-  const unsigned blocks = (unsigned)((n_blocks * 128 + tb - 1) / tb);
+  vbf::Launches on(vbf::as_stream(stream));
+  const unsigned blocks = (unsigned)((n_blocks * 128 + 255) / 256);
   if (elem == VOID_ELEM_F32)
-    vbf::dense_gather_kernel<float><<<blocks, tb, 0, st>>>(static_cast<const float*>(matrix), ld, M, N, block_rows,
-                                                            block_cols, n_blocks, static_cast<float*>(values));
+    on.run(vbf::dense_gather_kernel<float>, blocks, 256, static_cast<const float*>(matrix), ld, M, N, block_rows, block_cols, n_blocks,
+           static_cast<float*>(values));
   else if (elem == VOID_ELEM_F16)
-    vbf::dense_gather_kernel<__half><<<blocks, tb, 0, st>>>(static_cast<const __half*>(matrix), ld, M, N, block_rows,
-                                                             block_cols, n_blocks, static_cast<__half*>(values));
+    on.run(vbf::dense_gather_kernel<__half>, blocks, 256, static_cast<const __half*>(matrix), ld, M, N, block_rows, block_cols, n_blocks,
+           static_cast<__half*>(values));
   else
-    vbf::dense_gather_kernel<__nv_bfloat16><<<blocks, tb, 0, st>>>(static_cast<const __nv_bfloat16*>(matrix), ld, M, N,
-                                                                    block_rows, block_cols, n_blocks,
-                                                                    static_cast<__nv_bfloat16*>(values));
-  return vbf::last_status();
+    on.run(vbf::dense_gather_kernel<__nv_bfloat16>, blocks, 256, static_cast<const __nv_bfloat16*>(matrix), ld, M, N, block_rows, block_cols,
+           n_blocks, static_cast<__nv_bfloat16*>(values));
+  return on.status();
 }
 
 int void_dense_emit(const void* ws, const void* matrix, int32_t elem, int64_t ld, int32_t M, int32_t N, int64_t n_blocks,
@@ -530,10 +532,9 @@ int void_dense_emit(const void* ws, const void* matrix, int32_t elem, int64_t ld
   if (matrix == nullptr || block_rows == nullptr || block_cols == nullptr || morton_codes == nullptr || values == nullptr)
     return VOID_ERR_BAD_ARG;
   cudaStream_t st = vbf::as_stream(stream);
-  if (elem == VOID_ELEM_F32) vbf::launch_emit_tiles<float>(w, ws, matrix, ld, M, N, n_blocks, block_rows, block_cols, morton_codes, values, st);
-  else if (elem == VOID_ELEM_F16) vbf::launch_emit_tiles<__half>(w, ws, matrix, ld, M, N, n_blocks, block_rows, block_cols, morton_codes, values, st);
-  else vbf::launch_emit_tiles<__nv_bfloat16>(w, ws, matrix, ld, M, N, n_blocks, block_rows, block_cols, morton_codes, values, st);
-  return vbf::last_status();
+  if (elem == VOID_ELEM_F32) return vbf::launch_emit_tiles<float>(w, ws, matrix, ld, M, N, n_blocks, block_rows, block_cols, morton_codes, values, st);
+  if (elem == VOID_ELEM_F16) return vbf::launch_emit_tiles<__half>(w, ws, matrix, ld, M, N, n_blocks, block_rows, block_cols, morton_codes, values, st);
+  return vbf::launch_emit_tiles<__nv_bfloat16>(w, ws, matrix, ld, M, N, n_blocks, block_rows, block_cols, morton_codes, values, st);
 }
 
 int void_csr_scatter(const int32_t* crow, const int32_t* col, const float* data, int32_t M, int32_t N, const void* ws,
@@ -547,10 +548,10 @@ int void_csr_scatter(const int32_t* crow, const int32_t* col, const float* data,
   cudaStream_t st = vbf::as_stream(stream);
   if (cudaMemsetAsync(values, 0, (size_t)n_blocks * 4096, st) != cudaSuccess) return VOID_ERR_CUDA;
   const unsigned char* base = static_cast<const unsigned char*>(ws);
-  const int tb = 256;
-  vbf::csr_scatter_kernel<<<(unsigned)(((int64_t)M * 32 + tb - 1) / tb), tb, 0, st>>>(
-      crow, col, data, M, vbf::bitmap_of(ws), reinterpret_cast<const int32_t*>(base + w.off_prefix), values);
-  return vbf::last_status();
+  vbf::Launches on(st);
+  on.run(vbf::csr_scatter_kernel, (unsigned)(((int64_t)M * 32 + 255) / 256), 256, crow, col, data, M, vbf::bitmap_of(ws),
+         reinterpret_cast<const int32_t*>(base + w.off_prefix), values);
+  return on.status();
 }
 
 }  // extern "C"

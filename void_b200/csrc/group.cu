@@ -459,8 +459,7 @@ template <int KIND>
 int launch_group(const GroupParams& p, const CUtensorMap& mb, int grid, int smem, cudaStream_t st) {
   auto kernel = group_kernel<KIND>;
   if (ensure_smem((const void*)kernel, smem)) return VOID_ERR_CUDA;
-  launch_pdl(kernel, grid, kThreads, smem, st, mb, p);
-  return cudaGetLastError() == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
+  return status_of(launch_pdl(kernel, grid, kThreads, smem, st, mb, p));
 }
 
 }  // namespace
@@ -487,16 +486,17 @@ int void_group_build(const int32_t* row_ptr, const int32_t* row_order, const int
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int32_t *counts = ws, *blob_base = ws + n_groups, *tile_at = ws + 2 * (size_t)n_groups;
   const int units = tile_bytes / 128, blocks = (n_groups + 3) / 4;
-  group_rows_kernel<<<(n_groups * kMaxGroupRows + 255) / 256, 256, 0, st>>>(row_order, nbr, n_groups, group_rows);
-  group_walk_kernel<false><<<blocks, 128, 0, st>>>(row_ptr, tile_cols, group_rows, n_groups, max_entries, max_tiles, units, panel_units, nullptr,
-                                                   nullptr, counts, nullptr, nullptr, nullptr);
-  group_scan_kernel<<<1, 1024, 0, st>>>(counts, row_ptr, group_rows, n_groups, units, stage_ptr, blob_base);
-  group_walk_kernel<true><<<blocks, 128, 0, st>>>(row_ptr, tile_cols, group_rows, n_groups, max_entries, max_tiles, units, panel_units, stage_ptr,
-                                                  blob_base, counts, records, reinterpret_cast<uint8_t*>(blob), tile_at);
   const int64_t pieces = nnz * (tile_bytes / 16);
-  group_copy_kernel<<<(unsigned)((pieces + 255) / 256), 256, 0, st>>>(reinterpret_cast<const uint4*>(tiles), tile_at, nnz,
-                                                                      tile_bytes / 16, reinterpret_cast<uint4*>(blob));
-  return cudaGetLastError() == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
+  Launches on(st);
+  on.run(group_rows_kernel, (unsigned)((n_groups * kMaxGroupRows + 255) / 256), 256, row_order, nbr, n_groups, group_rows);
+  on.run(group_walk_kernel<false>, (unsigned)blocks, 128, row_ptr, tile_cols, group_rows, n_groups, max_entries, max_tiles, units, panel_units,
+         nullptr, nullptr, counts, nullptr, nullptr, nullptr);
+  on.run(group_scan_kernel, 1, 1024, counts, row_ptr, group_rows, n_groups, units, stage_ptr, blob_base);
+  on.run(group_walk_kernel<true>, (unsigned)blocks, 128, row_ptr, tile_cols, group_rows, n_groups, max_entries, max_tiles, units, panel_units,
+         stage_ptr, blob_base, counts, records, reinterpret_cast<uint8_t*>(blob), tile_at);
+  on.run(group_copy_kernel, (unsigned)((pieces + 255) / 256), 256, reinterpret_cast<const uint4*>(tiles), tile_at, nnz, tile_bytes / 16,
+         reinterpret_cast<uint4*>(blob));
+  return on.status();
 }
 
 int void_spmm_grouped(const void_spmm_args* a, const void_group_store* s, int32_t kind, void_stream_t stream) {

@@ -74,9 +74,9 @@ inline int ensure_smem(const void* kernel, int bytes) {
 
 template <typename T>
 struct same_type { using type = T; };
-// A launch that may start beside the end of the kernel before it.
+// overlapped: the launch may start beside the end of the kernel before it.
 template <typename... P>
-cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem_bytes, cudaStream_t stream, const typename same_type<P>::type&... args) {
+cudaError_t launch_kernel(bool overlapped, void (*kernel)(P...), dim3 grid, int threads, int smem_bytes, cudaStream_t stream, const typename same_type<P>::type&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)threads);
@@ -86,9 +86,30 @@ cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem_by
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlapped ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
+template <typename... P>
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem_bytes, cudaStream_t stream, const typename same_type<P>::type&... args) {
+  return launch_kernel<P...>(true, kernel, grid, threads, smem_bytes, stream, args...);
+}
+// Every launch reports its own status.  (The runtime's last error is the last call's that failed, which may be an earlier entry's:
+// cudaGetLastError behind a launch would report that one.)
+inline int status_of(cudaError_t rc) { return rc == cudaSuccess ? VOID_OK : VOID_ERR_CUDA; }
+// Launches that follow one another on a stream; none after the first that failed.
+class Launches {
+ public:
+  explicit Launches(cudaStream_t stream) : stream_(stream) {}
+  template <typename... P>
+  void run(void (*kernel)(P...), dim3 grid, int threads, const typename same_type<P>::type&... args) {
+    if (rc_ == cudaSuccess) rc_ = launch_kernel<P...>(false, kernel, grid, threads, 0, stream_, args...);
+  }
+  int status() const { return status_of(rc_); }
+
+ private:
+  cudaStream_t stream_;
+  cudaError_t rc_ = cudaSuccess;
+};
 
 // B as a tensor for the copy engine, 128-byte swizzle, zero fill outside [K, N].  Elements of es bytes: every box is 128
 // bytes (kPanelN / es columns) wide, a panel takes es of them.

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "../../include/void_b200.h"
+#include "launch.cuh"
 
 namespace vb {
 
@@ -312,8 +313,7 @@ int void_plan_segments(const int32_t* row_ptr, int32_t nbr, int32_t n_chunks, in
   if (row_cost < 1) return VOID_ERR_BAD_ARG;
   PlanIn in{row_ptr, woff, nbr, n_chunks, n_cta, split_rows, chunk_tiles, row_cost};
   const PlanWs w = carve_ws(reinterpret_cast<int32_t*>(ws), n_cta);
-  plan_kernel<<<1, 1024, 0, reinterpret_cast<cudaStream_t>(stream)>>>(in, w, segs, segs_capacity, cta_seg_ptr, counts);
-  return cudaGetLastError() == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
+  return status_of(launch_kernel(false, plan_kernel, 1, 1024, 0, reinterpret_cast<cudaStream_t>(stream), in, w, segs, segs_capacity, cta_seg_ptr, counts));
 }
 
 // Host twin of void_plan_segments over HOST arrays: the same splitting arithmetic run as plain

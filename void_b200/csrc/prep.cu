@@ -19,7 +19,6 @@
 namespace vb {
 
 static inline cudaStream_t as_stream(void_stream_t s) { return reinterpret_cast<cudaStream_t>(s); }
-static inline int last_status() { return cudaGetLastError() == cudaSuccess ? VOID_OK : VOID_ERR_CUDA; }
 
 // Exclusive prefix sum of n int32 values by ONE block of 1024 threads; out[n] = total.
 // in and out may alias.
@@ -980,10 +979,7 @@ static ClusterRoom cluster_room() {
     int room[2] = {0, 0};
     for (int ctas = 1; ctas <= 2; ++ctas) {
       cfg.dynamicSmemBytes = (size_t)(kFusedMaxSmem / ctas);
-      if (cudaOccupancyMaxActiveClusters(&room[ctas - 1], kernel, &cfg) != cudaSuccess) {
-        (void)cudaGetLastError();   // no error of the launch
-        return r;
-      }
+      if (cudaOccupancyMaxActiveClusters(&room[ctas - 1], kernel, &cfg) != cudaSuccess) return r;
     }
     packed = 1u + ((uint32_t)room[1] << 16 | (uint32_t)room[0]);
     rooms[dev].store(packed, std::memory_order_relaxed);   // (threads that ask at once store the same)
@@ -1096,27 +1092,23 @@ static int build_tile_index(const int32_t* block_rows, const int32_t* block_cols
     const int smem = one_block_smem(nbr * pitch);
     if (smem > 48 * 1024 && ensure_smem((const void*)tile_index_kernel, one_block_smem(kOneBlockWords))) return VOID_ERR_CUDA;
     *ordered = row_order != nullptr && nbr <= kOneBlockOrder;
-    launch_pdl(tile_index_kernel, 1, 1024, smem, st, block_rows, block_cols, (int)nnz, nbr, nbc, pitch, row_ptr, block_indices,
-               *ordered ? row_order : nullptr);
-    return last_status();
+    return status_of(launch_pdl(tile_index_kernel, 1, 1024, smem, st, block_rows, block_cols, (int)nnz, nbr, nbc, pitch, row_ptr, block_indices,
+                                *ordered ? row_order : nullptr));
   }
   uint32_t* bitmap = reinterpret_cast<uint32_t*>(ws);
   int32_t* counts = reinterpret_cast<int32_t*>(bitmap + (size_t)nbr * wpr);
   if (cudaMemsetAsync(bitmap, 0, (size_t)nbr * wpr * 4, st) != cudaSuccess) return VOID_ERR_CUDA;
-  const int tb = 256;
-  if (nnz > 0)
-    mark_tiles_kernel<<<(unsigned)((nnz + tb - 1) / tb), tb, 0, st>>>(block_rows, block_cols, nnz, nbr, nbc, wpr, bitmap,
-                                                                     block_indices);
+  const unsigned blocks = (unsigned)((nnz + 255) / 256);
+  Launches on(st);
+  if (nnz > 0) on.run(mark_tiles_kernel, blocks, 256, block_rows, block_cols, nnz, nbr, nbc, wpr, bitmap, block_indices);
   if ((int64_t)nbr * wpr <= kOneBlockBitmap) {
-    count_scan_rows_kernel<<<1, 1024, 0, st>>>(bitmap, nbr, wpr, counts, row_ptr);
+    on.run(count_scan_rows_kernel, 1, 1024, bitmap, nbr, wpr, counts, row_ptr);
   } else {
-    count_rows_kernel<<<(unsigned)(((int64_t)nbr * 32 + tb - 1) / tb), tb, 0, st>>>(bitmap, nbr, wpr, counts);
-    scan_rows_kernel<<<1, 1024, 0, st>>>(counts, row_ptr, nbr);
+    on.run(count_rows_kernel, (unsigned)(((int64_t)nbr * 32 + 255) / 256), 256, bitmap, nbr, wpr, counts);
+    on.run(scan_rows_kernel, 1, 1024, counts, row_ptr, nbr);
   }
-  if (nnz > 0)
-    rank_tiles_kernel<<<(unsigned)((nnz + tb - 1) / tb), tb, 0, st>>>(block_rows, block_cols, nnz, nbr, nbc, wpr, bitmap,
-                                                                     row_ptr, block_indices);
-  return last_status();
+  if (nnz > 0) on.run(rank_tiles_kernel, blocks, 256, block_rows, block_cols, nnz, nbr, nbc, wpr, bitmap, row_ptr, block_indices);
+  return on.status();
 }
 
 int void_build_tile_index(const int32_t* block_rows, const int32_t* block_cols, int64_t nnz, int32_t nbr,
@@ -1139,8 +1131,7 @@ int void_row_order(const int32_t* row_ptr, int32_t nbr, int32_t* order, void_str
   if (nbr < 0) return VOID_ERR_BAD_ARG;
   if (nbr == 0) return VOID_OK;
   if (row_ptr == nullptr || order == nullptr) return VOID_ERR_BAD_ARG;
-  launch_pdl(row_order_kernel, (int)(((int64_t)nbr * 32 + 255) / 256), 256, 0, as_stream(stream), row_ptr, nbr, order);
-  return last_status();
+  return status_of(launch_pdl(row_order_kernel, (int)(((int64_t)nbr * 32 + 255) / 256), 256, 0, as_stream(stream), row_ptr, nbr, order));
 }
 
 int void_pack_tiles(const void* values, const float* scales, int64_t n_scales, const int32_t* block_cols,
@@ -1162,10 +1153,9 @@ int void_pack_tiles(const void* values, const float* scales, int64_t n_scales, c
     rows.nbr = nbr;
   }
   const unsigned blocks = rows.pack_blocks + (unsigned)((rows.nbr + 7) / 8);
-  if (blocks > 0)
-    launch_pdl(pack_tiles_kernel, (int)blocks, 256, 0, st, reinterpret_cast<const uint4*>(values), block_indices, nnz,
-               reinterpret_cast<uint4*>(packed), TileMeta{block_cols, scales, n_scales, tile_cols, tile_scales}, rows);
-  return last_status();
+  if (blocks == 0) return VOID_OK;
+  return status_of(launch_pdl(pack_tiles_kernel, (int)blocks, 256, 0, st, reinterpret_cast<const uint4*>(values), block_indices, nnz,
+                              reinterpret_cast<uint4*>(packed), TileMeta{block_cols, scales, n_scales, tile_cols, tile_scales}, rows));
 }
 
 int void_pack_tiles_f8_split(const void* values, const float* scales, int64_t n_scales, const int32_t* block_rows,
@@ -1175,7 +1165,6 @@ int void_pack_tiles_f8_split(const void* values, const float* scales, int64_t n_
   if (nnz < 0 || nbr < 0 || (terms != 2 && terms != 3)) return VOID_ERR_BAD_ARG;
   if (row_ptr == nullptr || row_scale == nullptr) return VOID_ERR_BAD_ARG;
   cudaStream_t st = as_stream(stream);
-  const int tb = 256;
   if (nnz > 0) {
     if (values == nullptr || block_rows == nullptr || block_cols == nullptr || block_indices == nullptr ||
         packed == nullptr || tile_cols == nullptr || tile_scales == nullptr)
@@ -1183,22 +1172,15 @@ int void_pack_tiles_f8_split(const void* values, const float* scales, int64_t n_
     if ((reinterpret_cast<uintptr_t>(values) & 15u) != 0 || (reinterpret_cast<uintptr_t>(packed) & 1023u) != 0)
       return VOID_ERR_ALIGN;
     if (scales != nullptr && n_scales != 1 && n_scales != nnz) return VOID_ERR_BAD_ARG;
-    gather_tile_meta_kernel<<<(unsigned)((nnz + tb - 1) / tb), tb, 0, st>>>(block_cols, scales, n_scales, block_indices,
-                                                                           nnz, tile_cols, tile_scales);
   }
-  if (nbr > 0) row_max_scale_kernel<<<(nbr + tb - 1) / tb, tb, 0, st>>>(row_ptr, tile_scales, nbr, row_scale);
-  if (nnz > 0) {
-    const unsigned blocks = (unsigned)((nnz * 64 + tb - 1) / tb);
-    if (terms == 2)
-      pack_tiles_f8_split_kernel<2><<<blocks, tb, 0, st>>>(reinterpret_cast<const uint4*>(values), scales, n_scales,
-                                                           block_rows, block_indices, row_scale, nnz, nbr,
-                                                           reinterpret_cast<uint4*>(packed));
-    else
-      pack_tiles_f8_split_kernel<3><<<blocks, tb, 0, st>>>(reinterpret_cast<const uint4*>(values), scales, n_scales,
-                                                           block_rows, block_indices, row_scale, nnz, nbr,
-                                                           reinterpret_cast<uint4*>(packed));
-  }
-  return last_status();
+  Launches on(st);
+  if (nnz > 0)
+    on.run(gather_tile_meta_kernel, (unsigned)((nnz + 255) / 256), 256, block_cols, scales, n_scales, block_indices, nnz, tile_cols, tile_scales);
+  if (nbr > 0) on.run(row_max_scale_kernel, (unsigned)((nbr + 255) / 256), 256, row_ptr, tile_scales, nbr, row_scale);
+  if (nnz > 0)
+    on.run(terms == 2 ? pack_tiles_f8_split_kernel<2> : pack_tiles_f8_split_kernel<3>, (unsigned)((nnz * 64 + 255) / 256), 256,
+           reinterpret_cast<const uint4*>(values), scales, n_scales, block_rows, block_indices, row_scale, nnz, nbr, reinterpret_cast<uint4*>(packed));
+  return on.status();
 }
 
 int void_reduce_slots(const void* slots, const uint8_t* contrib, int32_t n_ranks, int32_t rows_owned, int32_t row0,
@@ -1210,10 +1192,10 @@ int void_reduce_slots(const void* slots, const uint8_t* contrib, int32_t n_ranks
   if (rows_owned == 0) return VOID_OK;
   if (slots == nullptr || contrib == nullptr || row_scale == nullptr || out == nullptr || ldc < N) return VOID_ERR_BAD_ARG;
   if ((long long)n_panels * 128 < N) return VOID_ERR_SHAPE;
-  reduce_slots_kernel<<<(unsigned)(rows_owned * n_panels), 128, 0, as_stream(stream)>>>(
-      reinterpret_cast<const int32_t*>(slots), contrib, n_ranks, rows_owned, row0, n_panels, panels_per_item, row_scale, col_scale, b_scale,
-      bias, act, out, ldc, out_dtype, M, N);
-  return last_status();
+  Launches on(as_stream(stream));
+  on.run(reduce_slots_kernel, (unsigned)(rows_owned * n_panels), 128, reinterpret_cast<const int32_t*>(slots), contrib, n_ranks, rows_owned, row0,
+         n_panels, panels_per_item, row_scale, col_scale, b_scale, bias, act, out, ldc, out_dtype, M, N);
+  return on.status();
 }
 
 int void_pack_tiles_fp(const void* values, int32_t elem_bytes, const int32_t* block_cols, const int32_t* block_indices,
@@ -1224,17 +1206,11 @@ int void_pack_tiles_fp(const void* values, int32_t elem_bytes, const int32_t* bl
     return VOID_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(values) & 15u) != 0 || (reinterpret_cast<uintptr_t>(packed) & 1023u) != 0)
     return VOID_ERR_ALIGN;
-  cudaStream_t st = as_stream(stream);
-  const int tb = 256;
-  const unsigned blocks = (unsigned)((nnz * 64 * elem_bytes + tb - 1) / tb);
-  const TileMeta meta{block_cols, nullptr, 0, tile_cols, nullptr};
-  if (elem_bytes == 2)
-    pack_tiles_fp_kernel<2><<<blocks, tb, 0, st>>>(reinterpret_cast<const uint4*>(values), block_indices, nnz,
-                                                   reinterpret_cast<uint4*>(packed), meta);
-  else
-    pack_tiles_fp_kernel<4><<<blocks, tb, 0, st>>>(reinterpret_cast<const uint4*>(values), block_indices, nnz,
-                                                   reinterpret_cast<uint4*>(packed), meta);
-  return last_status();
+  Launches on(as_stream(stream));
+  on.run(elem_bytes == 2 ? pack_tiles_fp_kernel<2> : pack_tiles_fp_kernel<4>, (unsigned)((nnz * 64 * elem_bytes + 255) / 256), 256,
+         reinterpret_cast<const uint4*>(values), block_indices, nnz, reinterpret_cast<uint4*>(packed),
+         TileMeta{block_cols, nullptr, 0, tile_cols, nullptr});
+  return on.status();
 }
 
 int void_repack_tiles_fp(const void* values, int32_t elem_bytes, const int32_t* block_indices, int64_t nnz,
@@ -1244,19 +1220,14 @@ int void_repack_tiles_fp(const void* values, int32_t elem_bytes, const int32_t* 
   if (values == nullptr || block_indices == nullptr || packed == nullptr) return VOID_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(values) & 15u) != 0 || (reinterpret_cast<uintptr_t>(packed) & 1023u) != 0)
     return VOID_ERR_ALIGN;
-  cudaStream_t st = as_stream(stream);
-  const int tb = 256;
-  const unsigned blocks = (unsigned)((nnz * 64 * elem_bytes + tb - 1) / tb);   // one thread per 16 bytes in both forms
-  const uint4* v = reinterpret_cast<const uint4*>(values);
+  const unsigned blocks = (unsigned)((nnz * 64 * elem_bytes + 255) / 256);   // one thread per 16 bytes in both forms
   uint4* o = reinterpret_cast<uint4*>(packed);
-  if (transposed) {
-    if (elem_bytes == 2) pack_tiles_fp_t_kernel<2><<<blocks, tb, 0, st>>>(values, block_indices, nnz, o);
-    else pack_tiles_fp_t_kernel<4><<<blocks, tb, 0, st>>>(values, block_indices, nnz, o);
-  } else {
-    if (elem_bytes == 2) pack_tiles_fp_kernel<2><<<blocks, tb, 0, st>>>(v, block_indices, nnz, o, TileMeta{});
-    else pack_tiles_fp_kernel<4><<<blocks, tb, 0, st>>>(v, block_indices, nnz, o, TileMeta{});
-  }
-  return last_status();
+  Launches on(as_stream(stream));
+  if (transposed) on.run(elem_bytes == 2 ? pack_tiles_fp_t_kernel<2> : pack_tiles_fp_t_kernel<4>, blocks, 256, values, block_indices, nnz, o);
+  else
+    on.run(elem_bytes == 2 ? pack_tiles_fp_kernel<2> : pack_tiles_fp_kernel<4>, blocks, 256, reinterpret_cast<const uint4*>(values), block_indices,
+           nnz, o, TileMeta{});
+  return on.status();
 }
 
 int void_copy_rows(const void* in, int64_t ld_in, void* out, int64_t ld_out, int32_t elem_bytes, int64_t rows, int32_t cols,
@@ -1285,7 +1256,7 @@ int void_copy_rows(const void* in, int64_t ld_in, void* out, int64_t ld_out, int
   if (elem_bytes == 1) rc = cudaLaunchKernelEx(&cfg, copy_rows_kernel<uint8_t>, reinterpret_cast<const uint8_t*>(in), ld_in, dst, pieces, rows, cols, early);
   else if (elem_bytes == 2) rc = cudaLaunchKernelEx(&cfg, copy_rows_kernel<uint16_t>, reinterpret_cast<const uint16_t*>(in), ld_in / 2, dst, pieces, rows, cols, early);
   else rc = cudaLaunchKernelEx(&cfg, copy_rows_kernel<uint32_t>, reinterpret_cast<const uint32_t*>(in), ld_in / 4, dst, pieces, rows, cols, early);
-  return rc == cudaSuccess ? last_status() : VOID_ERR_CUDA;
+  return status_of(rc);
 }
 
 int void_transpose(const void* in, int64_t ld_in, void* out, int64_t ld_out, int32_t elem_bytes, int32_t rows, int32_t cols,
@@ -1314,7 +1285,7 @@ int void_transpose(const void* in, int64_t ld_in, void* out, int64_t ld_out, int
   if (elem_bytes == 1) rc = cudaLaunchKernelEx(&cfg, transpose_kernel<uint8_t>, reinterpret_cast<const uint8_t*>(in), li, reinterpret_cast<uint8_t*>(out), lo, rows, cols, whole);
   else if (elem_bytes == 2) rc = cudaLaunchKernelEx(&cfg, transpose_kernel<uint16_t>, reinterpret_cast<const uint16_t*>(in), li, reinterpret_cast<uint16_t*>(out), lo, rows, cols, whole);
   else rc = cudaLaunchKernelEx(&cfg, transpose_kernel<uint32_t>, reinterpret_cast<const uint32_t*>(in), li, reinterpret_cast<uint32_t*>(out), lo, rows, cols, whole);
-  return rc == cudaSuccess ? last_status() : VOID_ERR_CUDA;
+  return status_of(rc);
 }
 
 int void_column_sum(const void* in, int32_t elem, int64_t ld, int32_t rows, int32_t cols, void* out, void_stream_t stream) {
@@ -1325,7 +1296,7 @@ int void_column_sum(const void* in, int32_t elem, int64_t ld, int32_t rows, int3
   const bool ok = elem == VOID_ELEM_F32   ? launch_column_sum<float>(in, ld, rows, cols, out, st)
                   : elem == VOID_ELEM_F16 ? launch_column_sum<__half>(in, ld, rows, cols, out, st)
                                           : launch_column_sum<__nv_bfloat16>(in, ld, rows, cols, out, st);
-  return ok ? last_status() : VOID_ERR_CUDA;
+  return ok ? VOID_OK : VOID_ERR_CUDA;
 }
 
 int void_quant_tiles(const void* values, int32_t elem, int64_t nnz, int32_t kind, void* q, float* scale, float* scale_inv,
@@ -1341,17 +1312,12 @@ int void_quant_tiles(const void* values, int32_t elem, int64_t nnz, int32_t kind
   const unsigned blocks = (unsigned)((nnz * 32 + 255) / 256);
   uint8_t* dst = reinterpret_cast<uint8_t*>(q);
   cudaStream_t st = as_stream(stream);
-#define VB_QUANT(T)                                                                                                             \
-  do {                                                                                                                          \
-    const T* v = reinterpret_cast<const T*>(values);                                                                            \
-    if (kind == VOID_KIND_I8) launch_pdl(quant_tiles_kernel<VOID_KIND_I8, T>, (int)blocks, 256, 0, st, v, nnz, dst, scale, scale_inv, amax, x); \
-    else launch_pdl(quant_tiles_kernel<VOID_KIND_F8E4M3, T>, (int)blocks, 256, 0, st, v, nnz, dst, scale, scale_inv, amax, x);   \
-  } while (0)
-  if (elem == VOID_ELEM_F32) VB_QUANT(float);
-  else if (elem == VOID_ELEM_F16) VB_QUANT(__half);
-  else VB_QUANT(__nv_bfloat16);
+#define VB_QUANT(T)                                                                                                            \
+  status_of(launch_pdl(kind == VOID_KIND_I8 ? quant_tiles_kernel<VOID_KIND_I8, T> : quant_tiles_kernel<VOID_KIND_F8E4M3, T>,    \
+                       (int)blocks, 256, 0, st, reinterpret_cast<const T*>(values), nnz, dst, scale, scale_inv, amax, x))
+  if (elem == VOID_ELEM_F32) return VB_QUANT(float);
+  return elem == VOID_ELEM_F16 ? VB_QUANT(__half) : VB_QUANT(__nv_bfloat16);
 #undef VB_QUANT
-  return last_status();
 }
 
 int void_quant_i8_tiles(const float* values, int64_t nnz, int8_t* q, float* scales, void_stream_t stream) {
@@ -1366,7 +1332,7 @@ int void_quant_fp8_tiles(const float* values, int64_t nnz, uint8_t* q, float* sc
 }
 
 static void quant_pass(const float* b, int64_t ldb, int K, int N, int kind, void* q, int64_t ldq, const float* scale,
-                       int scale_stride, cudaStream_t st) {
+                       int scale_stride, Launches& on) {
   const bool words = (ldq % 4 == 0) && ((reinterpret_cast<uintptr_t>(q) & 3u) == 0);
   const bool vec4 = words && (N % 4 == 0) && (ldb % 4 == 0) && ((reinterpret_cast<uintptr_t>(b) & 15u) == 0) &&
                     ((reinterpret_cast<uintptr_t>(scale) & 15u) == 0);
@@ -1377,11 +1343,10 @@ static void quant_pass(const float* b, int64_t ldb, int K, int N, int kind, void
     uint8_t* dst = reinterpret_cast<uint8_t*>(q) + (size_t)k0 * ldq;
     if (words) {
       dim3 g2((unsigned)((ldq / 4 + 127) / 128), (unsigned)((kk + kColRows - 1) / kColRows));
-      auto kernel = vec4 ? quant_cols4_kernel<true> : quant_cols4_kernel<false>;
-      kernel<<<g2, 128, 0, st>>>(src, ldb, kk, N, kind, dst, ldq, scale, scale_stride);
+      on.run(vec4 ? quant_cols4_kernel<true> : quant_cols4_kernel<false>, g2, 128, src, ldb, kk, N, kind, dst, ldq, scale, scale_stride);
     } else {
       dim3 g2((unsigned)((ldq + 255) / 256), kk);
-      quant_cols_kernel<<<g2, 256, 0, st>>>(src, ldb, kk, N, kind, dst, ldq, scale, scale_stride);
+      on.run(quant_cols_kernel, g2, 256, src, ldb, kk, N, kind, dst, ldq, scale, scale_stride);
     }
   }
 }
@@ -1394,13 +1359,14 @@ int void_quant_cols(const float* b, int64_t ldb, int32_t K, int32_t N, int32_t k
   if (ldb < N || ldq < N) return VOID_ERR_SHAPE;
   if (K > 65535 * kRowSlab) return VOID_ERR_TOO_LARGE;
   cudaStream_t st = as_stream(stream);
-  if (quant_cols_fused(b, ldb, K, N, kind, q, ldq, col_scale, col_scale_inv, st)) return last_status();
+  if (quant_cols_fused(b, ldb, K, N, kind, q, ldq, col_scale, col_scale_inv, st)) return VOID_OK;
   if (cudaMemsetAsync(col_scale, 0, (size_t)N * 4, st) != cudaSuccess) return VOID_ERR_CUDA;
   dim3 g1((N + kColBlock - 1) / kColBlock, (K + kRowSlab - 1) / kRowSlab);
-  col_amax_kernel<<<g1, kColBlock, 0, st>>>(b, ldb, K, N, col_scale);
-  col_scale_kernel<<<(N + 255) / 256, 256, 0, st>>>(col_scale, col_scale_inv, N, kind);
-  quant_pass(b, ldb, K, N, kind, q, ldq, col_scale, 1, st);
-  return last_status();
+  Launches on(st);
+  on.run(col_amax_kernel, g1, kColBlock, b, ldb, K, N, col_scale);
+  on.run(col_scale_kernel, (unsigned)((N + 255) / 256), 256, col_scale, col_scale_inv, N, kind);
+  quant_pass(b, ldb, K, N, kind, q, ldq, col_scale, 1, on);
+  return on.status();
 }
 
 int void_quant_i8_tensor(const float* b, int64_t ldb, int32_t K, int32_t N, void* q, int64_t ldq, float* scale,
@@ -1413,10 +1379,11 @@ int void_quant_i8_tensor(const float* b, int64_t ldb, int32_t K, int32_t N, void
   if (ldb < N || ldq < N) return VOID_ERR_SHAPE;
   if (K > 65535 * kRowSlab) return VOID_ERR_TOO_LARGE;
   dim3 g1((N + kColBlock - 1) / kColBlock, (K + kRowSlab - 1) / kRowSlab);
-  tensor_amax_kernel<<<g1, kColBlock, 0, st>>>(b, ldb, K, N, scale);
-  col_scale_kernel<<<1, 32, 0, st>>>(scale, nullptr, 1, VOID_KIND_I8);
-  quant_pass(b, ldb, K, N, VOID_KIND_I8, q, ldq, scale, 0, st);
-  return last_status();
+  Launches on(st);
+  on.run(tensor_amax_kernel, g1, kColBlock, b, ldb, K, N, scale);
+  on.run(col_scale_kernel, 1, 32, scale, nullptr, 1, VOID_KIND_I8);
+  quant_pass(b, ldb, K, N, VOID_KIND_I8, q, ldq, scale, 0, on);
+  return on.status();
 }
 
 int64_t void_streamk_table_capacity(int64_t nnz, int32_t nbr) {
@@ -1442,11 +1409,11 @@ int void_streamk_table(const int32_t* row_ptr, int32_t nbr, int64_t nnz, int32_t
     return VOID_ERR_BAD_ARG;
   const int target = void_streamk_target(nnz, n_workers_req, max_work);
   if (target <= 0) return VOID_ERR_BAD_ARG;
-  cudaStream_t st = as_stream(stream);
-  streamk_offsets_kernel<<<1, 1024, 0, st>>>(row_ptr, nbr, target, ws, n_workers_out);
-  streamk_fill_kernel<<<(nbr + 255) / 256, 256, 0, st>>>(row_ptr, nbr, target, ws, worker_rows, worker_block_start,
-                                                        worker_block_end, worker_needs_atomic);
-  return last_status();
+  Launches on(as_stream(stream));
+  on.run(streamk_offsets_kernel, 1, 1024, row_ptr, nbr, target, ws, n_workers_out);
+  on.run(streamk_fill_kernel, (unsigned)((nbr + 255) / 256), 256, row_ptr, nbr, target, ws, worker_rows, worker_block_start, worker_block_end,
+         worker_needs_atomic);
+  return on.status();
 }
 
 }  // extern "C"

@@ -407,10 +407,9 @@ template <int KIND, class C, int TR, int EPI>
 int launch_rowacc(const RowaccLaunch& l) {
   auto kernel = spmm_rowacc_kernel<KIND, C, TR, EPI>;
   if (ensure_smem((const void*)kernel, l.smem_bytes)) return VOID_ERR_CUDA;
-  if constexpr ((EPI & kStaged) != 0) launch_pdl(kernel, l.grid, C::THREADS, l.smem_bytes, l.stream, l.b, l.c, l.p);
-  else if constexpr ((EPI & kSplit) != 0) launch_pdl(kernel, l.grid, C::THREADS, l.smem_bytes, l.stream, l.b, l.peers, l.p);
-  else launch_pdl(kernel, l.grid, C::THREADS, l.smem_bytes, l.stream, l.b, Nothing{}, l.p);
-  return VOID_OK;
+  if constexpr ((EPI & kStaged) != 0) return status_of(launch_pdl(kernel, l.grid, C::THREADS, l.smem_bytes, l.stream, l.b, l.c, l.p));
+  else if constexpr ((EPI & kSplit) != 0) return status_of(launch_pdl(kernel, l.grid, C::THREADS, l.smem_bytes, l.stream, l.b, l.peers, l.p));
+  else return status_of(launch_pdl(kernel, l.grid, C::THREADS, l.smem_bytes, l.stream, l.b, Nothing{}, l.p));
 }
 template <int KIND, class C>
 int launch_rowacc(const RowaccLaunch& l) {

@@ -288,7 +288,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
     s.terms = a->tile_terms == 0 ? 1 : a->tile_terms;
     s.a_stable = (a->flags & 4) ? 1 : 0;
     if (s.terms < 1 || s.terms > 3 || (s.terms > 1 && kind != VOID_KIND_F8E4M3)) return VOID_ERR_BAD_ARG;
-    return skinny_launch(s, kind, tr, a->nbr, a->nnz, stream) == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
+    return status_of(skinny_launch(s, kind, tr, a->nbr, a->nnz, stream));
   }
   const int total_panels = (a->N + kPanelN - 1) / kPanelN;
   int np = a->panels_per_item;
@@ -536,7 +536,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
 #define VB_LAUNCH(KERNEL, SHAPE)                                                               \
   do {                                                                                        \
     if (ensure_smem((const void*)KERNEL, smem_bytes)) return VOID_ERR_CUDA;                   \
-    launch_pdl(KERNEL, grid, SHAPE::THREADS, smem_bytes, stream, tmap, p);                    \
+    return status_of(launch_pdl(KERNEL, grid, SHAPE::THREADS, smem_bytes, stream, tmap, p));  \
   } while (0)
   const bool traced = a->trace != nullptr;
   if (!drain) {
@@ -544,11 +544,10 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
     const bool active = split || traced || a->act != VOID_ACT_NONE || a->row_bias != nullptr;
     const int epilogue = (staged ? kStaged : 0) | (split ? kSplit : 0) | (active ? kActive : 0) | (traced ? kTraced : 0);
     const RowaccLaunch l = {shape, a->transposed, epilogue, grid, smem_bytes, stream, tmap, tmap_c, peers, p};
-    const int st = kind == VOID_KIND_I8       ? launch_rowacc<VOID_KIND_I8>(l)
-                   : kind == VOID_KIND_F8E4M3 ? launch_rowacc<VOID_KIND_F8E4M3>(l)
-                   : kind == VOID_KIND_TF32   ? launch_rowacc<VOID_KIND_TF32>(l)
-                                              : launch_rowacc<VOID_KIND_F16>(l);   // fp16 and bf16 differ in the descriptor only
-    if (st != VOID_OK) return st;
+    return kind == VOID_KIND_I8       ? launch_rowacc<VOID_KIND_I8>(l)
+           : kind == VOID_KIND_F8E4M3 ? launch_rowacc<VOID_KIND_F8E4M3>(l)
+           : kind == VOID_KIND_TF32   ? launch_rowacc<VOID_KIND_TF32>(l)
+                                      : launch_rowacc<VOID_KIND_F16>(l);   // fp16 and bf16 differ in the descriptor only
   } else if (kind == VOID_KIND_I8) {
     if (np == 1 && shape == 2) VB_LAUNCH((spmm_drain_kernel<VOID_KIND_I8, 1, Slim>), Slim);
     else if (np == 1 && shape == 3) VB_LAUNCH((spmm_drain_kernel<VOID_KIND_I8, 1, Slim3>), Slim3);
@@ -571,7 +570,6 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
     else VB_LAUNCH((spmm_drain_kernel<VOID_KIND_F8E4M3, 4, Wide>), Wide);
   }
 #undef VB_LAUNCH
-  return cudaGetLastError() == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -640,8 +638,7 @@ extern "C" {
 int void_launch_floor(int32_t grid, int32_t threads, int32_t smem_bytes, void_stream_t stream) {
   if (grid < 1 || threads < 32 || threads > 1024 || smem_bytes < 0) return VOID_ERR_BAD_ARG;
   if (vb::ensure_smem((const void*)vb::floor_kernel, smem_bytes)) return VOID_ERR_CUDA;
-  vb::launch_pdl(vb::floor_kernel, grid, threads, smem_bytes, reinterpret_cast<cudaStream_t>(stream));
-  return cudaGetLastError() == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
+  return vb::status_of(vb::launch_pdl(vb::floor_kernel, grid, threads, smem_bytes, reinterpret_cast<cudaStream_t>(stream)));
 }
 
 int void_spmm_i8_static_scratch(const void_spmm_args* args, int32_t n_split_rows, void_stream_t stream) {

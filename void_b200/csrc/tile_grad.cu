@@ -254,8 +254,7 @@ static int launch(const GradParams& p, const CUtensorMap& map_b, const CUtensorM
   if (ensure_smem((const void*)kernel, smem)) return VOID_ERR_CUDA;
   int grid = 2 * sms;
   if (grid > p.n_items) grid = p.n_items;
-  kernel<<<grid, kThreads, smem, st>>>(map_b, map_g, p);
-  return cudaGetLastError() == cudaSuccess ? VOID_OK : VOID_ERR_CUDA;
+  return status_of(launch_kernel(false, kernel, grid, kThreads, smem, st, map_b, map_g, p));
 }
 
 static int tile_grad(const void* grad_out, int64_t ldg, const void* b, int64_t ldb, int M, int K, int N, int kind,
