@@ -457,6 +457,55 @@ def test_large_floating_products_are_exact_on_small_integers(dtype, m, k, n, den
     void.check_device_status()
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,k,n,density,linear", [
+    (94720, 96, 128, 0.9, False), (94721, 96, 65, 0.9, False),                # one panel in all
+    (31580, 300, 384, 0.7, False), (31580, 130, 257, 0.9, False),             # three: one per item, mid and slim CTAs
+    (18950, 300, 640, 0.7, False), (18950, 130, 515, 0.9, False),             # five: one, and two with short rows
+    (31580, 640, 384, 0.95, True), (10530, 300, 1152, 0.7, False)])           # three, transposed; nine: two
+def test_products_with_an_odd_number_of_panels_are_exact_on_small_integers(dtype, m, k, n, density, linear):
+    dense, gen = _integer_matrix(m, k, density, m + n)
+    a = void.dense_to_void(dense.cuda()).to_dtype(dtype)
+    b = torch.randint(-2, 3, (n, k) if linear else (k, n), generator=gen).cuda().to(dtype)
+    ref = b.double() @ dense.cuda().double().t() if linear else dense.cuda().double() @ b.double()
+    y = void.void_linear(a, b) if linear else void.void_spmm(a, b)
+    assert torch.equal(y.double(), ref.to(dtype).double())
+    void.check_device_status()
+
+
+@pytest.mark.parametrize("m,k,n,density,linear", [(131072, 1024, 128, 0.3, False), (32768, 2048, 384, 0.2, False), (131072, 2048, 64, 0.3, True)])
+def test_items_of_two_panels_are_no_slower_than_items_of_one(m, k, n, density, linear):
+    """Where the launch chooses the panels per item (43, 18 and 29 % over the better shape of one panel when an item of two was
+    half empty)."""
+    from void_b200 import _lib, _spmm
+    from void_b200.ops import packed_fp
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    mask = torch.rand(m // 32, k // 32, generator=gen, device="cuda") < density
+    a = void.void_from_block_mask(mask.cpu().numpy(), torch.randn(int(mask.sum()), 32, 32, generator=gen, device="cuda"), shape=(m, k)).to_dtype(torch.float16)
+    p = packed_fp(a, _lib.FP_KIND[torch.float16])
+    b = torch.randn((n, k) if linear else (k, n), generator=gen, device="cuda").half()
+    out = torch.empty((n, m) if linear else (m, n), dtype=torch.float16, device="cuda")
+
+    def time_of(**options):
+        stream, times = torch.cuda.Stream(), []
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            for _ in range(8):
+                _spmm.spmm(p, b, out, scale_mode=_lib.SCALE_ROW_MEAN, transposed=linear, **options)
+        for _ in range(8):
+            begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            begin.record()
+            graph.replay()
+            end.record()
+            end.synchronize()
+            times.append(begin.elapsed_time(end))
+        return min(times)
+
+    one = min(time_of(panels_per_item=1, cta_shape=shape) for shape in (1, 2, 6))
+    assert time_of() < 1.1 * one
+
+
 # ------------------------------------------------------------------------------------------ products behind what prepares B
 @pytest.mark.parametrize("dtype,k,n", [
     (torch.bfloat16, 6880, 333), (torch.bfloat16, 6912, 333), (torch.float32, 64, 33),     # row copies: 1183, 1188 and 3 blocks

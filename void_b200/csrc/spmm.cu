@@ -300,10 +300,17 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   // 16384 rows, N = 2048, 3 / 6 / 13 tiles per row 28.1 24.8, 38.9 36.3, 69.6 61.7; 8192^2, 80 %, N = 2048 117 112; C transposed,
   // 51 tiles 256 231; both transposed, N = 4096, 8192 x 3328 89.4 85.4, 8192 x 6656 156 150.  With B transposed not for rows of
   // up to 16 tiles under forty items per SM (6 tiles 30.9 32.4, 13 tiles 45.2 44.8).
+  // An odd number of panels leaves half of the last item's stages unused: two per item from nine panels on, with short rows (slim
+  // CTAs) from five.  us, one panel and two: one panel in all, 131072 rows, N = 128, 6 / 13 / 19 tiles 22 30, 39 55, 53 78; three, N = 384
+  // 3 / 10 / 13 / 19 tiles 42 44, 75 86, 94 106, 130 148, B transposed 13 tiles 121 154; five, 3 / 10 / 19 tiles 66 61, 120 125, 209 222,
+  // B transposed 10 / 19 tiles 163 159, 289 314; seven, 65536 rows 3 / 19 tiles 49.7 46.9, 153 157; nine, 16384 rows, 13 / 19 tiles 38.4
+  // 37.9, 52.5 51.0.
   const long long row_panels = (long long)a->nbr * total_panels;
   const bool plain = floating && a->cta_shape == 0 && a->segs == nullptr && a->acc_out == nullptr && a->worker_partials == nullptr;
-  const bool two_panels = plain && es == 2 && np == 0 && row_panels >= 20ll * dev.sms &&
-                          (!tr_b || row_panels >= 40ll * dev.sms || a->nnz > 16ll * a->nbr);
+  const bool large16 = plain && es == 2 && np == 0 && row_panels >= 20ll * dev.sms &&
+                       (!tr_b || row_panels >= 40ll * dev.sms || a->nnz > 16ll * a->nbr);
+  const bool slim_rows = a->nnz < (tr_b ? 10ll : 5ll) * a->nbr;   // of large 16-bit products
+  const bool two_panels = large16 && (total_panels % 2 == 0 || total_panels >= (slim_rows ? 5 : 9));
   if (np == 0 && floating) np = two_panels ? 2 : 1;
   if (np == 0) {
     // two panels per item keep two CTAs on an SM, which measured faster than four panels with one
@@ -323,8 +330,9 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   // 26.4 20.6, 39.2 37.1, 55.6 52.2; B transposed, N = 1024 6 / 9 / 13 / 20 tiles 19.0 18.4, 21.6 20.2, 25.0 24.8, 33.0 33.6; 2048 rows,
   // N = 1024 (512 items) 9 tiles 7.85 8.03.  32-bit tiles with B transposed, N = 1024, 3 / 6 / 9 / 13 tiles: 22.8 22.3, 27.4 25.5,
   // 33.0 31.9, 41.6 40.9; 2048 rows, N = 512 26 tiles 21.7 22.1.
-  // Between them the mid shape, slim CTAs three to an SM with rings in between: 16-bit products of two panels with rows of 5
-  // tiles and more (10 with B transposed), and 32-bit ones from six items per SM on.  fp32, 8192 rows, wide, slim, mid: N = 512, 3 /
+  // Between them the mid shape, slim CTAs three to an SM with rings in between: large 16-bit products of several panels with rows
+  // of 5 tiles and more (10 with B transposed; one panel per item, N = 384, wide, slim, mid: 32768 rows of 13 / 19 tiles 30.6 29.0
+  // 26.4, 39.0 38.7 36.7, 131072 108 95 94, 143 135 130), and 32-bit ones from six items per SM on.  fp32, 8192 rows, wide, slim, mid: N = 512, 3 /
   // 6 / 13 tiles per row 9.6 9.1 8.4, 12.1 12.4 12.1, 20.6 21.0 20.5; N = 2048 28.9 25.3 24.5, 40.1 37.9 37.6, 73.1 70.9 65.6; 20 tiles
   // 101 to 105 in all; B transposed, N = 2048, 6 / 9 / 13 / 20 tiles 52.4 48.1 50.1, 67.6 60.4 63.2, 86.3 79.7 77.8, 116 104 104.  With 512
   // items it holds one and a half per CTA: 4096^2, 90 %, N = 512 12.1 13.0 13.9.
@@ -340,7 +348,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
     else if (tr_b) short_row = 10;
   }
   const bool short_rows = a->nnz <= short_row * a->nbr;
-  if (plain && np == 2 && two_panels) shape = a->nnz >= (tr_b ? 10ll : 5ll) * a->nbr ? 6 : 2;
+  if (large16 && total_panels > 1) shape = slim_rows ? 2 : 6;
   if (plain && np == 1 && es == 4 && n_items > 6ll * dev.sms && !(tr_b && short_rows)) shape = 6;
   if (shape == 0) shape = (!drain && np <= 2) ? ((floating && np == 1 && a->segs == nullptr && !short_rows) ? 1 : 2) : ((drain && np == 1) ? kDefaultDrainShape : 1);
   if (shape == 2 && (np > 2 || (drain && np > 1))) return VOID_ERR_BAD_ARG;
