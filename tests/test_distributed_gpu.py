@@ -149,6 +149,79 @@ def test_in_kernel_reduction_bookkeeping_on_one_gpu(strategy, world, mode):
             assert torch.equal(torch.cat(parts), full), (strategy, world, out_dtype, order, mode)
 
 
+def _one_rank_launch(q, bq, bs, out, plan, scratch, owner):
+    """The reducing launch of a single rank with a plan that splits rows: void_spmm_i8 with n_peers = 1."""
+    import ctypes
+    from void_b200 import _lib
+    segs = plan.segs.view(-1, 8).clone()
+    segs[:, 5] = owner
+    p, a = q.packed(), _lib.SpmmArgs()
+    a.tiles, a.tile_cols, a.tile_scales = p.tiles.data_ptr(), p.tile_cols.data_ptr(), p.tile_scales.data_ptr()
+    a.row_ptr, a.row_scale, a.nbr, a.nbc, a.nnz = p.row_ptr.data_ptr(), p.row_scale.data_ptr(), p.nbr, p.nbc, p.nnz
+    a.b, a.ldb, a.K, a.N = bq.data_ptr(), bq.stride(0), q.shape[1], bq.shape[1]
+    a.col_scale, a.b_scale, a.status = bs.data_ptr(), 1.0, _lib.status_word(bq.device).data_ptr()
+    a.out, a.ldc, a.M, a.out_dtype, a.scale_mode = out.data_ptr(), out.stride(0), q.shape[0], _lib.OUT_DTYPE_CODE[out.dtype], _lib.SCALE_ROW_MEAN
+    a.segs, a.cta_seg_ptr, a.n_cta, a.panels_per_item = segs.data_ptr(), plan.cta_seg_ptr.data_ptr(), plan.n_cta, plan.np
+    a.partials_bytes, a.n_peers = scratch[0].numel() * 4, 1
+    a.peer_partials[0], a.peer_counters[0], a.peer_out[0] = scratch[0].data_ptr(), scratch[1].data_ptr(), out.data_ptr()
+    _lib.check(_lib.load().void_spmm_i8(ctypes.byref(a), _lib.stream_ptr(bq.device)), "void_spmm_i8")
+    torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n", [256, 328, 301])                  # 301: rows of C that the copy engine cannot write
+def test_a_sum_over_one_rank_is_the_product(dtype, n):
+    from void_b200 import stream_k
+    from void_b200.reduce import fused_reduce_spmm
+    mask = workloads.zipf_mask(22, 96, 1.5, 80, 14.0, seed=3)
+    mask[5] = False
+    w = workloads.block_sparse(mask, n, seed=3)
+    q = void.quantize_void_tensor(w.a)
+    bq, bs = void.quantize_cols_int8(w.b)
+    want = void.void_spmm_int8(q, bq, bs, out_dtype=dtype)
+    d = void.shard_void_tensor(q, void.ShardingStrategy.COLUMN_WISE, 1, 0)
+    assert torch.equal(fused_reduce_spmm(d, bq, bs, dtype), want)
+    plan = stream_k.stream_k_plan(q, n, void.compute_stream_k_workload(q), n_cta=48)      # rows in several pieces
+    assert plan.n_counters >= 2
+    scratch = torch.zeros_like(plan.partials), torch.zeros_like(plan.counters)
+    for _ in range(2):
+        out = torch.full_like(want, float("nan"))
+        _one_rank_launch(q, bq, bs, out, plan, scratch, 0)
+        void.check_device_status()
+        assert torch.equal(out, want) and not scratch[0].any() and not scratch[1].any()
+    _one_rank_launch(q, bq, bs, torch.empty_like(want), plan, scratch, 1)                # rows of a rank there is not
+    with pytest.raises(void.VoidB200Error, match="does not fit"):
+        void.check_device_status()
+
+
+def test_16_bit_rows_of_a_sum_over_one_rank_leave_in_tiles():
+    """Half the bytes of fp32 results and one store per tile: 0.88 of their time measured, 1.01 with a store per element."""
+    from void_b200.reduce import fused_reduce_spmm
+    mask = workloads.uniform_mask(128, 128, 0.9, seed=4)
+    w = workloads.block_sparse(mask, 512, seed=4)
+    q = void.quantize_void_tensor(w.a)
+    bq, bs = void.quantize_cols_int8(w.b)
+    d = void.shard_void_tensor(q, void.ShardingStrategy.COLUMN_WISE, 1, 0)
+    took = []
+    for dtype in (torch.float16, torch.float32):
+        fused_reduce_spmm(d, bq, bs, dtype)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(40):
+                fused_reduce_spmm(d, bq, bs, dtype)
+        times = []
+        for _ in range(10):
+            begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            begin.record()
+            graph.replay()
+            end.record()
+            end.synchronize()
+            times.append(begin.elapsed_time(end))
+        took.append(min(times))
+    assert took[0] < 0.95 * took[1], took
+
+
 def test_sharded_workload_shape_vs_oracle():
     """The multi-GPU workload's shape (2048 x 2048 block grid at 95 %, N = 1024: eight panels, four chunks and about
     a hundred tiles per tile row): the shard of rank 3 of 8 against the oracle on sampled tile rows, first and last

@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
       if (!whole) {
         const int owner = word_of(seg, 5), ctr = word_of(seg, 7);
         // a split row whose scratch index lies outside what the caller provided is skipped and reported
-        const bool bad_split = nseg > 1 && (ctr < 0 || ctr >= p.ctr_limit || (peers && (unsigned)owner >= (unsigned)p.n_peers));
+        const bool bad_split = nseg > 1 && (ctr < 0 || ctr >= p.ctr_limit || (p.n_peers > 0 && (unsigned)owner >= (unsigned)p.n_peers));
         int32_t *split_partials = p.partials, *counter = p.counters + ctr;
         if constexpr (SPLIT && !STAGED)
           if (peers && !bad_split) {

@@ -386,8 +386,11 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   if (terms > 1 && (kind != VOID_KIND_F8E4M3 || drain || tr)) return VOID_ERR_BAD_ARG;  // FP8 row-accumulate only
   // 16-bit outputs of the slim row-accumulate kernel leave through a staging tile (32 x 128 x 2 bytes behind the
   // ring) and a tiled TMA store, when C qualifies as a tensor for the copy engine (16-byte aligned base and pitch)
-  // (with a plan, whole-row segments take this route and the pieces of split rows the ordinary one)
-  const bool staged = !drain && !tr && slim && a->acc_out == nullptr && a->n_peers == 0 &&
+  // (with a plan, whole-row segments take this route and the pieces of split rows the ordinary one; a sum over one rank, whose
+  // rows are all whole or this GPU's, is a product with a plan: fp16 4096^2, 90 %, N = 512 7.6 us, 8.7 with direct stores,
+  // 16384 x 4096, N = 1024 24.8 and 27.5)
+  const bool one_rank = a->n_peers == 1 && a->peer_slots == 0 && a->peer_out[0] == a->out;
+  const bool staged = !drain && !tr && slim && a->acc_out == nullptr && (a->n_peers == 0 || one_rank) &&
                          a->worker_partials == nullptr && (a->flags & 2) == 0 &&
                          (a->out_dtype == VOID_OUT_F16 || a->out_dtype == VOID_OUT_BF16) &&
                          (reinterpret_cast<uintptr_t>(a->out) & 15u) == 0 && ((a->ldc * 2) & 15) == 0;
@@ -464,6 +467,10 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
       peers.partials[r] = reinterpret_cast<int32_t*>(a->peer_partials[r]);
       peers.counters[r] = a->peer_counters[r];
       peers.out[r] = a->peer_out[r];
+    }
+    if (one_rank) {
+      p.partials = peers.partials[0];
+      p.counters = peers.counters[0];
     }
   }
   p.trace = reinterpret_cast<unsigned long long*>(a->trace);
