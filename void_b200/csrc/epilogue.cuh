@@ -81,7 +81,7 @@ __device__ __forceinline__ void row_bias_activation(const OutDesc& o, int r0, f3
     const int rows = o.M - r0;  // rows left below r0
 #pragma unroll
     for (int k = 0; k < PAIRS; ++k)
-      x[k] = add2(x[k], pair(2 * k < rows ? __ldg(o.row_bias + r0 + 2 * k) : 0.0f, 2 * k + 1 < rows ? __ldg(o.row_bias + r0 + 2 * k + 1) : 0.0f));
+      x[k] = add2(x[k], pair(2 * k < rows ? o.row_bias[r0 + 2 * k] : 0.0f, 2 * k + 1 < rows ? o.row_bias[r0 + 2 * k + 1] : 0.0f));
   }
   activate<PAIRS>(x, o.act);
 }
@@ -221,7 +221,7 @@ __device__ __forceinline__ void finish_fragments(const OutDesc& o, int r0, const
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       const int r = r0 + 8 * g + 2 * (lane & 3);
-      const f32x2 rb = pair(r < o.M ? __ldg(o.row_bias + r) : 0.0f, r + 1 < o.M ? __ldg(o.row_bias + r + 1) : 0.0f);
+      const f32x2 rb = pair(r < o.M ? o.row_bias[r] : 0.0f, r + 1 < o.M ? o.row_bias[r + 1] : 0.0f);
 #pragma unroll
       for (int q = 0; q < 4; ++q) x[4 * g + q] = add2(x[4 * g + q], rb);
     }

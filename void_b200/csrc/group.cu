@@ -120,12 +120,12 @@ __global__ void __launch_bounds__(kThreads, kCtas) group_kernel(const __grid_con
     bool ok = true;
     for (int i = blockIdx.x; i < p.n_items && ok; i += gridDim.x) {
       const int g = i / p.n_chunks, chunk = i - g * p.n_chunks;
-      const int s0 = __ldg(p.stage_ptr + g), s1 = __ldg(p.stage_ptr + g + 1);
+      const int s0 = p.stage_ptr[g], s1 = p.stage_ptr[g + 1];
       int s = s0 + ((warp - first) & (kProducers - 1));
-      int rec_next = s < s1 && lane < 8 ? __ldg(p.records + (size_t)s * 8 + lane) : 0;
+      int rec_next = s < s1 && lane < 8 ? p.records[(size_t)s * 8 + lane] : 0;
       for (; s < s1; s += kProducers) {
         const int rec = rec_next;
-        if (s + kProducers < s1 && lane < 8) rec_next = __ldg(p.records + (size_t)(s + kProducers) * 8 + lane);
+        if (s + kProducers < s1 && lane < 8) rec_next = p.records[(size_t)(s + kProducers) * 8 + lane];
         const uint32_t off = (uint32_t)__shfl_sync(0xffffffffu, rec, 0);
         const int meta = __shfl_sync(0xffffffffu, rec, 1);
         const int tiles = meta & 0xff, entries = (meta >> 8) & 0xff;
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kThreads, kCtas) group_kernel(const __grid_con
       bool ok = true;
       for (int i = blockIdx.x; i < p.n_items && ok; i += gridDim.x, ++it) {
         const int g = i / p.n_chunks;
-        const int s0 = __ldg(p.stage_ptr + g), s1 = __ldg(p.stage_ptr + g + 1);
+        const int s0 = p.stage_ptr[g], s1 = p.stage_ptr[g + 1];
         const uint32_t buf = n_buf == 2 ? (it & 1u) : 0u, use = n_buf == 2 ? (it >> 1) : it;
         ok = mbar_wait(smem_u32(&bars.acc_empty[buf]), (use & 1u) ^ 1u, ctl);
         if (!ok) break;
@@ -227,12 +227,12 @@ __global__ void __launch_bounds__(kThreads, kCtas) group_kernel(const __grid_con
       const int g = i / p.n_chunks, chunk = i - g * p.n_chunks;
       const uint32_t buf = n_buf == 2 ? (it & 1u) : 0u, use = n_buf == 2 ? (it >> 1) : it;
       // this lane's row of the group, with what its epilogue needs; scales and biases of the columns
-      const int my_row = lane < p.rows ? __ldg(p.group_rows + g * kMaxGroupRows + lane) : -1;
+      const int my_row = lane < p.rows ? p.group_rows[g * kMaxGroupRows + lane] : -1;
       int my_has = 0;
       float my_scale = 1.0f;
       if (my_row >= 0) {
-        my_has = __ldg(p.row_ptr + my_row + 1) > __ldg(p.row_ptr + my_row) ? 1 : 0;
-        if (p.row_scale != nullptr && my_has) my_scale = __ldg(p.row_scale + my_row);
+        my_has = p.row_ptr[my_row + 1] > p.row_ptr[my_row] ? 1 : 0;
+        if (p.row_scale != nullptr && my_has) my_scale = p.row_scale[my_row];
       }
       // one thread waits and the named barrier passes its verdict on: eight polling warps slow the MMA warp down
       if (threadIdx.x == 32 * kEpiWarp0) ok_s[it & 1u] = mbar_wait(smem_u32(&bars.acc_full[buf]), use & 1u, ctl) ? 1 : 0;
@@ -242,8 +242,8 @@ __global__ void __launch_bounds__(kThreads, kCtas) group_kernel(const __grid_con
       const int n = chunk * kPanelN + quad * 32 + lane;
       float cs = p.b_scale, bias = 0.0f;
       if (n < od.N) {
-        if (p.col_scale != nullptr) cs *= __ldg(p.col_scale + n);
-        if (p.bias != nullptr) bias = __ldg(p.bias + n);
+        if (p.col_scale != nullptr) cs *= p.col_scale[n];
+        if (p.bias != nullptr) bias = p.bias[n];
       }
 #pragma unroll 1
       for (int r = 0; r < p.rows; ++r) {

@@ -189,7 +189,7 @@ __device__ __forceinline__ Seg load_seg(const SpmmParams& p, int i) {
   Seg s;
   if (PLAN && p.segs != nullptr) {
     const int4* q = reinterpret_cast<const int4*>(p.segs) + 2 * (size_t)i;
-    const int4 a = __ldg(q), b = __ldg(q + 1);
+    const int4 a = q[0], b = q[1];
     s.row = a.x; s.chunk = a.y; s.t0 = a.z; s.t1 = a.w;
     s.nseg = b.x; s.slot0 = b.y; s.my_idx = b.z; s.ctr = b.w;
   } else {
@@ -197,11 +197,11 @@ __device__ __forceinline__ Seg load_seg(const SpmmParams& p, int i) {
     p.passes.item(i, k, s.chunk);
     s.row = k;
     if (p.row_order != nullptr) {
-      const int r = __ldg(p.row_order + k);
+      const int r = p.row_order[k];
       s.row = r < 0 ? 0 : (r >= p.nbr ? p.nbr - 1 : r);
     }
-    s.t0 = __ldg(p.row_ptr + s.row);
-    s.t1 = __ldg(p.row_ptr + s.row + 1);
+    s.t0 = p.row_ptr[s.row];
+    s.t1 = p.row_ptr[s.row + 1];
     s.nseg = 1; s.slot0 = 0; s.my_idx = 0; s.ctr = 0;
   }
   return s;
@@ -210,15 +210,15 @@ __device__ __forceinline__ Seg load_seg(const SpmmParams& p, int i) {
 // The same for a warp that waits with many values in registers: lane k holds word k (in the order of Seg's fields).
 template <bool PLAN>
 __device__ __forceinline__ int load_seg_word(const SpmmParams& p, int i, int lane) {
-  if (PLAN && p.segs != nullptr) return lane < 8 ? __ldg(p.segs + 8 * (size_t)i + lane) : 0;
+  if (PLAN && p.segs != nullptr) return lane < 8 ? p.segs[8 * (size_t)i + lane] : 0;
   int k, chunk;
   p.passes.item(i, k, chunk);
   int row = k;
   if (p.row_order != nullptr) {
-    const int r = __ldg(p.row_order + k);
+    const int r = p.row_order[k];
     row = r < 0 ? 0 : (r >= p.nbr ? p.nbr - 1 : r);
   }
-  if (lane == 2 || lane == 3) return __ldg(p.row_ptr + row + lane - 2);
+  if (lane == 2 || lane == 3) return p.row_ptr[row + lane - 2];
   return lane == 0 ? row : (lane == 1 ? chunk : (lane == 4 ? 1 : 0));
 }
 __device__ __forceinline__ int word_of(int words, int k) { return __shfl_sync(0xffffffffu, words, k); }
@@ -227,8 +227,8 @@ __device__ __forceinline__ int word_of(int words, int k) { return __shfl_sync(0x
 template <bool PLAN>
 __device__ __forceinline__ void seg_range(const SpmmParams& p, int& begin, int& end, int& step) {
   if (PLAN && p.segs != nullptr) {
-    begin = __ldg(p.cta_seg_ptr + blockIdx.x);
-    end = __ldg(p.cta_seg_ptr + blockIdx.x + 1);
+    begin = p.cta_seg_ptr[blockIdx.x];
+    end = p.cta_seg_ptr[blockIdx.x + 1];
     step = 1;
   } else {
     begin = blockIdx.x;
@@ -315,7 +315,7 @@ __device__ __forceinline__ void producer_loop(const SpmmParams& p, const CUtenso
       cs = (cs + 1 == S) ? 0 : cs + 1;
     }
     int col = 0;
-    if (ct + lane < s.t1 && lane < stage_cap(p, cs)) col = __ldg(p.tile_cols + ct + lane);
+    if (ct + lane < s.t1 && lane < stage_cap(p, cs)) col = p.tile_cols[ct + lane];
     if (TRACE && i == begin && pw == 0 && lane == 0) {
       asm volatile("" ::"r"(col) : "memory");
       stamp<TRACE>(p, 58);   // the first block columns have arrived
@@ -332,7 +332,7 @@ __device__ __forceinline__ void producer_loop(const SpmmParams& p, const CUtenso
           ns = (ns + 1 == S) ? 0 : ns + 1;
         }
         int col_next = 0;
-        if (nt + lane < s.t1 && lane < stage_cap(p, ns)) col_next = __ldg(p.tile_cols + nt + lane);
+        if (nt + lane < s.t1 && lane < stage_cap(p, ns)) col_next = p.tile_cols[nt + lane];
         const uint32_t full = smem_u32(&bars->full[stage]);
         const uint32_t sbase = ring_base + (uint32_t)stage * stage_bytes;
         // test hook: the first group of the CTA is never delivered, so the consumer's bounded wait runs out

@@ -229,9 +229,8 @@ __device__ __forceinline__ void mean_scale(const RowScales& rows, const TileMeta
   }
   if (lane == 0) rows.row_scale[r] = t1 > t0 ? __fdiv_rn(s, (float)(t1 - t0)) : 0.0f;
 }
-// The kernels of a store's set-up (quantised tiles, index, packing, row order) start when the one before is complete and let the
-// next start when they are: a product packed inside a stream capture follows them without a host's wait in between, and with each
-// let in before the one ahead was through, a first replay was seen to multiply with arrays that had not been written yet.
+// The kernels of a store's set-up (quantised tiles, index, packing, row order) let the next one start when they are through; a
+// product packed inside a stream capture follows them without a host's wait in between.
 __global__ void __launch_bounds__(256) pack_tiles_kernel(const uint4* values, const int32_t* block_indices, int64_t nnz, uint4* packed,
                                                          TileMeta meta, RowScales rows) {
   grid_dependency_wait();
@@ -505,9 +504,8 @@ __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
 }
 // One warp per tile: 1024 values, 32 per lane, read once and in their own type.
 template <int KIND, typename T>
-__global__ void __launch_bounds__(256) quant_tiles_kernel(const T* values, int64_t nnz, uint8_t* __restrict__ q,
-                                                          float* __restrict__ scale_out, float* __restrict__ scale_inv_out,
-                                                          float* __restrict__ amax_out, StoreExtras x) {
+__global__ void __launch_bounds__(256) quant_tiles_kernel(const T* values, int64_t nnz, uint8_t* q, float* scale_out, float* scale_inv_out,
+                                                          float* amax_out, StoreExtras x) {
   const int64_t tile = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   grid_dependency_wait();
@@ -633,10 +631,8 @@ __global__ void __launch_bounds__(128) quant_cols4_kernel(const float* __restric
 constexpr int kFusedThreads = 256, kFusedCtas = 8, kFusedCols = 16;
 constexpr int kFusedSmem = 64 * 1024, kFusedMaxSmem = 208 * 1024;   // several CTAs per SM, one CTA per SM
 template <int KIND, bool VEC>
-__global__ void __launch_bounds__(kFusedThreads) quant_cols_fused_kernel(const float* __restrict__ b, int64_t ldb, int K, int N,
-                                                                         uint8_t* __restrict__ q, int64_t ldq,
-                                                                         float* __restrict__ scale_out,
-                                                                         float* __restrict__ scale_inv_out, int early) {
+__global__ void __launch_bounds__(kFusedThreads) quant_cols_fused_kernel(const float* b, int64_t ldb, int K, int N, uint8_t* q, int64_t ldq,
+                                                                         float* scale_out, float* scale_inv_out, int early) {
   namespace cg = cooperative_groups;
   constexpr int W = kFusedCols;
   constexpr int E = VEC ? 4 : 1;                        // columns a thread owns
@@ -657,7 +653,7 @@ __global__ void __launch_bounds__(kFusedThreads) quant_cols_fused_kernel(const f
   const int k0 = rank * per;
   const int rows = (K - k0) < per ? ((K - k0) > 0 ? K - k0 : 0) : per;
   const uint32_t bytes = n < N ? 4u * E : 0u;           // (N is a multiple of 4 in the vector form); 0: zero fill
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  grid_dependency_wait();
 
   const float* src = b + (size_t)k0 * ldb + (n < N ? n : 0);
   for (int r = r0; r < rows; r += ROWS) {
@@ -761,8 +757,7 @@ template <> __device__ __forceinline__ float as_float<float>(float v) { return v
 template <> __device__ __forceinline__ float as_float<__half>(__half v) { return __half2float(v); }
 template <> __device__ __forceinline__ float as_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(kSumThreads) column_sum_kernel(const T* __restrict__ in, int64_t ld, int rows, int cols,
-                                                                 T* __restrict__ out) {
+__global__ void __launch_bounds__(kSumThreads) column_sum_kernel(const T* in, int64_t ld, int rows, int cols, T* out) {
   namespace cg = cooperative_groups;
   constexpr int E = VEC ? 4 : 1, TPR = kSumCols / E, ROWS = kSumThreads / TPR, WARPS = kSumThreads / 32;
   __shared__ float part[WARPS][kSumCols];
@@ -772,8 +767,8 @@ __global__ void __launch_bounds__(kSumThreads) column_sum_kernel(const T* __rest
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int col = (tid % TPR) * E, c0 = (int)(blockIdx.x / ctas) * kSumCols + col;
   const int per = (rows + ctas - 1) / ctas, r_end = (rank + 1) * per < rows ? (rank + 1) * per : rows;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  grid_dependency_wait();
+  grid_launch_dependents();
   float s[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) s[e] = 0.0f;
@@ -847,11 +842,10 @@ static bool launch_column_sum(const void* in, int64_t ld, int rows, int cols, vo
 // to settle beside, and it may start with them: bf16 GELU 3001 x 5003, N = 333 (821 blocks) 11.7 -> 10.5 us, 4096 x 1111, N = 777
 // 12.9 -> 11.5; started early behind 4032 blocks 47.1 -> 47.4 (fp16 8192^2, 90 %, N = 1001).
 template <typename T>
-__global__ void __launch_bounds__(256) copy_rows_kernel(const T* __restrict__ in, int64_t ld_in, uint4* __restrict__ out,
-                                                        int64_t pieces, int64_t rows, int cols, int early) {
+__global__ void __launch_bounds__(256) copy_rows_kernel(const T* in, int64_t ld_in, uint4* out, int64_t pieces, int64_t rows, int cols, int early) {
   constexpr int E = 16 / (int)sizeof(T);
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  grid_dependency_wait();
   if (early) grid_launch_dependents();
   if (i >= rows * pieces) return;
   const int64_t r = i / pieces;
@@ -868,12 +862,11 @@ __global__ void __launch_bounds__(256) copy_rows_kernel(const T* __restrict__ in
 // rows, and eight of its lanes write one 128-byte row of the result, each collecting its piece from a column of shared
 // memory (rows of 33 words).  Bound by memory: 2048 x 4096 bf16 (17 MB each way) 7.9 us.
 template <typename T>
-__global__ void __launch_bounds__(256) transpose_kernel(const T* __restrict__ in, int64_t ld_in, T* __restrict__ out, int64_t ld_out,
-                                                        int rows, int cols, int whole) {
+__global__ void __launch_bounds__(256) transpose_kernel(const T* in, int64_t ld_in, T* out, int64_t ld_out, int rows, int cols, int whole) {
   constexpr int S = 128 / (int)sizeof(T), V = 16 / (int)sizeof(T), C = 4 / (int)sizeof(T);
   __shared__ uint32_t tile[S][33];
   const int r0 = blockIdx.y * S, c0 = blockIdx.x * S;
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  grid_dependency_wait();
 #pragma unroll
   for (int i = threadIdx.x; i < S * 8; i += 256) {
     const int r = i >> 3, c = i & 7;
@@ -882,7 +875,7 @@ __global__ void __launch_bounds__(256) transpose_kernel(const T* __restrict__ in
     if (r0 + r < rows) {
       const T* src = in + (int64_t)(r0 + r) * ld_in + c0 + c * V;
       if (whole && c0 + (c + 1) * V <= cols) {
-        x.v = __ldg(reinterpret_cast<const uint4*>(src));
+        x.v = *reinterpret_cast<const uint4*>(src);
       } else {
 #pragma unroll
         for (int k = 0; k < V; ++k)
@@ -895,7 +888,7 @@ __global__ void __launch_bounds__(256) transpose_kernel(const T* __restrict__ in
   __syncthreads();
   const int word = threadIdx.x >> 3, first = (threadIdx.x & 7) * V;   // C columns of the tile, V rows of it
   if (r0 + first >= ld_out) return;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  grid_launch_dependents();
   uint32_t w[V], o[C][4];
 #pragma unroll
   for (int k = 0; k < V; ++k) w[k] = tile[first + k][word];

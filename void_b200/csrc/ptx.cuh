@@ -137,6 +137,13 @@ __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.w
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // Programmatic dependent launch: block until the kernel before this one in the stream has completed and its
 // writes are visible; let the kernel after this one begin its own set-up.
+// Such a kernel is resident while the one before it still writes, so every kernel that waits keeps to two rules:
+//  - What an earlier kernel may have written is read behind the wait, by ordinary loads.  No const __restrict__ parameter and no
+//    __ldg: both say that the data do not change while the kernel runs, which is not true here, and let a load move ahead of the
+//    wait or be served from a cache that nothing has refreshed.  (The only explanation that reading has left for a store that was
+//    packed inside a stream capture and multiplied with an index not written yet.)
+//  - The next kernel is let in behind the wait, not ahead of it, so that in a row of small kernels only neighbours overlap.  (Products
+//    let it in at their end.)
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Linear bulk copy global -> shared (16-byte aligned addresses, size a multiple of 16).

@@ -176,13 +176,13 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
       const uint32_t buf = it & 1u, aph = (it >> 1) & 1u;
       const bool has = word_of(seg, 3) > word_of(seg, 2);
       // an empty tile row is zeros (+ bias): nothing to scale, no scales to wait for
-      const float rs = (p.row_scale != nullptr && (has || nseg > 1)) ? __ldg(p.row_scale + row) : 1.0f;
+      const float rs = (p.row_scale != nullptr && (has || nseg > 1)) ? p.row_scale[row] : 1.0f;
       const int n_base = chunk * p.np * kPanelN + quad * 32 + lane;
       // per-column scale and bias of the first panel are fetched before the accumulator is ready
       float cs = p.b_scale, bias = 0.0f;
       if (n_base < p.N) {
-        if (p.col_scale != nullptr && (has || nseg > 1)) cs = __ldg(p.col_scale + n_base) * p.b_scale;
-        if (p.bias != nullptr) bias = __ldg(p.bias + n_base);
+        if (p.col_scale != nullptr && (has || nseg > 1)) cs = p.col_scale[n_base] * p.b_scale;
+        if (p.bias != nullptr) bias = p.bias[n_base];
       }
       // one thread waits, the named barrier hands its verdict to all epilogue warps, so that they
       // leave the loop together if the wait gave up (a warp that went on alone would wait at the next
@@ -212,8 +212,8 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
           const int n = n_base + q * kPanelN;
           float csq = p.b_scale, biasq = 0.0f;
           if (!STAGED && n < p.N) {
-            if (p.col_scale != nullptr) csq = __ldg(p.col_scale + n) * p.b_scale;
-            if (p.bias != nullptr) biasq = __ldg(p.bias + n);
+            if (p.col_scale != nullptr) csq = p.col_scale[n] * p.b_scale;
+            if (p.bias != nullptr) biasq = p.bias[n];
           }
           // all columns of the panel with one wait, then the accumulator buffer goes back to the MMA warp
           uint32_t ra[C::COLS];
@@ -304,8 +304,8 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
         if (q > 0) {
           csq = p.b_scale; biasq = 0.0f;
           if (n < p.N) {
-            if (p.col_scale != nullptr) csq = __ldg(p.col_scale + n) * p.b_scale;
-            if (p.bias != nullptr) biasq = __ldg(p.bias + n);
+            if (p.col_scale != nullptr) csq = p.col_scale[n] * p.b_scale;
+            if (p.bias != nullptr) biasq = p.bias[n];
           }
         }
         if constexpr (STAGED) {

@@ -70,12 +70,12 @@ template <int ES>
 __device__ __forceinline__ void load_a(const uint8_t* tile, int rg, int g, int t, uint32_t (&w)[2 * ES]) {
   const uint8_t* p = tile + rg * (256 * ES);
   if constexpr (ES == 1) {
-    const uint2 v = __ldg(reinterpret_cast<const uint2*>(p + (t >> 1) * 128 + g * 16 + (t & 1) * 8));
+    const uint2 v = *reinterpret_cast<const uint2*>(p + (t >> 1) * 128 + g * 16 + (t & 1) * 8);
     w[0] = v.x; w[1] = v.y;
   } else {
 #pragma unroll
     for (int h = 0; h < ES / 2; ++h) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(p + (h * 4 + t) * 128 + g * 16));
+      const uint4 v = *reinterpret_cast<const uint4*>(p + (h * 4 + t) * 128 + g * 16);
       w[4 * h] = v.x; w[4 * h + 1] = v.y; w[4 * h + 2] = v.z; w[4 * h + 3] = v.w;
     }
     order_words<ES>(w);
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(512) skinny_kernel(const __grid_constant__ Ski
   const int g = lane >> 2, t = lane & 3;
   const int row = blockIdx.x, n0 = blockIdx.y * NB;
   if (!p.a_stable) grid_dependency_wait();
-  const int t0 = __ldg(p.row_ptr + row), t1 = __ldg(p.row_ptr + row + 1);
+  const int t0 = p.row_ptr[row], t1 = p.row_ptr[row + 1];
   T d[2][NG][4];
 #pragma unroll
   for (int h = 0; h < 2; ++h)
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(512) skinny_kernel(const __grid_constant__ Ski
   const int terms = KIND == VOID_KIND_F8E4M3 ? p.terms : 1;
   const uint8_t* b = p.b;
   int cols = 0;    // block columns of this warp's next 32 tiles, one per lane
-  if (t0 + warp + lane * warps < t1) cols = __ldg(p.tile_cols + t0 + warp + lane * warps);
+  if (t0 + warp + lane * warps < t1) cols = p.tile_cols[t0 + warp + lane * warps];
   if (p.a_stable) grid_dependency_wait();
   int seen = 0;
 #pragma unroll 2
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(512) skinny_kernel(const __grid_constant__ Ski
     if (seen == 32) {
       seen = 0;
       cols = 0;
-      if (tile + lane * warps < t1) cols = __ldg(p.tile_cols + tile + lane * warps);
+      if (tile + lane * warps < t1) cols = p.tile_cols[tile + lane * warps];
     }
     const int k0 = __shfl_sync(0xffffffffu, cols, seen) * 32;
     uint32_t bw[NG][2 * ES];
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(512) skinny_kernel(const __grid_constant__ Ski
         mine[m * PITCH + (TR ? 8 * i + j : NG * j + i)] = d[h][i][e];
       }
   __syncthreads();
-  const float rs = p.row_scale != nullptr && t1 > t0 ? __ldg(p.row_scale + row) : 1.0f;
+  const float rs = p.row_scale != nullptr && t1 > t0 ? p.row_scale[row] : 1.0f;
   for (int o = threadIdx.x; o < 32 * NB; o += blockDim.x) {
     if (!ACT || o >= (int)blockDim.x) x = output(o);
     if (!x.in) continue;
