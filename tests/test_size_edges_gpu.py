@@ -307,6 +307,49 @@ def test_two_layers_are_exact_on_small_integers(dtype, m, k, n, density=0.3):
 
 
 # ------------------------------------------------------------------------------------------ groups of tile rows
+def test_two_layers_ask_the_interpreter_for_little_and_notice_every_change():
+    """Calls the interpreter makes for a pass of two packed layers (17; 25 when every check was its own), and
+    what such a pass must not overlook: edited and replaced weights, operands of another shape, type or length."""
+    import sys
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    layer = lambda m, k: void.dense_to_void(torch.randint(-2, 3, (m, k), generator=gen, device="cuda").half())
+    w1, w2 = layer(128, 96), layer(64, 128)
+    x = torch.randint(-2, 3, (8, 96), generator=gen, device="cuda").half()
+    b1, b2 = (torch.randint(-2, 3, (m,), generator=gen, device="cuda").float() for m in (128, 64))
+
+    def same(x, b1, b2):
+        ref = (x.double() @ w1.to_dense().double().t() + (0 if b1 is None else b1.double())).clamp(min=0).to(x.dtype).double()
+        ref = (ref @ w2.to_dense().double().t() + (0 if b2 is None else b2.double())).to(x.dtype)
+        return torch.equal(void.fused_sparse_mlp(x, w1, w2, "relu", b1, b2), ref)
+
+    assert same(x, b1, b2) and same(x, b1, b2) and same(x, None, b2) and same(x, b1, None)
+    calls = [0]
+
+    def count(frame, event, arg):
+        calls[0] += event in ("call", "c_call")
+
+    sys.setprofile(count)
+    void.fused_sparse_mlp(x, w1, w2, "gelu", b1, b2)
+    sys.setprofile(None)
+    assert calls[0] <= 20, calls[0]
+    w1.values[0, 0, 0] += 1                                                     # edited
+    assert same(x, b1, b2)
+    w2.values = w2.values * -1                                                  # replaced
+    assert same(x, b1, b2) and same(x, b1, b2)
+    assert same(x.reshape(2, 4, 96), b1, b2) and same(x[:, :].t().contiguous().t(), b1, b2)
+    w32 = w1.to_dtype(torch.float32)                                            # types that differ
+    assert torch.equal(void.fused_sparse_mlp(x, w32, w2, "none"), void.void_linear(w2, void.void_linear(w32, x)))
+    with torch.inference_mode():                                                # nothing has a version: packed every time
+        w1.values = w1.values * 1
+        assert same(x, b1, b2)
+        w1.values[0, 0, 1] += 1
+        assert same(x, b1, b2)
+    for bad in ((x[:, :64], b1, b2), (x, b1[:100], b2), (x, b1, b2[:32]), (x.cpu(), b1, b2)):
+        with pytest.raises((AssertionError, RuntimeError, ValueError)):
+            void.fused_sparse_mlp(bad[0], w1, w2, "relu", *bad[1:])
+    void.check_device_status()
+
+
 @pytest.mark.parametrize("kind,dtype,out", [("I8", torch.int8, torch.float32), ("I8", torch.int8, torch.float16),
                                             ("I8", torch.int8, torch.bfloat16), ("F16", torch.float16, torch.float16),
                                             ("BF16", torch.bfloat16, torch.bfloat16), ("TF32", torch.float32, torch.float32)])

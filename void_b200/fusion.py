@@ -20,7 +20,7 @@ from . import _lib
 from .format import VOIDTensor
 from .fp8 import FP8VOIDTensor, void_spmm_fp8
 from .int_quant import Int8VOIDTensor, void_spmm_int8
-from .ops import _KIND_DTYPE, packed_fp, product_kind, void_linear, void_spmm
+from .ops import _KIND_DTYPE, cached_fp, packed_fp, product_kind, void_linear, void_spmm
 
 
 class FusedOpType(Enum):
@@ -42,12 +42,14 @@ class ActivationType(Enum):
     SIGMOID = "sigmoid"
 
 
+_ACTIVATION_CODES = {"none": 0, "relu": 1, "gelu": 2, "silu": 3, "swish": 3, "tanh": 4, "sigmoid": 5}
+
+
 def get_activation_code(activation: Union[str, ActivationType]) -> int:
     """Integer code of an activation name, same table as void/fusion.py:77-91."""
     if isinstance(activation, ActivationType):
         activation = activation.value
-    codes = {"none": 0, "relu": 1, "gelu": 2, "silu": 3, "swish": 3, "tanh": 4, "sigmoid": 5}
-    return codes.get(activation.lower(), 0)
+    return _ACTIVATION_CODES.get(activation.lower(), 0)
 
 
 def _void_spmm_activation(a, b, bias, out, activation: str, **kw) -> torch.Tensor:
@@ -114,6 +116,14 @@ def fused_sparse_mlp(x: torch.Tensor, w1: VOIDTensor, w2: VOIDTensor, activation
     code = get_activation_code(activation)
     if code > _lib.ACT_SILU:
         raise NotImplementedError("activation %r is not fused on B200 (none, relu, gelu, silu are)" % activation)
+    if isinstance(w1, VOIDTensor) and isinstance(w2, VOIDTensor):
+        kind = _lib.FP_KIND.get(x.dtype)
+        p1, p2 = cached_fp(w1, kind), cached_fp(w2, kind)
+        if p1 is not None and p2 is not None:       # None: one of the checks that follow says why
+            y = _lib.native().mlp_packed(p1.native, w1.values, w1.block_rows, w1.block_cols, w1.shape, p2.native, w2.values, w2.block_rows,
+                                         w2.block_cols, w2.shape, x, bias1, code, bias2)
+            if y is not None:
+                return y
     if isinstance(w1, VOIDTensor) and isinstance(w2, VOIDTensor) and x.is_cuda and x.dtype in _lib.OUT_DTYPE_CODE:
         kind, (m1, k1), (m2, k2) = product_kind(w1, x), w1.shape, w2.shape
         if (_KIND_DTYPE[kind] is x.dtype and product_kind(w2, x) == kind and x.dim() >= 2 and x.shape[-1] == k1 and m1 == k2

@@ -29,6 +29,12 @@ def product_kind(a: VOIDTensor, b: torch.Tensor) -> int:
     return _lib.KIND_TF32
 
 
+def cached_fp(a: VOIDTensor, kind) -> Optional[_spmm.PackedTiles]:
+    """The packed copy for ``kind`` that the tensor keeps, whether it is still current or not."""
+    cache = a.__dict__.get("_packed_fp_cache")
+    return None if cache is None else cache.get(kind)
+
+
 def packed_fp(a: VOIDTensor, kind: int) -> _spmm.PackedTiles:
     """Packed copy of a floating VOIDTensor for ``kind`` (built once per kind, cached on the tensor)."""
     cache = a.__dict__.get("_packed_fp_cache")
