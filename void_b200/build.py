@@ -103,7 +103,8 @@ def build(force=False, verbose=False):
         host_obj = os.path.join(tmp, "host.o")
         _run_all([[_nvcc()] + NVCC_FLAGS + extra + ["-c", os.path.join(CSRC, s), "-o", o] for s, o in zip(srcs, objs)]
                  + [_host_compile(host_obj)], verbose)
-        _run_all([[_nvcc()] + NVCC_FLAGS + ["-shared", "-o", LIB_PATH] + objs], verbose)
+        # (by name, so that the host path finds the library beside it, not the place where both were linked)
+        _run_all([[_nvcc()] + NVCC_FLAGS + ["-shared", "-Xlinker", "-soname=" + os.path.basename(LIB_PATH), "-o", LIB_PATH] + objs], verbose)
         _run_all([_host_link(host_obj)], verbose)
     for f in os.listdir(LIB_DIR):    # host paths of earlier sources
         if f.startswith("_native") and f.endswith(".so") and f != os.path.basename(native_path()):
