@@ -28,9 +28,9 @@ struct Nothing {};
 template <int EPI>
 using ExtraOf = std::conditional_t<(EPI & kStaged) != 0, CUtensorMap, std::conditional_t<(EPI & kSplit) != 0, PeerParams, Nothing>>;
 
-// TR: 1 = B and C transposed ([N, K] and [N, M]), 2 = C alone.  EPI: what the epilogue is asked for (kStaged ...).  One kernel
-// that could do all of it took 6.83 us for a launch that runs in 5.46 without activations and in 5.67 with them (INT8 4096^2,
-// 90 %, N = 512, fp16 results): what is not run costs too, in spilled registers and in instructions fetched around it.
+// TR: 1 = B and C transposed ([N, K] and [N, M]), 2 = C alone.  EPI: what the epilogue is asked for (kStaged ...).  What is not run
+// costs a little too, in spilled registers and in instructions fetched around it: INT8 4096^2, 90 %, N = 512, fp16 results 6.10 us,
+// through the kernel that also splits rows and activates 6.20; with GELU 6.57, through that kernel 6.60.
 template <int KIND, class C, int TR, int EPI>
 __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel(const __grid_constant__ CUtensorMap tmap_b,
                                                                                  const __grid_constant__ ExtraOf<EPI> x,
