@@ -77,7 +77,6 @@ __global__ void __launch_bounds__(kThreads, kCtas) group_kernel(const __grid_con
   __shared__ Bars bars;
   __shared__ uint32_t tmem_base_s;
   __shared__ int ctl_s[2];   // abort flag, wait limit in ms
-  __shared__ int ok_s[2];
   constexpr int ES = Elem<KIND>::ES;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -132,16 +131,13 @@ __global__ void __launch_bounds__(kThreads, kCtas) group_kernel(const __grid_con
         const int col = __shfl_sync(0xffffffffu, rec, 2 + (lane < kMaxEntries ? lane : 0));
         const uint32_t full = smem_u32(&bars.full[slot]), base = ring + (uint32_t)slot * (uint32_t)p.stage_bytes;
         const uint32_t blob_bytes = (uint32_t)(kHeaderBytes + tiles * kTileBytes * ES);
-        int fine = 1;
+        ok = mbar_wait_warp(smem_u32(&bars.empty[slot]), phase ^ 1u, ctl);
+        if (!ok) break;
         if (lane == 0) {
-          fine = mbar_wait(smem_u32(&bars.empty[slot]), phase ^ 1u, ctl) ? 1 : 0;
-          if (fine) {
-            mbar_expect_tx(full, blob_bytes + (uint32_t)(entries * kPanelBytes * ES));
-            bulk_load(base + (uint32_t)p.panel_bytes, p.blob + (size_t)off * 128, blob_bytes, full);
-          }
+          mbar_expect_tx(full, blob_bytes + (uint32_t)(entries * kPanelBytes * ES));
+          bulk_load(base + (uint32_t)p.panel_bytes, p.blob + (size_t)off * 128, blob_bytes, full);
         }
-        fine = __shfl_sync(0xffffffffu, fine, 0);
-        if (!fine) { ok = false; break; }
+        __syncwarp();
         if (!waited) {   // B may be the output of the previous kernel
           grid_dependency_wait();
           waited = true;
@@ -234,10 +230,7 @@ __global__ void __launch_bounds__(kThreads, kCtas) group_kernel(const __grid_con
         my_has = p.row_ptr[my_row + 1] > p.row_ptr[my_row] ? 1 : 0;
         if (p.row_scale != nullptr && my_has) my_scale = p.row_scale[my_row];
       }
-      // one thread waits and the named barrier passes its verdict on: eight polling warps slow the MMA warp down
-      if (threadIdx.x == 32 * kEpiWarp0) ok_s[it & 1u] = mbar_wait(smem_u32(&bars.acc_full[buf]), use & 1u, ctl) ? 1 : 0;
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
-      if (!ok_s[it & 1u]) break;
+      if (!mbar_wait_warp(smem_u32(&bars.acc_full[buf]), use & 1u, ctl)) break;
       tc_fence_after();
       const int n = chunk * kPanelN + quad * 32 + lane;
       float cs = p.b_scale, bias = 0.0f;

@@ -339,17 +339,13 @@ __device__ __forceinline__ void producer_loop(const SpmmParams& p, const CUtenso
         const uint32_t sbase = ring_base + (uint32_t)stage * stage_bytes;
         // test hook: the first group of the CTA is never delivered, so the consumer's bounded wait runs out
         const bool drop = p.drop_group != 0 && gcount == 0;
-        int ok = 1;
-        if (lane == 0) {
-          ok = mbar_wait(smem_u32(&bars->empty[stage]), phase ^ 1u, ctl) ? 1 : 0;
-          if (ok && !drop) {
-            mbar_expect_tx(full, unit_bytes * (uint32_t)gcnt);
-            bulk_load(sbase + tile_off<ES>(p, cap, 0), p.tiles + (size_t)t * (size_t)(kTileBytes * ES * p.terms),
-                      (uint32_t)(gcnt * p.terms) * (kTileBytes * ES), full);
-          }
+        if (!mbar_wait_warp(smem_u32(&bars->empty[stage]), phase ^ 1u, ctl)) return;
+        if (lane == 0 && !drop) {
+          mbar_expect_tx(full, unit_bytes * (uint32_t)gcnt);
+          bulk_load(sbase + tile_off<ES>(p, cap, 0), p.tiles + (size_t)t * (size_t)(kTileBytes * ES * p.terms),
+                    (uint32_t)(gcnt * p.terms) * (kTileBytes * ES), full);
         }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) return;
+        __syncwarp();
         if (TRACE && i == begin && pw == 0 && lane == 0 && k == 0) stamp<TRACE>(p, 59);   // tiles of the first group requested
         if (!waited) {  // B may be the output of the previous kernel
           grid_dependency_wait();

@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
         if (i + step < end) seg_next = load_seg<SPLIT>(p, i + step);
         const int npan = panels_in_chunk(p, s.chunk);
         const uint32_t buf = it & 1u, aph = (it >> 1) & 1u;
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.acc_empty[buf]), aph ^ 1u, ctl));
+        ok = mbar_wait_warp(smem_u32(&bars.acc_empty[buf]), aph ^ 1u, ctl);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d0 = tmem_base + buf * acc_cols;
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
           const int gcnt = (s.t1 - t) < cap ? (s.t1 - t) : cap;
           t += gcnt;
           if (TRACE && leader && i == begin && gidx < 8) stamp<TRACE>(p, 48 + gidx);
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.full[stage]), phase, ctl));
+          ok = mbar_wait_warp(smem_u32(&bars.full[stage]), phase, ctl);
           if (!ok) break;
           if (TRACE && leader && i == begin && gidx < 12) stamp<TRACE>(p, 16 + gidx);   // slots 28 .. 31: last arriver of a split row
           tc_fence_after();
@@ -184,10 +184,13 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
         if (p.col_scale != nullptr && (has || nseg > 1)) cs = p.col_scale[n_base] * p.b_scale;
         if (p.bias != nullptr) bias = p.bias[n_base];
       }
-      // one thread waits, the named barrier hands its verdict to all epilogue warps, so that they
+      // one warp waits, the named barrier hands its verdict to all epilogue warps, so that they
       // leave the loop together if the wait gave up (a warp that went on alone would wait at the next
       // named barrier for ever)
-      if (epi_tid == 0) ok_s[it & 1u] = mbar_wait(smem_u32(&bars.acc_full[buf]), aph, ctl) ? 1 : 0;
+      if (epi_tid < 32) {
+        const bool in = mbar_wait_warp(smem_u32(&bars.acc_full[buf]), aph, ctl);
+        if (epi_tid == 0) ok_s[it & 1u] = in ? 1 : 0;
+      }
       asm volatile("bar.sync 1, %0;" ::"n"(C::EPI_THREADS) : "memory");
       if (!ok_s[it & 1u]) break;
       if (epi_tid == 0 && i == begin) stamp<TRACE>(p, 5);

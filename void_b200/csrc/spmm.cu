@@ -67,9 +67,9 @@ __global__ void __launch_bounds__(C::THREADS, (NP == 4) ? 1 : C::CTAS_PER_SM) sp
         const int npan = panels_in_chunk(p, s.chunk);
         for (int t = s.t0; t < s.t1; t += G) {
           const int gcnt = (s.t1 - t) < G ? (s.t1 - t) : G;
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.full[stage]), phase, ctl));
+          ok = mbar_wait_warp(smem_u32(&bars.full[stage]), phase, ctl);
           if (!ok) break;
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.acc_empty[slot]), sphase ^ 1u, ctl));
+          ok = mbar_wait_warp(smem_u32(&bars.acc_empty[slot]), sphase ^ 1u, ctl);
           if (!ok) break;
           tc_fence_after();
           uint64_t ad = smem_desc(hi_a, sbase);
@@ -126,10 +126,8 @@ __global__ void __launch_bounds__(C::THREADS, (NP == 4) ? 1 : C::CTAS_PER_SM) sp
         const int gcnt = (s.t1 - t) < G ? (s.t1 - t) : G;
         // scale of lane j's tile, fetched before the products are ready
         const float my_ts = (lane < gcnt) ? p.tile_scales[t + lane] : 0.0f;
-        int ok = 1;
-        if (lane == 0) ok = mbar_wait(smem_u32(&bars.acc_full[slot]), sphase, ctl) ? 1 : 0;
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) { alive = false; break; }
+        alive = mbar_wait_warp(smem_u32(&bars.acc_full[slot]), sphase, ctl);
+        if (!alive) break;
         tc_fence_after();
         const uint32_t slot_addr = tmem_base + lane_sel + (uint32_t)slot * group_cols + (uint32_t)m_first;
         for (int j = 0; j < gcnt; j += TPW) {

@@ -120,13 +120,10 @@ __global__ void __launch_bounds__(kThreads, 2) tile_grad_kernel(const __grid_con
         const uint32_t phase = (g / kStages) & 1u;
         const uint32_t full = smem_u32(&bars.full[stage]);
         const uint32_t base = ring + (uint32_t)stage * kStageBytes;
-        int ok = 1;
-        if (lane == 0) {
-          ok = mbar_wait(smem_u32(&bars.empty[stage]), phase ^ 1u, abort_flag) ? 1 : 0;
-          if (ok) mbar_expect_tx(full, (uint32_t)(cnt + 1) * kBlockBytes);
-        }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) { alive = false; break; }
+        alive = mbar_wait_warp(smem_u32(&bars.empty[stage]), phase ^ 1u, abort_flag);
+        if (!alive) break;
+        if (lane == 0) mbar_expect_tx(full, (uint32_t)(cnt + 1) * kBlockBytes);
+        __syncwarp();
         if (mine)
           tma_load_2d(base + (uint32_t)lane * kBlockBytes, lane == 4 ? &tmap_g : &tmap_b, MN ? y : s * p.slice_elems,
                       MN ? s * p.slice_elems : y, full);
@@ -143,7 +140,7 @@ __global__ void __launch_bounds__(kThreads, 2) tile_grad_kernel(const __grid_con
       bool ok = true;
       for (int i = blockIdx.x; i < p.n_items && ok; i += gridDim.x, ++n) {
         const uint32_t buf = n & 1u, aph = (n >> 1) & 1u;
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.acc_empty[buf]), aph ^ 1u, abort_flag));
+        ok = mbar_wait_warp(smem_u32(&bars.acc_empty[buf]), aph ^ 1u, abort_flag);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d = tmem_base + buf * 32u;
@@ -151,7 +148,7 @@ __global__ void __launch_bounds__(kThreads, 2) tile_grad_kernel(const __grid_con
         for (int s = 0; s < p.n_slices; ++s, ++g) {
           const int stage = (int)(g % kStages);
           const uint32_t phase = (g / kStages) & 1u;
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.full[stage]), phase, abort_flag));
+          ok = mbar_wait_warp(smem_u32(&bars.full[stage]), phase, abort_flag);
           if (!ok) break;
           tc_fence_after();
           const uint32_t base = ring + (uint32_t)stage * kStageBytes;
@@ -183,10 +180,7 @@ __global__ void __launch_bounds__(kThreads, 2) tile_grad_kernel(const __grid_con
       const uint32_t buf = n & 1u, aph = (n >> 1) & 1u;
       long long orig = 0;
       if (j < cnt) orig = __ldg(p.block_indices + t0 + j);
-      int ok = 1;
-      if (lane == 0) ok = mbar_wait(smem_u32(&bars.acc_full[buf]), aph, abort_flag) ? 1 : 0;
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) break;
+      if (!mbar_wait_warp(smem_u32(&bars.acc_full[buf]), aph, abort_flag)) break;
       tc_fence_after();
       uint32_t r[32];
       if (j < cnt && p.n_slices > 0) {
