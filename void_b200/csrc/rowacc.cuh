@@ -117,14 +117,14 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
             uint64_t adq = ad;
             uint32_t d = d0;
             for (int q = 0; q < npan; ++q) {
-              if (leader) issue_mma<KIND>(d, adq, bd, idesc, acc);
+              issue_mma<KIND>(leader, d, adq, bd, idesc, acc);
 #pragma unroll
               for (int kk = 1; kk < ES; ++kk)
-                if (leader) issue_mma<KIND>(d, adq + kk * kPanelKStep, bd + kk * kTileKStep, idesc, 1u);
+                issue_mma<KIND>(leader, d, adq + kk * kPanelKStep, bd + kk * kTileKStep, idesc, 1u);
               // a tile stored as a sum of terms: every further term multiplies the same panel
               if (KIND == VOID_KIND_F8E4M3)
                 for (int v = 1; v < terms; ++v)
-                  if (leader) issue_mma<KIND>(d, adq, bd + (uint64_t)v * kTileStep, idesc, 1u);
+                  issue_mma<KIND>(leader, d, adq, bd + (uint64_t)v * kTileStep, idesc, 1u);
               adq += kPanelStep;
               d += 32u;
             }

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(C::THREADS, (NP == 4) ? 1 : C::CTAS_PER_SM) sp
             uint64_t adq = ad;
             uint32_t dq = d;
             for (int q = 0; q < npan; ++q) {
-              if (leader) issue_mma<KIND>(dq, adq, bd, idesc, 0u);
+              issue_mma<KIND>(leader, dq, adq, bd, idesc, 0u);
               adq += kPanelStep;
               dq += 32u;
             }

@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kThreads, 2) tile_grad_kernel(const __grid_con
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {  // 32 bytes of n per MMA (inside the swizzle atom), or 1024 bytes of its rows
             constexpr uint64_t kStep = MN ? (1024u >> 4) : 2u;
-            if (leader) issue_mma<KIND>(d, ad + kStep * kk, bd + kStep * kk, idesc, acc);
+            issue_mma<KIND>(leader, d, ad + kStep * kk, bd + kStep * kk, idesc, acc);
             acc = 1u;
           }
           if (leader) tc_commit(smem_u32(&bars.empty[stage]));
