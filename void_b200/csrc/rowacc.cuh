@@ -114,20 +114,18 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
           uint64_t ad = smem_desc(hi_a, sbase);
           uint64_t bd = smem_desc(hi_b, sbase + tile_off<ES>(p, cap, 0));
           for (int j = 0; j < gcnt; ++j) {
-            uint64_t adq = ad;
-            uint32_t d = d0;
-            for (int q = 0; q < npan; ++q) {
-              issue_mma<KIND>(leader, d, adq, bd, idesc, acc);
+            auto panel = [&](uint64_t a, uint32_t d) {
 #pragma unroll
-              for (int kk = 1; kk < ES; ++kk)
-                issue_mma<KIND>(leader, d, adq + kk * kPanelKStep, bd + kk * kTileKStep, idesc, 1u);
+              for (int kk = 0; kk < ES; ++kk) issue_mma<KIND>(leader, d, a + kk * kPanelKStep, bd + kk * kTileKStep, idesc, kk == 0 ? acc : 1u);
               // a tile stored as a sum of terms: every further term multiplies the same panel
-              if (KIND == VOID_KIND_F8E4M3)
-                for (int v = 1; v < terms; ++v)
-                  issue_mma<KIND>(leader, d, adq, bd + (uint64_t)v * kTileStep, idesc, 1u);
-              adq += kPanelStep;
-              d += 32u;
-            }
+              if (KIND == VOID_KIND_F8E4M3) {
+                if (terms > 1) issue_mma<KIND>(leader, d, a, bd + kTileStep, idesc, 1u);
+                if (terms > 2) issue_mma<KIND>(leader, d, a, bd + 2 * kTileStep, idesc, 1u);
+              }
+            };
+            panel(ad, d0);
+            if (npan > 1) panel(ad + kPanelStep, d0 + 32u);
+            for (int q = 2; q < npan; ++q) panel(ad + kPanelStep * (uint64_t)q, d0 + 32u * (uint32_t)q);
             ad += kPanelStep * (uint64_t)np;
             bd += kTileStep * (uint64_t)terms;
             acc = 1u;
