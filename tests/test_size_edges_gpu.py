@@ -357,6 +357,24 @@ def test_two_layers_ask_the_interpreter_for_little_and_notice_every_change():
     (40, 70, 40, 0.9, 1, 1, 2), (250, 300, 129, 0.6, 1, 1, 8), (2500, 333, 384, 0.4, 12, 2, 8), (1111, 2000, 200, 0.95, 18, 1, 2),
     (10000, 640, 515, 0.1, 60, 2, 16)])
 def test_grouped_products_are_exact_on_small_integers(kind, dtype, out, m, k, n, density, groups, entries, tiles):
+    if dtype == torch.float32:                                            # (two stages have to fit a CTA's shared memory)
+        entries, tiles = 1, ((m + 31) // 32 + groups - 1) // groups
+    _grouped_exact(kind, dtype, out, m, k, n, density, groups, entries, tiles)
+
+
+# Stages that end in the middle of a block column, runs of one to four rows, groups of two, five and eight rows, more groups than CTAs,
+# and the stage shapes that products choose for 8 and 7 rows.
+@pytest.mark.parametrize("kind,dtype,out,m,k,n,density,groups,entries,tiles", [
+    ("I8", torch.int8, torch.float16, 256, 640, 130, 1.0, 1, 6, 2), ("I8", torch.int8, torch.float32, 2100, 900, 128, 0.5, 9, 6, 26),
+    ("I8", torch.int8, torch.bfloat16, 500, 500, 77, 0.7, 8, 5, 14), ("BF16", torch.bfloat16, torch.bfloat16, 155, 700, 264, 0.8, 1, 3, 5),
+    ("F16", torch.float16, torch.float16, 4800, 2100, 640, 0.15, 20, 3, 5), ("F16", torch.float16, torch.float16, 1000, 333, 512, 0.5, 4, 2, 1),
+    ("TF32", torch.float32, torch.float32, 224, 640, 200, 0.6, 1, 1, 5), ("TF32", torch.float32, torch.float32, 2048, 1000, 384, 0.3, 8, 2, 5),
+    ("TF32", torch.float32, torch.float16, 300, 700, 128, 0.9, 2, 2, 1)])
+def test_grouped_stages_and_runs_are_exact_on_small_integers(kind, dtype, out, m, k, n, density, groups, entries, tiles):
+    _grouped_exact(kind, dtype, out, m, k, n, density, groups, entries, tiles)
+
+
+def _grouped_exact(kind, dtype, out, m, k, n, density, groups, entries, tiles):
     import ctypes
     from void_b200 import _lib, _spmm
     lib, kd = _lib.load(), getattr(_lib, "KIND_" + kind)
@@ -366,8 +384,6 @@ def test_grouped_products_are_exact_on_small_integers(kind, dtype, out, m, k, n,
     p = _spmm._mark_ready(_spmm.pack(vals, torch.ones(a.n_blocks, device="cuda") if kd == _lib.KIND_I8 else None, a.block_rows,
                                      a.block_cols, (m, k), kd))
     es, P = vals.element_size(), _lib.ptr
-    if es == 4:                                                           # (two stages have to fit a CTA's shared memory)
-        entries, tiles = 1, (p.nbr + groups - 1) // groups
     ints = dict(dtype=torch.int32, device="cuda")
     rows, stages = torch.empty(groups * 16, **ints), torch.empty(groups + 1, **ints)
     records, ws = torch.empty(8 * p.nnz, **ints), torch.empty(2 * groups + p.nnz, **ints)

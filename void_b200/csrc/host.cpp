@@ -393,9 +393,10 @@ at::Tensor fp32_vector(PyObject* o, c10::Device dev, const char* what, int64_t a
 // How the tile rows are dealt to groups for N columns, and what that saves.  In units of a row-accumulate launch's bytes: a
 // CTA slot (two per SM) takes `turns` groups, each the panels of the block columns that any of its rows stores and its tiles;
 // the other kernel takes a panel with every tile.  More than four rows leave no second accumulator set, which costs where a
-// slot has more than one group (16384 x 4096, N = 2048, INT8 70 %: 7 rows 87.1 us, 4 rows 80.6).
+// slot has more than one group (16384 x 4096, N = 2048, fp16, 7 and 4 rows, us: 70 % 131 133, 80 % 102 100, 85 % 86 80, 90 % - 59; fp32
+// 70 % 255 -, 80 % 199 211).
 struct GroupShape {
-  int groups = 0, entries = 0, tiles = 0;
+  int groups = 0;
   double saves = 0.0;
 };
 double group_saves(const Packed* p, int64_t N, int groups, int slots) {
@@ -404,41 +405,56 @@ double group_saves(const Packed* p, int64_t N, int groups, int slots) {
   const double d = nnz / (nbr * nbc), panel = 4.0 * es, tile = es;
   const double rows = std::ceil(nbr / groups), turns = std::ceil(groups * chunks / slots);
   double cost = turns * nbc * ((1.0 - std::pow(1.0 - d, rows)) * panel + d * rows * tile);
-  if (rows > 4 && turns > 1) cost *= 1.1;
+  if (rows > 4 && turns > 1) cost *= es == 4 ? 1.15 : 1.25;
   return nnz * chunks / slots * (panel + tile) / cost;
+}
+// What a stage holds: the split of a CTA's shared memory into stages of E block columns and T tiles with which the ring holds the
+// most block columns, T / (tiles that a column's panel serves) or E of them per stage.  Of equal ones that with three stages: a
+// stage costs the same chain of waits whatever is in it.  (8192^2, N = 1024, us: fp16 80 % 3 x (3 + 5) 46.2, 2 x (4 + 8) 49, 4 x (2 + 4) 49;
+// INT8 50 % 3 x (4 + 18) 42.0, 2 x (6 + 21) 43.6; fp32 50 % 3 x (1 + 5) 148, 2 x (2 + 4) 165, 80 % 2 x (2 + 5) 92.6, 4 x (1 + 2) 98.8.)
+void stage_shape(void_group_store& s, double tiles_per_column, int es) {
+  const int room = 116736 - 3072 - 8192;   // half of an SM's shared memory less the kernel's own and the staging of its results
+  double most = 0.0;
+  for (int n : {3, 4, 5, 6, 2}) {
+    const int bytes = room / n / 1024 * 1024;
+    for (int e = 1; e <= 6; ++e) {
+      const int t = std::min((bytes - e * 4096 * es) / (1024 * es), 32);
+      if (t < 1) break;
+      const double columns = n * std::min((double)e, t / tiles_per_column);
+      if (columns > 1.01 * most) {
+        most = columns;
+        s.max_entries = e;
+        s.max_tiles = t;
+      }
+    }
+  }
 }
 GroupShape group_shape(const Packed* p, int64_t N, int slots) {
   GroupShape best;
-  const int es = elem_bytes(p->kind);
   const int64_t chunks = (N + 127) / 128, nbr = p->args.nbr;
-  const double d = (double)p->args.nnz / ((double)nbr * p->args.nbc);
-  // 32-bit stages hold one block column, so that rows which rarely store it leave the room of their tiles unused
-  const int64_t most = es == 4 ? (d >= 0.4 ? 4 : 2) : 8;
   for (int64_t turns = 1; turns <= 256; ++turns) {
     const int64_t groups = turns * slots / chunks;
     if (groups < 1) continue;
     const int64_t rows = (nbr + groups - 1) / groups;
-    if (rows > most) continue;
+    if (rows > 8) continue;
     if (rows < 2) break;
     const double saves = group_saves(p, N, (int)groups, slots);
     if (saves > best.saves) {
       best.saves = saves;
       best.groups = (int)groups;
-      best.entries = es == 4 ? 1 : (es == 2 ? 2 : 4);
-      best.tiles = es == 4 ? (int)rows : (p->kind == VOID_KIND_I8 && rows * d > 2.2 * (1.0 - std::pow(1.0 - d, (double)rows)) ? 16 : 8);
     }
   }
   return best;
 }
-// The saving from which the grouped kernel is the faster one; swept at 2048^2 ... 16384 x 4096, N = 256 ... 2048, 50 - 90 %
-// sparsity.  Predicted saving and measured gain, fp16: 1.25 0.97, 1.41 1.05, 1.74 1.17, 2.34 1.35; INT8 1.41 0.97 - 1.03,
-// 1.53 1.0 (25 tiles per row) and 1.14 (51), 1.82 1.10 - 1.23; fp32 1.14 1.06, 1.25 1.14, 1.74 1.3.
+// The saving from which the grouped kernel is the faster one; swept at 4096^2, 8192^2 (N = 1024), 16384 x 4096 and 4096 x 16384 (N = 2048),
+// 50 - 90 % sparsity.  Predicted saving and measured gain, fp16: 1.09 1.01, 1.11 1.07, 1.18 1.10, 1.22 1.07, 1.36 1.14, 1.52 1.24, 2.32
+// 1.53; fp32 1.11 0.98, 1.18 1.07, 1.24 1.04, 1.38 1.13 - 1.16, 1.80 1.39, 2.32 1.72; INT8 1.36 - 1.38 0.99 - 1.01, 1.50 1.13, 1.52 1.06, 1.80 1.21,
+// and with rows of 100 tiles 1.26 1.07, 1.40 1.11.
 double group_line(const Packed* p) {
-  const bool long_rows = p->args.nnz >= 48ll * p->args.nbr;
   switch (p->kind) {
-    case VOID_KIND_I8: return long_rows ? 1.5 : 1.75;
+    case VOID_KIND_I8: return p->args.nnz >= 96ll * p->args.nbr ? 1.3 : 1.45;
     case VOID_KIND_TF32: return 1.15;
-    default: return 1.45;
+    default: return 1.1;
   }
 }
 // Whether the kernels that write the store are through.  Asked without waiting; not while the stream is captured, where the
@@ -455,10 +471,10 @@ bool complete(GroupStore* g, void_stream_t st) {
   g->built = nullptr;
   return true;
 }
-// Queues the kernels that lay the tiles out for `shape`; null where there is no memory for it.
-std::unique_ptr<GroupStore> build_group_store(const Packed* p, const GroupShape& shape, void_stream_t st) {
+// Queues the kernels that lay the tiles out for G groups; null where there is no memory for it.
+std::unique_ptr<GroupStore> build_group_store(const Packed* p, int64_t G, void_stream_t st) {
   std::unique_ptr<GroupStore> g(new GroupStore);
-  const int64_t G = shape.groups, nnz = p->args.nnz, es = elem_bytes(p->kind);
+  const int64_t nnz = p->args.nnz, es = elem_bytes(p->kind);
   at::Tensor ws;
   try {
     const c10::Device dev(c10::kCUDA, p->device);
@@ -475,11 +491,11 @@ std::unique_ptr<GroupStore> build_group_store(const Packed* p, const GroupShape&
   g->store.stage_ptr = stages;
   g->store.group_rows = rows;
   g->store.n_groups = (int32_t)G;
-  g->store.max_entries = shape.entries;
-  g->store.max_tiles = shape.tiles;
+  const double d = (double)nnz / ((double)p->args.nbr * p->args.nbc), in_group = std::ceil((double)p->args.nbr / (double)G);
+  stage_shape(g->store, in_group * d / (1.0 - std::pow(1.0 - d, in_group)), (int)es);
   if (cudaEventCreateWithFlags(&g->built, cudaEventDisableTiming) != cudaSuccess) return nullptr;
   check(void_group_build(p->args.row_ptr, p->row_order, p->args.tile_cols, p->args.tiles, p->args.nbr, nnz, (int32_t)es, (int32_t)G,
-                         shape.entries, shape.tiles, rows, stages, records, blob, ws.data_ptr<int32_t>(), st),
+                         g->store.max_entries, g->store.max_tiles, rows, stages, records, blob, ws.data_ptr<int32_t>(), st),
         "void_group_build");
   if (cudaEventRecord(g->built, reinterpret_cast<cudaStream_t>(st)) != cudaSuccess) throw std::runtime_error("CUDA error: recording an event failed");
   return g;
@@ -506,7 +522,7 @@ GroupStore* group_store(Packed* p, int64_t N, void_stream_t st) {
   if (best < 0.93 * shape.saves && n < kMaxGroupStores && p->stable && bytes <= (4ll << 30) && p->group_calls >= 0 && !capturing(st) &&
       ++p->group_calls >= 3) {
     p->group_calls = -1;   // for good, if there is no room for it
-    p->groups[n] = build_group_store(p, shape, st);
+    p->groups[n] = build_group_store(p, shape.groups, st);
     if (p->groups[n] != nullptr) p->group_calls = 0;
   }
   return hit_saves >= line ? hit : nullptr;

@@ -31,15 +31,15 @@ __device__ __forceinline__ void issue_mma(bool leader, uint32_t d, uint64_t a, u
 #undef VB_MMA
 }
 
-// By one thread for itself, the descriptors in halves (their upper halves do not change from one instruction to the next).
+// The same with the descriptors in halves (their upper halves do not change from one instruction to the next).
 template <int KIND>
-__device__ __forceinline__ void mma_halves(uint32_t d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
-                                           uint32_t acc) {
+__device__ __forceinline__ void mma_halves(bool leader, uint32_t d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                           uint32_t idesc, uint32_t acc) {
 #define VB_MMA(NAME)                                                                                                   \
   asm volatile(                                                                                                        \
-      "{\n .reg .pred p;\n .reg .b64 a, b;\n mov.b64 a, {%1, %2};\n mov.b64 b, {%3, %4};\n setp.ne.b32 p, %6, 0;\n"    \
-      " tcgen05.mma.cta_group::1." NAME " [%0], a, b, %5, p;\n}\n"                                                      \
-      ::"r"(d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc) : "memory")
+      "{\n .reg .pred p, q;\n .reg .b64 a, b;\n mov.b64 a, {%1, %2};\n mov.b64 b, {%3, %4};\n setp.ne.b32 p, %6, 0;\n" \
+      " setp.ne.b32 q, %7, 0;\n @q tcgen05.mma.cta_group::1." NAME " [%0], a, b, %5, p;\n}\n"                          \
+      ::"r"(d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc), "r"((uint32_t)leader) : "memory")
   if constexpr (KIND == VOID_KIND_I8) VB_MMA("kind::i8");
   else if constexpr (KIND == VOID_KIND_F8E4M3) VB_MMA("kind::f8f6f4");
   else if constexpr (KIND == VOID_KIND_TF32) VB_MMA("kind::tf32");

@@ -189,6 +189,14 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
                : "memory");
 }
 
+// The same by the leader of a converged warp, without a branch.
+__device__ __forceinline__ void tc_commit_if(bool leader, uint32_t bar) {
+  asm volatile(
+      "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+      " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar), "r"((uint32_t)leader)
+      : "memory");
+}
+
 // 32 lanes x 32 columns of 32-bit accumulators: thread t of the warp gets lane (base + t),
 // columns [col, col + 32).
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {
