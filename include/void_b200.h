@@ -236,7 +236,10 @@ VOID_API int void_quant_i8_tensor(const float* b, int64_t ldb, int32_t K, int32_
  * void_plan_segments cuts the tile stream into n_cta contiguous shares of (nearly) equal
  * weight.  With split_rows = 0 share boundaries fall on tile-row boundaries; with
  * split_rows = 1 a boundary may fall on a chunk boundary of the worker table inside a heavy
- * row; with split_rows = 2 every worker of the table becomes a segment of its own.
+ * row; with split_rows = 2 every worker of the table becomes a segment of its own.  With
+ * split_rows = 3 nothing is contiguous: whole rows, and pieces of those heavier than one and a half
+ * shares, are dealt out, the heaviest first, to the CTA that has the least so far (n_cta <= 1024 and
+ * nbr * n_chunks + 2 * n_cta <= 8190, else VOID_ERR_TOO_LARGE; chunk_tiles is not used).
  * Output: segs (8 int32 each: row, n_chunk, t0, t1, nseg, slot0, my_idx, counter),
  * cta_seg_ptr[n_cta+1], counts[4] = {n_segs, n_slots, n_counters, overflow flag}; segs needs
  * void_plan_capacity(...) entries.  n_counters is the number of split rows: each needs one
@@ -255,7 +258,7 @@ VOID_API int64_t void_plan_capacity(int64_t nnz, int32_t nbr, int32_t n_chunks, 
 VOID_API size_t void_plan_ws_bytes(int32_t nbr, int32_t n_cta);
 /* row_cost (>= 1): what finishing one (tile row, column chunk) costs relative to one tile of work; it
  * weights the shares so that a CTA handed many short rows is not handed many tiles as well.
- * chunk_tiles: chunk length of the worker table (void_streamk_target), used when split_rows > 0.
+ * chunk_tiles: chunk length of the worker table (void_streamk_target), used when split_rows is 1 or 2.
  * woff: (nbr + 1) workers-before-row prefix left in the ws of void_streamk_table, needed for
  * split_rows = 2 only.  ws: device scratch of void_plan_ws_bytes(nbr, n_cta) bytes.          */
 VOID_API int void_plan_segments(const int32_t* row_ptr, int32_t nbr, int32_t n_chunks, int32_t n_cta,

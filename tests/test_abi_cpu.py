@@ -189,6 +189,26 @@ def test_plan_invariants_random():
                         int(rng.integers(1, 12)))
 
 
+def test_dealt_plan_invariants_and_balance():
+    rng = np.random.default_rng(5)
+    draws = (lambda n: rng.integers(0, 20, n), lambda n: np.minimum(rng.zipf(1.5, n), 512), lambda n: np.minimum(rng.zipf(1.2, n), 5000),
+             lambda n: (rng.random(n) < 0.3) * rng.integers(0, 300, n))
+    for trial in range(80):
+        cnt = draws[trial % 4](int(rng.integers(1, 300)))
+        if cnt.sum() == 0:
+            continue
+        row_ptr = np.concatenate([[0], np.cumsum(cnt)]).astype(np.int32)
+        n_cta, cost = int(rng.integers(1, 1025)), int(rng.integers(1, 12))
+        segs, cptr = _check_plan(row_ptr, int(rng.integers(1, 4)), n_cta, 3, 0, cost)
+        if len(segs) >= n_cta:      # no CTA has more than the share at which rows are cut and a segment on top
+            load = np.array([sum(s[3] - s[2] + (4 * cost if s[4] > 1 else cost) for s in segs[cptr[k]:cptr[k + 1]]) for k in range(n_cta)])
+            heaviest = max(s[3] - s[2] + (4 * cost if s[4] > 1 else cost) for s in segs)
+            assert load.max() <= load.mean() + 2 * heaviest
+    lib = _lib.load()
+    assert lib.void_plan_segments_host(row_ptr.ctypes.data, len(row_ptr) - 1, 1, 1025, 3, 0, 1, None, segs.ctypes.data, len(segs),
+                                       cptr.ctypes.data, cptr.ctypes.data) == -8      # VOID_ERR_TOO_LARGE
+
+
 def test_plan_splits_heavy_rows_only_when_asked():
     cnt = np.full(64, 4)
     cnt[10] = 400                                  # one row far heavier than a CTA's share

@@ -226,3 +226,25 @@ def test_staged_results_of_slim_ctas_equal_direct_stores(kind, m, n, biased):
             outs.append(out)
         assert torch.equal(*outs)
     void.check_device_status()
+
+
+@pytest.mark.parametrize("nbr,n_chunks,n_cta,heaviest", [(1, 1, 1, 40), (1, 3, 592, 3000), (37, 2, 600, 9), (512, 2, 592, 512), (1023, 4, 592, 60),
+                                                         (1024, 6, 1000, 2), (2000, 3, 1024, 900)])
+def test_dealt_plan_on_the_device_is_the_host_plan(nbr, n_chunks, n_cta, heaviest):
+    """Sorted, scanned and dealt by one block: sizes around its 1024 threads, one row, more CTAs than segments, 8192 segments at most."""
+    from test_abi_cpu import _check_plan
+    from void_b200 import _lib, _spmm
+    rng = np.random.default_rng(nbr)
+    cnt = np.minimum(rng.zipf(1.5, nbr), heaviest) if heaviest > 9 else rng.integers(0, heaviest, nbr) + (np.arange(nbr) == 0)
+    cnt[-1] = heaviest
+    row_ptr = np.concatenate([[0], np.cumsum(cnt)]).astype(np.int32)
+    segs, cta_seg_ptr = _check_plan(row_ptr, n_chunks, n_cta, 3, 0, _spmm.ROW_COST)
+    lib, dev = _lib.load(), torch.device("cuda:0")
+    rp, words = torch.from_numpy(row_ptr).to(dev), dict(dtype=torch.int32, device=dev)
+    cap = lib.void_plan_capacity(int(row_ptr[-1]), nbr, n_chunks, n_cta, 3, 0)
+    got, ptr, counts = torch.zeros(cap * 8, **words), torch.empty(n_cta + 1, **words), torch.zeros(4, **words)
+    ws = torch.empty(lib.void_plan_ws_bytes(nbr, n_cta), dtype=torch.uint8, device=dev)
+    _lib.check(lib.void_plan_segments(_lib.ptr(rp), nbr, n_chunks, n_cta, 3, 0, _spmm.ROW_COST, None, _lib.ptr(got), cap, _lib.ptr(ptr),
+                                      _lib.ptr(counts), _lib.ptr(ws), ws.numel(), _lib.stream_ptr(dev)), "void_plan_segments")
+    assert counts.tolist()[0] == len(segs) and counts.tolist()[3] == 0
+    assert np.array_equal(ptr.cpu().numpy(), cta_seg_ptr) and np.array_equal(got.cpu().numpy().reshape(-1, 8)[:len(segs)], segs)

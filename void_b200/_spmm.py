@@ -249,9 +249,15 @@ def streamk_table(row_ptr: torch.Tensor, nbr: int, nnz: int, n_workers: Optional
 ROW_COST = 8   # epilogue of one (tile row, chunk) in units of one tile of work, swept on B200 (power-law rows, N = 256 / 1024, us: 4 15.6 / 45.7, 6 14.4 / 39.4, 8 13.9 / 37.0, 12 14.0 / 37.4, 16 14.8 / 39.4)
 
 
+def split_mode(nbr: int, n_chunks: int, n_cta: int) -> int:
+    """How heavy tile rows are split (split_rows of void_plan_segments): the segments dealt out by weight (3) as long as one
+    block can sort them, else contiguous shares (1), whose many segments per CTA even out by themselves."""
+    return 3 if n_cta <= 1024 and nbr * n_chunks + 2 * n_cta + 2 <= 8192 else 1
+
+
 def make_plan(packed: PackedTiles, N: int, np_: int, n_cta: int, mode: int, chunk_tiles: int = 0,
               woff: Optional[torch.Tensor] = None, row_cost: int = ROW_COST) -> Plan:
-    """Cut the tile stream of ``packed`` into ``n_cta`` shares on the device (void_plan_segments)."""
+    """Cut the tile stream of ``packed`` into ``n_cta`` shares, or deal its rows out, on the device (void_plan_segments)."""
     lib = _lib.load()
     dev = packed.row_ptr.device
     panels = (N + PANEL - 1) // PANEL

@@ -50,19 +50,25 @@ def compute_stream_k_workload(void_tensor, n_workers: Optional[int] = None,
                            chunk_tiles=target, worker_offsets=woff)
 
 
-def _plan_for(a, packed, N: int, workload: StreamKWorkload, per_worker: bool, n_cta: Optional[int]):
+def _plan_for(a, packed, N: int, workload: Optional[StreamKWorkload], per_worker: bool, n_cta: Optional[int]):
+    """The plan for N columns, kept on the tensor: cut along the worker table where one is given or its workers' sums are asked
+    for, else dealt out, which needs no table, as long as that can be (split_mode)."""
     sms = packed.sms
     np_ = _spmm.default_panels(packed.nbr, N, sms) if _lib.KIND_ELEM_BYTES[packed.kind] == 1 else 1
     if n_cta is None:
         n_cta = sms * 4          # four slim CTAs per SM
-    mode = 2 if per_worker else 1
-    key = ("streamk", packed.kind, N, np_, n_cta, mode, workload.chunk_tiles)
+    n_chunks = (N + _spmm.PANEL * np_ - 1) // (_spmm.PANEL * np_)
+    mode = 2 if per_worker else (1 if workload is not None else _spmm.split_mode(packed.nbr, n_chunks, n_cta))
+    if mode != 3 and workload is None:
+        workload = _cached_workload(a, packed)
+    chunk_tiles, offsets = (0, None) if mode == 3 else (workload.chunk_tiles, workload.worker_offsets)
+    key = ("streamk", packed.kind, N, np_, n_cta, mode, chunk_tiles)
     cache = getattr(a, "_plan_cache", None)
     if cache is None:
         cache = a._plan_cache = {}
     plan = cache.get(key)
     if plan is None:
-        plan = _spmm.make_plan(packed, N, np_, n_cta, mode, workload.chunk_tiles, workload.worker_offsets)
+        plan = _spmm.make_plan(packed, N, np_, n_cta, mode, chunk_tiles, offsets)
         cache[key] = plan
     return plan
 
@@ -97,8 +103,6 @@ def void_spmm_stream_k(a: Int8VOIDTensor, b: torch.Tensor, workload: Optional[St
     packed = a.packed()
     opts = None
     if a.n_blocks != 0:
-        if workload is None:
-            workload = _cached_workload(a, packed)
         plan = _plan_for(a, packed, b.shape[1], workload, worker_partials is not None, n_cta)
         _require_room(worker_partials, plan, b.shape[1])
         opts = plan.options(acc_out, worker_partials)
@@ -121,8 +125,6 @@ def _stream_k_fp(a: VOIDTensor, b, workload, out, activation, bias, worker_parti
     if a.n_blocks == 0:
         return ops.void_spmm(a, b, out, activation=activation, bias=bias)
     packed = ops.packed_fp(a, ops.product_kind(a, b))
-    if workload is None:
-        workload = _cached_workload(a, packed)
     plan = _plan_for(a, packed, b.shape[1], workload, worker_partials is not None, n_cta)
     _require_room(worker_partials, plan, b.shape[1])
     return ops.void_spmm(a, b, out, activation=activation, bias=bias, plan=plan, acc_out=acc_out,
