@@ -606,3 +606,34 @@ def test_products_wait_for_the_kernel_that_prepares_their_operand(dtype, k, n):
                      else void.void_spmm_fp8(q, x, torch.float32, b_scale=scale))
             assert torch.equal(c, alone)
     void.check_device_status()
+
+
+@pytest.mark.parametrize("kind", ["int8", "fp8"])
+@pytest.mark.parametrize("rows,k,n", [(592, 96, 128), (593, 96, 128), (148, 1312, 512), (149, 1312, 512), (1, 64, 40), (3, 4000, 136), (37, 700, 2000)])
+def test_results_staged_in_the_ring_are_those_stored_directly(kind, rows, k, n):
+    """One item per CTA up to 592 items (the staging tile then lies in the ring), more from there on; empty rows, ragged edges."""
+    from void_b200 import _lib, _spmm
+    gen = torch.Generator().manual_seed(rows + n)
+    dense = torch.randn(rows * 32 - 5, k, generator=gen)
+    keep = torch.rand(rows, (k + 31) // 32, generator=gen) < 0.4
+    keep[rows // 2] = False                                              # an empty row of tiles
+    keep[0] = True
+    dense *= keep.repeat_interleave(32, 0).repeat_interleave(32, 1)[:dense.shape[0], :k]
+    a = void.dense_to_void(dense.cuda())
+    b = torch.randn(k, n, generator=gen).cuda()
+    if kind == "int8":
+        t = void.quantize_void_tensor(a)
+        p, (q, scale) = t.packed(), void.quantize_cols_int8(b)
+    else:
+        t = void.void_tensor_to_fp8(a)
+        p, (q, scale) = t.packed_split(2), void.quantize_cols_fp8(b)[:2]
+        q = q.view(torch.uint8)
+    bias = torch.randn(n, generator=gen).cuda()
+    for dtype in (torch.float16, torch.bfloat16):
+        outs = []
+        for options in ({}, {"flags": 2}, {"grid": 5}):
+            out = torch.full((dense.shape[0], n), float("nan"), dtype=dtype, device="cuda")
+            _spmm.spmm(p, q, out, scale_mode=_lib.SCALE_ROW_MEAN, col_scale=scale, bias=bias, act=2, cta_shape=2, **options)
+            outs.append(out)
+        assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    void.check_device_status()

@@ -149,6 +149,7 @@ struct SpmmParams {
   int group;    // tiles per ring stage
   int stages;   // ring depth
   int last_group;   // tiles of the ring's last stage (1 .. group): the shared memory left over by the full stages
+  int part_off;     // staging of 16-bit results, bytes from the ring's start: behind the ring, or in it (spmm.cu)
   int use3d;    // B panels of a tile fetched by one 3-D TMA
   int tmem_cols;  // tensor-memory columns of the drain kernel (256: two CTAs per SM, 512: one)
   int n_items;  // without a plan: nbr * n_chunks

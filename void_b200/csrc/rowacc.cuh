@@ -51,7 +51,6 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
   constexpr int ES = Elem<KIND>::ES;
   const uint32_t unit_smem = (uint32_t)((p.np * kPanelBytes + kTileBytes * p.terms) * ES);
   const uint32_t stage_bytes = (uint32_t)p.group * unit_smem;   // the last stage may be shorter (p.last_group tiles)
-  const uint32_t ring_bytes = (uint32_t)((p.stages - 1) * p.group + p.last_group) * unit_smem;
   const uint32_t acc_cols = (uint32_t)p.np * 32u;  // TMEM columns of one accumulator buffer
   uint32_t tmem_cols = 32;
   while (tmem_cols < 2u * acc_cols) tmem_cols <<= 1;
@@ -153,8 +152,8 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS_PER_SM) spmm_rowacc_kernel
     const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
     const int m_first = half * C::COLS;
     const OutDesc od = out_desc(p);
-    // this warp's part of the staging tile behind the ring
-    const uint32_t part = ring_base + ring_bytes + (uint32_t)(warp - C::EPI0) * (32u * kTile * 2u);
+    // this warp's part of the staging tile
+    const uint32_t part = ring_base + (uint32_t)p.part_off + (uint32_t)(warp - C::EPI0) * (32u * kTile * 2u);
     bool store_pending = false;
     // the column scales and biases this role reads and the C it writes may be the previous kernel's; the index
     // of A may be read ahead of it when the caller vouches for A

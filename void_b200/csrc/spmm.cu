@@ -361,27 +361,6 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
     const long long per_sm = ((long long)a->nbr * n_chunks + dev.sms - 1) / dev.sms;
     if (per_sm < share) share = per_sm < 1 ? 1 : (int)per_sm;
   }
-  int group = a->tiles_per_stage;  // 0 = default
-  // What a CTA streams is bounded by the bytes its ring keeps in flight over a stage's round trip, so the defaults fill
-  // the shared memory the CTAs of an SM leave each other: nine (tile + panel) units as 3 stages x 3 for one 8-bit panel per
-  // item and four CTAs (swept on B200, headline / 70 % / 16384^2: 2 x 4 units 7.02 / 11.06 / 69.9 us, 3 x 3: 6.76 / 10.21 /
-  // 65.1, 4 x 2: 6.96 / 10.87 / 69.4, 9 x 1: 8.64 / 16.2 / 111); stages of one or two tiles pay the fixed cost of a stage
-  // too often.  With fewer CTAs on the SM longer stages pay (1024 x 8192, 70 %, N = 256, one CTA per SM: INT8 3 x 3 12.4
-  // us, 7 x 6 10.4; FP8 of two terms 17.4 -> 13.3; fp16 21.5 -> 13.4 with 6 x 3; fp32 41.2 -> 25.3 with 8 x 1).
-  if (group == 0) {
-    if (floating) group = (es == 2 && np == 1) ? ((tr_b && share > 1) || slim ? 2 : 3) : 1;
-    // (a tile stored as several terms is that much longer: 3 stages x 2 at four CTAs, headline 7.66 us, 2 x 3: 7.93)
-    else if (a->tile_terms > 1) group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 3 : 2)) : 1;
-    else group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 4 : 3)) : 2;
-  }
-  if (group < 1 || group > 8) return VOID_ERR_BAD_ARG;
-  if (drain && np == 1 && shape != 1 && a->tiles_per_stage == 0) group = 2;
-  int drain_tmem = 32;   // the largest power of two that lets ctas_per_sm CTAs share the SM's 512 columns
-  while (drain_tmem * 2 * ctas_per_sm <= 512) drain_tmem *= 2;
-  if (drain && group * np * 32 * 2 > drain_tmem) return VOID_ERR_BAD_ARG;  // two slot groups of products in TMEM
-  int terms = a->tile_terms == 0 ? 1 : a->tile_terms;
-  if (terms < 1 || terms > 3) return VOID_ERR_BAD_ARG;
-  if (terms > 1 && (kind != VOID_KIND_F8E4M3 || drain || tr)) return VOID_ERR_BAD_ARG;  // FP8 row-accumulate only
   // 16-bit outputs of the slim row-accumulate kernel leave through a staging tile (32 x 128 x 2 bytes behind the
   // ring) and a tiled TMA store, when C qualifies as a tensor for the copy engine (16-byte aligned base and pitch)
   // (with a plan, whole-row segments take this route and the pieces of split rows the ordinary one; a sum over one rank, whose
@@ -392,8 +371,34 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
                          a->worker_partials == nullptr && (a->flags & 2) == 0 &&
                          (a->out_dtype == VOID_OUT_F16 || a->out_dtype == VOID_OUT_BF16) &&
                          (reinterpret_cast<uintptr_t>(a->out) & 15u) == 0 && ((a->ldc * 2) & 15) == 0;
+  // Where every CTA has one item, the staging tile lies in the ring (ten KB at least), whose stages have all been multiplied by
+  // then, and the ring has its 8 KB: ten (tile + panel) units of INT8 instead of nine, nine of FP8 tiles of two terms instead of
+  // six.  4096^2, N = 512, us: FP8 80 % 10.2 (3 stages x 2) -> 9.3 (3 x 3; 4 x 2 9.6, 2 x 4 9.7), 90 % 7.0 -> 6.3, 70 % 12.7 -> 11.6; INT8 90 %
+  // 5.66 (3 x 3) -> 5.54 (2 x 5; 5 x 2 5.9, 2 x 4 5.9), 70 % 9.3 -> 9.2.
+  const bool single = staged && a->segs == nullptr && n_items <= (a->grid > 0 ? a->grid : dev.sms * ctas_per_sm);
+  int group = a->tiles_per_stage;  // 0 = default
+  // What a CTA streams is bounded by the bytes its ring keeps in flight over a stage's round trip, so the defaults fill
+  // the shared memory the CTAs of an SM leave each other: nine (tile + panel) units as 3 stages x 3 for one 8-bit panel per
+  // item and four CTAs (swept on B200, headline / 70 % / 16384^2: 2 x 4 units 7.02 / 11.06 / 69.9 us, 3 x 3: 6.76 / 10.21 /
+  // 65.1, 4 x 2: 6.96 / 10.87 / 69.4, 9 x 1: 8.64 / 16.2 / 111); stages of one or two tiles pay the fixed cost of a stage
+  // too often.  With fewer CTAs on the SM longer stages pay (1024 x 8192, 70 %, N = 256, one CTA per SM: INT8 3 x 3 12.4
+  // us, 7 x 6 10.4; FP8 of two terms 17.4 -> 13.3; fp16 21.5 -> 13.4 with 6 x 3; fp32 41.2 -> 25.3 with 8 x 1).
+  if (group == 0) {
+    if (floating) group = (es == 2 && np == 1) ? ((tr_b && share > 1) || slim ? 2 : 3) : 1;
+    // (a tile stored as several terms is that much longer: 3 stages x 2 at four CTAs, headline 7.66 us, 2 x 3: 7.93)
+    else if (a->tile_terms > 1) group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 3 : (single && a->tile_terms == 2 ? 3 : 2))) : 1;
+    else group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 4 : (single ? 5 : 3))) : 2;
+  }
+  if (group < 1 || group > 8) return VOID_ERR_BAD_ARG;
+  if (drain && np == 1 && shape != 1 && a->tiles_per_stage == 0) group = 2;
+  int drain_tmem = 32;   // the largest power of two that lets ctas_per_sm CTAs share the SM's 512 columns
+  while (drain_tmem * 2 * ctas_per_sm <= 512) drain_tmem *= 2;
+  if (drain && group * np * 32 * 2 > drain_tmem) return VOID_ERR_BAD_ARG;  // two slot groups of products in TMEM
+  int terms = a->tile_terms == 0 ? 1 : a->tile_terms;
+  if (terms < 1 || terms > 3) return VOID_ERR_BAD_ARG;
+  if (terms > 1 && (kind != VOID_KIND_F8E4M3 || drain || tr)) return VOID_ERR_BAD_ARG;  // FP8 row-accumulate only
   const int stage_bytes = group * (np * kPanelBytes + kTileBytes * terms) * es;
-  const int staging_bytes = staged ? kTile * kPanelN * 2 : 0;
+  const int staging_bytes = staged && !single ? kTile * kPanelN * 2 : 0;
   int stages = a->stages;
   if (stages == 0) {
     // dynamic shared memory a CTA may use so that its share of them fits an SM: the SM's bytes less the kilobyte
@@ -477,6 +482,7 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   p.group = group;
   p.stages = stages;
   p.last_group = last_group;
+  p.part_off = single ? 0 : smem_bytes - 1024 - staging_bytes;
   p.use3d = (!tr_b && a->N % (kPanelN / es) == 0) ? 1 : 0;
   p.tmem_cols = drain_tmem;
   p.n_items = a->nbr * n_chunks;
