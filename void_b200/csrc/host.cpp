@@ -393,8 +393,8 @@ at::Tensor fp32_vector(PyObject* o, c10::Device dev, const char* what, int64_t a
 // How the tile rows are dealt to groups for N columns, and what that saves.  In units of a row-accumulate launch's bytes: a
 // CTA slot (two per SM) takes `turns` groups, each the panels of the block columns that any of its rows stores and its tiles;
 // the other kernel takes a panel with every tile.  More than four rows leave no second accumulator set, which costs where a
-// slot has more than one group (16384 x 4096, N = 2048, fp16, 7 and 4 rows, us: 70 % 131 133, 80 % 102 100, 85 % 86 80, 90 % - 59; fp32
-// 70 % 255 -, 80 % 199 211).
+// slot has more than one group (16384 x 4096, N = 2048, fp16, 7 and 4 rows, us: 70 % 131 133, 80 % 102 100, 85 % 86 80; fp32 70 % 255 -,
+// 80 % 199 211); with up to four there is still the end of each.
 struct GroupShape {
   int groups = 0;
   double saves = 0.0;
@@ -405,7 +405,7 @@ double group_saves(const Packed* p, int64_t N, int groups, int slots) {
   const double d = nnz / (nbr * nbc), panel = 4.0 * es, tile = es;
   const double rows = std::ceil(nbr / groups), turns = std::ceil(groups * chunks / slots);
   double cost = turns * nbc * ((1.0 - std::pow(1.0 - d, rows)) * panel + d * rows * tile);
-  if (rows > 4 && turns > 1) cost *= es == 4 ? 1.15 : 1.25;
+  if (turns > 1) cost *= rows > 4 ? (es == 4 ? 1.2 : 1.3) : 1.05;
   return nnz * chunks / slots * (panel + tile) / cost;
 }
 // What a stage holds: the split of a CTA's shared memory into stages of E block columns and T tiles with which the ring holds the
@@ -447,13 +447,13 @@ GroupShape group_shape(const Packed* p, int64_t N, int slots) {
   return best;
 }
 // The saving from which the grouped kernel is the faster one; swept at 4096^2, 8192^2 (N = 1024), 16384 x 4096 and 4096 x 16384 (N = 2048),
-// 50 - 90 % sparsity.  Predicted saving and measured gain, fp16: 1.09 1.01, 1.11 1.07, 1.18 1.10, 1.22 1.07, 1.36 1.14, 1.52 1.24, 2.32
-// 1.53; fp32 1.11 0.98, 1.18 1.07, 1.24 1.04, 1.38 1.13 - 1.16, 1.80 1.39, 2.32 1.72; INT8 1.36 - 1.38 0.99 - 1.01, 1.50 1.13, 1.52 1.06, 1.80 1.21,
-// and with rows of 100 tiles 1.26 1.07, 1.40 1.11.
+// 50 - 90 % sparsity.  Predicted saving and measured gain, fp16: 1.06 0.99 - 1.07, 1.09 1.01, 1.12 1.06 - 1.15, 1.12 1.10, 1.22 1.07, 1.36 1.14,
+// 1.52 1.24, 2.32 1.53; fp32 1.06 0.98, 1.15 1.07, 1.24 1.04, 1.38 1.13, 1.80 1.39, 2.32 1.72; INT8 1.36 - 1.38 0.99 - 1.01, 1.50 1.13, 1.52 1.06,
+// 1.80 1.21, and with rows of 100 tiles 1.26 1.07, 1.40 1.11.
 double group_line(const Packed* p) {
   switch (p->kind) {
     case VOID_KIND_I8: return p->args.nnz >= 96ll * p->args.nbr ? 1.3 : 1.45;
-    case VOID_KIND_TF32: return 1.15;
+    case VOID_KIND_TF32: return 1.12;
     default: return 1.1;
   }
 }
