@@ -248,3 +248,24 @@ def test_dealt_plan_on_the_device_is_the_host_plan(nbr, n_chunks, n_cta, heavies
                                       _lib.ptr(counts), _lib.ptr(ws), ws.numel(), _lib.stream_ptr(dev)), "void_plan_segments")
     assert counts.tolist()[0] == len(segs) and counts.tolist()[3] == 0
     assert np.array_equal(ptr.cpu().numpy(), cta_seg_ptr) and np.array_equal(got.cpu().numpy().reshape(-1, 8)[:len(segs)], segs)
+
+
+@pytest.mark.parametrize("warm,captured", [(True, False), (False, True), (False, False)])
+def test_a_captured_product_takes_the_plan_that_is_kept(warm, captured):
+    """With a worker table and without one the plans differ, the results do not; in a capture neither can be built."""
+    mask = workloads.zipf_mask(40, 64, 1.5, 60, 8.0, seed=2)
+    w = workloads.block_sparse(mask, 160, seed=2)
+    q = void.quantize_void_tensor(w.a)
+    b, scale = void.quantize_cols_int8(w.b)
+    table = void.compute_stream_k_workload(q)
+    want = void.void_spmm_stream_k(q, b, table if warm else None, b_scale=scale, out_dtype=torch.float16)
+    assert torch.equal(want, void.void_spmm_int8(q, b, scale, out_dtype=torch.float16))
+    side, graph, out = torch.cuda.Stream(), torch.cuda.CUDAGraph(), torch.empty_like(want)
+    with torch.cuda.graph(graph, stream=side):
+        void.void_spmm_stream_k(q, b, table if captured else None, out, b_scale=scale)
+    for _ in range(2):
+        out.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    void.check_device_status()
