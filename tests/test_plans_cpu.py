@@ -1,0 +1,90 @@
+"""Which kept work plan a power-law product takes: host logic, with the packed store and the capture state replaced by stand-ins."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from void_b200 import _lib, _spmm, stream_k
+
+
+class Tensor:
+    def __init__(self, tiles):
+        self.set_list(tiles)
+
+    def set_list(self, tiles):
+        self.block_rows, self.block_cols = torch.arange(tiles, dtype=torch.int32), torch.zeros(tiles, dtype=torch.int32)
+
+
+def _store(nbr=40, kind=_lib.KIND_I8):
+    """A store as packing makes it: with an index of its own."""
+    return SimpleNamespace(sms=148, nbr=nbr, kind=kind, row_ptr=torch.zeros(nbr + 1, dtype=torch.int32), shape=(32 * nbr, 640))
+
+
+@pytest.fixture
+def host(monkeypatch):
+    state = SimpleNamespace(capturing=False, built=0)
+
+    def make_plan(packed, N, np_, n_cta, mode, chunk_tiles=0, woff=None):
+        state.built += 1
+        plan = object.__new__(_spmm.Plan)
+        plan.row_ptr, plan.tile_list, plan.shape, plan.mode = packed.row_ptr, None, packed.shape, mode
+        return plan
+
+    def cached_workload(a, packed):
+        assert not state.capturing, "the worker table is read back on the host"
+        return SimpleNamespace(chunk_tiles=16, worker_offsets=None)
+
+    monkeypatch.setattr(_spmm, "make_plan", make_plan)
+    monkeypatch.setattr(stream_k, "_cached_workload", cached_workload)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: state.capturing)
+    return state
+
+
+TABLE = SimpleNamespace(chunk_tiles=16, worker_offsets=None)
+
+
+@pytest.mark.parametrize("kind", [_lib.KIND_I8, _lib.KIND_TF32])
+@pytest.mark.parametrize("tiles", [30, 100, 200])
+@pytest.mark.parametrize("warm", [None, TABLE])
+@pytest.mark.parametrize("captured", [None, TABLE])
+def test_a_plan_of_another_tile_list_is_refused_inside_a_capture(host, kind, tiles, warm, captured):
+    a = Tensor(100)
+    stream_k._plan_for(a, _store(kind=kind), 256, warm, False, None)
+    a.set_list(tiles)
+    host.capturing = True
+    with pytest.raises(_lib.VoidB200Error, match="capture"):
+        stream_k._plan_for(a, _store(kind=kind), 256, captured, False, None)
+
+
+@pytest.mark.parametrize("per_worker", [False, True])
+def test_a_plan_of_another_tile_list_is_not_taken_outside_of_one(host, per_worker):
+    a = Tensor(100)
+    old = stream_k._plan_for(a, _store(), 256, TABLE, per_worker, None)
+    a.block_rows[0] = 3
+    store = _store()
+    new = stream_k._plan_for(a, store, 256, TABLE, per_worker, None)
+    assert new is not old and new.row_ptr is store.row_ptr and host.built == 2
+    assert stream_k._plan_for(a, store, 256, TABLE, per_worker, None) is new
+
+
+def test_worker_sums_of_another_tile_list_are_refused_inside_a_capture(host):
+    a = Tensor(100)
+    stream_k._plan_for(a, _store(), 256, TABLE, True, None)
+    a.block_cols[3] = 1
+    host.capturing = True
+    with pytest.raises(_lib.VoidB200Error, match="capture"):
+        stream_k._plan_for(a, _store(), 256, TABLE, True, None)
+
+
+def test_a_store_of_the_same_list_takes_the_plan_that_is_kept(host):
+    """Tiles edited, list and shape as they were: a store that the capture packs has another index of the same tiles."""
+    a = Tensor(100)
+    plan = stream_k._plan_for(a, _store(), 256, None, False, None)
+    host.capturing = True
+    assert stream_k._plan_for(a, _store(), 256, None, False, None) is plan
+    assert stream_k._plan_for(a, _store(), 256, TABLE, False, None) is plan
+    other = _store()
+    other.shape = (32 * 40, 672)
+    with pytest.raises(_lib.VoidB200Error, match="capture"):
+        stream_k._plan_for(a, other, 256, None, False, None)
+    assert host.built == 1

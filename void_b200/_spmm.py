@@ -178,10 +178,21 @@ class Plan:
     counters: torch.Tensor
     mode: int
     chunk_tiles: int
+    # the tile list whose tiles the segments name: its index, the identity of its coordinates, the shape of A
+    row_ptr: Optional[torch.Tensor] = None
+    tile_list: object = None
+    shape: Optional[tuple] = None
     scratch: dict = field(default_factory=dict, init=False, repr=False)   # launch key: (partials, counters)
 
     def __post_init__(self):
         self.scratch[_lib.native().launch_key(self.counters.device.index)] = self.partials, self.counters
+
+    def serves(self, a, packed: PackedTiles) -> bool:
+        """Whether the plan was made for the tile list of ``packed``, the store of ``a`` as it is now: from the same index, or from
+        one of the same coordinates (a store that is packed inside a capture has an index of its own)."""
+        return self.row_ptr is packed.row_ptr or (
+            self.tile_list is not None and self.shape == packed.shape
+            and _lib.native().unchanged(self.tile_list, a.block_rows, a.block_cols))
 
     def native_args(self) -> tuple:
         key = _lib.native().launch_key(self.counters.device.index)
@@ -280,7 +291,7 @@ def make_plan(packed: PackedTiles, N: int, np_: int, n_cta: int, mode: int, chun
             partials = torch.zeros(n_ctr * np_ * PANEL * TILE, dtype=torch.int32, device=dev)
         counters = torch.zeros(max(n_ctr, 1), dtype=torch.int32, device=dev)
     plan = Plan(segs, cta_seg_ptr, n_cta, np_, n_chunks, n_segs, n_slots, n_ctr, partials, counters, mode,
-                chunk_tiles)
+                chunk_tiles, packed.row_ptr, shape=packed.shape)
     _LIVE_PLANS.add(plan)
     return plan
 

@@ -67,14 +67,19 @@ def _plan_for(a, packed, N: int, workload: Optional[StreamKWorkload], per_worker
     if cache is None:
         cache = a._plan_cache = {}
     plan = cache.get(key)
-    if plan is None and not per_worker and torch.cuda.is_current_stream_capturing():
-        # nothing can be built here: a plan of either kind that is kept for this width does as well
-        plan = next((p for k, p in cache.items() if k[:5] == key[:5] and k[5] in (1, 3)), None)
-        if plan is not None:
-            return plan
-    if plan is None:
-        plan = _spmm.make_plan(packed, N, np_, n_cta, mode, chunk_tiles, offsets)
-        cache[key] = plan
+    if plan is not None and plan.serves(a, packed):
+        return plan
+    if torch.cuda.is_current_stream_capturing():
+        # Nothing can be built here: a plan of either kind that is kept for this width and this tile list does as well.
+        if not per_worker:
+            plan = next((p for k, p in cache.items() if k[:5] == key[:5] and k[5] in (1, 3) and p.serves(a, packed)), None)
+            if plan is not None:
+                return plan
+        raise _lib.VoidB200Error("a work plan cannot be built inside a stream capture: multiply the tensor once, with %d columns "
+                                 "and its tile list as it is now, before the capture" % N)
+    plan = _spmm.make_plan(packed, N, np_, n_cta, mode, chunk_tiles, offsets)
+    plan.tile_list = _lib.native().identity(a.block_rows, a.block_cols)
+    cache[key] = plan
     return plan
 
 
