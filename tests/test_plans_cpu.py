@@ -88,3 +88,20 @@ def test_a_store_of_the_same_list_takes_the_plan_that_is_kept(host):
     with pytest.raises(_lib.VoidB200Error, match="capture"):
         stream_k._plan_for(a, other, 256, None, False, None)
     assert host.built == 1
+
+
+def test_plans_that_a_graph_reads_stay_when_a_store_of_no_graph_is_replaced():
+    """One that a product packed inside a capture took, and one of a tensor that is packed for a further operand type."""
+    def plan(captured):
+        p = object.__new__(_spmm.Plan)
+        p.captured = captured
+        return p
+
+    a, read, other = Tensor(10), plan(True), plan(False)
+    a._plan_cache = {1: read, 2: other}
+    _spmm.retire(a, SimpleNamespace(native=None), None)
+    a._plan_cache = {}
+    assert any(p is read for _, plans in a._captured_stores for p in plans)
+    assert not any(p is other for _, plans in a._captured_stores for p in plans)
+    _spmm.retire(a, None)
+    assert len(a._captured_stores) == 1

@@ -65,3 +65,36 @@ def test_a_capture_after_an_edit_of_the_tiles_alone(kind):
     torch.cuda.synchronize()
     _same(kind, out, want * 2)
     void.check_device_status()
+
+
+@pytest.mark.parametrize("how", ["edited tiles", "another operand type"])
+def test_a_graph_keeps_its_plan_when_the_tensor_is_packed_again(how):
+    t, _ = _case("fp32", 5) if how == "another operand type" else _case("int8", 5)
+    n = 160
+    b = torch.randint(-3, 4, (t.shape[1], n), device="cuda")
+    if how == "another operand type":
+        t, b = t.to_dtype(torch.float16), b.half()
+        t.values.round_()                               # whole numbers: sums do not depend on the order
+        product = lambda out=None: void.void_spmm_stream_k(t, b, out=out)
+    else:
+        b = b.to(torch.int8)
+        product = lambda out=None: void.void_spmm_stream_k(t, b, out=out)
+    product()
+    if how == "edited tiles":
+        t.scales.mul_(2)
+    torch.cuda.synchronize()
+    plan = next(iter(t._plan_cache.values()))
+    out, graph = torch.empty(t.shape[0], n, dtype=b.dtype if b.is_floating_point() else torch.float32, device="cuda"), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        product(out)
+    want = product()
+    if how == "another operand type":
+        void.void_spmm(t, b.float())
+    assert not any(p is plan for p in t._plan_cache.values())
+    assert any(p is plan for _, plans in t._captured_stores for p in plans)
+    del plan
+    junk = [torch.full((k,), 0x55, dtype=torch.uint8, device="cuda") for k in (512, 4096, 1 << 14, 1 << 16, 1 << 18) for _ in range(40)]
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want) and len(junk) == 200
+    void.check_device_status()

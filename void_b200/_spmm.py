@@ -115,11 +115,13 @@ def allow_group_stores(a, allowed: bool) -> None:
 
 
 def retire(owner, *stores) -> None:
-    """Stores of ``owner`` whose place is being taken: those that a captured graph reads, and their plans, stay as long as
-    ``owner`` does, so that a replay reads what it was captured with."""
+    """Stores of ``owner`` whose place is being taken, and its plans, which go with them: those that a captured graph reads stay as
+    long as ``owner`` does, so that a replay reads what it was captured with.  (A graph may read a plan and none of these stores:
+    that of a product packed inside its capture, or of another operand type.)"""
     kept = [p for p in stores if p is not None and p.native is not None and _lib.native().packed_captured(p.native)]
-    if kept:
-        owner.__dict__.setdefault("_captured_stores", []).append((kept, owner.__dict__.get("_plan_cache")))
+    plans = [p for p in list(owner.__dict__.get("_plan_cache", {}).values()) if p.captured]
+    if kept or plans:
+        owner.__dict__.setdefault("_captured_stores", []).append((kept, plans))
 
 
 def new_store(owner, p: PackedTiles, *made_from) -> PackedTiles:
@@ -182,6 +184,7 @@ class Plan:
     row_ptr: Optional[torch.Tensor] = None
     tile_list: object = None
     shape: Optional[tuple] = None
+    captured: bool = field(default=False, init=False)   # a graph reads it
     scratch: dict = field(default_factory=dict, init=False, repr=False)   # launch key: (partials, counters)
 
     def __post_init__(self):
@@ -196,6 +199,8 @@ class Plan:
 
     def native_args(self) -> tuple:
         key = _lib.native().launch_key(self.counters.device.index)
+        if key == CAPTURED:
+            self.captured = True
         partials, counters = self.scratch.get(key) or self._new_scratch(key)
         return self.segs, self.cta_seg_ptr, self.n_cta, partials, counters, self.np
 
