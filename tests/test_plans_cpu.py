@@ -13,6 +13,7 @@ class Tensor:
 
     def set_list(self, tiles):
         self.block_rows, self.block_cols = torch.arange(tiles, dtype=torch.int32), torch.zeros(tiles, dtype=torch.int32)
+        self.n_blocks = tiles
 
 
 def _store(nbr=40, kind=_lib.KIND_I8):
@@ -30,12 +31,12 @@ def host(monkeypatch):
         plan.row_ptr, plan.tile_list, plan.shape, plan.mode = packed.row_ptr, None, packed.shape, mode
         return plan
 
-    def cached_workload(a, packed):
-        assert not state.capturing, "the worker table is read back on the host"
-        return SimpleNamespace(chunk_tiles=16, worker_offsets=None)
+    def workload(a):
+        assert not state.capturing, "the size of a worker table is read back on the host"
+        return SimpleNamespace(chunk_tiles=16, worker_offsets=None, total_work=a.n_blocks)
 
     monkeypatch.setattr(_spmm, "make_plan", make_plan)
-    monkeypatch.setattr(stream_k, "_cached_workload", cached_workload)
+    monkeypatch.setattr(stream_k, "compute_stream_k_workload", workload)
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: state.capturing)
     return state
 
@@ -105,3 +106,28 @@ def test_plans_that_a_graph_reads_stay_when_a_store_of_no_graph_is_replaced():
     assert not any(p is other for _, plans in a._captured_stores for p in plans)
     _spmm.retire(a, None)
     assert len(a._captured_stores) == 1
+
+
+@pytest.mark.parametrize("warm,captured", [(TABLE, None), (None, TABLE), (None, None), (TABLE, TABLE)])
+@pytest.mark.parametrize("n_cta", [None, 1025])
+def test_a_captured_product_finds_the_plan_of_the_other_way(host, warm, captured, n_cta):
+    """From 1025 CTAs on the shares are cut along a table, which cannot be built inside a capture."""
+    a, store = Tensor(100), _store()
+    plan = stream_k._plan_for(a, store, 256, warm, False, n_cta)
+    assert plan.mode == (1 if warm is not None or n_cta == 1025 else 3)
+    host.capturing = True
+    assert stream_k._plan_for(a, store, 256, captured, False, n_cta) is plan
+
+
+def test_a_further_width_may_be_added_while_a_kept_plan_is_looked_for(host):
+    a, store = Tensor(100), _store()
+    plan = stream_k._plan_for(a, store, 256, TABLE, False, None)
+
+    class Key(tuple):
+        def __getitem__(self, i):                       # (looked at while the plans are walked)
+            a._plan_cache[len(a._plan_cache)] = plan
+            return tuple.__getitem__(self, i)
+
+    a._plan_cache = {Key(("streamk", store.kind, 128, 1, 592, 1, 16)): plan, **a._plan_cache}
+    host.capturing = True
+    assert stream_k._plan_for(a, store, 256, None, False, None) is plan

@@ -98,3 +98,22 @@ def test_a_graph_keeps_its_plan_when_the_tensor_is_packed_again(how):
     torch.cuda.synchronize()
     assert torch.equal(out, want) and len(junk) == 200
     void.check_device_status()
+
+
+@pytest.mark.parametrize("kind", ["int8", "fp32"])
+def test_a_capture_without_a_table_takes_the_plan_that_was_made_along_one(kind):
+    """Beyond 1024 CTAs shares are cut along a table either way; one that is given is not kept on the tensor."""
+    w = workloads.block_sparse(workloads.zipf_mask(40, 64, 1.5, 60, 8.0, seed=6), 160, seed=6)
+    t, b, scale = w.a, w.b, None
+    if kind == "int8":
+        t = void.quantize_void_tensor(w.a)
+        b, scale = void.quantize_cols_int8(w.b)
+    want = void.void_spmm_stream_k(t, b, void.compute_stream_k_workload(t), b_scale=scale, n_cta=1025)
+    out, graph = torch.empty_like(want), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        void.void_spmm_stream_k(t, b, None, out, b_scale=scale, n_cta=1025)
+    graph.replay()
+    torch.cuda.synchronize()
+    _same(kind, out, want)
+    void.check_device_status()

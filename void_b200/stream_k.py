@@ -60,8 +60,8 @@ def _plan_for(a, packed, N: int, workload: Optional[StreamKWorkload], per_worker
     n_chunks = (N + _spmm.PANEL * np_ - 1) // (_spmm.PANEL * np_)
     mode = 2 if per_worker else (1 if workload is not None else _spmm.split_mode(packed.nbr, n_chunks, n_cta))
     if mode != 3 and workload is None:
-        workload = _cached_workload(a, packed)
-    chunk_tiles, offsets = (0, None) if mode == 3 else (workload.chunk_tiles, workload.worker_offsets)
+        workload = _cached_workload(a, packed)   # (none inside a capture, unless it is kept)
+    chunk_tiles, offsets = (0, None) if mode == 3 or workload is None else (workload.chunk_tiles, workload.worker_offsets)
     key = ("streamk", packed.kind, N, np_, n_cta, mode, chunk_tiles)
     cache = getattr(a, "_plan_cache", None)
     if cache is None:
@@ -71,8 +71,8 @@ def _plan_for(a, packed, N: int, workload: Optional[StreamKWorkload], per_worker
         return plan
     if torch.cuda.is_current_stream_capturing():
         # Nothing can be built here: a plan of either kind that is kept for this width and this tile list does as well.
-        if not per_worker:
-            plan = next((p for k, p in cache.items() if k[:5] == key[:5] and k[5] in (1, 3) and p.serves(a, packed)), None)
+        if not per_worker:   # (another thread may be adding one for a further width)
+            plan = next((p for k, p in list(cache.items()) if k[:5] == key[:5] and k[5] in (1, 3) and p.serves(a, packed)), None)
             if plan is not None:
                 return plan
         raise _lib.VoidB200Error("a work plan cannot be built inside a stream capture: multiply the tensor once, with %d columns "
@@ -120,10 +120,13 @@ def void_spmm_stream_k(a: Int8VOIDTensor, b: torch.Tensor, workload: Optional[St
                               activation, False, opts)
 
 
-def _cached_workload(a, packed) -> StreamKWorkload:
-    """The table depends on A's structure only: built once per tile index, then reused."""
+def _cached_workload(a, packed) -> Optional[StreamKWorkload]:
+    """The table depends on A's structure only: built once per tile index, then reused.  Its size is read back, so that inside a
+    stream capture there is only the one that is kept."""
     row_ptr, workload = getattr(a, "_streamk_workload_cache", (None, None))
     if row_ptr is not packed.row_ptr or workload.total_work != a.n_blocks:
+        if torch.cuda.is_current_stream_capturing():
+            return None
         workload = compute_stream_k_workload(a)
         a._streamk_workload_cache = packed.row_ptr, workload
     return workload
