@@ -1,6 +1,7 @@
 """Which kept work plan a power-law product takes: host logic, with the packed store and the capture state replaced by stand-ins."""
 from types import SimpleNamespace
 
+import numpy as np
 import pytest
 import torch
 
@@ -131,3 +132,24 @@ def test_a_further_width_may_be_added_while_a_kept_plan_is_looked_for(host):
     a._plan_cache = {Key(("streamk", store.kind, 128, 1, 592, 1, 16)): plan, **a._plan_cache}
     host.capturing = True
     assert stream_k._plan_for(a, store, 256, None, False, None) is plan
+
+
+@pytest.mark.parametrize("seed,n_cta,heavy,tiles,light", [(0, 64, 32, 100, 640), (1, 64, 4, 1000, 700), (2, 592, 40, 500, 4000), (3, 592, 300, 60, 6000),
+                                                          (4, 1024, 16, 5000, 6000)])
+@pytest.mark.parametrize("n_chunks", [1, 0])
+def test_dealt_segments_go_where_the_least_is(seed, n_cta, heavy, tiles, light, n_chunks):
+    """Few heavy rows among many light ones, several segments per CTA (which is why a piece costs four rows).  A CTA that takes a light
+    row late is among the quarter with the least, so that none ends more than two light rows above the mean, unless it is by its one
+    heavy segment; the same segments dealt in turn, in their order by weight, end above that."""
+    from test_abi_cpu import _check_plan
+    rng, cost = np.random.default_rng(seed), _spmm.ROW_COST
+    cnt = rng.permutation(np.concatenate([np.full(heavy, tiles), rng.integers(1, 6, light)]))
+    row_ptr = np.concatenate([[0], np.cumsum(cnt)]).astype(np.int32)
+    n_chunks = n_chunks or max(1, (8190 - 2 * n_cta) // len(cnt))
+    segs, cptr = _check_plan(row_ptr, n_chunks, n_cta, 3, 0, cost)
+    assert len(segs) >= n_cta
+    costs = segs[:, 3] - segs[:, 2] + np.where(segs[:, 4] > 1, 4 * cost, cost)
+    load = np.bincount(np.repeat(np.arange(n_cta), np.diff(cptr)), costs, n_cta)
+    in_turn = np.bincount(np.arange(len(segs)) % n_cta, np.sort(costs)[::-1], n_cta)
+    most = max(costs.max(), load.mean() + 2 * (5 + cost))
+    assert load.max() <= most < in_turn.max()
