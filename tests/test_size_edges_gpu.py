@@ -637,3 +637,21 @@ def test_results_staged_in_the_ring_are_those_stored_directly(kind, rows, k, n):
             outs.append(out)
         assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
     void.check_device_status()
+
+
+@pytest.mark.parametrize("kind,stages", [("int8", 2), ("int8", 3), ("int8", 9), ("int8", 10), ("int8", 14), ("fp8", 2), ("fp8", 12), ("fp8", 13), ("fp8", 16)])
+def test_rings_of_as_many_ordinary_stages_as_are_asked_for(kind, stages):
+    """One item per CTA, three CTAs per SM and 16-bit results: 14 stages of three INT8 units, 16 of two FP8 units of two terms fit a
+    CTA's shared memory."""
+    from void_b200 import _lib, _spmm, workloads
+    w = workloads.block_sparse(workloads.uniform_mask(110, 40, 0.4, seed=stages), 384, seed=stages)
+    if kind == "int8":
+        p, (b, scale) = void.quantize_void_tensor(w.a).packed(), void.quantize_cols_int8(w.b)
+    else:
+        p, (b, scale) = void.void_tensor_to_fp8(w.a).packed_split(2), void.quantize_cols_fp8(w.b)[:2]
+    outs = []
+    for s in (0, stages):
+        outs.append(torch.full((3520, 384), 7.0, dtype=torch.float16, device="cuda"))
+        _spmm.spmm(p, b, outs[-1], scale_mode=_lib.SCALE_ROW_MEAN, col_scale=scale, panels_per_item=1, stages=s)
+    assert torch.equal(*outs)
+    void.check_device_status()

@@ -383,11 +383,12 @@ static int spmm_launch(const void_spmm_args* a, int kind, cudaStream_t stream) {
   // 65.1, 4 x 2: 6.96 / 10.87 / 69.4, 9 x 1: 8.64 / 16.2 / 111); stages of one or two tiles pay the fixed cost of a stage
   // too often.  With fewer CTAs on the SM longer stages pay (1024 x 8192, 70 %, N = 256, one CTA per SM: INT8 3 x 3 12.4
   // us, 7 x 6 10.4; FP8 of two terms 17.4 -> 13.3; fp16 21.5 -> 13.4 with 6 x 3; fp32 41.2 -> 25.3 with 8 x 1).
+  const bool longer = single && a->stages == 0;   // (a number of stages that is asked for is one of the ordinary length)
   if (group == 0) {
     if (floating) group = (es == 2 && np == 1) ? ((tr_b && share > 1) || slim ? 2 : 3) : 1;
     // (a tile stored as several terms is that much longer: 3 stages x 2 at four CTAs, headline 7.66 us, 2 x 3: 7.93)
-    else if (a->tile_terms > 1) group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 3 : (single && a->tile_terms == 2 ? 3 : 2))) : 1;
-    else group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 4 : (single ? 5 : 3))) : 2;
+    else if (a->tile_terms > 1) group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 3 : (longer && a->tile_terms == 2 ? 3 : 2))) : 1;
+    else group = np == 1 ? (share == 1 ? 6 : (share == 2 ? 4 : (longer ? 5 : 3))) : 2;
   }
   if (group < 1 || group > 8) return VOID_ERR_BAD_ARG;
   if (drain && np == 1 && shape != 1 && a->tiles_per_stage == 0) group = 2;
