@@ -401,12 +401,13 @@ typedef struct void_spmm_args {
  * out in the order their block columns meet B: stages of at most max_entries block columns and max_tiles tiles; behind the
  * tiles lies what the kernel is told about each stage.  void_group_build makes that store from a packed one (void_pack_tiles,
  * void_pack_tiles_fp; tile_bytes = 1024 * element bytes):
- *   group_rows [n_groups * 16], stage_ptr [n_groups + 1], records [8 * nnz], blob (nnz * (tile_bytes + 128) bytes,
+ *   group_rows [n_groups * 16], stage_ptr [n_groups + 1], records [8 * nnz], blob (nnz * (tile_bytes + VOID_GROUP_HEAD_BYTES) bytes,
  *   128-byte aligned), ws [2 * n_groups + nnz]; row_order as in void_spmm_args (rows are dealt to the groups in that order
  *   back and forth), or NULL; n_groups * 16 >= nbr and ceil(nbr / n_groups) <= 8; max_tiles <= 32; max_entries <= 6.
  * void_spmm_grouped multiplies it: args as for void_spmm_i8 / _fp (tiles, tile_cols and tile_scales are not read; no
  * plan, no raw accumulators); args->transposed 0 or 2.
  * ------------------------------------------------------------------------------------- */
+#define VOID_GROUP_HEAD_BYTES 32
 typedef struct void_group_store {
   const void* blob;
   const int32_t* records;

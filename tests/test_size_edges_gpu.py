@@ -655,3 +655,45 @@ def test_rings_of_as_many_ordinary_stages_as_are_asked_for(kind, stages):
         _spmm.spmm(p, b, outs[-1], scale_mode=_lib.SCALE_ROW_MEAN, col_scale=scale, panels_per_item=1, stages=s)
     assert torch.equal(*outs)
     void.check_device_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.int8, torch.float16, torch.float32])
+def test_a_group_store_takes_what_its_kernels_use(dtype):
+    """Tiles, 32 bytes of heads and a record of 32 bytes each; what belongs to groups and rows is within the slack."""
+    from void_b200 import _lib, ops, workloads
+    w = workloads.block_sparse(workloads.uniform_mask(157, 61, 0.1, seed=3), 1500, seed=3)
+    if dtype == torch.int8:
+        a, (b, scale) = void.quantize_void_tensor(w.a), void.quantize_cols_int8(w.b)
+        product, packed = lambda: void.void_spmm_int8(a, b, scale), lambda: a.packed()
+    else:
+        a, b = w.a.to_dtype(dtype), w.b.to(dtype)
+        product, packed = lambda: void.void_spmm(a, b), lambda: ops.packed_fp(a, ops.product_kind(a, b))
+    for _ in range(4):
+        product()
+        torch.cuda.synchronize()
+    assert _lib.native().packed_grouped(packed().native, None)[1] == 1
+    requested = lambda: torch.cuda.memory_stats()["requested_bytes.all.current"]
+    before = requested()
+    void.allow_group_stores(a, False)
+    assert 0 < before - requested() - a.n_blocks * 1024 * a.values.element_size() <= a.n_blocks * 64 + 32768
+
+
+@pytest.mark.parametrize("es", [1, 2, 4])
+def test_a_group_store_is_written_inside_its_blob(es):
+    """Every tile a stage of its own, so that there are as many heads as there can be."""
+    from void_b200 import _lib
+    lib, P = _lib.load(), _lib.ptr
+    nbr, nbc, groups = 24, 37, 3
+    nnz, ints = nbr * nbc, dict(dtype=torch.int32, device="cuda")
+    row_ptr, cols = torch.arange(0, nnz + 1, nbc, **ints), torch.arange(nbc, **ints).repeat(nbr)
+    tiles = torch.randint(0, 255, (nnz * 1024 * es,), dtype=torch.uint8, device="cuda")
+    rows, stages, records, ws = (torch.zeros(n, **ints) for n in (groups * 16, groups + 1, 8 * nnz, 2 * groups + nnz))
+    size = nnz * (1024 * es + 32)
+    blob = torch.full((size + 4096,), 0xa5, dtype=torch.uint8, device="cuda")
+    _lib.check(lib.void_group_build(P(row_ptr), None, P(cols), P(tiles), nbr, nnz, es, groups, 1, 1, P(rows), P(stages), P(records), P(blob),
+                                    P(ws), _lib.stream_ptr(blob.device)), "void_group_build")
+    assert stages.tolist() == [0, nnz // 3, 2 * nnz // 3, nnz] and bool((blob[size:] == 0xa5).all())
+    place = ws[2 * groups:].long()
+    assert torch.equal(blob[:nnz * 1024 * es].view(nnz, -1)[place], tiles.view(nnz, -1))
+    heads = blob[nnz * 1024 * es:size].view(2, nnz, 16)
+    assert torch.equal(heads[:, :, 1].sum(0), torch.ones(nnz, dtype=torch.int64, device="cuda"))     # one run in all per stage

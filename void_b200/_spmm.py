@@ -104,7 +104,7 @@ def _mark_ready(p: PackedTiles) -> PackedTiles:
 def allow_group_stores(a, allowed: bool) -> None:
     """Whether products of ``a`` (VOIDTensor, Int8VOIDTensor) may keep its tiles a second time, laid out for groups of tile
     rows (by default they may).  From the third large product on of a tensor whose tile rows share enough block columns (up to
-    85 - 90 % sparsity), such a store - as large as the packed tiles and an eighth more for 8-bit tiles, at most 4 GB, for up to
+    85 - 90 % sparsity), such a store - as large as the packed tiles and a sixteenth more for 8-bit tiles, at most 4 GB, for up to
     two widths of B - is built behind a product and used once it is complete.  False gives the stores of ``a`` back - those that a
     captured graph reads, with ``a`` itself - and keeps further ones from being built."""
     a._group_stores = bool(allowed)

@@ -48,6 +48,7 @@ constexpr int kMaxStageTiles = 32;   // tiles per stage (a lane each while they 
 constexpr int kRecordWords = 8;
 constexpr int kHeadBytes = 16;       // of a stage, per class: its first tile, its number of runs, then a byte for each run
 constexpr int kMaxRuns = kHeadBytes - 2;
+static_assert(kClasses * kHeadBytes == VOID_GROUP_HEAD_BYTES, "room for the heads of as many stages as there are tiles");
 constexpr int kMaxRing = 12;
 constexpr int kThreads = 32 * (kProducers + kClasses + kEpiWarps);
 constexpr int kNone = 0x7fffffff;

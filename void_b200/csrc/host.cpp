@@ -471,6 +471,7 @@ bool complete(GroupStore* g, void_stream_t st) {
   g->built = nullptr;
   return true;
 }
+int64_t group_blob_bytes(const Packed* p) { return p->args.nnz * (1024 * (int64_t)elem_bytes(p->kind) + VOID_GROUP_HEAD_BYTES); }
 // Queues the kernels that lay the tiles out for G groups; null where there is no memory for it.
 std::unique_ptr<GroupStore> build_group_store(const Packed* p, int64_t G, void_stream_t st) {
   std::unique_ptr<GroupStore> g(new GroupStore);
@@ -479,7 +480,7 @@ std::unique_ptr<GroupStore> build_group_store(const Packed* p, int64_t G, void_s
   try {
     const c10::Device dev(c10::kCUDA, p->device);
     g->index = new_cuda({16 * G + (G + 4) / 4 * 4 + 8 * nnz}, at::kInt, dev);
-    g->blob = new_cuda({nnz * (1024 * es + 128) + 128}, at::kByte, dev);
+    g->blob = new_cuda({group_blob_bytes(p) + 128}, at::kByte, dev);
     ws = new_cuda({2 * G + nnz}, at::kInt, dev);
   } catch (const c10::OutOfMemoryError&) {
     return nullptr;
@@ -518,8 +519,7 @@ GroupStore* group_store(Packed* p, int64_t N, void_stream_t st) {
     best = std::max(best, saves);
     if (saves > hit_saves && complete(p->groups[n].get(), st)) { hit = p->groups[n].get(); hit_saves = saves; }
   }
-  const int64_t bytes = p->args.nnz * (1024 * (int64_t)elem_bytes(p->kind) + 128);
-  if (best < 0.93 * shape.saves && n < kMaxGroupStores && p->stable && bytes <= (4ll << 30) && p->group_calls >= 0 && !capturing(st) &&
+  if (best < 0.93 * shape.saves && n < kMaxGroupStores && p->stable && group_blob_bytes(p) <= (4ll << 30) && p->group_calls >= 0 && !capturing(st) &&
       ++p->group_calls >= 3) {
     p->group_calls = -1;   // for good, if there is no room for it
     p->groups[n] = build_group_store(p, shape.groups, st);
