@@ -170,22 +170,6 @@ __device__ __forceinline__ void finish16(const OutDesc& o, int row, int n, int m
   }
 }
 
-// Sixteen finished 16-bit values of output column n into a staging tile [32 m][PITCH n] in shared memory
-// (stage_col points at element [0][n - n0]); same arithmetic as finish16.
-template <int KIND, int PITCH, bool ACT = true>
-__device__ __forceinline__ void finish16_stage(const OutDesc& o, int row, int n, int m0, const uint32_t* r,
-                                               float row_scale, float cs, float bias, uint16_t* stage_col) {
-  float v[16];
-  finished<KIND, 8, ACT>(o, row * kTile + m0, r, row_scale, cs, bias, v);
-#pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    uint16_t h;
-    if (o.dtype == VOID_OUT_F16) h = __half_as_ushort(__float2half_rn(v[k]));
-    else h = __bfloat16_as_ushort(__float2bfloat16_rn(v[k]));
-    stage_col[(m0 + k) * PITCH] = h;
-  }
-}
-
 // A warp's 32 columns of a tile row of raw accumulators, as fragments (tmem_ld_fragments: lanes are columns), to finished
 // 16-bit values in a part of shared memory, rows of 64 bytes whose 16-byte pieces lie as the copy engine's 64-byte swizzle
 // has them (piece ^ row / 2 % 4; a part starts on 512 bytes).  cs and bias: those of the lane's own column.

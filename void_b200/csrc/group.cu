@@ -42,7 +42,7 @@ constexpr int kCtas = 2, kProducers = 2, kClasses = 2, kEpiWarps = 4;
 constexpr int kMmaWarp0 = kProducers, kEpiWarp0 = kMmaWarp0 + kClasses;
 constexpr int kClassRows = 4;                    // tile rows whose products one MMA warp issues
 constexpr int kMaxRows = kClasses * kClassRows;   // tile rows of a group: their accumulators fill the CTA's tensor memory
-constexpr int kMaxGroupRows = 16;                 // and the places group_rows has for them
+constexpr int kMaxGroupRows = 16;                 // and the places group_rows has for them (callers size it by the header)
 constexpr int kMaxEntries = 6;       // block columns per stage (what a record holds)
 constexpr int kMaxStageTiles = 32;   // tiles per stage (a lane each while they are laid out)
 constexpr int kRecordWords = 8;
@@ -364,7 +364,8 @@ __global__ void group_rows_kernel(const int32_t* __restrict__ row_order, int nbr
   group_rows[i] = row;
 }
 
-constexpr unsigned kClassStarts = 0x1111u;      // first rows of the classes
+constexpr unsigned kClassStarts = 0x11u;        // first rows of the classes
+static_assert(kClasses == 2 && kClassRows == 4, "kClassStarts");
 constexpr uint32_t kRunStart = 1u << 8;         // (marks a run's byte while a stage is open)
 __device__ __forceinline__ unsigned class_lanes(int k) { return ((1u << kClassRows) - 1u) << (k * kClassRows); }   // rows of MMA warp k
 // One warp per group merges its rows' sorted column lists, lane r holding row r's place.  Pass 1 counts the group's stages;
@@ -465,7 +466,7 @@ __global__ void __launch_bounds__(128) group_walk_kernel(const int32_t* __restri
   if (!EMIT && lane == 0) counts[g] = stage;
 }
 
-// stage_ptr and blob_base from the groups' stage and tile counts, by one block
+// stage_ptr and tile_base from the groups' stage and tile counts, by one block
 __global__ void __launch_bounds__(1024) group_scan_kernel(const int32_t* __restrict__ counts, const int32_t* __restrict__ row_ptr,
                                                           const int32_t* __restrict__ group_rows, int n_groups,
                                                           int32_t* __restrict__ stage_ptr, int32_t* __restrict__ tile_base) {
