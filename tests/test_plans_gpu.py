@@ -1,9 +1,11 @@
 """Work plans of power-law products: which tile list they were made for, and how long graphs may read them."""
+import ctypes
+
 import pytest
 import torch
 
 import void_b200 as void
-from void_b200 import workloads
+from void_b200 import _lib, _spmm, stream_k, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -117,3 +119,63 @@ def test_a_capture_without_a_table_takes_the_plan_that_was_made_along_one(kind):
     torch.cuda.synchronize()
     _same(kind, out, want)
     void.check_device_status()
+
+
+# ------------------------------------------------------------------------------------------ the plan of a product without a table
+DROP_FIRST_GROUP = 1 << 16      # test hook: the producers never deliver a CTA's first group of tiles
+
+
+def _dealt():
+    w = workloads.block_sparse(workloads.zipf_mask(64, 256, 1.5, 200, 10.0, seed=7), 256, seed=7)
+    q = void.quantize_void_tensor(w.a)
+    b, scale = void.quantize_cols_int8(w.b)
+    product = lambda: void.void_spmm_stream_k(q, b, b_scale=scale, out_dtype=torch.float16, n_cta=48)
+    want = product()
+    plan = stream_k.stream_k_plan(q, 256, None, n_cta=48)
+    assert plan is next(iter(q._plan_cache.values())) and plan.mode == 3 and plan.n_counters >= 2
+    void.check_device_status()
+    return q, b.contiguous(), scale, product, want, plan
+
+
+def test_a_dealt_launch_that_gave_up_leaves_no_partial_sums_behind():
+    """The wait for the ring is limited to 5 ms."""
+    q, b, scale, product, want, plan = _dealt()
+    _spmm.spmm(q.packed(), b, torch.zeros_like(want), scale_mode=_lib.SCALE_ROW_MEAN, col_scale=scale, plan=plan, test_hooks=DROP_FIRST_GROUP | 5)
+    torch.cuda.synchronize()
+    with pytest.raises(void.VoidB200Error, match="wait gave up"):
+        void.check_device_status()
+    assert not plan.partials.any() and not plan.counters.any()
+    assert torch.equal(product(), want)
+    void.check_device_status()
+
+
+def test_a_dealt_plan_that_points_outside_its_scratch_is_reported_not_followed():
+    q, b, scale, product, want, plan = _dealt()
+    room = (plan.n_counters - 1) * plan.np * 128 * 32                 # for one split row less than the plan needs
+    guard = torch.zeros(room + plan.np * 128 * 32 + 4096, dtype=torch.int32, device="cuda")
+    short = _spmm.Plan(plan.segs, plan.cta_seg_ptr, plan.n_cta, plan.np, plan.n_chunks, plan.n_segs, plan.n_slots, plan.n_counters,
+                       guard[:room], torch.zeros_like(plan.counters), plan.mode, plan.chunk_tiles)
+    _spmm.spmm(q.packed(), b, torch.zeros_like(want), scale_mode=_lib.SCALE_ROW_MEAN, col_scale=scale, plan=short)
+    torch.cuda.synchronize()
+    assert not guard[room:].any()
+    with pytest.raises(void.VoidB200Error, match="does not fit"):
+        void.check_device_status()
+    assert torch.equal(product(), want)
+    void.check_device_status()
+
+
+def test_a_dealt_plan_with_scratch_inside_the_library():
+    q, b, scale, product, want, plan = _dealt()
+    for _ in range(2):
+        out = torch.full_like(want, float("nan"))
+        p, a = q.packed(), _lib.SpmmArgs()
+        a.tiles, a.tile_cols, a.tile_scales = p.tiles.data_ptr(), p.tile_cols.data_ptr(), p.tile_scales.data_ptr()
+        a.row_ptr, a.row_scale, a.nbr, a.nbc, a.nnz = p.row_ptr.data_ptr(), p.row_scale.data_ptr(), p.nbr, p.nbc, p.nnz
+        a.b, a.ldb, a.K, a.N, a.col_scale, a.b_scale = b.data_ptr(), b.stride(0), b.shape[0], b.shape[1], scale.data_ptr(), 1.0
+        a.out, a.ldc, a.M, a.out_dtype, a.scale_mode = out.data_ptr(), out.stride(0), out.shape[0], _lib.OUT_DTYPE_CODE[out.dtype], _lib.SCALE_ROW_MEAN
+        a.segs, a.cta_seg_ptr, a.n_cta, a.panels_per_item = plan.segs.data_ptr(), plan.cta_seg_ptr.data_ptr(), plan.n_cta, plan.np
+        a.status = _lib.status_word(out.device).data_ptr()
+        _lib.check(_lib.load().void_spmm_i8_static_scratch(ctypes.byref(a), plan.n_counters, _lib.stream_ptr()), "void_spmm_i8_static_scratch")
+        torch.cuda.synchronize()
+        void.check_device_status()
+        assert torch.equal(out, want)
