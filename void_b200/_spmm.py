@@ -262,12 +262,15 @@ def streamk_table(row_ptr: torch.Tensor, nbr: int, nnz: int, n_workers: Optional
     return rows[:n], start[:n], end[:n], atomic[:n].to(torch.bool), woff, target
 
 
-ROW_COST = 8   # epilogue of one (tile row, chunk) in units of one tile of work, swept on B200 (power-law rows, N = 256 / 1024, us: 4 15.6 / 45.7, 6 14.4 / 39.4, 8 13.9 / 37.0, 12 14.0 / 37.4, 16 14.8 / 39.4)
+ROW_COST = 8   # epilogue of one (tile row, chunk) in units of one tile of work, swept on B200 (power-law rows, N = 256 / 1024, us: 4 15.6 / 45.7, 6 14.4 / 39.4, 8 13.9 / 37.0, 12 14.0 / 37.4, 16 14.8 / 39.4; with contiguous shares: dealt plans take it for whole rows as it is, and four of it for a piece)
 
 
 def split_mode(nbr: int, n_chunks: int, n_cta: int) -> int:
     """How heavy tile rows are split (split_rows of void_plan_segments): the segments dealt out by weight (3) as long as one
-    block can sort them, else contiguous shares (1), whose many segments per CTA even out by themselves."""
+    block can sort them in shared memory, else contiguous shares (1).  Dealt ones were the faster at every size measured below
+    that line (27 from 2048 x 2048 to 56000 x 4096; contiguous and dealt, us: 10 - 28 % up to 1300 segments, 30000 x 3000, N = 60 10.7 8.7;
+    4096 segments 56.8 51.7, 6400 67.9 61.3 and 56.6 55.5, 7000 61.4 56.9, 5500 of shorter rows 43.7 43.5), so what lies beyond it is
+    left for want of room, not because shares even out there."""
     return 3 if n_cta <= 1024 and nbr * n_chunks + 2 * n_cta + 2 <= 8192 else 1
 
 

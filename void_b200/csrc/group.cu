@@ -6,8 +6,8 @@
 // columns in tensor memory, and walks the block columns that ANY of its rows stores: a panel is fetched once and multiplied
 // by the 1 ... R tiles of that column.  With density d a panel serves R d / (1 - (1 - d)^R) tiles: 1.4 at 90 % sparsity and
 // R = 8, 2.3 at 70 % and R = 7, 3.5 at 50 %.  Measured against that kernel, us (back to back, one size after the other): fp16
-// 8192^2, N = 1024 50 % 120 -> 79, 70 % 85 -> 63, 80 % 57 -> 46, 90 % 31 -> 29; 4096 x 16384, N = 2048 90 % 65 -> 56; fp32 8192^2 50 % 256
-// -> 148, 70 % 175 -> 126, 80 % 118 -> 93; INT8 50 % 60 -> 42, 70 % 40 -> 33, slower from 85 % on.
+// 8192^2, N = 1024 50 % 120 -> 79, 70 % 85 -> 63, 80 % 57 -> 46, 90 % 31 -> 29; 4096 x 16384, N = 2048 90 % 65 -> 56; fp32 8192^2 50 % 255
+// -> 152, 70 % 157 -> 119, 80 % 108 -> 86; INT8 50 % 60 -> 42, 70 % 40 -> 33, slower from 85 % on.
 //
 // What is left is the chain of a CTA's stages: wait, products, commit take its warps about 550 clocks a stage whatever is in it
 // (an answered wait 100, a product 44 - 60, the bookkeeping the rest), so a stage takes what a third of the CTA's shared memory holds.

@@ -411,7 +411,9 @@ double group_saves(const Packed* p, int64_t N, int groups, int slots) {
 // What a stage holds: the split of a CTA's shared memory into stages of E block columns and T tiles with which the ring holds the
 // most block columns, T / (tiles that a column's panel serves) or E of them per stage.  Of equal ones that with three stages: a
 // stage costs the same chain of waits whatever is in it.  (8192^2, N = 1024, us: fp16 80 % 3 x (3 + 5) 46.2, 2 x (4 + 8) 49, 4 x (2 + 4) 49;
-// INT8 50 % 3 x (4 + 18) 42.0, 2 x (6 + 21) 43.6; fp32 50 % 3 x (1 + 5) 148, 2 x (2 + 4) 165, 80 % 2 x (2 + 5) 92.6, 4 x (1 + 2) 98.8.)
+// INT8 50 % 3 x (4 + 18) 42.0, 2 x (6 + 21) 43.6.)  The room is that beside staged results, which those of fp32 tiles are with an operand of 16
+// bits only; with all of it fp32 stages would hold a tile more: chosen and best seen, 50 % 3 x (1 + 4) 166, 3 x (1 + 5) 157, 70 % 4 x (1 + 2) 129,
+// 3 x (1 + 5) 117, 80 % 4 x (1 + 2) 93, 2 x (2 + 5) 90, but 16-bit results 3 x (1 + 4) 164, (1 + 5), of which two are left beside the staging, 185.
 void stage_shape(void_group_store& s, double tiles_per_column, int es) {
   const int room = 116736 - 3072 - 8192;   // half of an SM's shared memory less the kernel's own and the staging of its results
   double most = 0.0;
@@ -448,7 +450,8 @@ GroupShape group_shape(const Packed* p, int64_t N, int slots) {
 }
 // The saving from which the grouped kernel is the faster one; swept at 4096^2, 8192^2 (N = 1024), 16384 x 4096 and 4096 x 16384 (N = 2048),
 // 50 - 90 % sparsity.  Predicted saving and measured gain, fp16: 1.06 0.99 - 1.07, 1.09 1.01, 1.12 1.06 - 1.15, 1.12 1.10, 1.22 1.07, 1.36 1.14,
-// 1.52 1.24, 2.32 1.53; fp32 1.06 0.98, 1.15 1.07, 1.24 1.04, 1.38 1.13, 1.80 1.39, 2.32 1.72; INT8 1.36 - 1.38 0.99 - 1.01, 1.50 1.13, 1.52 1.06,
+// 1.52 1.24, 2.32 1.53; fp32 0.97 0.99, 1.03 1.08, 1.06 0.95, 1.09 1.19, 1.12 1.15, 1.15 1.15, 1.22 1.22, 1.24 1.12, 1.26 1.20,
+// 1.38 1.18, 1.40 1.24, 1.50 1.27 - 1.31, 1.52 1.25, 1.68 1.24, 1.80 1.32, 1.93 1.72, 2.17 1.70, 2.32 1.67; INT8 1.36 - 1.38 0.99 - 1.01, 1.50 1.13, 1.52 1.06,
 // 1.80 1.21, and with rows of 100 tiles 1.26 1.07, 1.40 1.11.
 double group_line(const Packed* p) {
   switch (p->kind) {

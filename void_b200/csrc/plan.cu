@@ -258,9 +258,10 @@ __global__ void __launch_bounds__(1024) plan_kernel(PlanIn in, PlanWs ws, int32_
 // to a CTA that has the least so far.  A piece costs what its tiles do and `piece` units more, since its sums travel through memory
 // and its last arriver reads them back: from time stamps, a CTA's end moves by 0.14 us per tile, 1.7 per whole row and 2.5 - 4 per
 // piece (16384^2, N = 256, power-law rows), so contiguous shares of equal tiles and rows ended between 8 and 15 us.  us, shares of
-// mode 1 and dealt: 16384^2, N = 256 14.9 13.0, N = 500 29.6 25.9, N = 1024 36.7 32.6; 32768 x 8192, N = 512 28.1 25.3; 8192 x 32768, N = 200
-// 16.8 15.6; 30000 x 3000, N = 60 11.1 8.7; 4096 x 8192, N = 128 8.1 6.2.  (A piece at 2, 3, 4, 6 row costs 13.5 13.2 13.0 14.8; limits
-// of 1.15, 1.3, 1.5, 2 shares 13.1 13.0 13.0 14.1, N = 1024 36.8 35.1 32.6 -; dealt back and forth without regard to the load 17.)
+// mode 1 and dealt, products of a graph: 16384^2, N = 256 13.5 12.2, N = 500 28.5 25.3, N = 1024 34.4 31.3; 32768 x 8192, N = 512 27.0 24.0;
+// 8192 x 32768, N = 200 16.6 15.1; 30000 x 3000, N = 60 10.7 8.7; 4096 x 8192, N = 128 8.1 6.0; 2048 x 16384, N = 128 8.6 6.2.  (Launched one by one, 16384^2,
+// N = 256: a piece at 2, 3, 4, 6 row costs 13.5 13.2 13.0 14.8; limits of 1.15, 1.3, 1.5, 2 shares 13.1 13.0 13.0 14.1, N = 1024 36.8 35.1 32.6 -;
+// dealt back and forth without regard to the load 17.)
 constexpr double kDealLimit = 1.5;
 constexpr int kDealMaxSegs = 8192, kDealMaxCtas = 1024;   // sorted and kept in one block's shared memory
 constexpr int kDealThreads = 1024;
@@ -273,7 +274,13 @@ __host__ __device__ inline int deal_pieces(int cnt, int row_cost, int piece, dou
   return k < 2.0 ? 1 : (k < (double)cnt ? (int)k : cnt);
 }
 __host__ __device__ inline int deal_cost(int cnt, int k, int row_cost, int piece) { return k > 1 ? cnt + k * piece : cnt + row_cost; }
-// Rounds that settle the share: pieces make work, which makes the share larger.
+// Rounds in which the share is taken from the work at the share before.  Pieces make work and a larger share makes fewer pieces, so it
+// swings about the one at which the work fits, and an odd number of rounds ends on the high side.  With many rows the two are close
+// (512 rows, two chunks: 40.7, 63.9, 51.6, 54.5; 54.2 fits), with few long ones far apart (64 rows of 27 tiles: 3.8, 28.3, 5.3, 21.0; 11.4
+// fits), and then fewer segments than CTAs are the better plan: 155 against 336 of 592, 2048 x 32768, N = 60 7.6 against 10.1 us.  Three rounds, the
+// share that fits (found by halving), contiguous shares: N = 256 there 7.6 9.5 9.4; 2048 x 16384, N = 128 6.2 8.7 8.6; 4096 x 32768, N = 128 8.0 9.4
+// 9.4; 4096 x 16384, N = 256 8.1 9.3 10.7.  Between, where the segments nearly fill the CTAs, the other way round: 8192 x 16384, N = 256 10.1 9.0
+// 10.9; 8192 x 32768, N = 200 15.1 14.9 16.6.  From two segments per CTA on no difference.
 constexpr int kDealRounds = 3;
 // What a piece costs: four row costs, two where that leaves CTAs without a segment.
 __host__ __device__ inline int deal_piece(int row_cost, int attempt) { return (attempt == 0 ? 4 : 2) * row_cost; }
@@ -423,7 +430,7 @@ __global__ void __launch_bounds__(kDealThreads) deal_kernel(PlanIn in, DealWs ws
     counts[2] = in.n_chunks * ws.split_off[in.nbr];
     counts[3] = (S > capacity || S > kDealMaxSegs) ? 1 : 0;
   }
-  if (S > capacity || S > kDealMaxSegs) {   // (not with the capacity asked for: pieces hold half a share at least)
+  if (S > capacity || S > kDealMaxSegs) {   // (not with the capacity asked for)
     for (int j = tid; j <= G; j += kDealThreads) cta_seg_ptr[j] = 0;
     return;
   }
@@ -578,7 +585,8 @@ int64_t void_plan_capacity(int64_t nnz, int32_t nbr, int32_t n_chunks, int32_t n
   if (nnz < 0 || nbr < 0 || n_chunks <= 0 || n_cta <= 0) return 0;
   int64_t per_chunk = nbr;
   if (split_rows == 2 && chunk_tiles > 0) per_chunk = nnz / chunk_tiles + nbr + 1;
-  if (split_rows == 3) return per_chunk * n_chunks + 2 * (int64_t)n_cta + 2;   // (a piece holds half a share at least)
+  // (a row of cnt tiles makes at most cnt / (share / 2) + 1 segments, and the shares together are no less than all tiles)
+  if (split_rows == 3) return per_chunk * n_chunks + 2 * (int64_t)n_cta + 2;
   return per_chunk * n_chunks + n_cta + 1;
 }
 

@@ -6,10 +6,14 @@ void_spmm_stream_k (:233-301) and analyze_workload_balance (:467-492).
 The worker table is the reference's, bit for bit, but it is built by a device kernel instead of a
 Python loop with one .item() per row (:76-97).  The SpMM differs in how partial rows are joined:
 the reference lets every partial worker lock the output tile and read-modify-write it in the
-output dtype (:198-219, an unbounded spin); here consecutive workers of a row that land on the
-same CTA keep accumulating in tensor memory, rows that are shared between CTAs add their partial
-sums into one accumulator per row with atomic adds, and the CTA that arrives last reads it back
-and runs the epilogue - no lock and no wait.  For an Int8VOIDTensor the sums are int32, exact and
+output dtype (:198-219, an unbounded spin); here rows that are shared between CTAs add their
+partial sums into one accumulator per row with atomic adds, and the CTA that arrives last reads it
+back and runs the epilogue - no lock and no wait.  Without a table, whole rows and pieces of the
+heavy ones are dealt to the CTAs by weight (csrc/plan.cu, mode 3).  With one, the rows in order are
+cut into contiguous shares at the table's chunk boundaries (mode 1): consecutive workers of a row
+that land on the same CTA keep accumulating in tensor memory.  The result is the same, the dealt
+plan is the faster one; products of more segments than one block can sort take shares either way.
+For an Int8VOIDTensor the sums are int32, exact and
 independent of arrival order; for a floating VOIDTensor (the reference's own argument type) they
 are fp32 and their last bits depend on the order, as the reference's locked adds do.
 """
@@ -101,6 +105,10 @@ def void_spmm_stream_k(a: Int8VOIDTensor, b: torch.Tensor, workload: Optional[St
     ``worker_partials`` (int32 [n_segments, 32, N], see the plan's segment list) makes every worker of
     the table a segment of its own and records its partial sum - the check that the sum of the
     partials is the row accumulator.
+
+    Inside a stream capture the product takes a work plan that is kept for its width and its tile
+    list; where there is none it is refused (so is a list made in inference mode, which leaves no trace of
+    its edits).  A replay of a product that was packed inside its capture needs the list as it was then.
     """
     assert b.dim() == 2
     assert a.shape[1] == b.shape[0]
@@ -144,10 +152,10 @@ def _stream_k_fp(a: VOIDTensor, b, workload, out, activation, bias, worker_parti
                          worker_partials=worker_partials)
 
 
-def stream_k_plan(a, N: int, workload: StreamKWorkload, per_worker: bool = False, n_cta: Optional[int] = None,
+def stream_k_plan(a, N: int, workload: Optional[StreamKWorkload], per_worker: bool = False, n_cta: Optional[int] = None,
                   kind: Optional[int] = None) -> _spmm.Plan:
-    """The device-built work plan void_spmm_stream_k uses for an N-column product (``kind``: the
-    product kind of a floating VOIDTensor, fp32 operands by default)."""
+    """The device-built work plan that void_spmm_stream_k uses for an N-column product with this ``workload``; None: without
+    one, which is another plan (``kind``: the product kind of a floating VOIDTensor, fp32 operands by default)."""
     if isinstance(a, VOIDTensor):
         from . import ops
         packed = ops.packed_fp(a, _lib.FP_KIND.get(a.values.dtype, _lib.KIND_TF32) if kind is None else kind)
